@@ -132,6 +132,80 @@ def run(state):
     return [o.detach(), *rest, *grads]
 
 
+def _exact_tdp(case, ins, dz, alpha):
+    """Dense fp64 triple-dot-product, in chunks of queries: the output and, for a training step, the five gradients."""
+    T, causal = case["T"], case["causal"]
+    w1, w2, kl, kr = (min(case[k] or T, T) for k in ("k1w", "k2w", "kkl", "kkr"))
+    Q, K1, K2, V1, V2 = ins
+    sig = torch.sigmoid(V1)
+    S1 = V1 * sig
+    O = torch.zeros_like(Q)
+    dQ, dK1, dK2, dS1, dV2 = (torch.zeros_like(Q) for _ in range(5))
+    n = max(1, min(64, int(6e7 / min(T, max(w1, w2) + 64) ** 2)))
+    for h in range(Q.shape[0]):
+        for a in range(0, T, n):
+            b = min(T, a + n)
+            j0, k0, end = (max(0, a - w1), max(0, a - w2), b) if causal else (0, 0, T)
+            k1, s1, k2, v2 = K1[h, j0:end], S1[h, j0:end], K2[h, k0:end], V2[h, k0:end]
+            A = alpha * Q[h, a:b, None] * k2                                     # [q, k, h]
+            P = A @ k1.T                                                         # [q, k, j]
+            if causal:
+                q = torch.arange(a, b, device=Q.device)[:, None]
+                j, k = (torch.arange(x, end, device=Q.device) for x in (j0, k0))
+                ok = ((k <= q) & (q - k <= w2))[:, :, None] & ((j <= q) & (q - j <= w1))[:, None, :]
+                ok &= ((j >= k[:, None] - kl) & (j <= k[:, None] + kr))
+                P.masked_fill_(~ok, -math.inf)
+            P.sub_(P.amax((1, 2), keepdim=True)).exp_()
+            P.div_(P.sum((1, 2), keepdim=True))
+            U = P @ s1
+            O[h, a:b] = (U * v2).sum(1)
+            if case["mode"] == "fwd":
+                continue
+            do = dz[h, a:b, None]
+            A2 = do * v2
+            dV2[h, k0:end] += (U * do).sum(0)
+            dS1[h, j0:end] += P.flatten(0, 1).T @ A2.flatten(0, 1)
+            dP = A2 @ s1.T
+            dP.sub_((do[:, 0] * O[h, a:b]).sum(-1)[:, None, None]).mul_(P)       # the scores' gradient
+            G = alpha * (dP @ k1)
+            dQ[h, a:b] = (G * k2).sum(1)
+            dK2[h, k0:end] += (G * Q[h, a:b, None]).sum(0)
+            dK1[h, j0:end] += dP.flatten(0, 1).T @ A.flatten(0, 1)
+    if case["mode"] == "fwd":
+        return [O]
+    return [O, dQ, dK1, dK2, dS1 * (sig + S1 * (1 - sig)), dV2]
+
+
+def _exact_dps(case, ins, dz, alpha):
+    """Dense fp64 dot-product-sum: the soft-max over (s, t) as two chained ones, autograd for the gradients."""
+    T = case["T"]
+    ins = [x.requires_grad_(True) for x in ins]
+    Q, K1, K2, V1, V2 = ins
+    t = torch.arange(T, device=Q.device)
+    E, F = alpha * (K2 @ K1.transpose(1, 2)), alpha * (Q @ K2.transpose(1, 2))   # [t, s], [q, t]
+    if case["causal"]:
+        kd = case["k_diff"] or T
+        E = E.masked_fill(~((t <= t[:, None]) & (t[:, None] - t <= kd)), -math.inf)
+        F = F.masked_fill(t > t[:, None], -math.inf)
+    F = F + torch.logsumexp(E, -1)[:, None]
+    o = torch.softmax(F, -1) @ (torch.softmax(E, -1) @ torch.nn.functional.silu(V1) * V2)
+    out = [o, torch.logsumexp(F, -1)]
+    if case["mode"] == "train":
+        out += torch.autograd.grad(o, ins, dz)
+    return [x.detach() for x in out]
+
+
+def exact(case, seed):
+    """The outputs of ``run`` for the same inputs by plain fp64 tensor algebra."""
+    state = prepare(case, seed)
+    alpha = 1.0 / case["D"] if case["dist"] == "half" else 1.0 / 8.0
+    shape = state["dz"].shape
+    ins = [x.detach().double().flatten(0, 1) for x in state["ins"]]
+    dz = state["dz"].double().flatten(0, 1)
+    out = (_exact_dps if case["op"] == "dps" else _exact_tdp)(case, ins, dz, alpha)
+    return [x.unflatten(0, shape[:2]) for x in out]
+
+
 def _attended(case):
     """Attended (q, j, k) triples of one head (tdp), or pairs of the two chained attentions (dps)."""
     T = case["T"]
