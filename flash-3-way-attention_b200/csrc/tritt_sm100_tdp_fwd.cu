@@ -76,7 +76,11 @@ struct FwdBarriers {
   uint64_t ring_full[4], ring_empty[4];
   uint64_t k2_full, a_ready, a_free;
   uint64_t s_ready[2], p_ready[2];               // per tile, one phase per slab
-  uint64_t o_done, o_free[2], stats_ready[2];    // per k-tile hand-offs with the fold warpgroup
+  // Per k-tile hand-offs with the fold warpgroup.  stats_ready is doubled by k-tile parity: with one slab per k-tile
+  // (short sequences, narrow windows) the soft-max warps can hand over the next k-tile's statistics before the fold
+  // warpgroup, still storing the previous item, has looked at this one's, and a barrier two phases ahead of its waiter
+  // reads as not ready for ever.
+  uint64_t o_done, o_free[2], stats_ready[2][2];
   uint64_t fold_sync;
   uint32_t tmem_base;
   int abort_flag;
@@ -112,7 +116,8 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
       mbar_init(&bars.s_ready[x], 1);
       mbar_init(&bars.p_ready[x], 256);
       mbar_init(&bars.o_free[x], 128);
-      mbar_init(&bars.stats_ready[x], 256);
+      mbar_init(&bars.stats_ready[0][x], 256);
+      mbar_init(&bars.stats_ready[1][x], 256);
     }
     mbar_init(&bars.o_done, 1);
     mbar_init(&bars.fold_sync, 128);
@@ -560,7 +565,7 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
             } else {
               srow[2] = l_sum[x];
             }
-            mbar_arrive(&bars.stats_ready[x]);
+            mbar_arrive(&bars.stats_ready[kt_count & 1][x]);
           }
         } else {
           // ---- walk over the slabs, one warpgroup per tile (warpgroup 0: tile a), one whole row per thread: row
@@ -631,7 +636,7 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
           srow[0] = m_used;
           srow[1] = l_sum;
           srow[2] = 0.f;
-          mbar_arrive_n(&bars.stats_ready[x], 2);
+          mbar_arrive_n(&bars.stats_ready[kt_count & 1][x], 2);
         }
       }
       if (!alive) break;
@@ -669,7 +674,7 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
         bool valid[2];
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
-          alive = alive && __all_sync(0xffffffffu, mbar_wait(&bars.stats_ready[x], par, abort_flag));
+          alive = alive && __all_sync(0xffffffffu, mbar_wait(&bars.stats_ready[par][x], (kt_count >> 1) & 1, abort_flag));
           if (!alive) break;
           const float* srow = stats + ((par * 2 + x) * 128 + row) * 4;
           m_r[x] = srow[0];

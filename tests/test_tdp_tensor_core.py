@@ -317,6 +317,25 @@ def test_windows_with_query_shards(windows):
         assert_close(name + " (shards vs whole)", a, b, torch.bfloat16)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("scale", [0.5, 1.0])
+def test_forward_of_many_one_slab_items(D, scale):
+    """Items of a single k-tile with a single slab follow one another as fast as the roles can hand them over: no wait
+    may miss a phase (a wait that does runs out and sets the status word), and every launch gives the same output."""
+    B, N, T = 8, 16, 100
+    q, k1, k2, v1, v2, _ = orc.make_inputs(B, N, T, D, scale=scale, seed=5 + D, dtype=torch.bfloat16)
+    t = [x.to(DEV) for x in (q, k1, k2, v1, v2)]
+    outs = [torch.empty_like(t[0]) for _ in range(2)]
+    lse = torch.empty(B, N, T, device=DEV)
+    alpha = 1.0 / D if scale == 0.5 else 1 / 8
+    _native.tdp_fwd(*t, outs[0], lse, alpha, True, None, None, None, None)
+    for _ in range(200):
+        _native.tdp_fwd(*t, outs[1], lse, alpha, True, None, None, None, None)
+    torch.cuda.synchronize()
+    assert _native.read_status(torch.device(DEV)) == 0, "a bounded barrier wait ran out"
+    assert torch.equal(outs[0], outs[1])
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_forward_with_and_without_the_score_bound(dtype):
     """The forward takes the score bound |A_row| max|K1_j| as soft-max reference when the workspace has the tail for
