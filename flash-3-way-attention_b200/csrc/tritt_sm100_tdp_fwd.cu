@@ -773,80 +773,111 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
   if (tid == 0 && bars.abort_flag && p.status) atomicOr(p.status, 2);
 }
 
-// Per-head statistics behind the score bounds, over the rows r of the three [BN*T, D] tensors:
-//   out[bh] = max_j |K1[bh, j, :]|^2,  out[BN + bh] = max_q |Q[bh, q, :]|^2,  out[2 BN + bh] = max element^2 of K2[bh]
-// (fp32, compared as integers: non-negative floats order like their bit patterns).  A warp takes kStatRows
-// consecutive rows and issues its three atomics once per head it met, not once per row.  `out` must be zero on entry.
-constexpr int kStatRows = 8;
+// What both forward kernels need before they start, in one pass over the tensors: SiLU(V1) in the inputs' type and, when
+// `stats` is not null, the per-head statistics behind the score bounds,
+//   stats[bh] = max_j |K1[bh, j, :]|^2,  stats[BN + bh] = max_q |Q[bh, q, :]|^2,  stats[2 BN + bh] = max element^2 of K2[bh].
+// A cluster of blocks takes one head: the maxima meet in the first block's shared memory, so that no launch has to
+// zero anything and no atomics are needed.  8 elements per thread and step; a row is held by D / 8 neighbouring lanes.
+constexpr int kPrepThreads = 256;
 template <typename T16>
-__global__ void head_stats_kernel(const T16* __restrict__ k1, const T16* __restrict__ q, const T16* __restrict__ k2,
-                                  float* __restrict__ out, size_t rows, int T, int D, int BN) {
-  const size_t w = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const size_t r0 = w * kStatRows;
-  if (r0 >= rows) return;
-  const size_t r1 = r0 + kStatRows < rows ? r0 + kStatRows : rows;
-  float m1 = 0.f, mq = 0.f, m2 = 0.f;   // maxima over the rows of the current head
-  size_t bh = r0 / T;
-  auto flush = [&]() {
-    if (lane == 0) {
-      atomicMax(reinterpret_cast<int*>(out + bh), __float_as_int(m1));
-      atomicMax(reinterpret_cast<int*>(out + BN + bh), __float_as_int(mq));
-      atomicMax(reinterpret_cast<int*>(out + 2 * (size_t)BN + bh), __float_as_int(m2));
-    }
-  };
-  for (size_t r = r0; r < r1; ++r) {
-    if (r / T != bh) {
-      flush();
-      bh = r / T;
-      m1 = mq = m2 = 0.f;
-    }
-    const uint32_t* s1 = reinterpret_cast<const uint32_t*>(k1 + r * D);
-    const uint32_t* sq = reinterpret_cast<const uint32_t*>(q + r * D);
-    const uint32_t* s2 = reinterpret_cast<const uint32_t*>(k2 + r * D);
-    float n1 = 0.f, nq = 0.f, e2 = 0.f;
-    for (int i = lane; i < D / 2; i += 32) {
-      const float2 a = unpack2<T16>(s1[i]), b = unpack2<T16>(sq[i]), c = unpack2<T16>(s2[i]);
-      n1 = fmaf(a.x, a.x, fmaf(a.y, a.y, n1));
-      nq = fmaf(b.x, b.x, fmaf(b.y, b.y, nq));
-      e2 = fmaxf(e2, fmaxf(c.x * c.x, c.y * c.y));
-    }
+__global__ void __launch_bounds__(kPrepThreads)
+fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const T16* __restrict__ q,
+                   const T16* __restrict__ k2, T16* __restrict__ sv1, float* __restrict__ stats, int head_elems, int D,
+                   int BN, int blocks) {
+  __shared__ float red[8][3];           // [block of the cluster]; used in the first block
+  __shared__ float wred[kPrepThreads / 32][3];
+  const int bh = blockIdx.x / blocks, part = blockIdx.x % blocks;
+  const size_t base = (size_t)bh * head_elems;
+  const int lanes = D / 8;
+  float m1 = 0.f, mq = 0.f, m2 = 0.f;
+  // (the bound is the same for all lanes of a row: head_elems is a multiple of D)
+  for (int i = (part * kPrepThreads + threadIdx.x) * 8; i < head_elems; i += blocks * kPrepThreads * 8) {
+    const uint4 v = *reinterpret_cast<const uint4*>(v1 + base + i);
+    const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
+    uint32_t o[4];
 #pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-      n1 += __shfl_xor_sync(0xffffffffu, n1, o);
-      nq += __shfl_xor_sync(0xffffffffu, nq, o);
-      e2 = fmaxf(e2, __shfl_xor_sync(0xffffffffu, e2, o));
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = unpack2<T16>(wv[e]);
+      o[e] = pack2<T16>(silu_f(f.x), silu_f(f.y));
     }
-    m1 = fmaxf(m1, n1);
-    mq = fmaxf(mq, nq);
-    m2 = fmaxf(m2, e2);
+    *reinterpret_cast<uint4*>(sv1 + base + i) = make_uint4(o[0], o[1], o[2], o[3]);
+    if (stats) {
+      const uint4 a = *reinterpret_cast<const uint4*>(k1 + base + i), b = *reinterpret_cast<const uint4*>(q + base + i),
+                  c = *reinterpret_cast<const uint4*>(k2 + base + i);
+      const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w}, wc[4] = {c.x, c.y, c.z, c.w};
+      float n1 = 0.f, nq = 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 x = unpack2<T16>(wa[e]), y = unpack2<T16>(wb[e]), z = unpack2<T16>(wc[e]);
+        n1 = fmaf(x.x, x.x, fmaf(x.y, x.y, n1));
+        nq = fmaf(y.x, y.x, fmaf(y.y, y.y, nq));
+        m2 = fmaxf(m2, fmaxf(z.x * z.x, z.y * z.y));
+      }
+      // (the lanes of a row are all here or all gone; which lanes of the warp are is not the same everywhere)
+      const uint32_t row_lanes = ((lanes == 32 ? 0u : 1u << lanes) - 1u) << ((threadIdx.x & 31) / lanes * lanes);
+      for (int o2 = lanes / 2; o2 >= 1; o2 >>= 1) {
+        n1 += __shfl_xor_sync(row_lanes, n1, o2);
+        nq += __shfl_xor_sync(row_lanes, nq, o2);
+      }
+      m1 = fmaxf(m1, n1);
+      mq = fmaxf(mq, nq);
+    }
   }
-  flush();
+  if (!stats) return;
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+    mq = fmaxf(mq, __shfl_xor_sync(0xffffffffu, mq, o));
+    m2 = fmaxf(m2, __shfl_xor_sync(0xffffffffu, m2, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    wred[threadIdx.x >> 5][0] = m1;
+    wred[threadIdx.x >> 5][1] = mq;
+    wred[threadIdx.x >> 5][2] = m2;
+  }
+  cluster_sync_all();   // every block of the cluster runs: its shared memory may be written (a block barrier as well)
+  if (threadIdx.x < 3) {
+    float m = 0.f;
+#pragma unroll
+    for (int w = 0; w < kPrepThreads / 32; ++w) m = fmaxf(m, wred[w][threadIdx.x]);
+    uint32_t dst;   // the first block's red[part][.]
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(&red[part][threadIdx.x])), "r"(0));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(m) : "memory");
+  }
+  cluster_sync_all();
+  if (part == 0 && threadIdx.x < 3) {
+    float m = 0.f;
+    for (int c = 0; c < blocks; ++c) m = fmaxf(m, red[c][threadIdx.x]);
+    stats[(size_t)threadIdx.x * BN + bh] = m;
+  }
 }
 
-// What both forward kernels need before they start: SiLU(V1) in the inputs' type at the head of the workspace and,
-// when the workspace has the optional tail, the per-head statistics of head_stats_kernel (for the score bounds; the
-// returned pointer is to the first of its three arrays of B*N values, the K1 row norms).
+// SiLU(V1) at the head of the workspace and, when the workspace has the optional tail, the statistics (the returned
+// pointer is to the first of its three arrays of B*N values, the K1 row norms).
 template <typename T16>
 int prepare_fwd(const TdpArgs& a, T16** sv1_out, float** k1n_out) {
   const int BN = a.B * a.N;
-  const size_t n = (size_t)BN * a.T * a.D;
+  const size_t n = (size_t)BN * a.T * a.D, tail = align_up(n * 2, 256);
   T16* sv1 = (T16*)a.workspace;
-  silu_kernel<T16><<<(unsigned)((n / 8 + 255) / 256 + 1), 256, 0, a.stream>>>((const T16*)a.v1, sv1, n);
-  count_launch();
-  TRITT_CUDA_OK(cudaGetLastError());
   float* k1n = nullptr;
-  const size_t tail = align_up(n * 2, 256);
-  if (a.workspace_bytes >= tail + 3 * (size_t)BN * sizeof(float)) {
-    k1n = reinterpret_cast<float*>((char*)a.workspace + tail);
-    TRITT_CUDA_OK(cudaMemsetAsync(k1n, 0, 3 * (size_t)BN * sizeof(float), a.stream));
-    const size_t rows = (size_t)BN * a.T;
-    const size_t warps = (rows + kStatRows - 1) / kStatRows;
-    head_stats_kernel<T16><<<(unsigned)((warps + 7) / 8), 256, 0, a.stream>>>((const T16*)a.k1, (const T16*)a.q,
-                                                                             (const T16*)a.k2, k1n, rows, a.T, a.D, BN);
-    count_launch();
-    TRITT_CUDA_OK(cudaGetLastError());
-  }
+  if (a.workspace_bytes >= tail + 3 * (size_t)BN * sizeof(float)) k1n = reinterpret_cast<float*>((char*)a.workspace + tail);
+  const int head_elems = a.T * a.D;
+  int blocks = 1;
+  while (blocks < 8 && blocks * kPrepThreads * 8 < head_elems) blocks *= 2;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = blocks;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)(BN * blocks), 1, 1);
+  cfg.blockDim = dim3(kPrepThreads, 1, 1);
+  cfg.stream = a.stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  TRITT_CUDA_OK(cudaLaunchKernelEx(&cfg, fwd_prepare_kernel<T16>, (const T16*)a.v1, (const T16*)a.k1, (const T16*)a.q,
+                                   (const T16*)a.k2, sv1, k1n, head_elems, a.D, BN, blocks));
+  count_launch();
   *sv1_out = sv1;
   *k1n_out = k1n;
   return 0;
