@@ -170,32 +170,27 @@ int sm100_silu_16(const void* in, void* out, size_t n, int dtype, cudaStream_t s
 struct AttnBwdTcArgs {
   const void *xq, *kc, *vc, *dout;  // 16-bit [BN, T, D]
   const float *bias, *lse, *drow;   // [BN, T]: per column (or null), per row, per row
-  // row owner: with `out_rows` (the attention's 16-bit output) drow[r] = dout[r] . out_rows[r] is computed by the
-  // kernel, used, and stored to `drow_out` for the column-owner launch that follows
-  const void* out_rows;
-  float* drow_out;
+  // row owner
   void* d_rows_t;
   const float* d_rows_add;          // [BN, T, D] or null
+  // column owner: one of d_kc_f32, d_kc_t, and one of the two forms of the value gradient d_vc
   float* d_kc_f32;
   void* d_kc_t;
-  float* d_vc_f32;                  // column owner: sum_r P dout, fp32, or null when one of the two forms below is asked
-  // column owner, instead of d_vc_f32: d_vc_t = d_vc * SiLU'(silu_src)  (16-bit; silu_src = the raw value tensor)
+  // d_vc_t = d_vc * SiLU'(silu_src)  (16-bit; silu_src = the raw value tensor)
   const void* silu_src;
   void* d_vc_t;
-  // column owner, instead of d_vc_f32 (with dW = d_vc): mid_dv2 = dW * mid_y, mid_dy_t = dW * mid_v2 (both 16-bit),
-  // mid_dt[c] = sum_h (dW mid_v2 mid_y)[c, h] - gsum[c]
+  // with dW = d_vc: mid_dv2 = dW * mid_y, mid_dy_t = dW * mid_v2 (both 16-bit),
+  // mid_dt[c] = sum_h (dW mid_v2 mid_y)[c, h] - sum_r dS[r, c]
   const float* mid_y;
   const void* mid_v2;
   void *mid_dv2, *mid_dy_t;
   float* mid_dt;
-  float* gsum;                      // [BN, T] or null
   int BN, T, D, dtype, causal, win;
   float alpha;
   int* status;
   cudaStream_t stream;
 };
-int sm100_attn_bwd_rows(const AttnBwdTcArgs& a);
-int sm100_attn_bwd_cols(const AttnBwdTcArgs& a);
+int sm100_attn_bwd(const AttnBwdTcArgs& a);
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 

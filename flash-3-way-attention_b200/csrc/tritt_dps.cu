@@ -111,36 +111,33 @@ int dps_bwd_tensor_cores(const DpsArgs& a, const DpsWs& w) {
   int rc = 0;
   // Y, LSEin, SiLU(V1), Y*V2: taken from the forward's workspace when the caller kept it, else computed again
   if (!a.fwd_state && (rc = dps_fwd_tensor_cores(a, w, true))) return rc;
-  // ---- outer attention: rows q (Q), columns t (K2, W = Y*V2, bias LSEin).  The row owner also forms
-  // Dq = sum_h dO O per query and leaves it for the column owner; the column owner's epilogue turns dW into
+  // Dq = sum_h dO O per query, for both kinds of owner
+  const size_t r = (size_t)a.B * a.N * a.T;
+  rowdot_kernel<T><<<(unsigned)((r + 3) / 4), 128, 0, a.stream>>>((const T*)a.d_o, (const T*)a.o, w.Dq, r, a.D);
+  count_launch();
+  TRITT_CUDA_OK(cudaGetLastError());
+  // ---- outer attention: rows q (Q), columns t (K2, W = Y*V2, bias LSEin).  The column owner's epilogue turns dW into
   // dV2 = dW * Y, dY = dW * V2 and the inner attention's row term Dt = sum_h dY Y - sum_q dS.
   AttnBwdTcArgs o{};
   o.xq = a.q; o.kc = a.k2; o.vc = w.w_16; o.dout = a.d_o;
   o.bias = w.lse_in; o.lse = a.m_in; o.drow = w.Dq;
   o.BN = a.B * a.N; o.T = a.T; o.D = a.D; o.dtype = a.dtype; o.causal = a.causal; o.win = a.T;
   o.alpha = a.alpha; o.status = a.status_word; o.stream = a.stream;
-  AttnBwdTcArgs orow = o;
-  orow.d_rows_t = a.dq;
-  orow.out_rows = a.o; orow.drow_out = w.Dq;
-  if ((rc = sm100_attn_bwd_rows(orow))) return rc;
-  AttnBwdTcArgs ocol = o;
-  ocol.d_kc_f32 = w.dK2a;
-  ocol.mid_y = w.Y; ocol.mid_v2 = a.v2; ocol.mid_dv2 = a.dv2; ocol.mid_dy_t = w.dy_16; ocol.mid_dt = w.Dt;
-  if ((rc = sm100_attn_bwd_cols(ocol))) return rc;
+  o.d_rows_t = a.dq;
+  o.d_kc_f32 = w.dK2a;
+  o.mid_y = w.Y; o.mid_v2 = a.v2; o.mid_dv2 = a.dv2; o.mid_dy_t = w.dy_16; o.mid_dt = w.Dt;
+  if ((rc = sm100_attn_bwd(o))) return rc;
   // ---- inner attention: rows t (K2), columns s (K1, SiLU(V1)); upstream gradient dY
   AttnBwdTcArgs i{};
   i.xq = a.k2; i.kc = a.k1; i.vc = w.sv1_16; i.dout = w.dy_16;
   i.lse = w.lse_in; i.drow = w.Dt;
   i.BN = a.B * a.N; i.T = a.T; i.D = a.D; i.dtype = a.dtype; i.causal = a.causal; i.win = a.k_diff;
   i.alpha = a.alpha; i.status = a.status_word; i.stream = a.stream;
-  AttnBwdTcArgs irow = i;
-  irow.d_rows_t = a.dk2;      // dK2 = (as outer key) + (as inner query)
-  irow.d_rows_add = w.dK2a;
-  if ((rc = sm100_attn_bwd_rows(irow))) return rc;
-  AttnBwdTcArgs icol = i;
-  icol.d_kc_t = a.dk1;
-  icol.silu_src = a.v1; icol.d_vc_t = a.dv1;  // dV1 = dSiLU(V1) * SiLU'(V1) in the epilogue
-  return sm100_attn_bwd_cols(icol);
+  i.d_rows_t = a.dk2;      // dK2 = (as outer key) + (as inner query)
+  i.d_rows_add = w.dK2a;
+  i.d_kc_t = a.dk1;
+  i.silu_src = a.v1; i.d_vc_t = a.dv1;  // dV1 = dSiLU(V1) * SiLU'(V1) in the epilogue
+  return sm100_attn_bwd(i);
 }
 
 template <typename T>

@@ -10,10 +10,14 @@
 // reference splits its backward the same way, a query-owner kernel and a key-owner kernel:
 // dot_product_sum/kernels/bwd_dq_kernel.py:28-350, bwd_dk1_dv1_kernel.py:29-416.)
 //
-// Roles per CTA (256 threads): warp 0 TMA producer (the owner's two operand tiles once, then a two-stage ring of
+// Both kinds of owner run in ONE launch (they only read what earlier launches left), heaviest tiles first: the chain
+// of a long owner tile then overlaps the other kind's, and SMs that a single kind leaves idle have work.
+//
+// Roles per CTA (384 threads): warp 0 TMA producer (the owner's two operand tiles once, then a two-stage ring of
 // the other side's two tiles), warp 1 issues tcgen05.mma (S and dP into TMEM; then the accumulations with P / dS
-// read from TMEM, 16-bit, over the columns of S / dP, and the ring tile used row-major), warps 4-7 one owner row
-// per thread (P and dS from S, dP and the row / column vectors; epilogue).
+// read from TMEM, 16-bit, over the columns of S / dP, and the ring tile used row-major), warps 4-7 and 8-11 one owner
+// row per thread, half of a tile's columns each (P and dS from S, dP and the row / column vectors; half of the
+// epilogue's columns each).
 #include "tritt_common.cuh"
 #include "tritt_sm100.cuh"
 #include "tritt_sm100_tdp.cuh"
@@ -24,23 +28,22 @@ namespace tritt {
 namespace {
 using namespace sm100;
 
-constexpr int kAttnBwdThreads = 256;
+constexpr int kAttnBwdThreads = 384;
 
 template <int D> struct AttnBwdCfg {
   static constexpr int kTile = 128 * D * 2;
   static constexpr int kStages = 2;
   static constexpr int kOffOwn = 0;                  // owner tiles: [0] keys side (X or K), [1] values side (dOut or V)
   static constexpr int kOffRing = 2 * kTile;         // stage s: tiles [0], [1] of the other side
-  static constexpr int kOffVec = kOffRing + kStages * 2 * kTile;  // [4 warps][2 parities][2 vectors][128] fp32
-  static constexpr int kOffBars = kOffVec + 4 * 2 * 2 * 128 * 4;
+  static constexpr int kOffVec = kOffRing + kStages * 2 * kTile;  // [8 warps][2 parities][2 vectors][64] fp32
+  static constexpr int kOffPart = kOffVec + 8 * 2 * 2 * 64 * 4;   // [128] fp32: the second warpgroup's row terms
+  static constexpr int kOffBars = kOffPart + 128 * 4;
   static constexpr int kSmem = kOffBars + 128;
   static constexpr int kTmemS = 0, kTmemDP = 128, kTmemAcc0 = 256, kTmemAcc1 = 256 + D;
 };
 
 struct AttnBwdParams {
   const float *bias, *lse, *drow;  // per column (or null); per row; per row
-  const void *out_rows, *dout_rows;  // row-owner: drow = dout . out computed here (then drow is not read) ...
-  float* drow_out;                   // ... and stored for the column-owner launch
   const void* silu_src;            // column-owner epilogue variants (see AttnBwdTcArgs)
   void* d_vc_t;
   const float* mid_y;
@@ -51,8 +54,6 @@ struct AttnBwdParams {
   const float* d_rows_add;         // row-owner: fp32 term added before rounding, or null
   float* d_kc_f32;                 // column-owner: one of the two
   void* d_kc_t;
-  float* d_vc_f32;                 // column-owner
-  float* gsum;                     // column-owner, or null
   int T, causal, win;
   float scale2, alpha;             // alpha log2(e); alpha
   int* status;
@@ -60,16 +61,15 @@ struct AttnBwdParams {
 
 struct AttnBwdBarriers {
   uint64_t ring_full[2], ring_empty[2];
-  uint64_t own_full, sd_ready, pd_ready, acc_done;
+  uint64_t own_full, sd_ready, pd_ready, acc_done, part_ready;
   uint32_t tmem_base;
   int abort_flag;
 };
 
+// One owner tile: `ot` of head `bh`; Own0 / Own1 and Oth0 / Oth1 are the operand tensors of the owner and of the other side.
 template <int D, typename T16, bool COL>
-__global__ void __launch_bounds__(kAttnBwdThreads, 1)
-attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmOwn0, const __grid_constant__ CUtensorMap tmOwn1,
-                      const __grid_constant__ CUtensorMap tmOth0, const __grid_constant__ CUtensorMap tmOth1,
-                      AttnBwdParams p) {
+__device__ __forceinline__ void attn_bwd_tile(const CUtensorMap& tmOwn0, const CUtensorMap& tmOwn1, const CUtensorMap& tmOth0,
+                                              const CUtensorMap& tmOth1, const AttnBwdParams& p, const int bh, const int ot) {
   using Cfg = AttnBwdCfg<D>;
   constexpr int NS = Cfg::kStages;
   constexpr int KH = D / 64;
@@ -89,8 +89,9 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmOwn0, const __grid_c
     }
     mbar_init(&bars.own_full, 1);
     mbar_init(&bars.sd_ready, 1);
-    mbar_init(&bars.pd_ready, 128);
+    mbar_init(&bars.pd_ready, 256);
     mbar_init(&bars.acc_done, 1);
+    mbar_init(&bars.part_ready, 128);
     fence_barrier_init();
   }
   if (warp == 0) {
@@ -105,9 +106,6 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmOwn0, const __grid_c
 
   const int T = p.T;
   const int n_tiles = (T + 127) / 128;
-  const int bh = blockIdx.y;
-  // the owner tiles with the most work start first: the last rows / the first columns under the causal mask
-  const int ot = COL ? (int)blockIdx.x : n_tiles - 1 - (int)blockIdx.x;
   const int o0 = ot * 128;
   const bool banded = p.causal && p.win < T;
   // tiles of the other side that hold an attended entry of this tile
@@ -194,7 +192,7 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmOwn0, const __grid_c
         }
         commit(&bars.sd_ready);
       };
-      // accumulations with the 16-bit P / dS read from TMEM and the ring tiles used row-major
+      // accumulations with the 16-bit P / dS read from TMEM (each warpgroup's over the first half of its 64 columns) and the ring tiles used row-major
       auto issue_acc = [&](int st, uint32_t acc) {
         const uint32_t m0 = desc_lo(smem_u32(smem + Cfg::kOffRing + st * 2 * Cfg::kTile), 16384);
         const uint32_t m1 = desc_lo(smem_u32(smem + Cfg::kOffRing + st * 2 * Cfg::kTile + Cfg::kTile), 16384);
@@ -203,19 +201,19 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmOwn0, const __grid_c
 #pragma unroll
           for (int k = 0; k < 8; ++k)
             if (leader)
-              mma_ts_lo(tmem + Cfg::kTmemAcc0, tmem + Cfg::kTmemS + k * 8, m1 + k * (2048 >> 4), kHi, idesc_acc,
+              mma_ts_lo(tmem + Cfg::kTmemAcc0, tmem + Cfg::kTmemS + (k >> 2) * 64 + (k & 3) * 8, m1 + k * (2048 >> 4), kHi, idesc_acc,
                         k > 0 ? 1u : acc);
 #pragma unroll
           for (int k = 0; k < 8; ++k)
             if (leader)
-              mma_ts_lo(tmem + Cfg::kTmemAcc1, tmem + Cfg::kTmemDP + k * 8, m0 + k * (2048 >> 4), kHi, idesc_acc,
+              mma_ts_lo(tmem + Cfg::kTmemAcc1, tmem + Cfg::kTmemDP + (k >> 2) * 64 + (k & 3) * 8, m0 + k * (2048 >> 4), kHi, idesc_acc,
                         k > 0 ? 1u : acc);
         } else {
           // d_rows += dS * K
 #pragma unroll
           for (int k = 0; k < 8; ++k)
             if (leader)
-              mma_ts_lo(tmem + Cfg::kTmemAcc0, tmem + Cfg::kTmemDP + k * 8, m0 + k * (2048 >> 4), kHi, idesc_acc,
+              mma_ts_lo(tmem + Cfg::kTmemAcc0, tmem + Cfg::kTmemDP + (k >> 2) * 64 + (k & 3) * 8, m0 + k * (2048 >> 4), kHi, idesc_acc,
                         k > 0 ? 1u : acc);
         }
       };
@@ -241,14 +239,15 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmOwn0, const __grid_c
     }
   } else if (warp >= 4) {
     // ------------------------------------------------------------------ P, dS and the epilogue: one owner row per thread
-    const int wq = warp & 3;
+    const int wg = (warp - 4) >> 2, wq = warp & 3;
     const int row = wq * 32 + lane;
     const int own = o0 + row;
     const bool own_ok = own < T;
     const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
-    const uint32_t tS = tmem + lane_base + Cfg::kTmemS;
-    const uint32_t tD = tmem + lane_base + Cfg::kTmemDP;
-    float* svec = reinterpret_cast<float*>(smem + Cfg::kOffVec) + wq * 2 * 2 * 128;
+    const uint32_t tS = tmem + lane_base + Cfg::kTmemS + wg * 64;
+    const uint32_t tD = tmem + lane_base + Cfg::kTmemDP + wg * 64;
+    float* svec = reinterpret_cast<float*>(smem + Cfg::kOffVec) + (warp - 4) * 2 * 2 * 64;
+    float* part = reinterpret_cast<float*>(smem + Cfg::kOffPart);
     // the owner's scalars
     float own_a = 0.f, own_b = 0.f;
     if (own_ok) {
@@ -256,26 +255,7 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmOwn0, const __grid_c
         own_a = p.bias ? __ldg(p.bias + (size_t)bh * T + own) * kLog2e : 0.f;
       } else {
         own_a = __ldg(p.lse + (size_t)bh * T + own) * kLog2e;
-        if (p.out_rows) {
-          // drow = sum_h dOut[own, h] Out[own, h]  (the reference's preprocess kernel, bwd_preprocess.py:5-49)
-          const uint4* a4 = reinterpret_cast<const uint4*>((const T16*)p.dout_rows + ((size_t)bh * T + own) * D);
-          const uint4* b4 = reinterpret_cast<const uint4*>((const T16*)p.out_rows + ((size_t)bh * T + own) * D);
-          float acc = 0.f;
-#pragma unroll
-          for (int i = 0; i < D / 8; ++i) {
-            const uint4 av = __ldg(a4 + i), bv = __ldg(b4 + i);
-            const uint32_t aw[4] = {av.x, av.y, av.z, av.w}, bw[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 fa = unpack2<T16>(aw[e]), fb = unpack2<T16>(bw[e]);
-              acc = fmaf(fa.x, fb.x, fmaf(fa.y, fb.y, acc));
-            }
-          }
-          own_b = acc;
-          p.drow_out[(size_t)bh * T + own] = acc;
-        } else {
-          own_b = __ldg(p.drow + (size_t)bh * T + own);
-        }
+        own_b = __ldg(p.drow + (size_t)bh * T + own);
       }
     }
     // attended indices of the other side for this owner: [j_lo, j_hi]
@@ -293,19 +273,19 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmOwn0, const __grid_c
     float gs = 0.f;
     bool alive = true;
     for (int i = 0; i < n_t; ++i) {
-      const int j0 = (t0 + i) * 128;
+      const int j0 = (t0 + i) * 128 + wg * 64;
       // per-index vectors of the other side (log2 units where they enter the exponent), staged per warp
-      float* va = svec + (i & 1) * 2 * 128;
-      float* vb = va + 128;
+      float* va = svec + (i & 1) * 2 * 64;
+      float* vb = va + 64;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int j = j0 + lane * 4 + e;
+      for (int e = 0; e < 2; ++e) {
+        const int j = j0 + lane * 2 + e;
         const bool ok = j < T;
         if (COL) {
-          va[lane * 4 + e] = ok ? __ldg(p.lse + (size_t)bh * T + j) * kLog2e : 0.f;
-          vb[lane * 4 + e] = ok ? __ldg(p.drow + (size_t)bh * T + j) : 0.f;
+          va[lane * 2 + e] = ok ? __ldg(p.lse + (size_t)bh * T + j) * kLog2e : 0.f;
+          vb[lane * 2 + e] = ok ? __ldg(p.drow + (size_t)bh * T + j) : 0.f;
         } else {
-          va[lane * 4 + e] = (ok && p.bias) ? __ldg(p.bias + (size_t)bh * T + j) * kLog2e : 0.f;
+          va[lane * 2 + e] = (ok && p.bias) ? __ldg(p.bias + (size_t)bh * T + j) * kLog2e : 0.f;
         }
       }
       __syncwarp();
@@ -314,7 +294,7 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmOwn0, const __grid_c
       tc_fence_after();
       const int lo = j_lo - j0, hi = j_hi - j0;
 #pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
+      for (int ch = 0; ch < 2; ++ch) {
         uint32_t sr[32], dr[32];
         tmem_ld32(tS + ch * 32, sr);
         tmem_ld32(tD + ch * 32, dr);
@@ -357,7 +337,8 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmOwn0, const __grid_c
       const size_t off = ((size_t)bh * T + own) * D;
       float mid_dot = 0.f;  // column owner with the `mid` epilogue: sum_h dY Y of this column
 #pragma unroll
-      for (int ch = 0; ch < D / 32; ++ch) {
+      for (int ch2 = 0; ch2 < D / 64; ++ch2) {
+        const int ch = wg * (D / 64) + ch2;
         uint32_t a0[32];
         tmem_ld32(tmem + lane_base + Cfg::kTmemAcc0 + ch * 32, a0);
         tmem_wait_ld();
@@ -366,13 +347,7 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmOwn0, const __grid_c
           tmem_ld32(tmem + lane_base + Cfg::kTmemAcc1 + ch * 32, a1);
           tmem_wait_ld();
           if (!own_ok) continue;
-          if (p.d_vc_f32) {
-#pragma unroll
-            for (int e = 0; e < 32; e += 4)
-              *reinterpret_cast<float4*>(p.d_vc_f32 + off + ch * 32 + e) =
-                  make_float4(__uint_as_float(a0[e]), __uint_as_float(a0[e + 1]), __uint_as_float(a0[e + 2]),
-                              __uint_as_float(a0[e + 3]));
-          } else if (p.silu_src) {
+          if (p.silu_src) {
             // d(value) of a SiLU-gated value tensor: times SiLU'(raw value), in the operands' type
 #pragma unroll
             for (int e = 0; e < 32; e += 8) {
@@ -447,8 +422,16 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmOwn0, const __grid_c
                            pack2<T16>(v[e + 6], v[e + 7]));
         }
       }
-      if (COL && own_ok && p.gsum) p.gsum[(size_t)bh * T + own] = gs;
-      if (COL && own_ok && p.mid_dt) p.mid_dt[(size_t)bh * T + own] = mid_dot - gs;
+      if (COL && p.mid_dt) {
+        // the row term of the inner attention, from both halves of the columns
+        if (wg == 1) {
+          part[row] = mid_dot - gs;
+          mbar_arrive(&bars.part_ready);
+        } else {
+          alive = __all_sync(0xffffffffu, mbar_wait(&bars.part_ready, 0, abort_flag));
+          if (alive && own_ok) p.mid_dt[(size_t)bh * T + own] = mid_dot - gs + part[row];
+        }
+      }
     }
   }
 
@@ -459,7 +442,22 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmOwn0, const __grid_c
   if (tid == 0 && bars.abort_flag && p.status) atomicOr(p.status, 32);
 }
 
-template <int D, typename T16, bool COL>
+// blockIdx.x: head; blockIdx.y: 2 i (row owner) or 2 i + 1 (column owner), i-th heaviest tile of its kind (under the
+// causal mask the last rows and the first columns)
+template <int D, typename T16>
+__global__ void __launch_bounds__(kAttnBwdThreads, 1)
+attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmK,
+                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
+                      const __grid_constant__ AttnBwdParams p) {
+  const int i = blockIdx.y >> 1;
+  // owner side: rows (X, dOut) or columns (K, V); the other side streams through the ring
+  if (blockIdx.y & 1)
+    attn_bwd_tile<D, T16, true>(tmK, tmV, tmX, tmDO, p, blockIdx.x, i);
+  else
+    attn_bwd_tile<D, T16, false>(tmX, tmDO, tmK, tmV, p, blockIdx.x, (p.T + 127) / 128 - 1 - i);
+}
+
+template <int D, typename T16>
 int launch_attn_bwd(const AttnBwdTcArgs& a) {
   using Cfg = AttnBwdCfg<D>;
   CUtensorMap tmX, tmK, tmV, tmDO;
@@ -470,37 +468,28 @@ int launch_attn_bwd(const AttnBwdTcArgs& a) {
   if ((rc = make_tmap_3d(&tmDO, a.dout, 2, D, a.T, a.BN, 64, 128))) return rc;
   AttnBwdParams p{};
   p.bias = a.bias; p.lse = a.lse; p.drow = a.drow;
-  p.out_rows = a.out_rows; p.dout_rows = a.dout; p.drow_out = a.drow_out;
   p.silu_src = a.silu_src; p.d_vc_t = a.d_vc_t;
   p.mid_y = a.mid_y; p.mid_v2 = a.mid_v2; p.mid_dv2 = a.mid_dv2; p.mid_dy_t = a.mid_dy_t; p.mid_dt = a.mid_dt;
   p.d_rows_t = a.d_rows_t; p.d_rows_add = a.d_rows_add;
-  p.d_kc_f32 = a.d_kc_f32; p.d_kc_t = a.d_kc_t; p.d_vc_f32 = a.d_vc_f32; p.gsum = a.gsum;
+  p.d_kc_f32 = a.d_kc_f32; p.d_kc_t = a.d_kc_t;
   p.T = a.T; p.causal = a.causal; p.win = a.win < 0 ? 0 : (a.win > a.T ? a.T : a.win);
   p.scale2 = a.alpha * kLog2e; p.alpha = a.alpha;
   p.status = a.status;
-  auto kern = attn_bwd_sm100_kernel<D, T16, COL>;
+  auto kern = attn_bwd_sm100_kernel<D, T16>;
   TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
-  const dim3 grid((a.T + 127) / 128, a.BN);
-  // owner side: rows (X, dOut) or columns (K, V); the other side streams through the ring
-  if (COL)
-    kern<<<grid, kAttnBwdThreads, Cfg::kSmem, a.stream>>>(tmK, tmV, tmX, tmDO, p);
-  else
-    kern<<<grid, kAttnBwdThreads, Cfg::kSmem, a.stream>>>(tmX, tmDO, tmK, tmV, p);
+  const dim3 grid(a.BN, 2 * ((a.T + 127) / 128));
+  kern<<<grid, kAttnBwdThreads, Cfg::kSmem, a.stream>>>(tmX, tmK, tmV, tmDO, p);
   count_launch();
   TRITT_CUDA_OK(cudaGetLastError());
   return 0;
 }
 
-template <bool COL>
-int dispatch_attn_bwd(const AttnBwdTcArgs& a) {
-  if (a.dtype == TRITT_BF16)
-    return a.D == 128 ? launch_attn_bwd<128, __nv_bfloat16, COL>(a) : launch_attn_bwd<64, __nv_bfloat16, COL>(a);
-  return a.D == 128 ? launch_attn_bwd<128, __half, COL>(a) : launch_attn_bwd<64, __half, COL>(a);
-}
-
 }  // namespace
 
-int sm100_attn_bwd_rows(const AttnBwdTcArgs& a) { return dispatch_attn_bwd<false>(a); }
-int sm100_attn_bwd_cols(const AttnBwdTcArgs& a) { return dispatch_attn_bwd<true>(a); }
+int sm100_attn_bwd(const AttnBwdTcArgs& a) {
+  if (a.dtype == TRITT_BF16)
+    return a.D == 128 ? launch_attn_bwd<128, __nv_bfloat16>(a) : launch_attn_bwd<64, __nv_bfloat16>(a);
+  return a.D == 128 ? launch_attn_bwd<128, __half>(a) : launch_attn_bwd<64, __half>(a);
+}
 
 }  // namespace tritt

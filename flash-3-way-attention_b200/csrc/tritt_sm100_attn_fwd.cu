@@ -6,13 +6,15 @@
 // 196-220, but recompute the inner leg for every query block).
 //
 // One CTA owns 128 rows of one head and walks the 128-column tiles its rows attend to:
-//   warp 0      TMA producer: the row operand once, then a two-stage ring of (key tile, value tile)
+//   warp 0      TMA producer: the row operand once, then a ring of key and value tiles
 //   warp 1      issues tcgen05.mma:  S = X * Kc^T  (128x128 fp32 in TMEM)  and  acc += P * Vc  with P read from
 //               TMEM (16-bit, over the columns of S already consumed) and the value tile used row-major
-//   warps 4-7   one row per thread: scale, bias and mask, row maximum, exp2 with lazy rescaling of the accumulator,
-//               P written back to TMEM; at the end the row is normalised and stored (fp32 and / or 16-bit, and
-//               optionally the 16-bit product with a second tensor, which is the outer leg's value operand)
-// The chain S -> soft-max -> P*V of a CTA is serial; two CTAs share an SM when the head dimension is 64.
+//   warps 4-7, 8-11   two soft-max warpgroups, one row per thread, that take the column tiles in turn, each with scores,
+//               maximum, sum and accumulator of its own: scale, bias and mask, row maximum, exp2 with lazy rescaling of
+//               the accumulator, P written back to TMEM; at the end the two halves of a row are merged, normalised and
+//               stored (fp32 and / or 16-bit, and optionally the 16-bit product with a second tensor, which is the outer
+//               leg's value operand)
+// The chain S -> soft-max -> P*V of one warpgroup is serial; the other's runs beside it.
 #include "tritt_common.cuh"
 #include "tritt_sm100.cuh"
 #include "tritt_sm100_tdp.cuh"
@@ -23,19 +25,20 @@ namespace tritt {
 namespace {
 using namespace sm100;
 
-constexpr int kAttnThreads = 256;
+constexpr int kAttnThreads = 384;
 constexpr float kAttnRescaleGap = 8.f;  // rescale the accumulator only when the row max grew by more than 2^8
 
 template <int D> struct AttnCfg {
   static constexpr int kTile = 128 * D * 2;   // bytes of one 128-row operand tile
-  static constexpr int kStages = 2;
+  static constexpr int kStages = D == 64 ? 8 : 5;   // key and value tiles in turn: K(0), V(0), K(1), V(1), ...
   static constexpr int kOffX = 0;
-  static constexpr int kOffRing = kTile;      // stage s: key tile at kOffRing + 2 s kTile, value tile right behind
-  static constexpr int kOffBias = kOffRing + kStages * 2 * kTile;  // [4 warps][2 parities][128] fp32, log2 units
-  static constexpr int kOffBars = kOffBias + 4 * 2 * 128 * 4;
-  static constexpr int kSmem = kOffBars + 128;
-  static constexpr int kTmemO = 128;          // S | acc
-  static constexpr int kTmemCols = 256;
+  static constexpr int kOffRing = kTile;
+  static constexpr int kOffBias = kOffRing + kStages * kTile;  // [8 warps][128] fp32, log2 units
+  static constexpr int kOffMl = kOffBias + 8 * 128 * 4;        // [2 warpgroups][128][2] fp32: row maximum, row sum
+  static constexpr int kOffBars = kOffMl + 2 * 128 * 2 * 4;
+  static constexpr int kSmem = kOffBars + 256;
+  static constexpr int kTmemO = 256;          // S_0 | S_1 | acc_0 | acc_1
+  static constexpr int kTmemCols = 512;
 };
 
 struct AttnFwdParams {
@@ -51,21 +54,21 @@ struct AttnFwdParams {
 };
 
 struct AttnBarriers {
-  uint64_t ring_full[2], ring_empty[2];
-  uint64_t x_full, s_ready, p_ready, o_done;
+  uint64_t ring_full[8], ring_empty[8];
+  uint64_t x_full, s_ready[2], p_ready[2], o_done, ml_ready;
   uint32_t tmem_base;
   int abort_flag;
 };
 
 template <int D, typename T16>
-__global__ void __launch_bounds__(kAttnThreads, D == 64 ? 2 : 1)
+__global__ void __launch_bounds__(kAttnThreads, 1)
 attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, AttnFwdParams p) {
   using Cfg = AttnCfg<D>;
   constexpr int NS = Cfg::kStages;
   constexpr int KH = D / 64;
   extern __shared__ __align__(1024) uint8_t smem[];
-  static_assert(sizeof(AttnBarriers) <= 128, "barrier block too large");
+  static_assert(sizeof(AttnBarriers) <= 256, "barrier block too large");
   AttnBarriers& bars = *reinterpret_cast<AttnBarriers*>(smem + Cfg::kOffBars);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (smem_u32(smem) & 1023u) {
@@ -79,9 +82,12 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       mbar_init(&bars.ring_empty[i], 1);
     }
     mbar_init(&bars.x_full, 1);
-    mbar_init(&bars.s_ready, 1);
-    mbar_init(&bars.p_ready, 128);
+    for (int g = 0; g < 2; ++g) {
+      mbar_init(&bars.s_ready[g], 1);
+      mbar_init(&bars.p_ready[g], 128);
+    }
     mbar_init(&bars.o_done, 1);
+    mbar_init(&bars.ml_ready, 256);
     fence_barrier_init();
   }
   if (warp == 0) {
@@ -120,15 +126,13 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
         tma_load_3d(smem + Cfg::kOffX + hh * 16384, &tmX, &bars.x_full, hh * 64, r0, bh);
       int issued = 0;
       bool alive = true;
-      for (int i = 0; i < n_ct && alive; ++i) {
+      for (int i = 0; i < 2 * n_ct && alive; ++i) {
         const int st = i % NS;
         if (!mbar_wait(&bars.ring_empty[st], ((i / NS) & 1) ^ 1, abort_flag)) { alive = false; break; }
-        mbar_arrive_expect_tx(&bars.ring_full[st], 2 * Cfg::kTile);
-        uint8_t* kdst = smem + Cfg::kOffRing + st * 2 * Cfg::kTile;
-        for (int hh = 0; hh < KH; ++hh) {
-          tma_load_3d(kdst + hh * 16384, &tmK, &bars.ring_full[st], hh * 64, (ct0 + i) * 128, bh);
-          tma_load_3d(kdst + Cfg::kTile + hh * 16384, &tmV, &bars.ring_full[st], hh * 64, (ct0 + i) * 128, bh);
-        }
+        mbar_arrive_expect_tx(&bars.ring_full[st], Cfg::kTile);
+        uint8_t* dst = smem + Cfg::kOffRing + st * Cfg::kTile;
+        for (int hh = 0; hh < KH; ++hh)
+          tma_load_3d(dst + hh * 16384, i & 1 ? &tmV : &tmK, &bars.ring_full[st], hh * 64, (ct0 + i / 2) * 128, bh);
         ++issued;
       }
       if (!alive) {
@@ -160,67 +164,75 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       constexpr uint32_t idesc_pv = make_idesc_f16(128, D, kFmt, false, true);
       constexpr uint32_t kHi = desc_hi(1024);
       const uint32_t xLo = desc_lo(smem_u32(smem + Cfg::kOffX), 16);
-      auto issue_s = [&](int st) {
-        const uint32_t bLo = desc_lo(smem_u32(smem + Cfg::kOffRing + st * 2 * Cfg::kTile), 16);
+      bool alive = true;
+      auto wait_stage = [&](int pos) { return wait_all(&bars.ring_full[pos % NS], (pos / NS) & 1); };
+      // S_{i % 2} = X K(i)^T
+      auto issue_s = [&](int i) {
+        const int pos = 2 * i;
+        if (!wait_stage(pos)) return false;
+        tc_fence_after();
+        const uint32_t bLo = desc_lo(smem_u32(smem + Cfg::kOffRing + (pos % NS) * Cfg::kTile), 16);
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t kk = (k >> 2) * (16384 >> 4) + (k & 3) * 2;
-          if (leader) mma_ss_lo(tmem, xLo + kk, bLo + kk, kHi, idesc_s, k > 0);
+          if (leader) mma_ss_lo(tmem + (i & 1) * 128, xLo + kk, bLo + kk, kHi, idesc_s, k > 0);
         }
-        commit(&bars.s_ready);
+        commit(&bars.s_ready[i & 1]);
+        commit(&bars.ring_empty[pos % NS]);
+        return true;
       };
-      auto issue_pv = [&](int st, uint32_t acc) {
-        // value tile used row-major: 64-column blocks 16 KiB apart, 16 rows (one instruction) 2 KiB apart
-        const uint32_t bLo = desc_lo(smem_u32(smem + Cfg::kOffRing + st * 2 * Cfg::kTile + Cfg::kTile), 16384);
+      // acc_{i % 2} (+)= P(i) V(i); the value tile is used row-major: 64-column blocks 16 KiB apart, 16 rows (one
+      // instruction) 2 KiB apart
+      auto issue_pv = [&](int i) {
+        const int pos = 2 * i + 1;
+        if (!wait_stage(pos)) return false;
+        tc_fence_after();
+        const uint32_t bLo = desc_lo(smem_u32(smem + Cfg::kOffRing + (pos % NS) * Cfg::kTile), 16384);
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          if (leader) mma_ts_lo(tmem + Cfg::kTmemO, tmem + k * 8, bLo + k * (2048 >> 4), kHi, idesc_pv, k > 0 ? 1u : acc);
+          if (leader)
+            mma_ts_lo(tmem + Cfg::kTmemO + (i & 1) * D, tmem + (i & 1) * 128 + k * 8, bLo + k * (2048 >> 4), kHi, idesc_pv,
+                      k > 0 || i > 1);
+        commit(&bars.ring_empty[pos % NS]);
+        return true;
       };
-      bool alive = wait_all(&bars.x_full, 0) && wait_all(&bars.ring_full[0], 0);
-      if (alive) {
-        tc_fence_after();
-        issue_s(0);
-      }
+      alive = wait_all(&bars.x_full, 0) && issue_s(0) && (n_ct < 2 || issue_s(1));
       for (int i = 0; i < n_ct && alive; ++i) {
-        const int st = i % NS;
-        if (!wait_all(&bars.p_ready, i & 1)) { alive = false; break; }
+        alive = wait_all(&bars.p_ready[i & 1], (i >> 1) & 1);
+        if (!alive) break;
         tc_fence_after();
-        issue_pv(st, i > 0);
-        commit(&bars.ring_empty[st]);
-        if (i + 1 < n_ct) {
-          if (!wait_all(&bars.ring_full[(i + 1) % NS], ((i + 1) / NS) & 1)) { alive = false; break; }
-          tc_fence_after();
-          issue_s((i + 1) % NS);   // (overwrites P(i): the pipe runs it after P(i)*V(i), issued just above)
-        } else {
-          commit(&bars.o_done);
-        }
+        // (S(i + 2) overwrites P(i): the pipe runs it after P(i) V(i))
+        alive = issue_pv(i) && (i + 2 >= n_ct || issue_s(i + 2));
       }
+      if (alive) commit(&bars.o_done);
     }
   } else if (warp >= 4) {
     // ------------------------------------------------------------------ soft-max and epilogue, one row per thread
-    const int wq = warp & 3;
+    // Warpgroup g takes the column tiles g, g + 2, ... with a running maximum, sum and accumulator of its own: while one
+    // is in its exponentials the other's products run, and a row's two halves meet in the epilogue.
+    const int wg = (warp - 4) >> 2, wq = warp & 3;
     const int row = wq * 32 + lane;
     const int r = r0 + row;
     const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
-    const uint32_t tS = tmem + lane_base;
-    const uint32_t tO = tmem + lane_base + Cfg::kTmemO;
-    float* sbias = reinterpret_cast<float*>(smem + Cfg::kOffBias);
+    const uint32_t tS = tmem + lane_base + wg * 128;
+    const uint32_t tO = tmem + lane_base + Cfg::kTmemO + wg * D;
+    float* sb = reinterpret_cast<float*>(smem + Cfg::kOffBias) + (warp - 4) * 128;
     // this row's attended columns [c_lo, c_hi]
     const int c_hi = p.causal ? min(r, T - 1) : T - 1;
     const int c_lo = (p.causal && p.win < T) ? max(0, r - p.win) : 0;
     float m_used = -INFINITY, l_sum = 0.f;
     bool alive = true;
-    for (int i = 0; i < n_ct; ++i) {
+    for (int i = wg; i < n_ct; i += 2) {
       const int c0 = (ct0 + i) * 128;
       // this tile's column biases (log2 units), staged per warp so that no hand-off between warps is needed
-      float* sb = sbias + (wq * 2 + (i & 1)) * 128;
+      __syncwarp();   // every lane is done with the previous tile's
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int c = c0 + lane * 4 + e;
         sb[lane * 4 + e] = (p.bias && c < T) ? __ldg(p.bias + (size_t)bh * T + c) * kLog2e : 0.f;
       }
       __syncwarp();
-      alive = __all_sync(0xffffffffu, mbar_wait(&bars.s_ready, i & 1, abort_flag));
+      alive = __all_sync(0xffffffffu, mbar_wait(&bars.s_ready[wg], (i >> 1) & 1, abort_flag));
       if (!alive) break;
       tc_fence_after();
       const int lo = c_lo - c0, hi = c_hi - c0;
@@ -250,7 +262,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
             if (c >= l2 && c <= h2) mx = fmaxf(mx, fmaf(__uint_as_float(sr[c]), p.scale2, sb[hf * 64 + c]));
         }
       }
-      if (i == 0) {
+      if (i < 2) {
         m_used = mx;  // nothing accumulated yet
       } else {
         const bool grow = mx > m_used + kAttnRescaleGap;
@@ -310,23 +322,38 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       l_sum += psum;
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(&bars.p_ready);
+      mbar_arrive(&bars.p_ready[wg]);
     }
+    float2* ml = reinterpret_cast<float2*>(smem + Cfg::kOffMl);
+    ml[wg * 128 + row] = make_float2(m_used, l_sum);
+    mbar_arrive(&bars.ml_ready);
+    if (alive) alive = __all_sync(0xffffffffu, mbar_wait(&bars.ml_ready, 0, abort_flag));
     if (alive) alive = __all_sync(0xffffffffu, mbar_wait(&bars.o_done, 0, abort_flag));
     if (alive) {
       tc_fence_after();
-      const float inv = 1.f / l_sum;
+      // the row's two halves on their common maximum (a half without an attended column has maximum -inf and weight 0)
+      const float2 ml0 = ml[row], ml1 = ml[128 + row];
+      const float m = fmaxf(ml0.x, ml1.x), w0 = exp2f(ml0.x - m), w1 = exp2f(ml1.x - m);
+      const float l = ml0.y * w0 + ml1.y * w1, inv = 1.f / l;
+      const float f0 = w0 * inv, f1 = w1 * inv;
       const bool in_range = r < T;
       const size_t off = ((size_t)bh * T + r) * D;
 #pragma unroll
-      for (int ch = 0; ch < D / 32; ++ch) {
+      for (int ch2 = 0; ch2 < D / 64; ++ch2) {
+        const int ch = wg * (D / 64) + ch2;   // half of the output columns per warpgroup
         uint32_t o[32];
-        tmem_ld32(tO + ch * 32, o);
-        tmem_wait_ld();
-        if (!in_range) continue;
         float v[32];
+        tmem_ld32(tmem + lane_base + Cfg::kTmemO + ch * 32, o);
+        tmem_wait_ld();
 #pragma unroll
-        for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(o[e]) * inv;
+        for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(o[e]) * f0;
+        if (n_ct > 1) {
+          tmem_ld32(tmem + lane_base + Cfg::kTmemO + D + ch * 32, o);
+          tmem_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) v[e] = fmaf(__uint_as_float(o[e]), f1, v[e]);
+        }
+        if (!in_range) continue;
         if (p.out_f32) {
 #pragma unroll
           for (int e = 0; e < 32; e += 4)
@@ -351,7 +378,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
           }
         }
       }
-      if (in_range && p.out_lse) p.out_lse[(size_t)bh * T + r] = (m_used + log2f(l_sum)) * kLn2;
+      if (wg == 0 && in_range && p.out_lse) p.out_lse[(size_t)bh * T + r] = (m + log2f(l)) * kLn2;
     }
   }
 
