@@ -30,17 +30,18 @@ struct SimtTdpParams {
   float* out_lse;    // MODE_LSE
   void* out_o;       // MODE_FWD
   void* dq;          // MODE_BWD role 0
-  float *dX, *dY;    // MODE_BWD: fp32 accumulators for the row-side tensors
+  float *dX[2], *dY[2];  // MODE_BWD: fp32 accumulators for the row-side tensors, per role
   int T, D, nq;
   float alpha;
   TdpMask mask;
-  int q_mod, q_rem, role;
+  int q_mod, q_rem;
 };
 
 template <int MODE> __host__ __device__ constexpr int num_vecs() { return MODE == MODE_LSE ? 1 : (MODE == MODE_FWD ? 2 : 4); }
 
 template <typename T, int MODE>
-__global__ void tdp_simt_kernel(SimtTdpParams p) {
+__global__ void tdp_simt_kernel(const __grid_constant__ SimtTdpParams p) {
+  const int role = MODE == MODE_BWD ? blockIdx.z : 0;
   extern __shared__ float smem[];
   const int NT = blockDim.x, tid = threadIdx.x, D = p.D, T_ = p.T;
   const int bh = blockIdx.y;
@@ -48,11 +49,11 @@ __global__ void tdp_simt_kernel(SimtTdpParams p) {
   const int q = p.q_rem + qi * p.q_mod;
   const size_t base = (size_t)bh * T_ * D;
   const T* Q = (const T*)p.q + base;
-  const T* Xp = (const T*)(p.role == 0 ? p.k2 : p.k1) + base;
-  const T* Yp = (const T*)(p.role == 0 ? p.v2 : p.v1) + base;
-  const T* Kc = (const T*)(p.role == 0 ? p.k1 : p.k2) + base;
-  const T* Vc = (const T*)(p.role == 0 ? p.v1 : p.v2) + base;
-  const bool silu_y = p.role == 1, silu_vc = p.role == 0;
+  const T* Xp = (const T*)(role == 0 ? p.k2 : p.k1) + base;
+  const T* Yp = (const T*)(role == 0 ? p.v2 : p.v1) + base;
+  const T* Kc = (const T*)(role == 0 ? p.k1 : p.k2) + base;
+  const T* Vc = (const T*)(role == 0 ? p.v1 : p.v2) + base;
+  const bool silu_y = role == 1, silu_vc = role == 0;
 
   // shared memory carve-up
   constexpr int NV = num_vecs<MODE>();
@@ -92,11 +93,11 @@ __global__ void tdp_simt_kernel(SimtTdpParams p) {
 
   const TdpMask mk = p.mask;
   const bool single = mk.single_pair(q);         // one attended pair: the score gradient is exactly zero
-  const int xw = p.role == 0 ? mk.k2w : mk.k1w;  // window of the row axis against q
-  const int cw = p.role == 0 ? mk.k1w : mk.k2w;
+  const int xw = role == 0 ? mk.k2w : mk.k1w;  // window of the row axis against q
+  const int cw = role == 0 ? mk.k1w : mk.k2w;
   // band of the column axis around a row index x: c in [x - below, x + above]
-  const int below = p.role == 0 ? mk.kkl : mk.kkr;
-  const int above = p.role == 0 ? mk.kkr : mk.kkl;
+  const int below = role == 0 ? mk.kkl : mk.kkr;
+  const int above = role == 0 ? mk.kkr : mk.kkl;
   int xlo = 0, xhi = T_ - 1, clo_q = 0, chi_q = T_ - 1;
   if (mk.causal) {
     xlo = max(0, q - xw);
@@ -150,7 +151,7 @@ __global__ void tdp_simt_kernel(SimtTdpParams p) {
       for (int cc = 0; cc < kTileC; ++cc) {
         const int c = c0 + cc;
         if (c < clo || c > chi) continue;
-        const int j = p.role == 0 ? c : x, k = p.role == 0 ? x : c;
+        const int j = role == 0 ? c : x, k = role == 0 ? x : c;
         if (!mk.valid(q, j, k)) continue;
         float s = 0.f;
         for (int h = 0; h < D; ++h) s = fmaf(VEC(0, h), tK[cc * D + h], s);
@@ -182,13 +183,13 @@ __global__ void tdp_simt_kernel(SimtTdpParams p) {
       if (MODE == MODE_FWD) {
         for (int h = 0; h < D; ++h) atomicAdd(&outacc[h], VEC(1, h) * to_f(Yp[(size_t)x * D + h]));
       } else if (MODE == MODE_BWD) {
-        float* dX = p.dX + base + (size_t)x * D;
-        float* dY = p.dY + base + (size_t)x * D;
+        float* dX = p.dX[role] + base + (size_t)x * D;
+        float* dY = p.dY[role] + base + (size_t)x * D;
         for (int h = 0; h < D; ++h) {
           const float g = p.alpha * VEC(2, h);
           atomicAdd(&dX[h], g * qr[h]);
           atomicAdd(&dY[h], VEC(3, h) * dor[h]);
-          if (p.role == 0) atomicAdd(&outacc[h], g * to_f(Xp[(size_t)x * D + h]));
+          if (role == 0) atomicAdd(&outacc[h], g * to_f(Xp[(size_t)x * D + h]));
         }
       }
     }
@@ -214,7 +215,7 @@ __global__ void tdp_simt_kernel(SimtTdpParams p) {
     __syncthreads();
     if (MODE == MODE_FWD) {
       for (int h = tid; h < D; h += NT) ((T*)p.out_o + base)[(size_t)q * D + h] = from_f<T>(outacc[h]);
-    } else if (p.role == 0) {
+    } else if (role == 0) {
       for (int h = tid; h < D; h += NT) ((T*)p.dq + base)[(size_t)q * D + h] = from_f<T>(outacc[h]);
     }
   }
@@ -247,19 +248,23 @@ size_t smem_bytes(int nvec, int D, int nt) {
 template <typename T, int MODE, int DQ, int LPR>
 int launch_quad(const SimtTdpParams& p, int BN, cudaStream_t stream) {
   if (p.nq <= 0) return 0;
-  tdp_simt_quad_kernel<T, MODE, DQ, LPR><<<dim3(p.nq, BN), 128, 0, stream>>>(p);
+  tdp_simt_quad_kernel<T, MODE, DQ, LPR><<<dim3(p.nq, BN, MODE == MODE_BWD ? 2 : 1), 128, 0, stream>>>(p);
   count_launch();
   TRITT_CUDA_OK(cudaGetLastError());
   return 0;
 }
 
+bool quad_head_dim(int D) { return D >= 16 && D <= 128; }   // (head dimensions are powers of two)
+
 template <typename T, int MODE>
 int launch(const SimtTdpParams& p, int BN, cudaStream_t stream) {
   // head dimensions 16 to 128: the register-resident kernels (four lanes per row, eight at 128)
+  if constexpr (MODE != MODE_LSE) {
   if (p.D == 128) return launch_quad<T, MODE, 16, 8>(p, BN, stream);
   if (p.D == 64) return launch_quad<T, MODE, 16, 4>(p, BN, stream);
   if (p.D == 32) return launch_quad<T, MODE, 8, 4>(p, BN, stream);
   if (p.D == 16) return launch_quad<T, MODE, 4, 4>(p, BN, stream);
+  }
   constexpr int NV = num_vecs<MODE>();
   const int nt = pick_threads(NV, p.D);
   const size_t sm = smem_bytes(NV, p.D, nt);
@@ -270,7 +275,7 @@ int launch(const SimtTdpParams& p, int BN, cudaStream_t stream) {
   auto kern = tdp_simt_kernel<T, MODE>;
   TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   if (p.nq <= 0) return 0;
-  kern<<<dim3(p.nq, BN), nt, sm, stream>>>(p);
+  kern<<<dim3(p.nq, BN, MODE == MODE_BWD ? 2 : 1), nt, sm, stream>>>(p);
   count_launch();
   TRITT_CUDA_OK(cudaGetLastError());
   return 0;
@@ -307,12 +312,13 @@ size_t simt_tdp_workspace(int op, int B, int N, int T, int D, int /*dtype*/) {
 
 int simt_tdp_fwd(const TdpArgs& a) {
   SimtTdpParams p = base_params(a);
-  p.role = 0;
   p.out_lse = a.out_lse;
-  int rc = launch_dtype<MODE_LSE>(p, a.B * a.N, a.dtype, a.stream);
-  if (rc) return rc;
   p.lse = a.out_lse;
   p.out_o = a.out_o;
+  if (!quad_head_dim(p.D)) {   // (the register-resident kernel forms the log-sum-exp itself)
+    const int rc = launch_dtype<MODE_LSE>(p, a.B * a.N, a.dtype, a.stream);
+    if (rc) return rc;
+  }
   return launch_dtype<MODE_FWD>(p, a.B * a.N, a.dtype, a.stream);
 }
 
@@ -349,17 +355,12 @@ int simt_tdp_bwd(const TdpArgs& a) {
   SimtTdpParams p = base_params(a);
   p.lse = a.lse_in;
   p.dq = a.dq;
-  // role 0: rows (q, k): dQ, dK2, dV2
-  p.role = 0;
-  p.dX = part + n;      // dK2
-  p.dY = part + 3 * n;  // dV2
-  int rc = launch_dtype<MODE_BWD>(p, a.B * a.N, a.dtype, a.stream);
-  if (rc) return rc;
-  // role 1: rows (q, j): dK1, dSiLU(V1)
-  p.role = 1;
-  p.dX = part;          // dK1
-  p.dY = part + 2 * n;  // dSiLU(V1)
-  rc = launch_dtype<MODE_BWD>(p, a.B * a.N, a.dtype, a.stream);
+  // Both roles in one launch (blockIdx.z): a short sequence leaves most SMs idle under either alone.
+  p.dX[0] = part + n;      // role 0, rows (q, k): dQ, dK2, dV2
+  p.dY[0] = part + 3 * n;
+  p.dX[1] = part;          // role 1, rows (q, j): dK1, dSiLU(V1)
+  p.dY[1] = part + 2 * n;
+  const int rc = launch_dtype<MODE_BWD>(p, a.B * a.N, a.dtype, a.stream);
   if (rc) return rc;
   if (a.flags & TRITT_FLAG_BWD_PARTIAL) return 0;
   return simt_tdp_bwd_finalize(a.v1, a.dk1, a.dk2, a.dv1, a.dv2, n, a.dtype, part, a.stream);

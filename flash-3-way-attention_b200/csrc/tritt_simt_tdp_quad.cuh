@@ -24,25 +24,32 @@ template <int LPR> __device__ __forceinline__ float tdp_rows_sum(float v) {
   return v;
 }
 
+template <int D> struct QuadShared {
+  alignas(16) float tK[kQuadCols * D];
+  alignas(16) float tV[kQuadCols * D];
+  float qs[D], qr[D], dor[D], outacc[D];
+  float red[128];
+};
+
+// One pass of a CTA over its query's pairs.  `lse`: natural-log log-sum-exp of the query (MODE_FWD, MODE_BWD); MODE_LSE
+// returns it, in every thread.
 template <typename T, int MODE, int DQ, int LPR>
-__global__ void __launch_bounds__(128) tdp_simt_quad_kernel(SimtTdpParams p) {
+__device__ __forceinline__ float tdp_quad_pass(const SimtTdpParams& p, const int role, float* const dX_sum, float* const dY_sum,
+                                               QuadShared<DQ * LPR>& sh, const float lse) {
   constexpr int D = DQ * LPR;
   constexpr int kQuadRows = 128 / LPR;   // pair rows per pass of a CTA (128 threads)
-  __shared__ __align__(16) float tK[kQuadCols * D];
-  __shared__ __align__(16) float tV[kQuadCols * D];
-  __shared__ float qs[D], qr[D], dor[D], outacc[D];
-  __shared__ float red[128];
+  float *tK = sh.tK, *tV = sh.tV, *qs = sh.qs, *qr = sh.qr, *dor = sh.dor, *outacc = sh.outacc, *red = sh.red;
   const int tid = threadIdx.x, lane = tid & 31, qd = tid & (LPR - 1), T_ = p.T;
   const int bh = blockIdx.y;
   const int qi = p.nq - 1 - (int)blockIdx.x;  // long rows first
   const int q = p.q_rem + qi * p.q_mod;
   const size_t base = (size_t)bh * T_ * D;
   const T* Q = (const T*)p.q + base;
-  const T* Xp = (const T*)(p.role == 0 ? p.k2 : p.k1) + base;
-  const T* Yp = (const T*)(p.role == 0 ? p.v2 : p.v1) + base;
-  const T* Kc = (const T*)(p.role == 0 ? p.k1 : p.k2) + base;
-  const T* Vc = (const T*)(p.role == 0 ? p.v1 : p.v2) + base;
-  const bool silu_y = p.role == 1, silu_vc = p.role == 0;
+  const T* Xp = (const T*)(role == 0 ? p.k2 : p.k1) + base;
+  const T* Yp = (const T*)(role == 0 ? p.v2 : p.v1) + base;
+  const T* Kc = (const T*)(role == 0 ? p.k1 : p.k2) + base;
+  const T* Vc = (const T*)(role == 0 ? p.v1 : p.v2) + base;
+  const bool silu_y = role == 1, silu_vc = role == 0;
 
   float dq_part = 0.f;
   for (int h = tid; h < D; h += 128) {
@@ -57,7 +64,7 @@ __global__ void __launch_bounds__(128) tdp_simt_quad_kernel(SimtTdpParams p) {
     }
   }
   float lse2 = 0.f, Dq = 0.f;
-  if (MODE != MODE_LSE) lse2 = p.lse[(size_t)bh * T_ + q] * kLog2e;
+  if (MODE != MODE_LSE) lse2 = lse * kLog2e;
   if (MODE == MODE_BWD) {
     // Dq = sum_h dO[q,h] * O[q,h]  (reference flash_trittention.py:167)
     red[tid] = dq_part;
@@ -72,11 +79,11 @@ __global__ void __launch_bounds__(128) tdp_simt_quad_kernel(SimtTdpParams p) {
 
   const TdpMask mk = p.mask;
   const bool single = mk.single_pair(q);         // one attended pair: the score gradient is exactly zero
-  const int xw = p.role == 0 ? mk.k2w : mk.k1w;  // window of the row axis against q
-  const int cw = p.role == 0 ? mk.k1w : mk.k2w;
+  const int xw = role == 0 ? mk.k2w : mk.k1w;  // window of the row axis against q
+  const int cw = role == 0 ? mk.k1w : mk.k2w;
   // band of the column axis around a row index x: c in [x - below, x + above]
-  const int below = p.role == 0 ? mk.kkl : mk.kkr;
-  const int above = p.role == 0 ? mk.kkr : mk.kkl;
+  const int below = role == 0 ? mk.kkl : mk.kkr;
+  const int above = role == 0 ? mk.kkr : mk.kkl;
   int xlo = 0, xhi = T_ - 1, clo_q = 0, chi_q = T_ - 1;
   if (mk.causal) {
     xlo = max(0, q - xw);
@@ -148,7 +155,7 @@ __global__ void __launch_bounds__(128) tdp_simt_quad_kernel(SimtTdpParams p) {
 #pragma unroll
         for (int cc = 0; cc < kQuadCols; ++cc) {
           const int c = c0 + cc;
-          const int j = p.role == 0 ? c : x, k = p.role == 0 ? x : c;
+          const int j = role == 0 ? c : x, k = role == 0 ? x : c;
           const bool ok = active && c >= clo && c <= chi && mk.valid(q, j, k);
           const float4* k4 = reinterpret_cast<const float4*>(tK + cc * D + qd * DQ);
           float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;   // four independent chains
@@ -183,13 +190,13 @@ __global__ void __launch_bounds__(128) tdp_simt_quad_kernel(SimtTdpParams p) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           const int c = c0 + cg + e;
-          any_ok = any_ok || (active && c >= clo && c <= chi && mk.valid(q, p.role == 0 ? c : x, p.role == 0 ? x : c));
+          any_ok = any_ok || (active && c >= clo && c <= chi && mk.valid(q, role == 0 ? c : x, role == 0 ? x : c));
         }
         if (!__any_sync(0xffffffffu, any_ok)) continue;
 #pragma unroll
       for (int cc = cg; cc < cg + 8; ++cc) {
         const int c = c0 + cc;
-        const int j = p.role == 0 ? c : x, k = p.role == 0 ? x : c;
+        const int j = role == 0 ? c : x, k = role == 0 ? x : c;
         const bool ok = active && c >= clo && c <= chi && mk.valid(q, j, k);
         const float4* k4 = reinterpret_cast<const float4*>(tK + cc * D + qd * DQ);
         const float4* v4 = reinterpret_cast<const float4*>(tV + cc * D + qd * DQ);
@@ -248,8 +255,8 @@ __global__ void __launch_bounds__(128) tdp_simt_quad_kernel(SimtTdpParams p) {
         if (lane < LPR) atomicAdd(&outacc[h], v);
       }
     } else if (MODE == MODE_BWD) {
-      float* dX = p.dX + base + (size_t)x * D;
-      float* dY = p.dY + base + (size_t)x * D;
+      float* dX = dX_sum + base + (size_t)x * D;
+      float* dY = dY_sum + base + (size_t)x * D;
 #pragma unroll
       for (int i = 0; i < DQ; ++i) {
         const int h = qd * DQ + i;
@@ -258,7 +265,7 @@ __global__ void __launch_bounds__(128) tdp_simt_quad_kernel(SimtTdpParams p) {
           atomicAdd(&dX[h], gg * qr[h]);
           atomicAdd(&dY[h], u[i] * dor[h]);
         }
-        if (p.role == 0) {
+        if (role == 0) {
           float v = active ? gg * to_f(Xp[(size_t)x * D + h]) : 0.f;
           v = tdp_rows_sum<LPR>(v);
           if (lane < LPR) atomicAdd(&outacc[h], v);
@@ -283,13 +290,30 @@ __global__ void __launch_bounds__(128) tdp_simt_quad_kernel(SimtTdpParams p) {
       if (tid < s) red[tid] += red[tid + s];
       __syncthreads();
     }
-    if (tid == 0) p.out_lse[(size_t)bh * T_ + q] = (M + log2f(red[0])) * kLn2;
+    return (M + log2f(red[0])) * kLn2;
   } else {
     __syncthreads();
     if (MODE == MODE_FWD) {
       for (int h = tid; h < D; h += 128) ((T*)p.out_o + base)[(size_t)q * D + h] = from_f<T>(outacc[h]);
-    } else if (p.role == 0) {
+    } else if (role == 0) {
       for (int h = tid; h < D; h += 128) ((T*)p.dq + base)[(size_t)q * D + h] = from_f<T>(outacc[h]);
     }
+  }
+  return 0.f;
+}
+
+// MODE_FWD: log-sum-exp, then the output, in one launch (a CTA owns its query throughout);  MODE_BWD: blockIdx.z is the role.
+template <typename T, int MODE, int DQ, int LPR>
+__global__ void __launch_bounds__(128) tdp_simt_quad_kernel(const __grid_constant__ SimtTdpParams p) {
+  __shared__ QuadShared<DQ * LPR> sh;
+  const size_t row = (size_t)blockIdx.y * p.T + p.q_rem + (p.nq - 1 - (int)blockIdx.x) * p.q_mod;
+  if constexpr (MODE == MODE_FWD) {
+    const float lse = tdp_quad_pass<T, MODE_LSE, DQ, LPR>(p, 0, nullptr, nullptr, sh, 0.f);
+    if (threadIdx.x == 0) p.out_lse[row] = lse;
+    __syncthreads();   // (the second pass rewrites what the first one's last reduction reads)
+    tdp_quad_pass<T, MODE_FWD, DQ, LPR>(p, 0, nullptr, nullptr, sh, lse);
+  } else {
+    const int role = blockIdx.z;
+    tdp_quad_pass<T, MODE_BWD, DQ, LPR>(p, role, p.dX[role], p.dY[role], sh, p.lse[row]);
   }
 }
