@@ -70,36 +70,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return mbar_wait_limit(bar, parity, abort_flag, kWaitTicks);
 }
 
-// ------------------------------------------------------------------ CTA pairs (thread-block clusters of two)
-// A pair of CTAs on the two SMs of one TPC can run tcgen05.mma with cta_group::2: one instruction, issued by the
-// even CTA, multiplies 256 rows (128 per CTA) with the B operand split along N between the two CTAs' shared
-// memories.  The helpers below are what the pair needs besides: rank, pair-wide barrier, arrival on a barrier of
-// the other CTA.
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// (hardware barrier over all threads of the cluster: every thread of both CTAs must reach it)
+// Hardware barrier over all threads of the cluster: every thread of every block of it must come here.
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// shared::cluster address of `bar` as seen in CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t mbar_in_cta(uint64_t* bar, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(bar)), "r"(rank));
-  return r;
-}
-// (default semantics, release at CTA scope, as for a local arrival: what is handed over lives in tensor memory or
-//  was published to the async proxy by the caller's fence; a cluster-scope release costs a memory barrier of
-//  several hundred cycles per arrival, measured as a doubled soft-max stage)
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// Bounded wait on a barrier of this CTA that, when PAIR, the other CTA of the pair may arrive on.
-template <bool PAIR>
-__device__ __forceinline__ bool mbar_wait_x(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  return mbar_wait(bar, parity, abort_flag);
 }
 
 // ------------------------------------------------------------------ fences
@@ -119,30 +92,6 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
-// The same load issued by a CTA of a pair, its bytes counted on a barrier of the pair's even CTA (`bar_cluster_addr`
-// from mbar_in_cta(bar, 0)); the destination is the issuing CTA's own shared memory.
-__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorMap* m, uint32_t bar_cluster_addr, int x, int y,
-                                                 int z) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(smem_dst)), "l"((uint64_t)m), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
-      : "memory");
-}
-
-// Tile reduce-add from shared memory into global memory (element type and swizzle come from the
-// tensor map; rows outside the tensor are dropped).  Completion is tracked per thread in bulk groups.
-__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* m, const void* smem_src, int x, int y, int z) {
-  asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
-                   (uint64_t)m),
-               "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// Wait until the shared-memory source of every committed bulk group of this thread has been read.
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// Wait until every committed bulk group of this thread has fully completed (writes performed).
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
 // ------------------------------------------------------------------ TMEM
 // Allocation is warp-collective (all 32 lanes execute it); `ncols` is a power of two >= 32.
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {
@@ -154,18 +103,6 @@ __device__ __forceinline__ void tmem_relinquish() {
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-
-// The same for a CTA pair (executed by the same warp of both CTAs).
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_dst, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish_pair() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
 // ------------------------------------------------------------------ descriptors
@@ -245,35 +182,6 @@ __device__ __forceinline__ void mma_ts_lo(uint32_t d_tmem, uint32_t a_tmem, uint
       "r"(a_tmem), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accum)
       : "memory");
 }
-// CTA-pair forms (cta_group::2, issued by one thread of the even CTA; M counts the rows of both CTAs, each CTA
-// supplies its own A rows and its half of B's N extent at the same shared / tensor memory offsets).
-__device__ __forceinline__ void mma_ss_lo_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
-                                               uint32_t accum) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-      "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accum)
-      : "memory");
-}
-__device__ __forceinline__ void mma_ts_lo_pair(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t hi, uint32_t idesc,
-                                               uint32_t accum) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-      "mov.b64 db, {%2, %3};\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accum)
-      : "memory");
-}
-// Arrive on the barrier at `bar`'s offset in both CTAs of the pair once every MMA issued so far has finished.
-__device__ __forceinline__ void mma_commit_pair(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-                   smem_u32(bar)),
-               "h"((uint16_t)3)
-               : "memory");
-}
 // Arrive on `bar` once every MMA issued so far by this thread has finished.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -344,6 +252,15 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
                "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                : "memory");
 }
+// 16 lanes x 16 columns as two 16 x 256-bit fragments: thread t gets, of columns 8 g + 2 (t % 4) and the next (g = 0, 1),
+// row t / 4 in r[4 g], r[4 g + 1] and row t / 4 + 8 in r[4 g + 2], r[4 g + 3].  The address names the first of the 16
+// lanes (the lower or upper half of the warp's 32).
+__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
 // width-generic wrappers
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
@@ -353,7 +270,44 @@ __device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[32])
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// ------------------------------------------------------------------ shared memory fragments
+// Four 8 x 8 blocks of 16-bit elements; lane l passes the address of row l % 8 of block l / 8, thread t gets of each
+// block row t / 4, columns 2 (t % 4) and the next (.trans: column t / 4, rows 2 (t % 4) and the next).
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t saddr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(saddr)
+               : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t saddr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(saddr)
+               : "memory");
+}
+
+// The inverse: stores the fragments (same lane -> row address rule).
+__device__ __forceinline__ void stmatrix_x4(uint32_t saddr, const uint32_t (&r)[4]) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(r[0]), "r"(r[1]),
+               "r"(r[2]), "r"(r[3])
+               : "memory");
+}
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t saddr, const uint32_t (&r)[4]) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(r[0]), "r"(r[1]),
+               "r"(r[2]), "r"(r[3])
+               : "memory");
+}
+
 // ------------------------------------------------------------------ misc
+// Changes the register budget of the executing warpgroup (all four warps execute it) from FROM to TO per thread.  The
+// instruction has one form that only lowers and one that only raises the count (the wrong one is an illegal
+// instruction); raising waits for registers that other warpgroups of the block gave up, so the shares must not add up
+// to more than the block was launched with.
+template <int FROM, int TO> __device__ __forceinline__ void set_regs() {
+  static_assert(TO % 8 == 0 && TO >= 24 && TO <= 256, "register count");
+  if constexpr (TO < FROM) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TO));
+  if constexpr (TO > FROM) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TO));
+}
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
@@ -368,9 +322,6 @@ __device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-// Same for a 64-byte-swizzled tile whose rows are 64 bytes (chunk 0..3): XOR with (row / 2) mod 4.
-__device__ __forceinline__ uint32_t swz64(uint32_t row, uint32_t chunk) { return row * 64u + ((chunk ^ ((row >> 1) & 3u)) << 4); }
-
 // Byte offset of the 16-byte chunk `chunk` (0..7) of row `row` inside a 128-byte-swizzled
 // tile whose rows are 128 bytes: the chunk index is XOR-ed with (row mod 8).
 __device__ __forceinline__ uint32_t swz128(uint32_t row, uint32_t chunk) { return row * 128u + ((chunk ^ (row & 7u)) << 4); }
@@ -382,9 +333,8 @@ __device__ __forceinline__ uint32_t swz128(uint32_t row, uint32_t chunk) { retur
 // with the 128-byte swizzle; box = {64 cols, box_rows, 1}.  Out-of-range rows read zero.
 int make_tmap_3d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t cols, uint64_t rows, uint64_t bn,
                  uint32_t box_cols, uint32_t box_rows);
-// Same over an fp32 tensor (used as the destination of TMA reduce-adds); the swizzle follows the box
-// width (64-byte rows -> 64-byte swizzle, 128-byte rows -> 128-byte swizzle).
-int make_tmap_3d_f32(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t bn, uint32_t box_cols,
-                     uint32_t box_rows);
+// The same over rows that are `row_stride` elements apart (heads `head_stride`): the rows of a query shard.
+int make_tmap_rows(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t bn, uint64_t row_stride,
+                   uint64_t head_stride, uint32_t box_rows);
 
 }  // namespace tritt

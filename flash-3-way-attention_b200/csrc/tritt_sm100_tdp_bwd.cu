@@ -1,43 +1,34 @@
 // Triple-dot-product trittention backward on Blackwell tensor cores (tcgen05 + TMEM + TMA).
 //
-// Same pair-row formulation as the forward kernel.  For one query q and a tile of 128 rows
-// x of a "row" key tensor X (with its value tensor Y), against 128-row slabs of the
-// "column" key/value tensors Kc / Vc:
-//     A [r,h] = alpha*log2(e) * Q[q,h]  * X[x_r,h]          A'[r,h] = dO[q,h] * Y[x_r,h]
-//     S  = A  Kc^T          P  = exp2(S - lse2[q])          (recomputed from the saved lse)
-//     dP = A' Vc^T          dS = P * (dP - Dq),  Dq = sum_h dO[q,h] O[q,h]
-//     G += dS Kc            U += P Vc                        (accumulated over the slabs in TMEM)
-// and per tile   dX[x_r,h] += alpha G[r,h] Q[q,h],   dY[x_r,h] += U[r,h] dO[q,h],
-//                dQ[q,h]   += alpha sum_r G[r,h] X[x_r,h].
-// Role 0 takes X = K2, Y = V2, Kc = K1, Vc = SiLU(V1) and yields dQ, dK2, dV2.  Role 1 swaps
-// the two key axes (the score and the gated value are symmetric under the swap): X = K1,
-// Y = SiLU(V1), Kc = K2, Vc = V2, and yields dK1 and dSiLU(V1).  Four GEMM-shaped products per
-// (tile, slab) and role - eight in all against the six of a minimal schedule - but every
-// key-side gradient is owned by rows of a tile, so the only cross-CTA reductions are one
-// 128 x D block per tile and tensor, added to fp32 accumulators by TMA reduce-add.
+// The score S[q,j,k] = alpha sum_h Q[q,h] K1[j,h] K2[k,h] and the gated value are trilinear, so any of the three
+// indices can be the one that is stepped over.  Here it is k: for one k the (q, j) plane is an ordinary attention
+// backward whose key and value operands carry the k-th rows of K2 and V2,
+//     A [j,h] = alpha*log2(e) * K1[j,h] * K2[k,h]      A'[j,h] = SiLU(V1)[j,h] * V2[k,h]
+//     S  = Q A^T          P  = exp2(S - lse2[q])       (recomputed from the saved lse)
+//     dP = dO A'^T        dS = P * (dP - Dq[q]),       Dq = sum_h dO O
+// and all five gradients follow from three more products:
+//     dQ[q,:] += dS A                                  (accumulated over k in tensor memory)
+//     G = dS^T Q:   dK1[j,h] += alpha K2[k,h] G[j,h],   dK2[k,h] += alpha sum_j K1[j,h] G[j,h]
+//     U = P^T dO:   dSV1[j,h] += V2[k,h] U[j,h],        dV2[k,h] += sum_j SiLU(V1)[j,h] U[j,h]
+// Five products per (q-tile, j-tile, k) where stepping over q needs six (and needed eight with every key-side
+// gradient owned by rows), and one exponential per attended triple instead of two.
 // (The reference runs one Triton kernel per gradient, recomputing P five times:
 // triple_dot_product/kernels/bwd_dq.py, bwd_dk1.py, bwd_dk2.py, bwd_dv1.py, bwd_dv2.py.)
 //
-// Tensor-core usage follows what the hardware rewards: 128-column slabs, so that every
-// accumulation chain is 8 instructions of 128x128x16 (an instruction below N = 128 costs the same
-// ~48-64 cycles), TMEM fully used
-// as S | dP | G | U (4 x 128 columns at D = 128).  P and dS are written back as 16-bit into the
-// first half of the S and dP column ranges and feed the G / U products from tensor memory.
+// A work item is a tile of 128 queries x JT rows j with its range of k; the item's Q, dO, K1 and SiLU(V1) tiles stay
+// in shared memory for the whole range, dQ in tensor memory, dK1 and dSiLU(V1) in the registers of the fold
+// warpgroups; per step only the two rows K2[k], V2[k] come in and two rows of dK2, dV2 go out (vector reductions into
+// fp32 sums that stay in L2).  All steps of a call are laid out in one line and cut in equal parts, one per CTA
+// (every sum is a reduction, so an item may be cut anywhere): no last wave.
 //
-// CTA layout (persistent, 512 threads): warp 0 TMA producer, warp 1 tcgen05.mma issuer, warps 4-11 two
-// soft-max warpgroups (64 columns of every slab each; they also form the operands), warps 12-15 the
-// fold warpgroup.  The slab pipeline is split in four hand-offs so that the exponentials (the MUFU
-// bound part) overlap the tensor pipe although S and dP are single-buffered:
-//     MMA:      U(c) S(c+1) | G(c) dP(c+1) | U(c+1) S(c+2) | ...
-//     soft-max:      [S(c+1) -> P(c+1)]  [dP(c+1), P(c+1) -> dS(c+1)]
-// (At head dimension 64, where tensor memory has room, P has buffers of its own and S(c+1) goes before U(c): see
-// kFreeS in the kernel.)
-// The fold warpgroup drains G / U of tile t (TMEM -> registers -> shared memory -> TMA reduce-add)
-// while the other warps already run tile t+1.  Work item = (query, head, role); it walks the row tiles
-// x <= q and, inside, the column slabs c <= q.
-// On request (TRITT_FLAG_BWD_CTA_PAIRS) the same kernel runs as clusters of two CTAs: each CTA keeps its own query,
-// operand tiles, soft-max and fold, the even CTA issues every product for both (cta_group::2, 256 rows), the column
-// tiles are split between the two shared memories, and hand-offs to the issuing thread cross the pair.
+// Tile shapes: the accumulators S | dP | G | U | dQ have to fit 512 columns of tensor memory.  Head dimension 64:
+// JT = 128, G and U as [j x h] (128 + 128 + 64 + 64 + 64).  Head dimension 128: JT = 64 and G, U transposed,
+// [h x j], so that their M extent is 128 (64 + 64 + 64 + 64 + 128); a JT of 128 would need 640 columns.
+//
+// CTA: 20 warps.  0-3 and 4-7: soft-max warpgroups (half of a step's columns each, one query per thread); 8-11: forms
+// A and folds G; 12-15: forms A' and folds U; 16: issues the products; 17: TMA and the K2 / V2 rows (18, 19
+// idle).  P and dS are written to shared memory, where both the transposed (U, G) and the plain (dQ) product can read them.
+// Order of the products of step n:   S(n+1)  U(n)  dP(n+1)  dQ(n)  G(n).
 #include "tritt_sm100_tdp.cuh"
 
 #include <type_traits>
@@ -46,107 +37,183 @@ namespace tritt {
 namespace {
 using namespace sm100;
 
-constexpr int kBC = 128;  // key columns per slab
+constexpr int kBwdThreads = 640;
+// Registers per thread: 640 threads are launched with 96 each (480 per lane of the five warpgroups) and split them anew.
+constexpr int kRegsLaunch = 96, kRegsSoftmax = 80, kRegsFold = 128, kRegsService = 64;
+static_assert(2 * kRegsSoftmax + 2 * kRegsFold + kRegsService <= 5 * kRegsLaunch, "more registers than the launch has");
+constexpr int kVecBatch = 4;     // K2 / V2 rows per hand-over
+constexpr int kVecSlots = 4;     // batches in flight
 
 template <int D> struct BwdCfg {
-  static constexpr int kTileA = 128 * D * 2;   // one 128-row operand / key / value tile
-  // ring of column tiles Kc(c), Vc(c), Kc(c+1), Vc(c+1), ...: two slabs deep at head dimension 128 (all the shared
-  // memory there is), four at 64
-  static constexpr int kStages = D == 64 ? 8 : 4;
-  static constexpr int kOffA = 0;              // A  (row-key pre-product)
-  static constexpr int kOffA2 = kTileA;        // A' (row-value pre-product)
-  static constexpr int kOffRing = 2 * kTileA;
-  static constexpr int kOffStage = kOffRing + kStages * kTileA;  // fold staging: 4 warps x 2 slots x 4 KiB
-  static constexpr int kStageBytes = 4 * 2 * 4096;
-  static constexpr int kOffDq = kOffStage + kStageBytes;         // [D] fp32: dQ column sums of the current query
-  static constexpr int kOffVec = kOffDq + D * 4;                 // [2 parities][2][D] fp32: Q[q], dO[q]
-  static constexpr int kOffMisc = kOffVec + 4 * D * 4;           // [4] fp32: Dq partials
-  static constexpr int kOffBars = kOffMisc + 16;                 // barriers (no static shared memory is used, so
-  static constexpr int kSmem = kOffBars + 288;                   //  the dynamic region starts 1024-byte aligned)
-  static constexpr int kTmemS = 0, kTmemDP = 128, kTmemG = 256, kTmemU = 256 + D;
-  static constexpr int kTmemP = 384;   // head dimension 64 only: two buffers of 64 columns for P (by slab parity)
+  static constexpr int JT = D == 64 ? 128 : 64;       // rows j of an item
+  static constexpr int CW = JT / 2;                   // columns of one soft-max thread
+  static constexpr int kTileQ = 128 * D * 2;          // Q, dO
+  static constexpr int kTileJ = JT * D * 2;           // K1, SiLU(V1), A, A'  (16 KiB for both head dimensions)
+  static constexpr int kTileP = 128 * JT * 2;         // P, dS
+  static constexpr int kOffQ = 0;
+  static constexpr int kOffDO = kOffQ + kTileQ;
+  static constexpr int kOffK1 = kOffDO + kTileQ;      // K1 | SiLU(V1)
+  static constexpr int kOffA = kOffK1 + 2 * kTileJ;   // A (two buffers) | A'
+  static constexpr int kOffP = kOffA + 3 * kTileJ;    // P | dS (two buffers)
+  static constexpr int kOffVec = kOffP + 3 * kTileP;  // [slot][row][scale2 * K2 | V2] fp32
+  static constexpr int kVecRow = 2 * D;               // floats
+  static constexpr int kOffBars = kOffVec + kVecSlots * kVecBatch * kVecRow * 4;
+  static constexpr int kSmem = kOffBars + 448;
+  static constexpr int kTmemS = 0, kTmemDP = JT, kTmemG = 2 * JT, kTmemU = kTmemG + 64, kTmemDQ = kTmemU + 64;
+  static constexpr int kTmemQ = kTmemDQ + D, kTmemDO = kTmemQ + D / 2;   // 16-bit, two elements a column
+  static_assert(kTmemDO + D / 2 <= 512 && kSmem <= 232448, "tensor / shared memory");
 };
 
-// NSW soft-max warpgroups (2 or 4) + 4 service warps (TMA, MMA, 2 idle) + the fold warpgroup
-template <int NSW> struct BwdThreads {
-  static constexpr int kSoftmax = 128 * NSW;
-  static constexpr int kTotal = 128 + kSoftmax + 128;
-  static constexpr int kFoldWarp0 = 4 + 4 * NSW;  // first warp of the fold warpgroup (a multiple of 4)
+// The steps (q-tile, j-tile, k) of a call in the order they are cut: heads, q-tiles, j-tiles, k.  Causal mask
+// j <= q <= j + k1w,  k <= q <= k + k2w,  k - kkl <= j <= k + kkr:  a q-tile [qa, qb] meets the j-tiles of rows
+// [qa - k1w, qb], and a pair of tiles the k in [max(qa - k2w, ja - kkr), min(qb, jb + kkl)].
+struct BwdGeometry {
+  int T, nq, q_mod, q_rem, causal;
+  int k1w, k2w, kkl, kkr;  // windows of the causal mask (T or more = unbounded)
+  int JT;                  // rows of a j-tile
+  __host__ __device__ int q_tiles() const { return (nq + 127) / 128; }
+  __host__ __device__ int first_q(int qt) const { return q_rem + qt * 128 * q_mod; }
+  __host__ __device__ int last_q(int qt) const {
+    const int i = qt * 128 + 127;
+    return q_rem + (i < nq ? i : nq - 1) * q_mod;
+  }
+  __host__ __device__ int j_first(int qt) const {
+    const int lo = first_q(qt) - k1w;
+    return causal && lo > 0 ? lo / JT : 0;
+  }
+  __host__ __device__ int j_last(int qt) const { return (causal ? last_q(qt) : T - 1) / JT; }
+  __host__ __device__ int k_range(int qt, int jt, int& k0) const {   // number of steps of a pair of tiles
+    k0 = 0;
+    if (!causal) return T;
+    const int qa = first_q(qt), qb = last_q(qt), ja = jt * JT, jb = ja + JT - 1;
+    if (qa - k2w > k0) k0 = qa - k2w;
+    if (ja - kkr > k0) k0 = ja - kkr;
+    const int k1 = qb < jb + kkl ? qb : jb + kkl;
+    return k1 >= k0 ? k1 - k0 + 1 : 0;
+  }
 };
 
 struct BwdParams {
-  const void *q, *o, *d_o;
-  const void* x[2];  // row key tensor per role (raw pointers, for the dQ fold)
-  const float* lse;
-  void* dq;
-  int T, BN, nq, q_mod, q_rem, causal;
-  int k1w, k2w, kkl, kkr;  // windows of the causal mask (T or more = unbounded)
+  const void *q, *d_o, *k2, *v2;
+  const float *lse, *drow;
+  float *dq, *dk1, *dk2, *dsv1, *dv2;   // fp32 sums, zero on entry
+  BwdGeometry g;
+  int BN;
+  int i_first;             // query rows (of the shard) before this one are not this kernel's
+  int parts;               // > 0: every head is cut in this many parts; 0: the whole line of steps in gridDim.x parts
+  long head_steps;         // steps of one head
   float alpha;
   int* status;
 };
 
+struct BwdItem {
+  int bh, qt, jt, k0, len, flags, pad[2];   // len 0: no more items
+};
+enum { kFirstOfQ = 1, kLastOfQ = 2 };       // the first / last item of a run over the j-tiles of one q-tile
+constexpr int kItemSlots = 4;               // (an item is read before its successor but one is written)
+
 struct BwdBarriers {
-  uint64_t ring_full[8], ring_empty[8];
-  uint64_t xy_full, ax_ready, ay_ready, a_free;  // A (score operand) and A' (dP operand) become ready separately
-  uint64_t s_ready, dp_ready, ds_ready;              // slab hand-offs
-  // P in two column halves, a pair of barriers per slab parity: with the early score product the soft-max warps
-  // can hand over P(c+1) before the issuing warp has looked at P(c) (it may be waiting for the fold at a tile's
-  // first slab), and a barrier that is two phases ahead of its waiter reads as not ready for ever
-  uint64_t p_ready[2][2];
-  uint64_t s_free;                                   // head dimension 64: the soft-max warps hold a slab's scores in registers
-  uint64_t gu_done, u_free, g_free;               // tile hand-offs with the fold warpgroup (U is drained first)
-  uint64_t sm_sync, fold_sync;
-  uint64_t vec_free[2];                           // fold warpgroup -> soft-max: a copy of Q[q] / dO[q] is no longer read
+  BwdItem items[kItemSlots];
+  uint64_t tile_full, tile_free;            // Q, dO, K1, SiLU(V1) of an item
+  uint64_t vec_full[kVecSlots], vec_empty[kVecSlots];
+  uint64_t a_ready[2], a_free[2], ap_ready;  // A: doubled by step parity (its producer may be two steps ahead)
+  uint64_t s_ready, s_free, p_ready, dp_ready, ds_ready, ds_free[2];
+  uint64_t acc_done[2], acc_free[2];         // G, U
+  uint64_t qdo_ready, dq_done, dq_free;
   uint32_t tmem_base;
   int abort_flag;
 };
 
+// One CTA's part of the line of steps, item by item (walked by the loader warp, which hands the items to the others).
+struct BwdWalk {
+  const BwdGeometry& g;
+  long left;                    // steps of this CTA not handed out yet
+  int bh, qt, jt, k0, len;      // next item (len 0: none)
+
+  __device__ void step() {
+    if (++jt > g.j_last(qt)) {
+      if (++qt == g.q_tiles()) {
+        qt = 0;
+        ++bh;
+      }
+      jt = g.j_first(qt);
+    }
+  }
+  __device__ void find(long skip) {   // first item with steps, from (bh, qt, jt) on, less `skip` steps
+    len = 0;
+    while (left > 0) {
+      const int n = g.k_range(qt, jt, k0);
+      if (n > skip) {
+        k0 += (int)skip;
+        len = n - (int)skip < left ? n - (int)skip : (int)left;
+        left -= len;
+        return;
+      }
+      skip -= n;
+      step();
+    }
+  }
+  __device__ explicit BwdWalk(const BwdParams& p) : g(p.g) {
+    long s0, s1;
+    const long H = p.head_steps;
+    if (p.parts > 0) {
+      const int b = blockIdx.x / p.parts, i = blockIdx.x % p.parts;
+      s0 = b * H + H * i / p.parts;
+      s1 = b * H + H * (i + 1) / p.parts;
+    } else {
+      const long total = H * p.BN, c = gridDim.x;
+      s0 = total / c * blockIdx.x + total % c * blockIdx.x / c;
+      s1 = total / c * (blockIdx.x + 1) + total % c * (blockIdx.x + 1) / c;
+    }
+    left = s1 - s0;
+    bh = (int)(s0 / H);
+    qt = 0;
+    jt = g.j_first(0);
+    find(s0 % H);
+  }
+  // hands out the item found last and looks for the one after it
+  __device__ BwdItem next(const BwdItem& prev) {
+    BwdItem it{bh, qt, jt, k0, len, 0, {0, 0}};
+    if (len == 0) return it;
+    if (bh != prev.bh || qt != prev.qt) it.flags |= kFirstOfQ;
+    step();
+    find(0);
+    if (len == 0 || bh != it.bh || qt != it.qt) it.flags |= kLastOfQ;
+    return it;
+  }
+};
 
 // fp16 only: the recomputed probabilities of a query that attends n pairs are ~1/n, which for late rows lies below
-// fp16's normal range (6e-5; 1/n = 2e-7 at q = 2048).  P and dS are therefore formed times 2^e, e = min(10, log2 of
-// the attended pairs' count bound), and the fold warpgroup divides it out of G and U.  2^10 keeps a probability of 1
-// times a dP - Dq of up to 64 finite.  bf16 has fp32's exponent range and needs none of this (e = 0).
+// fp16's normal range (6e-5; 1/n = 2e-7 at q = 2048).  P and dS are therefore formed times 2^e, and the folds divide
+// it out.  One e per q-tile, since G and U sum over its queries: it puts the tile's smallest mean probability at 2^-8
+// (e <= 10: a probability of 1 times a dP - Dq of up to 64 stays finite).  bf16 has fp32's exponent range: e = 0.
 template <typename T16>
-__device__ __forceinline__ int prob_shift(int q, int causal, int T, int k1w, int k2w) {
+__device__ __forceinline__ int prob_shift(int q_last, int causal, int T, int k1w, int k2w) {
   if constexpr (std::is_same<T16, __half>::value) {
-    const int n1 = causal ? min(q, k1w) + 1 : T, n2 = causal ? min(q, k2w) + 1 : T;
-    const int e = (31 - __clz(n1)) + (31 - __clz(n2));
-    return min(10, e);
+    const int n1 = causal ? min(q_last, k1w) + 1 : T, n2 = causal ? min(q_last, k2w) + 1 : T;
+    return max(0, min(10, (31 - __clz(n1)) + (31 - __clz(n2)) - 8));
   }
   return 0;
 }
 
-// The four 64-row-box maps of the key / value tensors are used by the CTA-pair variant only.
-struct BwdHalfMaps {
-  CUtensorMap k1, k2, sv1, v2;
-};
+__device__ __forceinline__ void red_add(float* p, float v) {
+  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
+__device__ __forceinline__ void red_add2(float* p, float a, float b) {
+  asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(a), "f"(b) : "memory");
+}
+__device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
 
-// PAIR: the kernel runs as clusters of two CTAs that take two queries of one (head, role) in lockstep: CTA `rank`
-// owns query 2 i + rank with its own operand tiles, soft-max and fold, and the even CTA issues every product for both
-// with cta_group::2 (M = 256: 128 pair rows per CTA).  The column tiles are then shared: each CTA holds half of a
-// tile's N extent per product (64 of its 128 rows for S / dP, 64 of its D columns for G / U), so the tensor cores
-// read 128 KB of shared memory per slab and SM instead of 192 KB.
-template <int D, typename T16, int NSW, bool PAIR>
-__global__ void __launch_bounds__(BwdThreads<NSW>::kTotal, 1)
-tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__ CUtensorMap tmK2,
-               const __grid_constant__ CUtensorMap tmSV1, const __grid_constant__ CUtensorMap tmV2,
-               const __grid_constant__ CUtensorMap tmDK1, const __grid_constant__ CUtensorMap tmDK2,
-               const __grid_constant__ CUtensorMap tmDSV1, const __grid_constant__ CUtensorMap tmDV2,
-               const __grid_constant__ BwdHalfMaps half, BwdParams p) {
-  static_assert(!PAIR || D == 128, "the CTA-pair tile layout is written for head dimension 128");
+template <int D, typename T16>
+__global__ void __launch_bounds__(kBwdThreads, 1)
+tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
+               const __grid_constant__ CUtensorMap tmK1, const __grid_constant__ CUtensorMap tmSV1, const BwdParams p) {
   using Cfg = BwdCfg<D>;
-  constexpr int NS = Cfg::kStages;
-  constexpr int KH = D / 64;
-  constexpr int kNumSoftmax = BwdThreads<NSW>::kSoftmax;
-  constexpr int kFoldWarp0 = BwdThreads<NSW>::kFoldWarp0;
-  constexpr int CW = kBC / NSW;  // slab columns owned by one soft-max warpgroup
-  // Head dimension 64 leaves 128 columns of tensor memory free: P then goes to a buffer of its own (two, by slab
-  // parity) instead of over the scores, and the next slab's score product is issued as soon as the soft-max warps hold
-  // this slab's scores in registers (`s_free`) instead of after U has consumed P: the loop S -> P -> U -> S is open.
-  // (U(c) is issued before S(c+2), and the pipe runs in order, so P(c) has been consumed when P(c+2) is written.)
-  constexpr bool kFreeS = D == 64 && !PAIR;
+  constexpr int JT = Cfg::JT, CW = Cfg::CW;
   extern __shared__ __align__(1024) uint8_t smem[];
-  static_assert(sizeof(BwdBarriers) <= 288, "barrier block too large");
+  static_assert(sizeof(BwdBarriers) <= 448, "barrier block too large");
   BwdBarriers& bars = *reinterpret_cast<BwdBarriers*>(smem + Cfg::kOffBars);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (smem_u32(smem) & 1023u) {
@@ -154,770 +221,822 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
     if (tid == 0 && p.status) atomicOr(p.status, 8);
     return;
   }
-
   if (tid == 0) {
     bars.abort_flag = 0;
-    for (int i = 0; i < NS; ++i) {
-      mbar_init(&bars.ring_full[i], 1);
-      mbar_init(&bars.ring_empty[i], 1);
+    mbar_init(&bars.tile_full, 1);
+    mbar_init(&bars.tile_free, 1 + 8);   // the item's last product, and the fold warps (they read K1, SiLU(V1))
+    for (int i = 0; i < kVecSlots; ++i) {
+      mbar_init(&bars.vec_full[i], 32);
+      mbar_init(&bars.vec_empty[i], 8);
     }
-    mbar_init(&bars.xy_full, 1);
-    // (hand-offs to the issuing thread: every thread arrives, or, in a pair, one lane per warp of both CTAs on the
-    //  even CTA's barrier)
-    constexpr uint32_t kToMmaSm = PAIR ? 2 * kNumSoftmax / 32 : kNumSoftmax, kToMmaFold = PAIR ? 2 * 4 : 128;
-    mbar_init(&bars.ax_ready, kToMmaSm);
-    mbar_init(&bars.ay_ready, kToMmaSm);
-    mbar_init(&bars.a_free, 1);   // a commit behind the tile's last score / dP products
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bars.a_ready[i], 4);
+      mbar_init(&bars.a_free[i], 1);
+      mbar_init(&bars.ds_free[i], 1);
+    }
+    mbar_init(&bars.ap_ready, 4);
     mbar_init(&bars.s_ready, 1);
+    mbar_init(&bars.s_free, 8);
+    mbar_init(&bars.p_ready, 8);
     mbar_init(&bars.dp_ready, 1);
-    for (int i = 0; i < 4; ++i) mbar_init(&bars.p_ready[i >> 1][i & 1], kToMmaSm);
-    mbar_init(&bars.ds_ready, kToMmaSm);
-    mbar_init(&bars.s_free, kToMmaSm);
-    mbar_init(&bars.gu_done, 1);
-    mbar_init(&bars.u_free, kToMmaFold);
-    mbar_init(&bars.g_free, kToMmaFold);
-    mbar_init(&bars.sm_sync, kNumSoftmax);
-    mbar_init(&bars.fold_sync, 128);
-    mbar_init(&bars.vec_free[0], 128);
-    mbar_init(&bars.vec_free[1], 128);
+    mbar_init(&bars.ds_ready, 8);
+    mbar_init(&bars.acc_done[1], 1);
+    mbar_init(&bars.acc_free[1], 4);
+    mbar_init(&bars.acc_done[0], 1);
+    mbar_init(&bars.acc_free[0], 4);
+    mbar_init(&bars.qdo_ready, 8);
+    mbar_init(&bars.dq_done, 1);
+    mbar_init(&bars.dq_free, 8);
     fence_barrier_init();
   }
-  if (warp == 0) {
-    if constexpr (PAIR) {
-      tmem_alloc_pair(&bars.tmem_base, 512);
-      tmem_relinquish_pair();
-    } else {
-      tmem_alloc(&bars.tmem_base, 512);
-      tmem_relinquish();
-    }
+  if (warp == 16) {
+    tmem_alloc(&bars.tmem_base, 512);
+    tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
-  if constexpr (PAIR) cluster_sync_all();  // the other CTA's barriers are initialised before anything arrives on them
   tc_fence_after();
   const uint32_t tmem = bars.tmem_base;
   volatile int* abort_flag = &bars.abort_flag;
-  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
-  // work is dealt to CTAs, or to CTA pairs
-  const long unit = PAIR ? (long)(blockIdx.x >> 1) : (long)blockIdx.x;
-  const long n_units = PAIR ? (long)(gridDim.x >> 1) : (long)gridDim.x;
-  // hand-off to the issuing thread (after the caller's fences)
-  auto to_mma = [&](uint64_t* bar) {
-    if constexpr (PAIR) {
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(mbar_in_cta(bar, 0));
-    } else {
-      mbar_arrive(bar);
-    }
+  const BwdGeometry& g = p.g;
+  const int T = g.T;
+  // (every lane waits; the vote keeps the warp converged whatever a lane's wait returned)
+  auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+  };
+  // one arrival per warp, after the caller's fences
+  auto arrive_warp = [&](uint64_t* bar) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
   };
 
-  const int T = p.T;
-  // items: (query, head, role), or in a pair (two queries, head, role)
-  const long n_items = (long)(PAIR ? p.nq / 2 : p.nq) * p.BN * 2;
-
-  // item -> (role, head, query); late (expensive) queries first.  Items 2r and 2r + 1 are the two roles of one (head,
-  // query); which of them is which alternates with r in blocks of half the grid, so that the items of one CTA
-  // (gridDim.x apart) alternate between the roles: role-0 tiles cost more (their fold also forms dQ), and a CTA
-  // that only ever saw one role would finish 6 % later than its neighbour.
-  // In a pair `q` is this CTA's query and `qr` the later one of the two, whose tile ranges both CTAs walk (the
-  // earlier query masks what lies beyond it).
-  auto decode = [&](long item, int& role, int& bh, int& q, int& qr) {
-    const long r = item >> 1;
-    role = (int)((item ^ (r / ((n_units + 1) >> 1))) & 1);
-    bh = (int)(r % p.BN);
-    if constexpr (PAIR) {
-      const int i_hi = p.nq - 1 - 2 * (int)(r / p.BN);
-      q = p.q_rem + (i_hi - 1 + (int)rank) * p.q_mod;
-      qr = p.q_rem + i_hi * p.q_mod;
-    } else {
-      q = p.q_rem + (p.nq - 1 - (int)(r / p.BN)) * p.q_mod;
-      qr = q;
-    }
-  };
-  // Causal mask j <= q <= j + k1w, k <= q <= k + k2w, k - kkl <= j <= k + kkr, seen from a role's rows x and
-  // columns c (role 0: x = k, c = j; role 1: x = j, c = k):  x in [q - xw, q],  c in [q - cw, q],  c in [x - below, x + above].
-  struct Win { int xw, cw, below, above; };
-  auto role_win = [&](int role) {
-    return role == 0 ? Win{p.k2w, p.k1w, p.kkl, p.kkr} : Win{p.k1w, p.k2w, p.kkr, p.kkl};
-  };
-  // row tiles of a query: rows [max(0, q - xw, q - cw - above), q]  (rows below the third bound see no column);
-  // column slabs of row tile xt: [max(0, q - cw, x_first - below), min(q, x_last + above)], never empty
-  auto x_range = [&](int q, const Win& w, int& xt0, int& nxt) {
-    if (!p.causal) {
-      xt0 = 0;
-      nxt = (T + 127) / 128;
-      return;
-    }
-    const int xlo = max(0, max(q - w.xw, q - w.cw - w.above));
-    xt0 = xlo / 128;
-    nxt = q / 128 - xt0 + 1;
-  };
-  auto c_range = [&](int q, const Win& w, int xt, int& c0, int& ncs) {
-    if (!p.causal) {
-      c0 = 0;
-      ncs = (T + kBC - 1) / kBC;
-      return;
-    }
-    const int xlo = max(0, max(q - w.xw, q - w.cw - w.above));
-    const int xa = max(xt * 128, xlo), xb = min(xt * 128 + 127, q);
-    const int ca = max(0, max(q - w.cw, xa - w.below)), cb = min(q, xb + w.above);
-    c0 = ca / kBC;
-    ncs = cb / kBC - c0 + 1;
+  // The item of phase `items` of tile_full; false: there is none, or the wait ran out (`alive` is then cleared).
+  auto next_item = [&](uint32_t items, BwdItem& it, bool& alive) -> bool {
+    alive = wait_all(&bars.tile_full, items & 1);
+    if (!alive) return false;
+    const int4 a = *reinterpret_cast<const int4*>(&bars.items[items % kItemSlots]);
+    const int2 b = *reinterpret_cast<const int2*>(&bars.items[items % kItemSlots].len);
+    it.bh = a.x; it.qt = a.y; it.jt = a.z; it.k0 = a.w; it.len = b.x; it.flags = b.y;
+    return it.len > 0;
   };
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    // (like the MMA warp: the whole warp walks the schedule converged, one elected lane issues the copies)
-    {
-      const bool leader = elect_one();
-      if (leader) {
-        const CUtensorMap* maps[8] = {&tmK1, &tmK2, &tmSV1, &tmV2, &tmDK1, &tmDK2, &tmDSV1, &tmDV2};
-        for (int i = 0; i < 8; ++i) tma_prefetch_desc(maps[i]);
-      }
-      uint32_t xt_count = 0, pos = 0;
-      bool alive = true;
-      // One column tile (128 rows of Kc or Vc) into the next ring stage.  In a pair each CTA fetches what its half
-      // of the products reads: rows [64 rank, 64 rank + 64) of the tile (both 64-column halves, 8 KB each: the B
-      // operand of S / dP) and columns [64 rank, 64 rank + 64) of all 128 rows (16 KB: the B operand of G / U); the
-      // bytes of both CTAs are counted on the even CTA's barrier, where the issuing thread waits.
-      auto load_stage = [&](const CUtensorMap* tm, const CUtensorMap* tm_half, int row0, int bh) -> bool {
-        const int st = pos % NS;
-        if (!__all_sync(0xffffffffu, mbar_wait_x<PAIR>(&bars.ring_empty[st], ((pos / NS) & 1) ^ 1, abort_flag)))
-          return false;
-        uint8_t* dst = smem + Cfg::kOffRing + st * Cfg::kTileA;
-        if (leader) {
-          if constexpr (PAIR) {
-            if (rank == 0) mbar_arrive_expect_tx(&bars.ring_full[st], 2 * Cfg::kTileA);
-            const uint32_t full0 = mbar_in_cta(&bars.ring_full[st], 0);
-            tma_load_3d_pair(dst, tm_half, full0, 0, row0 + 64 * (int)rank, bh);
-            tma_load_3d_pair(dst + 8192, tm_half, full0, 64, row0 + 64 * (int)rank, bh);
-            tma_load_3d_pair(dst + 16384, tm, full0, 64 * (int)rank, row0, bh);
-          } else {
-            mbar_arrive_expect_tx(&bars.ring_full[st], Cfg::kTileA);
-            for (int hh = 0; hh < KH; ++hh) tma_load_3d(dst + hh * 16384, tm, &bars.ring_full[st], hh * 64, row0, bh);
+  if (warp < 8) {
+    set_regs<kRegsLaunch, kRegsSoftmax>();
+    // ------------------------------------------------------------------ soft-max warpgroups
+    const int wg = warp >> 2, wq = warp & 3;
+    const int row = wq * 32 + lane;
+    const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
+    uint8_t* const prow = smem + Cfg::kOffP + (JT == 128 ? wg * 16384 : 0);
+    const int ch0 = JT == 128 ? 0 : wg * 4;    // first 16-byte chunk of this thread's columns in its 128-byte row
+    uint32_t n = 0, runs = 0, items = 0;
+    bool alive = true;
+    BwdItem it;
+    int q = 0;
+    bool q_ok = false, single = false;
+    float lse2 = 0.f, drow = 0.f, dq_scale = 0.f;
+    while (alive && next_item(items, it, alive)) {
+      ++items;
+      if (it.flags & kFirstOfQ) {
+        const int i = it.qt * 128 + row;
+        q_ok = i < g.nq && i >= p.i_first;
+        q = g.q_rem + (q_ok ? i : 0) * g.q_mod;
+        const int e = prob_shift<T16>(g.last_q(it.qt), g.causal, T, g.k1w, g.k2w);
+        lse2 = __ldg(p.lse + (size_t)it.bh * T + q) * kLog2e - (float)e;
+        drow = __ldg(p.drow + (size_t)it.bh * T + q);
+        dq_scale = exp2f(-(float)e) * kLn2;    // A carries alpha * log2(e)
+        // A query that attends a single pair has P = 1 and a score gradient of exactly zero (TdpMask::single_pair):
+        // P (dP - Dq) has two terms that are equal only up to the 16-bit rounding of the stored output, so its dS
+        // is set to zero.
+        {
+          // this query's row of Q (warpgroup 0) or dO (warpgroup 1) as the score products' operand in tensor memory
+          // (the previous run's products have all run: its dq_done was waited for)
+          const T16* src = (const T16*)(wg == 0 ? p.q : p.d_o) + ((size_t)it.bh * T + q) * D;
+#pragma unroll
+          for (int c = 0; c < D; c += 32) {
+            uint32_t v[16];
+#pragma unroll
+            for (int e4 = 0; e4 < 4; ++e4) {
+              const uint4 x = q_ok ? __ldg(reinterpret_cast<const uint4*>(src + c + e4 * 8)) : make_uint4(0, 0, 0, 0);
+              v[e4 * 4] = x.x;
+              v[e4 * 4 + 1] = x.y;
+              v[e4 * 4 + 2] = x.z;
+              v[e4 * 4 + 3] = x.w;
+            }
+            tmem_st16(tmem + lane_base + (wg == 0 ? Cfg::kTmemQ : Cfg::kTmemDO) + c / 2, v);
           }
+          tmem_wait_st();
+          tc_fence_before();
+          arrive_warp(&bars.qdo_ready);
         }
-        ++pos;
-        return true;
-      };
-      for (long item = unit; item < n_items && alive; item += n_units) {
-        int role, bh, q, qr, xt0, nxt;
-        decode(item, role, bh, q, qr);
-        const Win win = role_win(role);
-        x_range(qr, win, xt0, nxt);
-        // role 0: columns K1 / SiLU(V1), rows K2 / V2;   role 1: columns K2 / V2, rows K1 / SiLU(V1)
-        const CUtensorMap* tmKc = role == 0 ? &tmK1 : &tmK2;
-        const CUtensorMap* tmVc = role == 0 ? &tmSV1 : &tmV2;
-        const CUtensorMap* tmKcH = role == 0 ? &half.k1 : &half.k2;
-        const CUtensorMap* tmVcH = role == 0 ? &half.sv1 : &half.v2;
-        const CUtensorMap* tmX = role == 0 ? &tmK2 : &tmK1;
-        const CUtensorMap* tmY = role == 0 ? &tmV2 : &tmSV1;
-        for (int xt = xt0; xt < xt0 + nxt && alive; ++xt, ++xt_count) {
-          int c0, ncs;
-          c_range(qr, win, xt, c0, ncs);
-          // the tile's first key / value slab does not depend on the operand buffers: fetch it before waiting for them
-          alive = load_stage(tmKc, tmKcH, c0 * kBC, bh);
-          if (alive) alive = load_stage(tmVc, tmVcH, c0 * kBC, bh);
-          if (!alive || !__all_sync(0xffffffffu, mbar_wait_x<PAIR>(&bars.a_free, (xt_count & 1) ^ 1, abort_flag))) {
-            alive = false;
-            break;
+        single = TdpMask{g.causal, T, g.k1w, g.k2w, g.kkl, g.kkr}.single_pair(q);
+      }
+      const bool any_single = __any_sync(0xffffffffu, single);
+      const float2 nlse = make_float2(-lse2, -lse2), ndq = make_float2(-drow, -drow);
+      const int j0 = it.jt * JT + wg * CW;
+      for (int i = 0; i < it.len; ++i, ++n) {
+        const int k = it.k0 + i;
+        // columns this query sees at this k, relative to the thread's first: [lo, hi] (empty: hi < lo)
+        int lo = -j0, hi = T - 1 - j0;
+        if (g.causal) {
+          lo = max(q - g.k1w, k - g.kkl) - j0;
+          hi = k <= q && q - k <= g.k2w ? min(q, k + g.kkr) - j0 : lo - 1;
+        }
+        if (!q_ok) hi = lo - 1;
+        // 32 columns at a time: S -> P, then dP and P (still in fp32) -> dS
+        alive = wait_all(&bars.s_ready, n & 1);
+        if (!alive) break;
+        tc_fence_after();
+        uint8_t* const dsrow = prow + (1 + (n & 1)) * Cfg::kTileP;
+        const bool full = __all_sync(0xffffffffu, lo <= 0 && hi >= CW - 1);
+#pragma unroll 1
+        for (int c0 = 0; c0 < CW; c0 += 32) {
+          uint32_t s[32];
+          tmem_ld32(tmem + lane_base + Cfg::kTmemS + wg * CW + c0, s);
+          tmem_wait_ld();
+          if (c0 + 32 == CW) {
+            // the scores are in registers: the next step's product may overwrite them
+            tc_fence_before();
+            arrive_warp(&bars.s_free);
           }
-          if (leader) {
-            mbar_arrive_expect_tx(&bars.xy_full, 2 * Cfg::kTileA);
-            for (int hh = 0; hh < KH; ++hh) {
-              tma_load_3d(smem + Cfg::kOffA + hh * 16384, tmX, &bars.xy_full, hh * 64, xt * 128, bh);
-              tma_load_3d(smem + Cfg::kOffA2 + hh * 16384, tmY, &bars.xy_full, hh * 64, xt * 128, bh);
+          if (full) {
+#pragma unroll
+            for (int c = 0; c < 32; c += 2) {
+              const float2 x = __fadd2_rn(make_float2(__uint_as_float(s[c]), __uint_as_float(s[c + 1])), nlse);
+              s[c] = __float_as_uint(exp2f(x.x));
+              s[c + 1] = __float_as_uint(exp2f(x.y));
+            }
+          } else {
+#pragma unroll
+            for (int c = 0; c < 32; ++c)
+              s[c] = c0 + c >= lo && c0 + c <= hi ? __float_as_uint(exp2f(__uint_as_float(s[c]) - lse2)) : 0u;
+          }
+          if (c0 == 0) {
+            // the previous step's U has read P
+            alive = wait_all(&bars.acc_done[1], (n & 1) ^ 1);
+            if (!alive) break;
+          }
+#pragma unroll
+          for (int c = 0; c < 32; c += 8) {
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              w[e] = pack2<T16>(__uint_as_float(s[c + 2 * e]), __uint_as_float(s[c + 2 * e + 1]));
+            *reinterpret_cast<uint4*>(prow + swz128(row, ch0 + ((c0 + c) >> 3))) = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+          if (c0 + 32 == CW) {
+            fence_async_smem();
+            arrive_warp(&bars.p_ready);
+          }
+          if (any_single) {
+#pragma unroll
+            for (int c = 0; c < 32; ++c) s[c] = single ? 0u : s[c];
+          }
+          if (c0 == 0) {
+            alive = wait_all(&bars.dp_ready, n & 1);
+            if (alive) alive = wait_all(&bars.ds_free[n & 1], ((n >> 1) & 1) ^ 1);
+            if (!alive) break;
+            tc_fence_after();
+          }
+#pragma unroll
+          for (int c1 = 0; c1 < 32; c1 += 16) {
+            uint32_t dp[16];
+            tmem_ld16(tmem + lane_base + Cfg::kTmemDP + wg * CW + c0 + c1, dp);
+            tmem_wait_ld();
+#pragma unroll
+            for (int c = 0; c < 16; c += 8) {
+              uint32_t w[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float2 d =
+                    __fadd2_rn(make_float2(__uint_as_float(dp[c + 2 * e]), __uint_as_float(dp[c + 2 * e + 1])), ndq);
+                const float2 ds = __fmul2_rn(
+                    make_float2(__uint_as_float(s[c1 + c + 2 * e]), __uint_as_float(s[c1 + c + 2 * e + 1])), d);
+                w[e] = pack2<T16>(ds.x, ds.y);
+              }
+              *reinterpret_cast<uint4*>(dsrow + swz128(row, ch0 + ((c0 + c1 + c) >> 3))) = make_uint4(w[0], w[1], w[2], w[3]);
             }
           }
-          for (int c = c0 + 1; c < c0 + ncs && alive; ++c) {
-            alive = load_stage(tmKc, tmKcH, c * kBC, bh);
-            if (alive) alive = load_stage(tmVc, tmVcH, c * kBC, bh);
-          }
         }
+        if (!alive) break;
+        tc_fence_before();
+        fence_async_smem();
+        arrive_warp(&bars.ds_ready);
       }
-      if (!alive && (!PAIR || rank == 0)) {
-        const uint32_t first = pos > (uint32_t)NS ? pos - NS : 0;
-        for (uint32_t q2 = first; q2 < pos; ++q2) {
-          const long long t0 = clock64();
-          while (!mbar_try_wait(&bars.ring_full[q2 % NS], (q2 / NS) & 1) && clock64() - t0 < kWaitTicks / 8) {
+      if (!alive) break;
+      if ((it.flags & kLastOfQ)) {
+        // ---- dQ of this q-tile (over the j-tiles this CTA had of it): half of the columns per warpgroup
+        alive = wait_all(&bars.dq_done, runs & 1);
+        if (!alive) break;
+        tc_fence_after();
+        float* dst = p.dq + ((size_t)it.bh * T + q) * D + wg * (D / 2);
+#pragma unroll
+        for (int c0 = 0; c0 < D / 2; c0 += 32) {
+          uint32_t v[32];
+          tmem_ld32(tmem + lane_base + Cfg::kTmemDQ + wg * (D / 2) + c0, v);
+          tmem_wait_ld();
+          if (q_ok) {
+#pragma unroll
+            for (int c = 0; c < 32; c += 4)
+              red_add4(dst + c0 + c, __uint_as_float(v[c]) * dq_scale, __uint_as_float(v[c + 1]) * dq_scale,
+                       __uint_as_float(v[c + 2]) * dq_scale, __uint_as_float(v[c + 3]) * dq_scale);
           }
         }
+        tc_fence_before();
+        arrive_warp(&bars.dq_free);
+        ++runs;
       }
     }
-  } else if (warp == 1) {
+  } else if (warp < 16) {
+    set_regs<kRegsLaunch, kRegsFold>();
+    // ------------------------------------------------------------------ operand / fold warpgroups
+    // role 0: forms A two steps ahead, folds G into dK1 (registers) and dK2;  role 1: forms A' one step ahead, folds
+    // U into dSiLU(V1) and dV2.  The fold reads the accumulator as 16 x 256-bit fragments (thread t: rows t / 4 + 8 i,
+    // columns 8 g + 2 (t % 4) and the next), which is also how ldmatrix hands out the K1 / SiLU(V1) tile: the sums
+    // over the 32 rows of a warp are four rows within a thread and a 7-shuffle tree per 32 columns.
+    // (the role is a run-time value: one copy of the code for both warpgroups halves what the instruction caches have to
+    // hold of it)
+    const int role = (warp - 8) >> 2, w = warp & 3;
+    const float* const vec = reinterpret_cast<const float*>(smem + Cfg::kOffVec) + role * D;
+    const uint32_t tacc = tmem + ((uint32_t)(w * 32) << 16) + (role ? Cfg::kTmemU : Cfg::kTmemG);
+    const int ahead = 2 - role;
+    // address of this lane's row of the four 8 x 8 blocks of (16-column group c16, 16-lane half hl) within a tile
+    auto frag = [&](int c16, int hl) -> uint32_t {
+      if constexpr (D == 64) {
+        // (j 0-7, h 0-7), (j 8-15, h 0-7), (j 0-7, h 8-15), (j 8-15, h 8-15)
+        return swz128(w * 32 + hl * 16 + (lane & 15), c16 * 2 + (lane >> 4));
+      } else {
+        // (h 0-7, j 0-7), (h 8-15, j 0-7), (h 0-7, j 8-15), (h 8-15, j 8-15), transposed
+        const int ch = w * 4 + hl * 2 + ((lane >> 3) & 1), j = c16 * 16 + (lane >> 4) * 8 + (lane & 7);
+        return (ch >> 3) * (JT * 128) + swz128(j, ch & 7);
+      }
+    };
+    const uint32_t raw_u = smem_u32(smem + Cfg::kOffK1 + role * Cfg::kTileJ);
+    const uint32_t formed_u = smem_u32(smem + Cfg::kOffA + role * 2 * Cfg::kTileJ);
+    uint32_t n = 0, items = 0, vb0 = 0;
+    bool alive = true;
+    BwdItem it;
+    while (alive && next_item(items, it, alive)) {
+      float2 acc[32];   // [16-column group c16][16-lane half][8-column group][row of the pair]
+#pragma unroll
+      for (int i = 0; i < 32; ++i) acc[i] = make_float2(0.f, 0.f);
+      uint32_t x[4][2][4];   // this thread's elements of the K1 / SiLU(V1) tile, [c16][hl][8 x 8 block]
+#pragma unroll
+      for (int c16 = 0; c16 < 4; ++c16)
+#pragma unroll
+        for (int hl = 0; hl < 2; ++hl) {
+          if constexpr (D == 64) ldmatrix_x4(x[c16][hl], raw_u + frag(c16, hl));
+          else ldmatrix_x4_trans(x[c16][hl], raw_u + frag(c16, hl));
+        }
+      arrive_warp(&bars.tile_free);
+      const int len = it.len;
+      const int e = prob_shift<T16>(g.last_q(it.qt), g.causal, T, g.k1w, g.k2w);
+      const float unshift = exp2f(-(float)e);
+      const float zscale = role ? unshift : unshift * p.alpha;
+      float* zrow = (role ? p.dv2 : p.dk2) + ((size_t)it.bh * T + it.k0) * D;
+      auto form = [&](int i) -> bool {
+        const uint32_t m = n + i;
+        if ((i & (kVecBatch - 1)) == 0) {
+          const uint32_t vb = vb0 + i / kVecBatch;
+          if (!wait_all(&bars.vec_full[vb % kVecSlots], (vb / kVecSlots) & 1)) return false;
+        }
+        // A: the buffer's previous step has been through dQ;  A': the previous step's dP product has run
+        if (!wait_all(role ? &bars.dp_ready : &bars.a_free[m & 1], ((role ? m : m >> 1) & 1) ^ 1)) return false;
+        const float* v = vec + ((vb0 * kVecBatch + i) % (kVecSlots * kVecBatch)) * Cfg::kVecRow;
+        const uint32_t dst = formed_u + (role ? 0 : (m & 1) * Cfg::kTileJ);
+        float vr[4];
+        if constexpr (D == 128) {
+#pragma unroll
+          for (int r = 0; r < 4; ++r) vr[r] = v[w * 32 + r * 8 + (lane >> 2)];
+        }
+#pragma unroll
+        for (int c16 = 0; c16 < 4; ++c16) {
+          float2 v0, v1;
+          if constexpr (D == 64) {
+            v0 = *reinterpret_cast<const float2*>(v + c16 * 16 + 2 * (lane & 3));
+            v1 = *reinterpret_cast<const float2*>(v + c16 * 16 + 8 + 2 * (lane & 3));
+          }
+#pragma unroll
+          for (int hl = 0; hl < 2; ++hl) {
+            uint32_t a[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+              float2 m2;
+              if constexpr (D == 64) m2 = b < 2 ? v0 : v1;
+              else m2 = make_float2(vr[hl * 2 + (b & 1)], vr[hl * 2 + (b & 1)]);
+              const float2 f = __fmul2_rn(unpack2<T16>(x[c16][hl][b]), m2);
+              a[b] = pack2<T16>(f.x, f.y);
+            }
+            if constexpr (D == 64) stmatrix_x4(dst + frag(c16, hl), a);
+            else stmatrix_x4_trans(dst + frag(c16, hl), a);
+          }
+        }
+        fence_async_smem();
+        arrive_warp(role ? &bars.ap_ready : &bars.a_ready[m & 1]);
+        return true;
+      };
+      // (one loop, so that there is one copy of each of the two stages: step i forms operand i, folds step i - ahead)
+      for (int i0 = 0; i0 < len + ahead && alive; ++i0) {
+        const int i = i0 - ahead;
+        // (keeps the compiler from unpacking x once, outside the loop, into twice the registers)
+#pragma unroll
+        for (int c16 = 0; c16 < 4; ++c16)
+#pragma unroll
+          for (int b = 0; b < 8; ++b) asm volatile("" : "+r"(x[c16][b >> 2][b & 3]));
+        if (i0 < len) {
+          alive = form(i0);
+          if (!alive) break;
+        }
+        if (i < 0) continue;
+        alive = wait_all(&bars.acc_done[role], (n + i) & 1);
+        if (!alive) break;
+        tc_fence_after();
+        const float* v = vec + ((vb0 * kVecBatch + i) % (kVecSlots * kVecBatch)) * Cfg::kVecRow;
+        if constexpr (D == 64) {
+          // lanes are rows j, columns are h
+          float zout[2];
+#pragma unroll
+          for (int c32 = 0; c32 < 2; ++c32) {
+            float z[8];
+#pragma unroll
+            for (int g2 = 0; g2 < 2; ++g2) {
+              const int c16 = c32 * 2 + g2;
+              uint32_t d[2][8];
+#pragma unroll
+              for (int hl = 0; hl < 2; ++hl) tmem_ld_16x256b_x2(tacc + ((uint32_t)(hl * 16) << 16) + c16 * 16, d[hl]);
+              const float2 v0 = *reinterpret_cast<const float2*>(v + c16 * 16 + 2 * (lane & 3));
+              const float2 v1 = *reinterpret_cast<const float2*>(v + c16 * 16 + 8 + 2 * (lane & 3));
+              tmem_wait_ld();
+              if (c16 == 3) {
+                tc_fence_before();
+                arrive_warp(&bars.acc_free[role]);
+              }
+              float2 z0 = make_float2(0.f, 0.f), z1 = z0;
+#pragma unroll
+              for (int hl = 0; hl < 2; ++hl) {
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                  const float2 g0 = make_float2(__uint_as_float(d[hl][2 * r]), __uint_as_float(d[hl][2 * r + 1]));
+                  const float2 g1 = make_float2(__uint_as_float(d[hl][4 + 2 * r]), __uint_as_float(d[hl][5 + 2 * r]));
+                  float2& a0 = acc[c16 * 8 + hl * 4 + r];
+                  float2& a1 = acc[c16 * 8 + hl * 4 + 2 + r];
+                  a0 = __ffma2_rn(g0, v0, a0);
+                  a1 = __ffma2_rn(g1, v1, a1);
+                  z0 = __ffma2_rn(g0, unpack2<T16>(x[c16][hl][r]), z0);
+                  z1 = __ffma2_rn(g1, unpack2<T16>(x[c16][hl][2 + r]), z1);
+                }
+              }
+              z[g2 * 4 + 0] = z0.x;
+              z[g2 * 4 + 1] = z0.y;
+              z[g2 * 4 + 2] = z1.x;
+              z[g2 * 4 + 3] = z1.y;
+            }
+            // z[4 g2 + 2 g + e]: column 32 c32 + 16 g2 + 8 g + 2 (lane % 4) + e, over this thread's four rows; the tree
+            // over lane / 4 leaves one column per lane: g2 = lane bit 4, g = lane bit 3, e = lane bit 2
+#pragma unroll
+            for (int half = 4; half >= 1; half >>= 1) {
+              const bool upper = lane & (half * 4);
+#pragma unroll
+              for (int i2 = 0; i2 < half; ++i2) {
+                const float keep = upper ? z[i2 + half] : z[i2];
+                const float send = upper ? z[i2] : z[i2 + half];
+                z[i2] = keep + __shfl_xor_sync(0xffffffffu, send, half * 4);
+              }
+            }
+            zout[c32] = z[0];
+          }
+          const int col = (lane >> 4) * 16 + ((lane >> 3) & 1) * 8 + 2 * (lane & 3) + ((lane >> 2) & 1);
+          red_add(zrow + col, zout[0] * zscale);
+          red_add(zrow + 32 + col, zout[1] * zscale);
+        } else {
+          // lanes are columns h of the head, columns are rows j
+          float2 z[4];
+          float vr[4];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            z[r] = make_float2(0.f, 0.f);
+            vr[r] = v[w * 32 + r * 8 + (lane >> 2)];
+          }
+#pragma unroll
+          for (int c16 = 0; c16 < 4; ++c16) {
+            uint32_t d[2][8];
+#pragma unroll
+            for (int hl = 0; hl < 2; ++hl) tmem_ld_16x256b_x2(tacc + ((uint32_t)(hl * 16) << 16) + c16 * 16, d[hl]);
+            tmem_wait_ld();
+            if (c16 == 3) {
+              tc_fence_before();
+              arrive_warp(&bars.acc_free[role]);
+            }
+#pragma unroll
+            for (int hl = 0; hl < 2; ++hl) {
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                const float2 g0 = make_float2(__uint_as_float(d[hl][2 * r]), __uint_as_float(d[hl][2 * r + 1]));
+                const float2 g1 = make_float2(__uint_as_float(d[hl][4 + 2 * r]), __uint_as_float(d[hl][5 + 2 * r]));
+                const float2 vv = make_float2(vr[hl * 2 + r], vr[hl * 2 + r]);
+                float2& a0 = acc[c16 * 8 + hl * 4 + r];
+                float2& a1 = acc[c16 * 8 + hl * 4 + 2 + r];
+                a0 = __ffma2_rn(g0, vv, a0);
+                a1 = __ffma2_rn(g1, vv, a1);
+                float2& zz = z[hl * 2 + r];
+                zz = __ffma2_rn(g0, unpack2<T16>(x[c16][hl][r]), zz);
+                zz = __ffma2_rn(g1, unpack2<T16>(x[c16][hl][2 + r]), zz);
+              }
+            }
+          }
+          // z[r]: h = 32 w + 8 r + lane / 4 over this thread's 16 columns; the tree over lane % 4 leaves row r =
+          // 2 (lane bit 1) + (lane bit 0)
+          float zr[4];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) zr[r] = z[r].x + z[r].y;
+#pragma unroll
+          for (int half = 2; half >= 1; half >>= 1) {
+            const bool upper = lane & half;
+#pragma unroll
+            for (int i2 = 0; i2 < half; ++i2) {
+              const float keep = upper ? zr[i2 + half] : zr[i2];
+              const float send = upper ? zr[i2] : zr[i2 + half];
+              zr[i2] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+            }
+          }
+          red_add(zrow + w * 32 + (lane & 3) * 8 + (lane >> 2), zr[0] * zscale);
+        }
+        if ((i & (kVecBatch - 1)) == kVecBatch - 1 || i == len - 1)
+          arrive_warp(&bars.vec_empty[(vb0 + i / kVecBatch) % kVecSlots]);
+        zrow += D;
+      }
+      if (!alive) break;
+      n += len;
+      vb0 += (len + kVecBatch - 1) / kVecBatch;
+      ++items;
+      // ---- dK1 / dSiLU(V1) of this item
+      const float jscale = role ? unshift : unshift * kLn2;   // (the K2 rows carry alpha * log2(e))
+      float* const base = (role ? p.dsv1 : p.dk1) + (size_t)it.bh * T * D;
+#pragma unroll
+      for (int c16 = 0; c16 < 4; ++c16)
+#pragma unroll
+        for (int hl = 0; hl < 2; ++hl)
+#pragma unroll
+          for (int g = 0; g < 2; ++g)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              const float2 a = acc[c16 * 8 + hl * 4 + g * 2 + r];
+              const int lr = w * 32 + hl * 16 + r * 8 + (lane >> 2), lc = c16 * 16 + g * 8 + 2 * (lane & 3);
+              if constexpr (D == 64) {
+                const int j = it.jt * JT + lr;
+                if (j < T) red_add2(base + (size_t)j * D + lc, a.x * jscale, a.y * jscale);
+              } else {
+                const int j = it.jt * JT + lc;
+                if (j < T) red_add(base + (size_t)j * D + lr, a.x * jscale);
+                if (j + 1 < T) red_add(base + (size_t)(j + 1) * D + lr, a.y * jscale);
+              }
+            }
+    }
+  } else {
+   set_regs<kRegsLaunch, kRegsService>();
+   if (warp == 16) {
     // ------------------------------------------------------------------ MMA issuer
     // The whole warp walks the schedule in step and one elected lane issues: with converged control flow the
     // descriptor arithmetic stays on the uniform datapath, where a lone thread needs a register-to-uniform move
-    // per operand and loses its issue slots to the busy warps of its scheduler (a stand-alone loop of these chains
-    // under issue pressure: 15.3 k cycles per 32 instructions from one thread, 3.9 k from a converged warp).
-    if (rank == 0) {
-      const bool leader = elect_one();
-      constexpr int kFmt = std::is_same<T16, __nv_bfloat16>::value ? 1 : 0;
-      constexpr int kM = PAIR ? 256 : 128;   // rows of one instruction (both CTAs of a pair)
-      constexpr uint32_t idesc_s = make_idesc_f16(kM, kBC, kFmt, false, false);
-      constexpr uint32_t idesc_g = make_idesc_f16(kM, D, kFmt, false, true);
-      // descriptor low words; per instruction only a constant (in 16-byte units) is added
-      constexpr uint32_t kHi = desc_hi(1024);
-      constexpr uint32_t kTile16 = Cfg::kTileA >> 4;
-      const uint32_t aLo = desc_lo(smem_u32(smem + Cfg::kOffA), 16), a2Lo = desc_lo(smem_u32(smem + Cfg::kOffA2), 16);
-      const uint32_t ringK = desc_lo(smem_u32(smem + Cfg::kOffRing), 16);      // K-major view of a stage
-      // row-major (MN-major) view; in a pair the stage's second half: this CTA's 64 columns of all 128 rows
-      const uint32_t ringMN = desc_lo(smem_u32(smem + Cfg::kOffRing + (PAIR ? 16384 : 0)), 16384);
-      // K-major view: 64-column blocks of a tile are 16 KB apart, of a pair's 64-row half 8 KB
-      constexpr uint32_t kBlkK = (PAIR ? 8192 : 16384) >> 4;
-      auto commit = [&](uint64_t* bar) {
-        if (!leader) return;
-        if constexpr (PAIR) mma_commit_pair(bar); else mma_commit(bar);
-      };
-      auto mma_ss_any = [&](uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t acc) {
-        if (!leader) return;
-        if constexpr (PAIR) mma_ss_lo_pair(d, a_lo, b_lo, kHi, idesc, acc); else mma_ss_lo(d, a_lo, b_lo, kHi, idesc, acc);
-      };
-      auto mma_ts_any = [&](uint32_t d, uint32_t a_t, uint32_t b_lo, uint32_t idesc, uint32_t acc) {
-        if (!leader) return;
-        if constexpr (PAIR) mma_ts_lo_pair(d, a_t, b_lo, kHi, idesc, acc); else mma_ts_lo(d, a_t, b_lo, kHi, idesc, acc);
-      };
-      // (every lane waits; the vote keeps the warp converged whatever a lane's wait returned)
-      auto wait_all = [&](uint64_t* bar, uint32_t parity) {
-        return __all_sync(0xffffffffu, mbar_wait_x<PAIR>(bar, parity, abort_flag));
-      };
-      uint32_t xt_count = 0, base = 0, n = 0;
-      bool alive = true;
-      auto wait_full = [&](uint32_t pos) {
-        return wait_all(&bars.ring_full[pos % NS], (pos / NS) & 1);
-      };
-      // One 8-instruction accumulation chain each (D = 128): S = A Kc^T, dP = A' Vc^T (operands in shared
-      // memory, key/value tile K-major), U (+)= P Vc, G (+)= dS Kc (P / dS from tensor memory, the tile row-major).
-      auto issue_s = [&](uint32_t pos) -> bool {
-        if (!wait_full(pos)) return false;
-        const uint32_t bLo = ringK + (pos % NS) * kTile16;
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t kk = (k >> 2) * (16384 >> 4) + (k & 3) * 2, kb = (k >> 2) * kBlkK + (k & 3) * 2;
-          mma_ss_any(tmem + Cfg::kTmemS, aLo + kk, bLo + kb, idesc_s, k > 0);
-        }
-        commit(&bars.s_ready);
-        return true;
-      };
-      auto issue_dp = [&](uint32_t pos) -> bool {
-        if (!wait_full(pos)) return false;
-        const uint32_t bLo = ringK + (pos % NS) * kTile16;
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t kk = (k >> 2) * (16384 >> 4) + (k & 3) * 2, kb = (k >> 2) * kBlkK + (k & 3) * 2;
-          mma_ss_any(tmem + Cfg::kTmemDP, a2Lo + kk, bLo + kb, idesc_s, k > 0);
-        }
-        commit(&bars.dp_ready);
-        return true;
-      };
-      // soft-max warpgroup g packed its CW columns of P into S[CW*g, CW*g + CW/2) and of dS into dP[CW*g, ...)
-      constexpr int KPW = CW / 16;  // 16-deep MMA steps per warpgroup
-      // U is issued in two halves: the k-steps fed by the first half of every warpgroup's columns as soon as
-      // that half of P is there, the rest when the second half arrives (same accumulation chain).
-      auto issue_u_half = [&](uint32_t pos, uint32_t acc, int half, uint32_t pbuf) {
-        const uint32_t st = pos % NS;
-        bool first = half == 0;
-#pragma unroll
-        for (int k = 0; k < kBC / 16; ++k) {
-          if (((k % KPW) >= KPW / 2) != (half == 1)) continue;
-          const uint32_t a = kFreeS ? tmem + Cfg::kTmemP + pbuf * 64 + k * 8
-                                    : tmem + Cfg::kTmemS + (k / KPW) * CW + (k % KPW) * 8;
-          mma_ts_any(tmem + Cfg::kTmemU, a, ringMN + st * kTile16 + k * (2048 >> 4), idesc_g, first ? acc : 1u);
-          first = false;
-        }
-        if (half == 1) commit(&bars.ring_empty[st]);
-      };
-      auto issue_g = [&](uint32_t pos, uint32_t acc) {
-        const uint32_t st = pos % NS;
-#pragma unroll
-        for (int k = 0; k < kBC / 16; ++k) {
-          const uint32_t a = tmem + Cfg::kTmemDP + (k / KPW) * CW + (k % KPW) * 8;
-          mma_ts_any(tmem + Cfg::kTmemG, a, ringMN + st * kTile16 + k * (2048 >> 4), idesc_g, k > 0 ? 1u : acc);
-        }
-        commit(&bars.ring_empty[st]);
-      };
-
-      for (long item = unit; item < n_items && alive; item += n_units) {
-        int role, bh, q, qr, xt0, nxt;
-        decode(item, role, bh, q, qr);
-        const Win win = role_win(role);
-        x_range(qr, win, xt0, nxt);
-        for (int xt = xt0; xt < xt0 + nxt && alive; ++xt, ++xt_count) {
-          int c0, ncs;
-          c_range(qr, win, xt, c0, ncs);
-          // the first score product starts while the soft-max warps still form the dP operand
-          if (!wait_all(&bars.ax_ready, xt_count & 1)) { alive = false; break; }
-          tc_fence_after();
-          if (!issue_s(base)) { alive = false; break; }
-          if (!wait_all(&bars.ay_ready, xt_count & 1)) { alive = false; break; }
-          tc_fence_after();
-          if (!issue_dp(base + 1)) { alive = false; break; }
-          // Once the tile's last S and dP products have run, its operand tiles may be reloaded: the commit lets the
-          // producer fetch the next tile's rows a slab before the soft-max warps are done with this one.
-          if (ncs == 1) commit(&bars.a_free);
-          for (int c = 0; c < ncs && alive; ++c, ++n) {
-            const bool more = c + 1 < ncs;
-            if constexpr (kFreeS) {
-              if (!wait_all(&bars.s_free, n & 1)) { alive = false; break; }
-              tc_fence_after();
-              if (more && !issue_s(base + 2 * (c + 1))) { alive = false; break; }
-            }
-            if (!wait_all(&bars.p_ready[n & 1][0], (n >> 1) & 1)) { alive = false; break; }
-            if (c == 0) {
-              // the fold warpgroup must have drained the previous tile's U
-              if (!wait_all(&bars.u_free, (xt_count & 1) ^ 1)) { alive = false; break; }
-            }
-            tc_fence_after();
-            issue_u_half(base + 2 * c + 1, c > 0, 0, n & 1);
-            if (!wait_all(&bars.p_ready[n & 1][1], (n >> 1) & 1)) { alive = false; break; }
-            tc_fence_after();
-            issue_u_half(base + 2 * c + 1, c > 0, 1, n & 1);
-            if constexpr (!kFreeS) {
-              if (more && !issue_s(base + 2 * (c + 1))) { alive = false; break; }
-            }
-            if (!wait_all(&bars.ds_ready, n & 1)) { alive = false; break; }
-            if (c == 0) {
-              // ... and the previous tile's G
-              if (!wait_all(&bars.g_free, (xt_count & 1) ^ 1)) { alive = false; break; }
-            }
-            tc_fence_after();
-            issue_g(base + 2 * c, c > 0);
-            if (more && !issue_dp(base + 2 * (c + 1) + 1)) { alive = false; break; }
-            if (c + 2 == ncs) commit(&bars.a_free);   // that was the tile's last dP (its last S went before it)
-          }
-          if (alive) commit(&bars.gu_done);
-          base += 2 * ncs;
-        }
-      }
-    }
-  } else if (warp >= 4 && warp < kFoldWarp0) {
-    // ------------------------------------------------------------------ soft-max warpgroups
-    const int wg = (warp - 4) >> 2;            // owns columns [CW*wg, CW*wg + CW) of every slab
-    const int wq = warp & 3;
-    const int row = wq * 32 + lane;
-    const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
-    float* vec = (float*)(smem + Cfg::kOffVec);
-    float* misc = (float*)(smem + Cfg::kOffMisc);
-    uint32_t xt_count = 0, n = 0, sync_phase = 0, item_count = 0;
-    bool alive = true;
-    auto sm_sync = [&]() -> bool {
-      mbar_arrive(&bars.sm_sync);
-      const bool ok = mbar_wait_x<PAIR>(&bars.sm_sync, sync_phase & 1, abort_flag);
-      ++sync_phase;
-      return __all_sync(0xffffffffu, ok);
+    // per operand and loses its issue slots to the busy warps of its scheduler.
+    const bool leader = elect_one();
+    constexpr int kFmt = std::is_same<T16, __nv_bfloat16>::value ? 1 : 0;
+    constexpr uint32_t kHi = desc_hi(1024);
+    constexpr uint32_t idesc_s = make_idesc_f16(128, JT, kFmt, false, false);
+    constexpr uint32_t idesc_g = make_idesc_f16(128, 64, kFmt, true, true);
+    constexpr uint32_t idesc_dq = make_idesc_f16(128, D, kFmt, false, true);
+    // (leading-byte offsets: distance of 64-element blocks along M / N of a row-major tile)
+    const uint32_t qLo = desc_lo(smem_u32(smem + Cfg::kOffQ), 16384), doLo = desc_lo(smem_u32(smem + Cfg::kOffDO), 16384);
+    const uint32_t aLo = desc_lo(smem_u32(smem + Cfg::kOffA), JT * 128);
+    const uint32_t a2Lo = desc_lo(smem_u32(smem + Cfg::kOffA + 2 * Cfg::kTileJ), JT * 128);
+    const uint32_t pLo = desc_lo(smem_u32(smem + Cfg::kOffP), 16384);
+    constexpr uint32_t kTileP16 = Cfg::kTileP >> 4, kTileJ16 = Cfg::kTileJ >> 4;
+    auto commit = [&](uint64_t* bar) {
+      if (leader) mma_commit(bar);
     };
-
-    for (long item = unit; item < n_items && alive; item += n_units, ++item_count) {
-      int role, bh, q, qr, xt0, nxt;
-      decode(item, role, bh, q, qr);
-      const Win win = role_win(role);
-      x_range(qr, win, xt0, nxt);
-      const size_t hb = (size_t)bh * T * D;
-      float* qv = vec + (item_count & 1) * 2 * D;  // Q[q, :] (double-buffered by item: the fold warpgroup of the
-      float* dov = qv + D;                         // dO[q, :]  previous item may still be reading its copy)
-      if (!sm_sync()) { alive = false; break; }    // previous item's readers of misc are done
-      // the fold warpgroup can lag two items behind: wait until it has stopped reading this copy of the vectors
-      alive = __all_sync(0xffffffffu,
-                         mbar_wait_x<PAIR>(&bars.vec_free[item_count & 1], ((item_count >> 1) & 1) ^ 1, abort_flag));
-      if (!alive) break;
-      const float scale2 = p.alpha * kLog2e;
-      if (wg == 0) {
-        float dq_part = 0.f;
-        if (row < D) {
-          const float qf = to_f(((const T16*)p.q)[hb + (size_t)q * D + row]);
-          const float dof = to_f(((const T16*)p.d_o)[hb + (size_t)q * D + row]);
-          qv[row] = qf * scale2;   // (pre-scaled: the score operand is scale2 * Q[q] (.) X)
-          dov[row] = dof;
-          dq_part = dof * to_f(((const T16*)p.o)[hb + (size_t)q * D + row]);
-        }
+    // S = Q A^T and dP = dO A'^T: Q / dO from tensor memory, A / A' K-major, D / 16 instructions
+    auto issue_rows = [&](uint32_t dcol, uint32_t acol, uint32_t lo_b) {
 #pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) dq_part += __shfl_xor_sync(0xffffffffu, dq_part, o);
-        if (lane == 0) misc[wq] = dq_part;
-      }
-      if (!sm_sync()) { alive = false; break; }
-      const float Dq = misc[0] + misc[1] + misc[2] + misc[3];
-      // (minus the fp16 range shift: P below is the probability times 2^e)
-      const float lse2 = p.lse[(size_t)bh * T + q] * kLog2e - (float)prob_shift<T16>(q, p.causal, T, p.k1w, p.k2w);
-      const float2 nlse = make_float2(-lse2, -lse2), ndq = make_float2(-Dq, -Dq);
-
-      for (int xt = xt0; xt < xt0 + nxt && alive; ++xt, ++xt_count) {
-        int c0, ncs;
-        c_range(qr, win, xt, c0, ncs);
-        // ---- operand formation (in place): A = scale2*Q[q] (.) X tile,  A' = dO[q] (.) Y tile
-        alive = __all_sync(0xffffffffu, mbar_wait_x<PAIR>(&bars.xy_full, xt_count & 1, abort_flag));
-        if (!alive) break;
-        // (each warpgroup takes half of the columns; the eight Q / dO values of a 16-byte chunk are the same for all rows)
-#pragma unroll
-        for (int ci = 0; ci < D / 8 / NSW; ++ci) {
-          const int cc = wg * (D / 8 / NSW) + ci;
-          const uint32_t off = (cc >> 3) * 16384 + swz128(row, cc & 7);
-          const uint4 xv = *reinterpret_cast<const uint4*>(smem + Cfg::kOffA + off);
-          const float4 q0 = *reinterpret_cast<const float4*>(qv + cc * 8), q1 = *reinterpret_cast<const float4*>(qv + cc * 8 + 4);
-          const float2 qf[4] = {make_float2(q0.x, q0.y), make_float2(q0.z, q0.w), make_float2(q1.x, q1.y),
-                                make_float2(q1.z, q1.w)};
-          uint32_t wx[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 a2 = __fmul2_rn(unpack2<T16>(wx[e]), qf[e]);
-            wx[e] = pack2<T16>(a2.x, a2.y);
-          }
-          *reinterpret_cast<uint4*>(smem + Cfg::kOffA + off) = make_uint4(wx[0], wx[1], wx[2], wx[3]);
-        }
-        fence_async_smem();
-        to_mma(&bars.ax_ready);
-#pragma unroll
-        for (int ci = 0; ci < D / 8 / NSW; ++ci) {
-          const int cc = wg * (D / 8 / NSW) + ci;
-          const uint32_t off = (cc >> 3) * 16384 + swz128(row, cc & 7);
-          const uint4 yv = *reinterpret_cast<const uint4*>(smem + Cfg::kOffA2 + off);
-          const float4 d0 = *reinterpret_cast<const float4*>(dov + cc * 8), d1 = *reinterpret_cast<const float4*>(dov + cc * 8 + 4);
-          const float2 df[4] = {make_float2(d0.x, d0.y), make_float2(d0.z, d0.w), make_float2(d1.x, d1.y),
-                                make_float2(d1.z, d1.w)};
-          uint32_t wy[4] = {yv.x, yv.y, yv.z, yv.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 a2 = __fmul2_rn(unpack2<T16>(wy[e]), df[e]);
-            wy[e] = pack2<T16>(a2.x, a2.y);
-          }
-          *reinterpret_cast<uint4*>(smem + Cfg::kOffA2 + off) = make_uint4(wy[0], wy[1], wy[2], wy[3]);
-        }
-        fence_async_smem();
-        to_mma(&bars.ay_ready);
-
-        // columns this row sees: [c_lo, c_hi] (empty for a row outside its own range: its P is zero)
-        const int x_r = xt * 128 + row;
-        int c_lo = 0, c_hi = x_r < T ? T - 1 : -1;
-        if (p.causal) {
-          const bool row_valid = x_r <= q && q - x_r <= win.xw;
-          c_lo = max(q - win.cw, x_r - win.below);
-          c_hi = row_valid ? min(q, x_r + win.above) : c_lo - 1;
-        }
-        const uint32_t tS = tmem + lane_base + Cfg::kTmemS + wg * CW;
-        const uint32_t tDP = tmem + lane_base + Cfg::kTmemDP + wg * CW;
-
-        for (int c = 0; c < ncs; ++c, ++n) {
-          const int lo = c_lo - (c0 + c) * kBC - wg * CW, hi = c_hi - (c0 + c) * kBC - wg * CW;
-          uint32_t pk[CW / 2];
-          // ---- S -> P
-          alive = __all_sync(0xffffffffu, mbar_wait_x<PAIR>(&bars.s_ready, n & 1, abort_flag));
-          if (!alive) break;
-          tc_fence_after();
-          static_assert(CW == 64, "the two-half hand-off of P is written for two soft-max warpgroups");
-          // (the read of the second half is in flight while the first half is worked on)
-          uint32_t sh[2][32];
-          tmem_ld32(tS, sh[0]);
-          tmem_wait_ld();
-          tmem_ld32(tS + 32, sh[1]);
-#pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {
-            if (hf == 1) {
-              tmem_wait_ld();
-              if constexpr (kFreeS) {
-                // both halves of the scores are in registers: the next slab's product may overwrite them
-                tc_fence_before();
-                to_mma(&bars.s_free);
-              }
-            }
-            const uint32_t(&s)[32] = sh[hf];
-            const int l2 = lo - hf * 32, h2 = hi - hf * 32;
-            if (l2 <= 0 && h2 >= 31) {
-              // (packed fp32 pairs: one subtraction per two scores)
-#pragma unroll
-              for (int i = 0; i < 32; i += 2) {
-                const float2 x = __fadd2_rn(make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), nlse);
-                pk[hf * 16 + (i >> 1)] = pack2<T16>(exp2f(x.x), exp2f(x.y));
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; i += 2) {
-                const float p0 = (i >= l2 && i <= h2) ? exp2f(__uint_as_float(s[i]) - lse2) : 0.f;
-                const float p1 = (i + 1 >= l2 && i + 1 <= h2) ? exp2f(__uint_as_float(s[i + 1]) - lse2) : 0.f;
-                pk[hf * 16 + (i >> 1)] = pack2<T16>(p0, p1);
-              }
-            }
-            // P half -> S columns this thread has already read; hand it to the MMA warp right away
-            tmem_st16(kFreeS ? tmem + lane_base + Cfg::kTmemP + (n & 1) * 64 + wg * 32 + hf * 16 : tS + hf * 16,
-                      *reinterpret_cast<uint32_t(*)[16]>(&pk[hf * 16]));
-            tmem_wait_st();
-            tc_fence_before();
-            to_mma(&bars.p_ready[n & 1][hf]);
-          }
-          // ---- dP, P -> dS
-          alive = __all_sync(0xffffffffu, mbar_wait_x<PAIR>(&bars.dp_ready, n & 1, abort_flag));
-          if (!alive) break;
-          tc_fence_after();
-          uint32_t dk[CW / 2];
-          {
-            uint32_t dp[CW];
-#pragma unroll
-            for (int sc = 0; sc < CW / 32; ++sc) tmem_ld32(tDP + sc * 32, *reinterpret_cast<uint32_t(*)[32]>(&dp[sc * 32]));
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < CW; i += 2) {
-              const float2 d = __fadd2_rn(make_float2(__uint_as_float(dp[i]), __uint_as_float(dp[i + 1])), ndq);
-              const float2 ds = __fmul2_rn(unpack2<T16>(pk[i >> 1]), d);
-              dk[i >> 1] = pack2<T16>(ds.x, ds.y);
-            }
-          }
-          tmem_st(tDP, dk);  // dS -> first half of this warpgroup's dP columns
-          tmem_wait_st();
-          tc_fence_before();
-          to_mma(&bars.ds_ready);
-        }
-        if (!alive) break;
-      }
-    }
-  } else if (warp >= kFoldWarp0) {
-    // ------------------------------------------------------------------ fold warpgroup
-    // Drains G / U of a finished tile: 32-column pieces -> registers -> scaled by Q[q] / dO[q] -> shared memory
-    // (128-byte swizzle) -> TMA reduce-add into the fp32 accumulators; for role 0 also dQ[q] += sum_r G X.
-    const int wq = warp & 3;
-    const int row = wq * 32 + lane;
-    const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
-    uint8_t* slots = smem + Cfg::kOffStage + wq * 8192;  // two 4 KiB slots of this warp
-    float* dq_acc = (float*)(smem + Cfg::kOffDq);
-    float* vec = (float*)(smem + Cfg::kOffVec);
-    uint32_t xt_count = 0, sync_phase = 0, item_count = 0, round = 0;
-    bool alive = true;
-    auto fold_sync = [&]() -> bool {
-      mbar_arrive(&bars.fold_sync);
-      const bool ok = mbar_wait_x<PAIR>(&bars.fold_sync, sync_phase & 1, abort_flag);
-      ++sync_phase;
-      return __all_sync(0xffffffffu, ok);
+      for (int k = 0; k < D / 16; ++k)
+        if (leader)
+          mma_ts_lo(tmem + dcol, tmem + acol + k * 8, lo_b + (k >> 2) * ((JT * 128) >> 4) + (k & 3) * 2, kHi, idesc_s, k > 0);
     };
-    for (long item = unit; item < n_items && alive; item += n_units, ++item_count) {
-      int role, bh, q, qr, xt0, nxt;
-      decode(item, role, bh, q, qr);
-      const Win win = role_win(role);
-      x_range(qr, win, xt0, nxt);
-      const size_t hb = (size_t)bh * T * D;
-      const T16* Xg = (const T16*)p.x[role] + hb;
-      const CUtensorMap* tmDX = role == 0 ? &tmDK2 : &tmDK1;
-      const CUtensorMap* tmDY = role == 0 ? &tmDV2 : &tmDSV1;
-      const float* qv = vec + (item_count & 1) * 2 * D;
-      const float* dov = qv + D;
-      // A query that attends a single pair has P = 1 and a score gradient of exactly zero (TdpMask::single_pair):
-      // what G holds for it is P (dP - Dq) with the two terms equal only up to the 16-bit rounding of the stored
-      // output, so G is dropped (dQ = 0, nothing added to dK1 / dK2) instead of being folded.
-      const bool single = TdpMask{p.causal, T, p.k1w, p.k2w, p.kkl, p.kkr}.single_pair(q);
-      // undoes the fp16 range shift of P and dS (1 for bf16)
-      const float unshift = exp2f(-(float)prob_shift<T16>(q, p.causal, T, p.k1w, p.k2w));
-      const float alpha_u = p.alpha * unshift;
-      if (role == 0) {
-        if (row < D) dq_acc[row] = 0.f;
-        if (!fold_sync()) { alive = false; break; }
-      }
-      for (int xt = xt0; xt < xt0 + nxt && alive; ++xt, ++xt_count) {
-        const int x_r = xt * 128 + row;
-        const bool x_ok = (p.causal ? (x_r <= q && q - x_r <= win.xw) : true) && x_r < T;
-        // (rows outside the query's range carry zeros: a warp whose 32 rows all are has nothing to add)
-        const bool warp_rows_live = __any_sync(0xffffffffu, x_ok);
-        alive = __all_sync(0xffffffffu, mbar_wait_x<PAIR>(&bars.gu_done, xt_count & 1, abort_flag));
+    // G = dS^T Q, U = P^T dO (head dimension 128: the transposes): contraction over the 128 queries, both row-major
+    auto issue_fold = [&](uint32_t dcol, uint32_t lo_p, uint32_t lo_q) {
+      const uint32_t lo_a = D == 64 ? lo_p : lo_q, lo_b = D == 64 ? lo_q : lo_p;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (leader) mma_ss_lo(tmem + dcol, lo_a + k * (2048 >> 4), lo_b + k * (2048 >> 4), kHi, idesc_g, k > 0);
+    };
+    // dQ += dS A: contraction over the JT rows j
+    auto issue_dq = [&](uint32_t lo_ds, uint32_t lo_a, uint32_t acc) {
+#pragma unroll
+      for (int k = 0; k < JT / 16; ++k)
+        if (leader)
+          mma_ss_lo(tmem + Cfg::kTmemDQ, lo_ds + (k >> 2) * (16384 >> 4) + (k & 3) * 2, lo_a + k * (2048 >> 4), kHi, idesc_dq,
+                    k > 0 ? 1u : acc);
+    };
+    uint32_t n = 0, items = 0, runs = 0;
+    bool alive = true;
+    auto issue_s = [&](uint32_t m) -> bool {
+      if (!wait_all(&bars.a_ready[m & 1], (m >> 1) & 1)) return false;
+      if (!wait_all(&bars.s_free, (m & 1) ^ 1)) return false;
+      tc_fence_after();
+      issue_rows(Cfg::kTmemS, Cfg::kTmemQ, aLo + (m & 1) * kTileJ16);
+      commit(&bars.s_ready);
+      return true;
+    };
+    // (the previous step's dP has been read: its ds_ready was waited for)
+    auto issue_dp = [&](uint32_t m) -> bool {
+      if (!wait_all(&bars.ap_ready, m & 1)) return false;
+      tc_fence_after();
+      issue_rows(Cfg::kTmemDP, Cfg::kTmemDO, a2Lo);
+      commit(&bars.dp_ready);
+      return true;
+    };
+    BwdItem it;
+    while (alive && next_item(items, it, alive)) {
+      if (it.flags & kFirstOfQ) {
+        alive = wait_all(&bars.qdo_ready, runs & 1);   // (runs: q-tiles finished)
         if (!alive) break;
+      }
+      alive = issue_s(n) && issue_dp(n);
+      for (int i = 0; i < it.len && alive; ++i, ++n) {
+        const bool more = i + 1 < it.len;
+        alive = false;
+        if (more && !issue_s(n + 1)) break;
+        if (!wait_all(&bars.p_ready, n & 1) || !wait_all(&bars.acc_free[1], (n & 1) ^ 1)) break;
         tc_fence_after();
-#pragma unroll 1
-        for (int pc = 0; pc < 2 * (D / 32); ++pc, ++round) {
-          const bool is_u = pc < D / 32;   // U first: the next tile needs its accumulator earlier than G's
-          const int h0 = (is_u ? pc : pc - D / 32) * 32;
-          // role 0, G pieces: this row's X values for the dQ product (issued early to hide the latency)
-          uint4 xr[4];
-          const bool want_dq = !is_u && role == 0 && !single;
-          if (want_dq) {
-#pragma unroll
-            for (int i4 = 0; i4 < 4; ++i4)
-              xr[i4] = x_ok ? __ldg(reinterpret_cast<const uint4*>(Xg + (size_t)x_r * D + h0 + i4 * 8))
-                            : make_uint4(0, 0, 0, 0);
-          }
-          uint32_t g[32];
-          tmem_ld32(tmem + lane_base + (is_u ? Cfg::kTmemU : Cfg::kTmemG) + h0, g);
-          tmem_wait_ld();
-          // scale by Q[q] / dO[q] right away: after the hand-off below the soft-max warps may move on to a
-          // later query and overwrite an older copy of these vectors
-          float v[32];
-          {
-            const float4* mul = reinterpret_cast<const float4*>((is_u ? dov : qv) + h0);
-            // (the Q copy carries the factor alpha * log2(e) of the score operand)
-            const float sc = is_u ? unshift : unshift * (1.f / kLog2e);
-            const float2 sc2 = make_float2(sc, sc);
-#pragma unroll
-            for (int i4 = 0; i4 < 8; ++i4) {
-              const float4 m = mul[i4];
-              const float2 lo = __fmul2_rn(__fmul2_rn(make_float2(__uint_as_float(g[i4 * 4]), __uint_as_float(g[i4 * 4 + 1])), sc2),
-                                           make_float2(m.x, m.y));
-              const float2 hi = __fmul2_rn(__fmul2_rn(make_float2(__uint_as_float(g[i4 * 4 + 2]), __uint_as_float(g[i4 * 4 + 3])), sc2),
-                                           make_float2(m.z, m.w));
-              v[i4 * 4] = lo.x;
-              v[i4 * 4 + 1] = lo.y;
-              v[i4 * 4 + 2] = hi.x;
-              v[i4 * 4 + 3] = hi.y;
-            }
-          }
-          if (pc == D / 32 - 1) {
-            // last piece of U is in registers: that accumulator may be overwritten
-            tc_fence_before();
-            to_mma(&bars.u_free);
-          }
-          if (pc == 2 * (D / 32) - 1) {
-            // likewise G
-            tc_fence_before();
-            to_mma(&bars.g_free);
-            if (xt == xt0 + nxt - 1) mbar_arrive(&bars.vec_free[item_count & 1]);  // and this query's vectors are done with
-          }
-          uint8_t* slot = slots + (round & 1) * 4096;
-          // the reduce-add issued two rounds ago from this slot must have finished reading it
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-          __syncwarp();
-#pragma unroll
-          for (int i4 = 0; i4 < 8; ++i4)
-            *reinterpret_cast<float4*>(slot + swz128(lane, i4)) =
-                make_float4(v[i4 * 4], v[i4 * 4 + 1], v[i4 * 4 + 2], v[i4 * 4 + 3]);
-          fence_async_smem();
-          __syncwarp();
-          // (rows beyond the query carry zeros: a warp whose 32 rows are all beyond it has nothing to add)
-          if (lane == 0 && warp_rows_live && (is_u || !single)) {
-            tma_reduce_add_3d(is_u ? tmDY : tmDX, slot, h0, xt * 128 + wq * 32, bh);
-            bulk_commit();
-          }
-          if (want_dq) {
-#pragma unroll
-            for (int i4 = 0; i4 < 4; ++i4) {
-              const uint32_t wx[4] = {xr[i4].x, xr[i4].y, xr[i4].z, xr[i4].w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float2 gx = __fmul2_rn(__fmul2_rn(make_float2(__uint_as_float(g[i4 * 8 + 2 * e]),
-                                                                    __uint_as_float(g[i4 * 8 + 2 * e + 1])),
-                                                        make_float2(alpha_u, alpha_u)),
-                                             unpack2<T16>(wx[e]));
-                v[i4 * 8 + 2 * e] = gx.x;
-                v[i4 * 8 + 2 * e + 1] = gx.y;
-              }
-            }
-            const float colsum = warp_transpose_sum(v, lane);
-            atomicAdd(&dq_acc[h0 + lane], colsum);
-          }
+        issue_fold(Cfg::kTmemU, pLo, doLo);
+        commit(&bars.acc_done[1]);
+        if (!wait_all(&bars.ds_ready, n & 1)) break;
+        tc_fence_after();
+        if (more && !issue_dp(n + 1)) break;
+        const bool fresh = i == 0 && (it.flags & kFirstOfQ);
+        if (fresh) {
+          // the previous q-tile's dQ has been read
+          if (!wait_all(&bars.dq_free, (runs & 1) ^ 1)) break;
+          tc_fence_after();
         }
+        const uint32_t ds = pLo + (1 + (n & 1)) * kTileP16;
+        issue_dq(ds, aLo + (n & 1) * kTileJ16, fresh ? 0u : 1u);
+        commit(&bars.a_free[n & 1]);
+        if (!wait_all(&bars.acc_free[0], (n & 1) ^ 1)) break;
+        tc_fence_after();
+        issue_fold(Cfg::kTmemG, ds, qLo);
+        commit(&bars.acc_done[0]);
+        commit(&bars.ds_free[n & 1]);
+        alive = true;
       }
       if (!alive) break;
-      if (role == 0) {
-        if (!fold_sync()) { alive = false; break; }  // every warp's contribution to dq_acc has landed
-        if (row < D) ((T16*)p.dq)[hb + (size_t)q * D + row] = from_f<T16>(dq_acc[row]);
-        if (!fold_sync()) { alive = false; break; }  // dq_acc may be cleared for the next item
+      commit(&bars.tile_free);
+      ++items;
+      if ((it.flags & kLastOfQ)) {
+        commit(&bars.dq_done);
+        ++runs;
       }
     }
-    bulk_wait_all();  // reduce-adds still in flight must complete before the CTA retires
+   } else if (warp == 17) {
+    // ------------------------------------------------------------------ loader
+    const bool leader = elect_one();
+    if (leader) {
+      tma_prefetch_desc(&tmQ);
+      tma_prefetch_desc(&tmDO);
+      tma_prefetch_desc(&tmK1);
+      tma_prefetch_desc(&tmSV1);
+    }
+    const float scale2 = p.alpha * kLog2e;
+    constexpr int kChunks = kVecBatch * D / 8 / 32;   // 16-byte pieces of K2 (and of V2) per lane and batch
+    float* const vec = reinterpret_cast<float*>(smem + Cfg::kOffVec);
+    uint32_t items = 0, vb = 0;
+    bool alive = true, in_flight = false;
+    BwdWalk walk(p);
+    BwdItem it{-1, -1, 0, 0, 0, 0, {0, 0}};
+    while (alive) {
+      it = walk.next(it);
+      alive = wait_all(&bars.tile_free, (items & 1) ^ 1);
+      if (!alive) break;
+      if (leader) bars.items[items % kItemSlots] = it;
+      if (it.len == 0) {
+        if (leader) mbar_arrive(&bars.tile_full);
+        break;
+      }
+      if (leader) {
+        mbar_arrive_expect_tx(&bars.tile_full, ((it.flags & kFirstOfQ) ? 2 * Cfg::kTileQ : 0) + 2 * Cfg::kTileJ);
+#pragma unroll
+        for (int b = 0; b < D / 64; ++b) {
+          if ((it.flags & kFirstOfQ)) {
+            tma_load_3d(smem + Cfg::kOffQ + b * 16384, &tmQ, &bars.tile_full, b * 64, it.qt * 128, it.bh);
+            tma_load_3d(smem + Cfg::kOffDO + b * 16384, &tmDO, &bars.tile_full, b * 64, it.qt * 128, it.bh);
+          }
+          tma_load_3d(smem + Cfg::kOffK1 + b * JT * 128, &tmK1, &bars.tile_full, b * 64, it.jt * JT, it.bh);
+          tma_load_3d(smem + Cfg::kOffK1 + Cfg::kTileJ + b * JT * 128, &tmSV1, &bars.tile_full, b * 64, it.jt * JT, it.bh);
+        }
+      }
+      in_flight = true;
+      ++items;
+      // K2 / V2 rows, fp32 (K2 times alpha * log2(e)), a batch of rows at a time; rows past the item repeat its last
+      const size_t head = (size_t)it.bh * T * D;
+      for (int i = 0; i < it.len; i += kVecBatch, ++vb) {
+        uint4 x[2][kChunks];
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) {
+          const int at = c * 32 + lane, r = at / (D / 8), col = at % (D / 8) * 8;
+          const size_t off = head + (size_t)(it.k0 + min(i + r, it.len - 1)) * D + col;
+          x[0][c] = __ldg(reinterpret_cast<const uint4*>((const T16*)p.k2 + off));
+          x[1][c] = __ldg(reinterpret_cast<const uint4*>((const T16*)p.v2 + off));
+        }
+        alive = wait_all(&bars.vec_empty[vb % kVecSlots], ((vb / kVecSlots) & 1) ^ 1);
+        if (!alive) break;
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) {
+          const int at = c * 32 + lane, r = at / (D / 8), col = at % (D / 8) * 8;
+          float* dst = vec + ((vb % kVecSlots) * kVecBatch + r) * Cfg::kVecRow + col;
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            const float sc = m == 0 ? scale2 : 1.f;
+            const uint4 y = x[m][c];
+            const float2 f0 = unpack2<T16>(y.x), f1 = unpack2<T16>(y.y), f2 = unpack2<T16>(y.z), f3 = unpack2<T16>(y.w);
+            *reinterpret_cast<float4*>(dst + m * D) = make_float4(f0.x * sc, f0.y * sc, f1.x * sc, f1.y * sc);
+            *reinterpret_cast<float4*>(dst + m * D + 4) = make_float4(f2.x * sc, f2.y * sc, f3.x * sc, f3.y * sc);
+          }
+        }
+        mbar_arrive(&bars.vec_full[vb % kVecSlots]);
+      }
+    }
+    if (!alive && in_flight) {
+      // give copies still in flight a bounded chance to land before the CTA retires
+      const long long t0 = clock64();
+      while (!mbar_try_wait(&bars.tile_full, (items - 1) & 1) && clock64() - t0 < kWaitTicks / 8) {
+      }
+    }
+   }
   }
 
   // ------------------------------------------------------------------ teardown
   tc_fence_before();
   __syncthreads();
-  if constexpr (PAIR) cluster_sync_all();  // neither CTA frees tensor memory or leaves while the other may still use it
-  if (warp == 0) {
-    if constexpr (PAIR) tmem_dealloc_pair(tmem, 512); else tmem_dealloc(tmem, 512);
-  }
+  if (warp == 16) tmem_dealloc(tmem, 512);
   if (tid == 0 && bars.abort_flag && p.status) atomicOr(p.status, 4);
 }
 
-template <int D, typename T16, int NSW>
-int launch_bwd(const TdpArgs& a) {
+// What the kernel needs before it starts, in one pass over the tensors (8 elements per thread): zeroed fp32 sums,
+// SiLU(V1) in the inputs' type and Dq = sum_h dO O per query.
+template <typename T16>
+__global__ void tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, const T16* __restrict__ d_o,
+                                       float* __restrict__ sums, T16* __restrict__ sv1, float* __restrict__ drow, size_t n,
+                                       int D) {
+  const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;   // (n is a multiple of 64)
+  const bool in = i < n;
+  float dot = 0.f;
+  if (in) {
+#pragma unroll
+    for (int s = 0; s < 5; ++s) {
+      *reinterpret_cast<float4*>(sums + s * n + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(sums + s * n + i + 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const uint4 v = *reinterpret_cast<const uint4*>(v1 + i), a = *reinterpret_cast<const uint4*>(o + i),
+                b = *reinterpret_cast<const uint4*>(d_o + i);
+    const uint32_t wv[4] = {v.x, v.y, v.z, v.w}, wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
+    uint32_t r[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = unpack2<T16>(wv[e]), x = unpack2<T16>(wa[e]), y = unpack2<T16>(wb[e]);
+      r[e] = pack2<T16>(silu_f(f.x), silu_f(f.y));
+      dot = fmaf(x.x, y.x, fmaf(x.y, y.y, dot));
+    }
+    *reinterpret_cast<uint4*>(sv1 + i) = make_uint4(r[0], r[1], r[2], r[3]);
+  }
+  const int lanes = D / 8;   // 8 or 16 lanes hold one row
+  for (int s = lanes / 2; s >= 1; s >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, s);
+  if (in && (threadIdx.x & (lanes - 1)) == 0) drow[i / D] = dot;
+}
+
+// The fp32 sums -> gradients in the inputs' type, SiLU'(V1) applied to dV1 (reference flash_trittention.py:390-391), 8
+// elements per thread.  dq_only: just the query rows q_rem + i * q_mod of dQ (a query-sharded call).
+template <typename T16>
+__global__ void tdp_bwd_finish_kernel(const float* __restrict__ sums, const T16* __restrict__ v1, T16* __restrict__ dq,
+                                      T16* __restrict__ dk1, T16* __restrict__ dk2, T16* __restrict__ dv1,
+                                      T16* __restrict__ dv2, size_t n, int T, int D, int q_mod, int q_rem, bool dq_only) {
+  const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (i >= n) return;
+  auto put = [&](const float* src, T16* dst, const float (*mul)) {
+    const float4 a = *reinterpret_cast<const float4*>(src + i), b = *reinterpret_cast<const float4*>(src + i + 4);
+    float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    if (mul) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] *= mul[e];
+    }
+    *reinterpret_cast<uint4*>(dst + i) =
+        make_uint4(pack2<T16>(f[0], f[1]), pack2<T16>(f[2], f[3]), pack2<T16>(f[4], f[5]), pack2<T16>(f[6], f[7]));
+  };
+  if ((int)((i / D) % T) % q_mod == q_rem) put(sums + 4 * n, dq, nullptr);
+  if (dq_only) return;
+  put(sums, dk1, nullptr);
+  put(sums + n, dk2, nullptr);
+  const uint4 v = *reinterpret_cast<const uint4*>(v1 + i);
+  const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
+  float g[8];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 f = unpack2<T16>(wv[e]);
+    g[2 * e] = silu_grad_f(f.x);
+    g[2 * e + 1] = silu_grad_f(f.y);
+  }
+  put(sums + 2 * n, dv1, g);
+  put(sums + 3 * n, dv2, nullptr);
+}
+
+// workspace: fp32 sums dK1 | dK2 | dSiLU(V1) | dV2 | dQ, SiLU(V1) in the inputs' type, Dq fp32
+template <int D, typename T16>
+int launch_bwd_sums(const TdpArgs& a) {
   using Cfg = BwdCfg<D>;
   const int BN = a.B * a.N;
   const size_t n = (size_t)BN * a.T * a.D;
-  float* part = (float*)a.workspace;          // dK1 | dK2 | dSiLU(V1) | dV2
-  T16* sv1 = (T16*)(part + 4 * n);
-  TRITT_CUDA_OK(cudaMemsetAsync(part, 0, 4 * n * sizeof(float), a.stream));
-  silu_kernel<T16><<<(unsigned)((n / 8 + 255) / 256 + 1), 256, 0, a.stream>>>((const T16*)a.v1, sv1, n);
+  float* sums = (float*)a.workspace;
+  T16* sv1 = (T16*)(sums + 5 * n);
+  float* drow = (float*)(sv1 + n);
+  tdp_bwd_prepare_kernel<T16><<<(unsigned)((n / 8 + 255) / 256), 256, 0, a.stream>>>(
+      (const T16*)a.v1, (const T16*)a.o, (const T16*)a.d_o, sums, sv1, drow, n, D);
   count_launch();
   TRITT_CUDA_OK(cudaGetLastError());
-  CUtensorMap tmK1, tmK2, tmSV1, tmV2, tmDK1, tmDK2, tmDSV1, tmDV2;
-  int rc;
-  if ((rc = make_tmap_3d(&tmK1, a.k1, 2, D, a.T, BN, 64, 128))) return rc;
-  if ((rc = make_tmap_3d(&tmK2, a.k2, 2, D, a.T, BN, 64, 128))) return rc;
-  if ((rc = make_tmap_3d(&tmSV1, sv1, 2, D, a.T, BN, 64, 128))) return rc;
-  if ((rc = make_tmap_3d(&tmV2, a.v2, 2, D, a.T, BN, 64, 128))) return rc;
-  if ((rc = make_tmap_3d_f32(&tmDK1, part, D, a.T, BN, 32, 32))) return rc;
-  if ((rc = make_tmap_3d_f32(&tmDK2, part + n, D, a.T, BN, 32, 32))) return rc;
-  if ((rc = make_tmap_3d_f32(&tmDSV1, part + 2 * n, D, a.T, BN, 32, 32))) return rc;
-  if ((rc = make_tmap_3d_f32(&tmDV2, part + 3 * n, D, a.T, BN, 32, 32))) return rc;
   BwdParams p{};
-  p.q = a.q; p.o = a.o; p.d_o = a.d_o; p.lse = a.lse_in; p.dq = a.dq;
-  p.x[0] = a.k2; p.x[1] = a.k1;
-  p.T = a.T; p.BN = BN; p.q_mod = a.q_mod; p.q_rem = a.q_rem;
-  p.nq = a.q_rem < a.T ? (a.T - a.q_rem + a.q_mod - 1) / a.q_mod : 0;
-  p.causal = a.mask.causal;
-  p.k1w = a.mask.k1w;
-  p.k2w = a.mask.k2w;
-  p.kkl = a.mask.kkl;
-  p.kkr = a.mask.kkr;
+  p.q = a.q; p.d_o = a.d_o; p.k2 = a.k2; p.v2 = a.v2; p.lse = a.lse_in; p.drow = drow;
+  p.dk1 = sums; p.dk2 = sums + n; p.dsv1 = sums + 2 * n; p.dv2 = sums + 3 * n; p.dq = sums + 4 * n;
+  p.BN = BN;
   p.alpha = a.alpha;
+  // The gradients of the first queries are the largest by far (a query attends ~q^2 pairs: its dQ falls like 1/q, and so
+  // does what it adds to the first key rows), so on a long sequence their rounding to bf16 operands is most of the error
+  // of the whole result.  They are a vanishing part of the work: exact fp32 on the CUDA cores (~10 us beside > 1 ms).
+  // Short sequences have no such spread, and fp16 operands are eight times finer.
+  constexpr int kFirstQueries = 32, kFirstQueriesFromT = 1024;
+  if (std::is_same<T16, __nv_bfloat16>::value && a.mask.causal && a.T >= kFirstQueriesFromT) {
+    p.i_first = kFirstQueries;
+    const int rc = simt_tdp_bwd_first_queries(a, kFirstQueries, sums);
+    if (rc) return rc;
+  }
   p.status = a.status_word;
-  BwdHalfMaps half{};
-  // CTA pairs (on request: TRITT_FLAG_BWD_CTA_PAIRS): head dimension 128, an even number of queries, and a mask
-  // whose tile ranges are the same for two neighbouring queries (no windows); everything else runs one CTA per item.
-  const TdpMask& m = a.mask;
-  bool pair = (a.flags & TRITT_FLAG_BWD_CTA_PAIRS) && D == 128 && p.nq >= 2 && p.nq % 2 == 0 &&
-              (!m.causal || (m.k1w >= a.T && m.k2w >= a.T && m.kkl >= a.T && m.kkr >= a.T));
-  if (p.nq > 0 && pair) {
-    if constexpr (D == 128) {
-      auto kern = tdp_bwd_kernel<D, T16, NSW, true>;
-      TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
-      cudaLaunchConfig_t cfg{};
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 2;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.gridDim = dim3(2, 1, 1);
-      cfg.blockDim = dim3(BwdThreads<NSW>::kTotal, 1, 1);
-      cfg.dynamicSmemBytes = Cfg::kSmem;
-      cfg.stream = a.stream;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      int clusters = 0;
-      if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1) {
-        (void)cudaGetLastError();
-        pair = false;   // no room for a pair on this device: one CTA per item
-      } else {
-        if ((rc = make_tmap_3d(&half.k1, a.k1, 2, D, a.T, BN, 64, 64))) return rc;
-        if ((rc = make_tmap_3d(&half.k2, a.k2, 2, D, a.T, BN, 64, 64))) return rc;
-        if ((rc = make_tmap_3d(&half.sv1, sv1, 2, D, a.T, BN, 64, 64))) return rc;
-        if ((rc = make_tmap_3d(&half.v2, a.v2, 2, D, a.T, BN, 64, 64))) return rc;
-        const long items = (long)(p.nq / 2) * BN * 2;
-        cfg.gridDim = dim3((unsigned)(2 * (items < clusters ? items : clusters)), 1, 1);
-        TRITT_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tmK1, tmK2, tmSV1, tmV2, tmDK1, tmDK2, tmDSV1, tmDV2, half, p));
-        count_launch();
-      }
+  const int nq = a.q_rem < a.T ? (a.T - a.q_rem + a.q_mod - 1) / a.q_mod : 0;
+  if (nq == 0) return 0;
+  p.g = BwdGeometry{a.T, nq, a.q_mod, a.q_rem, a.mask.causal, a.mask.k1w, a.mask.k2w, a.mask.kkl, a.mask.kkr, Cfg::JT};
+  for (int qt = 0; qt < p.g.q_tiles(); ++qt)
+    for (int jt = p.g.j_first(qt); jt <= p.g.j_last(qt); ++jt) {
+      int k0;
+      p.head_steps += p.g.k_range(qt, jt, k0);
     }
+  if (p.head_steps == 0) return 0;
+  // Cut: equal parts of the whole line of steps; where a part is short (under kShortPart steps) the loads and
+  // reductions of a second, third item weigh more than a few idle SMs, so each head is cut by itself.
+  constexpr long kShortPart = 64;
+  const long total = p.head_steps * BN, sms = num_sms();
+  int grid = (int)(total < sms ? total : sms);
+  if (total < sms * kShortPart && BN <= sms) {
+    const long parts = sms / BN;
+    p.parts = (int)(parts < p.head_steps ? parts : p.head_steps);
+    grid = p.parts * BN;
   }
-  if (p.nq > 0 && !pair) {
-    auto kern = tdp_bwd_kernel<D, T16, NSW, false>;
-    TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
-    const long items = (long)p.nq * BN * 2;
-    const int grid = (int)(items < num_sms() ? items : num_sms());
-    kern<<<grid, BwdThreads<NSW>::kTotal, Cfg::kSmem, a.stream>>>(tmK1, tmK2, tmSV1, tmV2, tmDK1, tmDK2, tmDSV1, tmDV2, half, p);
-    count_launch();
-    TRITT_CUDA_OK(cudaGetLastError());
-  }
-  if (a.flags & TRITT_FLAG_BWD_PARTIAL) return 0;
-  return simt_tdp_bwd_finalize(a.v1, a.dk1, a.dk2, a.dv1, a.dv2, n, a.dtype, part, a.stream);
+  CUtensorMap tmQ, tmDO, tmK1, tmSV1;
+  int rc;
+  const size_t shard = (size_t)a.q_rem * D;   // first query row of the shard
+  if ((rc = make_tmap_rows(&tmQ, (const T16*)a.q + shard, D, nq, BN, (uint64_t)a.q_mod * D, (uint64_t)a.T * D, 128))) return rc;
+  if ((rc = make_tmap_rows(&tmDO, (const T16*)a.d_o + shard, D, nq, BN, (uint64_t)a.q_mod * D, (uint64_t)a.T * D, 128))) return rc;
+  if ((rc = make_tmap_3d(&tmK1, a.k1, 2, D, a.T, BN, 64, Cfg::JT))) return rc;
+  if ((rc = make_tmap_3d(&tmSV1, sv1, 2, D, a.T, BN, 64, Cfg::JT))) return rc;
+  auto kern = tdp_bwd_kernel<D, T16>;
+  TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
+  kern<<<grid, kBwdThreads, Cfg::kSmem, a.stream>>>(tmQ, tmDO, tmK1, tmSV1, p);
+  count_launch();
+  TRITT_CUDA_OK(cudaGetLastError());
+  return 0;
 }
 
-template <int D, typename T16>
-int launch_bwd_any(const TdpArgs& a) {
-  return launch_bwd<D, T16, 2>(a);
+template <typename T16>
+int launch_finish(const TdpArgs& a) {
+  const size_t n = (size_t)a.B * a.N * a.T * a.D;
+  tdp_bwd_finish_kernel<T16><<<(unsigned)((n / 8 + 255) / 256), 256, 0, a.stream>>>(
+      (const float*)a.workspace, (const T16*)a.v1, (T16*)a.dq, (T16*)a.dk1, (T16*)a.dk2, (T16*)a.dv1, (T16*)a.dv2, n, a.T,
+      a.D, a.q_mod, a.q_rem, (a.flags & TRITT_FLAG_BWD_PARTIAL) != 0);
+  count_launch();
+  TRITT_CUDA_OK(cudaGetLastError());
+  return 0;
 }
 
 }  // namespace
 
-
 size_t sm100_tdp_bwd_workspace(int B, int N, int T, int D) {
-  const size_t n = (size_t)B * N * T * D;
-  return 4 * n * sizeof(float) + n * 2;
+  const size_t r = (size_t)B * N * T, n = r * D;
+  return 5 * n * sizeof(float) + n * 2 + r * sizeof(float);
+}
+
+int sm100_tdp_bwd_sums(const TdpArgs& a) {
+  if (a.dtype == TRITT_BF16)
+    return a.D == 128 ? launch_bwd_sums<128, __nv_bfloat16>(a) : launch_bwd_sums<64, __nv_bfloat16>(a);
+  return a.D == 128 ? launch_bwd_sums<128, __half>(a) : launch_bwd_sums<64, __half>(a);
 }
 
 int sm100_tdp_bwd(const TdpArgs& a) {
-  if (a.dtype == TRITT_BF16)
-    return a.D == 128 ? launch_bwd_any<128, __nv_bfloat16>(a) : launch_bwd_any<64, __nv_bfloat16>(a);
-  return a.D == 128 ? launch_bwd_any<128, __half>(a) : launch_bwd_any<64, __half>(a);
+  const int rc = sm100_tdp_bwd_sums(a);
+  if (rc) return rc;
+  return a.dtype == TRITT_BF16 ? launch_finish<__nv_bfloat16>(a) : launch_finish<__half>(a);
 }
 
 }  // namespace tritt

@@ -65,15 +65,14 @@ __global__ void from_half_kernel(const __half* __restrict__ src, TO* __restrict_
     dst[i] = from_f<TO>(__half2float(src[i]));
 }
 
-// dq (fp16, from the kernel) and the fp32 key-side sums dK1 | dK2 | dSiLU(V1) | dV2 -> the five gradients in the
-// inputs' type, with the dO scale divided out and SiLU'(V1) applied (reference flash_trittention.py:390-391).
+// The fp32 sums dK1 | dK2 | dSiLU(V1) | dV2 | dQ -> the five gradients in the inputs' type, with the dO scale
+// divided out and SiLU'(V1) applied (reference flash_trittention.py:390-391).
 template <typename TO>
-__global__ void wide_bwd_finalize_kernel(const __half* __restrict__ dq16, const float* __restrict__ part,
-                                         const TO* __restrict__ v1, TO* dq, TO* dk1, TO* dk2, TO* dv1, TO* dv2, size_t n,
-                                         const unsigned* absmax_bits) {
+__global__ void wide_bwd_finalize_kernel(const float* __restrict__ part, const TO* __restrict__ v1, TO* dq, TO* dk1, TO* dk2,
+                                         TO* dv1, TO* dv2, size_t n, const unsigned* absmax_bits) {
   const float inv = 1.f / pow2_scale(absmax_bits);
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    dq[i] = from_f<TO>(__half2float(dq16[i]) * inv);
+    dq[i] = from_f<TO>(part[4 * n + i] * inv);
     dk1[i] = from_f<TO>(part[i] * inv);
     dk2[i] = from_f<TO>(part[n + i] * inv);
     dv1[i] = from_f<TO>(part[2 * n + i] * inv * silu_grad_f(to_f(v1[i])));
@@ -106,7 +105,7 @@ size_t tdp_wide_workspace(int op, int B, int N, int T, int D) {
   if (op == TRITT_OP_TDP_FWD)
     return 6 * half_seg(n) + align_up(sm100_tdp_workspace(op, B, N, T, D, TRITT_F16) +
                                       sm100_tdp_fwd_optional_workspace(B, N, T, D, TRITT_F16), 256);
-  return 8 * half_seg(n) + 256 + align_up(sm100_tdp_workspace(op, B, N, T, D, TRITT_F16), 256);
+  return 7 * half_seg(n) + 256 + align_up(sm100_tdp_workspace(op, B, N, T, D, TRITT_F16), 256);
 }
 
 int tdp_wide_fwd(const TdpArgs& a) {
@@ -146,7 +145,7 @@ int tdp_wide_bwd(const TdpArgs& a) {
   }
   const size_t n = (size_t)a.B * a.N * a.T * a.D, h = half_seg(n);
   char* ws = (char*)a.workspace;
-  unsigned* absmax = (unsigned*)(ws + 8 * h);
+  unsigned* absmax = (unsigned*)(ws + 7 * h);
   TRITT_CUDA_OK(cudaMemsetAsync(absmax, 0, 4, a.stream));
   if (a.dtype == TRITT_F32)
     absmax_kernel<float><<<blocks_for(n), 256, 0, a.stream>>>((const float*)a.d_o, n, absmax);
@@ -164,24 +163,21 @@ int tdp_wide_bwd(const TdpArgs& a) {
   int rc = a.dtype == TRITT_F32 ? convert_in<float>(b, 7, n, absmax, a.status_word, a.stream)
                                 : convert_in<__nv_bfloat16>(b, 7, n, absmax, a.status_word, a.stream);
   if (rc) return rc;
-  __half* dq16 = (__half*)(ws + 7 * h);
   TdpArgs in = a;
   in.q = b.dst[0]; in.k1 = b.dst[1]; in.k2 = b.dst[2]; in.v1 = b.dst[3]; in.v2 = b.dst[4];
   in.o = b.dst[5]; in.d_o = b.dst[6];
-  in.dq = dq16;
-  in.dk1 = in.dk2 = in.dv1 = in.dv2 = nullptr;
+  in.dq = in.dk1 = in.dk2 = in.dv1 = in.dv2 = nullptr;
   in.dtype = TRITT_F16;
-  in.flags = a.flags | TRITT_FLAG_BWD_PARTIAL;  // leave the fp32 key-side sums in the inner workspace
-  in.workspace = ws + 8 * h + 256;
-  in.workspace_bytes = a.workspace_bytes - (8 * h + 256);
-  if ((rc = sm100_tdp_bwd(in))) return rc;
+  in.workspace = ws + 7 * h + 256;
+  in.workspace_bytes = a.workspace_bytes - (7 * h + 256);
+  if ((rc = sm100_tdp_bwd_sums(in))) return rc;
   const float* part = (const float*)in.workspace;
   if (a.dtype == TRITT_F32)
     wide_bwd_finalize_kernel<float><<<blocks_for(n), 256, 0, a.stream>>>(
-        dq16, part, (const float*)a.v1, (float*)a.dq, (float*)a.dk1, (float*)a.dk2, (float*)a.dv1, (float*)a.dv2, n, absmax);
+        part, (const float*)a.v1, (float*)a.dq, (float*)a.dk1, (float*)a.dk2, (float*)a.dv1, (float*)a.dv2, n, absmax);
   else
     wide_bwd_finalize_kernel<__nv_bfloat16><<<blocks_for(n), 256, 0, a.stream>>>(
-        dq16, part, (const __nv_bfloat16*)a.v1, (__nv_bfloat16*)a.dq, (__nv_bfloat16*)a.dk1, (__nv_bfloat16*)a.dk2,
+        part, (const __nv_bfloat16*)a.v1, (__nv_bfloat16*)a.dq, (__nv_bfloat16*)a.dk1, (__nv_bfloat16*)a.dk2,
         (__nv_bfloat16*)a.dv1, (__nv_bfloat16*)a.dv2, n, absmax);
   count_launch();
   TRITT_CUDA_OK(cudaGetLastError());

@@ -56,11 +56,8 @@ enum {
                                  64 / 128); fp16 inputs already have it.  Needs the larger workspace that
                                  tritt_workspace_bytes_flags() reports; an input element beyond fp16's range (65504)
                                  sets status bit 64. */
-  TRITT_FLAG_BWD_CTA_PAIRS = 8  /* tritt_tdp_bwd, 16-bit inputs, head dimension 128, no windows, an even number of
-                                 queries: run the backward kernel as clusters of two CTAs that share every key / value
-                                 tile (tcgen05 cta_group::2, 256-row products).  Same results up to the order of the
-                                 fp32 reduce-adds; measured 2 % slower than one CTA per item on a B200, so it is not
-                                 the default.  Ignored where it does not apply. */
+  TRITT_FLAG_BWD_CTA_PAIRS = 8  /* tritt_tdp_bwd: accepted and ignored (an earlier backward kernel could run as clusters
+                                 of two CTAs; it was the slower form) */
 };
 
 /* kernel families, as reported by tritt_tdp_path() */
