@@ -6,6 +6,7 @@ point of the package fails loudly.  There is no PyTorch or CPU fallback.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 import threading
 
@@ -34,6 +35,7 @@ _lib = None
 _lock = threading.Lock()
 _status = {}  # device index -> pinned int32 status word (created under _lock)
 _status_np = {}  # device index -> numpy view of the same word (a host read without any tensor machinery)
+_status_ptr = {}  # device index -> address of the same word
 launches = 0  # kernels-enqueuing library calls made by this process (bench bookkeeping)
 
 
@@ -131,8 +133,15 @@ def status_word(device) -> torch.Tensor:
             if t is None:
                 t = torch.zeros(1, dtype=torch.int32).pin_memory()
                 _status_np[key] = t.numpy()
+                _status_ptr[key] = t.data_ptr()
                 _status[key] = t
     return t
+
+
+def _status_address(device: torch.device) -> int:
+    """Address of ``status_word(device)`` (the word is never freed)."""
+    ptr = _status_ptr.get(device.index)
+    return status_word(device).data_ptr() if ptr is None else ptr
 
 
 def _describe(v: int) -> str:
@@ -174,20 +183,31 @@ def check_status(device=None, synchronize: bool = True) -> None:
                          "are invalid")
 
 
+@functools.lru_cache(maxsize=1024)
+def _workspace_bytes(op: int, B: int, N: int, T: int, D: int, dtype: int, flags: int) -> int:
+    return max(int(lib().tritt_workspace_bytes_flags(op, B, N, T, D, dtype, flags)), 256)
+
+
 def workspace(op: int, B: int, N: int, T: int, D: int, dtype: int, device, flags: int = 0) -> torch.Tensor:
-    nbytes = lib().tritt_workspace_bytes_flags(op, B, N, T, D, dtype, flags)
-    return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
+    return torch.empty(_workspace_bytes(op, B, N, T, D, dtype, flags), dtype=torch.uint8, device=device)
 
 
 def aligned(t: torch.Tensor) -> torch.Tensor:
     """``t`` made contiguous and, if its storage offset leaves it off a 16-byte boundary (a view into a larger
     buffer), copied: the library's vector and TMA accesses require that alignment and reject other pointers."""
-    t = t.contiguous()
+    if not t.is_contiguous():
+        t = t.contiguous()
     return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
 
 
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+# The current stream's handle and the current device without the Python objects around them (a call of a short sequence
+# takes as long to enqueue as to run: the stream object alone is 1-2 us of ~45).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
+
+
+def _stream(dev: torch.device) -> int:
+    return _raw_stream(dev.index) if _raw_stream is not None else torch.cuda.current_stream(dev).cuda_stream
 
 
 class _on_device:
@@ -197,7 +217,7 @@ class _on_device:
     __slots__ = ("ctx",)
 
     def __init__(self, dev: torch.device):
-        self.ctx = None if dev.index == torch.cuda.current_device() else torch.cuda.device(dev)
+        self.ctx = None if dev.index == _current_device() else torch.cuda.device(dev)
 
     def __enter__(self):
         if self.ctx is not None:
@@ -234,7 +254,7 @@ def tdp_fwd(q, k1, k2, v1, v2, o, lse, alpha, causal, k1w, k2w, kkl, kkr, q_mod=
         rc = lib().tritt_tdp_fwd(q.data_ptr(), k1.data_ptr(), k2.data_ptr(), v1.data_ptr(), v2.data_ptr(),
                                  o.data_ptr(), lse.data_ptr(), B, N, T, D, dt, float(alpha), int(bool(causal)),
                                  _win(k1w, T), _win(k2w, T), _win(kkl, T), _win(kkr, T), q_mod, q_rem,
-                                 ws.data_ptr(), ws.numel(), status_word(q.device).data_ptr(), flags, _stream())
+                                 ws.data_ptr(), ws.numel(), _status_address(q.device), flags, _stream(q.device))
     _check(rc, "tritt_tdp_fwd")
     launches += 1
 
@@ -254,7 +274,7 @@ def tdp_bwd(q, k1, k2, v1, v2, o, do, lse, dq, dk1, dk2, dv1, dv2, alpha, causal
                                  o.data_ptr(), do.data_ptr(), lse.data_ptr(), dq.data_ptr(), ptr(dk1), ptr(dk2),
                                  ptr(dv1), ptr(dv2), B, N, T, D, dt, float(alpha), int(bool(causal)),
                                  _win(k1w, T), _win(k2w, T), _win(kkl, T), _win(kkr, T), q_mod, q_rem,
-                                 ws.data_ptr(), ws.numel(), status_word(q.device).data_ptr(), flags, _stream())
+                                 ws.data_ptr(), ws.numel(), _status_address(q.device), flags, _stream(q.device))
     _check(rc, "tritt_tdp_bwd")
     launches += 1
     return ws
@@ -267,7 +287,7 @@ def tdp_bwd_finalize(v1, dk1, dk2, dv1, dv2, ws):
     with _on_device(v1.device):
         rc = lib().tritt_tdp_bwd_finalize(v1.data_ptr(), dk1.data_ptr(), dk2.data_ptr(), dv1.data_ptr(),
                                           dv2.data_ptr(), B, N, T, D, dtype_code(v1.dtype), ws.data_ptr(),
-                                          ws.numel(), _stream())
+                                          ws.numel(), _stream(v1.device))
     _check(rc, "tritt_tdp_bwd_finalize")
     launches += 1
 
@@ -283,8 +303,8 @@ def dps_fwd(q, k1, k2, v1, v2, o, m, alpha, causal, k_diff, flags=0):
         ws = workspace(OP_DPS_FWD, B, N, T, D, dt, q.device)
         rc = lib().tritt_dps_fwd(q.data_ptr(), k1.data_ptr(), k2.data_ptr(), v1.data_ptr(), v2.data_ptr(),
                                  o.data_ptr(), m.data_ptr(), B, N, T, D, dt, float(alpha), int(bool(causal)),
-                                 int(k_diff), ws.data_ptr(), ws.numel(), status_word(q.device).data_ptr(), flags,
-                                 _stream())
+                                 int(k_diff), ws.data_ptr(), ws.numel(), _status_address(q.device), flags,
+                                 _stream(q.device))
     _check(rc, "tritt_dps_fwd")
     launches += 1
     return ws
@@ -302,10 +322,10 @@ def dps_bwd(q, k1, k2, v1, v2, o, do, m, dq, dk1, dk2, dv1, dv2, alpha, causal, 
                 m.data_ptr(), dq.data_ptr(), dk1.data_ptr(), dk2.data_ptr(), dv1.data_ptr(), dv2.data_ptr(), B, N, T, D,
                 dt, float(alpha), int(bool(causal)), int(k_diff), ws.data_ptr(), ws.numel())
         if fwd_ws is None:
-            rc = lib().tritt_dps_bwd(*args, status_word(q.device).data_ptr(), flags, _stream())
+            rc = lib().tritt_dps_bwd(*args, _status_address(q.device), flags, _stream(q.device))
         else:
-            rc = lib().tritt_dps_bwd_saved(*args, fwd_ws.data_ptr(), fwd_ws.numel(), status_word(q.device).data_ptr(),
-                                           flags, _stream())
+            rc = lib().tritt_dps_bwd_saved(*args, fwd_ws.data_ptr(), fwd_ws.numel(), _status_address(q.device),
+                                           flags, _stream(q.device))
     _check(rc, "tritt_dps_bwd")
     launches += 1
 
@@ -321,6 +341,6 @@ def tdp_fwd_noalloc(q, k1, k2, v1, v2, o, lse, alpha, causal, k1w, k2w, kkl, kkr
         rc = lib().tritt_tdp_fwd_noalloc(q.data_ptr(), k1.data_ptr(), k2.data_ptr(), v1.data_ptr(), v2.data_ptr(),
                                          o.data_ptr(), lse.data_ptr(), B, N, T, D, dtype_code(q.dtype), float(alpha),
                                          int(bool(causal)), _win(k1w, T), _win(k2w, T), _win(kkl, T), _win(kkr, T),
-                                         status_word(q.device).data_ptr(), flags, _stream())
+                                         _status_address(q.device), flags, _stream(q.device))
     _check(rc, "tritt_tdp_fwd_noalloc")
     launches += 1

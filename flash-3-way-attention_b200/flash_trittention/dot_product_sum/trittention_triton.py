@@ -35,7 +35,7 @@ class TrittentionTritonFunction(torch.autograd.Function):
         _native.dtype_code(q.dtype)
         q, k1, k2, v1, v2 = (_native.aligned(t) for t in (q, k1, k2, v1, v2))
         o = torch.empty_like(q)
-        m = torch.empty(q.shape[:3], device=q.device, dtype=torch.float32)
+        m = q.new_empty(q.shape[:3], dtype=torch.float32)
         # convert_to_float32 asks for fp32 operands inside the kernels (reference trittention_triton.py:98-117
         # forwards it to its launches): the CUDA-core path computes in fp32 on every dtype
         flags = _native.FLAG_FORCE_SIMT if (convert_to_float32 or input_precision == "ieee") else 0

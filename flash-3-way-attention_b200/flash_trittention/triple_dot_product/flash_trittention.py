@@ -19,13 +19,14 @@ from .kernels.utils import process_masking_variables
 def _validate(Q, K1, K2, V1, V2):
     if Q.dim() != 4:
         raise ValueError(f"expected [batch, heads, seq_len, head_dim] tensors, got shape {tuple(Q.shape)}")
+    shape, dtype, device = Q.shape, Q.dtype, Q.device
     for name, tensor in (("K1", K1), ("K2", K2), ("V1", V1), ("V2", V2)):
-        if tensor.shape != Q.shape:
-            raise ValueError(f"{name} shape {tuple(tensor.shape)} does not match Q shape {tuple(Q.shape)}")
-        if tensor.dtype != Q.dtype:
-            raise ValueError(f"{name} dtype {tensor.dtype} does not match Q dtype {Q.dtype}")
-        if tensor.device != Q.device:
-            raise ValueError(f"{name} device {tensor.device} does not match Q device {Q.device}")
+        if tensor.shape != shape:
+            raise ValueError(f"{name} shape {tuple(tensor.shape)} does not match Q shape {tuple(shape)}")
+        if tensor.dtype != dtype:
+            raise ValueError(f"{name} dtype {tensor.dtype} does not match Q dtype {dtype}")
+        if tensor.device != device:
+            raise ValueError(f"{name} device {tensor.device} does not match Q device {device}")
     head_dim = Q.shape[-1]
     if head_dim <= 0 or head_dim & (head_dim - 1):
         nxt = 1 << max(head_dim - 1, 0).bit_length()
@@ -47,7 +48,7 @@ class FlashTrittention(torch.autograd.Function):
         k1_window, k2_window, kk_left, kk_right = process_masking_variables(
             seq_len, k1_window, k2_window, kk_left, kk_right)
         O = torch.empty_like(Q)
-        lse = torch.empty(Q.shape[:3], dtype=torch.float32, device=Q.device)
+        lse = Q.new_empty(Q.shape[:3], dtype=torch.float32)
         # convert_to_float32 asks for fp32 operands inside the kernel, which the reference then feeds to TF32 dot
         # products: here bf16 inputs get operands of TF32's 11 significant bits (fp16 copies) on the tensor cores;
         # fp16 inputs have them already, fp32 inputs always run that way
