@@ -146,6 +146,32 @@ def test_backward_bf16_matches_oracle(T, D, causal):
 
 
 @pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("T,causal", [(2, True), (63, True), (65, False), (128, False), (191, True), (257, True)])
+def test_backward_at_tile_edges(T, D, causal):
+    """One row more or less than a tile of queries (128) or of K1 rows (128, or 64 at head dimension 128), items cut in
+    parts of a few steps, batches of K2 / V2 rows that end early."""
+    _bwd_case(1, 3, T, D, torch.float16, causal, 0.5, 1.0 / D, seed=7 * T + D)
+
+
+@pytest.mark.parametrize("windows", [(40, 30, 10, 12), (1100, 25, 1100, 1100)])
+@pytest.mark.parametrize("T", [1023, 1030])
+def test_backward_on_both_sides_of_the_exact_first_queries(T, windows):
+    """From T = 1024 on the first 32 queries of a bf16 call are formed in fp32 beside the tensor-core kernel."""
+    B, N, D, alpha = 1, 1, 64, 1 / 64
+    q, k1, k2, v1, v2, dz = orc.make_inputs(B, N, T, D, scale=0.5, seed=T, dtype=torch.bfloat16)
+    leaves = [x.to(DEV).requires_grad_(True) for x in (q, k1, k2, v1, v2)]
+    k1w, k2w, kkl, kkr = windows
+    out = flash_trittention(*leaves, alpha, kkl, kkr, k1w, k2w, True)
+    out.backward(dz.to(DEV))
+    torch.cuda.synchronize()
+    assert _native.read_status(torch.device(DEV)) == 0, "a bounded barrier wait ran out"
+    f = [x.float().to(DEV) for x in (q, k1, k2, v1, v2, dz)]   # (the oracle's tensor algebra on the GPU, in fp32)
+    g_ref = orc.tdp_backward(*f, alpha, True, *windows, chunk=64, device=DEV)
+    for name, leaf, ref in zip(("dq", "dk1", "dk2", "dv1", "dv2"), leaves, g_ref):
+        assert_close(name, leaf.grad, ref, torch.bfloat16)
+
+
+@pytest.mark.parametrize("D", [64, 128])
 def test_backward_fp16_matches_oracle(D):
     _bwd_case(2, 2, 200, D, torch.float16, True, 0.5, 1.0 / D, seed=4)
 
