@@ -14,7 +14,8 @@
 //               the accumulator, P written back to TMEM; at the end the two halves of a row are merged, normalised and
 //               stored (fp32 and / or 16-bit, and optionally the 16-bit product with a second tensor, which is the outer
 //               leg's value operand)
-// The chain S -> soft-max -> P*V of one warpgroup is serial; the other's runs beside it.
+// The chain S -> soft-max -> P*V of one warpgroup is serial and bounds the kernel (8 tiles at T = 1024, ~3 us each); the
+// other's runs beside it.
 #include "tritt_common.cuh"
 #include "tritt_sm100.cuh"
 #include "tritt_sm100_tdp.cuh"
