@@ -24,6 +24,14 @@ template <> __device__ __forceinline__ float2 unpack2<__half>(uint32_t v) {
   return __half22float2(*reinterpret_cast<__half2*>(&v));
 }
 
+// Bits c of [lo, hi] among 0..31: with a mask of a row's columns a per-element test is one logic instruction (a constant
+// bit into a predicate) instead of two comparisons.
+__device__ __forceinline__ uint32_t column_mask(int lo, int hi) {
+  const uint32_t up = hi < 0 ? 0u : hi >= 31 ? ~0u : (2u << hi) - 1u;
+  const uint32_t down = lo <= 0 ? ~0u : lo > 31 ? 0u : ~0u << lo;
+  return up & down;
+}
+
 // Sum of v[0..31] over the 32 lanes of a warp, column-wise: on return lane i holds the
 // total of column i.  31 shuffles instead of 32 full reductions.
 __device__ __forceinline__ float warp_transpose_sum(float (&v)[32], int lane) {

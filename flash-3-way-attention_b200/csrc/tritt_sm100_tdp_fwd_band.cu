@@ -340,10 +340,10 @@ tdp_fwd_band_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_const
           uint32_t sr[32];
           tmem_ld32(tS + ch * 32, sr);
           tmem_wait_ld();
-          const int l2 = lo - ch * 32, h2 = hi - ch * 32;
+          const uint32_t cols = column_mask(lo - ch * 32, hi - ch * 32);
 #pragma unroll
           for (int c = 0; c < 32; ++c)
-            if (c >= l2 && c <= h2) mx = fmaxf(mx, __uint_as_float(sr[c]));
+            if (cols & (1u << c)) mx = fmaxf(mx, __uint_as_float(sr[c]));
         }
         m_used = mx;  // -inf for a row that attends nothing: every P below is then selected to 0
       }
@@ -370,14 +370,19 @@ tdp_fwd_band_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_const
             }
             psum += ps0 + ps1;
           } else {
-            const int l2 = lo - ch * 32, h2 = hi - ch * 32;
+            // (a mask and packed pairs instead of two comparisons and scalar sums per element: 2.22 -> 1.94 ms at B=2 N=8
+            // T=8192 D=64, windows 128/128/32/32)
+            const uint32_t cols = column_mask(lo - ch * 32, hi - ch * 32);
+            const float2 nm = make_float2(-m_used, -m_used);
+            float2 ps = make_float2(0.f, 0.f);
 #pragma unroll
             for (int c = 0; c < 32; c += 2) {
-              const float p0 = (c >= l2 && c <= h2) ? exp2f(__uint_as_float(sr[c]) - m_used) : 0.f;
-              const float p1 = (c + 1 >= l2 && c + 1 <= h2) ? exp2f(__uint_as_float(sr[c + 1]) - m_used) : 0.f;
-              psum += p0 + p1;
-              pk[c >> 1] = pack2<T16>(p0, p1);
+              const float2 x = __fadd2_rn(make_float2(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])), nm);
+              const float2 e = make_float2(cols & (1u << c) ? exp2f(x.x) : 0.f, cols & (2u << c) ? exp2f(x.y) : 0.f);
+              ps = __fadd2_rn(ps, e);
+              pk[c >> 1] = pack2<T16>(e.x, e.y);
             }
+            psum += ps.x + ps.y;
           }
         }
         // P chunk ch -> columns [16 ch, 16 ch + 16) of S_x, which the chunks before have already read
