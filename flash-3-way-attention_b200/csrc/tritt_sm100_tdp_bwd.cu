@@ -307,8 +307,10 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         q_ok = i < g.nq && i >= p.i_first;
         q = g.q_rem + (q_ok ? i : 0) * g.q_mod;
         const int e = prob_shift<T16>(g.last_q(it.qt), g.causal, T, g.k1w, g.k2w);
-        lse2 = __ldg(p.lse + (size_t)it.bh * T + q) * kLog2e - (float)e;
-        drow = __ldg(p.drow + (size_t)it.bh * T + q);
+        // (a row that is not this kernel's has P = 0 and a zero row of Q and dO, and needs Dq = 0 as well: 0 * (dP - Dq)
+        // of another query's infinite or NaN Dq would be NaN, which G sums into every key the tile meets)
+        lse2 = q_ok ? __ldg(p.lse + (size_t)it.bh * T + q) * kLog2e - (float)e : 0.f;
+        drow = q_ok ? __ldg(p.drow + (size_t)it.bh * T + q) : 0.f;
         dq_scale = exp2f(-(float)e) * kLn2;    // A carries alpha * log2(e)
         // A query that attends a single pair has P = 1 and a score gradient of exactly zero (TdpMask::single_pair):
         // P (dP - Dq) has two terms that are equal only up to the 16-bit rounding of the stored output, so its dS

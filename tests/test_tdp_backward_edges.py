@@ -1,0 +1,39 @@
+"""The tensor-core triple-dot-product backward where its tiles, ranges and scales end."""
+import pytest
+import torch
+
+from oracle import trittention_oracle as orc
+from flash_trittention import _native
+
+DEV = "cuda:0"
+NAMES = ("dq", "dk1", "dk2", "dv1", "dv2")
+
+
+def _backward(t, do, alpha, causal, windows=(None,) * 4):
+    B, N, T, _ = t[0].shape
+    o, lse = torch.empty_like(t[0]), torch.empty(B, N, T, device=DEV)
+    _native.tdp_fwd(*t, o, lse, alpha, causal, *windows)
+    g = [torch.empty_like(t[0]) for _ in range(5)]
+    _native.tdp_bwd(*t, o, do, lse, *g, alpha, causal, *windows)
+    torch.cuda.synchronize()
+    assert _native.read_status(torch.device(DEV)) == 0, "a bounded barrier wait ran out"
+    return g
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("T,D,dtype", [(260, 64, torch.float16), (260, 128, torch.bfloat16), (1100, 64, torch.bfloat16)])
+def test_a_query_that_is_not_finite_stays_in_its_tile(T, D, dtype, value):
+    """An infinite or NaN upstream row of query 0, which attends key 0 alone.  The products of its tile of 128 queries
+    and of 128 keys see it (0 * inf); the rows past the sequence and the rows that the tensor-core kernel leaves to the
+    exact first queries must not, so that every key past the first 128 and every other dQ row is what a zero row gives."""
+    t = [x.to(DEV) for x in orc.make_inputs(1, 2, T, D, scale=0.5, seed=T + D, dtype=dtype)]
+    do = t.pop()
+    bad, zero = do.clone(), do.clone()
+    bad[:, :, 0], zero[:, :, 0] = value, 0
+    got, want = _backward(t, bad, 1.0 / D, True), _backward(t, zero, 1.0 / D, True)
+    for name, a, b in zip(NAMES, got, want):
+        a, b = (x[:, :, 1 if name == "dq" else 128:].float() for x in (a, b))
+        assert torch.isfinite(a).all(), f"{name}: {int((~torch.isfinite(a)).sum())} of {a.numel()} values are not finite"
+        # (two runs of the same sums: the order of the fp32 reduce-adds, and where it meets the final rounding)
+        assert float((a - b).norm()) <= 1e-3 * float(b.norm()), name
