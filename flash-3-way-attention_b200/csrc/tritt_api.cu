@@ -235,6 +235,8 @@ int tritt_tdp_bwd_finalize(const void* v1, void* dk1, void* dk2, void* dv1, void
   return simt_tdp_bwd_finalize(v1, dk1, dk2, dv1, dv2, n, dtype, (const float*)workspace, (cudaStream_t)stream);
 }
 
+int tritt_selftest_bwd_registers(int launched) { return sm100_tdp_bwd_check_registers(launched); }
+
 static int norm_kdiff(int k_diff, int T) { return k_diff > T ? T : k_diff; }
 
 int tritt_dps_fwd(const void* q, const void* k1, const void* k2, const void* v1, const void* v2, void* o, float* m,

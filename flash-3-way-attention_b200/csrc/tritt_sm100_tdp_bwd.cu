@@ -37,6 +37,7 @@
 // Order of the products of step n:   S(n+1)  U(n)  dP(n+1)  dQ(n)  G(n).
 #include "tritt_sm100_tdp.cuh"
 
+#include <atomic>
 #include <type_traits>
 
 namespace tritt {
@@ -954,6 +955,28 @@ __global__ void tdp_bwd_finish_kernel(const float* __restrict__ sums, const T16*
   put(sums + 3 * n, dv2, nullptr);
 }
 
+// The register split of the kernel's warpgroups assumes the count it was launched with: setmaxnreg.inc waits without a limit
+// for registers that the block does not have, and .dec / .inc in the wrong direction is an illegal instruction.  A build
+// that gives the kernel another count is refused instead of being launched.
+int check_registers(int launched) {
+  if (launched == kRegsLaunch) return 0;
+  set_error("the backward kernel was built with %d registers per thread, its split needs %d", launched, kRegsLaunch);
+  return -30;
+}
+
+template <int D, typename T16, typename K>
+int check_kernel_registers(K kern) {
+  static std::atomic<int> launched{0};   // (per kernel: a property of the compiled code, the same on every device)
+  int n = launched.load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaFuncAttributes attr;
+    TRITT_CUDA_OK(cudaFuncGetAttributes(&attr, kern));
+    n = attr.numRegs;
+    launched.store(n, std::memory_order_relaxed);
+  }
+  return check_registers(n);
+}
+
 // workspace: fp32 sums dK1 | dK2 | dSiLU(V1) | dV2 | dQ, SiLU(V1) in the inputs' type, Dq fp32
 template <int D, typename T16>
 int launch_bwd_sums(const TdpArgs& a) {
@@ -1014,6 +1037,7 @@ int launch_bwd_sums(const TdpArgs& a) {
   if ((rc = make_tmap_3d(&tmK1, a.k1, 2, D, a.T, BN, 64, Cfg::JT))) return rc;
   if ((rc = make_tmap_3d(&tmSV1, sv1, 2, D, a.T, BN, 64, Cfg::JT))) return rc;
   auto kern = tdp_bwd_kernel<D, T16>;
+  if ((rc = check_kernel_registers<D, T16>(kern))) return rc;
   TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
   kern<<<grid, kBwdThreads, Cfg::kSmem, a.stream>>>(tmQ, tmDO, tmK1, tmSV1, p);
   count_launch();
@@ -1044,6 +1068,8 @@ int sm100_tdp_bwd_sums(const TdpArgs& a) {
     return a.D == 128 ? launch_bwd_sums<128, __nv_bfloat16>(a) : launch_bwd_sums<64, __nv_bfloat16>(a);
   return a.D == 128 ? launch_bwd_sums<128, __half>(a) : launch_bwd_sums<64, __half>(a);
 }
+
+int sm100_tdp_bwd_check_registers(int launched) { return check_registers(launched); }
 
 int sm100_tdp_bwd(const TdpArgs& a) {
   const int rc = sm100_tdp_bwd_sums(a);

@@ -28,7 +28,7 @@ SYMBOLS = (
     "tritt_tdp_fwd_min_workspace", "tritt_tdp_path", "tritt_dps_path", "tritt_tdp_fwd",
     "tritt_tdp_bwd", "tritt_tdp_bwd_finalize", "tritt_tdp_bwd_partials_offset", "tritt_dps_fwd",
     "tritt_dps_bwd", "tritt_dps_bwd_saved", "tritt_selftest_umma", "tritt_selftest_wait_expiry", "tritt_tdp_fwd_noalloc",
-    "tritt_noalloc_scratch_bytes",
+    "tritt_noalloc_scratch_bytes", "tritt_selftest_bwd_registers",
 )
 
 _lib = None
@@ -85,6 +85,8 @@ def lib():
                 L.tritt_tdp_fwd_noalloc.restype = i
                 L.tritt_tdp_fwd_noalloc.argtypes = [vp] * 7 + [i] * 5 + [f] + [i] * 5 + [vp, i, vp]
                 L.tritt_noalloc_scratch_bytes.restype = sz
+                L.tritt_selftest_bwd_registers.restype = i
+                L.tritt_selftest_bwd_registers.argtypes = [i]
                 L.tritt_selftest_umma.restype = i
                 L.tritt_selftest_umma.argtypes = [vp] * 5 + [i, vp, vp]
                 L.tritt_selftest_wait_expiry.restype = i

@@ -199,6 +199,13 @@ int tritt_selftest_umma(const void* A, const void* Bm, const void* V, float* C, 
  */
 int tritt_selftest_wait_expiry(int skip_arrival, long long limit_ticks, int* status_word, tritt_stream_t stream);
 
+/*
+ * Host-only self-test of the check in front of the backward kernel's launch: its warpgroups share out the registers it
+ * is launched with, and a build that gives it another count per thread than the split was written for is refused
+ * (0: `launched` registers per thread are what the split needs; -30: they are not).  No counterpart in the reference.
+ */
+int tritt_selftest_bwd_registers(int launched);
+
 #ifdef __cplusplus
 }
 #endif

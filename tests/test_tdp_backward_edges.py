@@ -37,3 +37,13 @@ def test_a_query_that_is_not_finite_stays_in_its_tile(T, D, dtype, value):
         assert torch.isfinite(a).all(), f"{name}: {int((~torch.isfinite(a)).sum())} of {a.numel()} values are not finite"
         # (two runs of the same sums: the order of the fp32 reduce-adds, and where it meets the final rounding)
         assert float((a - b).norm()) <= 1e-3 * float(b.norm()), name
+
+
+def test_backward_refuses_a_register_count_that_its_split_was_not_written_for():
+    """The warpgroups' shares add up to exactly the registers of the launch: with fewer, setmaxnreg.inc would wait for
+    ever (88 and below), with another count one of its directions would be wrong."""
+    check = _native.lib().tritt_selftest_bwd_registers
+    assert check(96) == 0
+    for launched in (64, 80, 88, 104, 128):
+        assert check(launched) == -30
+        assert b"registers per thread" in _native.lib().tritt_last_error()
