@@ -235,6 +235,24 @@ int tritt_tdp_bwd_finalize(const void* v1, void* dk1, void* dk2, void* dv1, void
   return simt_tdp_bwd_finalize(v1, dk1, dk2, dv1, dv2, n, dtype, (const float*)workspace, (cudaStream_t)stream);
 }
 
+int tritt_tdp_bwd_plan(int T, int D, int dtype, int causal, int k1_window, int k2_window, int kk_left, int kk_right, int q_mod,
+                       int q_rem, int flags, long long* out) {
+  int rc = check_shard(q_mod, q_rem);
+  if (rc) return rc;
+  TdpArgs a{};
+  a.B = a.N = 1; a.T = T; a.D = D;
+  a.mask = make_tdp_mask(causal, T, k1_window, k2_window, kk_left, kk_right);
+  a.q_mod = q_mod; a.q_rem = q_rem;
+  const bool wide = tdp_wide_applies(TRITT_OP_TDP_BWD, T, D, dtype, a.mask, flags);
+  if (!wide && !use_sm100(TRITT_OP_TDP_BWD, T, D, dtype, a.mask, flags)) {
+    set_error("tritt_tdp_bwd_plan is for calls on the tensor cores");
+    return -12;
+  }
+  a.dtype = wide ? TRITT_F16 : dtype;
+  sm100_tdp_bwd_plan(a, out);
+  return 0;
+}
+
 int tritt_selftest_bwd_registers(int launched) { return sm100_tdp_bwd_check_registers(launched); }
 
 static int norm_kdiff(int k_diff, int T) { return k_diff > T ? T : k_diff; }

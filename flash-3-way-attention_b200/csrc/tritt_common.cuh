@@ -137,6 +137,7 @@ int sm100_tdp_fwd(const TdpArgs& a);
 int sm100_tdp_bwd(const TdpArgs& a);
 // the same up to the fp32 sums: leaves dK1 | dK2 | dSiLU(V1) | dV2 | dQ at the head of the workspace
 int sm100_tdp_bwd_sums(const TdpArgs& a);
+void sm100_tdp_bwd_plan(const TdpArgs& a, long long* out);   // see tritt_tdp_bwd_plan()
 int sm100_tdp_bwd_check_registers(int launched);   // 0, or -30 if the backward kernel may not be launched with so many
 size_t sm100_tdp_workspace(int op, int B, int N, int T, int D, int dtype);
 size_t sm100_tdp_bwd_workspace(int B, int N, int T, int D);

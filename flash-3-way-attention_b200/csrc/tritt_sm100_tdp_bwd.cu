@@ -977,6 +977,42 @@ int check_kernel_registers(K kern) {
   return check_registers(n);
 }
 
+// The gradients of the first queries are the largest by far (a query attends ~q^2 pairs: its dQ falls like 1/q, and so
+// does what it adds to the first key rows), so on a long sequence their rounding to bf16 operands is most of the error
+// of the whole result.  They are a vanishing part of the work: exact fp32 on the CUDA cores, without a measurable cost
+// from this length on (419 us with and without it at B=1 N=1 T=1024 D=64); the error of a training step against fp64
+// goes from 3.6e-3 to 2.6e-3 at T=2048.  Short sequences have less of this spread, and fp16 operands are eight times
+// finer.  (Queries 0 to 31 themselves, not the first 32 rows of a shard: 8 interleaved shards have queries up to 248
+// among those, with 60 times the pairs, and at 64 shards and T=2048 they are the whole shard.)
+constexpr int kFirstQueries = 32, kFirstQueriesFromT = 1024;
+
+// What a call does, from its arguments alone.
+struct BwdPlan {
+  BwdGeometry g;
+  int i_first;        // query rows (of the shard) that the CUDA cores take, in exact fp32
+  long head_steps;    // steps of the kernel per head
+};
+
+template <int D> BwdPlan make_plan(const TdpArgs& a) {
+  BwdPlan p{};
+  const int nq = a.q_rem < a.T ? (a.T - a.q_rem + a.q_mod - 1) / a.q_mod : 0;
+  p.g = BwdGeometry{a.T, nq, a.q_mod, a.q_rem, a.mask.causal, a.mask.k1w, a.mask.k2w, a.mask.kkl, a.mask.kkr, BwdCfg<D>::JT};
+  if (nq == 0) return p;
+  if (a.dtype == TRITT_BF16 && a.mask.causal && a.T >= kFirstQueriesFromT && a.q_rem < kFirstQueries) {
+    p.i_first = (kFirstQueries - a.q_rem + a.q_mod - 1) / a.q_mod;
+    if (p.i_first >= nq) {   // nothing left for the kernel
+      p.i_first = nq;
+      return p;
+    }
+  }
+  for (int qt = 0; qt < p.g.q_tiles(); ++qt)
+    for (int jt = p.g.j_first(qt); jt <= p.g.j_last(qt); ++jt) {
+      int k0;
+      p.head_steps += p.g.k_range(qt, jt, k0);
+    }
+  return p;
+}
+
 // workspace: fp32 sums dK1 | dK2 | dSiLU(V1) | dV2 | dQ, SiLU(V1) in the inputs' type, Dq fp32
 template <int D, typename T16>
 int launch_bwd_sums(const TdpArgs& a) {
@@ -995,27 +1031,17 @@ int launch_bwd_sums(const TdpArgs& a) {
   p.dk1 = sums; p.dk2 = sums + n; p.dsv1 = sums + 2 * n; p.dv2 = sums + 3 * n; p.dq = sums + 4 * n;
   p.BN = BN;
   p.alpha = a.alpha;
-  // The gradients of the first queries are the largest by far (a query attends ~q^2 pairs: its dQ falls like 1/q, and so
-  // does what it adds to the first key rows), so on a long sequence their rounding to bf16 operands is most of the error
-  // of the whole result.  They are a vanishing part of the work: exact fp32 on the CUDA cores, without a measurable cost
-  // from this length on (419 us with and without it at B=1 N=1 T=1024 D=64); the error of a training step against fp64
-  // goes from 3.6e-3 to 2.6e-3 at T=2048.  Short sequences have less of this spread, and fp16 operands are eight times
-  // finer.
-  constexpr int kFirstQueries = 32, kFirstQueriesFromT = 1024;
-  if (std::is_same<T16, __nv_bfloat16>::value && a.mask.causal && a.T >= kFirstQueriesFromT) {
-    p.i_first = kFirstQueries;
-    const int rc = simt_tdp_bwd_first_queries(a, kFirstQueries, sums);
+  const BwdPlan plan = make_plan<D>(a);
+  const int nq = plan.g.nq;
+  if (nq == 0) return 0;
+  p.i_first = plan.i_first;
+  p.g = plan.g;
+  p.head_steps = plan.head_steps;
+  p.status = a.status_word;
+  if (plan.i_first > 0) {
+    const int rc = simt_tdp_bwd_first_queries(a, plan.i_first, sums);
     if (rc) return rc;
   }
-  p.status = a.status_word;
-  const int nq = a.q_rem < a.T ? (a.T - a.q_rem + a.q_mod - 1) / a.q_mod : 0;
-  if (nq == 0) return 0;
-  p.g = BwdGeometry{a.T, nq, a.q_mod, a.q_rem, a.mask.causal, a.mask.k1w, a.mask.k2w, a.mask.kkl, a.mask.kkr, Cfg::JT};
-  for (int qt = 0; qt < p.g.q_tiles(); ++qt)
-    for (int jt = p.g.j_first(qt); jt <= p.g.j_last(qt); ++jt) {
-      int k0;
-      p.head_steps += p.g.k_range(qt, jt, k0);
-    }
   if (p.head_steps == 0) return 0;
   // Cut: equal parts of the whole line of steps; where a part is short (under kShortPart steps) each head is cut by
   // itself, which keeps a part from setting up items of two heads at the price of a few idle SMs.  The two measure the
@@ -1067,6 +1093,12 @@ int sm100_tdp_bwd_sums(const TdpArgs& a) {
   if (a.dtype == TRITT_BF16)
     return a.D == 128 ? launch_bwd_sums<128, __nv_bfloat16>(a) : launch_bwd_sums<64, __nv_bfloat16>(a);
   return a.D == 128 ? launch_bwd_sums<128, __half>(a) : launch_bwd_sums<64, __half>(a);
+}
+
+void sm100_tdp_bwd_plan(const TdpArgs& a, long long* out) {
+  const BwdPlan p = a.D == 128 ? make_plan<128>(a) : make_plan<64>(a);
+  out[0] = p.i_first;
+  out[1] = p.head_steps * 128 * p.g.JT;
 }
 
 int sm100_tdp_bwd_check_registers(int launched) { return check_registers(launched); }

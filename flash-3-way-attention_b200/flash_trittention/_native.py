@@ -29,6 +29,7 @@ SYMBOLS = (
     "tritt_tdp_bwd", "tritt_tdp_bwd_finalize", "tritt_tdp_bwd_partials_offset", "tritt_dps_fwd",
     "tritt_dps_bwd", "tritt_dps_bwd_saved", "tritt_selftest_umma", "tritt_selftest_wait_expiry", "tritt_tdp_fwd_noalloc",
     "tritt_noalloc_scratch_bytes", "tritt_selftest_bwd_registers",
+    "tritt_tdp_bwd_plan",
 )
 
 _lib = None
@@ -87,6 +88,8 @@ def lib():
                 L.tritt_noalloc_scratch_bytes.restype = sz
                 L.tritt_selftest_bwd_registers.restype = i
                 L.tritt_selftest_bwd_registers.argtypes = [i]
+                L.tritt_tdp_bwd_plan.restype = i
+                L.tritt_tdp_bwd_plan.argtypes = [i] * 11 + [vp]
                 L.tritt_selftest_umma.restype = i
                 L.tritt_selftest_umma.argtypes = [vp] * 5 + [i, vp, vp]
                 L.tritt_selftest_wait_expiry.restype = i
@@ -280,6 +283,14 @@ def tdp_bwd(q, k1, k2, v1, v2, o, do, lse, dq, dk1, dk2, dv1, dv2, alpha, causal
     _check(rc, "tritt_tdp_bwd")
     launches += 1
     return ws
+
+
+def tdp_bwd_plan(T, D, dtype, causal, k1w, k2w, kkl, kkr, q_mod=1, q_rem=0, flags=0):
+    """(query rows in exact fp32, cells executed on the tensor cores) of one head of a backward call."""
+    out = (C.c_longlong * 2)()
+    _check(lib().tritt_tdp_bwd_plan(T, D, dtype, int(bool(causal)), _win(k1w, T), _win(k2w, T), _win(kkl, T), _win(kkr, T),
+                                    q_mod, q_rem, flags, out), "tritt_tdp_bwd_plan")
+    return tuple(out)
 
 
 def tdp_bwd_finalize(v1, dk1, dk2, dv1, dv2, ws):

@@ -200,6 +200,15 @@ int tritt_selftest_umma(const void* A, const void* Bm, const void* V, float* C, 
 int tritt_selftest_wait_expiry(int skip_arrival, long long limit_ticks, int* status_word, tritt_stream_t stream);
 
 /*
+ * What tritt_tdp_bwd does with these arguments on the tensor cores, per head (host only, for tests and planning):
+ *   out[0]  query rows that run in exact fp32 on the CUDA cores (of the shard, from its first)
+ *   out[1]  cells (q, j, k) that the tensor-core kernel executes, masked ones among them
+ * -12 if the call does not run on the tensor cores.  No counterpart in the reference.
+ */
+int tritt_tdp_bwd_plan(int T, int D, int dtype, int causal, int k1_window, int k2_window, int kk_left, int kk_right,
+                       int q_mod, int q_rem, int flags, long long* out);
+
+/*
  * Host-only self-test of the check in front of the backward kernel's launch: its warpgroups share out the registers it
  * is launched with, and a build that gives it another count per thread than the split was written for is refused
  * (0: `launched` registers per thread are what the split needs; -30: they are not).  No counterpart in the reference.

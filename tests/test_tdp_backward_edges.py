@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from _parity import assert_close
 from oracle import trittention_oracle as orc
 from flash_trittention import _native
 
@@ -47,3 +48,38 @@ def test_backward_refuses_a_register_count_that_its_split_was_not_written_for():
     for launched in (64, 80, 88, 104, 128):
         assert check(launched) == -30
         assert b"registers per thread" in _native.lib().tritt_last_error()
+
+
+@pytest.mark.parametrize("T", [1024, 2048, 2051])
+@pytest.mark.parametrize("q_mod", [1, 2, 3, 8, 64])
+def test_exact_first_queries_are_the_first_queries_of_the_sequence(T, q_mod):
+    """... and not the first 32 rows of a shard, whose queries lie q_mod apart."""
+    for q_rem in {0, 1 % q_mod, q_mod // 2, q_mod - 1}:
+        first, cells = _native.tdp_bwd_plan(T, 64, _native.BF16, True, None, None, None, None, q_mod, q_rem)
+        assert first == len(range(q_rem, 32, q_mod))
+        assert cells > 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,q_mod", [(1030, 8), (1024, 64)])
+def test_shards_with_exact_first_queries_sum_to_the_whole(T, q_mod):
+    """bf16 from T = 1024 on: shards that hold some of the first 32 queries, and shards that hold none."""
+    B, N, D, alpha = 1, 1, 64, 1 / 64
+    t = [x.to(DEV) for x in orc.make_inputs(B, N, T, D, scale=0.5, seed=T + q_mod, dtype=torch.bfloat16)]
+    do = t.pop()
+    full = _backward(t, do, alpha, True)
+    o, lse = torch.empty_like(do), torch.empty(B, N, T, device=DEV)
+    _native.tdp_fwd(*t, o, lse, alpha, True, None, None, None, None)
+    dq, n = torch.zeros_like(do), do.numel()
+    acc = torch.zeros(4 * n, device=DEV)
+    for rem in range(q_mod):
+        ws = _native.tdp_bwd(*t, o, do, lse, dq, None, None, None, None, alpha, True, None, None, None, None,
+                             q_mod=q_mod, q_rem=rem, flags=_native.FLAG_BWD_PARTIAL)
+        acc += ws[: 16 * n].view(torch.float32)
+    ws[: 16 * n].view(torch.float32).copy_(acc)
+    got = [dq] + [torch.empty_like(do) for _ in range(4)]
+    _native.tdp_bwd_finalize(t[3], *got[1:], ws)
+    torch.cuda.synchronize()
+    assert _native.read_status(torch.device(DEV)) == 0
+    for name, a, b in zip(NAMES, got, full):
+        assert_close(name, a, b, torch.bfloat16)
