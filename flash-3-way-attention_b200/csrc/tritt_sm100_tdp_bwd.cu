@@ -977,14 +977,15 @@ int check_kernel_registers(K kern) {
   return check_registers(n);
 }
 
-// The gradients of the first queries are the largest by far (a query attends ~q^2 pairs: its dQ falls like 1/q, and so
-// does what it adds to the first key rows), so on a long sequence their rounding to bf16 operands is most of the error
-// of the whole result.  They are a vanishing part of the work: exact fp32 on the CUDA cores, without a measurable cost
-// from this length on (419 us with and without it at B=1 N=1 T=1024 D=64); the error of a training step against fp64
-// goes from 3.6e-3 to 2.6e-3 at T=2048.  Short sequences have less of this spread, and fp16 operands are eight times
-// finer.  (Queries 0 to 31 themselves, not the first 32 rows of a shard: 8 interleaved shards have queries up to 248
-// among those, with 60 times the pairs, and at 64 shards and T=2048 they are the whole shard.)
-constexpr int kFirstQueries = 32, kFirstQueriesFromT = 1024;
+// The first queries of a causal call run in exact fp32 on the CUDA cores.  Their gradients are the largest by far (a query
+// attends ~q^2 pairs: its dQ falls like 1/q, and so does what it adds to the first key rows), so their rounding is most of
+// the error of the whole result; and with few pairs each, their probabilities are where it shows that S is formed from
+// another rounded product here (K1 K2) than in the forward (Q K2): P no longer sums to one.  From query 32 on (1089 pairs
+// without windows) the roundings of the pairs average out.  They are a vanishing part of the work: the error of a
+// training step against fp64 goes from 3.6e-3 to 2.6e-3 at T=2048 in bf16.
+// (Queries 0 to 31 themselves, not the first 32 rows of a shard: 8 interleaved shards have queries up to 248 among those,
+// with 60 times the pairs, and at 64 shards and T=2048 they are the whole shard.)
+constexpr int kFirstQueries = 32;
 
 // What a call does, from its arguments alone.
 struct BwdPlan {
@@ -998,7 +999,7 @@ template <int D> BwdPlan make_plan(const TdpArgs& a) {
   const int nq = a.q_rem < a.T ? (a.T - a.q_rem + a.q_mod - 1) / a.q_mod : 0;
   p.g = BwdGeometry{a.T, nq, a.q_mod, a.q_rem, a.mask.causal, a.mask.k1w, a.mask.k2w, a.mask.kkl, a.mask.kkr, BwdCfg<D>::JT};
   if (nq == 0) return p;
-  if (a.dtype == TRITT_BF16 && a.mask.causal && a.T >= kFirstQueriesFromT && a.q_rem < kFirstQueries) {
+  if (a.mask.causal && a.q_rem < kFirstQueries) {
     p.i_first = (kFirstQueries - a.q_rem + a.q_mod - 1) / a.q_mod;
     if (p.i_first >= nq) {   // nothing left for the kernel
       p.i_first = nq;

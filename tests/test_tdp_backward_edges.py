@@ -50,20 +50,23 @@ def test_backward_refuses_a_register_count_that_its_split_was_not_written_for():
         assert b"registers per thread" in _native.lib().tritt_last_error()
 
 
-@pytest.mark.parametrize("T", [1024, 2048, 2051])
+@pytest.mark.parametrize("dtype", [_native.BF16, _native.F16])
+@pytest.mark.parametrize("T", [200, 1024, 2051])
 @pytest.mark.parametrize("q_mod", [1, 2, 3, 8, 64])
-def test_exact_first_queries_are_the_first_queries_of_the_sequence(T, q_mod):
+def test_exact_first_queries_are_the_first_queries_of_the_sequence(T, q_mod, dtype):
     """... and not the first 32 rows of a shard, whose queries lie q_mod apart."""
     for q_rem in {0, 1 % q_mod, q_mod // 2, q_mod - 1}:
-        first, cells = _native.tdp_bwd_plan(T, 64, _native.BF16, True, None, None, None, None, q_mod, q_rem)
+        first, cells = _native.tdp_bwd_plan(T, 64, dtype, True, None, None, None, None, q_mod, q_rem)
         assert first == len(range(q_rem, 32, q_mod))
         assert cells > 0
+        assert _native.tdp_bwd_plan(T, 64, dtype, False, None, None, None, None, q_mod, q_rem)[0] == 0
+    assert _native.tdp_bwd_plan(30, 64, dtype, True, None, None, None, None) == (30, 0)
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("T,q_mod", [(1030, 8), (1024, 64)])
 def test_shards_with_exact_first_queries_sum_to_the_whole(T, q_mod):
-    """bf16 from T = 1024 on: shards that hold some of the first 32 queries, and shards that hold none."""
+    """Shards that hold some of the first 32 queries, and shards that hold none."""
     B, N, D, alpha = 1, 1, 64, 1 / 64
     t = [x.to(DEV) for x in orc.make_inputs(B, N, T, D, scale=0.5, seed=T + q_mod, dtype=torch.bfloat16)]
     do = t.pop()

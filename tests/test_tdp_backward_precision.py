@@ -1,0 +1,98 @@
+"""How exact the tensor-core triple-dot-product backward is against fp64.
+
+The yardstick is what the kernel's precision class gives: 16-bit operands, fp32 sums, with the row products formed per
+query as the forward forms them (Q K2 and dO V2 for dQ, dK2, dV2; Q K1 and dO SiLU(V1) for dK1, dV1), P and dS rounded to
+16 bits.  It is computed here beside the fp64 result; the kernel may not be further from fp64 than it, up to the spread
+between the roundings of two formations of one sum (the error of a norm over n rounded values spreads by about 1 / sqrt(n)
+and is small here, but the first queries carry most of a causal gradient: 8 % covers the seeds tried)."""
+import pytest
+import torch
+
+from oracle import trittention_oracle as orc
+from flash_trittention import _native
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+NAMES = ("dq", "dk1", "dk2", "dv1", "dv2")
+LOG2E = 1.4426950408889634
+SPREAD = 1.08
+
+
+def _mask(T, causal, windows):
+    q, j, k = (torch.arange(T, device=DEV).view(s) for s in ((-1, 1, 1), (1, 1, -1), (1, -1, 1)))   # [q, k, j]
+    if not causal:
+        return torch.ones(T, T, T, dtype=torch.bool, device=DEV)
+    w1, w2, kl, kr = (T if w is None else w for w in windows)
+    return (j <= q) & (q - j <= w1) & (k <= q) & (q - k <= w2) & (k - j <= kl) & (j - k <= kr)
+
+
+def _exact(x, do, alpha, ok):
+    """Dense fp64, one head: the five gradients."""
+    q, k1, k2, v1, v2 = (t.double() for t in x)
+    do, sig = do.double(), torch.sigmoid(v1)
+    s1 = v1 * sig
+    A = alpha * q[:, None] * k2
+    P = torch.where(ok, A @ k1.T, -torch.inf).flatten(1).softmax(1).view(ok.shape)
+    U = P @ s1
+    O = (U * v2).sum(1)
+    A2 = do[:, None] * v2
+    dS = P * (A2 @ s1.T - (do * O).sum(1)[:, None, None])
+    G = alpha * dS @ k1
+    return [(G * k2).sum(1), torch.einsum("qkj,qkh->jh", dS, A), (G * q[:, None]).sum(0),
+            torch.einsum("qkj,qkh->jh", P, A2) * (sig + s1 * (1 - sig)), (U * do[:, None]).sum(0)]
+
+
+def _rounded(x, do, o, lse, alpha, ok):
+    """The same with the precision class's roundings, from the forward's output and log-sum-exp."""
+    dt = x[0].dtype
+    rd = lambda t: t.to(dt).float()
+    q, k1, k2, v1, v2 = (t.float() for t in x)
+    do = do.float()
+    sig = torch.sigmoid(v1)
+    s1 = rd(v1 * sig)
+    Dq = (do * o.float()).sum(1)[:, None, None]
+    single = ok.flatten(1).sum(1).view(-1, 1, 1) == 1
+    # (P and dS take a power of two in fp16: probabilities below its normal range keep their bits)
+    sh = torch.exp2(ok.flatten(1).sum(1).float().log2().floor().clamp(max=10)).view(-1, 1, 1) if dt == torch.float16 else 1.0
+    out = {}
+    for row, col, yr, yc, m in ((k2, k1, v2, s1, ok), (k1, k2, s1, v2, ok.transpose(1, 2))):
+        S = rd(q[:, None] * (alpha * LOG2E) * row) @ col.T
+        P = torch.where(m, torch.exp2(S - lse[:, None, None] * LOG2E), 0.0) * sh
+        P = rd(P)
+        dS = torch.where(single, 0.0, rd(P * (rd(do[:, None] * yr) @ yc.T - Dq))) / sh
+        G, U = alpha * (dS @ col), (P / sh) @ yc
+        out[row is k1] = [(G * row).sum(1), (G * q[:, None]).sum(0), (U * do[:, None]).sum(0)]
+    return [rd(t) for t in (out[0][0], out[1][1], out[0][1], out[1][2] * (sig + v1 * sig * (1 - sig)), out[0][2])]
+
+
+def _errors(T, D, dtype, unit, causal, windows, names=NAMES, seeds=(0, 1)):
+    """Relative rms errors against fp64, kernel and yardstick, over a few heads and seeds."""
+    alpha = 1 / 8 if unit else 1.0 / D
+    got, bound = torch.zeros(5), torch.zeros(5)
+    ok = _mask(T, causal, windows)
+    for seed in seeds:
+        x = [t.to(DEV) for t in orc.make_inputs(1, 3, T, D, scale=1.0 if unit else 0.5, seed=100 * seed + T + D, dtype=dtype)]
+        do = x.pop()
+        o, lse = torch.empty_like(do), torch.empty(1, 3, T, device=DEV)
+        _native.tdp_fwd(*x, o, lse, alpha, causal, *windows)
+        g = [torch.empty_like(do) for _ in range(5)]
+        _native.tdp_bwd(*x, o, do, lse, *g, alpha, causal, *windows)
+        torch.cuda.synchronize()
+        assert _native.read_status(torch.device(DEV)) == 0
+        for h in range(3):
+            xh = [t[0, h] for t in x]
+            e = _exact(xh, do[0, h], alpha, ok)
+            r = _rounded(xh, do[0, h], o[0, h], lse[0, h], alpha, ok)
+            for i in range(5):
+                got[i] += float((g[i][0, h].double() - e[i]).norm() / e[i].norm())
+                bound[i] += float((r[i].double() - e[i]).norm() / e[i].norm())
+    return [(n, float(a / b)) for n, a, b in zip(NAMES, got, bound) if n in names]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,D", [(60, 64), (192, 64), (130, 128)])
+def test_probabilities_of_the_first_queries_sum_to_one(T, D, dtype):
+    """dV1 and dV2 are sums of P alone: where the recomputed P of a query with few pairs does not match the forward's
+    log-sum-exp, they are off by the difference."""
+    for name, ratio in _errors(T, D, dtype, True, True, (None,) * 4, names=("dv1", "dv2"), seeds=(0, 1, 2)):
+        assert ratio <= SPREAD, f"{name}: error {ratio:.2f} times that of the precision class"
