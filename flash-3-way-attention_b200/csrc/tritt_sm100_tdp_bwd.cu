@@ -191,14 +191,16 @@ struct BwdWalk {
 };
 
 // fp16 only: the recomputed probabilities of a query that attends n pairs are ~1/n, which for late rows lies below
-// fp16's normal range (6e-5; 1/n = 2e-7 at q = 2048).  P and dS are therefore formed times 2^e, and the folds divide
-// it out.  One e per q-tile, since G and U sum over its queries: it puts the tile's smallest mean probability at 2^-8
-// (e <= 10: a probability of 1 times a dP - Dq of up to 64 stays finite).  bf16 has fp32's exponent range: e = 0.
+// fp16's normal range (6e-5; 1/n = 2e-7 at q = 2048).  P and dS are therefore formed times 2^e, e = min(10, log2 of the
+// attended pairs' count bound), and the folds divide it out.  2^10 keeps a probability of 1 times a dP - Dq below 63
+// finite.  One e per q-tile, since G and U sum over its queries: that of the first query the kernel takes there, which
+// has the fewest pairs (without windows e = 10 everywhere, as the exact first queries leave none below 1089 pairs).
+// bf16 has fp32's exponent range: e = 0.
 template <typename T16>
-__device__ __forceinline__ int prob_shift(int q_last, int causal, int T, int k1w, int k2w) {
+__device__ __forceinline__ int prob_shift(int q, int causal, int T, int k1w, int k2w) {
   if constexpr (std::is_same<T16, __half>::value) {
-    const int n1 = causal ? min(q_last, k1w) + 1 : T, n2 = causal ? min(q_last, k2w) + 1 : T;
-    return max(0, min(10, (31 - __clz(n1)) + (31 - __clz(n2)) - 8));
+    const int n1 = causal ? min(q, k1w) + 1 : T, n2 = causal ? min(q, k2w) + 1 : T;
+    return min(10, (31 - __clz(n1)) + (31 - __clz(n2)));
   }
   return 0;
 }
@@ -307,7 +309,7 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         const int i = it.qt * 128 + row;
         q_ok = i < g.nq && i >= p.i_first;
         q = g.q_rem + (q_ok ? i : 0) * g.q_mod;
-        const int e = prob_shift<T16>(g.last_q(it.qt), g.causal, T, g.k1w, g.k2w);
+        const int e = prob_shift<T16>(g.q_rem + max(it.qt * 128, p.i_first) * g.q_mod, g.causal, T, g.k1w, g.k2w);
         // (a row that is not this kernel's has P = 0 and a zero row of Q and dO, and needs Dq = 0 as well: 0 * (dP - Dq)
         // of another query's infinite or NaN Dq would be NaN, which G sums into every key the tile meets)
         lse2 = q_ok ? __ldg(p.lse + (size_t)it.bh * T + q) * kLog2e - (float)e : 0.f;
@@ -498,7 +500,7 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         }
       arrive_warp(&bars.tile_free);
       const int len = it.len;
-      const int e = prob_shift<T16>(g.last_q(it.qt), g.causal, T, g.k1w, g.k2w);
+      const int e = prob_shift<T16>(g.q_rem + max(it.qt * 128, p.i_first) * g.q_mod, g.causal, T, g.k1w, g.k2w);
       const float unshift = exp2f(-(float)e);
       const float zscale = role ? unshift : unshift * p.alpha;
       float* zrow = (role ? p.dv2 : p.dk2) + ((size_t)it.bh * T + it.k0) * D;

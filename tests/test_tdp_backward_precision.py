@@ -5,6 +5,8 @@ query as the forward forms them (Q K2 and dO V2 for dQ, dK2, dV2; Q K1 and dO Si
 16 bits.  It is computed here beside the fp64 result; the kernel may not be further from fp64 than it, up to the spread
 between the roundings of two formations of one sum (the error of a norm over n rounded values spreads by about 1 / sqrt(n)
 and is small here, but the first queries carry most of a causal gradient: 8 % covers the seeds tried)."""
+import math
+
 import pytest
 import torch
 
@@ -43,8 +45,11 @@ def _exact(x, do, alpha, ok):
 
 
 def _rounded(x, do, o, lse, alpha, ok):
-    """The same with the precision class's roundings, from the forward's output and log-sum-exp."""
-    dt = x[0].dtype
+    """The same with the precision class's roundings, from the forward's output and log-sum-exp.  fp32 tensors run on fp16
+    copies, dO times the power of two that brings its largest value to (0.5, 1]."""
+    out_t, dt = x[0].dtype, torch.float16 if x[0].dtype == torch.float32 else x[0].dtype
+    scale = 2.0 ** -math.frexp(float(do.abs().max()))[1] if out_t == torch.float32 else 1.0
+    do, o = (do.float() * scale).to(dt), o.to(dt)
     rd = lambda t: t.to(dt).float()
     q, k1, k2, v1, v2 = (t.float() for t in x)
     do = do.float()
@@ -62,16 +67,18 @@ def _rounded(x, do, o, lse, alpha, ok):
         dS = torch.where(single, 0.0, rd(P * (rd(do[:, None] * yr) @ yc.T - Dq))) / sh
         G, U = alpha * (dS @ col), (P / sh) @ yc
         out[row is k1] = [(G * row).sum(1), (G * q[:, None]).sum(0), (U * do[:, None]).sum(0)]
-    return [rd(t) for t in (out[0][0], out[1][1], out[0][1], out[1][2] * (sig + v1 * sig * (1 - sig)), out[0][2])]
+    return [(t / scale).to(out_t) for t in (out[0][0], out[1][1], out[0][1], out[1][2] * (sig + v1 * sig * (1 - sig)), out[0][2])]
 
 
-def _errors(T, D, dtype, unit, causal, windows, names=NAMES, seeds=(0, 1)):
-    """Relative rms errors against fp64, kernel and yardstick, over a few heads and seeds."""
+def _errors(T, D, dtype, unit, causal, windows, names=NAMES, seeds=(0, 1), std=(1, 1, 1, 1)):
+    """Relative rms errors against fp64, kernel over yardstick, over a few heads and seeds.  std: Q, the keys, the values
+    and dO times this."""
     alpha = 1 / 8 if unit else 1.0 / D
     got, bound = torch.zeros(5), torch.zeros(5)
     ok = _mask(T, causal, windows)
     for seed in seeds:
-        x = [t.to(DEV) for t in orc.make_inputs(1, 3, T, D, scale=1.0 if unit else 0.5, seed=100 * seed + T + D, dtype=dtype)]
+        x = [t.to(DEV) for t in orc.make_inputs(1, 3, T, D, scale=1.0 if unit else 0.5, seed=100 * seed + T + D)]
+        x = [(t * std[i]).to(dtype) for t, i in zip(x, (0, 1, 1, 2, 2, 3))]
         do = x.pop()
         o, lse = torch.empty_like(do), torch.empty(1, 3, T, device=DEV)
         _native.tdp_fwd(*x, o, lse, alpha, causal, *windows)
@@ -95,4 +102,12 @@ def test_probabilities_of_the_first_queries_sum_to_one(T, D, dtype):
     """dV1 and dV2 are sums of P alone: where the recomputed P of a query with few pairs does not match the forward's
     log-sum-exp, they are off by the difference."""
     for name, ratio in _errors(T, D, dtype, True, True, (None,) * 4, names=("dv1", "dv2"), seeds=(0, 1, 2)):
+        assert ratio <= SPREAD, f"{name}: error {ratio:.2f} times that of the precision class"
+
+
+@pytest.mark.parametrize("T,windows", [(128, (None,) * 4), (300, (100, 60, 50, 40))])
+def test_small_score_gradients_keep_their_bits(T, windows):
+    """fp32 tensors (fp16 operands, no final rounding), values of 0.01: dP is about 1e-3, times a probability of 1 / 16000
+    at T = 128, against fp16's smallest normal value of 6e-5."""
+    for name, ratio in _errors(T, 64, torch.float32, False, True, windows, names=("dk1", "dk2"), std=(1, 1, 0.02, 1)):
         assert ratio <= SPREAD, f"{name}: error {ratio:.2f} times that of the precision class"
