@@ -133,7 +133,7 @@ size_t tritt_workspace_bytes_flags(int op, int B, int N, int T, int D, int dtype
     case TRITT_OP_TDP_BWD: {
       a = simt_tdp_workspace(op, B, N, T, D, dtype);
       b = sm100_tdp_workspace(op, B, N, T, D, dtype);
-      if (op == TRITT_OP_TDP_FWD && b) b += sm100_tdp_fwd_optional_workspace(B, N, T, D, dtype);
+      if (b) b += op == TRITT_OP_TDP_FWD ? sm100_tdp_fwd_optional_workspace(B, N, T, D, dtype) : sm100_tdp_bwd_optional_workspace(B, N);
       const TdpMask any = make_tdp_mask(1, T, T, T, T, T);
       if (tdp_wide_applies(op, T, D, dtype, any, flags)) {
         const size_t w = tdp_wide_workspace(op, B, N, T, D);
@@ -217,7 +217,7 @@ int tritt_tdp_bwd(const void* q, const void* k1, const void* k2, const void* v1,
   a.status_word = status_word; a.flags = flags; a.stream = (cudaStream_t)stream;
   const bool wide = tdp_wide_applies(TRITT_OP_TDP_BWD, T, D, dtype, a.mask, flags);
   const bool fast = use_sm100(TRITT_OP_TDP_BWD, T, D, dtype, a.mask, flags);
-  const size_t need = wide   ? tdp_wide_workspace(TRITT_OP_TDP_BWD, B, N, T, D)
+  const size_t need = wide   ? tdp_wide_workspace(TRITT_OP_TDP_BWD, B, N, T, D) - sm100_tdp_bwd_optional_workspace(B, N)
                       : fast ? sm100_tdp_workspace(TRITT_OP_TDP_BWD, B, N, T, D, dtype)
                              : simt_tdp_workspace(TRITT_OP_TDP_BWD, B, N, T, D, dtype);
   if ((rc = check_ws(need, workspace, workspace_bytes))) return rc;

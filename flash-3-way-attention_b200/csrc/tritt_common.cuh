@@ -141,6 +141,7 @@ void sm100_tdp_bwd_plan(const TdpArgs& a, long long* out);   // see tritt_tdp_bw
 int sm100_tdp_bwd_check_registers(int launched);   // 0, or -30 if the backward kernel may not be launched with so many
 size_t sm100_tdp_workspace(int op, int B, int N, int T, int D, int dtype);
 size_t sm100_tdp_bwd_workspace(int B, int N, int T, int D);
+size_t sm100_tdp_bwd_optional_workspace(int B, int N);   // behind it: statistics for the range shifts
 size_t sm100_tdp_fwd_optional_workspace(int B, int N, int T, int D, int dtype);
 // forward kernel for causal masks with a narrow (j, k) band (tiles of four queries x 32 K2 rows)
 bool sm100_tdp_fwd_band_applies(int T, const TdpMask& m);

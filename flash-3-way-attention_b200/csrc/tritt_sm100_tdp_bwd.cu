@@ -62,7 +62,7 @@ template <int D> struct BwdCfg {
   static constexpr int kOffK1 = kOffDO + kTileQ;      // K1 | SiLU(V1)
   static constexpr int kOffA = kOffK1 + 2 * kTileJ;   // A (two buffers) | A'
   static constexpr int kOffP = kOffA + 3 * kTileJ;    // P | dS (two buffers)
-  static constexpr int kOffVec = kOffP + 3 * kTileP;  // [slot][row][scale2 * K2 | V2] fp32
+  static constexpr int kOffVec = kOffP + 3 * kTileP;  // [slot][row][scale_k * K2 | scale_v * V2] fp32
   static constexpr int kVecRow = 2 * D;               // floats
   static constexpr int kOffBars = kOffVec + kVecSlots * kVecBatch * kVecRow * 4;
   static constexpr int kSmem = kOffBars + 448;
@@ -103,6 +103,8 @@ struct BwdGeometry {
 struct BwdParams {
   const void *q, *d_o, *k2, *v2;
   const float *lse, *drow;
+  const float* stats;      // [BN][stat_parts][8] (see tdp_bwd_prepare_kernel), or null
+  int stat_parts;
   float *dq, *dk1, *dk2, *dsv1, *dv2;   // fp32 sums, zero on entry
   BwdGeometry g;
   int BN;
@@ -114,13 +116,14 @@ struct BwdParams {
 };
 
 struct BwdItem {
-  int bh, qt, jt, k0, len, flags, pad[2];   // len 0: no more items
+  int bh, qt, jt, k0, len, flags;   // len 0: no more items
+  int ea, eb;                       // A and A' carry factors 2^ea and 2^eb (range_shift)
 };
 enum { kFirstOfQ = 1, kLastOfQ = 2 };       // the first / last item of a run over the j-tiles of one q-tile
 constexpr int kItemSlots = 4;               // (an item is read before its successor but one is written)
 
 struct BwdBarriers {
-  BwdItem items[kItemSlots];
+  alignas(16) BwdItem items[kItemSlots];
   uint64_t tile_full, tile_free;            // Q, dO, K1, SiLU(V1) of an item
   uint64_t vec_full[kVecSlots], vec_empty[kVecSlots];
   uint64_t a_ready[2], a_free[2], ap_ready;  // A: doubled by step parity (its producer may be two steps ahead)
@@ -180,7 +183,7 @@ struct BwdWalk {
   }
   // hands out the item found last and looks for the one after it
   __device__ BwdItem next(const BwdItem& prev) {
-    BwdItem it{bh, qt, jt, k0, len, 0, {0, 0}};
+    BwdItem it{bh, qt, jt, k0, len, 0, 0, 0};
     if (len == 0) return it;
     if (bh != prev.bh || qt != prev.qt) it.flags |= kFirstOfQ;
     step();
@@ -204,6 +207,20 @@ __device__ __forceinline__ int prob_shift(int q, int causal, int T, int k1w, int
   }
   return 0;
 }
+
+// fp16 only: A = alpha log2(e) K1 K2 and A' = SiLU(V1) V2 are products of two small factors (keys of 0.01: 1e-6, against
+// a smallest normal value of 6e-5) or of two large ones (beyond 65504 from 256 on), so they are formed times a power of
+// two per head that puts the largest product the head's elements allow into [2^14, 2^15): 28 binades below it stay normal.
+// The power is divided out in fp32, of S and dP in the soft-max warps and of the sums.  bf16 has fp32's range: 0.
+template <typename T16> __device__ __forceinline__ int range_shift(float bound) {
+  if constexpr (std::is_same<T16, __half>::value) {
+    if (!(bound > 0.f) || !isfinite(bound)) return 0;
+    return min(100, max(-100, 14 - ((__float_as_int(bound) >> 23) - 127)));
+  }
+  return 0;
+}
+
+__device__ __forceinline__ float pow2i(int e) { return __int_as_float((127 + e) << 23); }   // |e| <= 126, exact
 
 __device__ __forceinline__ void red_add(float* p, float v) {
   asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
@@ -284,8 +301,8 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     alive = wait_all(&bars.tile_full, items & 1);
     if (!alive) return false;
     const int4 a = *reinterpret_cast<const int4*>(&bars.items[items % kItemSlots]);
-    const int2 b = *reinterpret_cast<const int2*>(&bars.items[items % kItemSlots].len);
-    it.bh = a.x; it.qt = a.y; it.jt = a.z; it.k0 = a.w; it.len = b.x; it.flags = b.y;
+    const int4 b = *reinterpret_cast<const int4*>(&bars.items[items % kItemSlots].len);
+    it.bh = a.x; it.qt = a.y; it.jt = a.z; it.k0 = a.w; it.len = b.x; it.flags = b.y; it.ea = b.z; it.eb = b.w;
     return it.len > 0;
   };
 
@@ -303,6 +320,7 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     int q = 0;
     bool q_ok = false, single = false;
     float lse2 = 0.f, drow = 0.f, dq_scale = 0.f;
+    constexpr bool kShifted = std::is_same<T16, __half>::value;   // (S and dP carry factors 2^ea and 2^eb)
     while (alive && next_item(items, it, alive)) {
       ++items;
       if (it.flags & kFirstOfQ) {
@@ -314,7 +332,7 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         // of another query's infinite or NaN Dq would be NaN, which G sums into every key the tile meets)
         lse2 = q_ok ? __ldg(p.lse + (size_t)it.bh * T + q) * kLog2e - (float)e : 0.f;
         drow = q_ok ? __ldg(p.drow + (size_t)it.bh * T + q) : 0.f;
-        dq_scale = exp2f(-(float)e) * kLn2;    // A carries alpha * log2(e)
+        dq_scale = pow2i(-e - it.ea) * kLn2;    // A carries alpha * log2(e)
         // A query that attends a single pair has P = 1 and a score gradient of exactly zero (TdpMask::single_pair):
         // P (dP - Dq) has two terms that are equal only up to the 16-bit rounding of the stored output, so its dS
         // is set to zero.
@@ -343,6 +361,12 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       }
       const bool any_single = __any_sync(0xffffffffu, single);
       const float2 nlse = make_float2(-lse2, -lse2), ndq = make_float2(-drow, -drow);
+      const float sa = kShifted ? pow2i(-it.ea) : 1.f, sb = kShifted ? pow2i(-it.eb) : 1.f;
+      // v * scale + add; the scale of bf16 is 1
+      auto scaled = [](uint32_t v0, uint32_t v1, float scale, float2 add) {
+        const float2 v = make_float2(__uint_as_float(v0), __uint_as_float(v1));
+        return kShifted ? __ffma2_rn(v, make_float2(scale, scale), add) : __fadd2_rn(v, add);
+      };
       const int j0 = it.jt * JT + wg * CW;
       for (int i = 0; i < it.len; ++i, ++n) {
         const int k = it.k0 + i;
@@ -372,14 +396,14 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           if (full) {
 #pragma unroll
             for (int c = 0; c < 32; c += 2) {
-              const float2 x = __fadd2_rn(make_float2(__uint_as_float(s[c]), __uint_as_float(s[c + 1])), nlse);
+              const float2 x = scaled(s[c], s[c + 1], sa, nlse);
               s[c] = __float_as_uint(exp2f(x.x));
               s[c + 1] = __float_as_uint(exp2f(x.y));
             }
           } else {
 #pragma unroll
             for (int c = 0; c < 32; ++c)
-              s[c] = c0 + c >= lo && c0 + c <= hi ? __float_as_uint(exp2f(__uint_as_float(s[c]) - lse2)) : 0u;
+              s[c] = c0 + c >= lo && c0 + c <= hi ? __float_as_uint(exp2f(fmaf(__uint_as_float(s[c]), sa, -lse2))) : 0u;
           }
           if (c0 == 0) {
             // the previous step's U has read P
@@ -418,8 +442,7 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
               uint32_t w[4];
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
-                const float2 d =
-                    __fadd2_rn(make_float2(__uint_as_float(dp[c + 2 * e]), __uint_as_float(dp[c + 2 * e + 1])), ndq);
+                const float2 d = scaled(dp[c + 2 * e], dp[c + 2 * e + 1], sb, ndq);
                 const float2 ds = __fmul2_rn(
                     make_float2(__uint_as_float(s[c1 + c + 2 * e]), __uint_as_float(s[c1 + c + 2 * e + 1])), d);
                 w[e] = pack2<T16>(ds.x, ds.y);
@@ -501,7 +524,7 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       arrive_warp(&bars.tile_free);
       const int len = it.len;
       const int e = prob_shift<T16>(g.q_rem + max(it.qt * 128, p.i_first) * g.q_mod, g.causal, T, g.k1w, g.k2w);
-      const float unshift = exp2f(-(float)e);
+      const float unshift = pow2i(-e);
       const float zscale = role ? unshift : unshift * p.alpha;
       float* zrow = (role ? p.dv2 : p.dk2) + ((size_t)it.bh * T + it.k0) * D;
       auto form = [&](int i) -> bool {
@@ -680,7 +703,8 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       vb0 += (len + kVecBatch - 1) / kVecBatch;
       ++items;
       // ---- dK1 / dSiLU(V1) of this item
-      const float jscale = role ? unshift : unshift * kLn2;   // (the K2 rows carry alpha * log2(e))
+      // (the K2 rows carry alpha * log2(e) * 2^ea, the V2 rows 2^eb)
+      const float jscale = role ? unshift * pow2i(-it.eb) : unshift * pow2i(-it.ea) * kLn2;
       float* const base = (role ? p.dsv1 : p.dk1) + (size_t)it.bh * T * D;
 #pragma unroll
       for (int c16 = 0; c16 < 4; ++c16)
@@ -815,15 +839,34 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       tma_prefetch_desc(&tmK1);
       tma_prefetch_desc(&tmSV1);
     }
-    const float scale2 = p.alpha * kLog2e;
+    float scale_k = p.alpha * kLog2e, scale_v = 1.f;   // of the K2 and V2 rows, with the head's powers of two
+    int bh = -1, ea = 0, eb = 0;
     constexpr int kChunks = kVecBatch * D / 8 / 32;   // 16-byte pieces of K2 (and of V2) per lane and batch
     float* const vec = reinterpret_cast<float*>(smem + Cfg::kOffVec);
     uint32_t items = 0, vb = 0;
     bool alive = true, in_flight = false;
     BwdWalk walk(p);
-    BwdItem it{-1, -1, 0, 0, 0, 0, {0, 0}};
+    BwdItem it{-1, -1, 0, 0, 0, 0, 0, 0};
     while (alive) {
       it = walk.next(it);
+      if (it.len > 0 && it.bh != bh) {
+        bh = it.bh;
+        float m[4] = {0.f, 0.f, 0.f, 0.f};
+        if (p.stats && lane < p.stat_parts) {
+          const float4 x = __ldg(reinterpret_cast<const float4*>(p.stats + ((size_t)bh * p.stat_parts + lane) * 8));
+          m[0] = x.x; m[1] = x.y; m[2] = x.z; m[3] = x.w;
+        }
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], o));
+        ea = range_shift<T16>(fabsf(p.alpha * kLog2e) * m[0] * m[1]);
+        eb = range_shift<T16>(m[2] * m[3]);
+        scale_k = p.alpha * kLog2e * pow2i(ea);
+        scale_v = pow2i(eb);
+      }
+      it.ea = ea;
+      it.eb = eb;
       alive = wait_all(&bars.tile_free, (items & 1) ^ 1);
       if (!alive) break;
       if (leader) bars.items[items % kItemSlots] = it;
@@ -845,7 +888,7 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       }
       in_flight = true;
       ++items;
-      // K2 / V2 rows, fp32 (K2 times alpha * log2(e)), a batch of rows at a time; rows past the item repeat its last
+      // K2 / V2 rows, fp32, times their factors (K2's has alpha * log2(e)), a batch of rows at a time; rows past the item repeat its last
       const size_t head = (size_t)it.bh * T * D;
       for (int i = 0; i < it.len; i += kVecBatch, ++vb) {
         uint4 x[2][kChunks];
@@ -864,7 +907,7 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           float* dst = vec + ((vb % kVecSlots) * kVecBatch + r) * Cfg::kVecRow + col;
 #pragma unroll
           for (int m = 0; m < 2; ++m) {
-            const float sc = m == 0 ? scale2 : 1.f;
+            const float sc = m == 0 ? scale_k : scale_v;
             const uint4 y = x[m][c];
             const float2 f0 = unpack2<T16>(y.x), f1 = unpack2<T16>(y.y), f2 = unpack2<T16>(y.z), f3 = unpack2<T16>(y.w);
             *reinterpret_cast<float4*>(dst + m * D) = make_float4(f0.x * sc, f0.y * sc, f1.x * sc, f1.y * sc);
@@ -890,36 +933,79 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   if (tid == 0 && bars.abort_flag && p.status) atomicOr(p.status, 4);
 }
 
-// What the kernel needs before it starts, in one pass over the tensors (8 elements per thread): zeroed fp32 sums,
-// SiLU(V1) in the inputs' type and Dq = sum_h dO O per query.
+// What the kernel needs before it starts, in one pass over the tensors (8 elements per thread and step): zeroed fp32
+// sums, SiLU(V1) in the inputs' type, Dq = sum_h dO O per query and, when `stats` is not null, per head the largest
+// elements behind the range shifts, stats[head][part][0..3] = max |K1|, max |K2|, max |SiLU(V1)|, max |V2| of the part's
+// share of the head.  A head has up to kStatParts parts (blocks), which the kernel's loader warp reads one per lane: no
+// atomics, and nothing to zero before.
+constexpr int kStatParts = 32, kPrepThreads = 256;
 template <typename T16>
-__global__ void tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, const T16* __restrict__ d_o,
-                                       float* __restrict__ sums, T16* __restrict__ sv1, float* __restrict__ drow, size_t n,
-                                       int D) {
-  const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;   // (n is a multiple of 64)
-  const bool in = i < n;
-  float dot = 0.f;
-  if (in) {
+__global__ void __launch_bounds__(kPrepThreads)
+tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, const T16* __restrict__ d_o,
+                       const T16* __restrict__ k1, const T16* __restrict__ k2, const T16* __restrict__ v2,
+                       float* __restrict__ sums, T16* __restrict__ sv1, float* __restrict__ drow, float* __restrict__ stats,
+                       size_t n, int head_elems, int D, int parts) {
+  __shared__ float wmax[kPrepThreads / 32][4];
+  const int bh = blockIdx.x / parts, part = blockIdx.x % parts, lanes = D / 8;   // 8 or 16 lanes hold one row
+  const uint32_t row_lanes = ((1u << lanes) - 1u) << ((threadIdx.x & 31) / lanes * lanes);
+  float m[4] = {0.f, 0.f, 0.f, 0.f};
+  auto words = [](const T16* p, uint32_t (&w)[4]) {
+    const uint4 x = *reinterpret_cast<const uint4*>(p);
+    w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
+  };
+  auto grow = [](float& a, float2 x) { a = fmaxf(a, fmaxf(fabsf(x.x), fabsf(x.y))); };
+  // (the lanes of a row are all here or all gone: head_elems is a multiple of D)
+  for (int at = (part * kPrepThreads + threadIdx.x) * 8; at < head_elems; at += parts * kPrepThreads * 8) {
+    const size_t i = (size_t)bh * head_elems + at;
 #pragma unroll
     for (int s = 0; s < 5; ++s) {
       *reinterpret_cast<float4*>(sums + s * n + i) = make_float4(0.f, 0.f, 0.f, 0.f);
       *reinterpret_cast<float4*>(sums + s * n + i + 4) = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    const uint4 v = *reinterpret_cast<const uint4*>(v1 + i), a = *reinterpret_cast<const uint4*>(o + i),
-                b = *reinterpret_cast<const uint4*>(d_o + i);
-    const uint32_t wv[4] = {v.x, v.y, v.z, v.w}, wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
-    uint32_t r[4];
+    uint32_t wv[4], wa[4], wb[4], r[4];
+    words(v1 + i, wv);
+    words(o + i, wa);
+    words(d_o + i, wb);
+    float dot = 0.f;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float2 f = unpack2<T16>(wv[e]), x = unpack2<T16>(wa[e]), y = unpack2<T16>(wb[e]);
-      r[e] = pack2<T16>(silu_f(f.x), silu_f(f.y));
+      const float2 g = make_float2(silu_f(f.x), silu_f(f.y));
+      r[e] = pack2<T16>(g.x, g.y);
       dot = fmaf(x.x, y.x, fmaf(x.y, y.y, dot));
+      grow(m[2], unpack2<T16>(r[e]));
     }
     *reinterpret_cast<uint4*>(sv1 + i) = make_uint4(r[0], r[1], r[2], r[3]);
+    for (int s = lanes / 2; s >= 1; s >>= 1) dot += __shfl_xor_sync(row_lanes, dot, s);
+    if ((threadIdx.x & (lanes - 1)) == 0) drow[i / D] = dot;
+    if (stats) {
+      words(k1 + i, wv);
+      words(k2 + i, wa);
+      words(v2 + i, wb);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        grow(m[0], unpack2<T16>(wv[e]));
+        grow(m[1], unpack2<T16>(wa[e]));
+        grow(m[3], unpack2<T16>(wb[e]));
+      }
+    }
   }
-  const int lanes = D / 8;   // 8 or 16 lanes hold one row
-  for (int s = lanes / 2; s >= 1; s >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, s);
-  if (in && (threadIdx.x & (lanes - 1)) == 0) drow[i / D] = dot;
+  if (!stats) return;
+#pragma unroll
+  for (int o2 = 16; o2 >= 1; o2 >>= 1)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], o2));
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) wmax[threadIdx.x >> 5][i] = m[i];
+  }
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    float x = 0.f;
+#pragma unroll
+    for (int w = 0; w < kPrepThreads / 32; ++w) x = fmaxf(x, wmax[w][threadIdx.x]);
+    stats[(size_t)blockIdx.x * 8 + threadIdx.x] = x;
+  }
 }
 
 // The fp32 sums -> gradients in the inputs' type, SiLU'(V1) applied to dV1 (reference flash_trittention.py:390-391), 8
@@ -1016,7 +1102,8 @@ template <int D> BwdPlan make_plan(const TdpArgs& a) {
   return p;
 }
 
-// workspace: fp32 sums dK1 | dK2 | dSiLU(V1) | dV2 | dQ, SiLU(V1) in the inputs' type, Dq fp32
+// workspace: fp32 sums dK1 | dK2 | dSiLU(V1) | dV2 | dQ, SiLU(V1) in the inputs' type, Dq fp32; and, where the caller's has
+// it, the statistics (without them fp16 products are formed unshifted)
 template <int D, typename T16>
 int launch_bwd_sums(const TdpArgs& a) {
   using Cfg = BwdCfg<D>;
@@ -1025,11 +1112,19 @@ int launch_bwd_sums(const TdpArgs& a) {
   float* sums = (float*)a.workspace;
   T16* sv1 = (T16*)(sums + 5 * n);
   float* drow = (float*)(sv1 + n);
-  tdp_bwd_prepare_kernel<T16><<<(unsigned)((n / 8 + 255) / 256), 256, 0, a.stream>>>(
-      (const T16*)a.v1, (const T16*)a.o, (const T16*)a.d_o, sums, sv1, drow, n, D);
+  const size_t tail = align_up(sm100_tdp_bwd_workspace(a.B, a.N, a.T, D), 16);
+  const bool has_tail = a.workspace_bytes >= tail + (size_t)BN * kStatParts * 8 * sizeof(float);
+  float* stats = has_tail && std::is_same<T16, __half>::value ? (float*)((char*)a.workspace + tail) : nullptr;
+  const int head_elems = a.T * D, passes = (head_elems + kPrepThreads * 8 - 1) / (kPrepThreads * 8);
+  const int parts = passes < kStatParts ? passes : kStatParts;
+  tdp_bwd_prepare_kernel<T16><<<(unsigned)(BN * parts), kPrepThreads, 0, a.stream>>>(
+      (const T16*)a.v1, (const T16*)a.o, (const T16*)a.d_o, (const T16*)a.k1, (const T16*)a.k2, (const T16*)a.v2, sums, sv1,
+      drow, stats, n, head_elems, D, parts);
   count_launch();
   TRITT_CUDA_OK(cudaGetLastError());
   BwdParams p{};
+  p.stats = stats;
+  p.stat_parts = parts;
   p.q = a.q; p.d_o = a.d_o; p.k2 = a.k2; p.v2 = a.v2; p.lse = a.lse_in; p.drow = drow;
   p.dk1 = sums; p.dk2 = sums + n; p.dsv1 = sums + 2 * n; p.dv2 = sums + 3 * n; p.dq = sums + 4 * n;
   p.BN = BN;
@@ -1091,6 +1186,8 @@ size_t sm100_tdp_bwd_workspace(int B, int N, int T, int D) {
   const size_t r = (size_t)B * N * T, n = r * D;
   return 5 * n * sizeof(float) + n * 2 + r * sizeof(float);
 }
+
+size_t sm100_tdp_bwd_optional_workspace(int B, int N) { return align_up((size_t)B * N * kStatParts * 8 * sizeof(float) + 16, 256); }
 
 int sm100_tdp_bwd_sums(const TdpArgs& a) {
   if (a.dtype == TRITT_BF16)

@@ -105,7 +105,8 @@ size_t tdp_wide_workspace(int op, int B, int N, int T, int D) {
   if (op == TRITT_OP_TDP_FWD)
     return 6 * half_seg(n) + align_up(sm100_tdp_workspace(op, B, N, T, D, TRITT_F16) +
                                       sm100_tdp_fwd_optional_workspace(B, N, T, D, TRITT_F16), 256);
-  return 7 * half_seg(n) + 256 + align_up(sm100_tdp_workspace(op, B, N, T, D, TRITT_F16), 256);
+  return 7 * half_seg(n) + 256 + align_up(sm100_tdp_workspace(op, B, N, T, D, TRITT_F16), 256) +
+         sm100_tdp_bwd_optional_workspace(B, N);
 }
 
 int tdp_wide_fwd(const TdpArgs& a) {

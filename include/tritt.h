@@ -71,7 +71,9 @@ const char* tritt_last_error(void);
 /* Bytes of caller-provided scratch to pass to the given operation (0 if none).  For TRITT_OP_TDP_FWD on 16-bit inputs
    the figure includes a small tail (three floats per (batch, head), behind the SiLU(V1) copy of B*N*T*D elements) that
    lets the forward bound its scores and skip the row-maximum pass; a workspace without the tail is accepted and runs
-   the two-pass soft-max. */
+   the two-pass soft-max.  For TRITT_OP_TDP_BWD on the tensor cores it includes a tail of about 1 KiB per (batch, head)
+   for the largest elements behind the range shifts of fp16 products; a workspace without it is accepted and forms them
+   unshifted (small keys or values then lose bits to fp16's subnormals). */
 size_t tritt_workspace_bytes(int op, int B, int N, int T, int D, int dtype);
 /* The same for a call that will pass `flags` (TRITT_FLAG_WIDE_OPERANDS enlarges the triple-dot-product workspace of bf16
    inputs by the fp16 operand copies; tritt_workspace_bytes() equals flags = 0). */

@@ -51,7 +51,7 @@ def _rounded(x, do, o, lse, alpha, ok):
     scale = 2.0 ** -math.frexp(float(do.abs().max()))[1] if out_t == torch.float32 else 1.0
     do, o = (do.float() * scale).to(dt), o.to(dt)
     rd = lambda t: t.to(dt).float()
-    q, k1, k2, v1, v2 = (t.float() for t in x)
+    q, k1, k2, v1, v2 = (rd(t) for t in x)
     do = do.float()
     sig = torch.sigmoid(v1)
     s1 = rd(v1 * sig)
@@ -105,9 +105,38 @@ def test_probabilities_of_the_first_queries_sum_to_one(T, D, dtype):
         assert ratio <= SPREAD, f"{name}: error {ratio:.2f} times that of the precision class"
 
 
-@pytest.mark.parametrize("T,windows", [(128, (None,) * 4), (300, (100, 60, 50, 40))])
+@pytest.mark.parametrize("T,windows", [(128, (None,) * 4), (300, (None,) * 4), (300, (100, 60, 50, 40))])
 def test_small_score_gradients_keep_their_bits(T, windows):
     """fp32 tensors (fp16 operands, no final rounding), values of 0.01: dP is about 1e-3, times a probability of 1 / 16000
     at T = 128, against fp16's smallest normal value of 6e-5."""
     for name, ratio in _errors(T, 64, torch.float32, False, True, windows, names=("dk1", "dk2"), std=(1, 1, 0.02, 1)):
         assert ratio <= SPREAD, f"{name}: error {ratio:.2f} times that of the precision class"
+
+
+@pytest.mark.parametrize("dtype,T,D", [(torch.float16, 192, 64), (torch.float16, 130, 128), (torch.float32, 192, 64)])
+@pytest.mark.parametrize("keys,dout", [(0.02, 2048), (0.01, 2048), (200, 1 / 1024)])
+def test_products_of_small_and_large_keys(dtype, T, D, keys, dout):
+    """Keys of 0.01 and 0.005 under a loss scale of 1024: K1 K2 is far below fp16's smallest normal value.  Keys of 100 (Q of
+    0.001, as such keys want it): K1 K2 reaches fp16's largest value."""
+    ratios = _errors(T, D, dtype, False, True, (None,) * 4, std=(1 if keys < 1 else 2e-3, keys, 1, dout))
+    assert all(r <= SPREAD for _, r in ratios), f"errors over those of the precision class: {ratios}"
+
+
+def test_a_workspace_without_the_statistics_is_accepted():
+    """... and forms the fp16 products unshifted, as good for inputs of ordinary size."""
+    T, D = 200, 64
+    x = [t.to(DEV) for t in orc.make_inputs(1, 2, T, D, scale=0.5, seed=5, dtype=torch.float16)]
+    do = x.pop()
+    o, lse = torch.empty_like(do), torch.empty(1, 2, T, device=DEV)
+    _native.tdp_fwd(*x, o, lse, 1 / D, True, None, None, None, None)
+    n, full = do.numel(), _native.workspace(_native.OP_TDP_BWD, 1, 2, T, D, _native.F16, DEV)
+    out = []
+    for ws in (full, full[: 22 * n + 4 * 2 * T]):
+        out.append([torch.empty_like(do) for _ in range(5)])
+        _native.tdp_bwd(*x, o, do, lse, *out[-1], 1 / D, True, None, None, None, None, ws=ws)
+    with pytest.raises(ValueError, match="workspace"):
+        _native.tdp_bwd(*x, o, do, lse, *out[-1], 1 / D, True, None, None, None, None, ws=full[: 22 * n])
+    torch.cuda.synchronize()
+    assert _native.read_status(torch.device(DEV)) == 0
+    for name, a, b in zip(NAMES, *out):
+        assert float((a.float() - b.float()).norm()) <= 2e-3 * float(b.float().norm()), name
