@@ -121,9 +121,6 @@ struct DpsArgs {
 // kernel families (defined in their own translation units)
 int simt_tdp_fwd(const TdpArgs& a);
 int simt_tdp_bwd(const TdpArgs& a);
-// The contributions of the first `queries` query rows (of the shard) in exact fp32, added to the fp32 sums
-// dK1 | dK2 | dSiLU(V1) | dV2; their dQ rows are stored to the fifth tensor behind them.
-int simt_tdp_bwd_first_queries(const TdpArgs& a, int queries, float* sums);
 int simt_tdp_bwd_finalize(const void* v1, void* dk1, void* dk2, void* dv1, void* dv2, size_t n_elems, int dtype,
                           const float* partials, cudaStream_t stream);
 size_t simt_tdp_workspace(int op, int B, int N, int T, int D, int dtype);
@@ -137,6 +134,9 @@ int sm100_tdp_fwd(const TdpArgs& a);
 int sm100_tdp_bwd(const TdpArgs& a);
 // the same up to the fp32 sums: leaves dK1 | dK2 | dSiLU(V1) | dV2 | dQ at the head of the workspace
 int sm100_tdp_bwd_sums(const TdpArgs& a);
+// The contributions of the first `queries` rows of the shard (queries below 32, causal, head dimension 64 or 128, 16-bit)
+// in exact fp32, added to the fp32 sums dK1 | dK2 | dSiLU(V1) | dV2; their dQ rows are stored to the fifth tensor.
+int tdp_bwd_first_queries(const TdpArgs& a, int queries, float* sums, const float* drow);
 void sm100_tdp_bwd_plan(const TdpArgs& a, long long* out);   // see tritt_tdp_bwd_plan()
 int sm100_tdp_bwd_check_registers(int launched);   // 0, or -30 if the backward kernel may not be launched with so many
 size_t sm100_tdp_workspace(int op, int B, int N, int T, int D, int dtype);

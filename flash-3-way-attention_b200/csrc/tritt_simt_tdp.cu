@@ -29,8 +29,7 @@ struct SimtTdpParams {
   const float* lse;  // MODE_FWD / MODE_BWD: natural-log lse per row
   float* out_lse;    // MODE_LSE
   void* out_o;       // MODE_FWD
-  void* dq;          // MODE_BWD role 0 ...
-  float* dq_sum;     // ... or, if set, this fp32 tensor instead
+  void* dq;          // MODE_BWD role 0
   float *dX[2], *dY[2];  // MODE_BWD: fp32 accumulators for the row-side tensors, per role
   int T, D, nq;
   float alpha;
@@ -216,8 +215,6 @@ __global__ void tdp_simt_kernel(const __grid_constant__ SimtTdpParams p) {
     __syncthreads();
     if (MODE == MODE_FWD) {
       for (int h = tid; h < D; h += NT) ((T*)p.out_o + base)[(size_t)q * D + h] = from_f<T>(outacc[h]);
-    } else if (role == 0 && p.dq_sum) {
-      for (int h = tid; h < D; h += NT) p.dq_sum[base + (size_t)q * D + h] = outacc[h];
     } else if (role == 0) {
       for (int h = tid; h < D; h += NT) ((T*)p.dq + base)[(size_t)q * D + h] = from_f<T>(outacc[h]);
     }
@@ -367,19 +364,6 @@ int simt_tdp_bwd(const TdpArgs& a) {
   if (rc) return rc;
   if (a.flags & TRITT_FLAG_BWD_PARTIAL) return 0;
   return simt_tdp_bwd_finalize(a.v1, a.dk1, a.dk2, a.dv1, a.dv2, n, a.dtype, part, a.stream);
-}
-
-int simt_tdp_bwd_first_queries(const TdpArgs& a, int queries, float* sums) {
-  const size_t n = (size_t)a.B * a.N * a.T * a.D;
-  SimtTdpParams p = base_params(a);
-  p.nq = p.nq < queries ? p.nq : queries;
-  p.lse = a.lse_in;
-  p.dq_sum = sums + 4 * n;
-  p.dX[0] = sums + n;
-  p.dY[0] = sums + 3 * n;
-  p.dX[1] = sums;
-  p.dY[1] = sums + 2 * n;
-  return launch_dtype<MODE_BWD>(p, a.B * a.N, a.dtype, a.stream);
 }
 
 }  // namespace tritt

@@ -295,8 +295,6 @@ __device__ __forceinline__ float tdp_quad_pass(const SimtTdpParams& p, const int
     __syncthreads();
     if (MODE == MODE_FWD) {
       for (int h = tid; h < D; h += 128) ((T*)p.out_o + base)[(size_t)q * D + h] = from_f<T>(outacc[h]);
-    } else if (role == 0 && p.dq_sum) {
-      for (int h = tid; h < D; h += 128) p.dq_sum[base + (size_t)q * D + h] = outacc[h];
     } else if (role == 0) {
       for (int h = tid; h < D; h += 128) ((T*)p.dq + base)[(size_t)q * D + h] = from_f<T>(outacc[h]);
     }

@@ -1137,7 +1137,7 @@ int launch_bwd_sums(const TdpArgs& a) {
   p.head_steps = plan.head_steps;
   p.status = a.status_word;
   if (plan.i_first > 0) {
-    const int rc = simt_tdp_bwd_first_queries(a, plan.i_first, sums);
+    const int rc = tdp_bwd_first_queries(a, plan.i_first, sums, drow);
     if (rc) return rc;
   }
   if (p.head_steps == 0) return 0;
