@@ -4,7 +4,8 @@
 // indices can be the one that is stepped over.  Here it is k: for one k the (q, j) plane is an ordinary attention
 // backward whose key and value operands carry the k-th rows of K2 and V2,
 //     A [j,h] = alpha*log2(e) * K1[j,h] * K2[k,h]      A'[j,h] = SiLU(V1)[j,h] * V2[k,h]
-//     S  = Q A^T          P  = exp2(S - lse2[q])       (recomputed from the saved lse)
+//     S  = Q A^T (for large scores R K1^T with R [q,h] = alpha*log2(e) * Q[q,h] * K2[k,h])
+//                         P  = exp2(S - lse2[q])       (recomputed from the saved lse)
 //     dP = dO A'^T        dS = P * (dP - Dq[q]),       Dq = sum_h dO O
 // and all five gradients follow from three more products:
 //     dQ[q,:] += dS A                                  (accumulated over k in tensor memory)
@@ -32,8 +33,8 @@
 // [h x j], so that their M extent is 128 (64 + 64 + 64 + 64 + 128); a JT of 128 would need 640 columns.
 //
 // CTA: 20 warps.  0-3 and 4-7: soft-max warpgroups (half of a step's columns each, one query per thread); 8-11: forms
-// A and folds G; 12-15: forms A' and folds U; 16: issues the products; 17: TMA and the K2 / V2 rows (18, 19
-// idle).  P and dS are written to shared memory, where both the transposed (U, G) and the plain (dQ) product can read them.
+// A and folds G; 12-15: forms A' and folds U; 16: issues the products; 17: TMA and the K2 / V2 rows; 18,
+// 19: R.  P and dS are written to shared memory, where both the transposed (U, G) and the plain (dQ) product can read them.
 // Order of the products of step n:   S(n+1)  U(n)  dP(n+1)  dQ(n)  G(n).
 #include "tritt_sm100_tdp.cuh"
 
@@ -50,6 +51,17 @@ constexpr int kRegsLaunch = 96, kRegsSoftmax = 80, kRegsFold = 128, kRegsService
 static_assert(2 * kRegsSoftmax + 2 * kRegsFold + kRegsService <= 5 * kRegsLaunch, "more registers than the launch has");
 constexpr int kVecBatch = 4;     // K2 / V2 rows per hand-over
 constexpr int kVecSlots = 4;     // batches in flight
+// S = Q A^T rounds the product K1 K2 where the forward rounds R = Q K2, so that P does not match the saved log-sum-exp and no
+// longer sums to one; and the rounding of A is also dQ's.  Where scores are of order 1 or more and few pairs carry a query,
+// the gradients were up to 2.4 times further from fp64 than with the forward's operand (scores of order 3, not causal, T=200:
+// dQ 2.0 to 2.4 times, dV2 1.5 to 2.3; of order 1, D=128, bf16: dQ 1.33).  CTAs with such heads form S = R K1^T, from
+// the rows that the forward formed: 0.5 to 1.06 times there, dV2 1.00.  R is 128 x D for any JT and is formed by two warps, so
+// this costs speed (B200, against S = Q A^T): T=512 D=64 16 heads 0.95 -> 0.99 ms, T=4096 D=64 4 heads 81.5 -> 86.7 ms,
+// T=2048 D=128 16 heads 73 -> 82 ms.  Hence the bound, on |Q row| |K1 row| max|K2| in log2 units: Gaussian inputs with
+// a bound of 21 to 82 (their scores are 1/60 to 1/80 of it) show no excess with A (dQ 0.85 to 1.0), aligned inputs come
+// closer to their bound.
+constexpr float kScoreBound = 16.f;
+constexpr int kStatParts = 32, kStatFloats = 8;
 
 template <int D> struct BwdCfg {
   static constexpr int JT = D == 64 ? 128 : 64;       // rows j of an item
@@ -62,7 +74,9 @@ template <int D> struct BwdCfg {
   static constexpr int kOffK1 = kOffDO + kTileQ;      // K1 | SiLU(V1)
   static constexpr int kOffA = kOffK1 + 2 * kTileJ;   // A (two buffers) | A'
   static constexpr int kOffP = kOffA + 3 * kTileJ;    // P | dS (two buffers)
-  static constexpr int kOffVec = kOffP + 3 * kTileP;  // [slot][row][scale_k * K2 | scale_v * V2] fp32
+  // R (see tdp_bwd_body), in blocks of 64 columns: over the SiLU(V1) tile, and behind P | dS
+  static constexpr int kOffR0 = kOffK1 + kTileJ, kOffR1 = kOffP + 3 * kTileP;
+  static constexpr int kOffVec = kOffR1 + (D / 64 - 1) * 16384;  // [slot][row][scale_k * K2 | scale_v * V2] fp32
   static constexpr int kVecRow = 2 * D;               // floats
   static constexpr int kOffBars = kOffVec + kVecSlots * kVecBatch * kVecRow * 4;
   static constexpr int kSmem = kOffBars + 448;
@@ -103,7 +117,7 @@ struct BwdGeometry {
 struct BwdParams {
   const void *q, *d_o, *k2, *v2;
   const float *lse, *drow;
-  const float* stats;      // [BN][stat_parts][8] (see tdp_bwd_prepare_kernel), or null
+  const float* stats;      // [BN][stat_parts][kStatFloats] (see tdp_bwd_prepare_kernel), or null
   int stat_parts;
   float *dq, *dk1, *dk2, *dsv1, *dv2;   // fp32 sums, zero on entry
   BwdGeometry g;
@@ -119,20 +133,36 @@ struct BwdItem {
   int bh, qt, jt, k0, len, flags;   // len 0: no more items
   int ea, eb;                       // A and A' carry factors 2^ea and 2^eb (range_shift)
 };
-enum { kFirstOfQ = 1, kLastOfQ = 2 };       // the first / last item of a run over the j-tiles of one q-tile
+enum {
+  kFirstOfQ = 1, kLastOfQ = 2   // the first / last item of a run over the j-tiles of one q-tile
+};
 constexpr int kItemSlots = 4;               // (an item is read before its successor but one is written)
 
 struct BwdBarriers {
   alignas(16) BwdItem items[kItemSlots];
   uint64_t tile_full, tile_free;            // Q, dO, K1, SiLU(V1) of an item
   uint64_t vec_full[kVecSlots], vec_empty[kVecSlots];
-  uint64_t a_ready[2], a_free[2], ap_ready;  // A: doubled by step parity (its producer may be two steps ahead)
+  uint64_t a_ready[2], a_free[2], r_ready, ap_ready;  // A: doubled by step parity (its producer may be two steps ahead)
   uint64_t s_ready, s_free, p_ready, dp_ready, ds_ready, ds_free[2];
   uint64_t acc_done[2], acc_free[2];         // G, U
   uint64_t qdo_ready, dq_done, dq_free;
   uint32_t tmem_base;
   int abort_flag;
 };
+
+// the steps [s0, s1) of the line that are this CTA's
+__device__ __forceinline__ void cta_part(const BwdParams& p, long& s0, long& s1) {
+  const long H = p.head_steps;
+  if (p.parts > 0) {
+    const int b = blockIdx.x / p.parts, i = blockIdx.x % p.parts;
+    s0 = b * H + H * i / p.parts;
+    s1 = b * H + H * (i + 1) / p.parts;
+  } else {
+    const long total = H * p.BN, c = gridDim.x;
+    s0 = total / c * blockIdx.x + total % c * blockIdx.x / c;
+    s1 = total / c * (blockIdx.x + 1) + total % c * (blockIdx.x + 1) / c;
+  }
+}
 
 // One CTA's part of the line of steps, item by item (walked by the loader warp, which hands the items to the others).
 struct BwdWalk {
@@ -166,15 +196,7 @@ struct BwdWalk {
   __device__ explicit BwdWalk(const BwdParams& p) : g(p.g) {
     long s0, s1;
     const long H = p.head_steps;
-    if (p.parts > 0) {
-      const int b = blockIdx.x / p.parts, i = blockIdx.x % p.parts;
-      s0 = b * H + H * i / p.parts;
-      s1 = b * H + H * (i + 1) / p.parts;
-    } else {
-      const long total = H * p.BN, c = gridDim.x;
-      s0 = total / c * blockIdx.x + total % c * blockIdx.x / c;
-      s1 = total / c * (blockIdx.x + 1) + total % c * (blockIdx.x + 1) / c;
-    }
+    cta_part(p, s0, s1);
     left = s1 - s0;
     bh = (int)(s0 / H);
     qt = 0;
@@ -232,10 +254,43 @@ __device__ __forceinline__ void red_add4(float* p, float a, float b, float c, fl
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-template <int D, typename T16>
-__global__ void __launch_bounds__(kBwdThreads, 1)
-tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
-               const __grid_constant__ CUtensorMap tmK1, const __grid_constant__ CUtensorMap tmSV1, const BwdParams p) {
+// The statistics of a head over its parts, in every lane (zeros without them).
+struct BwdStats {
+  float qk1, k2, sv1, v2;    // largest element of Q and K1, of K2, SiLU(V1), V2
+  float k1_row, q_row;       // largest squared norm of a row
+};
+__device__ __forceinline__ BwdStats head_stats(const BwdParams& p, int bh, int lane) {
+  float m[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (p.stats && lane < p.stat_parts) {
+    const float4* src = reinterpret_cast<const float4*>(p.stats + ((size_t)bh * p.stat_parts + lane) * kStatFloats);
+    const float4 x = __ldg(src), y = __ldg(src + 1);
+    m[0] = x.x; m[1] = x.y; m[2] = x.z; m[3] = x.w; m[4] = y.x; m[5] = y.y;
+  }
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < 6; ++i) m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], o));
+  return BwdStats{m[0], m[1], m[2], m[3], m[4], m[5]};
+}
+
+// Whether a head of this CTA's part may have large scores (the same for every thread; without statistics: yes).
+__device__ __forceinline__ bool large_scores(const BwdParams& p) {
+  long s0, s1;
+  cta_part(p, s0, s1);
+  bool large = !p.stats;
+  const int last = (int)((s1 - 1) / p.head_steps);
+  for (int bh = (int)(s0 / p.head_steps) + (threadIdx.x >> 5); bh <= last && p.stats; bh += kBwdThreads / 32) {
+    const BwdStats st = head_stats(p, bh, threadIdx.x & 31);
+    // |S| <= |Q row| |K1 row| max|K2|, in log2 units, as S is  (not >, so that a NaN counts as large)
+    large |= !(fabsf(p.alpha * kLog2e) * sqrtf(st.k1_row * st.q_row) * st.k2 <= kScoreBound);
+  }
+  return __syncthreads_or(large);
+}
+
+// LARGE: S = R K1^T with R [q,h] = alpha*log2(e) * Q[q,h] * K2[k,h] instead of S = Q A^T (see kScoreBound).
+template <int D, typename T16, bool LARGE>
+__device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUtensorMap& tmDO, const CUtensorMap& tmK1,
+                                             const CUtensorMap& tmSV1, const BwdParams& p) {
   using Cfg = BwdCfg<D>;
   constexpr int JT = Cfg::JT, CW = Cfg::CW;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -260,6 +315,7 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       mbar_init(&bars.a_free[i], 1);
       mbar_init(&bars.ds_free[i], 1);
     }
+    mbar_init(&bars.r_ready, 2);
     mbar_init(&bars.ap_ready, 4);
     mbar_init(&bars.s_ready, 1);
     mbar_init(&bars.s_free, 8);
@@ -743,6 +799,8 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     const uint32_t qLo = desc_lo(smem_u32(smem + Cfg::kOffQ), 16384), doLo = desc_lo(smem_u32(smem + Cfg::kOffDO), 16384);
     const uint32_t aLo = desc_lo(smem_u32(smem + Cfg::kOffA), JT * 128);
     const uint32_t a2Lo = desc_lo(smem_u32(smem + Cfg::kOffA + 2 * Cfg::kTileJ), JT * 128);
+    const uint32_t rLo[2] = {desc_lo(smem_u32(smem + Cfg::kOffR0), 16), desc_lo(smem_u32(smem + Cfg::kOffR1), 16)};
+    const uint32_t k1Lo = desc_lo(smem_u32(smem + Cfg::kOffK1), 16);
     const uint32_t pLo = desc_lo(smem_u32(smem + Cfg::kOffP), 16384);
     constexpr uint32_t kTileP16 = Cfg::kTileP >> 4, kTileJ16 = Cfg::kTileJ >> 4;
     auto commit = [&](uint64_t* bar) {
@@ -773,10 +831,18 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     uint32_t n = 0, items = 0, runs = 0;
     bool alive = true;
     auto issue_s = [&](uint32_t m) -> bool {
-      if (!wait_all(&bars.a_ready[m & 1], (m >> 1) & 1)) return false;
+      if (!(LARGE ? wait_all(&bars.r_ready, m & 1) : wait_all(&bars.a_ready[m & 1], (m >> 1) & 1))) return false;
       if (!wait_all(&bars.s_free, (m & 1) ^ 1)) return false;
       tc_fence_after();
-      issue_rows(Cfg::kTmemS, Cfg::kTmemQ, aLo + (m & 1) * kTileJ16);
+      if constexpr (LARGE) {
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k)
+          if (leader)
+            mma_ss_lo(tmem + Cfg::kTmemS, rLo[k >> 2] + (k & 3) * 2, k1Lo + (k >> 2) * ((JT * 128) >> 4) + (k & 3) * 2, kHi, idesc_s,
+                      k > 0);
+      } else {
+        issue_rows(Cfg::kTmemS, Cfg::kTmemQ, aLo + (m & 1) * kTileJ16);
+      }
       commit(&bars.s_ready);
       return true;
     };
@@ -810,6 +876,10 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         if (fresh) {
           // the previous q-tile's dQ has been read
           if (!wait_all(&bars.dq_free, (runs & 1) ^ 1)) break;
+          tc_fence_after();
+        }
+        if constexpr (LARGE) {
+          if (!wait_all(&bars.a_ready[n & 1], (n >> 1) & 1)) break;
           tc_fence_after();
         }
         const uint32_t ds = pLo + (1 + (n & 1)) * kTileP16;
@@ -851,17 +921,9 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       it = walk.next(it);
       if (it.len > 0 && it.bh != bh) {
         bh = it.bh;
-        float m[4] = {0.f, 0.f, 0.f, 0.f};
-        if (p.stats && lane < p.stat_parts) {
-          const float4 x = __ldg(reinterpret_cast<const float4*>(p.stats + ((size_t)bh * p.stat_parts + lane) * 8));
-          m[0] = x.x; m[1] = x.y; m[2] = x.z; m[3] = x.w;
-        }
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], o));
-        ea = range_shift<T16>(fabsf(p.alpha * kLog2e) * m[0] * m[1]);
-        eb = range_shift<T16>(m[2] * m[3]);
+        const BwdStats st = head_stats(p, bh, lane);
+        ea = range_shift<T16>(fabsf(p.alpha * kLog2e) * st.qk1 * st.k2);
+        eb = range_shift<T16>(st.sv1 * st.v2);
         scale_k = p.alpha * kLog2e * pow2i(ea);
         scale_v = pow2i(eb);
       }
@@ -923,6 +985,72 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       while (!mbar_try_wait(&bars.tile_full, (items - 1) & 1) && clock64() - t0 < kWaitTicks / 8) {
       }
     }
+   } else if constexpr (LARGE) {
+    // ------------------------------------------------------------------ R (warps 18, 19)
+    // One step ahead of S, from the Q tile and the step's K2 row, rounded as the forward rounds it.  The first block's buffer
+    // is the SiLU(V1) tile, which nothing reads any more once the fold warps have it in registers.  A thread takes one
+    // 16-byte column of every kRowStep-th row.
+    constexpr int kCols = D / 8, kRowStep = 64 / kCols;
+    const int t = tid - 18 * 32, col = t % kCols, row0 = t / kCols;
+    const uint8_t* const src = smem + Cfg::kOffQ + (col >> 3) * 16384;
+    uint8_t* const dst = smem + (col >> 3 ? Cfg::kOffR1 : Cfg::kOffR0);
+    const float* const vec = reinterpret_cast<const float*>(smem + Cfg::kOffVec) + col * 8;
+    constexpr int kPieces = 2, kGroups = 128 / kRowStep / kPieces;
+    // byte offset of piece e of group g: the swizzle of a row depends on its last three bits, that is on e alone
+    uint32_t swz[kPieces];
+#pragma unroll
+    for (int e = 0; e < kPieces; ++e) swz[e] = swz128(row0 + e * kRowStep, col & 7);
+    auto at = [&](int g, int e) -> uint32_t { return swz[e] + g * kPieces * kRowStep * 128; };
+    uint4 next[kPieces];
+    auto fetch = [&](int g) {
+#pragma unroll
+      for (int e = 0; e < kPieces; ++e) next[e] = *reinterpret_cast<const uint4*>(src + at(g, e));
+    };
+    uint32_t n = 0, items = 0, vb0 = 0;
+    bool alive = true;
+    BwdItem it;
+    while (alive && next_item(items, it, alive)) {
+      ++items;
+      fetch(0);
+      // (the fold warps have read their tile: they have formed the item's first A')
+      alive = wait_all(&bars.ap_ready, n & 1);
+      for (int i = 0; i < it.len && alive; ++i) {
+        if ((i & (kVecBatch - 1)) == 0) {
+          const uint32_t vb = vb0 + i / kVecBatch;
+          alive = wait_all(&bars.vec_full[vb % kVecSlots], (vb / kVecSlots) & 1);
+        }
+        // the previous step's S has read the buffer (a second buffer would need a barrier of its own: two S may then have run
+        // before this wait, and a barrier two phases ahead of its waiter reads as not ready for ever)
+        if (alive && i > 0) alive = wait_all(&bars.s_ready, (n + i - 1) & 1);
+        if (!alive) break;
+        const float* v = vec + ((vb0 * kVecBatch + i) % (kVecSlots * kVecBatch)) * Cfg::kVecRow;
+        const float4 va = *reinterpret_cast<const float4*>(v), vb = *reinterpret_cast<const float4*>(v + 4);
+        const float2 m[4] = {make_float2(va.x, va.y), make_float2(va.z, va.w), make_float2(vb.x, vb.y), make_float2(vb.z, vb.w)};
+        // (the Q pieces of a group are fetched while the one before is worked on; those of the first, below, from the
+        // step before: they do not depend on the step)
+#pragma unroll 2
+        for (int g = 0; g < kGroups; ++g) {
+          uint4 x[kPieces];
+#pragma unroll
+          for (int e = 0; e < kPieces; ++e) x[e] = next[e];
+          fetch((g + 1) % kGroups);
+#pragma unroll
+          for (int e = 0; e < kPieces; ++e) {
+            uint32_t wx[4] = {x[e].x, x[e].y, x[e].z, x[e].w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const float2 f = __fmul2_rn(unpack2<T16>(wx[c]), m[c]);
+              wx[c] = pack2<T16>(f.x, f.y);
+            }
+            *reinterpret_cast<uint4*>(dst + at(g, e)) = make_uint4(wx[0], wx[1], wx[2], wx[3]);
+          }
+        }
+        fence_async_smem();
+        arrive_warp(&bars.r_ready);
+      }
+      n += it.len;
+      vb0 += (it.len + kVecBatch - 1) / kVecBatch;
+    }
    }
   }
 
@@ -933,22 +1061,31 @@ tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   if (tid == 0 && bars.abort_flag && p.status) atomicOr(p.status, 4);
 }
 
+template <int D, typename T16>
+__global__ void __launch_bounds__(kBwdThreads, 1)
+tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
+               const __grid_constant__ CUtensorMap tmK1, const __grid_constant__ CUtensorMap tmSV1,
+               const __grid_constant__ BwdParams p) {
+  if (large_scores(p)) tdp_bwd_body<D, T16, true>(tmQ, tmDO, tmK1, tmSV1, p);
+  else tdp_bwd_body<D, T16, false>(tmQ, tmDO, tmK1, tmSV1, p);
+}
+
 // What the kernel needs before it starts, in one pass over the tensors (8 elements per thread and step): zeroed fp32
 // sums, SiLU(V1) in the inputs' type, Dq = sum_h dO O per query and, when `stats` is not null, per head the largest
-// elements behind the range shifts, stats[head][part][0..3] = max |K1|, max |K2|, max |SiLU(V1)|, max |V2| of the part's
-// share of the head.  A head has up to kStatParts parts (blocks), which the kernel's loader warp reads one per lane: no
+// elements and row norms behind the range shifts and the score bound (BwdStats, kStatFloats floats per head and part) of
+// the part's share of the head.  A head has up to kStatParts parts (blocks), which the kernel's loader warp reads one per lane: no
 // atomics, and nothing to zero before.
-constexpr int kStatParts = 32, kPrepThreads = 256;
+constexpr int kPrepThreads = 256;
 template <typename T16>
 __global__ void __launch_bounds__(kPrepThreads)
 tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, const T16* __restrict__ d_o,
-                       const T16* __restrict__ k1, const T16* __restrict__ k2, const T16* __restrict__ v2,
-                       float* __restrict__ sums, T16* __restrict__ sv1, float* __restrict__ drow, float* __restrict__ stats,
+                       const T16* __restrict__ q, const T16* __restrict__ k1, const T16* __restrict__ k2,
+                       const T16* __restrict__ v2, float* __restrict__ sums, T16* __restrict__ sv1, float* __restrict__ drow, float* __restrict__ stats,
                        size_t n, int head_elems, int D, int parts) {
-  __shared__ float wmax[kPrepThreads / 32][4];
+  __shared__ float wmax[kPrepThreads / 32][6];
   const int bh = blockIdx.x / parts, part = blockIdx.x % parts, lanes = D / 8;   // 8 or 16 lanes hold one row
   const uint32_t row_lanes = ((1u << lanes) - 1u) << ((threadIdx.x & 31) / lanes * lanes);
-  float m[4] = {0.f, 0.f, 0.f, 0.f};
+  float qk1_max = 0.f, k2_max = 0.f, sv1_max = 0.f, v2_max = 0.f, k1_row = 0.f, q_row = 0.f;
   auto words = [](const T16* p, uint32_t (&w)[4]) {
     const uint4 x = *reinterpret_cast<const uint4*>(p);
     w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
@@ -973,7 +1110,7 @@ tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, co
       const float2 g = make_float2(silu_f(f.x), silu_f(f.y));
       r[e] = pack2<T16>(g.x, g.y);
       dot = fmaf(x.x, y.x, fmaf(x.y, y.y, dot));
-      grow(m[2], unpack2<T16>(r[e]));
+      grow(sv1_max, unpack2<T16>(r[e]));
     }
     *reinterpret_cast<uint4*>(sv1 + i) = make_uint4(r[0], r[1], r[2], r[3]);
     for (int s = lanes / 2; s >= 1; s >>= 1) dot += __shfl_xor_sync(row_lanes, dot, s);
@@ -984,27 +1121,44 @@ tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, co
       words(v2 + i, wb);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        grow(m[0], unpack2<T16>(wv[e]));
-        grow(m[1], unpack2<T16>(wa[e]));
-        grow(m[3], unpack2<T16>(wb[e]));
+        grow(qk1_max, unpack2<T16>(wv[e]));
+        grow(k2_max, unpack2<T16>(wa[e]));
+        grow(v2_max, unpack2<T16>(wb[e]));
       }
+      words(q + i, wa);
+      float n1 = 0.f, nq = 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 x = unpack2<T16>(wv[e]), y = unpack2<T16>(wa[e]);
+        grow(qk1_max, y);
+        n1 = fmaf(x.x, x.x, fmaf(x.y, x.y, n1));
+        nq = fmaf(y.x, y.x, fmaf(y.y, y.y, nq));
+      }
+      for (int s = lanes / 2; s >= 1; s >>= 1) {
+        n1 += __shfl_xor_sync(row_lanes, n1, s);
+        nq += __shfl_xor_sync(row_lanes, nq, s);
+      }
+      k1_row = fmaxf(k1_row, n1);
+      q_row = fmaxf(q_row, nq);
     }
   }
   if (!stats) return;
+  float w[6] = {qk1_max, k2_max, sv1_max, v2_max, k1_row, q_row};
 #pragma unroll
   for (int o2 = 16; o2 >= 1; o2 >>= 1)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], o2));
+    for (int i = 0; i < 6; ++i) w[i] = fmaxf(w[i], __shfl_xor_sync(0xffffffffu, w[i], o2));
   if ((threadIdx.x & 31) == 0) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) wmax[threadIdx.x >> 5][i] = m[i];
+    for (int i = 0; i < 6; ++i) wmax[threadIdx.x >> 5][i] = w[i];
   }
   __syncthreads();
-  if (threadIdx.x < 4) {
+  if (threadIdx.x < kStatFloats) {
     float x = 0.f;
+    if (threadIdx.x < 6)
 #pragma unroll
-    for (int w = 0; w < kPrepThreads / 32; ++w) x = fmaxf(x, wmax[w][threadIdx.x]);
-    stats[(size_t)blockIdx.x * 8 + threadIdx.x] = x;
+      for (int i = 0; i < kPrepThreads / 32; ++i) x = fmaxf(x, wmax[i][threadIdx.x]);
+    stats[(size_t)blockIdx.x * kStatFloats + threadIdx.x] = x;
   }
 }
 
@@ -1113,13 +1267,13 @@ int launch_bwd_sums(const TdpArgs& a) {
   T16* sv1 = (T16*)(sums + 5 * n);
   float* drow = (float*)(sv1 + n);
   const size_t tail = align_up(sm100_tdp_bwd_workspace(a.B, a.N, a.T, D), 16);
-  const bool has_tail = a.workspace_bytes >= tail + (size_t)BN * kStatParts * 8 * sizeof(float);
-  float* stats = has_tail && std::is_same<T16, __half>::value ? (float*)((char*)a.workspace + tail) : nullptr;
+  const bool has_tail = a.workspace_bytes >= tail + (size_t)BN * kStatParts * kStatFloats * sizeof(float);
+  float* stats = has_tail ? (float*)((char*)a.workspace + tail) : nullptr;
   const int head_elems = a.T * D, passes = (head_elems + kPrepThreads * 8 - 1) / (kPrepThreads * 8);
   const int parts = passes < kStatParts ? passes : kStatParts;
   tdp_bwd_prepare_kernel<T16><<<(unsigned)(BN * parts), kPrepThreads, 0, a.stream>>>(
-      (const T16*)a.v1, (const T16*)a.o, (const T16*)a.d_o, (const T16*)a.k1, (const T16*)a.k2, (const T16*)a.v2, sums, sv1,
-      drow, stats, n, head_elems, D, parts);
+      (const T16*)a.v1, (const T16*)a.o, (const T16*)a.d_o, (const T16*)a.q, (const T16*)a.k1, (const T16*)a.k2, (const T16*)a.v2,
+      sums, sv1, drow, stats, n, head_elems, D, parts);
   count_launch();
   TRITT_CUDA_OK(cudaGetLastError());
   BwdParams p{};
@@ -1187,7 +1341,7 @@ size_t sm100_tdp_bwd_workspace(int B, int N, int T, int D) {
   return 5 * n * sizeof(float) + n * 2 + r * sizeof(float);
 }
 
-size_t sm100_tdp_bwd_optional_workspace(int B, int N) { return align_up((size_t)B * N * kStatParts * 8 * sizeof(float) + 16, 256); }
+size_t sm100_tdp_bwd_optional_workspace(int B, int N) { return align_up((size_t)B * N * kStatParts * kStatFloats * sizeof(float) + 16, 256); }
 
 int sm100_tdp_bwd_sums(const TdpArgs& a) {
   if (a.dtype == TRITT_BF16)

@@ -70,23 +70,27 @@ def _rounded(x, do, o, lse, alpha, ok):
     return [(t / scale).to(out_t) for t in (out[0][0], out[1][1], out[0][1], out[1][2] * (sig + v1 * sig * (1 - sig)), out[0][2])]
 
 
-def _errors(T, D, dtype, unit, causal, windows, names=NAMES, seeds=(0, 1), std=(1, 1, 1, 1)):
+def _errors(T, D, dtype, unit, causal, windows, names=NAMES, seeds=(0, 1), std=(1, 1, 1, 1), columns=None, heads=3,
+            head_scale=None):
     """Relative rms errors against fp64, kernel over yardstick, over a few heads and seeds.  std: Q, the keys, the values
-    and dO times this."""
+    and dO times this.  columns [D], head_scale [heads]: Q and K1 times this."""
     alpha = 1 / 8 if unit else 1.0 / D
     got, bound = torch.zeros(5), torch.zeros(5)
     ok = _mask(T, causal, windows)
     for seed in seeds:
-        x = [t.to(DEV) for t in orc.make_inputs(1, 3, T, D, scale=1.0 if unit else 0.5, seed=100 * seed + T + D)]
+        x = [t.to(DEV) for t in orc.make_inputs(1, heads, T, D, scale=1.0 if unit else 0.5, seed=100 * seed + T + D)]
+        for t in x[:2]:
+            t *= 1 if columns is None else columns.to(DEV)
+            t *= 1 if head_scale is None else head_scale.view(1, -1, 1, 1).to(DEV)
         x = [(t * std[i]).to(dtype) for t, i in zip(x, (0, 1, 1, 2, 2, 3))]
         do = x.pop()
-        o, lse = torch.empty_like(do), torch.empty(1, 3, T, device=DEV)
+        o, lse = torch.empty_like(do), torch.empty(1, heads, T, device=DEV)
         _native.tdp_fwd(*x, o, lse, alpha, causal, *windows)
         g = [torch.empty_like(do) for _ in range(5)]
         _native.tdp_bwd(*x, o, do, lse, *g, alpha, causal, *windows)
         torch.cuda.synchronize()
         assert _native.read_status(torch.device(DEV)) == 0
-        for h in range(3):
+        for h in range(heads):
             xh = [t[0, h] for t in x]
             e = _exact(xh, do[0, h], alpha, ok)
             r = _rounded(xh, do[0, h], o[0, h], lse[0, h], alpha, ok)
@@ -140,3 +144,38 @@ def test_a_workspace_without_the_statistics_is_accepted():
     assert _native.read_status(torch.device(DEV)) == 0
     for name, a, b in zip(NAMES, *out):
         assert float((a.float() - b.float()).norm()) <= 2e-3 * float(b.float().norm()), name
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("unit", [True, False])
+@pytest.mark.parametrize("T,D,causal,windows", [
+    (192, 64, True, (None,) * 4), (330, 128, True, (None,) * 4), (300, 64, False, (None,) * 4), (200, 128, False, (None,) * 4),
+    (400, 64, True, (128, 128, 32, 32)), (350, 128, True, (40, 100, 20, 9)), (350, 64, True, (9, 5, 3, 2))])
+def test_errors_are_those_of_the_precision_class(T, D, causal, windows, dtype, unit):
+    """All five gradients, scores of order 1 to 10 and of order 0.01."""
+    ratios = _errors(T, D, dtype, unit, causal, windows)
+    print(T, D, causal, windows, dtype, unit, " ".join(f"{n} {r:.2f}" for n, r in ratios))
+    assert all(r <= SPREAD for _, r in ratios), f"errors over those of the precision class: {ratios}"
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("half", [0, 1])
+def test_scores_that_few_pairs_carry(half, D, dtype):
+    """Scores of order 3, from one half of the columns: P has to match the forward's log-sum-exp."""
+    columns = torch.full((D,), 0.05)
+    columns[half * D // 2:(half + 1) * D // 2] = 1.6
+    ratios = _errors(200, D, dtype, True, False, (None,) * 4, columns=columns)
+    print(half, D, dtype, " ".join(f"{n} {r:.2f}" for n, r in ratios))
+    assert all(r <= SPREAD for _, r in ratios), f"errors over those of the precision class: {ratios}"
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("T", [33, 70, 150])
+def test_heads_with_small_and_large_scores_in_one_cta(T, D):
+    """More heads than SMs, so that a CTA's part holds heads of both kinds; short, ragged lengths."""
+    heads = 160
+    ratios = _errors(T, D, torch.bfloat16, True, True, (None,) * 4, heads=heads, seeds=(0,),
+                     head_scale=torch.tensor([0.1, 1.2, 1.2, 0.2] * (heads // 4)))
+    print(T, D, " ".join(f"{n} {r:.2f}" for n, r in ratios))
+    assert all(r <= SPREAD for _, r in ratios), f"errors over those of the precision class: {ratios}"
