@@ -137,6 +137,10 @@ int sm100_tdp_bwd_sums(const TdpArgs& a);
 // The contributions of the first `queries` rows of the shard (queries below 32, causal, head dimension 64 or 128, 16-bit)
 // in exact fp32, added to the fp32 sums dK1 | dK2 | dSiLU(V1) | dV2; their dQ rows are stored to the fifth tensor.
 int tdp_bwd_first_queries(const TdpArgs& a, int queries, float* sums, const float* drow);
+// The backward of a query shard by the kernel that steps over queries: dQ rows stored, fp32 sums at the head of the
+// workspace; and the cells (q, j, k) that it executes per head (of one of its two roles).
+int sm100_tdp_bwd_queries(const TdpArgs& a);
+long long sm100_tdp_bwd_queries_cells(int T, const TdpMask& m, int q_mod, int q_rem);
 void sm100_tdp_bwd_plan(const TdpArgs& a, long long* out);   // see tritt_tdp_bwd_plan()
 int sm100_tdp_bwd_check_registers(int launched);   // 0, or -30 if the backward kernel may not be launched with so many
 size_t sm100_tdp_workspace(int op, int B, int N, int T, int D, int dtype);

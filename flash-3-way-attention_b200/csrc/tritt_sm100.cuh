@@ -92,6 +92,18 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
+// Tile reduce-add from shared memory into global memory (element type and swizzle come from the
+// tensor map; rows outside the tensor are dropped).  Completion is tracked per thread in bulk groups.
+__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* m, const void* smem_src, int x, int y, int z) {
+  asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
+                   (uint64_t)m),
+               "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// Wait until every committed bulk group of this thread has fully completed (writes performed).
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // ------------------------------------------------------------------ TMEM
 // Allocation is warp-collective (all 32 lanes execute it); `ncols` is a power of two >= 32.
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {
@@ -336,5 +348,8 @@ int make_tmap_3d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t co
 // The same over rows that are `row_stride` elements apart (heads `head_stride`): the rows of a query shard.
 int make_tmap_rows(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t bn, uint64_t row_stride,
                    uint64_t head_stride, uint32_t box_rows);
+// An fp32 tensor as the destination of TMA reduce-adds of 32-column pieces (128-byte rows, 128-byte swizzle).
+int make_tmap_3d_f32(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t bn, uint32_t box_cols,
+                     uint32_t box_rows);
 
 }  // namespace tritt

@@ -1234,7 +1234,17 @@ struct BwdPlan {
   BwdGeometry g;
   int i_first;        // query rows (of the shard) that the CUDA cores take, in exact fp32
   long head_steps;    // steps of the kernel per head
+  bool by_queries;    // the kernel that steps over queries instead: every row is its, as items of its own
+  long long cells;    // cells (q, j, k) executed per head
 };
+
+// A tile's 128 rows of a shard lie q_mod apart, and each of its steps is executed for all of them: at 8 shards the rows of
+// a tile span 1024 queries, and one shard of T=1024 executes 0.31 of the whole call's cells instead of 0.125, of T=2048
+// 0.21, of T=4096 0.17, of windows 128/128/32/32 0.63.  The kernel that steps over queries executes just a shard's share, at
+// a higher price per cell: stepping over k costs 0.76 (D=64) to 0.78 of it per cell (0.82 to 0.9 for large scores).
+// ms per call of one of 8 shards, k / queries: T=1024 D=64 16 heads 3.22 / 1.12, T=2048 D=128 16 heads 19.9 / 11.4, T=4096
+// D=64 4 heads 14.7 / 13.4, those windows 0.77 / 0.51; of one of 2: 3.65 / 4.35, 38.7 / 44.8, 41.8 / 52.6, 0.95 / 1.96.
+constexpr double kCellPrice = 0.8;
 
 template <int D> BwdPlan make_plan(const TdpArgs& a) {
   BwdPlan p{};
@@ -1253,13 +1263,22 @@ template <int D> BwdPlan make_plan(const TdpArgs& a) {
       int k0;
       p.head_steps += p.g.k_range(qt, jt, k0);
     }
+  p.cells = (long long)p.head_steps * 128 * BwdCfg<D>::JT;
+  if (a.q_mod > 1) {
+    const long long cells = sm100_tdp_bwd_queries_cells(a.T, a.mask, a.q_mod, a.q_rem);
+    if (kCellPrice * (double)p.cells > (double)cells) {
+      p.by_queries = true;
+      p.i_first = 0;
+      p.cells = cells;
+    }
+  }
   return p;
 }
 
 // workspace: fp32 sums dK1 | dK2 | dSiLU(V1) | dV2 | dQ, SiLU(V1) in the inputs' type, Dq fp32; and, where the caller's has
 // it, the statistics (without them fp16 products are formed unshifted)
 template <int D, typename T16>
-int launch_bwd_sums(const TdpArgs& a) {
+int launch_bwd_sums(const TdpArgs& a, const BwdPlan& plan) {
   using Cfg = BwdCfg<D>;
   const int BN = a.B * a.N;
   const size_t n = (size_t)BN * a.T * a.D;
@@ -1283,7 +1302,6 @@ int launch_bwd_sums(const TdpArgs& a) {
   p.dk1 = sums; p.dk2 = sums + n; p.dsv1 = sums + 2 * n; p.dv2 = sums + 3 * n; p.dq = sums + 4 * n;
   p.BN = BN;
   p.alpha = a.alpha;
-  const BwdPlan plan = make_plan<D>(a);
   const int nq = plan.g.nq;
   if (nq == 0) return 0;
   p.i_first = plan.i_first;
@@ -1343,22 +1361,30 @@ size_t sm100_tdp_bwd_workspace(int B, int N, int T, int D) {
 
 size_t sm100_tdp_bwd_optional_workspace(int B, int N) { return align_up((size_t)B * N * kStatParts * kStatFloats * sizeof(float) + 16, 256); }
 
-int sm100_tdp_bwd_sums(const TdpArgs& a) {
+static BwdPlan plan_of(const TdpArgs& a) { return a.D == 128 ? make_plan<128>(a) : make_plan<64>(a); }
+
+static int launch_sums(const TdpArgs& a, const BwdPlan& plan) {
   if (a.dtype == TRITT_BF16)
-    return a.D == 128 ? launch_bwd_sums<128, __nv_bfloat16>(a) : launch_bwd_sums<64, __nv_bfloat16>(a);
-  return a.D == 128 ? launch_bwd_sums<128, __half>(a) : launch_bwd_sums<64, __half>(a);
+    return a.D == 128 ? launch_bwd_sums<128, __nv_bfloat16>(a, plan) : launch_bwd_sums<64, __nv_bfloat16>(a, plan);
+  return a.D == 128 ? launch_bwd_sums<128, __half>(a, plan) : launch_bwd_sums<64, __half>(a, plan);
 }
 
+// (not sharded: the wide path is the only caller)
+int sm100_tdp_bwd_sums(const TdpArgs& a) { return launch_sums(a, plan_of(a)); }
+
 void sm100_tdp_bwd_plan(const TdpArgs& a, long long* out) {
-  const BwdPlan p = a.D == 128 ? make_plan<128>(a) : make_plan<64>(a);
+  const BwdPlan p = plan_of(a);
   out[0] = p.i_first;
-  out[1] = p.head_steps * 128 * p.g.JT;
+  out[1] = p.cells;
+  out[2] = p.by_queries;
 }
 
 int sm100_tdp_bwd_check_registers(int launched) { return check_registers(launched); }
 
 int sm100_tdp_bwd(const TdpArgs& a) {
-  const int rc = sm100_tdp_bwd_sums(a);
+  const BwdPlan plan = plan_of(a);
+  if (plan.by_queries) return sm100_tdp_bwd_queries(a);   // (a shard: its key-side sums stay sums)
+  const int rc = launch_sums(a, plan);
   if (rc) return rc;
   return a.dtype == TRITT_BF16 ? launch_finish<__nv_bfloat16>(a) : launch_finish<__half>(a);
 }

@@ -1,6 +1,6 @@
 // Host-side construction of the TMA tensor maps the tensor-core kernels take as launch parameters
 // (cuTensorMapEncodeTiled, looked up through the runtime so that the library has no link-time dependency on
-// libcuda): 3-D tiled maps over [B*N, rows, cols] 16-bit tensors with the 128-byte swizzle.
+// libcuda): 3-D tiled maps over [B*N, rows, cols] tensors with the 128-byte swizzle (16-bit operands, fp32 sums).
 #include "tritt_common.cuh"
 #include "tritt_sm100.cuh"
 
@@ -58,6 +58,16 @@ int make_tmap_rows(CUtensorMap* out, const void* base, uint64_t cols, uint64_t r
                    uint64_t head_stride, uint32_t box_rows) {
   return encode_3d(out, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, CU_TENSOR_MAP_SWIZZLE_128B, base, cols, rows, bn, row_stride,
                    head_stride, 64, box_rows);
+}
+
+int make_tmap_3d_f32(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t bn, uint32_t box_cols,
+                     uint32_t box_rows) {
+  if (box_cols != 32) {
+    set_error("make_tmap_3d_f32 is for pieces of 32 columns");
+    return -21;
+  }
+  return encode_3d(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, CU_TENSOR_MAP_SWIZZLE_128B, base, cols, rows, bn, cols, rows * cols,
+                   box_cols, box_rows);
 }
 
 }  // namespace tritt

@@ -286,8 +286,9 @@ def tdp_bwd(q, k1, k2, v1, v2, o, do, lse, dq, dk1, dk2, dv1, dv2, alpha, causal
 
 
 def tdp_bwd_plan(T, D, dtype, causal, k1w, k2w, kkl, kkr, q_mod=1, q_rem=0, flags=0):
-    """(query rows in exact fp32, cells executed on the tensor cores) of one head of a backward call."""
-    out = (C.c_longlong * 2)()
+    """(query rows in exact fp32, cells executed on the tensor cores, by the kernel that steps over queries) of one head of a
+    backward call."""
+    out = (C.c_longlong * 3)()
     _check(lib().tritt_tdp_bwd_plan(T, D, dtype, int(bool(causal)), _win(k1w, T), _win(k2w, T), _win(kkl, T), _win(kkr, T),
                                     q_mod, q_rem, flags, out), "tritt_tdp_bwd_plan")
     return tuple(out)

@@ -56,11 +56,11 @@ def test_backward_refuses_a_register_count_that_its_split_was_not_written_for():
 def test_exact_first_queries_are_the_first_queries_of_the_sequence(T, q_mod, dtype):
     """... and not the first 32 rows of a shard, whose queries lie q_mod apart."""
     for q_rem in {0, 1 % q_mod, q_mod // 2, q_mod - 1}:
-        first, cells = _native.tdp_bwd_plan(T, 64, dtype, True, None, None, None, None, q_mod, q_rem)
-        assert first == len(range(q_rem, 32, q_mod))
+        first, cells, by_queries = _native.tdp_bwd_plan(T, 64, dtype, True, None, None, None, None, q_mod, q_rem)
+        assert first == (0 if by_queries else len(range(q_rem, 32, q_mod)))
         assert cells > 0
         assert _native.tdp_bwd_plan(T, 64, dtype, False, None, None, None, None, q_mod, q_rem)[0] == 0
-    assert _native.tdp_bwd_plan(30, 64, dtype, True, None, None, None, None) == (30, 0)
+    assert _native.tdp_bwd_plan(30, 64, dtype, True, None, None, None, None) == (30, 0, 0)
 
 
 @pytest.mark.gpu
@@ -86,3 +86,53 @@ def test_shards_with_exact_first_queries_sum_to_the_whole(T, q_mod):
     assert _native.read_status(torch.device(DEV)) == 0
     for name, a, b in zip(NAMES, got, full):
         assert_close(name, a, b, torch.bfloat16)
+
+
+FULL = (None,) * 4
+
+
+@pytest.mark.parametrize("T,D,windows", [(333, 128, FULL), (1024, 64, FULL), (2048, 128, FULL), (4096, 64, FULL),
+                                         (2048, 64, (128, 128, 32, 32)), (1500, 64, (10, 700, 3, 5)), (1500, 128, (300, 20, 50, 9))])
+@pytest.mark.parametrize("q_mod", [2, 3, 4, 8, 64])
+def test_a_shard_executes_its_share_of_the_cells(T, D, windows, q_mod):
+    """Either kernel costs at most what the one that steps over queries costs, whose cells are the queries' own and whose
+    shards add up to the whole; the shares of the ranks are alike."""
+    causal, cost = True, []
+    whole = sum((q // 128 + 1) ** 2 * 128 * 128 for q in range(T))   # cells of the queries' tiles, without windows
+    for q_rem in range(q_mod):
+        first, cells, by_queries = _native.tdp_bwd_plan(T, D, _native.BF16, causal, *windows, q_mod, q_rem)
+        cost.append(cells if by_queries else 0.8 * cells)
+        if windows == FULL:
+            own = sum((q // 128 + 1) ** 2 * 128 * 128 for q in range(q_rem, T, q_mod))
+            assert cells == own if by_queries else 0.8 * cells <= own
+    if windows == FULL:
+        assert sum(cost) <= whole
+    assert max(cost) <= 1.25 * min(cost) + 64 * 128 * 128
+    assert _native.tdp_bwd_plan(T, D, _native.BF16, causal, *windows, 1, 0)[2] == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,D,q_mod,windows", [(130, 64, 2, FULL), (257, 128, 4, FULL), (300, 64, 8, (40, 100, 20, 9)),
+                                               (300, 128, 3, (100, 40, 10, 30)), (600, 64, 2, FULL)])
+def test_shards_sum_to_the_whole(T, D, q_mod, windows, dtype):
+    """Both kernels: the dQ rows of the shards and the sum of their key-side sums are those of the whole call."""
+    B, N, alpha = 1, 2, 1.0 / D
+    t = [x.to(DEV) for x in orc.make_inputs(B, N, T, D, scale=0.5, seed=T + q_mod, dtype=dtype)]
+    do = t.pop()
+    full = _backward(t, do, alpha, True, windows)
+    o, lse = torch.empty_like(do), torch.empty(B, N, T, device=DEV)
+    _native.tdp_fwd(*t, o, lse, alpha, True, *windows)
+    dq, n = torch.full_like(do, float("nan")), do.numel()
+    acc = torch.zeros(4 * n, device=DEV)
+    for rem in range(q_mod):
+        ws = _native.tdp_bwd(*t, o, do, lse, dq, None, None, None, None, alpha, True, *windows, q_mod=q_mod, q_rem=rem,
+                             flags=_native.FLAG_BWD_PARTIAL)
+        acc += ws[: 16 * n].view(torch.float32)
+    ws[: 16 * n].view(torch.float32).copy_(acc)
+    got = [dq] + [torch.empty_like(do) for _ in range(4)]
+    _native.tdp_bwd_finalize(t[3], *got[1:], ws)
+    torch.cuda.synchronize()
+    assert _native.read_status(torch.device(DEV)) == 0
+    for name, a, b in zip(NAMES, got, full):
+        assert_close(name, a, b, dtype)
