@@ -123,7 +123,6 @@ struct BwdParams {
   BwdGeometry g;
   int BN;
   int i_first;             // query rows (of the shard) before this one are not this kernel's
-  int parts;               // > 0: every head is cut in this many parts; 0: the whole line of steps in gridDim.x parts
   long head_steps;         // steps of one head
   float alpha;
   int* status;
@@ -153,15 +152,9 @@ struct BwdBarriers {
 // the steps [s0, s1) of the line that are this CTA's
 __device__ __forceinline__ void cta_part(const BwdParams& p, long& s0, long& s1) {
   const long H = p.head_steps;
-  if (p.parts > 0) {
-    const int b = blockIdx.x / p.parts, i = blockIdx.x % p.parts;
-    s0 = b * H + H * i / p.parts;
-    s1 = b * H + H * (i + 1) / p.parts;
-  } else {
-    const long total = H * p.BN, c = gridDim.x;
-    s0 = total / c * blockIdx.x + total % c * blockIdx.x / c;
-    s1 = total / c * (blockIdx.x + 1) + total % c * (blockIdx.x + 1) / c;
-  }
+  const long total = H * p.BN, c = gridDim.x;
+  s0 = total / c * blockIdx.x + total % c * blockIdx.x / c;
+  s1 = total / c * (blockIdx.x + 1) + total % c * (blockIdx.x + 1) / c;
 }
 
 // One CTA's part of the line of steps, item by item (walked by the loader warp, which hands the items to the others).
@@ -1313,18 +1306,8 @@ int launch_bwd_sums(const TdpArgs& a, const BwdPlan& plan) {
     if (rc) return rc;
   }
   if (p.head_steps == 0) return 0;
-  // Cut: equal parts of the whole line of steps; where a part is short (under kShortPart steps) each head is cut by
-  // itself, which keeps a part from setting up items of two heads at the price of a few idle SMs.  The two measure the
-  // same there (backward, even against per head: T=333 4 heads D=64 125.1 / 125.5 us, D=128 176.3 / 176.1 us; T=128 64
-  // heads D=64 168.7 / 169.0 us).
-  constexpr long kShortPart = 64;
-  const long total = p.head_steps * BN, sms = num_sms();
-  int grid = (int)(total < sms ? total : sms);
-  if (total < sms * kShortPart && BN <= sms) {
-    const long parts = sms / BN;
-    p.parts = (int)(parts < p.head_steps ? parts : p.head_steps);
-    grid = p.parts * BN;
-  }
+  const long total = p.head_steps * BN, sms = num_sms();   // (equal parts of the whole line of steps)
+  const int grid = (int)(total < sms ? total : sms);
   CUtensorMap tmQ, tmDO, tmK1, tmSV1;
   int rc;
   const size_t shard = (size_t)a.q_rem * D;   // first query row of the shard
