@@ -134,7 +134,8 @@ int sm100_tdp_fwd(const TdpArgs& a);
 int sm100_tdp_bwd(const TdpArgs& a);
 // the same up to the fp32 sums: leaves dK1 | dK2 | dSiLU(V1) | dV2 | dQ at the head of the workspace
 int sm100_tdp_bwd_sums(const TdpArgs& a);
-// The contributions of the first `queries` rows of the shard (queries below 32, causal, head dimension 64 or 128, 16-bit)
+constexpr int kTdpFirstQueries = 16;
+// The contributions of the first `queries` rows of the shard (queries below kTdpFirstQueries, causal, head dimension 64 or 128, 16-bit)
 // in exact fp32, added to the fp32 sums dK1 | dK2 | dSiLU(V1) | dV2; their dQ rows are stored to the fifth tensor.
 int tdp_bwd_first_queries(const TdpArgs& a, int queries, float* sums, const float* drow);
 // The backward of a query shard by the kernel that steps over queries: dQ rows stored, fp32 sums at the head of the

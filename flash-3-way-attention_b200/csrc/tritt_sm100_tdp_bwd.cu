@@ -133,7 +133,8 @@ struct BwdItem {
   int ea, eb;                       // A and A' carry factors 2^ea and 2^eb (range_shift)
 };
 enum {
-  kFirstOfQ = 1, kLastOfQ = 2   // the first / last item of a run over the j-tiles of one q-tile
+  kFirstOfQ = 1, kLastOfQ = 2,   // the first / last item of a run over the j-tiles of one q-tile
+  kShiftBits = 8                 // (flags >> kShiftBits: dS carries a factor 2^that, beside P's)
 };
 constexpr int kItemSlots = 4;               // (an item is read before its successor but one is written)
 
@@ -211,8 +212,9 @@ struct BwdWalk {
 // fp16 only: the recomputed probabilities of a query that attends n pairs are ~1/n, which for late rows lies below
 // fp16's normal range (6e-5; 1/n = 2e-7 at q = 2048).  P and dS are therefore formed times 2^e, e = min(10, log2 of the
 // attended pairs' count bound), and the folds divide it out.  2^10 keeps a probability of 1 times a dP - Dq below 63
-// finite.  One e per q-tile, since G and U sum over its queries: that of the first query the kernel takes there, which
-// has the fewest pairs (without windows e = 10 everywhere, as the exact first queries leave none below 1089 pairs).
+// finite (dS has a further power of two where dP is small: ds_shift).  One e per q-tile, since G and U sum over its queries:
+// that of the first query the kernel takes there, which has the fewest pairs (without windows 8 in the first tile, as the
+// exact first queries leave none below 289 pairs, and 10 in the others).
 // bf16 has fp32's exponent range: e = 0.
 template <typename T16>
 __device__ __forceinline__ int prob_shift(int q, int causal, int T, int k1w, int k2w) {
@@ -230,7 +232,18 @@ __device__ __forceinline__ int prob_shift(int q, int causal, int T, int k1w, int
 template <typename T16> __device__ __forceinline__ int range_shift(float bound) {
   if constexpr (std::is_same<T16, __half>::value) {
     if (!(bound > 0.f) || !isfinite(bound)) return 0;
-    return min(100, max(-100, 14 - ((__float_as_int(bound) >> 23) - 127)));
+    return min(80, max(-80, 14 - ((__float_as_int(bound) >> 23) - 127)));
+  }
+  return 0;
+}
+
+// fp16 only: the further power of two of dS = P (dP - Dq), from a bound on |dP|, which holds for |Dq| (a mean of dP) as well:
+// with P's 2^10 the product stays below 2^15.  0 where the bound leaves no room, that is from 8 on (as a bound it is far above
+// what occurs: values of order 1 run without it).
+template <typename T16> __device__ __forceinline__ int ds_shift(float bound) {
+  if constexpr (std::is_same<T16, __half>::value) {
+    if (!(bound > 0.f) || !isfinite(bound)) return 0;
+    return min(24, max(0, 3 - ((__float_as_int(bound) >> 23) - 127)));
   }
   return 0;
 }
@@ -250,20 +263,20 @@ __device__ __forceinline__ void red_add4(float* p, float a, float b, float c, fl
 // The statistics of a head over its parts, in every lane (zeros without them).
 struct BwdStats {
   float qk1, k2, sv1, v2;    // largest element of Q and K1, of K2, SiLU(V1), V2
-  float k1_row, q_row;       // largest squared norm of a row
+  float k1_row, q_row, do_row, sv1_row;   // largest squared norm of a row
 };
 __device__ __forceinline__ BwdStats head_stats(const BwdParams& p, int bh, int lane) {
-  float m[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  float m[kStatFloats] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (p.stats && lane < p.stat_parts) {
     const float4* src = reinterpret_cast<const float4*>(p.stats + ((size_t)bh * p.stat_parts + lane) * kStatFloats);
     const float4 x = __ldg(src), y = __ldg(src + 1);
-    m[0] = x.x; m[1] = x.y; m[2] = x.z; m[3] = x.w; m[4] = y.x; m[5] = y.y;
+    m[0] = x.x; m[1] = x.y; m[2] = x.z; m[3] = x.w; m[4] = y.x; m[5] = y.y; m[6] = y.z; m[7] = y.w;
   }
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1)
 #pragma unroll
-    for (int i = 0; i < 6; ++i) m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], o));
-  return BwdStats{m[0], m[1], m[2], m[3], m[4], m[5]};
+    for (int i = 0; i < kStatFloats; ++i) m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], o));
+  return BwdStats{m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7]};
 }
 
 // Whether a head of this CTA's part may have large scores (the same for every thread; without statistics: yes).
@@ -380,8 +393,9 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
         // (a row that is not this kernel's has P = 0 and a zero row of Q and dO, and needs Dq = 0 as well: 0 * (dP - Dq)
         // of another query's infinite or NaN Dq would be NaN, which G sums into every key the tile meets)
         lse2 = q_ok ? __ldg(p.lse + (size_t)it.bh * T + q) * kLog2e - (float)e : 0.f;
-        drow = q_ok ? __ldg(p.drow + (size_t)it.bh * T + q) : 0.f;
-        dq_scale = pow2i(-e - it.ea) * kLn2;    // A carries alpha * log2(e)
+        const int f = it.flags >> kShiftBits;
+        drow = q_ok ? __ldg(p.drow + (size_t)it.bh * T + q) * pow2i(f) : 0.f;
+        dq_scale = pow2i(-e - it.ea - f) * kLn2;    // A carries alpha * log2(e)
         // A query that attends a single pair has P = 1 and a score gradient of exactly zero (TdpMask::single_pair):
         // P (dP - Dq) has two terms that are equal only up to the 16-bit rounding of the stored output, so its dS
         // is set to zero.
@@ -410,7 +424,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       }
       const bool any_single = __any_sync(0xffffffffu, single);
       const float2 nlse = make_float2(-lse2, -lse2), ndq = make_float2(-drow, -drow);
-      const float sa = kShifted ? pow2i(-it.ea) : 1.f, sb = kShifted ? pow2i(-it.eb) : 1.f;
+      const float sa = kShifted ? pow2i(-it.ea) : 1.f, sb = kShifted ? pow2i((it.flags >> kShiftBits) - it.eb) : 1.f;
       // v * scale + add; the scale of bf16 is 1
       auto scaled = [](uint32_t v0, uint32_t v1, float scale, float2 add) {
         const float2 v = make_float2(__uint_as_float(v0), __uint_as_float(v1));
@@ -574,7 +588,8 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       const int len = it.len;
       const int e = prob_shift<T16>(g.q_rem + max(it.qt * 128, p.i_first) * g.q_mod, g.causal, T, g.k1w, g.k2w);
       const float unshift = pow2i(-e);
-      const float zscale = role ? unshift : unshift * p.alpha;
+      const float unshift_ds = unshift * pow2i(-(it.flags >> kShiftBits));
+      const float zscale = role ? unshift : unshift_ds * p.alpha;
       float* zrow = (role ? p.dv2 : p.dk2) + ((size_t)it.bh * T + it.k0) * D;
       auto form = [&](int i) -> bool {
         const uint32_t m = n + i;
@@ -753,7 +768,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       ++items;
       // ---- dK1 / dSiLU(V1) of this item
       // (the K2 rows carry alpha * log2(e) * 2^ea, the V2 rows 2^eb)
-      const float jscale = role ? unshift * pow2i(-it.eb) : unshift * pow2i(-it.ea) * kLn2;
+      const float jscale = role ? unshift * pow2i(-it.eb) : unshift_ds * pow2i(-it.ea) * kLn2;
       float* const base = (role ? p.dsv1 : p.dk1) + (size_t)it.bh * T * D;
 #pragma unroll
       for (int c16 = 0; c16 < 4; ++c16)
@@ -903,7 +918,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       tma_prefetch_desc(&tmSV1);
     }
     float scale_k = p.alpha * kLog2e, scale_v = 1.f;   // of the K2 and V2 rows, with the head's powers of two
-    int bh = -1, ea = 0, eb = 0;
+    int bh = -1, ea = 0, eb = 0, f = 0;
     constexpr int kChunks = kVecBatch * D / 8 / 32;   // 16-byte pieces of K2 (and of V2) per lane and batch
     float* const vec = reinterpret_cast<float*>(smem + Cfg::kOffVec);
     uint32_t items = 0, vb = 0;
@@ -917,11 +932,13 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
         const BwdStats st = head_stats(p, bh, lane);
         ea = range_shift<T16>(fabsf(p.alpha * kLog2e) * st.qk1 * st.k2);
         eb = range_shift<T16>(st.sv1 * st.v2);
+        f = ds_shift<T16>(sqrtf(st.do_row * st.sv1_row) * st.v2);
         scale_k = p.alpha * kLog2e * pow2i(ea);
         scale_v = pow2i(eb);
       }
       it.ea = ea;
       it.eb = eb;
+      it.flags |= f << kShiftBits;
       alive = wait_all(&bars.tile_free, (items & 1) ^ 1);
       if (!alive) break;
       if (leader) bars.items[items % kItemSlots] = it;
@@ -1075,10 +1092,10 @@ tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, co
                        const T16* __restrict__ q, const T16* __restrict__ k1, const T16* __restrict__ k2,
                        const T16* __restrict__ v2, float* __restrict__ sums, T16* __restrict__ sv1, float* __restrict__ drow, float* __restrict__ stats,
                        size_t n, int head_elems, int D, int parts) {
-  __shared__ float wmax[kPrepThreads / 32][6];
+  __shared__ float wmax[kPrepThreads / 32][kStatFloats];
   const int bh = blockIdx.x / parts, part = blockIdx.x % parts, lanes = D / 8;   // 8 or 16 lanes hold one row
   const uint32_t row_lanes = ((1u << lanes) - 1u) << ((threadIdx.x & 31) / lanes * lanes);
-  float qk1_max = 0.f, k2_max = 0.f, sv1_max = 0.f, v2_max = 0.f, k1_row = 0.f, q_row = 0.f;
+  float qk1_max = 0.f, k2_max = 0.f, sv1_max = 0.f, v2_max = 0.f, k1_row = 0.f, q_row = 0.f, do_row = 0.f, sv1_row = 0.f;
   auto words = [](const T16* p, uint32_t (&w)[4]) {
     const uint4 x = *reinterpret_cast<const uint4*>(p);
     w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
@@ -1096,14 +1113,17 @@ tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, co
     words(v1 + i, wv);
     words(o + i, wa);
     words(d_o + i, wb);
-    float dot = 0.f;
+    float dot = 0.f, nd = 0.f, ns = 0.f;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float2 f = unpack2<T16>(wv[e]), x = unpack2<T16>(wa[e]), y = unpack2<T16>(wb[e]);
       const float2 g = make_float2(silu_f(f.x), silu_f(f.y));
       r[e] = pack2<T16>(g.x, g.y);
       dot = fmaf(x.x, y.x, fmaf(x.y, y.y, dot));
-      grow(sv1_max, unpack2<T16>(r[e]));
+      const float2 g16 = unpack2<T16>(r[e]);
+      grow(sv1_max, g16);
+      ns = fmaf(g16.x, g16.x, fmaf(g16.y, g16.y, ns));
+      nd = fmaf(y.x, y.x, fmaf(y.y, y.y, nd));
     }
     *reinterpret_cast<uint4*>(sv1 + i) = make_uint4(r[0], r[1], r[2], r[3]);
     for (int s = lanes / 2; s >= 1; s >>= 1) dot += __shfl_xor_sync(row_lanes, dot, s);
@@ -1130,25 +1150,28 @@ tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, co
       for (int s = lanes / 2; s >= 1; s >>= 1) {
         n1 += __shfl_xor_sync(row_lanes, n1, s);
         nq += __shfl_xor_sync(row_lanes, nq, s);
+        nd += __shfl_xor_sync(row_lanes, nd, s);
+        ns += __shfl_xor_sync(row_lanes, ns, s);
       }
+      do_row = fmaxf(do_row, nd);
+      sv1_row = fmaxf(sv1_row, ns);
       k1_row = fmaxf(k1_row, n1);
       q_row = fmaxf(q_row, nq);
     }
   }
   if (!stats) return;
-  float w[6] = {qk1_max, k2_max, sv1_max, v2_max, k1_row, q_row};
+  float w[kStatFloats] = {qk1_max, k2_max, sv1_max, v2_max, k1_row, q_row, do_row, sv1_row};
 #pragma unroll
   for (int o2 = 16; o2 >= 1; o2 >>= 1)
 #pragma unroll
-    for (int i = 0; i < 6; ++i) w[i] = fmaxf(w[i], __shfl_xor_sync(0xffffffffu, w[i], o2));
+    for (int i = 0; i < kStatFloats; ++i) w[i] = fmaxf(w[i], __shfl_xor_sync(0xffffffffu, w[i], o2));
   if ((threadIdx.x & 31) == 0) {
 #pragma unroll
-    for (int i = 0; i < 6; ++i) wmax[threadIdx.x >> 5][i] = w[i];
+    for (int i = 0; i < kStatFloats; ++i) wmax[threadIdx.x >> 5][i] = w[i];
   }
   __syncthreads();
   if (threadIdx.x < kStatFloats) {
     float x = 0.f;
-    if (threadIdx.x < 6)
 #pragma unroll
       for (int i = 0; i < kPrepThreads / 32; ++i) x = fmaxf(x, wmax[i][threadIdx.x]);
     stats[(size_t)blockIdx.x * kStatFloats + threadIdx.x] = x;
@@ -1214,13 +1237,13 @@ int check_kernel_registers(K kern) {
 
 // The first queries of a causal call run in exact fp32 on the CUDA cores.  Their gradients are the largest by far (a query
 // attends ~q^2 pairs: its dQ falls like 1/q, and so does what it adds to the first key rows), so their rounding is most of
-// the error of the whole result; and with few pairs each, their probabilities are where it shows that S is formed from
-// another rounded product here (K1 K2) than in the forward (Q K2): P no longer sums to one.  From query 32 on (1089 pairs
-// without windows) the roundings of the pairs average out.  They are a vanishing part of the work: the error of a
-// training step against fp64 goes from 3.6e-3 to 2.6e-3 at T=2048 in bf16.
-// (Queries 0 to 31 themselves, not the first 32 rows of a shard: 8 interleaved shards have queries up to 248 among those,
-// with 60 times the pairs, and at 64 shards and T=2048 they are the whole shard.)
-constexpr int kFirstQueries = 32;
+// the error of the whole result; and in fp16 the first query of a tile sets the tile's range shift (prob_shift).  They are
+// a vanishing part of the work: a training step's error against fp64 goes from 3.6e-3 to 2.6e-3 at T=2048 in bf16.  16 of
+// them: with 32 the error is 2 to 10 % lower still, at eight times the pairs and atomics (160 heads of T=70: 305 against
+// 237 us a call, 204 without any; 4 heads of T=333 D=128: 201, 195, 179).
+// (Queries 0 to 15 themselves, not the first 16 rows of a shard: 8 interleaved shards have queries up to 127 among those, with
+// 60 times the pairs, and at 64 shards and T=1024 they are the whole shard.)
+constexpr int kFirstQueries = kTdpFirstQueries;
 
 // What a call does, from its arguments alone.
 struct BwdPlan {

@@ -1,21 +1,22 @@
 // The first queries of a causal triple-dot-product backward, in exact fp32 on the CUDA cores: what they add to the sums
 // dK1 | dK2 | dSiLU(V1) | dV2, and their dQ.  (Why they are not the tensor-core kernel's: see kFirstQueries there.)
 //
-// One CTA per (head, query); a query q < 32 attends keys 0 .. q, at most 32 x 32 pairs, so everything it needs stays in
+// One CTA per (head, query); a query q < 16 attends keys 0 .. q, at most 16 x 16 pairs, so everything it needs stays in
 // shared memory.  With the rows A[k] = alpha log2(e) Q K2[k] and B[k] = dO V2[k]:
 //     S[k,j] = A[k] . K1[j]     P = exp2(S - lse2)      dP[k,j] = B[k] . SiLU(V1)[j]     dS = P (dP - Dq)
 //     F = dS K1:    dK2[k] += alpha Q F[k],   dQ = alpha sum_k K2[k] F[k]        W = P SiLU(V1):  dV2[k] += dO W[k]
 //     G = dS^T A:   dK1[j] += ln(2) G[j]                                         U = P^T B:       dSV1[j] += U[j]
-// It is latency that counts (it runs ahead of the tensor-core kernel): 12.5 us at 4 heads, D=128 and 18 us at 16 heads,
-// D=64 (where the reductions of 32 queries into the same 32 rows show), against 60 and 50 us of the general CUDA-core
-// kernel, which walks a query's rows one tile after the other.
+// It is latency that counts (it runs ahead of the tensor-core kernel), so every query has a CTA, which adds its share to the
+// sums: about 8 us at 4 heads, D=128 and at 16 heads, D=64.  (The general CUDA-core kernel, which walks a query's rows one
+// tile after the other, took 60 and 50 us for twice as many queries, this one 12.5 and 18 us for those.)
 #include "tritt_common.cuh"
 #include "tritt_sm100_tdp.cuh"
 
 namespace tritt {
 namespace {
 
-constexpr int kFirst = 32, kFirstThreads = 256;
+constexpr int kFirst = kTdpFirstQueries, kFirstThreads = 256;
+static_assert(kFirst * kFirst == kFirstThreads, "one pair per thread");
 
 template <int D> struct FirstShared {
   static constexpr int kPitch = D + 4;   // (rows 4 banks apart: 8 lanes' 16-byte reads of 8 rows do not conflict)
@@ -91,37 +92,28 @@ __global__ void __launch_bounds__(kFirstThreads) tdp_bwd_first_kernel(const __gr
     store8(&sh.b[row][h], f);
   }
   __syncthreads();
-  // ---- P and dS: lane = key j, four keys k per warp
+  // ---- P and dS: one pair per thread
   {
-    const int j = tid & 31, k0 = (tid >> 5) * 4;
+    const int j = tid % kFirst, k = tid / kFirst;
     const float lse2 = __ldg(p.lse + (size_t)bh * p.T + q) * kLog2e, Dq = __ldg(p.drow + (size_t)bh * p.T + q);
-    const bool single = p.mask.single_pair(q);   // (its score gradient is exactly zero)
-    if (k0 < nk) {
-      float s[4] = {0.f, 0.f, 0.f, 0.f}, dp[4] = {0.f, 0.f, 0.f, 0.f};
-      const int jr = min(j, q);
-#pragma unroll 4
+    float pr = 0.f, ds = 0.f;
+    if (p.mask.valid(q, j, k)) {
+      float s = 0.f, dp = 0.f;
+#pragma unroll 8
       for (int h = 0; h < D; h += 4) {
-        const float4 x = *reinterpret_cast<const float4*>(&sh.k1[jr][h]), y = *reinterpret_cast<const float4*>(&sh.s1[jr][h]);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int k = min(k0 + e, q);
-          s[e] = dot4(x, *reinterpret_cast<const float4*>(&sh.a[k][h]), s[e]);
-          dp[e] = dot4(y, *reinterpret_cast<const float4*>(&sh.b[k][h]), dp[e]);
-        }
+        s = dot4(*reinterpret_cast<const float4*>(&sh.k1[j][h]), *reinterpret_cast<const float4*>(&sh.a[k][h]), s);
+        dp = dot4(*reinterpret_cast<const float4*>(&sh.s1[j][h]), *reinterpret_cast<const float4*>(&sh.b[k][h]), dp);
       }
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int k = k0 + e;
-        const float pr = p.mask.valid(q, j, k) ? exp2f(s[e] - lse2) : 0.f;
-        const float ds = pr != 0.f && !single ? pr * (dp[e] - Dq) : 0.f;
-        sh.p_kj[k][j] = sh.p_jk[j][k] = pr;
-        sh.ds_kj[k][j] = sh.ds_jk[j][k] = ds;
-      }
+      pr = exp2f(s - lse2);
+      // (a query with a single pair has a score gradient of exactly zero)
+      if (pr != 0.f && !p.mask.single_pair(q)) ds = pr * (dp - Dq);
     }
+    sh.p_kj[k][j] = sh.p_jk[j][k] = pr;
+    sh.ds_kj[k][j] = sh.ds_jk[j][k] = ds;
   }
   __syncthreads();
   // ---- the four products: 4 columns h of R rows per thread
-  constexpr int kChunks = D / 4, kGroups = kFirstThreads / kChunks, R = kFirst / kGroups;   // D=128: 8 groups of 4, 64: 16 of 2
+  constexpr int kChunks = D / 4, kGroups = kFirstThreads / kChunks, R = kFirst / kGroups;   // D=128: 8 groups of 2, 64: 16 of 1
   const int h = tid % kChunks * 4, r0 = tid / kChunks * R;
   float4 dq = make_float4(0.f, 0.f, 0.f, 0.f);
   if (r0 < nk) {
