@@ -9,13 +9,15 @@
 //   warp 0      TMA producer: the row operand once, then a ring of key and value tiles
 //   warp 1      issues tcgen05.mma:  S = X * Kc^T  (128x128 fp32 in TMEM)  and  acc += P * Vc  with P read from
 //               TMEM (16-bit, over the columns of S already consumed) and the value tile used row-major
-//   warps 4-7, 8-11   two soft-max warpgroups, one row per thread, that take the column tiles in turn, each with scores,
-//               maximum, sum and accumulator of its own: scale, bias and mask, row maximum, exp2 with lazy rescaling of
-//               the accumulator, P written back to TMEM; at the end the two halves of a row are merged, normalised and
-//               stored (fp32 and / or 16-bit, and optionally the 16-bit product with a second tensor, which is the outer
-//               leg's value operand)
-// The chain S -> soft-max -> P*V of one warpgroup is serial and bounds the kernel (8 tiles at T = 1024, ~3 us each); the
-// other's runs beside it.
+//   warps 4-7, 8-11   one or two soft-max warpgroups (NG), one row per thread, that take the column tiles in turn, each
+//               with scores, maximum, sum and accumulator of its own: scale, bias and mask, row maximum, exp2 with lazy
+//               rescaling of the accumulator, P written back to TMEM; at the end the halves of a row are merged, normalised
+//               and stored (fp32 and / or 16-bit, and optionally the 16-bit product with a second tensor, which is the
+//               outer leg's value operand)
+// The chain S -> soft-max -> P*V of one warpgroup is serial and bounds the kernel (8 tiles at T = 1024, ~3 us each).  With
+// two warpgroups the other's runs beside it, on the tiles of the same rows: shorter for a launch that leaves SMs idle.  One
+// warpgroup needs half of the tensor memory, so that at head dimension 64 two CTAs share an SM, with a producer, an issuer
+// and an epilogue each: more for a launch that fills the chip (see launch_attn_fwd).
 #include "tritt_common.cuh"
 #include "tritt_sm100.cuh"
 #include "tritt_sm100_tdp.cuh"
@@ -26,20 +28,20 @@ namespace tritt {
 namespace {
 using namespace sm100;
 
-constexpr int kAttnThreads = 384;
+template <int NG> constexpr int kAttnThreads = 128 + 128 * NG;
 constexpr float kAttnRescaleGap = 8.f;  // rescale the accumulator only when the row max grew by more than 2^8
 
-template <int D> struct AttnCfg {
+template <int D, int NG> struct AttnCfg {
   static constexpr int kTile = 128 * D * 2;   // bytes of one 128-row operand tile
-  static constexpr int kStages = D == 64 ? 8 : 5;   // key and value tiles in turn: K(0), V(0), K(1), V(1), ...
+  static constexpr int kStages = NG == 1 ? 4 : D == 64 ? 8 : 5;   // key and value tiles in turn: K(0), V(0), K(1), V(1), ...
   static constexpr int kOffX = 0;
   static constexpr int kOffRing = kTile;
-  static constexpr int kOffBias = kOffRing + kStages * kTile;  // [8 warps][128] fp32, log2 units
-  static constexpr int kOffMl = kOffBias + 8 * 128 * 4;        // [2 warpgroups][128][2] fp32: row maximum, row sum
-  static constexpr int kOffBars = kOffMl + 2 * 128 * 2 * 4;
+  static constexpr int kOffBias = kOffRing + kStages * kTile;  // [4 NG warps][128] fp32, log2 units
+  static constexpr int kOffMl = kOffBias + 4 * NG * 128 * 4;   // [NG warpgroups][128][2] fp32: row maximum, row sum
+  static constexpr int kOffBars = kOffMl + NG * 128 * 2 * 4;
   static constexpr int kSmem = kOffBars + 256;
-  static constexpr int kTmemO = 256;          // S_0 | S_1 | acc_0 | acc_1
-  static constexpr int kTmemCols = 512;
+  static constexpr int kTmemO = 128 * NG;     // S_0 | S_1 | acc_0 | acc_1
+  static constexpr int kTmemCols = 256 * NG;
 };
 
 struct AttnFwdParams {
@@ -61,11 +63,11 @@ struct AttnBarriers {
   int abort_flag;
 };
 
-template <int D, typename T16>
-__global__ void __launch_bounds__(kAttnThreads, 1)
+template <int D, typename T16, int NG>
+__global__ void __launch_bounds__(kAttnThreads<NG>, D == 64 && NG == 1 ? 2 : 1)
 attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, AttnFwdParams p) {
-  using Cfg = AttnCfg<D>;
+  using Cfg = AttnCfg<D, NG>;
   constexpr int NS = Cfg::kStages;
   constexpr int KH = D / 64;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -88,7 +90,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       mbar_init(&bars.p_ready[g], 128);
     }
     mbar_init(&bars.o_done, 1);
-    mbar_init(&bars.ml_ready, 256);
+    mbar_init(&bars.ml_ready, 128 * NG);
     fence_barrier_init();
   }
   if (warp == 0) {
@@ -167,7 +169,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       const uint32_t xLo = desc_lo(smem_u32(smem + Cfg::kOffX), 16);
       bool alive = true;
       auto wait_stage = [&](int pos) { return wait_all(&bars.ring_full[pos % NS], (pos / NS) & 1); };
-      // S_{i % 2} = X K(i)^T
+      // S_{i % NG} = X K(i)^T
       auto issue_s = [&](int i) {
         const int pos = 2 * i;
         if (!wait_stage(pos)) return false;
@@ -176,13 +178,13 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t kk = (k >> 2) * (16384 >> 4) + (k & 3) * 2;
-          if (leader) mma_ss_lo(tmem + (i & 1) * 128, xLo + kk, bLo + kk, kHi, idesc_s, k > 0);
+          if (leader) mma_ss_lo(tmem + (i % NG) * 128, xLo + kk, bLo + kk, kHi, idesc_s, k > 0);
         }
-        commit(&bars.s_ready[i & 1]);
+        commit(&bars.s_ready[i % NG]);
         commit(&bars.ring_empty[pos % NS]);
         return true;
       };
-      // acc_{i % 2} (+)= P(i) V(i); the value tile is used row-major: 64-column blocks 16 KiB apart, 16 rows (one
+      // acc_{i % NG} (+)= P(i) V(i); the value tile is used row-major: 64-column blocks 16 KiB apart, 16 rows (one
       // instruction) 2 KiB apart
       auto issue_pv = [&](int i) {
         const int pos = 2 * i + 1;
@@ -192,25 +194,25 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
 #pragma unroll
         for (int k = 0; k < 8; ++k)
           if (leader)
-            mma_ts_lo(tmem + Cfg::kTmemO + (i & 1) * D, tmem + (i & 1) * 128 + k * 8, bLo + k * (2048 >> 4), kHi, idesc_pv,
-                      k > 0 || i > 1);
+            mma_ts_lo(tmem + Cfg::kTmemO + (i % NG) * D, tmem + (i % NG) * 128 + k * 8, bLo + k * (2048 >> 4), kHi, idesc_pv,
+                      k > 0 || i >= NG);
         commit(&bars.ring_empty[pos % NS]);
         return true;
       };
-      alive = wait_all(&bars.x_full, 0) && issue_s(0) && (n_ct < 2 || issue_s(1));
+      alive = wait_all(&bars.x_full, 0) && issue_s(0) && (NG == 1 || n_ct < 2 || issue_s(1));
       for (int i = 0; i < n_ct && alive; ++i) {
-        alive = wait_all(&bars.p_ready[i & 1], (i >> 1) & 1);
+        alive = wait_all(&bars.p_ready[i % NG], (i / NG) & 1);
         if (!alive) break;
         tc_fence_after();
-        // (S(i + 2) overwrites P(i): the pipe runs it after P(i) V(i))
-        alive = issue_pv(i) && (i + 2 >= n_ct || issue_s(i + 2));
+        // (S(i + NG) overwrites P(i): the pipe runs it after P(i) V(i))
+        alive = issue_pv(i) && (i + NG >= n_ct || issue_s(i + NG));
       }
       if (alive) commit(&bars.o_done);
     }
   } else if (warp >= 4) {
     // ------------------------------------------------------------------ soft-max and epilogue, one row per thread
-    // Warpgroup g takes the column tiles g, g + 2, ... with a running maximum, sum and accumulator of its own: while one
-    // is in its exponentials the other's products run, and a row's two halves meet in the epilogue.
+    // Warpgroup g takes the column tiles g, g + NG, ... with a running maximum, sum and accumulator of its own: while one
+    // is in its exponentials the other's products run, and a row's halves meet in the epilogue.
     const int wg = (warp - 4) >> 2, wq = warp & 3;
     const int row = wq * 32 + lane;
     const int r = r0 + row;
@@ -223,7 +225,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     const int c_lo = (p.causal && p.win < T) ? max(0, r - p.win) : 0;
     float m_used = -INFINITY, l_sum = 0.f;
     bool alive = true;
-    for (int i = wg; i < n_ct; i += 2) {
+    for (int i = wg; i < n_ct; i += NG) {
       const int c0 = (ct0 + i) * 128;
       // this tile's column biases (log2 units), staged per warp so that no hand-off between warps is needed
       __syncwarp();   // every lane is done with the previous tile's
@@ -233,7 +235,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
         sb[lane * 4 + e] = (p.bias && c < T) ? __ldg(p.bias + (size_t)bh * T + c) * kLog2e : 0.f;
       }
       __syncwarp();
-      alive = __all_sync(0xffffffffu, mbar_wait(&bars.s_ready[wg], (i >> 1) & 1, abort_flag));
+      alive = __all_sync(0xffffffffu, mbar_wait(&bars.s_ready[wg], (i / NG) & 1, abort_flag));
       if (!alive) break;
       tc_fence_after();
       const int lo = c_lo - c0, hi = c_hi - c0;
@@ -263,7 +265,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
             if (c >= l2 && c <= h2) mx = fmaxf(mx, fmaf(__uint_as_float(sr[c]), p.scale2, sb[hf * 64 + c]));
         }
       }
-      if (i < 2) {
+      if (i < NG) {
         m_used = mx;  // nothing accumulated yet
       } else {
         const bool grow = mx > m_used + kAttnRescaleGap;
@@ -326,29 +328,38 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
       mbar_arrive(&bars.p_ready[wg]);
     }
     float2* ml = reinterpret_cast<float2*>(smem + Cfg::kOffMl);
-    ml[wg * 128 + row] = make_float2(m_used, l_sum);
-    mbar_arrive(&bars.ml_ready);
-    if (alive) alive = __all_sync(0xffffffffu, mbar_wait(&bars.ml_ready, 0, abort_flag));
+    if constexpr (NG == 2) {
+      ml[wg * 128 + row] = make_float2(m_used, l_sum);
+      mbar_arrive(&bars.ml_ready);
+    }
+    if (NG == 2 && alive) alive = __all_sync(0xffffffffu, mbar_wait(&bars.ml_ready, 0, abort_flag));
     if (alive) alive = __all_sync(0xffffffffu, mbar_wait(&bars.o_done, 0, abort_flag));
     if (alive) {
       tc_fence_after();
-      // the row's two halves on their common maximum (a half without an attended column has maximum -inf and weight 0)
-      const float2 ml0 = ml[row], ml1 = ml[128 + row];
-      const float m = fmaxf(ml0.x, ml1.x), w0 = exp2f(ml0.x - m), w1 = exp2f(ml1.x - m);
-      const float l = ml0.y * w0 + ml1.y * w1, inv = 1.f / l;
-      const float f0 = w0 * inv, f1 = w1 * inv;
+      // the row's halves on their common maximum (a half without an attended column has maximum -inf and weight 0)
+      float m = m_used, l = l_sum, f0 = 1.f, f1 = 0.f;
+      if constexpr (NG == 2) {
+        const float2 ml0 = ml[row], ml1 = ml[128 + row];
+        m = fmaxf(ml0.x, ml1.x);
+        f0 = exp2f(ml0.x - m);
+        f1 = exp2f(ml1.x - m);
+        l = ml0.y * f0 + ml1.y * f1;
+      }
+      const float inv = 1.f / l;
+      f0 *= inv;
+      f1 *= inv;
       const bool in_range = r < T;
       const size_t off = ((size_t)bh * T + r) * D;
 #pragma unroll
-      for (int ch2 = 0; ch2 < D / 64; ++ch2) {
-        const int ch = wg * (D / 64) + ch2;   // half of the output columns per warpgroup
+      for (int ch2 = 0; ch2 < D / 32 / NG; ++ch2) {
+        const int ch = wg * (D / 32 / NG) + ch2;   // (half of the output columns per warpgroup where there are two)
         uint32_t o[32];
         float v[32];
         tmem_ld32(tmem + lane_base + Cfg::kTmemO + ch * 32, o);
         tmem_wait_ld();
 #pragma unroll
         for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(o[e]) * f0;
-        if (n_ct > 1) {
+        if (NG == 2 && n_ct > 1) {
           tmem_ld32(tmem + lane_base + Cfg::kTmemO + D + ch * 32, o);
           tmem_wait_ld();
 #pragma unroll
@@ -390,9 +401,9 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
   if (tid == 0 && bars.abort_flag && p.status) atomicOr(p.status, 16);
 }
 
-template <int D, typename T16>
-int launch_attn_fwd(const AttnTcArgs& a) {
-  using Cfg = AttnCfg<D>;
+template <int D, typename T16, int NG>
+int launch_attn_fwd_ng(const AttnTcArgs& a) {
+  using Cfg = AttnCfg<D, NG>;
   CUtensorMap tmX, tmK, tmV;
   int rc;
   if ((rc = make_tmap_3d(&tmX, a.xq, 2, D, a.T, a.BN, 64, 128))) return rc;
@@ -410,13 +421,24 @@ int launch_attn_fwd(const AttnTcArgs& a) {
   p.win = a.win < 0 ? 0 : a.win;
   p.scale2 = a.alpha * kLog2e;
   p.status = a.status;
-  auto kern = attn_fwd_sm100_kernel<D, T16>;
+  auto kern = attn_fwd_sm100_kernel<D, T16, NG>;
   TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
   const dim3 grid((a.T + 127) / 128, a.BN);
-  kern<<<grid, kAttnThreads, Cfg::kSmem, a.stream>>>(tmX, tmK, tmV, p);
+  kern<<<grid, kAttnThreads<NG>, Cfg::kSmem, a.stream>>>(tmX, tmK, tmV, p);
   count_launch();
   TRITT_CUDA_OK(cudaGetLastError());
   return 0;
+}
+
+// One warpgroup where the launch has a CTA for every place that it makes: two an SM at head dimension 64, and at 128, where
+// it makes none, only for a single column tile, which two warpgroups cannot share.  us per dot-product-sum forward, one / two
+// warpgroups: D=64: 600 heads of T=64 45.5 / 66, of T=300 193 / 242, 128 heads of T=2048 447 / 507, 37 of T=1024 (296
+// CTAs) 63 / 70, but 16 of T=2048 (256) 102 / 95, of T=1024 52 / 39;  D=128: 600 heads of T=128 109 / 117, 128 of T=300 88 / 80.
+template <int D, typename T16>
+int launch_attn_fwd(const AttnTcArgs& a) {
+  const long tiles = (a.T + 127) / 128, ctas = tiles * a.BN;
+  if (ctas >= 2 * num_sms() && (D == 64 || tiles == 1)) return launch_attn_fwd_ng<D, T16, 1>(a);
+  return launch_attn_fwd_ng<D, T16, 2>(a);
 }
 
 }  // namespace

@@ -146,3 +146,26 @@ def test_backward_with_the_forward_workspace_equals_the_recomputing_backward(dty
     assert _native.read_status(torch.device(DEV)) == 0
     for name, x, y in zip(("dq", "dk1", "dk2", "dv1", "dv2"), a, b):
         assert torch.equal(x, y), name
+
+
+@pytest.mark.parametrize("N,T,D,k_diff,causal", [(300, 128, 64, 128, True), (160, 130, 64, 40, True), (100, 300, 64, 300, False),
+                                                 (301, 70, 128, 70, True)])
+def test_forward_of_many_heads_matches_that_of_few(N, T, D, k_diff, causal):
+    """From two CTAs per SM on, the forward runs one soft-max warpgroup per CTA (head dimension 64, or one column tile):
+    the same attention as with two, whose rows are summed in two halves."""
+    ins = orc.make_inputs(1, N, T, D, scale=0.5, seed=N + T, dtype=torch.float16)
+    t = [x.to(DEV) for x in ins[:5]]
+    many, few = [], []
+    for heads in (slice(0, N), slice(0, 3)):
+        x = [y[:, heads].contiguous() for y in t]
+        o, m = torch.empty_like(x[0]), torch.empty(x[0].shape[:3], device=DEV)
+        _native.dps_fwd(*x, o, m, 1 / D, causal, k_diff)
+        (few if heads.stop == 3 else many).extend((o, m))
+    torch.cuda.synchronize()
+    assert _native.read_status(torch.device(DEV)) == 0
+    z, lse = orc.dps_forward(*(x[:, N - 2:].float() for x in ins[:5]), 1 / D, causal, k_diff)
+    assert_close("o", many[0][:, N - 2:].cpu(), z, torch.float16)
+    assert float((many[1][:, N - 2:].cpu() - lse).abs().max()) <= 5e-3
+    # (16-bit probabilities against another running maximum: half a unit in the last place of P and of the output)
+    assert_close("o (many heads against few)", many[0][:, :3], few[0], torch.float16, scale=0.25)
+    assert float((many[1][:, :3] - few[1]).abs().max()) <= 1e-5
