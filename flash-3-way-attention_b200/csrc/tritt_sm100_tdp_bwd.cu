@@ -1068,6 +1068,8 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
   tc_fence_before();
   __syncthreads();
   if (warp == 16) tmem_dealloc(tmem, 512);
+  // what comes after this kernel also reads what the exact first queries, which may still be running, add to the sums
+  if (tid == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
   if (tid == 0 && bars.abort_flag && p.status) atomicOr(p.status, 4);
 }
 
@@ -1341,9 +1343,21 @@ int launch_bwd_sums(const TdpArgs& a, const BwdPlan& plan) {
   auto kern = tdp_bwd_kernel<D, T16>;
   if ((rc = check_kernel_registers<D, T16>(kern))) return rc;
   TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
-  kern<<<grid, kBwdThreads, Cfg::kSmem, a.stream>>>(tmQ, tmDO, tmK1, tmSV1, p);
+  // With exact first queries ahead of it the kernel starts as soon as all their blocks have: it needs the preparation pass,
+  // which was done before they began, and nothing of theirs (both add to the sums).  us per backward
+  // with this / one after the other: T=333 D=128 4 heads 192 / 198, T=128 D=64 64 heads 171 / 181, T=60 D=64 2 heads 29 / 35.
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3((unsigned)grid, 1, 1);
+  cfg.blockDim = dim3(kBwdThreads, 1, 1);
+  cfg.dynamicSmemBytes = Cfg::kSmem;
+  cfg.stream = a.stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = plan.i_first > 0 ? 1 : 0;
+  TRITT_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tmQ, tmDO, tmK1, tmSV1, p));
   count_launch();
-  TRITT_CUDA_OK(cudaGetLastError());
   return 0;
 }
 

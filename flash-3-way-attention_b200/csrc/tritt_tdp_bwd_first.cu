@@ -49,6 +49,7 @@ __device__ __forceinline__ void add_to(float* p, float4 v) {
 template <int D, typename T16>
 __global__ void __launch_bounds__(kFirstThreads) tdp_bwd_first_kernel(const __grid_constant__ FirstParams p) {
   extern __shared__ __align__(16) uint8_t raw[];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the tensor-core kernel need not wait for this one
   FirstShared<D>& sh = *reinterpret_cast<FirstShared<D>*>(raw);
   const int tid = threadIdx.x, bh = blockIdx.y;
   const int q = p.q_rem + ((int)gridDim.x - 1 - (int)blockIdx.x) * p.q_mod;   // the longest first

@@ -136,3 +136,35 @@ def test_shards_sum_to_the_whole(T, D, q_mod, windows, dtype):
     assert _native.read_status(torch.device(DEV)) == 0
     for name, a, b in zip(NAMES, got, full):
         assert_close(name, a, b, dtype)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,D,dtype", [(100, 64, torch.float16), (14, 128, torch.bfloat16), (700, 128, torch.bfloat16)])
+def test_captured_backward_replays(T, D, dtype):
+    """The exact first queries run beside the tensor-core kernel: the same under capture, for new inputs in the same buffers,
+    and for a replay right behind another that uses the same workspace."""
+    t = [x.to(DEV) for x in orc.make_inputs(1, 2, T, D, scale=0.5, seed=T, dtype=dtype)]
+    do = t.pop()
+    o, lse = torch.empty_like(do), torch.empty(1, 2, T, device=DEV)
+    g = [torch.empty_like(do) for _ in range(5)]
+    ws = _native.workspace(_native.OP_TDP_BWD, 1, 2, T, D, _native.dtype_code(dtype), do.device)
+    call = lambda: _native.tdp_bwd(*t, o, do, lse, *g, 1.0 / D, True, *FULL, ws=ws)
+    _native.tdp_fwd(*t, o, lse, 1.0 / D, True, *FULL)
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call()
+    for x, y in zip(t + [do], orc.make_inputs(1, 2, T, D, scale=0.5, seed=T + 1, dtype=dtype)):
+        x.copy_(y)
+    _native.tdp_fwd(*t, o, lse, 1.0 / D, True, *FULL)
+    for x in g:
+        x.fill_(float("nan"))
+    for _ in range(20):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert _native.read_status(torch.device(DEV)) == 0
+    got = [x.clone() for x in g]
+    want = _backward(t, do, 1.0 / D, True)
+    for name, a, b in zip(NAMES, got, want):
+        assert float((a.float() - b.float()).norm()) <= 2e-3 * float(b.float().norm()), name
