@@ -134,8 +134,9 @@ int sm100_tdp_fwd(const TdpArgs& a);
 int sm100_tdp_bwd(const TdpArgs& a);
 // the same up to the fp32 sums: leaves dK1 | dK2 | dSiLU(V1) | dV2 | dQ at the head of the workspace
 int sm100_tdp_bwd_sums(const TdpArgs& a);
-constexpr int kTdpFirstQueries = 16;
-// The contributions of the first `queries` rows of the shard (queries below kTdpFirstQueries, causal, head dimension 64 or 128, 16-bit)
+// Queries of a causal sequence that run in exact fp32 (see make_plan in tritt_sm100_tdp_bwd.cu for the figures).
+inline int tdp_bwd_first_count(int T) { return T >= 1024 ? 32 : 16; }
+// The contributions of the first `queries` rows of the shard (queries below tdp_bwd_first_count(), causal, head dimension 64 or 128, 16-bit)
 // in exact fp32, added to the fp32 sums dK1 | dK2 | dSiLU(V1) | dV2; their dQ rows are stored to the fifth tensor.
 int tdp_bwd_first_queries(const TdpArgs& a, int queries, float* sums, const float* drow);
 // The backward of a query shard by the kernel that steps over queries: dQ rows stored, fp32 sums at the head of the

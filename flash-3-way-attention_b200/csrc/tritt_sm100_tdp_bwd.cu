@@ -213,8 +213,8 @@ struct BwdWalk {
 // fp16's normal range (6e-5; 1/n = 2e-7 at q = 2048).  P and dS are therefore formed times 2^e, e = min(10, log2 of the
 // attended pairs' count bound), and the folds divide it out.  2^10 keeps a probability of 1 times a dP - Dq below 63
 // finite (dS has a further power of two where dP is small: ds_shift).  One e per q-tile, since G and U sum over its queries:
-// that of the first query the kernel takes there, which has the fewest pairs (without windows 8 in the first tile, as the
-// exact first queries leave none below 289 pairs, and 10 in the others).
+// that of the first query the kernel takes there, which has the fewest pairs (without windows 8 or 10 in the first tile, as
+// the exact first queries leave none below 289 or 1089 pairs, and 10 in the others).
 // bf16 has fp32's exponent range: e = 0.
 template <typename T16>
 __device__ __forceinline__ int prob_shift(int q, int causal, int T, int k1w, int k2w) {
@@ -1240,12 +1240,11 @@ int check_kernel_registers(K kern) {
 // The first queries of a causal call run in exact fp32 on the CUDA cores.  Their gradients are the largest by far (a query
 // attends ~q^2 pairs: its dQ falls like 1/q, and so does what it adds to the first key rows), so their rounding is most of
 // the error of the whole result; and in fp16 the first query of a tile sets the tile's range shift (prob_shift).  They are
-// a vanishing part of the work: a training step's error against fp64 goes from 3.6e-3 to 2.6e-3 at T=2048 in bf16.  16 of
-// them: with 32 the error is 2 to 10 % lower still, at eight times the pairs and atomics (160 heads of T=70: 305 against
-// 237 us a call, 204 without any; 4 heads of T=333 D=128: 201, 195, 179).
-// (Queries 0 to 15 themselves, not the first 16 rows of a shard: 8 interleaved shards have queries up to 127 among those, with
-// 60 times the pairs, and at 64 shards and T=1024 they are the whole shard.)
-constexpr int kFirstQueries = kTdpFirstQueries;
+// a vanishing part of the work on long sequences: a training step's error against fp64 goes from 3.6e-3 to 2.6e-3 at T=2048
+// in bf16 with 32 of them.  Short ones take 16: the error is 2 to 10 % higher than with 32, at an eighth of the pairs and
+// atomics (160 heads of T=70: 237 against 305 us a call, 204 without any; 4 heads of T=333 D=128: 195, 201, 179).
+// (Queries 0 to 31 themselves, not the first 32 rows of a shard: 8 interleaved shards have queries up to 248 among those, with
+// 60 times the pairs, and at 64 shards and T=2048 they are the whole shard.)
 
 // What a call does, from its arguments alone.
 struct BwdPlan {
@@ -1269,8 +1268,9 @@ template <int D> BwdPlan make_plan(const TdpArgs& a) {
   const int nq = a.q_rem < a.T ? (a.T - a.q_rem + a.q_mod - 1) / a.q_mod : 0;
   p.g = BwdGeometry{a.T, nq, a.q_mod, a.q_rem, a.mask.causal, a.mask.k1w, a.mask.k2w, a.mask.kkl, a.mask.kkr, BwdCfg<D>::JT};
   if (nq == 0) return p;
-  if (a.mask.causal && a.q_rem < kFirstQueries) {
-    p.i_first = (kFirstQueries - a.q_rem + a.q_mod - 1) / a.q_mod;
+  const int first = tdp_bwd_first_count(a.T);
+  if (a.mask.causal && a.q_rem < first) {
+    p.i_first = (first - a.q_rem + a.q_mod - 1) / a.q_mod;
     if (p.i_first >= nq) {   // nothing left for the kernel
       p.i_first = nq;
       return p;

@@ -1,7 +1,7 @@
 // The first queries of a causal triple-dot-product backward, in exact fp32 on the CUDA cores: what they add to the sums
 // dK1 | dK2 | dSiLU(V1) | dV2, and their dQ.  (Why they are not the tensor-core kernel's: see kFirstQueries there.)
 //
-// One CTA per (head, query); a query q < 16 attends keys 0 .. q, at most 16 x 16 pairs, so everything it needs stays in
+// One CTA per (head, query); a query q < 16 (or 32) attends keys 0 .. q, at most 16 x 16 pairs, so everything it needs stays in
 // shared memory.  With the rows A[k] = alpha log2(e) Q K2[k] and B[k] = dO V2[k]:
 //     S[k,j] = A[k] . K1[j]     P = exp2(S - lse2)      dP[k,j] = B[k] . SiLU(V1)[j]     dS = P (dP - Dq)
 //     F = dS K1:    dK2[k] += alpha Q F[k],   dQ = alpha sum_k K2[k] F[k]        W = P SiLU(V1):  dV2[k] += dO W[k]
@@ -15,14 +15,13 @@
 namespace tritt {
 namespace {
 
-constexpr int kFirst = kTdpFirstQueries, kFirstThreads = 256;
-static_assert(kFirst * kFirst == kFirstThreads, "one pair per thread");
+constexpr int kFirstThreads = 256;
 
-template <int D> struct FirstShared {
+template <int D, int NF> struct FirstShared {   // NF: queries below this, and so keys
   static constexpr int kPitch = D + 4;   // (rows 4 banks apart: 8 lanes' 16-byte reads of 8 rows do not conflict)
-  float k1[kFirst][kPitch], s1[kFirst][kPitch], a[kFirst][kPitch], b[kFirst][kPitch];
-  float p_kj[kFirst][kFirst + 4], ds_kj[kFirst][kFirst + 4];   // [k][j], and transposed
-  float p_jk[kFirst][kFirst + 4], ds_jk[kFirst][kFirst + 4];
+  float k1[NF][kPitch], s1[NF][kPitch], a[NF][kPitch], b[NF][kPitch];
+  float p_kj[NF][NF + 4], ds_kj[NF][NF + 4];   // [k][j], and transposed
+  float p_jk[NF][NF + 4], ds_jk[NF][NF + 4];
   float q[D], d_o[D], dq[kFirstThreads / (D / 4)][D];
 };
 
@@ -46,11 +45,11 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float c) {
 __device__ __forceinline__ void add_to(float* p, float4 v) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
-template <int D, typename T16>
+template <int D, typename T16, int NF>
 __global__ void __launch_bounds__(kFirstThreads) tdp_bwd_first_kernel(const __grid_constant__ FirstParams p) {
   extern __shared__ __align__(16) uint8_t raw[];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the tensor-core kernel need not wait for this one
-  FirstShared<D>& sh = *reinterpret_cast<FirstShared<D>*>(raw);
+  FirstShared<D, NF>& sh = *reinterpret_cast<FirstShared<D, NF>*>(raw);
   const int tid = threadIdx.x, bh = blockIdx.y;
   const int q = p.q_rem + ((int)gridDim.x - 1 - (int)blockIdx.x) * p.q_mod;   // the longest first
   const size_t head = (size_t)bh * p.T * D;
@@ -93,28 +92,39 @@ __global__ void __launch_bounds__(kFirstThreads) tdp_bwd_first_kernel(const __gr
     store8(&sh.b[row][h], f);
   }
   __syncthreads();
-  // ---- P and dS: one pair per thread
+  // ---- P and dS: one key j and E keys k per thread
   {
-    const int j = tid % kFirst, k = tid / kFirst;
+    constexpr int E = NF * NF / kFirstThreads;
+    const int j = tid % NF, k0 = tid / NF * E;
     const float lse2 = __ldg(p.lse + (size_t)bh * p.T + q) * kLog2e, Dq = __ldg(p.drow + (size_t)bh * p.T + q);
-    float pr = 0.f, ds = 0.f;
-    if (p.mask.valid(q, j, k)) {
-      float s = 0.f, dp = 0.f;
-#pragma unroll 8
+    const bool single = p.mask.single_pair(q);   // (its score gradient is exactly zero)
+    float s[E], dp[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) s[e] = dp[e] = 0.f;
+    if (j < nk && k0 < nk) {
+#pragma unroll 4
       for (int h = 0; h < D; h += 4) {
-        s = dot4(*reinterpret_cast<const float4*>(&sh.k1[j][h]), *reinterpret_cast<const float4*>(&sh.a[k][h]), s);
-        dp = dot4(*reinterpret_cast<const float4*>(&sh.s1[j][h]), *reinterpret_cast<const float4*>(&sh.b[k][h]), dp);
+        const float4 x = *reinterpret_cast<const float4*>(&sh.k1[j][h]), y = *reinterpret_cast<const float4*>(&sh.s1[j][h]);
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const int k = min(k0 + e, q);
+          s[e] = dot4(x, *reinterpret_cast<const float4*>(&sh.a[k][h]), s[e]);
+          dp[e] = dot4(y, *reinterpret_cast<const float4*>(&sh.b[k][h]), dp[e]);
+        }
       }
-      pr = exp2f(s - lse2);
-      // (a query with a single pair has a score gradient of exactly zero)
-      if (pr != 0.f && !p.mask.single_pair(q)) ds = pr * (dp - Dq);
     }
-    sh.p_kj[k][j] = sh.p_jk[j][k] = pr;
-    sh.ds_kj[k][j] = sh.ds_jk[j][k] = ds;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int k = k0 + e;
+      const float pr = p.mask.valid(q, j, k) ? exp2f(s[e] - lse2) : 0.f;
+      const float ds = pr != 0.f && !single ? pr * (dp[e] - Dq) : 0.f;
+      sh.p_kj[k][j] = sh.p_jk[j][k] = pr;
+      sh.ds_kj[k][j] = sh.ds_jk[j][k] = ds;
+    }
   }
   __syncthreads();
   // ---- the four products: 4 columns h of R rows per thread
-  constexpr int kChunks = D / 4, kGroups = kFirstThreads / kChunks, R = kFirst / kGroups;   // D=128: 8 groups of 2, 64: 16 of 1
+  constexpr int kChunks = D / 4, kGroups = kFirstThreads / kChunks, R = NF / kGroups;   // NF=16: 8 groups of 2 at D=128, 16 of 1 at 64
   const int h = tid % kChunks * 4, r0 = tid / kChunks * R;
   float4 dq = make_float4(0.f, 0.f, 0.f, 0.f);
   if (r0 < nk) {
@@ -123,7 +133,7 @@ __global__ void __launch_bounds__(kFirstThreads) tdp_bwd_first_kernel(const __gr
     const size_t row0 = head + (size_t)r0 * D + h;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     // sum over the pair's other key: two weight matrices (columns of R rows) against two key matrices
-    auto products = [&](const float (*wx)[kFirst + 4], const float (*wy)[kFirst + 4], const float (*x)[D + 4], const float (*y)[D + 4],
+    auto products = [&](const float (*wx)[NF + 4], const float (*wy)[NF + 4], const float (*x)[D + 4], const float (*y)[D + 4],
                         float4 (&gx)[R], float4 (&gy)[R]) {
 #pragma unroll
       for (int r = 0; r < R; ++r) gx[r] = gy[r] = zero;
@@ -168,18 +178,25 @@ __global__ void __launch_bounds__(kFirstThreads) tdp_bwd_first_kernel(const __gr
   }
 }
 
-template <int D, typename T16>
-int launch_first(const TdpArgs& a, int queries, float* sums, const float* drow) {
+template <int D, typename T16, int NF>
+int launch_first_nf(const TdpArgs& a, int queries, float* sums, const float* drow) {
   FirstParams p{};
   p.q = a.q; p.k1 = a.k1; p.k2 = a.k2; p.v1 = a.v1; p.v2 = a.v2; p.d_o = a.d_o;
   p.lse = a.lse_in; p.drow = drow; p.sums = sums; p.n = (size_t)a.B * a.N * a.T * D;
   p.T = a.T; p.q_mod = a.q_mod; p.q_rem = a.q_rem; p.alpha = a.alpha; p.mask = a.mask;
-  auto kern = tdp_bwd_first_kernel<D, T16>;
-  TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FirstShared<D>)));
-  kern<<<dim3(queries, a.B * a.N), kFirstThreads, sizeof(FirstShared<D>), a.stream>>>(p);
+  auto kern = tdp_bwd_first_kernel<D, T16, NF>;
+  TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FirstShared<D, NF>)));
+  kern<<<dim3(queries, a.B * a.N), kFirstThreads, sizeof(FirstShared<D, NF>), a.stream>>>(p);
   count_launch();
   TRITT_CUDA_OK(cudaGetLastError());
   return 0;
+}
+
+template <int D, typename T16>
+int launch_first(const TdpArgs& a, int queries, float* sums, const float* drow) {
+  // (the plan takes 16 or 32 queries of the sequence)
+  return tdp_bwd_first_count(a.T) == 16 ? launch_first_nf<D, T16, 16>(a, queries, sums, drow)
+                                        : launch_first_nf<D, T16, 32>(a, queries, sums, drow);
 }
 
 }  // namespace

@@ -57,7 +57,7 @@ def test_exact_first_queries_are_the_first_queries_of_the_sequence(T, q_mod, dty
     """... and not the first 32 rows of a shard, whose queries lie q_mod apart."""
     for q_rem in {0, 1 % q_mod, q_mod // 2, q_mod - 1}:
         first, cells, by_queries = _native.tdp_bwd_plan(T, 64, dtype, True, None, None, None, None, q_mod, q_rem)
-        assert first == (0 if by_queries else len(range(q_rem, 16, q_mod)))
+        assert first == (0 if by_queries else len(range(q_rem, 32 if T >= 1024 else 16, q_mod)))
         assert cells > 0
         assert _native.tdp_bwd_plan(T, 64, dtype, False, None, None, None, None, q_mod, q_rem)[0] == 0
     assert _native.tdp_bwd_plan(14, 64, dtype, True, None, None, None, None) == (14, 0, 0)
