@@ -133,7 +133,10 @@ size_t tritt_workspace_bytes_flags(int op, int B, int N, int T, int D, int dtype
     case TRITT_OP_TDP_BWD: {
       a = simt_tdp_workspace(op, B, N, T, D, dtype);
       b = sm100_tdp_workspace(op, B, N, T, D, dtype);
-      if (b) b += op == TRITT_OP_TDP_FWD ? sm100_tdp_fwd_optional_workspace(B, N, T, D, dtype) : sm100_tdp_bwd_optional_workspace(B, N);
+      if (b) {
+        b += op == TRITT_OP_TDP_FWD ? sm100_tdp_fwd_optional_workspace(B, N, T, D, dtype)
+                                    : sm100_tdp_bwd_optional_workspace(B, N);
+      }
       const TdpMask any = make_tdp_mask(1, T, T, T, T, T);
       if (tdp_wide_applies(op, T, D, dtype, any, flags)) {
         const size_t w = tdp_wide_workspace(op, B, N, T, D);

@@ -136,8 +136,8 @@ int sm100_tdp_bwd(const TdpArgs& a);
 int sm100_tdp_bwd_sums(const TdpArgs& a);
 // Queries of a causal sequence that run in exact fp32 (see make_plan in tritt_sm100_tdp_bwd.cu for the figures).
 inline int tdp_bwd_first_count(int T) { return T >= 1024 ? 32 : 16; }
-// The contributions of the first `queries` rows of the shard (queries below tdp_bwd_first_count(), causal, head dimension 64 or 128, 16-bit)
-// in exact fp32, added to the fp32 sums dK1 | dK2 | dSiLU(V1) | dV2; their dQ rows are stored to the fifth tensor.
+// The contributions of the first `queries` rows of the shard (queries below tdp_bwd_first_count(), causal, head dimension 64
+// or 128, 16-bit) in exact fp32, added to the fp32 sums dK1 | dK2 | dSiLU(V1) | dV2; their dQ rows are stored to the fifth tensor.
 int tdp_bwd_first_queries(const TdpArgs& a, int queries, float* sums, const float* drow);
 // The backward of a query shard by the kernel that steps over queries: dQ rows stored, fp32 sums at the head of the
 // workspace; and the cells (q, j, k) that it executes per head (of one of its two roles).
@@ -178,9 +178,9 @@ bool sm100_attn_fwd_supported(int T, int D, int dtype);
 int sm100_attn_fwd(const AttnTcArgs& a);
 int sm100_silu_16(const void* in, void* out, size_t n, int dtype, cudaStream_t stream);  // out = SiLU(in), 16-bit
 
-// Backward of the same attention, as a row-owner and a column-owner kernel.  With P = exp(alpha x.k + bias - lse),
-// dP = dout.v and dS = P (dP - drow):  rows: d_rows_t = alpha sum_c dS k (+ d_rows_add);  columns: d_vc_f32 =
-// sum_r P dout, d_kc = alpha sum_r dS x (fp32 or the operands' type), gsum = sum_r dS.
+// Backward of the same attention, row owners and column owners in one launch.  With P = exp(alpha x.k + bias - lse),
+// dP = dout.v and dS = P (dP - drow):  rows: d_rows_t = alpha sum_c dS k (+ d_rows_add);  columns: d_kc = alpha sum_r dS x and
+// d_vc = sum_r P dout, which leaves in one of the two forms below.
 struct AttnBwdTcArgs {
   const void *xq, *kc, *vc, *dout;  // 16-bit [BN, T, D]
   const float *bias, *lse, *drow;   // [BN, T]: per column (or null), per row, per row

@@ -1,12 +1,14 @@
 // Two-way soft-max attention backward on Blackwell tensor cores: the gradients of the two attentions that make up
 // dot-product-sum trittention (see tritt_sm100_attn_fwd.cu for the decomposition).  With P[r,c] =
 // exp(alpha X[r].K[c] + bias[c] - lse[r]), dP[r,c] = dOut[r].V[c] and dS = P (dP - drow[r]):
-//   row-owner kernel  (COL = false): a CTA owns 128 rows r and walks the column tiles:
+//   row owner  (COL = false): a CTA owns 128 rows r and walks the column tiles:
 //        d_rows[r] = alpha sum_c dS[r,c] K[c]
-//   column-owner kernel (COL = true): a CTA owns 128 columns c and walks the row tiles, working on the transposed
+//   column owner (COL = true): a CTA owns 128 columns c and walks the row tiles, working on the transposed
 //   products S^T = K X^T and dP^T = V dOut^T so that its threads again own one accumulator row each:
-//        d_vc[c] = sum_r P[r,c] dOut[r],   d_kc[c] = alpha sum_r dS[r,c] X[r],   gsum[c] = sum_r dS[r,c]
-// Neither kernel needs atomics or a transposed operand; the price is that S and dP are formed twice.  (The
+//        dW[c] = sum_r P[r,c] dOut[r],   d_kc[c] = alpha sum_r dS[r,c] X[r],   sum_r dS[r,c]
+//   and its epilogue turns dW into what the other attention or the caller needs: dV1 = dW SiLU'(V1), or dV2 = dW Y,
+//   dY = dW V2 and the inner attention's row term sum_h dY Y - sum_r dS.
+// Neither kind needs atomics or a transposed operand; the price is that S and dP are formed twice.  (The
 // reference splits its backward the same way, a query-owner kernel and a key-owner kernel:
 // dot_product_sum/kernels/bwd_dq_kernel.py:28-350, bwd_dk1_dv1_kernel.py:29-416.)
 //
@@ -194,7 +196,8 @@ __device__ __forceinline__ void attn_bwd_tile(const CUtensorMap& tmOwn0, const C
         }
         commit(&bars.sd_ready);
       };
-      // accumulations with the 16-bit P / dS read from TMEM (each warpgroup's over the first half of its 64 columns) and the ring tiles used row-major
+      // accumulations with the 16-bit P / dS read from TMEM (each warpgroup's over the first half of its 64 columns) and
+      // the ring tiles used row-major
       auto issue_acc = [&](int st, uint32_t acc) {
         const uint32_t m0 = desc_lo(smem_u32(smem + Cfg::kOffRing + st * 2 * Cfg::kTile), 16384);
         const uint32_t m1 = desc_lo(smem_u32(smem + Cfg::kOffRing + st * 2 * Cfg::kTile + Cfg::kTile), 16384);

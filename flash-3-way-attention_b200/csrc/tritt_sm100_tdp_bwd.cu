@@ -46,7 +46,9 @@ namespace {
 using namespace sm100;
 
 constexpr int kBwdThreads = 640;
-// Registers per thread: 640 threads are launched with 96 each (480 per lane of the five warpgroups) and split them anew.
+// Registers per thread: 640 threads are launched with 96 each (480 per lane of the five warpgroups) and split them anew.  The
+// shares are tight: a body spills 84 to 204 bytes a thread (-Xptxas -v gives the sum over the two), counters and addresses
+// that a step reads once or twice.
 constexpr int kRegsLaunch = 96, kRegsSoftmax = 80, kRegsFold = 128, kRegsService = 64;
 static_assert(2 * kRegsSoftmax + 2 * kRegsFold + kRegsService <= 5 * kRegsLaunch, "more registers than the launch has");
 constexpr int kVecBatch = 4;     // K2 / V2 rows per hand-over
@@ -248,7 +250,10 @@ template <typename T16> __device__ __forceinline__ int ds_shift(float bound) {
   return 0;
 }
 
-__device__ __forceinline__ float pow2i(int e) { return __int_as_float((127 + e) << 23); }   // |e| <= 126, exact
+// 2^e for the shifts above, exact, |e| <= 126 (1, without looking at e, for bf16, whose shifts are all 0)
+template <typename T16> __device__ __forceinline__ float pow2i(int e) {
+  return std::is_same<T16, __half>::value ? __int_as_float((127 + e) << 23) : 1.f;
+}
 
 __device__ __forceinline__ void red_add(float* p, float v) {
   asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
@@ -394,8 +399,8 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
         // of another query's infinite or NaN Dq would be NaN, which G sums into every key the tile meets)
         lse2 = q_ok ? __ldg(p.lse + (size_t)it.bh * T + q) * kLog2e - (float)e : 0.f;
         const int f = it.flags >> kShiftBits;
-        drow = q_ok ? __ldg(p.drow + (size_t)it.bh * T + q) * pow2i(f) : 0.f;
-        dq_scale = pow2i(-e - it.ea - f) * kLn2;    // A carries alpha * log2(e)
+        drow = q_ok ? __ldg(p.drow + (size_t)it.bh * T + q) * pow2i<T16>(f) : 0.f;
+        dq_scale = pow2i<T16>(-e - it.ea - f) * kLn2;    // A carries alpha * log2(e)
         // A query that attends a single pair has P = 1 and a score gradient of exactly zero (TdpMask::single_pair):
         // P (dP - Dq) has two terms that are equal only up to the 16-bit rounding of the stored output, so its dS
         // is set to zero.
@@ -424,7 +429,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       }
       const bool any_single = __any_sync(0xffffffffu, single);
       const float2 nlse = make_float2(-lse2, -lse2), ndq = make_float2(-drow, -drow);
-      const float sa = kShifted ? pow2i(-it.ea) : 1.f, sb = kShifted ? pow2i((it.flags >> kShiftBits) - it.eb) : 1.f;
+      const float sa = pow2i<T16>(-it.ea), sb = pow2i<T16>((it.flags >> kShiftBits) - it.eb);
       // v * scale + add; the scale of bf16 is 1
       auto scaled = [](uint32_t v0, uint32_t v1, float scale, float2 add) {
         const float2 v = make_float2(__uint_as_float(v0), __uint_as_float(v1));
@@ -587,8 +592,8 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       arrive_warp(&bars.tile_free);
       const int len = it.len;
       const int e = prob_shift<T16>(g.q_rem + max(it.qt * 128, p.i_first) * g.q_mod, g.causal, T, g.k1w, g.k2w);
-      const float unshift = pow2i(-e);
-      const float unshift_ds = unshift * pow2i(-(it.flags >> kShiftBits));
+      const float unshift = pow2i<T16>(-e);
+      const float unshift_ds = unshift * pow2i<T16>(-(it.flags >> kShiftBits));
       const float zscale = role ? unshift : unshift_ds * p.alpha;
       float* zrow = (role ? p.dv2 : p.dk2) + ((size_t)it.bh * T + it.k0) * D;
       auto form = [&](int i) -> bool {
@@ -768,7 +773,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       ++items;
       // ---- dK1 / dSiLU(V1) of this item
       // (the K2 rows carry alpha * log2(e) * 2^ea, the V2 rows 2^eb)
-      const float jscale = role ? unshift * pow2i(-it.eb) : unshift_ds * pow2i(-it.ea) * kLn2;
+      const float jscale = role ? unshift * pow2i<T16>(-it.eb) : unshift_ds * pow2i<T16>(-it.ea) * kLn2;
       float* const base = (role ? p.dsv1 : p.dk1) + (size_t)it.bh * T * D;
 #pragma unroll
       for (int c16 = 0; c16 < 4; ++c16)
@@ -933,8 +938,8 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
         ea = range_shift<T16>(fabsf(p.alpha * kLog2e) * st.qk1 * st.k2);
         eb = range_shift<T16>(st.sv1 * st.v2);
         f = ds_shift<T16>(sqrtf(st.do_row * st.sv1_row) * st.v2);
-        scale_k = p.alpha * kLog2e * pow2i(ea);
-        scale_v = pow2i(eb);
+        scale_k = p.alpha * kLog2e * pow2i<T16>(ea);
+        scale_v = pow2i<T16>(eb);
       }
       it.ea = ea;
       it.eb = eb;

@@ -187,10 +187,10 @@ def test_backward_reference_test_distribution(dtype, D, causal):
 
 @pytest.mark.parametrize("dtype,causal,T", [(torch.bfloat16, True, 384), (torch.float16, True, 200),
                                             (torch.bfloat16, False, 192)])
-def test_backward_on_cta_pairs_matches_oracle_and_default_path(dtype, causal, T):
-    """TRITT_FLAG_BWD_CTA_PAIRS: the backward kernel as clusters of two CTAs (cta_group::2 products over two queries
-    that share every key / value tile).  Checked against the oracle with the usual bounds, and against the default
-    one-CTA-per-item launch, from which it may differ only by the order of the fp32 reduce-adds."""
+def test_backward_accepts_and_ignores_the_cta_pair_flag(dtype, causal, T):
+    """TRITT_FLAG_BWD_CTA_PAIRS asked for a form of an earlier kernel (clusters of two CTAs).  A call that passes it is
+    accepted and runs as one that does not: checked against the oracle with the usual bounds and against the call
+    without it, from which it may differ only by the order of the fp32 reduce-adds."""
     B, N, D, alpha = 1, 3, 128, 1 / 128
     q, k1, k2, v1, v2, dz = orc.make_inputs(B, N, T, D, scale=0.5, seed=31 + T, dtype=dtype)
     t = [x.to(DEV) for x in (q, k1, k2, v1, v2)]
@@ -199,14 +199,14 @@ def test_backward_on_cta_pairs_matches_oracle_and_default_path(dtype, causal, T)
     _native.tdp_fwd(*t, o, lse, alpha, causal, None, None, None, None)
     base = [torch.empty_like(t[0]) for _ in range(5)]
     _native.tdp_bwd(*t, o, do, lse, *base, alpha, causal, None, None, None, None)
-    pair = [torch.full_like(t[0], float("nan")) for _ in range(5)]
-    _native.tdp_bwd(*t, o, do, lse, *pair, alpha, causal, None, None, None, None, flags=_native.FLAG_BWD_CTA_PAIRS)
+    flagged = [torch.full_like(t[0], float("nan")) for _ in range(5)]
+    _native.tdp_bwd(*t, o, do, lse, *flagged, alpha, causal, None, None, None, None, flags=_native.FLAG_BWD_CTA_PAIRS)
     torch.cuda.synchronize()
     assert _native.read_status(torch.device(DEV)) == 0
     ref = orc.tdp_backward(q.float(), k1.float(), k2.float(), v1.float(), v2.float(), dz.float(), alpha, causal)
-    for name, got, want, same in zip(("dq", "dk1", "dk2", "dv1", "dv2"), pair, ref, base):
-        assert_close(name + " (pairs)", got, want, dtype)
-        assert_close(name + " (pairs vs default launch)", got, same, torch.float32, scale=100.0)
+    for name, got, want, same in zip(("dq", "dk1", "dk2", "dv1", "dv2"), flagged, ref, base):
+        assert_close(name + " (flag)", got, want, dtype)
+        assert_close(name + " (flag against none)", got, same, torch.float32, scale=100.0)
 
 
 def test_backward_query_shards_sum_to_full_gradient():
