@@ -242,6 +242,11 @@ int tritt_tdp_bwd_plan(int T, int D, int dtype, int causal, int k1_window, int k
                        int q_rem, int flags, long long* out) {
   int rc = check_shard(q_mod, q_rem);
   if (rc) return rc;
+  if ((rc = check_windows(causal, k1_window, k2_window, kk_left, kk_right))) return rc;
+  if (T <= 0 || !out) {
+    set_error("tritt_tdp_bwd_plan needs a positive length and a place for its results");
+    return -1;
+  }
   TdpArgs a{};
   a.B = a.N = 1; a.T = T; a.D = D;
   a.mask = make_tdp_mask(causal, T, k1_window, k2_window, kk_left, kk_right);

@@ -168,3 +168,32 @@ def test_captured_backward_replays(T, D, dtype):
     want = _backward(t, do, 1.0 / D, True)
     for name, a, b in zip(NAMES, got, want):
         assert float((a.float() - b.float()).norm()) <= 2e-3 * float(b.float().norm()), name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,D,dtype", [(150, 64, torch.float16), (1100, 64, torch.bfloat16), (333, 128, torch.bfloat16)])
+def test_calls_in_turn_on_the_same_buffers(T, D, dtype):
+    """Two sets of inputs that take turns in the same tensors and workspace, back to back: every call sees its own inputs
+    and its own preparation, although its kernels overlap (small scores, then large ones: the other operand as well)."""
+    sets = [[x.to(DEV) for x in orc.make_inputs(1, 4, T, D, scale=sc, seed=T + i, dtype=dtype)] for i, sc in ((0, 0.5), (1, 1.0))]
+    want, saved = [], []
+    for x in sets:
+        o, lse = torch.empty_like(x[0]), torch.empty(1, 4, T, device=DEV)
+        _native.tdp_fwd(*x[:5], o, lse, 1 / 8, True, *FULL)
+        saved.append((o, lse))
+        want.append(_backward(x[:5], x[5], 1 / 8, True))
+    t = [torch.empty_like(x) for x in sets[0]]
+    o, lse = torch.empty_like(t[0]), torch.empty(1, 4, T, device=DEV)
+    ws = _native.workspace(_native.OP_TDP_BWD, 1, 4, T, D, _native.dtype_code(dtype), o.device)
+    results = []
+    for i in range(40):
+        for dst, src in zip(t + [o, lse], sets[i & 1] + list(saved[i & 1])):
+            dst.copy_(src)
+        g = [torch.empty_like(o) for _ in range(5)]
+        _native.tdp_bwd(*t[:5], o, t[5], lse, *g, 1 / 8, True, *FULL, ws=ws)
+        results.append(g)
+    torch.cuda.synchronize()
+    assert _native.read_status(torch.device(DEV)) == 0
+    for i, g in enumerate(results):
+        for name, a, b in zip(NAMES, g, want[i & 1]):
+            assert float((a.float() - b.float()).norm()) <= 2e-3 * float(b.float().norm()), (i, name)
