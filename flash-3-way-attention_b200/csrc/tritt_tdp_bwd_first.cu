@@ -3,9 +3,12 @@
 //
 // One CTA per (head, query); a query q < 16 (or 32) attends keys 0 .. q, at most 16 x 16 pairs, so everything it needs stays in
 // shared memory.  With the rows A[k] = alpha log2(e) Q K2[k] and B[k] = dO V2[k]:
-//     S[k,j] = A[k] . K1[j]     P = exp2(S - lse2)      dP[k,j] = B[k] . SiLU(V1)[j]     dS = P (dP - Dq)
+//     S[k,j] = A[k] . K1[j]     P = c exp2(S - lse2)      dP[k,j] = B[k] . SiLU(V1)[j]     dS = P (dP - Dq)
 //     F = dS K1:    dK2[k] += alpha Q F[k],   dQ = alpha sum_k K2[k] F[k]        W = P SiLU(V1):  dV2[k] += dO W[k]
 //     G = dS^T A:   dK1[j] += ln(2) G[j]                                         U = P^T B:       dSV1[j] += U[j]
+// c brings P to the mass that the forward's scores (A rounded to the inputs' type) have under the saved log-sum-exp, 1 for a
+// whole soft-max: without it a query of few pairs and large scores does not sum to one, and dV2 is 1.05 to 1.19 times as
+// far from fp64 as with the forward's scores (scores of order 4, T=50 to 120).
 // It is latency that counts (it runs ahead of the tensor-core kernel), so every query has a CTA, which adds its share to the
 // sums: about 8 us at 4 heads, D=128 and at 16 heads, D=64.  (The general CUDA-core kernel, which walks a query's rows one
 // tile after the other, took 60 and 50 us for twice as many queries, this one 12.5 and 18 us for those.)
@@ -22,6 +25,7 @@ template <int D, int NF> struct FirstShared {   // NF: queries below this, and s
   float k1[NF][kPitch], s1[NF][kPitch], a[NF][kPitch], b[NF][kPitch];
   float p_kj[NF][NF + 4], ds_kj[NF][NF + 4];   // [k][j], and transposed
   float p_jk[NF][NF + 4], ds_jk[NF][NF + 4];
+  float2 mass[kFirstThreads / 32];
   float q[D], d_o[D], dq[kFirstThreads / (D / 4)][D];
 };
 
@@ -98,9 +102,9 @@ __global__ void __launch_bounds__(kFirstThreads) tdp_bwd_first_kernel(const __gr
     const int j = tid % NF, k0 = tid / NF * E;
     const float lse2 = __ldg(p.lse + (size_t)bh * p.T + q) * kLog2e, Dq = __ldg(p.drow + (size_t)bh * p.T + q);
     const bool single = p.mask.single_pair(q);   // (its score gradient is exactly zero)
-    float s[E], dp[E];
+    float s[E], s16[E], dp[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) s[e] = dp[e] = 0.f;
+    for (int e = 0; e < E; ++e) s[e] = s16[e] = dp[e] = 0.f;
     if (j < nk && k0 < nk) {
 #pragma unroll 4
       for (int h = 0; h < D; h += 4) {
@@ -108,15 +112,41 @@ __global__ void __launch_bounds__(kFirstThreads) tdp_bwd_first_kernel(const __gr
 #pragma unroll
         for (int e = 0; e < E; ++e) {
           const int k = min(k0 + e, q);
-          s[e] = dot4(x, *reinterpret_cast<const float4*>(&sh.a[k][h]), s[e]);
+          const float4 a = *reinterpret_cast<const float4*>(&sh.a[k][h]);
+          const float2 r0 = unpack2<T16>(pack2<T16>(a.x, a.y)), r1 = unpack2<T16>(pack2<T16>(a.z, a.w));
+          s[e] = dot4(x, a, s[e]);
+          s16[e] = dot4(x, make_float4(r0.x, r0.y, r1.x, r1.y), s16[e]);
           dp[e] = dot4(y, *reinterpret_cast<const float4*>(&sh.b[k][h]), dp[e]);
         }
       }
     }
+    // the mass of the exact P brought to that of the forward's
+    float sum = 0.f, sum16 = 0.f;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const bool ok = p.mask.valid(q, j, k0 + e);
+      s[e] = ok ? exp2f(s[e] - lse2) : 0.f;
+      sum += s[e];
+      sum16 += ok ? exp2f(s16[e] - lse2) : 0.f;
+    }
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+      sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      sum16 += __shfl_xor_sync(0xffffffffu, sum16, o);
+    }
+    if ((tid & 31) == 0) sh.mass[tid >> 5] = make_float2(sum, sum16);
+    __syncthreads();
+    sum = sum16 = 0.f;
+#pragma unroll
+    for (int w = 0; w < kFirstThreads / 32; ++w) {
+      sum += sh.mass[w].x;
+      sum16 += sh.mass[w].y;
+    }
+    const float c = sum > 0.f ? sum16 / sum : 1.f;   // (nothing attended: P is zero; NaN: it stays)
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int k = k0 + e;
-      const float pr = p.mask.valid(q, j, k) ? exp2f(s[e] - lse2) : 0.f;
+      const float pr = s[e] * c;
       const float ds = pr != 0.f && !single ? pr * (dp[e] - Dq) : 0.f;
       sh.p_kj[k][j] = sh.p_jk[j][k] = pr;
       sh.ds_kj[k][j] = sh.ds_jk[j][k] = ds;

@@ -179,3 +179,12 @@ def test_heads_with_small_and_large_scores_in_one_cta(T, D):
                      head_scale=torch.tensor([0.1, 1.2, 1.2, 0.2] * (heads // 4)))
     print(T, D, " ".join(f"{n} {r:.2f}" for n, r in ratios))
     assert all(r <= SPREAD for _, r in ratios), f"errors over those of the precision class: {ratios}"
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,D,windows", [(50, 64, (None,) * 4), (120, 128, (None,) * 4), (120, 128, (9, 5, 3, 2))])
+def test_first_queries_with_large_scores(T, D, windows, dtype):
+    """Scores of order 4 to 6: single pairs carry the first queries, in whichever kernel forms them."""
+    ratios = _errors(T, D, dtype, True, True, windows, seeds=(0, 1, 2), std=(3, 1, 1, 1))
+    print(T, D, dtype, windows, " ".join(f"{n} {r:.2f}" for n, r in ratios))
+    assert all(r <= SPREAD for _, r in ratios), f"errors over those of the precision class: {ratios}"
