@@ -3,12 +3,12 @@
 //
 // One CTA per (head, query); a query q < 16 (or 32) attends keys 0 .. q, at most 16 x 16 pairs, so everything it needs stays in
 // shared memory.  With the rows A[k] = alpha log2(e) Q K2[k] and B[k] = dO V2[k]:
-//     S[k,j] = A[k] . K1[j]     P = c exp2(S - lse2)      dP[k,j] = B[k] . SiLU(V1)[j]     dS = P (dP - Dq)
+//     S[k,j] = A[k] . K1[j]     P = c exp2(S - max)      dP[k,j] = B[k] . SiLU(V1)[j]     dS = P (dP - Dq)
 //     F = dS K1:    dK2[k] += alpha Q F[k],   dQ = alpha sum_k K2[k] F[k]        W = P SiLU(V1):  dV2[k] += dO W[k]
 //     G = dS^T A:   dK1[j] += ln(2) G[j]                                         U = P^T B:       dSV1[j] += U[j]
 // c brings P to the mass that the forward's scores (A rounded to the inputs' type) have under the saved log-sum-exp, 1 for a
-// whole soft-max: without it a query of few pairs and large scores does not sum to one, and dV2 is 1.05 to 1.19 times as
-// far from fp64 as with the forward's scores (scores of order 4, T=50 to 120).
+// whole soft-max: exp2(S - lse2) of a query of few pairs and large scores does not sum to one (dV2 1.05 to 1.19 times as
+// far from fp64 as with the forward's scores, for scores of order 4 and T=50 to 120), and overflows for scores of order 1e5.
 // It is latency that counts (it runs ahead of the tensor-core kernel), so every query has a CTA, which adds its share to the
 // sums: about 8 us at 4 heads, D=128 and at 16 heads, D=64.  (The general CUDA-core kernel, which walks a query's rows one
 // tile after the other, took 60 and 50 us for twice as many queries, this one 12.5 and 18 us for those.)
@@ -25,7 +25,7 @@ template <int D, int NF> struct FirstShared {   // NF: queries below this, and s
   float k1[NF][kPitch], s1[NF][kPitch], a[NF][kPitch], b[NF][kPitch];
   float p_kj[NF][NF + 4], ds_kj[NF][NF + 4];   // [k][j], and transposed
   float p_jk[NF][NF + 4], ds_jk[NF][NF + 4];
-  float2 mass[kFirstThreads / 32];
+  float3 mass[kFirstThreads / 32];   // (each warp's largest score, sum, and sum of the forward's scores)
   float q[D], d_o[D], dq[kFirstThreads / (D / 4)][D];
 };
 
@@ -120,12 +120,18 @@ __global__ void __launch_bounds__(kFirstThreads) tdp_bwd_first_kernel(const __gr
         }
       }
     }
-    // the mass of the exact P brought to that of the forward's
-    float sum = 0.f, sum16 = 0.f;
+    // P: the exact soft-max, with the mass of the forward's scores.  (Not exp2(S - lse2): rounding moves large scores by
+    // more than the exponent's range, and an exponential that overflows cannot be scaled back.)
+    float top = -INFINITY, sum = 0.f, sum16 = 0.f;
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+      if (p.mask.valid(q, j, k0 + e)) top = fmaxf(top, s[e]);
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const bool ok = p.mask.valid(q, j, k0 + e);
-      s[e] = ok ? exp2f(s[e] - lse2) : 0.f;
+      s[e] = ok ? exp2f(s[e] - top) : 0.f;
       sum += s[e];
       sum16 += ok ? exp2f(s16[e] - lse2) : 0.f;
     }
@@ -134,15 +140,19 @@ __global__ void __launch_bounds__(kFirstThreads) tdp_bwd_first_kernel(const __gr
       sum += __shfl_xor_sync(0xffffffffu, sum, o);
       sum16 += __shfl_xor_sync(0xffffffffu, sum16, o);
     }
-    if ((tid & 31) == 0) sh.mass[tid >> 5] = make_float2(sum, sum16);
+    if ((tid & 31) == 0) sh.mass[tid >> 5] = make_float3(top, sum, sum16);
     __syncthreads();
+    float row_top = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kFirstThreads / 32; ++w) row_top = fmaxf(row_top, sh.mass[w].x);
     sum = sum16 = 0.f;
 #pragma unroll
     for (int w = 0; w < kFirstThreads / 32; ++w) {
-      sum += sh.mass[w].x;
-      sum16 += sh.mass[w].y;
+      const float3 m = sh.mass[w];
+      sum += m.x == -INFINITY ? m.y : m.y * exp2f(m.x - row_top);   // (a warp without a pair: 0; a NaN stays one)
+      sum16 += m.z;
     }
-    const float c = sum > 0.f ? sum16 / sum : 1.f;   // (nothing attended: P is zero; NaN: it stays)
+    const float c = sum > 0.f ? exp2f(top - row_top) * (sum16 / sum) : 1.f;   // (nothing attended: P is zero; NaN: it stays)
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int k = k0 + e;

@@ -197,3 +197,23 @@ def test_calls_in_turn_on_the_same_buffers(T, D, dtype):
     for i, g in enumerate(results):
         for name, a, b in zip(NAMES, g, want[i & 1]):
             assert float((a.float() - b.float()).norm()) <= 2e-3 * float(b.float().norm()), (i, name)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,dtype,scale", [(64, torch.bfloat16, 16.0), (128, torch.bfloat16, 24.0), (128, torch.float16, 24.0),
+                                           (64, torch.float32, 24.0)])
+@pytest.mark.parametrize("T", [8, 300])
+def test_scores_past_the_exponents_range_stay_finite(T, D, dtype, scale):
+    """Scores of order 1e5 to 1e6, which rounding moves by hundreds: the exponential of an exact score less the
+    log-sum-exp of rounded ones overflows.  All gradients are finite, and dV2 is what probabilities can give."""
+    g = torch.Generator().manual_seed(T + D)
+    t = [torch.randn(1, 8, T, D, generator=g) for _ in range(6)]
+    t = [(x * scale if i < 3 else x).to(dtype).to(DEV) for i, x in enumerate(t)]
+    do = t.pop()
+    got = _backward(t, do, 1.0, True)
+    for name, x in zip(NAMES, got):
+        assert torch.isfinite(x).all(), f"{name}: {int((~torch.isfinite(x)).sum())} of {x.numel()} values are not finite"
+    # every P is at most 1 but for the fp32 rounding of a score in its exponent (1e6 * 2^-24 * a few: less than 1 in log2)
+    silu = torch.nn.functional.silu(t[3].float()).abs().amax()
+    bound = 2 * silu * do.float().abs().sum(2, keepdim=True)
+    assert (got[4].float().abs() <= bound).all()
