@@ -9,6 +9,10 @@
 // c brings P to the mass that the forward's scores (A rounded to the inputs' type) have under the saved log-sum-exp, 1 for a
 // whole soft-max: exp2(S - lse2) of a query of few pairs and large scores does not sum to one (dV2 1.05 to 1.19 times as
 // far from fp64 as with the forward's scores, for scores of order 4 and T=50 to 120), and overflows for scores of order 1e5.
+// Dq is the exact sum P dP: dO . O has the forward's rounding of SiLU(V1) and of O, which dP has not, and a query of one
+// dominant pair is left with that difference as its dS (16 heads, T=2 to 12, scores of order 3 to 10: dQ 5e-3 to 9e-3 of its
+// norm from fp64 in bf16, 6e-4 to 1.3e-3 in fp16; with the exact sum the rounding of the result to 16 bits is what is left,
+// 1.7e-3 and 2.1e-4).
 // It is latency that counts (it runs ahead of the tensor-core kernel), so every query has a CTA, which adds its share to the
 // sums: about 8 us at 4 heads, D=128 and at 16 heads, D=64.  (The general CUDA-core kernel, which walks a query's rows one
 // tile after the other, took 60 and 50 us for twice as many queries, this one 12.5 and 18 us for those.)
@@ -25,7 +29,7 @@ template <int D, int NF> struct FirstShared {   // NF: queries below this, and s
   float k1[NF][kPitch], s1[NF][kPitch], a[NF][kPitch], b[NF][kPitch];
   float p_kj[NF][NF + 4], ds_kj[NF][NF + 4];   // [k][j], and transposed
   float p_jk[NF][NF + 4], ds_jk[NF][NF + 4];
-  float3 mass[kFirstThreads / 32];   // (each warp's largest score, sum, and sum of the forward's scores)
+  float4 mass[kFirstThreads / 32];   // (each warp's largest score, sum of P, of the forward's P, and of P dP)
   float q[D], d_o[D], dq[kFirstThreads / (D / 4)][D];
 };
 
@@ -100,7 +104,7 @@ __global__ void __launch_bounds__(kFirstThreads) tdp_bwd_first_kernel(const __gr
   {
     constexpr int E = NF * NF / kFirstThreads;
     const int j = tid % NF, k0 = tid / NF * E;
-    const float lse2 = __ldg(p.lse + (size_t)bh * p.T + q) * kLog2e, Dq = __ldg(p.drow + (size_t)bh * p.T + q);
+    const float lse2 = __ldg(p.lse + (size_t)bh * p.T + q) * kLog2e;
     const bool single = p.mask.single_pair(q);   // (its score gradient is exactly zero)
     float s[E], s16[E], dp[E];
 #pragma unroll
@@ -122,7 +126,7 @@ __global__ void __launch_bounds__(kFirstThreads) tdp_bwd_first_kernel(const __gr
     }
     // P: the exact soft-max, with the mass of the forward's scores.  (Not exp2(S - lse2): rounding moves large scores by
     // more than the exponent's range, and an exponential that overflows cannot be scaled back.)
-    float top = -INFINITY, sum = 0.f, sum16 = 0.f;
+    float top = -INFINITY, sum = 0.f, sum16 = 0.f, sum_dp = 0.f;
 #pragma unroll
     for (int e = 0; e < E; ++e)
       if (p.mask.valid(q, j, k0 + e)) top = fmaxf(top, s[e]);
@@ -134,25 +138,32 @@ __global__ void __launch_bounds__(kFirstThreads) tdp_bwd_first_kernel(const __gr
       s[e] = ok ? exp2f(s[e] - top) : 0.f;
       sum += s[e];
       sum16 += ok ? exp2f(s16[e] - lse2) : 0.f;
+      if (s[e] != 0.f) sum_dp = fmaf(s[e], dp[e], sum_dp);
     }
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) {
       sum += __shfl_xor_sync(0xffffffffu, sum, o);
       sum16 += __shfl_xor_sync(0xffffffffu, sum16, o);
+      sum_dp += __shfl_xor_sync(0xffffffffu, sum_dp, o);
     }
-    if ((tid & 31) == 0) sh.mass[tid >> 5] = make_float3(top, sum, sum16);
+    if ((tid & 31) == 0) sh.mass[tid >> 5] = make_float4(top, sum, sum16, sum_dp);
     __syncthreads();
     float row_top = -INFINITY;
 #pragma unroll
     for (int w = 0; w < kFirstThreads / 32; ++w) row_top = fmaxf(row_top, sh.mass[w].x);
-    sum = sum16 = 0.f;
+    sum = sum16 = sum_dp = 0.f;
 #pragma unroll
     for (int w = 0; w < kFirstThreads / 32; ++w) {
-      const float3 m = sh.mass[w];
-      sum += m.x == -INFINITY ? m.y : m.y * exp2f(m.x - row_top);   // (a warp without a pair: 0; a NaN stays one)
+      const float4 m = sh.mass[w];
+      const float f = m.x == -INFINITY ? 1.f : exp2f(m.x - row_top);   // (a warp without a pair: 0; a NaN stays one)
+      sum = fmaf(m.y, f, sum);
       sum16 += m.z;
+      if (f != 0.f) sum_dp = fmaf(m.w, f, sum_dp);
     }
     const float c = sum > 0.f ? exp2f(top - row_top) * (sum16 / sum) : 1.f;   // (nothing attended: P is zero; NaN: it stays)
+    // Dq = sum P dP where P is the whole soft-max (to 2^-11: its mass has the fp32 rounding of a score in the exponent), else
+    // the given dO . O, the sum over all that the log-sum-exp counts
+    const float Dq = fabsf(sum16 - 1.f) < 0x1p-11f ? sum_dp / sum : __ldg(p.drow + (size_t)bh * p.T + q);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int k = k0 + e;

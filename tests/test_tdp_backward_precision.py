@@ -188,3 +188,23 @@ def test_first_queries_with_large_scores(T, D, windows, dtype):
     ratios = _errors(T, D, dtype, True, True, windows, seeds=(0, 1, 2), std=(3, 1, 1, 1))
     print(T, D, dtype, windows, " ".join(f"{n} {r:.2f}" for n, r in ratios))
     assert all(r <= SPREAD for _, r in ratios), f"errors over those of the precision class: {ratios}"
+
+
+@pytest.mark.parametrize("T", [2, 5, 12])
+@pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (128, torch.bfloat16), (64, torch.float16), (128, torch.float16)])
+def test_few_queries_of_large_scores_are_exact(T, D, dtype):
+    """Sequences that the exact first queries take alone, with scores of order 3 to 10, so that in most rows one pair has
+    nearly all the mass and dP - Dq cancels.  Everything is formed in fp32, so the gradients of 16 heads together are as far
+    from fp64 as rounding them to the 16-bit type may put them (u at most, 0.42 u in the mean; the fp32 sums need the rest)."""
+    x = [t.to(DEV) for t in orc.make_inputs(1, 16, T, D, scale=1.5, seed=T + D, dtype=dtype)]
+    do = x.pop()
+    o, lse = torch.empty_like(do), torch.empty(1, 16, T, device=DEV)
+    _native.tdp_fwd(*x, o, lse, 0.125, True, None, None, None, None)
+    g = [torch.empty_like(do) for _ in range(5)]
+    _native.tdp_bwd(*x, o, do, lse, *g, 0.125, True, None, None, None, None)
+    ok = _mask(T, True, (None,) * 4)
+    want = [torch.stack(t) for t in zip(*(_exact([t[0, h] for t in x], do[0, h], 0.125, ok) for h in range(16)))]
+    u = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    for name, a, b in zip(NAMES, g, want):
+        err = float((a[0].double() - b).norm() / b.norm())
+        assert err <= u, f"{name}: {err:.2e} of the norm, more than {u:.1e}"
