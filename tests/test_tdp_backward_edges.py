@@ -63,6 +63,15 @@ def test_exact_first_queries_are_the_first_queries_of_the_sequence(T, q_mod, dty
     assert _native.tdp_bwd_plan(14, 64, dtype, True, None, None, None, None) == (14, 0, 0)
 
 
+@pytest.mark.parametrize("T,windows,first", [
+    (1500, (None,) * 4, 32), (1000, (None,) * 4, 16), (479, (9, 5, 3, 2), 16), (480, (9, 5, 3, 2), 0), (1024, (127, 0, 1, 1), 0),
+    (1023, (127, 0, 1, 1), 16), (4096, (None, 0, 9, 9), 32), (40, (0, 4, 4, 4), 0), (39, (0, 4, 4, 4), 16), (12, (None,) * 4, 12)])
+@pytest.mark.parametrize("dtype", [_native.BF16, _native.F16])
+def test_narrow_windows_have_no_first_queries(T, windows, first, dtype):
+    """Where no query has more than T / 8 pairs the first ones are no larger than the others."""
+    assert _native.tdp_bwd_plan(T, 64, dtype, True, *windows, 1, 0)[0] == first
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("T,q_mod", [(1030, 8), (1024, 64)])
 def test_shards_with_exact_first_queries_sum_to_the_whole(T, q_mod):

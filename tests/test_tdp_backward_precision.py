@@ -150,7 +150,8 @@ def test_a_workspace_without_the_statistics_is_accepted():
 @pytest.mark.parametrize("unit", [True, False])
 @pytest.mark.parametrize("T,D,causal,windows", [
     (192, 64, True, (None,) * 4), (330, 128, True, (None,) * 4), (300, 64, False, (None,) * 4), (200, 128, False, (None,) * 4),
-    (400, 64, True, (128, 128, 32, 32)), (350, 128, True, (40, 100, 20, 9)), (350, 64, True, (9, 5, 3, 2))])
+    (400, 64, True, (128, 128, 32, 32)), (350, 128, True, (40, 100, 20, 9)), (350, 64, True, (9, 5, 3, 2)),
+    (480, 64, True, (9, 5, 3, 2)), (150, 128, True, (3, 2, 1, 2)), (200, 64, True, (0, 24, 24, 24))])
 def test_errors_are_those_of_the_precision_class(T, D, causal, windows, dtype, unit):
     """All five gradients, scores of order 1 to 10 and of order 0.01."""
     ratios = _errors(T, D, dtype, unit, causal, windows)
