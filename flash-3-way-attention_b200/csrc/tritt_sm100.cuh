@@ -46,6 +46,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// One look at a phase, without suspending the thread: issued ahead of work that hides its latency.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Wait limit: every wait in these kernels gives up after this many clock ticks (about a
 // second) and reports failure instead of spinning forever.
 constexpr long long kWaitTicks = 2000000000LL;
@@ -70,6 +83,22 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return mbar_wait_limit(bar, parity, abort_flag, kWaitTicks);
 }
 
+// The same with the limit as a number of looks: less code than with the clock (waits are inlined in many places and the
+// instruction caches are small) and fewer issue slots taken from the warps beside the waiting one; the abort flag is looked at
+// every 64 of them.  A look takes some 30 to 100 clock ticks, so the limit is about a second.  The backward kernel is faster
+// with it (16 heads T=512 D=64 not causal 1.83 -> 1.76 ms, windows 128/128/32/32 at T=2048 1.20 -> 1.13 ms), the forward ones
+// are not (band kernel 0.47 -> 0.49 ms).
+__device__ __forceinline__ bool mbar_wait_looks(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  uint32_t looks = 0;
+  while (!mbar_try_wait(bar, parity)) {
+    if (++looks % 64 == 0) {
+      if (looks >= 1u << 24) *abort_flag = 1;
+      if (*abort_flag) return false;
+    }
+  }
+  return true;
+}
+
 // Hardware barrier over all threads of the cluster: every thread of every block of it must come here.
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -90,6 +119,13 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
       ::"r"(smem_u32(smem_dst)), "l"((uint64_t)m), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
       : "memory");
+}
+
+// Copy of contiguous bytes (both addresses and the size multiples of 16)
+__device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem_dst)),
+               "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
 }
 
 // Tile reduce-add from shared memory into global memory (element type and swizzle come from the
@@ -273,13 +309,36 @@ __device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&r)
                : "r"(taddr)
                : "memory");
 }
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
 // width-generic wrappers
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[8]) { tmem_ld8(taddr, r); }
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
 __device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[8]) { tmem_st8(taddr, r); }
 __device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[16]) { tmem_st16(taddr, r); }
 __device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[32]) { tmem_st32(taddr, r); }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// The same where other work lies between the load and its wait: the registers are operands, so that no use of them moves ahead.
+template <int N> __device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[N]) {
+  static_assert(N % 8 == 0, "register count");
+  tmem_wait_ld();
+#pragma unroll
+  for (int i = 0; i < N; i += 8)
+    asm volatile("" : "+r"(r[i]), "+r"(r[i + 1]), "+r"(r[i + 2]), "+r"(r[i + 3]), "+r"(r[i + 4]), "+r"(r[i + 5]), "+r"(r[i + 6]),
+                 "+r"(r[i + 7]));
+}
+template <int N, int M> __device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[N], uint32_t (&q)[M]) {
+  tmem_wait_ld(r);
+#pragma unroll
+  for (int i = 0; i < M; i += 8)
+    asm volatile("" : "+r"(q[i]), "+r"(q[i + 1]), "+r"(q[i + 2]), "+r"(q[i + 3]), "+r"(q[i + 4]), "+r"(q[i + 5]), "+r"(q[i + 6]),
+                 "+r"(q[i + 7]));
+}
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ------------------------------------------------------------------ shared memory fragments

@@ -24,6 +24,17 @@ template <> __device__ __forceinline__ float2 unpack2<__half>(uint32_t v) {
   return __half22float2(*reinterpret_cast<__half2*>(&v));
 }
 
+// The products of two pairs, rounded once (a product is exact in fp32, so the same as a multiplication there and a rounding).
+template <typename T16> __device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b);
+template <> __device__ __forceinline__ uint32_t mul2<__nv_bfloat16>(uint32_t a, uint32_t b) {
+  const __nv_bfloat162 v = __hmul2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+template <> __device__ __forceinline__ uint32_t mul2<__half>(uint32_t a, uint32_t b) {
+  const __half2 v = __hmul2(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
 // Bits c of [lo, hi] among 0..31: with a mask of a row's columns a per-element test is one logic instruction (a constant
 // bit into a predicate) instead of two comparisons.
 __device__ __forceinline__ uint32_t column_mask(int lo, int hi) {

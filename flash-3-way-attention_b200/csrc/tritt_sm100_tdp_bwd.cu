@@ -3,8 +3,8 @@
 // The score S[q,j,k] = alpha sum_h Q[q,h] K1[j,h] K2[k,h] and the gated value are trilinear, so any of the three
 // indices can be the one that is stepped over.  Here it is k: for one k the (q, j) plane is an ordinary attention
 // backward whose key and value operands carry the k-th rows of K2 and V2,
-//     A [j,h] = alpha*log2(e) * K1[j,h] * K2[k,h]      A'[j,h] = SiLU(V1)[j,h] * V2[k,h]
-//     S  = Q A^T (for large scores R K1^T with R [q,h] = alpha*log2(e) * Q[q,h] * K2[k,h])
+//     A [j,h] = K1[j,h] * K2[k,h]      A'[j,h] = SiLU(V1)[j,h] * V2[k,h]
+//     S  = alpha*log2(e) * Q A^T (for large scores R K1^T with R [q,h] = alpha*log2(e) * Q[q,h] * K2[k,h])
 //                         P  = exp2(S - lse2[q])       (recomputed from the saved lse)
 //     dP = dO A'^T        dS = P * (dP - Dq[q]),       Dq = sum_h dO O
 // and all five gradients follow from three more products:
@@ -22,8 +22,13 @@
 // fp32 sums that stay in L2).  All steps of a call are laid out in one line and cut in equal parts, one per CTA
 // (every sum is a reduction, so an item may be cut anywhere): no last wave.
 //
-// What bounds it: the soft-max and fold warps' chains of tensor-memory reads, exponentials and shared-memory stores (issue
-// slots 63 % busy at head dimension 64, shared memory 71 %, tensor pipe 33 %; 53 / 67 / 41 % at 128), not a single unit.
+// What bounds it: the fold warps, which are busy all of a step (3200 cycles at head dimension 128, 3800 at 64): chains of
+// tensor-memory reads, shared-memory accesses and waits, each of 100 to 400 cycles while the tensor cores' operand reads keep
+// shared memory busy; at 64 the soft-max warps as well.  Issue slots are 56 to 61 % busy, the tensor pipe 35 to 47 %.
+// Operands formed by one 16-bit product per pair instead of fp32 products and conversions, the products issued by three warps
+// instead of one, A' doubled, exponentials beside the arithmetic of dS, looks at barriers ahead of the waits, and waits without
+// the clock, backward of T=2048 D=128 bf16 16 heads 71.2 -> 64.8 ms, T=4096 D=64 4 heads 80.4 -> 78.1, T=512 D=64 32 heads 1.80 ->
+// 1.70, not causal fp16 16 heads 1.83 -> 1.76, windows 128/128/32/32 at T=2048 1.22 -> 1.14, T=333 D=128 4 heads 189 -> 169 us.
 // Against a query and 128 rows of one key tensor per tile (eight products, exponentials twice), same call, training
 // steps: T=2048 D=128 bf16 16 heads 114.5 -> 94.9 ms, T=4096 D=64 4 heads 140.5 -> 113.8 ms, T=512 D=64 fp16 16 heads 2.37
 // -> 1.59 ms, windows 128/128/32/32 at T=2048 4.54 -> 1.77 ms.
@@ -33,9 +38,8 @@
 // [h x j], so that their M extent is 128 (64 + 64 + 64 + 64 + 128); a JT of 128 would need 640 columns.
 //
 // CTA: 20 warps.  0-3 and 4-7: soft-max warpgroups (half of a step's columns each, one query per thread); 8-11: forms
-// A and folds G; 12-15: forms A' and folds U; 16: issues the products; 17: TMA and the K2 / V2 rows; 18,
-// 19: R.  P and dS are written to shared memory, where both the transposed (U, G) and the plain (dQ) product can read them.
-// Order of the products of step n:   S(n+1)  U(n)  dP(n+1)  dQ(n)  G(n).
+// A and folds G; 12-15: forms A' and folds U; 16, 18, 19: issue the products S and dP, U, dQ and G (large scores: 16 all five,
+// 18 and 19 form R); 17: TMA and the K2 / V2 rows.  P and dS are written to shared memory, where both the transposed (U, G) and the plain (dQ) product can read them.
 #include "tritt_sm100_tdp.cuh"
 
 #include <atomic>
@@ -47,10 +51,15 @@ using namespace sm100;
 
 constexpr int kBwdThreads = 640;
 // Registers per thread: 640 threads are launched with 96 each (480 per lane of the five warpgroups) and split them anew.  The
-// shares are tight: a body spills 84 to 204 bytes a thread (-Xptxas -v gives the sum over the two), counters and addresses
-// that a step reads once or twice.
-constexpr int kRegsLaunch = 96, kRegsSoftmax = 80, kRegsFold = 128, kRegsService = 64;
-static_assert(2 * kRegsSoftmax + 2 * kRegsFold + kRegsService <= 5 * kRegsLaunch, "more registers than the launch has");
+// shares are tight: the two bodies spill 360 to 620 bytes a thread together, most of it what an item or a step reads once or
+// twice.  (80 / 128 / 64 or 96 / 120 / 48 for soft-max, fold and service warps: 5 to 8 % slower, as their loops spill.)
+constexpr int kRegsLaunch = 96;
+// (Large scores at head dimension 128 have the service warps form 32 KB of R per step, and soft-max warps that hold half as many
+// columns as at 64: with 48 registers those service warps spill, 1.60 -> 1.90 ms at 16 heads of T=512.)
+template <int D, bool LARGE> struct BwdRegs {
+  static constexpr int kSoftmax = D == 128 && LARGE ? 80 : 88, kFold = 128, kService = D == 128 && LARGE ? 64 : 48;
+  static_assert(2 * kSoftmax + 2 * kFold + kService <= 5 * kRegsLaunch, "more registers than the launch has");
+};
 constexpr int kVecBatch = 4;     // K2 / V2 rows per hand-over
 constexpr int kVecSlots = 4;     // batches in flight
 // S = Q A^T rounds the product K1 K2 where the forward rounds R = Q K2, so that P does not match the saved log-sum-exp and no
@@ -78,10 +87,10 @@ template <int D> struct BwdCfg {
   static constexpr int kOffP = kOffA + 3 * kTileJ;    // P | dS (two buffers)
   // R (see tdp_bwd_body), in blocks of 64 columns: over the SiLU(V1) tile, and behind P | dS
   static constexpr int kOffR0 = kOffK1 + kTileJ, kOffR1 = kOffP + 3 * kTileP;
-  static constexpr int kOffVec = kOffR1 + (D / 64 - 1) * 16384;  // [slot][row][scale_k * K2 | scale_v * V2] fp32
-  static constexpr int kVecRow = 2 * D;               // floats
-  static constexpr int kOffBars = kOffVec + kVecSlots * kVecBatch * kVecRow * 4;
-  static constexpr int kSmem = kOffBars + 448;
+  static constexpr int kOffVec = kOffR1 + (D / 64 - 1) * 16384;  // [slot][K2 rows | V2 rows][row of the batch][D], 16-bit
+  static constexpr int kVecPart = kVecBatch * D * 2;  // bytes of a batch of rows of one tensor
+  static constexpr int kOffBars = kOffVec + kVecSlots * 2 * kVecPart;
+  static constexpr int kSmem = kOffBars + 512;
   static constexpr int kTmemS = 0, kTmemDP = JT, kTmemG = 2 * JT, kTmemU = kTmemG + 64, kTmemDQ = kTmemU + 64;
   static constexpr int kTmemQ = kTmemDQ + D, kTmemDO = kTmemQ + D / 2;   // 16-bit, two elements a column
   static_assert(kTmemDO + D / 2 <= 512 && kSmem <= 232448, "tensor / shared memory");
@@ -132,7 +141,8 @@ struct BwdParams {
 
 struct BwdItem {
   int bh, qt, jt, k0, len, flags;   // len 0: no more items
-  int ea, eb;                       // A and A' carry factors 2^ea and 2^eb (range_shift)
+  int ea, eb;                       // A and A' carry factors 2^ea and 2^eb (range_shift), R 2^er (product_shift)
+  int er, pad_[3];
 };
 enum {
   kFirstOfQ = 1, kLastOfQ = 2,   // the first / last item of a run over the j-tiles of one q-tile
@@ -144,7 +154,7 @@ struct BwdBarriers {
   alignas(16) BwdItem items[kItemSlots];
   uint64_t tile_full, tile_free;            // Q, dO, K1, SiLU(V1) of an item
   uint64_t vec_full[kVecSlots], vec_empty[kVecSlots];
-  uint64_t a_ready[2], a_free[2], r_ready, ap_ready;  // A: doubled by step parity (its producer may be two steps ahead)
+  uint64_t a_ready[2], a_free[2], ap_ready[2], ap_free[2], r_ready;  // doubled by step parity (a producer may be two steps ahead)
   uint64_t s_ready, s_free, p_ready, dp_ready, ds_ready, ds_free[2];
   uint64_t acc_done[2], acc_free[2];         // G, U
   uint64_t qdo_ready, dq_done, dq_free;
@@ -201,7 +211,7 @@ struct BwdWalk {
   }
   // hands out the item found last and looks for the one after it
   __device__ BwdItem next(const BwdItem& prev) {
-    BwdItem it{bh, qt, jt, k0, len, 0, 0, 0};
+    BwdItem it{bh, qt, jt, k0, len, 0, 0, 0, 0, {0, 0, 0}};
     if (len == 0) return it;
     if (bh != prev.bh || qt != prev.qt) it.flags |= kFirstOfQ;
     step();
@@ -227,11 +237,21 @@ __device__ __forceinline__ int prob_shift(int q, int causal, int T, int k1w, int
   return 0;
 }
 
-// fp16 only: A = alpha log2(e) K1 K2 and A' = SiLU(V1) V2 are products of two small factors (keys of 0.01: 1e-6, against
-// a smallest normal value of 6e-5) or of two large ones (beyond 65504 from 256 on), so they are formed times a power of
-// two per head that puts the largest product the head's elements allow into [2^14, 2^15): 28 binades below it stay normal.
+// fp16 only: A = K1 K2 and A' = SiLU(V1) V2 are products of two small factors (keys of 0.01: 1e-4, against a smallest normal
+// value of 6e-5) or of two large ones (beyond 65504 from 256 on), so one factor, x, is taken times a power of two per head:
+// the largest that keeps both itself and the largest product the head's elements allow below 2^15.  With the other factor's
+// largest element at 1 or above the largest product has 28 binades of normal numbers below it, at 2^-b 28 - b.
 // The power is divided out in fp32, of S and dP in the soft-max warps and of the sums.  bf16 has fp32's range: 0.
-template <typename T16> __device__ __forceinline__ int range_shift(float bound) {
+template <typename T16> __device__ __forceinline__ int range_shift(float x, float other) {
+  if constexpr (std::is_same<T16, __half>::value) {
+    if (!(x > 0.f) || !isfinite(x) || !(other > 0.f) || !isfinite(other)) return 0;
+    const int a = (__float_as_int(x) >> 23) - 127, b = (__float_as_int(other) >> 23) - 127;
+    return 14 - a - max(b + 1, 0);
+  }
+  return 0;
+}
+// The same for R = alpha log2(e) Q K2, which is formed in fp32: the largest product is brought to [2^14, 2^15).
+template <typename T16> __device__ __forceinline__ int product_shift(float bound) {
   if constexpr (std::is_same<T16, __half>::value) {
     if (!(bound > 0.f) || !isfinite(bound)) return 0;
     return min(80, max(-80, 14 - ((__float_as_int(bound) >> 23) - 127)));
@@ -305,7 +325,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
   using Cfg = BwdCfg<D>;
   constexpr int JT = Cfg::JT, CW = Cfg::CW;
   extern __shared__ __align__(1024) uint8_t smem[];
-  static_assert(sizeof(BwdBarriers) <= 448, "barrier block too large");
+  static_assert(sizeof(BwdBarriers) <= 512, "barrier block too large");
   BwdBarriers& bars = *reinterpret_cast<BwdBarriers*>(smem + Cfg::kOffBars);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (smem_u32(smem) & 1023u) {
@@ -316,18 +336,19 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
   if (tid == 0) {
     bars.abort_flag = 0;
     mbar_init(&bars.tile_full, 1);
-    mbar_init(&bars.tile_free, 1 + 8);   // the item's last product, and the fold warps (they read K1, SiLU(V1))
+    mbar_init(&bars.tile_free, (LARGE ? 1 : 3) + 8);   // the item's last products, and the fold warps (they read K1, SiLU(V1))
     for (int i = 0; i < kVecSlots; ++i) {
-      mbar_init(&bars.vec_full[i], 32);
+      mbar_init(&bars.vec_full[i], 1);
       mbar_init(&bars.vec_empty[i], 8);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars.a_ready[i], 4);
       mbar_init(&bars.a_free[i], 1);
+      mbar_init(&bars.ap_ready[i], 4);
+      mbar_init(&bars.ap_free[i], 1);
       mbar_init(&bars.ds_free[i], 1);
     }
     mbar_init(&bars.r_ready, 2);
-    mbar_init(&bars.ap_ready, 4);
     mbar_init(&bars.s_ready, 1);
     mbar_init(&bars.s_free, 8);
     mbar_init(&bars.p_ready, 8);
@@ -355,7 +376,16 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
   const int T = g.T;
   // (every lane waits; the vote keeps the warp converged whatever a lane's wait returned)
   auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+    return __all_sync(0xffffffffu, LARGE ? mbar_wait(bar, parity, abort_flag) : mbar_wait_looks(bar, parity, abort_flag));
+  };
+  // the same for two barriers at once: half of the lanes look at each
+  auto wait_two = [&](uint64_t* b0, uint32_t p0, uint64_t* b1, uint32_t p1) -> bool {
+    const bool ok = wait_all(lane & 1 ? b1 : b0, lane & 1 ? p1 : p0);
+    __syncwarp();
+    return ok;
+  };
+  auto test_two = [&](uint64_t* b0, uint32_t p0, uint64_t* b1, uint32_t p1) -> bool {
+    return mbar_test(lane & 1 ? b1 : b0, lane & 1 ? p1 : p0);
   };
   // one arrival per warp, after the caller's fences
   auto arrive_warp = [&](uint64_t* bar) {
@@ -370,11 +400,12 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
     const int4 a = *reinterpret_cast<const int4*>(&bars.items[items % kItemSlots]);
     const int4 b = *reinterpret_cast<const int4*>(&bars.items[items % kItemSlots].len);
     it.bh = a.x; it.qt = a.y; it.jt = a.z; it.k0 = a.w; it.len = b.x; it.flags = b.y; it.ea = b.z; it.eb = b.w;
+    if (LARGE) it.er = bars.items[items % kItemSlots].er;
     return it.len > 0;
   };
 
   if (warp < 8) {
-    set_regs<kRegsLaunch, kRegsSoftmax>();
+    set_regs<kRegsLaunch, BwdRegs<D, LARGE>::kSoftmax>();
     // ------------------------------------------------------------------ soft-max warpgroups
     const int wg = warp >> 2, wq = warp & 3;
     const int row = wq * 32 + lane;
@@ -385,9 +416,11 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
     bool alive = true;
     BwdItem it;
     int q = 0;
-    bool q_ok = false, single = false;
+    bool q_ok = false, single = false, s_seen = false;
     float lse2 = 0.f, drow = 0.f, dq_scale = 0.f;
-    constexpr bool kShifted = std::is_same<T16, __half>::value;   // (S and dP carry factors 2^ea and 2^eb)
+    // S and dP carry factors: in fp16 powers of two, and S = Q A^T lacks alpha * log2(e), which R carries
+    constexpr bool kScaled = !LARGE || std::is_same<T16, __half>::value;
+    constexpr int H = CW / 2;
     while (alive && next_item(items, it, alive)) {
       ++items;
       if (it.flags & kFirstOfQ) {
@@ -400,7 +433,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
         lse2 = q_ok ? __ldg(p.lse + (size_t)it.bh * T + q) * kLog2e - (float)e : 0.f;
         const int f = it.flags >> kShiftBits;
         drow = q_ok ? __ldg(p.drow + (size_t)it.bh * T + q) * pow2i<T16>(f) : 0.f;
-        dq_scale = pow2i<T16>(-e - it.ea - f) * kLn2;    // A carries alpha * log2(e)
+        dq_scale = pow2i<T16>(-e - it.ea - f) * p.alpha;
         // A query that attends a single pair has P = 1 and a score gradient of exactly zero (TdpMask::single_pair):
         // P (dP - Dq) has two terms that are equal only up to the 16-bit rounding of the stored output, so its dS
         // is set to zero.
@@ -428,12 +461,15 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
         single = TdpMask{g.causal, T, g.k1w, g.k2w, g.kkl, g.kkr}.single_pair(q);
       }
       const bool any_single = __any_sync(0xffffffffu, single);
-      const float2 nlse = make_float2(-lse2, -lse2), ndq = make_float2(-drow, -drow);
-      const float sa = pow2i<T16>(-it.ea), sb = pow2i<T16>((it.flags >> kShiftBits) - it.eb);
-      // v * scale + add; the scale of bf16 is 1
+      const float2 nlse = make_float2(-lse2, -lse2);
+      const float2 ndq = kScaled && single ? make_float2(0.f, 0.f) : make_float2(-drow, -drow);
+      // (R carries alpha * log2(e), A does not)
+      const float sa = LARGE ? pow2i<T16>(-it.er) : pow2i<T16>(-it.ea) * (p.alpha * kLog2e);
+      const float sb = single ? 0.f : pow2i<T16>((it.flags >> kShiftBits) - it.eb);
+      // v * scale + add; without the scale where it is 1
       auto scaled = [](uint32_t v0, uint32_t v1, float scale, float2 add) {
         const float2 v = make_float2(__uint_as_float(v0), __uint_as_float(v1));
-        return kShifted ? __ffma2_rn(v, make_float2(scale, scale), add) : __fadd2_rn(v, add);
+        return kScaled ? __ffma2_rn(v, make_float2(scale, scale), add) : __fadd2_rn(v, add);
       };
       const int j0 = it.jt * JT + wg * CW;
       for (int i = 0; i < it.len; ++i, ++n) {
@@ -445,81 +481,95 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
           hi = k <= q && q - k <= g.k2w ? min(q, k + g.kkr) - j0 : lo - 1;
         }
         if (!q_ok) hi = lo - 1;
-        // 32 columns at a time: S -> P, then dP and P (still in fp32) -> dS
-        alive = wait_all(&bars.s_ready, n & 1);
+        // Half of the columns S -> P; then, eight columns at a time, the other half S -> P beside dP and P (still in fp32) ->
+        // dS of the first, so that exponentials and arithmetic overlap within a warp; then dS of the second half.
+        alive = __all_sync(0xffffffffu, s_seen) || wait_all(&bars.s_ready, n & 1);
         if (!alive) break;
         tc_fence_after();
+        bool seen = false;   // (looks at barriers ahead of their waits)
         uint8_t* const dsrow = prow + (1 + (n & 1)) * Cfg::kTileP;
         const bool full = __all_sync(0xffffffffu, lo <= 0 && hi >= CW - 1);
-#pragma unroll 1
-        for (int c0 = 0; c0 < CW; c0 += 32) {
-          uint32_t s[32];
-          tmem_ld32(tmem + lane_base + Cfg::kTmemS + wg * CW + c0, s);
-          tmem_wait_ld();
-          if (c0 + 32 == CW) {
+        const uint32_t tS = tmem + lane_base + Cfg::kTmemS + wg * CW, tDP = tmem + lane_base + Cfg::kTmemDP + wg * CW;
+        constexpr int SN = D == 128 ? H : 8;   // (head dimension 64 has no registers for all of them)
+        uint32_t s[H], sn[SN], dp[8];   // scores, then P; scores of the second half; dP
+        // columns c.. of S -> P
+        auto to_p = [&](int c, uint32_t* v, const uint32_t* x) {
+          if (full) {
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+              const float2 y = scaled(x[e], x[e + 1], sa, nlse);
+              v[e] = __float_as_uint(exp2f(y.x));
+              v[e + 1] = __float_as_uint(exp2f(y.y));
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              v[e] = c + e >= lo && c + e <= hi ? __float_as_uint(exp2f(fmaf(__uint_as_float(x[e]), sa, -lse2))) : 0u;
+          }
+        };
+        auto put = [&](uint8_t* row_base, int c, const uint32_t* v) {
+          uint32_t w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) w[e] = pack2<T16>(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));
+          *reinterpret_cast<uint4*>(row_base + swz128(row, ch0 + (c >> 3))) = make_uint4(w[0], w[1], w[2], w[3]);
+        };
+        // columns c..: P in v and dP in dp -> dS
+        auto to_ds = [&](int c, const uint32_t* v) {
+          uint32_t w[8];
+#pragma unroll
+          for (int e = 0; e < 8; e += 2) {
+            float2 pv = make_float2(__uint_as_float(v[e]), __uint_as_float(v[e + 1]));
+            if (!kScaled && any_single) pv = single ? make_float2(0.f, 0.f) : pv;
+            const float2 ds = __fmul2_rn(pv, scaled(dp[e], dp[e + 1], sb, ndq));
+            w[e] = __float_as_uint(ds.x);
+            w[e + 1] = __float_as_uint(ds.y);
+          }
+          put(dsrow, c, w);
+        };
+        tmem_ld(tS, s);
+        tmem_wait_ld(s);
+        seen = mbar_test(&bars.acc_done[1], (n & 1) ^ 1);
+        tmem_ld(tS + H, sn);
+#pragma unroll
+        for (int c = 0; c < H; c += 8) to_p(c, s + c, s + c);
+        // the previous step's U has read P
+        alive = __all_sync(0xffffffffu, seen) || wait_all(&bars.acc_done[1], (n & 1) ^ 1);
+        if (!alive) break;
+        seen = test_two(&bars.dp_ready, n & 1, &bars.ds_free[n & 1], ((n >> 1) & 1) ^ 1);
+#pragma unroll
+        for (int c = 0; c < H; c += 8) put(prow, c, s + c);
+        alive = __all_sync(0xffffffffu, seen) || wait_two(&bars.dp_ready, n & 1, &bars.ds_free[n & 1], ((n >> 1) & 1) ^ 1);
+        if (!alive) break;
+        tc_fence_after();
+        tmem_ld(tDP, dp);
+#pragma unroll
+        for (int c = 0; c < H; c += 8) {
+          tmem_wait_ld(sn, dp);
+          if (SN == H ? c == 0 : c + 8 == H) {
             // the scores are in registers: the next step's product may overwrite them
             tc_fence_before();
             arrive_warp(&bars.s_free);
           }
-          if (full) {
+          uint32_t x[8];
+          to_ds(c, s + c);
 #pragma unroll
-            for (int c = 0; c < 32; c += 2) {
-              const float2 x = scaled(s[c], s[c + 1], sa, nlse);
-              s[c] = __float_as_uint(exp2f(x.x));
-              s[c + 1] = __float_as_uint(exp2f(x.y));
-            }
-          } else {
-#pragma unroll
-            for (int c = 0; c < 32; ++c)
-              s[c] = c0 + c >= lo && c0 + c <= hi ? __float_as_uint(exp2f(fmaf(__uint_as_float(s[c]), sa, -lse2))) : 0u;
+          for (int e = 0; e < 8; ++e) x[e] = sn[SN == H ? c + e : e];
+          tmem_ld(tDP + c + 8, dp);
+          if constexpr (SN == 8) {
+            if (c + 8 < H) tmem_ld(tS + H + c + 8, sn);
           }
-          if (c0 == 0) {
-            // the previous step's U has read P
-            alive = wait_all(&bars.acc_done[1], (n & 1) ^ 1);
-            if (!alive) break;
-          }
-#pragma unroll
-          for (int c = 0; c < 32; c += 8) {
-            uint32_t w[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              w[e] = pack2<T16>(__uint_as_float(s[c + 2 * e]), __uint_as_float(s[c + 2 * e + 1]));
-            *reinterpret_cast<uint4*>(prow + swz128(row, ch0 + ((c0 + c) >> 3))) = make_uint4(w[0], w[1], w[2], w[3]);
-          }
-          if (c0 + 32 == CW) {
-            fence_async_smem();
-            arrive_warp(&bars.p_ready);
-          }
-          if (any_single) {
-#pragma unroll
-            for (int c = 0; c < 32; ++c) s[c] = single ? 0u : s[c];
-          }
-          if (c0 == 0) {
-            alive = wait_all(&bars.dp_ready, n & 1);
-            if (alive) alive = wait_all(&bars.ds_free[n & 1], ((n >> 1) & 1) ^ 1);
-            if (!alive) break;
-            tc_fence_after();
-          }
-#pragma unroll
-          for (int c1 = 0; c1 < 32; c1 += 16) {
-            uint32_t dp[16];
-            tmem_ld16(tmem + lane_base + Cfg::kTmemDP + wg * CW + c0 + c1, dp);
-            tmem_wait_ld();
-#pragma unroll
-            for (int c = 0; c < 16; c += 8) {
-              uint32_t w[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float2 d = scaled(dp[c + 2 * e], dp[c + 2 * e + 1], sb, ndq);
-                const float2 ds = __fmul2_rn(
-                    make_float2(__uint_as_float(s[c1 + c + 2 * e]), __uint_as_float(s[c1 + c + 2 * e + 1])), d);
-                w[e] = pack2<T16>(ds.x, ds.y);
-              }
-              *reinterpret_cast<uint4*>(dsrow + swz128(row, ch0 + ((c0 + c1 + c) >> 3))) = make_uint4(w[0], w[1], w[2], w[3]);
-            }
-          }
+          to_p(H + c, s + c, x);
+          put(prow, H + c, s + c);
         }
-        if (!alive) break;
+        fence_async_smem();
+        arrive_warp(&bars.p_ready);
+        s_seen = mbar_test(&bars.s_ready, (n + 1) & 1);
+#pragma unroll
+        for (int c = 0; c < H; c += 8) {
+          tmem_wait_ld(dp);
+          to_ds(H + c, s + c);
+          if (c + 8 < H) tmem_ld(tDP + H + c + 8, dp);
+        }
         tc_fence_before();
         fence_async_smem();
         arrive_warp(&bars.ds_ready);
@@ -549,7 +599,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       }
     }
   } else if (warp < 16) {
-    set_regs<kRegsLaunch, kRegsFold>();
+    set_regs<kRegsLaunch, BwdRegs<D, LARGE>::kFold>();
     // ------------------------------------------------------------------ operand / fold warpgroups
     // role 0: forms A two steps ahead, folds G into dK1 (registers) and dK2;  role 1: forms A' one step ahead, folds
     // U into dSiLU(V1) and dV2.  The fold reads the accumulator as 16 x 256-bit fragments (thread t: rows t / 4 + 8 i,
@@ -558,9 +608,13 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
     // (the role is a run-time value: one copy of the code for both warpgroups halves what the instruction caches have to
     // hold of it)
     const int role = (warp - 8) >> 2, w = warp & 3;
-    const float* const vec = reinterpret_cast<const float*>(smem + Cfg::kOffVec) + role * D;
+    const T16* const vec = reinterpret_cast<const T16*>(smem + Cfg::kOffVec + role * Cfg::kVecPart);
+    // row of step i of an item whose first batch is vb0
+    auto vec_row = [&](uint32_t vb0, int i) {
+      return vec + ((vb0 + i / kVecBatch) % kVecSlots * 2 * kVecBatch + i % kVecBatch) * D;
+    };
     const uint32_t tacc = tmem + ((uint32_t)(w * 32) << 16) + (role ? Cfg::kTmemU : Cfg::kTmemG);
-    const int ahead = 2 - role;
+    const int ahead = LARGE ? 2 - role : 2;   // (A' has a second buffer, over the SiLU(V1) tile, where R does not need that)
     // address of this lane's row of the four 8 x 8 blocks of (16-column group c16, 16-lane half hl) within a tile
     auto frag = [&](int c16, int hl) -> uint32_t {
       if constexpr (D == 64) {
@@ -590,54 +644,62 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
           else ldmatrix_x4_trans(x[c16][hl], raw_u + frag(c16, hl));
         }
       arrive_warp(&bars.tile_free);
+      const int ex = role ? it.eb : it.ea;   // (x carries 2^ex from here on)
+      if (std::is_same<T16, __half>::value) {
+        const float2 m = make_float2(pow2i<T16>(ex), pow2i<T16>(ex));
+#pragma unroll
+        for (int c16 = 0; c16 < 4; ++c16)
+#pragma unroll
+          for (int b = 0; b < 8; ++b) {
+            const float2 f = __fmul2_rn(unpack2<T16>(x[c16][b >> 2][b & 3]), m);
+            x[c16][b >> 2][b & 3] = pack2<T16>(f.x, f.y);
+          }
+      }
       const int len = it.len;
       const int e = prob_shift<T16>(g.q_rem + max(it.qt * 128, p.i_first) * g.q_mod, g.causal, T, g.k1w, g.k2w);
       const float unshift = pow2i<T16>(-e);
       const float unshift_ds = unshift * pow2i<T16>(-(it.flags >> kShiftBits));
-      const float zscale = role ? unshift : unshift_ds * p.alpha;
+      const float jscale = role ? unshift : unshift_ds * p.alpha;
+      const float zscale = jscale * pow2i<T16>(-ex);
       float* zrow = (role ? p.dv2 : p.dk2) + ((size_t)it.bh * T + it.k0) * D;
       auto form = [&](int i) -> bool {
         const uint32_t m = n + i;
-        if ((i & (kVecBatch - 1)) == 0) {
-          const uint32_t vb = vb0 + i / kVecBatch;
-          if (!wait_all(&bars.vec_full[vb % kVecSlots], (vb / kVecSlots) & 1)) return false;
-        }
-        // A: the buffer's previous step has been through dQ;  A': the previous step's dP product has run
-        if (!wait_all(role ? &bars.dp_ready : &bars.a_free[m & 1], ((role ? m : m >> 1) & 1) ^ 1)) return false;
-        const float* v = vec + ((vb0 * kVecBatch + i) % (kVecSlots * kVecBatch)) * Cfg::kVecRow;
-        const uint32_t dst = formed_u + (role ? 0 : (m & 1) * Cfg::kTileJ);
-        float vr[4];
+        // The operand's buffer: the product of its last step has run (A: two steps before, through dQ; A': dP, two steps before,
+        // or with a single buffer the step before).  At the first row of a batch half of the lanes look whether it is there.
+        const uint32_t mb = LARGE && role ? m - 1 : m, vb = vb0 + i / kVecBatch;
+        uint64_t* const bar = role ? &bars.ap_free[mb & 1] : &bars.a_free[mb & 1];
+        const uint32_t parity = ((mb >> 1) & 1) ^ (LARGE && role ? 0 : 1);
+        const bool first = (i & (kVecBatch - 1)) == 0;
+        if (!wait_two(bar, parity, first ? &bars.vec_full[vb % kVecSlots] : bar, first ? (vb / kVecSlots) & 1 : parity)) return false;
+        const T16* v = vec_row(vb0, i);
+        const uint32_t dst = role == 0 ? formed_u + (m & 1) * Cfg::kTileJ : LARGE || !(m & 1) ? formed_u : raw_u;
+        uint32_t vr[4];   // head dimension 128: twice the element of row r
         if constexpr (D == 128) {
 #pragma unroll
-          for (int r = 0; r < 4; ++r) vr[r] = v[w * 32 + r * 8 + (lane >> 2)];
+          for (int r = 0; r < 4; ++r)
+            vr[r] = __byte_perm(*reinterpret_cast<const uint16_t*>(v + w * 32 + r * 8 + (lane >> 2)), 0, 0x1010);
         }
 #pragma unroll
         for (int c16 = 0; c16 < 4; ++c16) {
-          float2 v0, v1;
+          uint32_t v0 = 0, v1 = 0;
           if constexpr (D == 64) {
-            v0 = *reinterpret_cast<const float2*>(v + c16 * 16 + 2 * (lane & 3));
-            v1 = *reinterpret_cast<const float2*>(v + c16 * 16 + 8 + 2 * (lane & 3));
+            v0 = *reinterpret_cast<const uint32_t*>(v + c16 * 16 + 2 * (lane & 3));
+            v1 = *reinterpret_cast<const uint32_t*>(v + c16 * 16 + 8 + 2 * (lane & 3));
           }
 #pragma unroll
           for (int hl = 0; hl < 2; ++hl) {
             uint32_t a[4];
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-              float2 m2;
-              if constexpr (D == 64) m2 = b < 2 ? v0 : v1;
-              else m2 = make_float2(vr[hl * 2 + (b & 1)], vr[hl * 2 + (b & 1)]);
-              const float2 f = __fmul2_rn(unpack2<T16>(x[c16][hl][b]), m2);
-              a[b] = pack2<T16>(f.x, f.y);
-            }
+            for (int b = 0; b < 4; ++b) a[b] = mul2<T16>(x[c16][hl][b], D == 64 ? (b < 2 ? v0 : v1) : vr[hl * 2 + (b & 1)]);
             if constexpr (D == 64) stmatrix_x4(dst + frag(c16, hl), a);
             else stmatrix_x4_trans(dst + frag(c16, hl), a);
           }
         }
         fence_async_smem();
-        arrive_warp(role ? &bars.ap_ready : &bars.a_ready[m & 1]);
+        arrive_warp(role ? &bars.ap_ready[LARGE ? 0 : m & 1] : &bars.a_ready[m & 1]);
         return true;
       };
-      // (one loop, so that there is one copy of each of the two stages: step i forms operand i, folds step i - ahead)
+      // (one loop, so that there is one copy of each of the two stages: step i0 forms operand i0, folds step i0 - ahead)
       for (int i0 = 0; i0 < len + ahead && alive; ++i0) {
         const int i = i0 - ahead;
         // (keeps the compiler from unpacking x once, outside the loop, into twice the registers)
@@ -645,71 +707,67 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
         for (int c16 = 0; c16 < 4; ++c16)
 #pragma unroll
           for (int b = 0; b < 8; ++b) asm volatile("" : "+r"(x[c16][b >> 2][b & 3]));
+        bool seen = false;   // (a look ahead of the wait)
+        if (i >= 0) seen = mbar_test(&bars.acc_done[role], (n + i) & 1);
         if (i0 < len) {
           alive = form(i0);
           if (!alive) break;
         }
         if (i < 0) continue;
-        alive = wait_all(&bars.acc_done[role], (n + i) & 1);
+        alive = __all_sync(0xffffffffu, seen) || wait_all(&bars.acc_done[role], (n + i) & 1);
         if (!alive) break;
         tc_fence_after();
-        const float* v = vec + ((vb0 * kVecBatch + i) % (kVecSlots * kVecBatch)) * Cfg::kVecRow;
+        const T16* v = vec_row(vb0, i);
         if constexpr (D == 64) {
           // lanes are rows j, columns are h
-          float zout[2];
+          float z2[8];
 #pragma unroll
-          for (int c32 = 0; c32 < 2; ++c32) {
-            float z[8];
+          for (int c16 = 0; c16 < 4; ++c16) {
+            uint32_t d[2][8];
 #pragma unroll
-            for (int g2 = 0; g2 < 2; ++g2) {
-              const int c16 = c32 * 2 + g2;
-              uint32_t d[2][8];
-#pragma unroll
-              for (int hl = 0; hl < 2; ++hl) tmem_ld_16x256b_x2(tacc + ((uint32_t)(hl * 16) << 16) + c16 * 16, d[hl]);
-              const float2 v0 = *reinterpret_cast<const float2*>(v + c16 * 16 + 2 * (lane & 3));
-              const float2 v1 = *reinterpret_cast<const float2*>(v + c16 * 16 + 8 + 2 * (lane & 3));
-              tmem_wait_ld();
-              if (c16 == 3) {
-                tc_fence_before();
-                arrive_warp(&bars.acc_free[role]);
-              }
-              float2 z0 = make_float2(0.f, 0.f), z1 = z0;
-#pragma unroll
-              for (int hl = 0; hl < 2; ++hl) {
-#pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                  const float2 g0 = make_float2(__uint_as_float(d[hl][2 * r]), __uint_as_float(d[hl][2 * r + 1]));
-                  const float2 g1 = make_float2(__uint_as_float(d[hl][4 + 2 * r]), __uint_as_float(d[hl][5 + 2 * r]));
-                  float2& a0 = acc[c16 * 8 + hl * 4 + r];
-                  float2& a1 = acc[c16 * 8 + hl * 4 + 2 + r];
-                  a0 = __ffma2_rn(g0, v0, a0);
-                  a1 = __ffma2_rn(g1, v1, a1);
-                  z0 = __ffma2_rn(g0, unpack2<T16>(x[c16][hl][r]), z0);
-                  z1 = __ffma2_rn(g1, unpack2<T16>(x[c16][hl][2 + r]), z1);
-                }
-              }
-              z[g2 * 4 + 0] = z0.x;
-              z[g2 * 4 + 1] = z0.y;
-              z[g2 * 4 + 2] = z1.x;
-              z[g2 * 4 + 3] = z1.y;
+            for (int hl = 0; hl < 2; ++hl) tmem_ld_16x256b_x2(tacc + ((uint32_t)(hl * 16) << 16) + c16 * 16, d[hl]);
+            const float2 v0 = unpack2<T16>(*reinterpret_cast<const uint32_t*>(v + c16 * 16 + 2 * (lane & 3)));
+            const float2 v1 = unpack2<T16>(*reinterpret_cast<const uint32_t*>(v + c16 * 16 + 8 + 2 * (lane & 3)));
+            tmem_wait_ld();
+            if (c16 == 3) {
+              tc_fence_before();
+              arrive_warp(&bars.acc_free[role]);
             }
-            // z[4 g2 + 2 g + e]: column 32 c32 + 16 g2 + 8 g + 2 (lane % 4) + e, over this thread's four rows; the tree
-            // over lane / 4 leaves one column per lane: g2 = lane bit 4, g = lane bit 3, e = lane bit 2
+            float2 z0 = make_float2(0.f, 0.f), z1 = z0;
 #pragma unroll
-            for (int half = 4; half >= 1; half >>= 1) {
-              const bool upper = lane & (half * 4);
+            for (int hl = 0; hl < 2; ++hl) {
 #pragma unroll
-              for (int i2 = 0; i2 < half; ++i2) {
-                const float keep = upper ? z[i2 + half] : z[i2];
-                const float send = upper ? z[i2] : z[i2 + half];
-                z[i2] = keep + __shfl_xor_sync(0xffffffffu, send, half * 4);
+              for (int r = 0; r < 2; ++r) {
+                const float2 g0 = make_float2(__uint_as_float(d[hl][2 * r]), __uint_as_float(d[hl][2 * r + 1]));
+                const float2 g1 = make_float2(__uint_as_float(d[hl][4 + 2 * r]), __uint_as_float(d[hl][5 + 2 * r]));
+                float2& a0 = acc[c16 * 8 + hl * 4 + r];
+                float2& a1 = acc[c16 * 8 + hl * 4 + 2 + r];
+                a0 = __ffma2_rn(g0, v0, a0);
+                a1 = __ffma2_rn(g1, v1, a1);
+                z0 = __ffma2_rn(g0, unpack2<T16>(x[c16][hl][r]), z0);
+                z1 = __ffma2_rn(g1, unpack2<T16>(x[c16][hl][2 + r]), z1);
               }
             }
-            zout[c32] = z[0];
+            // z0, z1: columns 16 c16 + 2 (lane % 4) and the next, and those 8 further, over this thread's four rows.  The sum
+            // over lane / 4 is a tree; its first exchange, here beside the reads, leaves columns 8 g.. with g = lane bit 4
+            const bool upper = lane & 16;
+            z2[2 * c16] = (upper ? z1.x : z0.x) + __shfl_xor_sync(0xffffffffu, upper ? z0.x : z1.x, 16);
+            z2[2 * c16 + 1] = (upper ? z1.y : z0.y) + __shfl_xor_sync(0xffffffffu, upper ? z0.y : z1.y, 16);
           }
-          const int col = (lane >> 4) * 16 + ((lane >> 3) & 1) * 8 + 2 * (lane & 3) + ((lane >> 2) & 1);
-          red_add(zrow + col, zout[0] * zscale);
-          red_add(zrow + 32 + col, zout[1] * zscale);
+          // z2[2 c16 + e]: column 16 c16 + 8 (lane bit 4) + 2 (lane % 4) + e; two more exchanges leave two columns per lane:
+          // c16 = 2 (lane bit 3) + (lane bit 2)
+#pragma unroll
+          for (int half = 4; half >= 2; half >>= 1) {
+            const bool upper = lane & (half * 2);
+#pragma unroll
+            for (int i2 = 0; i2 < half; ++i2) {
+              const float keep = upper ? z2[i2 + half] : z2[i2];
+              const float send = upper ? z2[i2] : z2[i2 + half];
+              z2[i2] = keep + __shfl_xor_sync(0xffffffffu, send, half * 2);
+            }
+          }
+          const int col = ((lane >> 2) & 3) * 16 + (lane >> 4) * 8 + 2 * (lane & 3);
+          red_add2(zrow + col, z2[0] * zscale, z2[1] * zscale);
         } else {
           // lanes are columns h of the head, columns are rows j
           float2 z[4];
@@ -717,7 +775,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
             z[r] = make_float2(0.f, 0.f);
-            vr[r] = v[w * 32 + r * 8 + (lane >> 2)];
+            vr[r] = to_f(v[w * 32 + r * 8 + (lane >> 2)]);
           }
 #pragma unroll
           for (int c16 = 0; c16 < 4; ++c16) {
@@ -772,8 +830,6 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       vb0 += (len + kVecBatch - 1) / kVecBatch;
       ++items;
       // ---- dK1 / dSiLU(V1) of this item
-      // (the K2 rows carry alpha * log2(e) * 2^ea, the V2 rows 2^eb)
-      const float jscale = role ? unshift * pow2i<T16>(-it.eb) : unshift_ds * pow2i<T16>(-it.ea) * kLn2;
       float* const base = (role ? p.dsv1 : p.dk1) + (size_t)it.bh * T * D;
 #pragma unroll
       for (int c16 = 0; c16 < 4; ++c16)
@@ -796,8 +852,9 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
             }
     }
   } else {
-   set_regs<kRegsLaunch, kRegsService>();
-   if (warp == 16) {
+   set_regs<kRegsLaunch, BwdRegs<D, LARGE>::kService>();
+   if (warp == 16 || (!LARGE && warp >= 18)) {
+    const bool do_rows = warp == 16, do_u = LARGE || warp == 18, do_ds = LARGE || warp == 19;
     // ------------------------------------------------------------------ MMA issuer
     // The whole warp walks the schedule in step and one elected lane issues: with converged control flow the
     // descriptor arithmetic stays on the uniform datapath, where a lone thread needs a register-to-uniform move
@@ -812,6 +869,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
     const uint32_t qLo = desc_lo(smem_u32(smem + Cfg::kOffQ), 16384), doLo = desc_lo(smem_u32(smem + Cfg::kOffDO), 16384);
     const uint32_t aLo = desc_lo(smem_u32(smem + Cfg::kOffA), JT * 128);
     const uint32_t a2Lo = desc_lo(smem_u32(smem + Cfg::kOffA + 2 * Cfg::kTileJ), JT * 128);
+    const uint32_t sv1Lo = desc_lo(smem_u32(smem + Cfg::kOffK1 + Cfg::kTileJ), JT * 128);
     const uint32_t rLo[2] = {desc_lo(smem_u32(smem + Cfg::kOffR0), 16), desc_lo(smem_u32(smem + Cfg::kOffR1), 16)};
     const uint32_t k1Lo = desc_lo(smem_u32(smem + Cfg::kOffK1), 16);
     const uint32_t pLo = desc_lo(smem_u32(smem + Cfg::kOffP), 16384);
@@ -843,9 +901,11 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
     };
     uint32_t n = 0, items = 0, runs = 0;
     bool alive = true;
+    // Three warps issue: S and dP, U, dQ and G, each as soon as its operands are there.  One warp for all five held them back
+    // behind each other's waits: a look at a barrier takes 100 to 200 cycles while the tensor cores read shared memory.  (Large
+    // scores: one, as the other two form R.)
     auto issue_s = [&](uint32_t m) -> bool {
-      if (!(LARGE ? wait_all(&bars.r_ready, m & 1) : wait_all(&bars.a_ready[m & 1], (m >> 1) & 1))) return false;
-      if (!wait_all(&bars.s_free, (m & 1) ^ 1)) return false;
+      if (!wait_two(LARGE ? &bars.r_ready : &bars.a_ready[m & 1], (LARGE ? m : m >> 1) & 1, &bars.s_free, (m & 1) ^ 1)) return false;
       tc_fence_after();
       if constexpr (LARGE) {
 #pragma unroll
@@ -859,12 +919,15 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       commit(&bars.s_ready);
       return true;
     };
-    // (the previous step's dP has been read: its ds_ready was waited for)
-    auto issue_dp = [&](uint32_t m) -> bool {
-      if (!wait_all(&bars.ap_ready, m & 1)) return false;
+    // (the first step of an item has no dP before it that anyone still reads)
+    auto issue_dp = [&](uint32_t m, bool after) -> bool {
+      uint64_t* const ap = &bars.ap_ready[LARGE ? 0 : m & 1];
+      const uint32_t parity = (LARGE ? m : m >> 1) & 1;
+      if (!wait_two(ap, parity, after ? &bars.ds_ready : ap, after ? (m - 1) & 1 : parity)) return false;
       tc_fence_after();
-      issue_rows(Cfg::kTmemDP, Cfg::kTmemDO, a2Lo);
+      issue_rows(Cfg::kTmemDP, Cfg::kTmemDO, LARGE || !(m & 1) ? a2Lo : sv1Lo);
       commit(&bars.dp_ready);
+      commit(&bars.ap_free[m & 1]);
       return true;
     };
     BwdItem it;
@@ -872,44 +935,50 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       if (it.flags & kFirstOfQ) {
         alive = wait_all(&bars.qdo_ready, runs & 1);   // (runs: q-tiles finished)
         if (!alive) break;
+        tc_fence_after();
       }
-      alive = issue_s(n) && issue_dp(n);
+      if (do_rows) alive = issue_s(n) && issue_dp(n, false);
       for (int i = 0; i < it.len && alive; ++i, ++n) {
         const bool more = i + 1 < it.len;
         alive = false;
-        if (more && !issue_s(n + 1)) break;
-        if (!wait_all(&bars.p_ready, n & 1) || !wait_all(&bars.acc_free[1], (n & 1) ^ 1)) break;
-        tc_fence_after();
-        issue_fold(Cfg::kTmemU, pLo, doLo);
-        commit(&bars.acc_done[1]);
-        if (!wait_all(&bars.ds_ready, n & 1)) break;
-        tc_fence_after();
-        if (more && !issue_dp(n + 1)) break;
-        const bool fresh = i == 0 && (it.flags & kFirstOfQ);
-        if (fresh) {
-          // the previous q-tile's dQ has been read
-          if (!wait_all(&bars.dq_free, (runs & 1) ^ 1)) break;
+        if (do_rows && more && !(issue_s(n + 1) && (LARGE || issue_dp(n + 1, true)))) break;
+        if (do_u) {
+          if (!wait_two(&bars.p_ready, n & 1, &bars.acc_free[1], (n & 1) ^ 1)) break;
           tc_fence_after();
+          issue_fold(Cfg::kTmemU, pLo, doLo);
+          commit(&bars.acc_done[1]);
         }
-        if constexpr (LARGE) {
-          if (!wait_all(&bars.a_ready[n & 1], (n >> 1) & 1)) break;
+        if (do_ds) {
+          const bool g_free = mbar_test(&bars.acc_free[0], (n & 1) ^ 1);
+          if (!wait_all(&bars.ds_ready, n & 1)) break;
           tc_fence_after();
+          if (LARGE && more && !issue_dp(n + 1, true)) break;
+          const bool fresh = i == 0 && (it.flags & kFirstOfQ);
+          if (fresh) {
+            // the previous q-tile's dQ has been read
+            if (!wait_all(&bars.dq_free, (runs & 1) ^ 1)) break;
+            tc_fence_after();
+          }
+          if constexpr (LARGE) {
+            if (!wait_all(&bars.a_ready[n & 1], (n >> 1) & 1)) break;
+            tc_fence_after();
+          }
+          const uint32_t ds = pLo + (1 + (n & 1)) * kTileP16;
+          issue_dq(ds, aLo + (n & 1) * kTileJ16, fresh ? 0u : 1u);
+          commit(&bars.a_free[n & 1]);
+          if (!__all_sync(0xffffffffu, g_free) && !wait_all(&bars.acc_free[0], (n & 1) ^ 1)) break;
+          tc_fence_after();
+          issue_fold(Cfg::kTmemG, ds, qLo);
+          commit(&bars.acc_done[0]);
+          commit(&bars.ds_free[n & 1]);
         }
-        const uint32_t ds = pLo + (1 + (n & 1)) * kTileP16;
-        issue_dq(ds, aLo + (n & 1) * kTileJ16, fresh ? 0u : 1u);
-        commit(&bars.a_free[n & 1]);
-        if (!wait_all(&bars.acc_free[0], (n & 1) ^ 1)) break;
-        tc_fence_after();
-        issue_fold(Cfg::kTmemG, ds, qLo);
-        commit(&bars.acc_done[0]);
-        commit(&bars.ds_free[n & 1]);
         alive = true;
       }
       if (!alive) break;
       commit(&bars.tile_free);
       ++items;
       if ((it.flags & kLastOfQ)) {
-        commit(&bars.dq_done);
+        if (do_ds) commit(&bars.dq_done);
         ++runs;
       }
     }
@@ -922,25 +991,22 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       tma_prefetch_desc(&tmK1);
       tma_prefetch_desc(&tmSV1);
     }
-    float scale_k = p.alpha * kLog2e, scale_v = 1.f;   // of the K2 and V2 rows, with the head's powers of two
-    int bh = -1, ea = 0, eb = 0, f = 0;
-    constexpr int kChunks = kVecBatch * D / 8 / 32;   // 16-byte pieces of K2 (and of V2) per lane and batch
-    float* const vec = reinterpret_cast<float*>(smem + Cfg::kOffVec);
+    int bh = -1, ea = 0, eb = 0, er = 0, f = 0;
     uint32_t items = 0, vb = 0;
     bool alive = true, in_flight = false;
     BwdWalk walk(p);
-    BwdItem it{-1, -1, 0, 0, 0, 0, 0, 0};
+    BwdItem it{-1, -1, 0, 0, 0, 0, 0, 0, 0, {0, 0, 0}};
     while (alive) {
       it = walk.next(it);
       if (it.len > 0 && it.bh != bh) {
         bh = it.bh;
         const BwdStats st = head_stats(p, bh, lane);
-        ea = range_shift<T16>(fabsf(p.alpha * kLog2e) * st.qk1 * st.k2);
-        eb = range_shift<T16>(st.sv1 * st.v2);
+        ea = range_shift<T16>(st.qk1, st.k2);
+        eb = range_shift<T16>(st.sv1, st.v2);
+        er = product_shift<T16>(fabsf(p.alpha * kLog2e) * st.qk1 * st.k2);
         f = ds_shift<T16>(sqrtf(st.do_row * st.sv1_row) * st.v2);
-        scale_k = p.alpha * kLog2e * pow2i<T16>(ea);
-        scale_v = pow2i<T16>(eb);
       }
+      it.er = er;
       it.ea = ea;
       it.eb = eb;
       it.flags |= f << kShiftBits;
@@ -965,33 +1031,19 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       }
       in_flight = true;
       ++items;
-      // K2 / V2 rows, fp32, times their factors (K2's has alpha * log2(e)), a batch of rows at a time; rows past the item repeat its last
-      const size_t head = (size_t)it.bh * T * D;
+      // K2 / V2 rows, a batch at a time (the last one of an item may be shorter)
+      const size_t head = ((size_t)it.bh * T + it.k0) * D;
       for (int i = 0; i < it.len; i += kVecBatch, ++vb) {
-        uint4 x[2][kChunks];
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c) {
-          const int at = c * 32 + lane, r = at / (D / 8), col = at % (D / 8) * 8;
-          const size_t off = head + (size_t)(it.k0 + min(i + r, it.len - 1)) * D + col;
-          x[0][c] = __ldg(reinterpret_cast<const uint4*>((const T16*)p.k2 + off));
-          x[1][c] = __ldg(reinterpret_cast<const uint4*>((const T16*)p.v2 + off));
-        }
-        alive = wait_all(&bars.vec_empty[vb % kVecSlots], ((vb / kVecSlots) & 1) ^ 1);
+        const uint32_t slot = vb % kVecSlots, bytes = min(kVecBatch, it.len - i) * D * 2;
+        alive = wait_all(&bars.vec_empty[slot], ((vb / kVecSlots) & 1) ^ 1);
         if (!alive) break;
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c) {
-          const int at = c * 32 + lane, r = at / (D / 8), col = at % (D / 8) * 8;
-          float* dst = vec + ((vb % kVecSlots) * kVecBatch + r) * Cfg::kVecRow + col;
-#pragma unroll
-          for (int m = 0; m < 2; ++m) {
-            const float sc = m == 0 ? scale_k : scale_v;
-            const uint4 y = x[m][c];
-            const float2 f0 = unpack2<T16>(y.x), f1 = unpack2<T16>(y.y), f2 = unpack2<T16>(y.z), f3 = unpack2<T16>(y.w);
-            *reinterpret_cast<float4*>(dst + m * D) = make_float4(f0.x * sc, f0.y * sc, f1.x * sc, f1.y * sc);
-            *reinterpret_cast<float4*>(dst + m * D + 4) = make_float4(f2.x * sc, f2.y * sc, f3.x * sc, f3.y * sc);
-          }
+        if (leader) {
+          uint8_t* dst = smem + Cfg::kOffVec + slot * 2 * Cfg::kVecPart;
+          const size_t src = head + (size_t)i * D;
+          mbar_arrive_expect_tx(&bars.vec_full[slot], 2 * bytes);
+          bulk_load(dst, (const T16*)p.k2 + src, bytes, &bars.vec_full[slot]);
+          bulk_load(dst + Cfg::kVecPart, (const T16*)p.v2 + src, bytes, &bars.vec_full[slot]);
         }
-        mbar_arrive(&bars.vec_full[vb % kVecSlots]);
       }
     }
     if (!alive && in_flight) {
@@ -999,6 +1051,9 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       const long long t0 = clock64();
       while (!mbar_try_wait(&bars.tile_full, (items - 1) & 1) && clock64() - t0 < kWaitTicks / 8) {
       }
+      for (uint32_t b = vb > (uint32_t)kVecSlots ? vb - kVecSlots : 0; b < vb; ++b)
+        while (!mbar_try_wait(&bars.vec_full[b % kVecSlots], (b / kVecSlots) & 1) && clock64() - t0 < kWaitTicks / 8) {
+        }
     }
    } else if constexpr (LARGE) {
     // ------------------------------------------------------------------ R (warps 18, 19)
@@ -1009,7 +1064,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
     const int t = tid - 18 * 32, col = t % kCols, row0 = t / kCols;
     const uint8_t* const src = smem + Cfg::kOffQ + (col >> 3) * 16384;
     uint8_t* const dst = smem + (col >> 3 ? Cfg::kOffR1 : Cfg::kOffR0);
-    const float* const vec = reinterpret_cast<const float*>(smem + Cfg::kOffVec) + col * 8;
+    const T16* const vec = reinterpret_cast<const T16*>(smem + Cfg::kOffVec) + col * 8;
     constexpr int kPieces = 2, kGroups = 128 / kRowStep / kPieces;
     // byte offset of piece e of group g: the swizzle of a row depends on its last three bits, that is on e alone
     uint32_t swz[kPieces];
@@ -1028,7 +1083,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       ++items;
       fetch(0);
       // (the fold warps have read their tile: they have formed the item's first A')
-      alive = wait_all(&bars.ap_ready, n & 1);
+      alive = wait_all(&bars.ap_ready[0], n & 1);
       for (int i = 0; i < it.len && alive; ++i) {
         if ((i & (kVecBatch - 1)) == 0) {
           const uint32_t vb = vb0 + i / kVecBatch;
@@ -1038,9 +1093,12 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
         // before this wait, and a barrier two phases ahead of its waiter reads as not ready for ever)
         if (alive && i > 0) alive = wait_all(&bars.s_ready, (n + i - 1) & 1);
         if (!alive) break;
-        const float* v = vec + ((vb0 * kVecBatch + i) % (kVecSlots * kVecBatch)) * Cfg::kVecRow;
-        const float4 va = *reinterpret_cast<const float4*>(v), vb = *reinterpret_cast<const float4*>(v + 4);
-        const float2 m[4] = {make_float2(va.x, va.y), make_float2(va.z, va.w), make_float2(vb.x, vb.y), make_float2(vb.z, vb.w)};
+        const uint4 v = *reinterpret_cast<const uint4*>(
+            vec + ((vb0 + i / kVecBatch) % kVecSlots * 2 * kVecBatch + i % kVecBatch) * D);
+        const float sr = p.alpha * kLog2e * pow2i<T16>(it.er);
+        const float2 sr2 = make_float2(sr, sr);
+        const float2 m[4] = {__fmul2_rn(unpack2<T16>(v.x), sr2), __fmul2_rn(unpack2<T16>(v.y), sr2),
+                             __fmul2_rn(unpack2<T16>(v.z), sr2), __fmul2_rn(unpack2<T16>(v.w), sr2)};
         // (the Q pieces of a group are fetched while the one before is worked on; those of the first, below, from the
         // step before: they do not depend on the step)
 #pragma unroll 2
