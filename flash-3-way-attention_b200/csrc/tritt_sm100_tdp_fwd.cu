@@ -19,13 +19,20 @@
 //                row-major (MN-major descriptor).  128-column slabs keep every accumulation chain at
 //                8 instructions of 128x128x16, the shape the pipe runs at full rate.
 //   warps 4-11   two soft-max warpgroups (one row per thread); they also form A_a, A_b.  Where a head-wide bound on
-//                the scores is small (per-head statistics from a small kernel before this one) every row takes its
-//                own score bound as the soft-max reference and the warpgroups work on the same slab, tile a then
+//                the scores is small (per-head statistics from a small kernel before this one) every row has the same
+//                soft-max reference and the warpgroups work on the same slab, tile a then
 //                tile b, 64 of its 128 columns each: one pass, exp2, P written back to TMEM as 16-bit over the
 //                first half of the columns just read.  Otherwise warpgroup x owns tile x and a thread its whole
 //                row: row maximum, exp2 with lazy rescaling of the accumulator, P over the first 64 columns of S_x
 //   warps 12-15  fold warpgroup: when a k-tile is finished, folds acc_x (times V2, soft-max over k) into
-//                the queries' running (max, sum, output) while the other warps start the next k-tile
+//                the queries' running (max, sum, output) while the other warps start the next k-tile; with one reference for
+//                a head the sums just add up in registers, without exchanges between threads
+// What bounds it: the soft-max stage of a slab (1300 cycles against 1024 of exponentials, and 200 between stages) and the change
+// of k-tiles (K2 tile, operands, first scores: 3300 to 4100 cycles before, 2000 of them the operands, now about 2200).  Operands
+// with a thread on one column of every 16th or 32nd row, norms only where a row's bound is asked for, and the fold without
+// exchanges: T=512 D=64 bf16 32 heads 1020 -> 928 us, T=2048 D=128 16 heads 24.0 -> 23.1 ms, T=512 D=128 fp16 16 heads with row
+// maxima 808 -> 765 us; T=4096 D=64 4 heads 33.7 -> 34.2 ms (its k-tiles have 16 slabs, and so little to gain).  The code size matters: with the stages
+// unrolled by tile and mode (165 to 235 KB for 115 to 140) the same changes were 4 to 15 % slower than before them.
 // Causal structure: for a fixed query the mask is "j <= q" on columns and "k <= q" on rows, so
 // whole slabs above q are never visited, only the last slab is masked (by a column bound that
 // is uniform over the rows), and rows with k > q get weight zero in the fold.
@@ -52,8 +59,8 @@ template <int D> struct FwdCfg {
   static constexpr int kOffStats = kOffRing + kStages * kTileA;  // [2 parities][2 tiles][128][4] fp32: row (reference, two partial sums, -)
   static constexpr int kOffRed = kOffStats + 2 * 2 * 128 * 4 * 4;  // [2 tiles][4 warps][D] fp32 column sums
   static constexpr int kOffFstat = kOffRed + 2 * 4 * D * 4;        // [2 tiles][8] fp32 warp max / sum
-  static constexpr int kOffNorm = kOffFstat + 2 * 8 * 4;            // [2 tiles][2 column halves][128] fp32: partial |A_row|^2
-  static constexpr int kOffBars = kOffNorm + 2 * 2 * 128 * 4;
+  static constexpr int kOffNorm = kOffFstat + 2 * 8 * 4;            // [2 tiles][128] fp32: |A_row|^2
+  static constexpr int kOffBars = kOffNorm + 2 * 128 * 4;
   static constexpr int kSmem = kOffBars + 256;
   static constexpr int kTmemO = 256;  // S_a | S_b | acc_a | acc_b
 };
@@ -80,7 +87,7 @@ struct FwdBarriers {
   // (short sequences, narrow windows) the soft-max warps can hand over the next k-tile's statistics before the fold
   // warpgroup, still storing the previous item, has looked at this one's, and a barrier two phases ahead of its waiter
   // reads as not ready for ever.
-  uint64_t o_done, o_free[2], stats_ready[2][2];
+  uint64_t o_done[2], o_free[2], stats_ready[2][2];
   uint64_t fold_sync;
   uint32_t tmem_base;
   int abort_flag;
@@ -128,8 +135,8 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
       mbar_init(&bars.o_free[x], 128);
       mbar_init(&bars.stats_ready[0][x], 256);
       mbar_init(&bars.stats_ready[1][x], 256);
+      mbar_init(&bars.o_done[x], 1);
     }
-    mbar_init(&bars.o_done, 1);
     mbar_init(&bars.fold_sync, 128);
     fence_barrier_init();
   }
@@ -195,9 +202,9 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
   auto halves = [](int ja, int jb, int j0) { return jb < j0 + 64 ? 1 : (ja >= j0 + 64 ? 2 : 0); };
   // How the soft-max warps divide a head's work.  Every score of the head is bounded by
   // |s| max_q |Q_q| max |K2 element| max_j |K1_j|  (|A_row|^2 = s^2 sum_h Q_h^2 K2_h^2 <= s^2 max_h K2_h^2 |Q_q|^2).
-  // Where that is below the limit, every row can take its own score bound as soft-max reference (one pass, nothing
-  // to agree on between threads) and the two warpgroups split every slab's columns; otherwise each warpgroup owns one
-  // tile and a thread its whole row (maximum pass, rescaling).  Uniform over a work item, read by every role.
+  // Where that is below the limit, the limit is every row's soft-max reference (one pass, nothing to agree on between threads, nothing
+  // to merge between tiles) and the two warpgroups split every slab's columns; otherwise each warpgroup owns one tile and a
+  // thread its whole row (maximum pass, rescaling).  Uniform over a work item, read by every role.
   auto head_split = [&](int bh) -> bool {
     if (!p.k1_norm2_max) return false;
     const float b = fabsf(p.scale2) * sqrtf(__ldg(p.q_norm2_max + bh)) * sqrtf(__ldg(p.k2_elem2_max + bh)) *
@@ -364,6 +371,7 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
               tc_fence_after();
               if (x == 0 && !wait_full(pv)) { alive = false; break; }
               issue_pv(x, pv, jt > 0, hm, split);
+              if (!more) commit(&bars.o_done[x]);
               if (x == 1) release(pv);
               if (more) {
                 if (x == 0 && !wait_full(pk)) { alive = false; break; }
@@ -373,7 +381,6 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
             }
             hm = hm_next;
           }
-          if (alive) commit(&bars.o_done);
           base += 2 * njt;
         }
       }
@@ -500,54 +507,63 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
           }
         }
         // ---- operand formation: A_a = s*Q[qa] (.) K2tile (in place), A_b = s*Q[qb] (.) K2tile
+        constexpr int kCols = D / 8, kRowStep = 256 / kCols;
+        const int col = st % kCols;
+        const uint32_t off0 = (col >> 3) * 16384 + swz128(st / kCols, col & 7);
+        float2 qv[2][4];   // this thread's columns of the two queries
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const uint4 v = __ldg(reinterpret_cast<const uint4*>(Qg + (size_t)(x ? qb : qa) * D + col * 8));
+          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) qv[x][e] = unpack2<T16>(w[e]);
+        }
         alive = __all_sync(0xffffffffu, mbar_wait(&bars.k2_full, kt_count & 1, abort_flag));
         if (!alive) break;
+        // A thread has one 16-byte column of every (256 / kCols)-th row.  (The backward forms the same products in the same
+        // order for large scores, where a rounding the other way would show.)
         {
-          const int r = st & 127;
-          constexpr int CPT = D / 16;  // 16-byte chunks per thread
-          const int c0 = (st >> 7) * CPT;
-          float na = 0.f, nb = 0.f;  // this thread's share of |A_a[r]|^2 and |A_b[r]|^2
-#pragma unroll
-          for (int i = 0; i < CPT; ++i) {
-            const int cc = c0 + i, hh = cc >> 3, c = cc & 7;
-            const uint32_t off = hh * 16384 + swz128(r, c);
+#pragma unroll 2
+          for (int i = 0; i < 128 / kRowStep; ++i) {
+            const uint32_t off = off0 + i * kRowStep * 128;
             const uint4 kv = *reinterpret_cast<const uint4*>(smem + Cfg::kOffAa + off);
-            const uint4 qav = __ldg(reinterpret_cast<const uint4*>(Qg + (size_t)qa * D + cc * 8));
-            const uint4 qbv = __ldg(reinterpret_cast<const uint4*>(Qg + (size_t)qb * D + cc * 8));
             const uint32_t w[4] = {kv.x, kv.y, kv.z, kv.w};
-            const uint32_t wa[4] = {qav.x, qav.y, qav.z, qav.w};
-            const uint32_t wb[4] = {qbv.x, qbv.y, qbv.z, qbv.w};
-            uint32_t oa[4], ob[4];
+            uint32_t a[2][4];
+            float nr[2] = {0.f, 0.f};   // this thread's share of |A_a[r]|^2 and |A_b[r]|^2
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              const float2 f = unpack2<T16>(w[e]);
-              const float2 fa = unpack2<T16>(wa[e]), fb = unpack2<T16>(wb[e]);
-              const float k0 = f.x * p.scale2, k1v = f.y * p.scale2;
-              const float a0 = k0 * fa.x, a1 = k1v * fa.y, b0 = k0 * fb.x, b1 = k1v * fb.y;
-              na = fmaf(a0, a0, fmaf(a1, a1, na));
-              nb = fmaf(b0, b0, fmaf(b1, b1, nb));
-              oa[e] = pack2<T16>(a0, a1);
-              ob[e] = pack2<T16>(b0, b1);
+              const float2 f = __fmul2_rn(unpack2<T16>(w[e]), make_float2(p.scale2, p.scale2));
+#pragma unroll
+              for (int x = 0; x < 2; ++x) {
+                const float2 g = __fmul2_rn(f, qv[x][e]);
+                a[x][e] = pack2<T16>(g.x, g.y);
+                if (!split) nr[x] = fmaf(g.x, g.x, fmaf(g.y, g.y, nr[x]));
+              }
             }
-            *reinterpret_cast<uint4*>(smem + Cfg::kOffAa + off) = make_uint4(oa[0], oa[1], oa[2], oa[3]);
-            *reinterpret_cast<uint4*>(smem + Cfg::kOffAb + off) = make_uint4(ob[0], ob[1], ob[2], ob[3]);
+            *reinterpret_cast<uint4*>(smem + Cfg::kOffAa + off) = make_uint4(a[0][0], a[0][1], a[0][2], a[0][3]);
+            *reinterpret_cast<uint4*>(smem + Cfg::kOffAb + off) = make_uint4(a[1][0], a[1][1], a[1][2], a[1][3]);
+            if (!split) {
+              // (read by the owner of the row after its first s_ready wait of this k-tile, which this thread's
+              //  a_ready arrival below precedes; rewritten only after it has passed a_free)
+#pragma unroll
+              for (int x = 0; x < 2; ++x) {
+#pragma unroll
+                for (int o = kCols / 2; o >= 1; o >>= 1) nr[x] += __shfl_xor_sync(0xffffffffu, nr[x], o);
+                if (col == 0) norms[x * 128 + st / kCols + i * kRowStep] = nr[x];
+              }
+            }
           }
-          // (read by both owners of row r after their first s_ready wait of this k-tile, which this thread's
-          //  a_ready arrival below precedes; rewritten only after both have passed a_free)
-          norms[(0 * 2 + (st >> 7)) * 128 + r] = na;
-          norms[(1 * 2 + (st >> 7)) * 128 + r] = nb;
         }
         fence_async_smem();   // generic-proxy stores above -> visible to the tensor core's reads
         mbar_arrive(&bars.a_ready);
 
         if (split) {
           // ---- walk over the slabs, both warpgroups on the same slab: tile a, then tile b; warpgroup `wg` takes the
-          // slab's columns [wg * 64, wg * 64 + 64) (32 of a half-width slab's 64).  The reference of every row is its
-          // score bound |A_row| * max_j |K1_j| (log2 units), which the head-wide bound keeps below the limit: P stays
-          // within [2^-2b, 1], representable in the 16-bit type, and no row maximum is needed.
-          float ref[2], l_sum[2] = {0.f, 0.f};
-#pragma unroll
-          for (int x = 0; x < 2; ++x) ref[x] = 0.f;
+          // slab's columns [wg * 64, wg * 64 + 64) (32 of a half-width slab's 64).  The reference of every row is the limit l itself
+          // (log2 units), which the head's score bound is below: P stays within [2^-2l, 1], representable in the 16-bit type, and
+          // no row maximum is needed.  (A launch parameter as the reference costs no register: 928 us at T=512 D=64, against 945
+          // with the head's bound; no reference at all, P = exp2(S), 917.)
+          float l_sum[2] = {0.f, 0.f};
           for (int jt = 0; jt < njt && alive; ++jt, ++n) {
             // A slab with attended columns in one 64-column half only was computed for that half alone: its scores
             // are in the first 64 columns of S_x and stand for the slab's columns [coff, coff + 64).
@@ -560,7 +576,6 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
               alive = __all_sync(0xffffffffu, mbar_wait(&bars.s_ready[x], n & 1, abort_flag));
               if (!alive) break;
               tc_fence_after();
-              if (jt == 0) ref[x] = sqrtf(norms[(x * 2 + 0) * 128 + row] + norms[(x * 2 + 1) * 128 + row]) * k1_max;
               // the last score product of this k-tile has read A_a and A_b
               if (x == 1 && jt == njt - 1) mbar_arrive(&bars.a_free);
               const uint32_t tS = tmem + lane_base + x * kBJ + wg * cw;
@@ -569,24 +584,18 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
               const int lo = c_lo[x] - j0, hi = c_hi[x] - j0;
               const bool full = __all_sync(0xffffffffu, lo <= 0 && hi >= cw - 1);
               // P over the first half of the columns this thread has read
-              l_sum[x] += nh == 2 ? form_p(std::integral_constant<int, 64>{}, tS, tS, full, lo, hi, ref[x])
-                                  : form_p(std::integral_constant<int, 32>{}, tS, tS, full, lo, hi, ref[x]);
+              l_sum[x] += nh == 2 ? form_p(std::integral_constant<int, 64>{}, tS, tS, full, lo, hi, p.bound_limit)
+                                  : form_p(std::integral_constant<int, 32>{}, tS, tS, false, lo, hi, p.bound_limit);
               tmem_wait_st();
               tc_fence_before();
               mbar_arrive(&bars.p_ready[x]);
             }
           }
           if (!alive) break;
-          // ---- hand this k-tile's row statistics to the fold warpgroup: (reference, sum of warpgroup 0, of warpgroup 1)
+          // ---- hand this k-tile's row sums to the fold warpgroup
 #pragma unroll
           for (int x = 0; x < 2; ++x) {
-            float* srow = stats + (((kt_count & 1) * 2 + x) * 128 + row) * 4;
-            if (wg == 0) {
-              srow[0] = ref[x];
-              srow[1] = l_sum[x];
-            } else {
-              srow[2] = l_sum[x];
-            }
+            stats[(((kt_count & 1) * 2 + x) * 128 + row) * 4 + 1 + wg] = l_sum[x];
             mbar_arrive(&bars.stats_ready[kt_count & 1][x]);
           }
         } else {
@@ -604,7 +613,7 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
             if (!alive) break;
             tc_fence_after();
             if (jt == 0) {
-              const float bound = sqrtf(norms[(x * 2 + 0) * 128 + row] + norms[(x * 2 + 1) * 128 + row]) * k1_max;
+              const float bound = sqrtf(norms[x * 128 + row]) * k1_max;
               fast = __all_sync(0xffffffffu, bound <= p.bound_limit);
               if (fast) m_used = bound;
             }
@@ -686,6 +695,133 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
       decode(item, bh, qa, qb);
       k_range(qa, qb, kt0, nkt);
       const T16* V2g = (const T16*)p.v2 + (size_t)bh * T * D;
+      if (head_split(bh)) {
+        // ---- every row has the same reference, so the k-tiles' sums just add up: sum_r acc_x[r,h] V2[k_r,h] over the rows a
+        // thread reads as 16 x 256-bit fragments (rows lane / 4 + 8 i, column pairs 2 (lane % 4) + 8 g), kept in registers to the
+        // end of the item: no exchange between threads per k-tile.  (One copy of the code for both tiles: their sums change
+        // places after each.)
+        float2 o[D / 8], other[D / 8];
+        float l = 0.f, l_other = 0.f;
+        auto swap_tiles = [&]() {
+#pragma unroll
+          for (int i = 0; i < D / 8; ++i) {
+            const float2 keep = o[i];
+            o[i] = other[i];
+            other[i] = keep;
+          }
+          const float keep = l;
+          l = l_other;
+          l_other = keep;
+        };
+#pragma unroll
+        for (int i = 0; i < D / 8; ++i) o[i] = other[i] = make_float2(0.f, 0.f);
+        auto valid = [&](int k, int q) { return p.causal ? k <= q && q - k <= p.k2w : k < T; };
+        for (int kt = kt0; kt < kt0 + nkt && alive; ++kt, ++kt_count) {
+          const uint32_t par = kt_count & 1;
+#pragma unroll 1
+          for (int x = 0; x < 2; ++x) {
+            const int qx = x ? qb : qa;
+            // V2 rows (r: 16-row half, row of the pair); a row outside the query's range counts as zero
+            const T16* v2r[4];
+            bool ok[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+              const int k = kt * 128 + wq * 32 + (r >> 1) * 16 + (r & 1) * 8 + (lane >> 2);
+              ok[r] = valid(k, qx);
+              v2r[r] = V2g + (size_t)min(k, T - 1) * D + 2 * (lane & 3);
+            }
+            constexpr int kC = D == 64 ? 32 : 16;   // columns whose V2 words are fetched together, ahead of the accumulator
+            uint32_t v2w[kC / 8][4];
+            auto fetch = [&](int c0) {
+#pragma unroll
+              for (int g = 0; g < kC / 8; ++g)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) v2w[g][r] = __ldg(reinterpret_cast<const uint32_t*>(v2r[r] + c0 + g * 8));
+            };
+            fetch(0);
+            alive = __all_sync(0xffffffffu, mbar_wait(&bars.o_done[x], par, abort_flag));
+            if (!alive) break;
+            tc_fence_after();
+#pragma unroll
+            for (int c0 = 0; c0 < D; c0 += kC) {
+              uint32_t d[kC / 16][2][8];
+#pragma unroll
+              for (int c16 = 0; c16 < kC / 16; ++c16)
+#pragma unroll
+                for (int hl = 0; hl < 2; ++hl)
+                  tmem_ld_16x256b_x2(tmem + lane_base + ((uint32_t)(hl * 16) << 16) + Cfg::kTmemO + x * D + c0 + c16 * 16, d[c16][hl]);
+              float2 v[kC / 8][4];
+#pragma unroll
+              for (int g = 0; g < kC / 8; ++g)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) v[g][r] = unpack2<T16>(ok[r] ? v2w[g][r] : 0u);
+              if (c0 + kC < D) fetch(c0 + kC);
+#pragma unroll
+              for (int c16 = 0; c16 < kC / 16; ++c16) tmem_wait_ld(d[c16][0], d[c16][1]);
+#pragma unroll
+              for (int g = 0; g < kC / 8; ++g)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                  const uint32_t* f = d[g >> 1][r >> 1] + (g & 1) * 4 + (r & 1) * 2;
+                  float2& a = o[c0 / 8 + g];
+                  a = __ffma2_rn(make_float2(__uint_as_float(f[0]), __uint_as_float(f[1])), v[g][r], a);
+                }
+            }
+            alive = __all_sync(0xffffffffu, mbar_wait(&bars.stats_ready[par][x], (kt_count >> 1) & 1, abort_flag));
+            if (!alive) break;
+            const float* srow = stats + ((par * 2 + x) * 128 + row) * 4;
+            if (valid(kt * 128 + row, qx)) l += srow[1] + srow[2];
+            // accumulator and statistics have been read: both may be overwritten (the statistics two k-tiles on, whose scores
+            // follow the next k-tile's values)
+            tc_fence_before();
+            mbar_arrive(&bars.o_free[x]);
+            swap_tiles();
+          }
+        }
+        if (!alive) break;
+        // ---- sums over the warp's rows (a tree over lane / 4) and over the warps, then the two output rows
+#pragma unroll 1
+        for (int x = 0; x < 2; ++x) {
+          float z[D / 4];
+#pragma unroll
+          for (int i = 0; i < D / 8; ++i) {
+            z[2 * i] = o[i].x;
+            z[2 * i + 1] = o[i].y;
+          }
+#pragma unroll
+          for (int b = 16, half = D / 8; b >= 4; b >>= 1, half >>= 1) {
+            const bool upper = lane & b;
+#pragma unroll
+            for (int i = 0; i < half; ++i) {
+              const float keep = upper ? z[i + half] : z[i], send = upper ? z[i] : z[i + half];
+              z[i] = keep + __shfl_xor_sync(0xffffffffu, send, b);
+            }
+          }
+          // z[i]: element f = (lane bits 4, 3, 2) * D / 32 + i of the thread's columns 8 (f / 2) + 2 (lane % 4) + f % 2
+#pragma unroll
+          for (int i = 0; i < D / 32; i += 2) {
+            const int f = (((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)) * (D / 32) + i;
+            *reinterpret_cast<float2*>(red + (x * 4 + wq) * D + 8 * (f >> 1) + 2 * (lane & 3)) = make_float2(z[i], z[i + 1]);
+          }
+#pragma unroll
+          for (int b = 16; b >= 1; b >>= 1) l += __shfl_xor_sync(0xffffffffu, l, b);
+          if (lane == 0) fstat[x * 8 + wq] = l;
+          swap_tiles();
+        }
+        if (!fold_sync()) { alive = false; break; }
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const float L = fstat[x * 8] + fstat[x * 8 + 1] + fstat[x * 8 + 2] + fstat[x * 8 + 3];
+          const int qx = x == 0 ? qa : qb;
+          if (row < D) {
+            const float O = red[(x * 4) * D + row] + red[(x * 4 + 1) * D + row] + red[(x * 4 + 2) * D + row] + red[(x * 4 + 3) * D + row];
+            ((T16*)p.out)[((size_t)bh * T + qx) * D + row] = from_f<T16>(O / L);
+          }
+          if (row == 0) p.lse[(size_t)bh * T + qx] = (p.bound_limit + log2f(L)) * kLn2;
+        }
+        if (!fold_sync()) { alive = false; break; }  // red / fstat are rewritten by the next item
+        continue;
+      }
       // running state per tile; thread `row` (< D) owns output column h = row
       float M_run[2] = {-INFINITY, -INFINITY}, L_run[2] = {0.f, 0.f}, O_run[2] = {0.f, 0.f};
       for (int kt = kt0; kt < kt0 + nkt && alive; ++kt, ++kt_count) {
@@ -723,11 +859,12 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
           if (lane == 0) fstat[x * 8 + 4 + wq] = lw;
         }
         // accumulators: the last P*V of both tiles must have landed
-        alive = __all_sync(0xffffffffu, mbar_wait(&bars.o_done, par, abort_flag));
+        alive = __all_sync(0xffffffffu, mbar_wait(&bars.o_done[0], par, abort_flag)) &&
+                __all_sync(0xffffffffu, mbar_wait(&bars.o_done[1], par, abort_flag));
         if (!alive) break;
         tc_fence_after();
         const bool in_range = k_r < T;
-#pragma unroll
+#pragma unroll 1
         for (int ch = 0; ch < D / 32; ++ch) {
           // this row's V2 values for the chunk (shared by both tiles)
           float v2f[32];
@@ -941,7 +1078,7 @@ int launch_fwd(const TdpArgs& a) {
   p.k1_norm2_max = k1n;
   p.q_norm2_max = k1n ? k1n + BN : nullptr;
   p.k2_elem2_max = k1n ? k1n + 2 * BN : nullptr;
-  // P = exp2(S - bound) lies in [2^-2 bound, 1]: normal numbers of the 16-bit type (bf16 2^-126, fp16 2^-14)
+  // P = exp2(S - reference) lies in [2^(-2 limit), 1]: normal numbers of the 16-bit type (bf16 2^-126, fp16 2^-14)
   p.bound_limit = std::is_same<T16, __nv_bfloat16>::value ? 40.f : 6.f;
   p.status = a.status_word;
   if (p.nq == 0) return 0;
