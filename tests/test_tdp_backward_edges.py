@@ -226,3 +226,16 @@ def test_scores_past_the_exponents_range_stay_finite(T, D, dtype, scale):
     silu = torch.nn.functional.silu(t[3].float()).abs().amax()
     bound = 2 * silu * do.float().abs().sum(2, keepdim=True)
     assert (got[4].float().abs() <= bound).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (128, torch.float16)])
+@pytest.mark.parametrize("T", [17, 18, 19, 20, 21, 131])
+def test_rows_of_a_short_last_batch(T, D, dtype):
+    """An item's K2 / V2 rows come in batches of four; the last batch copies what is left of the item, and the sequence's
+    last row is the tensor's end."""
+    t = orc.make_inputs(1, 2, T, D, scale=0.5, seed=T, dtype=dtype)
+    got = _backward([x.to(DEV) for x in t[:5]], t[5].to(DEV), 1.0 / D, True)
+    ref = orc.tdp_backward(*[x.float() for x in t], 1.0 / D, True)
+    for name, a, b in zip(NAMES, got, ref):
+        assert_close(name, a, b, dtype)
