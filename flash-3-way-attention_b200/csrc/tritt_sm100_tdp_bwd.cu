@@ -155,7 +155,9 @@ struct BwdBarriers {
   uint64_t tile_full, tile_free;            // Q, dO, K1, SiLU(V1) of an item
   uint64_t vec_full[kVecSlots], vec_empty[kVecSlots];
   uint64_t a_ready[2], a_free[2], ap_ready[2], ap_free[2], r_ready;  // doubled by step parity (a producer may be two steps ahead)
-  uint64_t s_ready, s_free, p_ready, dp_ready, ds_ready, ds_free[2];
+  // (ds_ready: warp 16 lets the soft-max warps go on to the next step's dS before warp 19 has looked at this one's, and a barrier
+  // two phases ahead of its waiter reads as not ready for ever)
+  uint64_t s_ready, s_free, p_ready, dp_ready, ds_ready[2], ds_free[2];
   uint64_t acc_done[2], acc_free[2];         // G, U
   uint64_t qdo_ready, dq_done, dq_free;
   uint32_t tmem_base;
@@ -346,6 +348,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       mbar_init(&bars.a_free[i], 1);
       mbar_init(&bars.ap_ready[i], 4);
       mbar_init(&bars.ap_free[i], 1);
+      mbar_init(&bars.ds_ready[i], 8);
       mbar_init(&bars.ds_free[i], 1);
     }
     mbar_init(&bars.r_ready, 2);
@@ -353,7 +356,6 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
     mbar_init(&bars.s_free, 8);
     mbar_init(&bars.p_ready, 8);
     mbar_init(&bars.dp_ready, 1);
-    mbar_init(&bars.ds_ready, 8);
     mbar_init(&bars.acc_done[1], 1);
     mbar_init(&bars.acc_free[1], 4);
     mbar_init(&bars.acc_done[0], 1);
@@ -572,7 +574,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
         }
         tc_fence_before();
         fence_async_smem();
-        arrive_warp(&bars.ds_ready);
+        arrive_warp(&bars.ds_ready[n & 1]);
       }
       if (!alive) break;
       if ((it.flags & kLastOfQ)) {
@@ -923,7 +925,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
     auto issue_dp = [&](uint32_t m, bool after) -> bool {
       uint64_t* const ap = &bars.ap_ready[LARGE ? 0 : m & 1];
       const uint32_t parity = (LARGE ? m : m >> 1) & 1;
-      if (!wait_two(ap, parity, after ? &bars.ds_ready : ap, after ? (m - 1) & 1 : parity)) return false;
+      if (!wait_two(ap, parity, after ? &bars.ds_ready[(m - 1) & 1] : ap, after ? ((m - 1) >> 1) & 1 : parity)) return false;
       tc_fence_after();
       issue_rows(Cfg::kTmemDP, Cfg::kTmemDO, LARGE || !(m & 1) ? a2Lo : sv1Lo);
       commit(&bars.dp_ready);
@@ -950,7 +952,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
         }
         if (do_ds) {
           const bool g_free = mbar_test(&bars.acc_free[0], (n & 1) ^ 1);
-          if (!wait_all(&bars.ds_ready, n & 1)) break;
+          if (!wait_all(&bars.ds_ready[n & 1], (n >> 1) & 1)) break;
           tc_fence_after();
           if (LARGE && more && !issue_dp(n + 1, true)) break;
           const bool fresh = i == 0 && (it.flags & kFirstOfQ);
