@@ -30,9 +30,10 @@
 // What bounds it: the soft-max stage of a slab (1300 cycles against 1024 of exponentials, and 200 between stages) and the change
 // of k-tiles (K2 tile, operands, first scores: 3300 to 4100 cycles before, 2000 of them the operands, now about 2200).  Operands
 // with a thread on one column of every 16th or 32nd row, norms only where a row's bound is asked for, and the fold without
-// exchanges: T=512 D=64 bf16 32 heads 1020 -> 928 us, T=2048 D=128 16 heads 24.0 -> 23.1 ms, T=512 D=128 fp16 16 heads with row
-// maxima 808 -> 765 us; T=4096 D=64 4 heads 33.7 -> 34.2 ms (its k-tiles have 16 slabs, and so little to gain).  The code size matters: with the stages
-// unrolled by tile and mode (165 to 235 KB for 115 to 140) the same changes were 4 to 15 % slower than before them.
+// exchanges: T=512 D=64 bf16 32 heads 1020 -> 921 us, T=2048 D=128 16 heads 23.1 -> 22.7 ms, T=512 D=128 fp16 16 heads with row
+// maxima 808 -> 765 us; T=4096 D=64 4 heads 33.6 ms as before (its k-tiles have 16 slabs, and so little to gain).  The code size
+// matters: with the stages unrolled by tile and mode (165 to 235 KB for 115 to 140) the same changes were 4 to 15 % slower than
+// before them.
 // Causal structure: for a fixed query the mask is "j <= q" on columns and "k <= q" on rows, so
 // whole slabs above q are never visited, only the last slab is masked (by a column bound that
 // is uniform over the rows), and rows with k > q get weight zero in the fold.
@@ -102,6 +103,13 @@ template <bool MASK> struct Columns {
   __device__ __forceinline__ Columns(int l, int h) : lo(l), hi(h), mask(MASK ? column_mask(l, h) : 0u) {}
   __device__ __forceinline__ bool has(int c) const { return MASK ? (mask >> c & 1u) != 0 : c >= lo && c <= hi; }
 };
+
+// Fraction of the soft-max reference that all rows of a head with a small score bound share: -log2(29 / 32).  Scores near zero
+// are the usual case, and their P, near 2^-reference, is then near 29 / 32 of a power of two: on the 16-bit grid, so that scores of
+// zero are not rounded at all, and where the grid's step is small against the value.  At a power of two it is twice as coarse:
+// error of the output against fp64 (bf16 T=64 D=64 / T=333 D=128) 2.90e-3 / 2.91e-3 with whole numbers, 2.57e-3 / 2.59e-3 with
+// this or with each row's own bound as the reference.
+constexpr float kReferenceFraction = 0.142019f;
 
 template <int D, typename T16>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -202,15 +210,17 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
   auto halves = [](int ja, int jb, int j0) { return jb < j0 + 64 ? 1 : (ja >= j0 + 64 ? 2 : 0); };
   // How the soft-max warps divide a head's work.  Every score of the head is bounded by
   // |s| max_q |Q_q| max |K2 element| max_j |K1_j|  (|A_row|^2 = s^2 sum_h Q_h^2 K2_h^2 <= s^2 max_h K2_h^2 |Q_q|^2).
-  // Where that is below the limit, the limit is every row's soft-max reference (one pass, nothing to agree on between threads, nothing
-  // to merge between tiles) and the two warpgroups split every slab's columns; otherwise each warpgroup owns one tile and a
-  // thread its whole row (maximum pass, rescaling).  Uniform over a work item, read by every role.
-  auto head_split = [&](int bh) -> bool {
-    if (!p.k1_norm2_max) return false;
-    const float b = fabsf(p.scale2) * sqrtf(__ldg(p.q_norm2_max + bh)) * sqrtf(__ldg(p.k2_elem2_max + bh)) *
-                    sqrtf(__ldg(p.k1_norm2_max + bh));
-    return b <= p.bound_limit;
+  // Where that is below the limit, all rows of the head have one soft-max reference (head_reference: one pass, nothing to agree on
+  // between threads, nothing to merge between tiles) and the two warpgroups split every slab's columns; otherwise each warpgroup
+  // owns one tile and a thread its whole row (maximum pass, rescaling).  Uniform over a work item, read by every role.
+  auto head_bound = [&](int bh) -> float {
+    if (!p.k1_norm2_max) return INFINITY;
+    return fabsf(p.scale2) * sqrtf(__ldg(p.q_norm2_max + bh)) * sqrtf(__ldg(p.k2_elem2_max + bh)) * sqrtf(__ldg(p.k1_norm2_max + bh));
   };
+  auto head_split = [&](int bh) -> bool { return head_bound(bh) <= p.bound_limit; };
+  // From the head's own bound: with the limit for all heads P of small scores would be 2^-40 in bf16, and the fold's products of
+  // it with values of 1e-13 below fp32's smallest normal number.
+  auto head_reference = [&](int bh) -> float { return ceilf(head_bound(bh)) + kReferenceFraction; };
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -487,6 +497,8 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
       // largest K1 row norm of this head: with |A_row| it bounds every score of the row (Cauchy-Schwarz)
       const float k1_max = p.k1_norm2_max ? sqrtf(__ldg(p.k1_norm2_max + bh)) : INFINITY;
       const bool split = head_split(bh);
+      // (every lane has the same value; the reduction leaves it in a uniform register)
+      const float reference = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(head_reference(bh))));
 
       for (int kt = kt0; kt < kt0 + nkt && alive; ++kt, ++kt_count) {
         int jt0, njt, ja, jb;
@@ -559,10 +571,10 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
 
         if (split) {
           // ---- walk over the slabs, both warpgroups on the same slab: tile a, then tile b; warpgroup `wg` takes the
-          // slab's columns [wg * 64, wg * 64 + 64) (32 of a half-width slab's 64).  The reference of every row is the limit l itself
-          // (log2 units), which the head's score bound is below: P stays within [2^-2l, 1], representable in the 16-bit type, and
-          // no row maximum is needed.  (A launch parameter as the reference costs no register: 928 us at T=512 D=64, against 945
-          // with the head's bound; no reference at all, P = exp2(S), 917.)
+          // slab's columns [wg * 64, wg * 64 + 64) (32 of a half-width slab's 64).  The reference of every row is the head's: with a
+          // bound b of the scores P stays within [2^-(2 b + 1.15), 1], representable in the 16-bit type, and no row maximum is needed.
+          // (B200, forward at T=512 D=64 bf16 32 heads / T=4096 D=64 / T=2048 D=128: 921 us / 33.6 ms / 22.7 ms; a launch parameter
+          // in its place 929 / 34.1 / 22.4.)
           float l_sum[2] = {0.f, 0.f};
           for (int jt = 0; jt < njt && alive; ++jt, ++n) {
             // A slab with attended columns in one 64-column half only was computed for that half alone: its scores
@@ -584,8 +596,8 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
               const int lo = c_lo[x] - j0, hi = c_hi[x] - j0;
               const bool full = __all_sync(0xffffffffu, lo <= 0 && hi >= cw - 1);
               // P over the first half of the columns this thread has read
-              l_sum[x] += nh == 2 ? form_p(std::integral_constant<int, 64>{}, tS, tS, full, lo, hi, p.bound_limit)
-                                  : form_p(std::integral_constant<int, 32>{}, tS, tS, false, lo, hi, p.bound_limit);
+              l_sum[x] += nh == 2 ? form_p(std::integral_constant<int, 64>{}, tS, tS, full, lo, hi, reference)
+                                  : form_p(std::integral_constant<int, 32>{}, tS, tS, full, lo, hi, reference);
               tmem_wait_st();
               tc_fence_before();
               mbar_arrive(&bars.p_ready[x]);
@@ -730,7 +742,7 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
               ok[r] = valid(k, qx);
               v2r[r] = V2g + (size_t)min(k, T - 1) * D + 2 * (lane & 3);
             }
-            constexpr int kC = D == 64 ? 32 : 16;   // columns whose V2 words are fetched together, ahead of the accumulator
+            constexpr int kC = 16;   // columns whose V2 words are fetched together, ahead of the accumulator
             uint32_t v2w[kC / 8][4];
             auto fetch = [&](int c0) {
 #pragma unroll
@@ -817,7 +829,7 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
             const float O = red[(x * 4) * D + row] + red[(x * 4 + 1) * D + row] + red[(x * 4 + 2) * D + row] + red[(x * 4 + 3) * D + row];
             ((T16*)p.out)[((size_t)bh * T + qx) * D + row] = from_f<T16>(O / L);
           }
-          if (row == 0) p.lse[(size_t)bh * T + qx] = (p.bound_limit + log2f(L)) * kLn2;
+          if (row == 0) p.lse[(size_t)bh * T + qx] = (head_reference(bh) + log2f(L)) * kLn2;
         }
         if (!fold_sync()) { alive = false; break; }  // red / fstat are rewritten by the next item
         continue;
@@ -1078,7 +1090,7 @@ int launch_fwd(const TdpArgs& a) {
   p.k1_norm2_max = k1n;
   p.q_norm2_max = k1n ? k1n + BN : nullptr;
   p.k2_elem2_max = k1n ? k1n + 2 * BN : nullptr;
-  // P = exp2(S - reference) lies in [2^(-2 limit), 1]: normal numbers of the 16-bit type (bf16 2^-126, fp16 2^-14)
+  // P = exp2(S - reference) lies in [2^-(2 limit + 1.15), 1]: normal numbers of the 16-bit type (bf16 2^-126, fp16 2^-14)
   p.bound_limit = std::is_same<T16, __nv_bfloat16>::value ? 40.f : 6.f;
   p.status = a.status_word;
   if (p.nq == 0) return 0;
