@@ -252,7 +252,7 @@ template <typename T16> __device__ __forceinline__ int range_shift(float x, floa
   }
   return 0;
 }
-// The same for R = alpha log2(e) Q K2, which is formed in fp32: the largest product is brought to [2^14, 2^15).
+// The same for R = alpha log2(e) Q K2, which is formed in fp32: the bound on the products is brought to [2^14, 2^15).
 template <typename T16> __device__ __forceinline__ int product_shift(float bound) {
   if constexpr (std::is_same<T16, __half>::value) {
     if (!(bound > 0.f) || !isfinite(bound)) return 0;
@@ -289,7 +289,7 @@ __device__ __forceinline__ void red_add4(float* p, float a, float b, float c, fl
 
 // The statistics of a head over its parts, in every lane (zeros without them).
 struct BwdStats {
-  float qk1, k2, sv1, v2;    // largest element of Q and K1, of K2, SiLU(V1), V2
+  float k1, k2, sv1, v2;    // largest element of K1, K2, SiLU(V1), V2
   float k1_row, q_row, do_row, sv1_row;   // largest squared norm of a row
 };
 __device__ __forceinline__ BwdStats head_stats(const BwdParams& p, int bh, int lane) {
@@ -1003,9 +1003,9 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       if (it.len > 0 && it.bh != bh) {
         bh = it.bh;
         const BwdStats st = head_stats(p, bh, lane);
-        ea = range_shift<T16>(st.qk1, st.k2);
+        ea = range_shift<T16>(st.k1, st.k2);
         eb = range_shift<T16>(st.sv1, st.v2);
-        er = product_shift<T16>(fabsf(p.alpha * kLog2e) * st.qk1 * st.k2);
+        er = product_shift<T16>(fabsf(p.alpha * kLog2e) * sqrtf(st.q_row) * st.k2);
         f = ds_shift<T16>(sqrtf(st.do_row * st.sv1_row) * st.v2);
       }
       it.er = er;
@@ -1162,7 +1162,7 @@ tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, co
   __shared__ float wmax[kPrepThreads / 32][kStatFloats];
   const int bh = blockIdx.x / parts, part = blockIdx.x % parts, lanes = D / 8;   // 8 or 16 lanes hold one row
   const uint32_t row_lanes = ((1u << lanes) - 1u) << ((threadIdx.x & 31) / lanes * lanes);
-  float qk1_max = 0.f, k2_max = 0.f, sv1_max = 0.f, v2_max = 0.f, k1_row = 0.f, q_row = 0.f, do_row = 0.f, sv1_row = 0.f;
+  float k1_max = 0.f, k2_max = 0.f, sv1_max = 0.f, v2_max = 0.f, k1_row = 0.f, q_row = 0.f, do_row = 0.f, sv1_row = 0.f;
   auto words = [](const T16* p, uint32_t (&w)[4]) {
     const uint4 x = *reinterpret_cast<const uint4*>(p);
     w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
@@ -1201,7 +1201,7 @@ tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, co
       words(v2 + i, wb);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        grow(qk1_max, unpack2<T16>(wv[e]));
+        grow(k1_max, unpack2<T16>(wv[e]));
         grow(k2_max, unpack2<T16>(wa[e]));
         grow(v2_max, unpack2<T16>(wb[e]));
       }
@@ -1210,7 +1210,6 @@ tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, co
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float2 x = unpack2<T16>(wv[e]), y = unpack2<T16>(wa[e]);
-        grow(qk1_max, y);
         n1 = fmaf(x.x, x.x, fmaf(x.y, x.y, n1));
         nq = fmaf(y.x, y.x, fmaf(y.y, y.y, nq));
       }
@@ -1227,7 +1226,7 @@ tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, co
     }
   }
   if (!stats) return;
-  float w[kStatFloats] = {qk1_max, k2_max, sv1_max, v2_max, k1_row, q_row, do_row, sv1_row};
+  float w[kStatFloats] = {k1_max, k2_max, sv1_max, v2_max, k1_row, q_row, do_row, sv1_row};
 #pragma unroll
   for (int o2 = 16; o2 >= 1; o2 >>= 1)
 #pragma unroll

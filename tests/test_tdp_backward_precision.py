@@ -126,6 +126,15 @@ def test_products_of_small_and_large_keys(dtype, T, D, keys, dout):
     assert all(r <= SPREAD for _, r in ratios), f"errors over those of the precision class: {ratios}"
 
 
+@pytest.mark.parametrize("T,D", [(192, 64), (130, 128)])
+@pytest.mark.parametrize("q,keys", [(30, 3e-4), (1, 1e-4), (30, 1e-4), (1e-3, 100)])
+def test_products_of_keys_beside_queries_of_another_size(T, D, q, keys):
+    """fp32 tensors (fp16 operands, no final rounding).  The range of K1 K2, which dQ is formed from, is that of the keys alone,
+    whatever the queries are."""
+    ratios = _errors(T, D, torch.float32, False, True, (None,) * 4, std=(2 * q, 2 * keys, 1, 1))
+    assert all(r <= SPREAD for _, r in ratios), f"errors over those of the precision class: {ratios}"
+
+
 def test_a_workspace_without_the_statistics_is_accepted():
     """... and forms the fp16 products unshifted, as good for inputs of ordinary size."""
     T, D = 200, 64
