@@ -244,15 +244,21 @@ __device__ __forceinline__ int prob_shift(int q, int causal, int T, int k1w, int
 // the largest that keeps both itself and the largest product the head's elements allow below 2^15.  With the other factor's
 // largest element at 1 or above the largest product has 28 binades of normal numbers below it, at 2^-b 28 - b.
 // The power is divided out in fp32, of S and dP in the soft-max warps and of the sums.  bf16 has fp32's range: 0.
-template <typename T16> __device__ __forceinline__ int range_shift(float x, float other) {
+// Without statistics (or with infinite ones) the power is `otherwise`.
+template <typename T16> __device__ __forceinline__ int range_shift(float x, float other, int otherwise) {
   if constexpr (std::is_same<T16, __half>::value) {
-    if (!(x > 0.f) || !isfinite(x) || !(other > 0.f) || !isfinite(other)) return 0;
+    if (!(x > 0.f) || !isfinite(x) || !(other > 0.f) || !isfinite(other)) return otherwise;
     const int a = (__float_as_int(x) >> 23) - 127, b = (__float_as_int(other) >> 23) - 127;
     return 14 - a - max(b + 1, 0);
   }
   return 0;
 }
-// The same for R = alpha log2(e) Q K2, which is formed in fp32: the bound on the products is brought to [2^14, 2^15).
+// A's power without statistics: as large as alpha log2(e), so that keys of 300 under an alpha of 1/64 do not overflow, and at most
+// 1; 2^-17 keeps every product of two fp16 numbers finite.
+__device__ __forceinline__ int alpha_shift(float alpha) {
+  return min(0, max(-17, (int)(__float_as_uint(fabsf(alpha * kLog2e)) >> 23) - 127));
+}
+// The power of R = alpha log2(e) Q K2, which is formed in fp32: the bound on the products is brought to [2^14, 2^15).
 template <typename T16> __device__ __forceinline__ int product_shift(float bound) {
   if constexpr (std::is_same<T16, __half>::value) {
     if (!(bound > 0.f) || !isfinite(bound)) return 0;
@@ -1003,8 +1009,8 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       if (it.len > 0 && it.bh != bh) {
         bh = it.bh;
         const BwdStats st = head_stats(p, bh, lane);
-        ea = range_shift<T16>(st.k1, st.k2);
-        eb = range_shift<T16>(st.sv1, st.v2);
+        ea = range_shift<T16>(st.k1, st.k2, alpha_shift(p.alpha));
+        eb = range_shift<T16>(st.sv1, st.v2, 0);
         er = product_shift<T16>(fabsf(p.alpha * kLog2e) * sqrtf(st.q_row) * st.k2);
         f = ds_shift<T16>(sqrtf(st.do_row * st.sv1_row) * st.v2);
       }
@@ -1363,7 +1369,7 @@ template <int D> BwdPlan make_plan(const TdpArgs& a) {
 }
 
 // workspace: fp32 sums dK1 | dK2 | dSiLU(V1) | dV2 | dQ, SiLU(V1) in the inputs' type, Dq fp32; and, where the caller's has
-// it, the statistics (without them fp16 products are formed unshifted)
+// it, the statistics (without them fp16 products are formed without regard to their size)
 template <int D, typename T16>
 int launch_bwd_sums(const TdpArgs& a, const BwdPlan& plan) {
   using Cfg = BwdCfg<D>;

@@ -73,7 +73,8 @@ const char* tritt_last_error(void);
    lets the forward bound its scores and skip the row-maximum pass; a workspace without the tail is accepted and runs
    the two-pass soft-max.  For TRITT_OP_TDP_BWD on the tensor cores it includes a tail of about 1 KiB per (batch, head)
    for the largest elements behind the range shifts of fp16 products; a workspace without it is accepted and forms them
-   unshifted (small keys or values then lose bits to fp16's subnormals). */
+   without regard to their size, times alpha (at most 1, to a power of two) for the keys: small keys or values then lose
+   bits to fp16's subnormals, and keys whose products times alpha reach 65504 overflow. */
 size_t tritt_workspace_bytes(int op, int B, int N, int T, int D, int dtype);
 /* The same for a call that will pass `flags` (TRITT_FLAG_WIDE_OPERANDS enlarges the triple-dot-product workspace of bf16
    inputs by the fp16 operand copies; tritt_workspace_bytes() equals flags = 0). */

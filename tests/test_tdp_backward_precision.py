@@ -135,10 +135,13 @@ def test_products_of_keys_beside_queries_of_another_size(T, D, q, keys):
     assert all(r <= SPREAD for _, r in ratios), f"errors over those of the precision class: {ratios}"
 
 
-def test_a_workspace_without_the_statistics_is_accepted():
-    """... and forms the fp16 products unshifted, as good for inputs of ordinary size."""
-    T, D = 200, 64
-    x = [t.to(DEV) for t in orc.make_inputs(1, 2, T, D, scale=0.5, seed=5, dtype=torch.float16)]
+@pytest.mark.parametrize("D,q,keys", [(64, 1, 1), (64, 1e-3, 400), (128, 1e-3, 600)])
+def test_a_workspace_without_the_statistics_is_accepted(D, q, keys):
+    """... and is as good for inputs of ordinary size, and for keys of 200 and 300, whose products are beyond fp16's range but
+    not those with alpha."""
+    T = 200
+    x = orc.make_inputs(1, 2, T, D, scale=0.5, seed=5)
+    x = [(t * s).to(DEV, torch.float16) for t, s in zip(x, (q, keys, keys, 1, 1, 1))]
     do = x.pop()
     o, lse = torch.empty_like(do), torch.empty(1, 2, T, device=DEV)
     _native.tdp_fwd(*x, o, lse, 1 / D, True, None, None, None, None)
