@@ -60,8 +60,9 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
 }
 
 // Wait limit: every wait in these kernels gives up after this many clock ticks (about a
-// second) and reports failure instead of spinning forever.
+// second) and reports failure instead of spinning forever, by one of the two functions below.
 constexpr long long kWaitTicks = 2000000000LL;
+static_assert(kWaitTicks < 1LL << 31, "mbar_wait_looks compares the low half of the clock");
 
 // Bounded wait.  `abort_flag` is a CTA-shared word that any thread sets when its wait ran
 // out; once set, every later wait returns false immediately so that all warps fall through
@@ -83,16 +84,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return mbar_wait_limit(bar, parity, abort_flag, kWaitTicks);
 }
 
-// The same with the limit as a number of looks: less code than with the clock (waits are inlined in many places and the
-// instruction caches are small) and fewer issue slots taken from the warps beside the waiting one; the abort flag is looked at
-// every 64 of them.  A look takes some 30 to 100 clock ticks, so the limit is about a second.  The backward kernel is faster
-// with it (16 heads T=512 D=64 not causal 1.83 -> 1.76 ms, windows 128/128/32/32 at T=2048 1.20 -> 1.13 ms), the forward ones
-// are not (band kernel 0.47 -> 0.49 ms).
-__device__ __forceinline__ bool mbar_wait_looks(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  uint32_t looks = 0;
+// The same with fewer instructions in the loop (waits are inlined in many places and the instruction caches are small) and fewer
+// issue slots taken from the warps beside the waiting one: the clock and the abort flag are looked at every 64 looks.  The
+// backward kernel is faster with it (16 heads T=512 D=64 not causal 1.83 -> 1.76 ms, windows 128/128/32/32 at T=2048 1.20 -> 1.13
+// ms), the forward ones are not (band kernel 0.47 -> 0.49 ms).  (The low half of the clock: the limit is below 2^31 ticks.)
+__device__ __forceinline__ bool mbar_wait_looks(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                uint32_t limit_ticks = (uint32_t)kWaitTicks) {
+  uint32_t looks = 0, t0 = 0;
   while (!mbar_try_wait(bar, parity)) {
     if (++looks % 64 == 0) {
-      if (looks >= 1u << 24) *abort_flag = 1;
+      const uint32_t now = (uint32_t)clock();
+      if (looks == 64) t0 = now;
+      if (now - t0 > limit_ticks) *abort_flag = 1;
       if (*abort_flag) return false;
     }
   }

@@ -115,16 +115,16 @@ umma_selftest_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   if (warp == 0) tmem_dealloc(tbase, 512);
 }
 
-// Exercises the time-out path every tensor-core kernel shares: one thread is meant to arrive on an mbarrier, a
-// warp waits for it with the bounded wait.  With `skip_arrival` the arrival never happens, the wait gives up after
-// `limit_ticks` clock ticks, the CTA records status bit 128, releases its tensor memory and returns normally.
-__global__ void __launch_bounds__(64, 1) wait_expiry_kernel(int skip_arrival, long long limit_ticks, int* status) {
+// Exercises the time-out path every tensor-core kernel shares: one thread is meant to arrive on an mbarrier, one warp waits for it
+// with each of the two bounded waits.  With `skip_arrival` the arrival never happens, the waits give up after `limit_ticks` clock
+// ticks, the CTA records status bit 128 (bit 1 if only one of the two gave up), releases its tensor memory and returns normally.
+__global__ void __launch_bounds__(96, 1) wait_expiry_kernel(int skip_arrival, long long limit_ticks, int* status) {
   __shared__ uint64_t bar;
   __shared__ uint32_t tmem_base_s;
-  __shared__ int abort_flag;
+  __shared__ int abort_flag[2];
   const int tid = threadIdx.x, warp = tid >> 5;
   if (tid == 0) {
-    abort_flag = 0;
+    abort_flag[0] = abort_flag[1] = 0;
     mbar_init(&bar, 1);
     fence_barrier_init();
   }
@@ -138,13 +138,15 @@ __global__ void __launch_bounds__(64, 1) wait_expiry_kernel(int skip_arrival, lo
   bool ok = true;
   if (warp == 0) {
     if (tid == 0 && !skip_arrival) mbar_arrive(&bar);
+  } else if (warp == 1) {
+    ok = __all_sync(0xffffffffu, mbar_wait_limit(&bar, 0, &abort_flag[0], limit_ticks));
   } else {
-    ok = __all_sync(0xffffffffu, mbar_wait_limit(&bar, 0, &abort_flag, limit_ticks));
+    ok = __all_sync(0xffffffffu, mbar_wait_looks(&bar, 0, &abort_flag[1], (uint32_t)limit_ticks));
   }
   tc_fence_before();
-  __syncthreads();
+  const int gave_up = __syncthreads_count(!ok);
   if (warp == 0) tmem_dealloc(tmem_base_s, 32);
-  if (tid == 32 && !ok && status) atomicOr(status, 128);
+  if (tid == 0 && gave_up && status) atomicOr(status, gave_up == 64 && abort_flag[0] && abort_flag[1] ? 128 : 1);
 }
 
 }  // namespace
@@ -157,7 +159,7 @@ extern "C" int tritt_selftest_wait_expiry(int skip_arrival, long long limit_tick
     set_error("limit_ticks must lie in [1, %lld]", sm100::kWaitTicks);
     return -1;
   }
-  wait_expiry_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(skip_arrival, limit_ticks, status_word);
+  wait_expiry_kernel<<<1, 96, 0, (cudaStream_t)stream>>>(skip_arrival, limit_ticks, status_word);
   count_launch();
   TRITT_CUDA_OK(cudaGetLastError());
   return 0;

@@ -194,10 +194,11 @@ int tritt_selftest_umma(const void* A, const void* Bm, const void* V, float* C, 
                         int* status_word, tritt_stream_t stream);
 
 /*
- * Self-test of the bounded barrier wait that every tensor-core kernel uses: a one-CTA kernel in which one
- * thread is to arrive on an mbarrier and a warp waits for it, giving up after `limit_ticks` clock ticks
- * (1 .. 2e9).  With skip_arrival != 0 the arrival is left out on purpose: the wait runs out, the kernel ORs
- * 128 into `status_word`, frees its tensor memory and returns; nothing faults and the context stays usable.
+ * Self-test of the two bounded barrier waits that the tensor-core kernels use: a one-CTA kernel in which one
+ * thread is to arrive on an mbarrier and a warp waits for it with each, giving up after `limit_ticks` clock ticks
+ * (1 .. 2e9).  With skip_arrival != 0 the arrival is left out on purpose: the waits run out, the kernel ORs
+ * 128 into `status_word` (1 if only one of them gave up), frees its tensor memory and returns; nothing faults and
+ * the context stays usable.
  * No counterpart in the reference (Triton kernels have no hand-written waits).
  */
 int tritt_selftest_wait_expiry(int skip_arrival, long long limit_ticks, int* status_word, tritt_stream_t stream);

@@ -1,9 +1,10 @@
 """A bounded device-side wait that runs out, on purpose and without a fault.
 
-Every tensor-core kernel waits on its mbarriers through one bounded wait (``mbar_wait_limit``): after the limit the
-CTA records a status bit, releases its tensor memory and returns.  ``tritt_selftest_wait_expiry`` runs exactly that
-path in a one-CTA kernel whose producer can be told to skip its arrival, with the limit passed in (a few hundred
-thousand ticks, i.e. well under a millisecond).  Checked here: the call returns, the status word is set, the context
+Every tensor-core kernel waits on its mbarriers through one of two bounded waits (``mbar_wait_limit``, and
+``mbar_wait_looks``, which reads the clock less often): after the limit the CTA records a status bit, releases its
+tensor memory and returns.  ``tritt_selftest_wait_expiry`` runs exactly that path, a warp for each of the two, in a
+one-CTA kernel whose producer can be told to skip its arrival, with the limit passed in (a few hundred thousand ticks,
+i.e. well under a millisecond).  Checked here: the call returns, the status word says that both gave up, the context
 stays usable (the next ordinary call is correct), and the Python layer raises at the next entry point."""
 import pytest
 import torch
