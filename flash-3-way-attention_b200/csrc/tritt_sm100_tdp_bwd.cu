@@ -51,8 +51,9 @@ using namespace sm100;
 
 constexpr int kBwdThreads = 640;
 // Registers per thread: 640 threads are launched with 96 each (480 per lane of the five warpgroups) and split them anew.  The
-// shares are tight: the two bodies spill 360 to 620 bytes a thread together, most of it what an item or a step reads once or
-// twice.  (80 / 128 / 64 or 96 / 120 / 48 for soft-max, fold and service warps: 5 to 8 % slower, as their loops spill.)
+// shares are tight: the two bodies spill 380 to 530 bytes a thread together, most of it what an item or a step reads once or
+// twice.  (80 / 128 / 64 or 96 / 120 / 48 for soft-max, fold and service warps in the small-score body: 5 to 8 % slower, as their
+// loops spill.)
 constexpr int kRegsLaunch = 96;
 // (Large scores at head dimension 128 have the service warps form 32 KB of R per step, and soft-max warps that hold half as many
 // columns as at 64: with 48 registers those service warps spill, 1.60 -> 1.90 ms at 16 heads of T=512.)
@@ -489,94 +490,169 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
           hi = k <= q && q - k <= g.k2w ? min(q, k + g.kkr) - j0 : lo - 1;
         }
         if (!q_ok) hi = lo - 1;
-        // Half of the columns S -> P; then, eight columns at a time, the other half S -> P beside dP and P (still in fp32) ->
-        // dS of the first, so that exponentials and arithmetic overlap within a warp; then dS of the second half.
         alive = __all_sync(0xffffffffu, s_seen) || wait_all(&bars.s_ready, n & 1);
         if (!alive) break;
         tc_fence_after();
-        bool seen = false;   // (looks at barriers ahead of their waits)
         uint8_t* const dsrow = prow + (1 + (n & 1)) * Cfg::kTileP;
         const bool full = __all_sync(0xffffffffu, lo <= 0 && hi >= CW - 1);
-        const uint32_t tS = tmem + lane_base + Cfg::kTmemS + wg * CW, tDP = tmem + lane_base + Cfg::kTmemDP + wg * CW;
-        constexpr int SN = D == 128 ? H : 8;   // (head dimension 64 has no registers for all of them)
-        uint32_t s[H], sn[SN], dp[8];   // scores, then P; scores of the second half; dP
-        // columns c.. of S -> P
-        auto to_p = [&](int c, uint32_t* v, const uint32_t* x) {
-          if (full) {
+        if constexpr (LARGE) {
+          // 32 columns at a time: S -> P, then dP and P (still in fp32) -> dS.  (What the other body does, half of the columns beside
+          // the other half, gains nothing behind one issuing warp, and spills: 944 against 920 us at 16 heads of T=512 D=64 fp16,
+          // 5460 against 5320 at T=1024 D=128 8 heads.)
+#pragma unroll 1
+          for (int c0 = 0; c0 < CW; c0 += 32) {
+            uint32_t s[32];
+            tmem_ld32(tmem + lane_base + Cfg::kTmemS + wg * CW + c0, s);
+            tmem_wait_ld();
+            if (c0 + 32 == CW) {
+              // the scores are in registers: the next step's product may overwrite them
+              tc_fence_before();
+              arrive_warp(&bars.s_free);
+            }
+            if (full) {
+#pragma unroll
+              for (int c = 0; c < 32; c += 2) {
+                const float2 x = scaled(s[c], s[c + 1], sa, nlse);
+                s[c] = __float_as_uint(exp2f(x.x));
+                s[c + 1] = __float_as_uint(exp2f(x.y));
+              }
+            } else {
+#pragma unroll
+              for (int c = 0; c < 32; ++c)
+                s[c] = c0 + c >= lo && c0 + c <= hi ? __float_as_uint(exp2f(fmaf(__uint_as_float(s[c]), sa, -lse2))) : 0u;
+            }
+            if (c0 == 0) {
+              // the previous step's U has read P
+              alive = wait_all(&bars.acc_done[1], (n & 1) ^ 1);
+              if (!alive) break;
+            }
+#pragma unroll
+            for (int c = 0; c < 32; c += 8) {
+              uint32_t w[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                w[e] = pack2<T16>(__uint_as_float(s[c + 2 * e]), __uint_as_float(s[c + 2 * e + 1]));
+              *reinterpret_cast<uint4*>(prow + swz128(row, ch0 + ((c0 + c) >> 3))) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+            if (c0 + 32 == CW) {
+              fence_async_smem();
+              arrive_warp(&bars.p_ready);
+            }
+            if (any_single) {
+#pragma unroll
+              for (int c = 0; c < 32; ++c) s[c] = single ? 0u : s[c];
+            }
+            if (c0 == 0) {
+              alive = wait_all(&bars.dp_ready, n & 1);
+              if (alive) alive = wait_all(&bars.ds_free[n & 1], ((n >> 1) & 1) ^ 1);
+              if (!alive) break;
+              tc_fence_after();
+            }
+#pragma unroll
+            for (int c1 = 0; c1 < 32; c1 += 16) {
+              uint32_t dp[16];
+              tmem_ld16(tmem + lane_base + Cfg::kTmemDP + wg * CW + c0 + c1, dp);
+              tmem_wait_ld();
+#pragma unroll
+              for (int c = 0; c < 16; c += 8) {
+                uint32_t w[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const float2 d = scaled(dp[c + 2 * e], dp[c + 2 * e + 1], sb, ndq);
+                  const float2 ds = __fmul2_rn(
+                      make_float2(__uint_as_float(s[c1 + c + 2 * e]), __uint_as_float(s[c1 + c + 2 * e + 1])), d);
+                  w[e] = pack2<T16>(ds.x, ds.y);
+                }
+                *reinterpret_cast<uint4*>(dsrow + swz128(row, ch0 + ((c0 + c1 + c) >> 3))) = make_uint4(w[0], w[1], w[2], w[3]);
+              }
+            }
+          }
+          if (!alive) break;
+        } else {
+          // Half of the columns S -> P; then, eight columns at a time, the other half S -> P beside dP and P (still in fp32) ->
+          // dS of the first, so that exponentials and arithmetic overlap within a warp; then dS of the second half.
+          bool seen = false;   // (looks at barriers ahead of their waits)
+          const uint32_t tS = tmem + lane_base + Cfg::kTmemS + wg * CW, tDP = tmem + lane_base + Cfg::kTmemDP + wg * CW;
+          constexpr int SN = D == 128 ? H : 8;   // (head dimension 64 has no registers for all of them)
+          uint32_t s[H], sn[SN], dp[8];   // scores, then P; scores of the second half; dP
+          // columns c.. of S -> P
+          auto to_p = [&](int c, uint32_t* v, const uint32_t* x) {
+            if (full) {
+#pragma unroll
+              for (int e = 0; e < 8; e += 2) {
+                const float2 y = scaled(x[e], x[e + 1], sa, nlse);
+                v[e] = __float_as_uint(exp2f(y.x));
+                v[e + 1] = __float_as_uint(exp2f(y.y));
+              }
+            } else {
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                v[e] = c + e >= lo && c + e <= hi ? __float_as_uint(exp2f(fmaf(__uint_as_float(x[e]), sa, -lse2))) : 0u;
+            }
+          };
+          auto put = [&](uint8_t* row_base, int c, const uint32_t* v) {
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) w[e] = pack2<T16>(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));
+            *reinterpret_cast<uint4*>(row_base + swz128(row, ch0 + (c >> 3))) = make_uint4(w[0], w[1], w[2], w[3]);
+          };
+          // columns c..: P in v and dP in dp -> dS
+          auto to_ds = [&](int c, const uint32_t* v) {
+            uint32_t w[8];
 #pragma unroll
             for (int e = 0; e < 8; e += 2) {
-              const float2 y = scaled(x[e], x[e + 1], sa, nlse);
-              v[e] = __float_as_uint(exp2f(y.x));
-              v[e + 1] = __float_as_uint(exp2f(y.y));
+              float2 pv = make_float2(__uint_as_float(v[e]), __uint_as_float(v[e + 1]));
+              if (!kScaled && any_single) pv = single ? make_float2(0.f, 0.f) : pv;
+              const float2 ds = __fmul2_rn(pv, scaled(dp[e], dp[e + 1], sb, ndq));
+              w[e] = __float_as_uint(ds.x);
+              w[e + 1] = __float_as_uint(ds.y);
             }
-          } else {
+            put(dsrow, c, w);
+          };
+          tmem_ld(tS, s);
+          tmem_wait_ld(s);
+          seen = mbar_test(&bars.acc_done[1], (n & 1) ^ 1);
+          tmem_ld(tS + H, sn);
 #pragma unroll
-            for (int e = 0; e < 8; ++e)
-              v[e] = c + e >= lo && c + e <= hi ? __float_as_uint(exp2f(fmaf(__uint_as_float(x[e]), sa, -lse2))) : 0u;
+          for (int c = 0; c < H; c += 8) to_p(c, s + c, s + c);
+          // the previous step's U has read P
+          alive = __all_sync(0xffffffffu, seen) || wait_all(&bars.acc_done[1], (n & 1) ^ 1);
+          if (!alive) break;
+          seen = test_two(&bars.dp_ready, n & 1, &bars.ds_free[n & 1], ((n >> 1) & 1) ^ 1);
+#pragma unroll
+          for (int c = 0; c < H; c += 8) put(prow, c, s + c);
+          alive = __all_sync(0xffffffffu, seen) || wait_two(&bars.dp_ready, n & 1, &bars.ds_free[n & 1], ((n >> 1) & 1) ^ 1);
+          if (!alive) break;
+          tc_fence_after();
+          tmem_ld(tDP, dp);
+#pragma unroll
+          for (int c = 0; c < H; c += 8) {
+            tmem_wait_ld(sn, dp);
+            if (SN == H ? c == 0 : c + 8 == H) {
+              // the scores are in registers: the next step's product may overwrite them
+              tc_fence_before();
+              arrive_warp(&bars.s_free);
+            }
+            uint32_t x[8];
+            to_ds(c, s + c);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[e] = sn[SN == H ? c + e : e];
+            tmem_ld(tDP + c + 8, dp);
+            if constexpr (SN == 8) {
+              if (c + 8 < H) tmem_ld(tS + H + c + 8, sn);
+            }
+            to_p(H + c, s + c, x);
+            put(prow, H + c, s + c);
           }
-        };
-        auto put = [&](uint8_t* row_base, int c, const uint32_t* v) {
-          uint32_t w[4];
+          fence_async_smem();
+          arrive_warp(&bars.p_ready);
+          s_seen = mbar_test(&bars.s_ready, (n + 1) & 1);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) w[e] = pack2<T16>(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));
-          *reinterpret_cast<uint4*>(row_base + swz128(row, ch0 + (c >> 3))) = make_uint4(w[0], w[1], w[2], w[3]);
-        };
-        // columns c..: P in v and dP in dp -> dS
-        auto to_ds = [&](int c, const uint32_t* v) {
-          uint32_t w[8];
-#pragma unroll
-          for (int e = 0; e < 8; e += 2) {
-            float2 pv = make_float2(__uint_as_float(v[e]), __uint_as_float(v[e + 1]));
-            if (!kScaled && any_single) pv = single ? make_float2(0.f, 0.f) : pv;
-            const float2 ds = __fmul2_rn(pv, scaled(dp[e], dp[e + 1], sb, ndq));
-            w[e] = __float_as_uint(ds.x);
-            w[e + 1] = __float_as_uint(ds.y);
+          for (int c = 0; c < H; c += 8) {
+            tmem_wait_ld(dp);
+            to_ds(H + c, s + c);
+            if (c + 8 < H) tmem_ld(tDP + H + c + 8, dp);
           }
-          put(dsrow, c, w);
-        };
-        tmem_ld(tS, s);
-        tmem_wait_ld(s);
-        seen = mbar_test(&bars.acc_done[1], (n & 1) ^ 1);
-        tmem_ld(tS + H, sn);
-#pragma unroll
-        for (int c = 0; c < H; c += 8) to_p(c, s + c, s + c);
-        // the previous step's U has read P
-        alive = __all_sync(0xffffffffu, seen) || wait_all(&bars.acc_done[1], (n & 1) ^ 1);
-        if (!alive) break;
-        seen = test_two(&bars.dp_ready, n & 1, &bars.ds_free[n & 1], ((n >> 1) & 1) ^ 1);
-#pragma unroll
-        for (int c = 0; c < H; c += 8) put(prow, c, s + c);
-        alive = __all_sync(0xffffffffu, seen) || wait_two(&bars.dp_ready, n & 1, &bars.ds_free[n & 1], ((n >> 1) & 1) ^ 1);
-        if (!alive) break;
-        tc_fence_after();
-        tmem_ld(tDP, dp);
-#pragma unroll
-        for (int c = 0; c < H; c += 8) {
-          tmem_wait_ld(sn, dp);
-          if (SN == H ? c == 0 : c + 8 == H) {
-            // the scores are in registers: the next step's product may overwrite them
-            tc_fence_before();
-            arrive_warp(&bars.s_free);
-          }
-          uint32_t x[8];
-          to_ds(c, s + c);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) x[e] = sn[SN == H ? c + e : e];
-          tmem_ld(tDP + c + 8, dp);
-          if constexpr (SN == 8) {
-            if (c + 8 < H) tmem_ld(tS + H + c + 8, sn);
-          }
-          to_p(H + c, s + c, x);
-          put(prow, H + c, s + c);
-        }
-        fence_async_smem();
-        arrive_warp(&bars.p_ready);
-        s_seen = mbar_test(&bars.s_ready, (n + 1) & 1);
-#pragma unroll
-        for (int c = 0; c < H; c += 8) {
-          tmem_wait_ld(dp);
-          to_ds(H + c, s + c);
-          if (c + 8 < H) tmem_ld(tDP + H + c + 8, dp);
         }
         tc_fence_before();
         fence_async_smem();
@@ -1073,8 +1149,8 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
     const uint8_t* const src = smem + Cfg::kOffQ + (col >> 3) * 16384;
     uint8_t* const dst = smem + (col >> 3 ? Cfg::kOffR1 : Cfg::kOffR0);
     const T16* const vec = reinterpret_cast<const T16*>(smem + Cfg::kOffVec) + col * 8;
-    constexpr int kPieces = 2, kGroups = 128 / kRowStep / kPieces;
-    // byte offset of piece e of group g: the swizzle of a row depends on its last three bits, that is on e alone
+    // byte offset of piece e of group g: the swizzle of a row depends on its last three bits, that is on e alone (a group is 8 rows)
+    constexpr int kPieces = 8 / kRowStep, kGroups = 128 / 8;
     uint32_t swz[kPieces];
 #pragma unroll
     for (int e = 0; e < kPieces; ++e) swz[e] = swz128(row0 + e * kRowStep, col & 7);
