@@ -30,8 +30,8 @@
 // What bounds it: the soft-max stage of a slab (1300 cycles against 1024 of exponentials, and 200 between stages) and the change
 // of k-tiles (K2 tile, operands, first scores: 3300 to 4100 cycles before, 2000 of them the operands, now about 2200).  Operands
 // with a thread on one column of every 16th or 32nd row, norms only where a row's bound is asked for, and the fold without
-// exchanges: T=512 D=64 bf16 32 heads 1020 -> 921 us, T=2048 D=128 16 heads 23.1 -> 22.7 ms, T=512 D=128 fp16 16 heads with row
-// maxima 808 -> 765 us; T=4096 D=64 4 heads 33.6 ms as before (its k-tiles have 16 slabs, and so little to gain).  The code size
+// exchanges: T=512 D=64 bf16 32 heads 1028 -> 925 us, T=4096 D=64 4 heads 33.5 -> 32.9 ms, T=2048 D=128 16 heads 23.5 -> 23.0 ms,
+// T=512 D=128 fp16 16 heads with row maxima 808 -> 757 us; with row maxima at T=2048 D=64 4 heads 5.33 -> 5.40 ms.  The code size
 // matters: with the stages unrolled by tile and mode (165 to 235 KB for 115 to 140) the same changes were 4 to 15 % slower than
 // before them.
 // Causal structure: for a fixed query the mask is "j <= q" on columns and "k <= q" on rows, so
@@ -351,6 +351,10 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
         }
       };
 
+      // Each tile's end is told to the fold warps as it comes (head dimension 128: T=2048 16 heads 23.0 ms against 23.3 with both at
+      // the end of the k-tile, T=333 94 against 96 us), or both at the end (64: the loop over the slabs is shorter by it, T=4096 4
+      // heads 32.9 against 33.5 ms, T=2048 with large scores 5.40 against 5.49, T=512 32 heads 925 against 922 us).
+      constexpr bool kDoneByTile = D == 128;
       for (long item = blockIdx.x; item < n_items && alive; item += gridDim.x) {
         int bh, qa, qb, kt0, nkt;
         decode(item, bh, qa, qb);
@@ -381,7 +385,7 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
               tc_fence_after();
               if (x == 0 && !wait_full(pv)) { alive = false; break; }
               issue_pv(x, pv, jt > 0, hm, split);
-              if (!more) commit(&bars.o_done[x]);
+              if (kDoneByTile && !more) commit(&bars.o_done[x]);
               if (x == 1) release(pv);
               if (more) {
                 if (x == 0 && !wait_full(pk)) { alive = false; break; }
@@ -390,6 +394,10 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
               }
             }
             hm = hm_next;
+          }
+          if (!kDoneByTile && alive) {
+            commit(&bars.o_done[0]);
+            commit(&bars.o_done[1]);
           }
           base += 2 * njt;
         }
@@ -573,8 +581,7 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
           // ---- walk over the slabs, both warpgroups on the same slab: tile a, then tile b; warpgroup `wg` takes the
           // slab's columns [wg * 64, wg * 64 + 64) (32 of a half-width slab's 64).  The reference of every row is the head's: with a
           // bound b of the scores P stays within [2^-(2 b + 1.15), 1], representable in the 16-bit type, and no row maximum is needed.
-          // (B200, forward at T=512 D=64 bf16 32 heads / T=4096 D=64 / T=2048 D=128: 921 us / 33.6 ms / 22.7 ms; a launch parameter
-          // in its place 929 / 34.1 / 22.4.)
+          // (T=2048 D=128 bf16 16 heads 22.7 ms, with a launch parameter in its place 22.4; T=333 93 against 92 us.)
           float l_sum[2] = {0.f, 0.f};
           for (int jt = 0; jt < njt && alive; ++jt, ++n) {
             // A slab with attended columns in one 64-column half only was computed for that half alone: its scores

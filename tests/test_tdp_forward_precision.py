@@ -56,9 +56,10 @@ def _references(x, alpha, causal):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("T,D,scale,causal,kinds", [
     (24, 64, 0.5, True, (1.0,)), (24, 128, 0.5, True, (1.0,)), (33, 128, 0.5, False, (1.0,)), (24, 64, 0.02, True, (1.0,)),
+    (24, 64, 0.5, True, (2.5,)), (24, 128, 0.5, True, (2.0,)),
     (40, 64, 0.5, True, (1.0, 4.0)), (40, 128, 0.5, True, (1.0, 1.0, 4.0))])
 def test_the_output_is_as_exact_as_the_precision_class(T, D, scale, causal, kinds, dtype):
-    """Small scores; heads with small and large scores (Q and the keys times 4: bounds of 80 and more) in one CTA."""
+    """Small scores (of 0.01 to 0.3, in log2 units); heads with small and large scores (Q and the keys times 4: bounds of 80 and more) in one CTA."""
     heads = 512
     x = [t.to(DEV) for t in orc.make_inputs(1, heads, T, D, scale=scale, seed=T + D)[:5]]
     kind = torch.tensor([kinds[h % len(kinds)] for h in range(heads)], device=DEV)
