@@ -27,13 +27,13 @@
 //   warps 12-15  fold warpgroup: when a k-tile is finished, folds acc_x (times V2, soft-max over k) into
 //                the queries' running (max, sum, output) while the other warps start the next k-tile; with one reference for
 //                a head the sums just add up in registers, without exchanges between threads
-// What bounds it: the soft-max stage of a slab (1300 cycles against 1024 of exponentials, and 200 between stages) and the change
-// of k-tiles (K2 tile, operands, first scores: 3300 to 4100 cycles before, 2000 of them the operands, now about 2200).  Operands
-// with a thread on one column of every 16th or 32nd row, norms only where a row's bound is asked for, and the fold without
-// exchanges: T=512 D=64 bf16 32 heads 1028 -> 925 us, T=4096 D=64 4 heads 33.5 -> 32.9 ms, T=2048 D=128 16 heads 23.5 -> 23.0 ms,
-// T=512 D=128 fp16 16 heads with row maxima 808 -> 757 us; with row maxima at T=2048 D=64 4 heads 5.33 -> 5.40 ms.  The code size
-// matters: with the stages unrolled by tile and mode (165 to 235 KB for 115 to 140) the same changes were 4 to 15 % slower than
-// before them.
+// What bounds it: the exponentials (65 % of the special-function unit's time at head dimension 64, 57 % at 128, where the products
+// take as long), the rest of the soft-max stage of a slab around them and the change of k-tiles.  A time trace of the form before had
+// 1300 cycles a stage against 1024 of exponentials, and 3300 to 4100 a change, 2000 of them the operands.  Operands with a thread on
+// one column of every 16th or 32nd row, norms only where a row's bound is asked for, and the fold without exchanges: T=512 D=64 bf16
+// 32 heads 1034 -> 900 us, T=4096 D=64 4 heads 33.6 -> 33.1 ms, T=2048 D=128 16 heads 23.1 -> 22.6 ms; with row maxima T=512 D=128
+// fp16 16 heads 812 -> 740 us, T=2048 D=64 4 heads 5.33 ms, same.  The code size matters: with the stages unrolled by tile and mode
+// (165 to 235 KB for 115 to 140) the same changes were 4 to 15 % slower than before them.
 // Causal structure: for a fixed query the mask is "j <= q" on columns and "k <= q" on rows, so
 // whole slabs above q are never visited, only the last slab is masked (by a column bound that
 // is uniform over the rows), and rows with k > q get weight zero in the fold.
@@ -351,9 +351,9 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
         }
       };
 
-      // Each tile's end is told to the fold warps as it comes (head dimension 128: T=2048 16 heads 23.0 ms against 23.3 with both at
-      // the end of the k-tile, T=333 94 against 96 us), or both at the end (64: the loop over the slabs is shorter by it, T=4096 4
-      // heads 32.9 against 33.5 ms, T=2048 with large scores 5.40 against 5.49, T=512 32 heads 925 against 922 us).
+      // Each tile's end is told to the fold warps as it comes (head dimension 128: T=1024 fp16 8 heads 3.54 ms against 3.56 with both
+      // at the end of the k-tile, T=2048 16 heads 22.6 against 22.7), or both at the end (64: the loop over the slabs is shorter by
+      // it, T=2048 with large scores 5.33 against 5.42 ms, fp16 6.03 against 6.14, T=512 32 heads 900 against 911 us).
       constexpr bool kDoneByTile = D == 128;
       for (long item = blockIdx.x; item < n_items && alive; item += gridDim.x) {
         int bh, qa, qb, kt0, nkt;
@@ -504,191 +504,198 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
       const T16* Qg = (const T16*)p.q + (size_t)bh * T * D;
       // largest K1 row norm of this head: with |A_row| it bounds every score of the row (Cauchy-Schwarz)
       const float k1_max = p.k1_norm2_max ? sqrtf(__ldg(p.k1_norm2_max + bh)) : INFINITY;
-      const bool split = head_split(bh);
-      // (every lane has the same value; the reduction leaves it in a uniform register)
-      const float reference = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(head_reference(bh))));
-
-      for (int kt = kt0; kt < kt0 + nkt && alive; ++kt, ++kt_count) {
-        int jt0, njt, ja, jb;
-        j_range(qa, qb, kt, jt0, njt);
-        col_span(qa, qb, kt, ja, jb);
-        // Columns this row may see, per tile: [c_lo, c_hi].  A row outside the k range of its query (its weight in
-        // the fold is zero) keeps the query's own column range so that it never sees an empty one by construction;
-        // a row inside can still see none in a slab, or at all: its maximum then stays -inf and its P zero.
-        int c_lo[2] = {0, 0}, c_hi[2] = {T - 1, T - 1};
-        if (p.causal) {
-          const int k_r = kt * 128 + row;
-#pragma unroll
-          for (int x = 0; x < 2; ++x) {
-            const int qx = x == 0 ? qa : qb;
-            const bool in_k = k_r <= qx && qx - k_r <= p.k2w;
-            c_lo[x] = max(qx - p.k1w, in_k ? k_r - p.kkl : 0);
-            c_hi[x] = in_k ? min(qx, k_r + p.kkr) : qx;
-          }
-        }
-        // ---- operand formation: A_a = s*Q[qa] (.) K2tile (in place), A_b = s*Q[qb] (.) K2tile
-        constexpr int kCols = D / 8, kRowStep = 256 / kCols;
-        const int col = st % kCols;
-        const uint32_t off0 = (col >> 3) * 16384 + swz128(st / kCols, col & 7);
-        float2 qv[2][4];   // this thread's columns of the two queries
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          const uint4 v = __ldg(reinterpret_cast<const uint4*>(Qg + (size_t)(x ? qb : qa) * D + col * 8));
-          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) qv[x][e] = unpack2<T16>(w[e]);
-        }
-        alive = __all_sync(0xffffffffu, mbar_wait(&bars.k2_full, kt_count & 1, abort_flag));
-        if (!alive) break;
-        // A thread has one 16-byte column of every (256 / kCols)-th row.  (The backward forms the same products in the same
-        // order for large scores, where a rounding the other way would show.)
-        {
-#pragma unroll 2
-          for (int i = 0; i < 128 / kRowStep; ++i) {
-            const uint32_t off = off0 + i * kRowStep * 128;
-            const uint4 kv = *reinterpret_cast<const uint4*>(smem + Cfg::kOffAa + off);
-            const uint32_t w[4] = {kv.x, kv.y, kv.z, kv.w};
-            uint32_t a[2][4];
-            float nr[2] = {0.f, 0.f};   // this thread's share of |A_a[r]|^2 and |A_b[r]|^2
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 f = __fmul2_rn(unpack2<T16>(w[e]), make_float2(p.scale2, p.scale2));
-#pragma unroll
-              for (int x = 0; x < 2; ++x) {
-                const float2 g = __fmul2_rn(f, qv[x][e]);
-                a[x][e] = pack2<T16>(g.x, g.y);
-                if (!split) nr[x] = fmaf(g.x, g.x, fmaf(g.y, g.y, nr[x]));
-              }
-            }
-            *reinterpret_cast<uint4*>(smem + Cfg::kOffAa + off) = make_uint4(a[0][0], a[0][1], a[0][2], a[0][3]);
-            *reinterpret_cast<uint4*>(smem + Cfg::kOffAb + off) = make_uint4(a[1][0], a[1][1], a[1][2], a[1][3]);
-            if (!split) {
-              // (read by the owner of the row after its first s_ready wait of this k-tile, which this thread's
-              //  a_ready arrival below precedes; rewritten only after it has passed a_free)
-#pragma unroll
-              for (int x = 0; x < 2; ++x) {
-#pragma unroll
-                for (int o = kCols / 2; o >= 1; o >>= 1) nr[x] += __shfl_xor_sync(0xffffffffu, nr[x], o);
-                if (col == 0) norms[x * 128 + st / kCols + i * kRowStep] = nr[x];
-              }
-            }
-          }
-        }
-        fence_async_smem();   // generic-proxy stores above -> visible to the tensor core's reads
-        mbar_arrive(&bars.a_ready);
-
-        if (split) {
-          // ---- walk over the slabs, both warpgroups on the same slab: tile a, then tile b; warpgroup `wg` takes the
-          // slab's columns [wg * 64, wg * 64 + 64) (32 of a half-width slab's 64).  The reference of every row is the head's: with a
-          // bound b of the scores P stays within [2^-(2 b + 1.15), 1], representable in the 16-bit type, and no row maximum is needed.
-          // (T=2048 D=128 bf16 16 heads 22.7 ms, with a launch parameter in its place 22.4; T=333 93 against 92 us.)
-          float l_sum[2] = {0.f, 0.f};
-          for (int jt = 0; jt < njt && alive; ++jt, ++n) {
-            // A slab with attended columns in one 64-column half only was computed for that half alone: its scores
-            // are in the first 64 columns of S_x and stand for the slab's columns [coff, coff + 64).
-            const int hm = halves(ja, jb, (jt0 + jt) * kBJ);
-            const int nh = hm ? 1 : 2, coff = hm == 2 ? 64 : 0;
-            const int cw = 32 * nh;                                  // columns of this warpgroup in this slab
-            const int j0 = (jt0 + jt) * kBJ + coff + wg * cw;      // its first column
+      // The item's k-tiles, one copy of the code for each organisation: with one copy for both, neither had the registers and the
+      // schedule of its own (T=512 D=64 32 heads 928 us against 900, T=557 fp16 not causal with large scores 3.70 ms against 3.60).
+      auto walk = [&](auto split_c) {
+        constexpr bool kSplit = decltype(split_c)::value;
+        // (every lane has the same value; the reduction leaves it in a uniform register)
+        const float reference = kSplit ? __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(head_reference(bh)))) : 0.f;
+        for (int kt = kt0; kt < kt0 + nkt && alive; ++kt, ++kt_count) {
+          int jt0, njt, ja, jb;
+          j_range(qa, qb, kt, jt0, njt);
+          col_span(qa, qb, kt, ja, jb);
+          // Columns this row may see, per tile: [c_lo, c_hi].  A row outside the k range of its query (its weight in
+          // the fold is zero) keeps the query's own column range so that it never sees an empty one by construction;
+          // a row inside can still see none in a slab, or at all: its maximum then stays -inf and its P zero.
+          int c_lo[2] = {0, 0}, c_hi[2] = {T - 1, T - 1};
+          if (p.causal) {
+            const int k_r = kt * 128 + row;
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
-              alive = __all_sync(0xffffffffu, mbar_wait(&bars.s_ready[x], n & 1, abort_flag));
-              if (!alive) break;
-              tc_fence_after();
-              // the last score product of this k-tile has read A_a and A_b
-              if (x == 1 && jt == njt - 1) mbar_arrive(&bars.a_free);
-              const uint32_t tS = tmem + lane_base + x * kBJ + wg * cw;
-              // this row's valid columns among the warpgroup's: [lo, hi]; the warp takes the unmasked code when all
-              // its rows see all of them
-              const int lo = c_lo[x] - j0, hi = c_hi[x] - j0;
-              const bool full = __all_sync(0xffffffffu, lo <= 0 && hi >= cw - 1);
-              // P over the first half of the columns this thread has read
-              l_sum[x] += nh == 2 ? form_p(std::integral_constant<int, 64>{}, tS, tS, full, lo, hi, reference)
-                                  : form_p(std::integral_constant<int, 32>{}, tS, tS, full, lo, hi, reference);
-              tmem_wait_st();
-              tc_fence_before();
-              mbar_arrive(&bars.p_ready[x]);
+              const int qx = x == 0 ? qa : qb;
+              const bool in_k = k_r <= qx && qx - k_r <= p.k2w;
+              c_lo[x] = max(qx - p.k1w, in_k ? k_r - p.kkl : 0);
+              c_hi[x] = in_k ? min(qx, k_r + p.kkr) : qx;
             }
           }
-          if (!alive) break;
-          // ---- hand this k-tile's row sums to the fold warpgroup
+          // ---- operand formation: A_a = s*Q[qa] (.) K2tile (in place), A_b = s*Q[qb] (.) K2tile
+          constexpr int kCols = D / 8, kRowStep = 256 / kCols;
+          const int col = st % kCols;
+          const uint32_t off0 = (col >> 3) * 16384 + swz128(st / kCols, col & 7);
+          float2 qv[2][4];   // this thread's columns of the two queries
 #pragma unroll
           for (int x = 0; x < 2; ++x) {
-            stats[(((kt_count & 1) * 2 + x) * 128 + row) * 4 + 1 + wg] = l_sum[x];
-            mbar_arrive(&bars.stats_ready[kt_count & 1][x]);
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(Qg + (size_t)(x ? qb : qa) * D + col * 8));
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) qv[x][e] = unpack2<T16>(w[e]);
           }
-        } else {
-          // ---- walk over the slabs, one warpgroup per tile (warpgroup 0: tile a), one whole row per thread: row
-          // maximum, exp2 with lazy rescaling of the accumulator.  A warp whose rows all have a score bound below the
-          // limit still uses the bound as reference and skips the maximum pass.  (Arrivals count twice: the barriers
-          // expect both warpgroups.)
-          const int x = wg;
-          const int c_lo_x = x ? c_lo[1] : c_lo[0], c_hi_x = x ? c_hi[1] : c_hi[0];
-          const uint32_t tS = tmem + lane_base + x * kBJ;
-          float m_used = -INFINITY, l_sum = 0.f;
-          bool fast = false;
-          for (int jt = 0; jt < njt && alive; ++jt, ++n) {
-            alive = __all_sync(0xffffffffu, mbar_wait(&bars.s_ready[x], n & 1, abort_flag));
-            if (!alive) break;
-            tc_fence_after();
-            if (jt == 0) {
-              const float bound = sqrtf(norms[x * 128 + row]) * k1_max;
-              fast = __all_sync(0xffffffffu, bound <= p.bound_limit);
-              if (fast) m_used = bound;
-            }
-            if (jt == njt - 1) mbar_arrive(&bars.a_free);  // the last score product of this k-tile has read A_x
-            const int hm = halves(ja, jb, (jt0 + jt) * kBJ);
-            const int nh = hm ? 1 : 2, coff = hm == 2 ? 64 : 0;
-            const int j0 = (jt0 + jt) * kBJ + coff;
-            const int lo = c_lo_x - j0, hi = c_hi_x - j0;
-            const bool full = __all_sync(0xffffffffu, lo <= 0 && hi >= 64 * nh - 1);
-            using N64 = std::integral_constant<int, 64>;
-            if (!fast) {
-              // pass 1: row maximum
-              float mx = row_max(N64{}, tS, full, lo, hi);
-              if (nh == 2) mx = fmaxf(mx, row_max(N64{}, tS + 64, full, lo - 64, hi - 64));
-              if (jt == 0) {
-                m_used = mx;  // nothing accumulated yet in this k-tile
-              } else {
-                const bool grow = mx > m_used + kRescaleGap;
-                if (__any_sync(0xffffffffu, grow)) {
-                  // some row of this warp moved its max up noticeably: rescale accumulator rows (factor 1 for the
-                  // rows that did not move)
-                  const float corr = grow ? exp2f(m_used - mx) : 1.f;
-                  if (grow) {
-                    m_used = mx;
-                    l_sum *= corr;
-                  }
-                  // (s_ready of this slab was committed after the previous P*V, so that product has landed)
-                  const uint32_t tO = tmem + lane_base + Cfg::kTmemO + x * D;
+          alive = __all_sync(0xffffffffu, mbar_wait(&bars.k2_full, kt_count & 1, abort_flag));
+          if (!alive) break;
+          // A thread has one 16-byte column of every (256 / kCols)-th row.  (The backward forms the same products in the same
+          // order for large scores, where a rounding the other way would show.)
+          {
+#pragma unroll 2
+            for (int i = 0; i < 128 / kRowStep; ++i) {
+              const uint32_t off = off0 + i * kRowStep * 128;
+              const uint4 kv = *reinterpret_cast<const uint4*>(smem + Cfg::kOffAa + off);
+              const uint32_t w[4] = {kv.x, kv.y, kv.z, kv.w};
+              uint32_t a[2][4];
+              float nr[2] = {0.f, 0.f};   // this thread's share of |A_a[r]|^2 and |A_b[r]|^2
 #pragma unroll
-                  for (int ch = 0; ch < D / 32; ++ch) {
-                    uint32_t o[32];
-                    tmem_ld32(tO + ch * 32, o);
-                    tmem_wait_ld();
+              for (int e = 0; e < 4; ++e) {
+                const float2 f = __fmul2_rn(unpack2<T16>(w[e]), make_float2(p.scale2, p.scale2));
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
-                    tmem_st32(tO + ch * 32, o);
-                  }
+                for (int x = 0; x < 2; ++x) {
+                  const float2 g = __fmul2_rn(f, qv[x][e]);
+                  a[x][e] = pack2<T16>(g.x, g.y);
+                  if constexpr (!kSplit) nr[x] = fmaf(g.x, g.x, fmaf(g.y, g.y, nr[x]));
+                }
+              }
+              *reinterpret_cast<uint4*>(smem + Cfg::kOffAa + off) = make_uint4(a[0][0], a[0][1], a[0][2], a[0][3]);
+              *reinterpret_cast<uint4*>(smem + Cfg::kOffAb + off) = make_uint4(a[1][0], a[1][1], a[1][2], a[1][3]);
+              if constexpr (!kSplit) {
+                // (read by the owner of the row after its first s_ready wait of this k-tile, which this thread's
+                //  a_ready arrival below precedes; rewritten only after it has passed a_free)
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+#pragma unroll
+                  for (int o = kCols / 2; o >= 1; o >>= 1) nr[x] += __shfl_xor_sync(0xffffffffu, nr[x], o);
+                  if (col == 0) norms[x * 128 + st / kCols + i * kRowStep] = nr[x];
                 }
               }
             }
-            // pass 2: P = exp2(S - m), packed to 16 bits over the columns already consumed
-            l_sum += form_p(N64{}, tS, tS, full, lo, hi, m_used);
-            if (nh == 2) l_sum += form_p(N64{}, tS + 64, tS + 32, full, lo - 64, hi - 64, m_used);
-            tmem_wait_st();
-            tc_fence_before();
-            mbar_arrive_n(&bars.p_ready[x], 2);
           }
-          if (!alive) break;
-          // ---- hand this k-tile's row statistics to the fold warpgroup
-          float* srow = stats + (((kt_count & 1) * 2 + x) * 128 + row) * 4;
-          srow[0] = m_used;
-          srow[1] = l_sum;
-          srow[2] = 0.f;
-          mbar_arrive_n(&bars.stats_ready[kt_count & 1][x], 2);
+          fence_async_smem();   // generic-proxy stores above -> visible to the tensor core's reads
+          mbar_arrive(&bars.a_ready);
+
+          if constexpr (kSplit) {
+            // ---- walk over the slabs, both warpgroups on the same slab: tile a, then tile b; warpgroup `wg` takes the
+            // slab's columns [wg * 64, wg * 64 + 64) (32 of a half-width slab's 64).  The reference of every row is the head's: with
+            // a bound b of the scores P stays within [2^-(2 b + 1.15), 1], representable in the 16-bit type, and no row maximum is
+            // needed.
+            // (The head's own bound instead of a launch parameter costs 1 to 2 % at head dimension 128, T=2048 16
+            // heads 22.4 -> 22.7 ms, and nothing at 64.)
+            float l_sum[2] = {0.f, 0.f};
+            for (int jt = 0; jt < njt && alive; ++jt, ++n) {
+              // A slab with attended columns in one 64-column half only was computed for that half alone: its scores
+              // are in the first 64 columns of S_x and stand for the slab's columns [coff, coff + 64).
+              const int hm = halves(ja, jb, (jt0 + jt) * kBJ);
+              const int nh = hm ? 1 : 2, coff = hm == 2 ? 64 : 0;
+              const int cw = 32 * nh;                                  // columns of this warpgroup in this slab
+              const int j0 = (jt0 + jt) * kBJ + coff + wg * cw;      // its first column
+#pragma unroll
+              for (int x = 0; x < 2; ++x) {
+                alive = __all_sync(0xffffffffu, mbar_wait(&bars.s_ready[x], n & 1, abort_flag));
+                if (!alive) break;
+                tc_fence_after();
+                // the last score product of this k-tile has read A_a and A_b
+                if (x == 1 && jt == njt - 1) mbar_arrive(&bars.a_free);
+                const uint32_t tS = tmem + lane_base + x * kBJ + wg * cw;
+                // this row's valid columns among the warpgroup's: [lo, hi]; the warp takes the unmasked code when all
+                // its rows see all of them
+                const int lo = c_lo[x] - j0, hi = c_hi[x] - j0;
+                const bool full = __all_sync(0xffffffffu, lo <= 0 && hi >= cw - 1);
+                // P over the first half of the columns this thread has read
+                l_sum[x] += nh == 2 ? form_p(std::integral_constant<int, 64>{}, tS, tS, full, lo, hi, reference)
+                                    : form_p(std::integral_constant<int, 32>{}, tS, tS, full, lo, hi, reference);
+                tmem_wait_st();
+                tc_fence_before();
+                mbar_arrive(&bars.p_ready[x]);
+              }
+            }
+            if (!alive) break;
+            // ---- hand this k-tile's row sums to the fold warpgroup
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+              stats[(((kt_count & 1) * 2 + x) * 128 + row) * 4 + 1 + wg] = l_sum[x];
+              mbar_arrive(&bars.stats_ready[kt_count & 1][x]);
+            }
+          } else {
+            // ---- walk over the slabs, one warpgroup per tile (warpgroup 0: tile a), one whole row per thread: row
+            // maximum, exp2 with lazy rescaling of the accumulator.  A warp whose rows all have a score bound below the
+            // limit still uses the bound as reference and skips the maximum pass.  (Arrivals count twice: the barriers
+            // expect both warpgroups.)
+            const int x = wg;
+            const int c_lo_x = x ? c_lo[1] : c_lo[0], c_hi_x = x ? c_hi[1] : c_hi[0];
+            const uint32_t tS = tmem + lane_base + x * kBJ;
+            float m_used = -INFINITY, l_sum = 0.f;
+            bool fast = false;
+            for (int jt = 0; jt < njt && alive; ++jt, ++n) {
+              alive = __all_sync(0xffffffffu, mbar_wait(&bars.s_ready[x], n & 1, abort_flag));
+              if (!alive) break;
+              tc_fence_after();
+              if (jt == 0) {
+                const float bound = sqrtf(norms[x * 128 + row]) * k1_max;
+                fast = __all_sync(0xffffffffu, bound <= p.bound_limit);
+                if (fast) m_used = bound;
+              }
+              if (jt == njt - 1) mbar_arrive(&bars.a_free);  // the last score product of this k-tile has read A_x
+              const int hm = halves(ja, jb, (jt0 + jt) * kBJ);
+              const int nh = hm ? 1 : 2, coff = hm == 2 ? 64 : 0;
+              const int j0 = (jt0 + jt) * kBJ + coff;
+              const int lo = c_lo_x - j0, hi = c_hi_x - j0;
+              const bool full = __all_sync(0xffffffffu, lo <= 0 && hi >= 64 * nh - 1);
+              using N64 = std::integral_constant<int, 64>;
+              if (!fast) {
+                // pass 1: row maximum
+                float mx = row_max(N64{}, tS, full, lo, hi);
+                if (nh == 2) mx = fmaxf(mx, row_max(N64{}, tS + 64, full, lo - 64, hi - 64));
+                if (jt == 0) {
+                  m_used = mx;  // nothing accumulated yet in this k-tile
+                } else {
+                  const bool grow = mx > m_used + kRescaleGap;
+                  if (__any_sync(0xffffffffu, grow)) {
+                    // some row of this warp moved its max up noticeably: rescale accumulator rows (factor 1 for the
+                    // rows that did not move)
+                    const float corr = grow ? exp2f(m_used - mx) : 1.f;
+                    if (grow) {
+                      m_used = mx;
+                      l_sum *= corr;
+                    }
+                    // (s_ready of this slab was committed after the previous P*V, so that product has landed)
+                    const uint32_t tO = tmem + lane_base + Cfg::kTmemO + x * D;
+#pragma unroll
+                    for (int ch = 0; ch < D / 32; ++ch) {
+                      uint32_t o[32];
+                      tmem_ld32(tO + ch * 32, o);
+                      tmem_wait_ld();
+#pragma unroll
+                      for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
+                      tmem_st32(tO + ch * 32, o);
+                    }
+                  }
+                }
+              }
+              // pass 2: P = exp2(S - m), packed to 16 bits over the columns already consumed
+              l_sum += form_p(N64{}, tS, tS, full, lo, hi, m_used);
+              if (nh == 2) l_sum += form_p(N64{}, tS + 64, tS + 32, full, lo - 64, hi - 64, m_used);
+              tmem_wait_st();
+              tc_fence_before();
+              mbar_arrive_n(&bars.p_ready[x], 2);
+            }
+            if (!alive) break;
+            // ---- hand this k-tile's row statistics to the fold warpgroup
+            float* srow = stats + (((kt_count & 1) * 2 + x) * 128 + row) * 4;
+            srow[0] = m_used;
+            srow[1] = l_sum;
+            srow[2] = 0.f;
+            mbar_arrive_n(&bars.stats_ready[kt_count & 1][x], 2);
+          }
         }
-      }
+      };
+      if (head_split(bh)) walk(std::true_type{});
+      else walk(std::false_type{});
       if (!alive) break;
     }
   } else if (warp >= 12) {
