@@ -515,7 +515,7 @@ def run_ours(args):
             # the 128-wide tiles on the diagonal of the causal mask (ratio for T=2048)
             "executed_over_algorithmic_flops": (5.0 / 6.0) * 1.095,
             # dram__bytes_read.sum of one backward launch: 50.8 MB captured at 16 heads, T=768 (profiles/), scaled by heads
-            # and length; 0.13 MB were written (the sums stay in L2)
+            # and length; 0.14 MB were written (the sums stay in L2)
             "traffic": 8.46e6 * per, "traffic_unit": "bytes read per launch (ncu at T=768, scaled by heads and length)",
         },
     }

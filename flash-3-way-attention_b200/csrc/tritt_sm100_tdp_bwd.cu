@@ -22,13 +22,14 @@
 // fp32 sums that stay in L2).  All steps of a call are laid out in one line and cut in equal parts, one per CTA
 // (every sum is a reduction, so an item may be cut anywhere): no last wave.
 //
-// What bounds it: the fold warps, which are busy all of a step (3200 cycles at head dimension 128, 3800 at 64): chains of
-// tensor-memory reads, shared-memory accesses and waits, each of 100 to 400 cycles while the tensor cores' operand reads keep
-// shared memory busy; at 64 the soft-max warps as well.  Issue slots are 56 to 61 % busy, the tensor pipe 35 to 47 %.
+// What bounds it: no unit, but the chains of tensor-memory reads, shared-memory accesses and waits of the soft-max and fold warps,
+// while the tensor cores' operand reads keep shared memory busy.  A step takes 2760 cycles at head dimension 128 and 3790 at 64;
+// 16 heads of T=768: issue slots 60 / 63 % busy, tensor pipe 49 / 37 %, shared memory 30 / 37 % by the warps and 47 / 38 % by the
+// tensor cores.
 // Operands formed by one 16-bit product per pair instead of fp32 products and conversions, the products issued by three warps
-// instead of one, A' doubled, exponentials beside the arithmetic of dS, looks at barriers ahead of the waits, and waits without
-// the clock, backward of T=2048 D=128 bf16 16 heads 71.2 -> 64.8 ms, T=4096 D=64 4 heads 80.4 -> 78.1, T=512 D=64 32 heads 1.80 ->
-// 1.70, not causal fp16 16 heads 1.83 -> 1.76, windows 128/128/32/32 at T=2048 1.22 -> 1.14, T=333 D=128 4 heads 189 -> 169 us.
+// instead of one, A' doubled, exponentials beside the arithmetic of dS, looks at barriers ahead of the waits, and waits that seldom
+// read the clock, backward of T=2048 D=128 bf16 16 heads 70.9 -> 64.1 ms, T=4096 D=64 4 heads 79.9 -> 78.1, T=512 D=64 32 heads 1.80 ->
+// 1.70, not causal fp16 16 heads 1.83 -> 1.78, windows 128/128/32/32 at T=2048 1.22 -> 1.14, T=333 D=128 4 heads 189 -> 169 us.
 // Against a query and 128 rows of one key tensor per tile (eight products, exponentials twice), same call, training
 // steps: T=2048 D=128 bf16 16 heads 114.5 -> 94.9 ms, T=4096 D=64 4 heads 140.5 -> 113.8 ms, T=512 D=64 fp16 16 heads 2.37
 // -> 1.59 ms, windows 128/128/32/32 at T=2048 4.54 -> 1.77 ms.
@@ -68,8 +69,8 @@ constexpr int kVecSlots = 4;     // batches in flight
 // the gradients were up to 2.4 times further from fp64 than with the forward's operand (scores of order 3, not causal, T=200:
 // dQ 2.0 to 2.4 times, dV2 1.5 to 2.3; of order 1, D=128, bf16: dQ 1.33).  CTAs with such heads form S = R K1^T, from
 // the rows that the forward formed: 0.5 to 1.06 times there, dV2 1.00.  R is 128 x D for any JT and is formed by two warps, so
-// this costs speed (B200, against S = Q A^T): T=512 D=64 16 heads 0.95 -> 0.99 ms, T=4096 D=64 4 heads 81.5 -> 86.7 ms,
-// T=2048 D=128 16 heads 73 -> 82 ms.  Hence the bound, on |Q row| |K1 row| max|K2| in log2 units: Gaussian inputs with
+// this costs speed (B200, against S = Q A^T, the same inputs): T=512 D=64 16 heads 0.87 -> 0.91 ms, T=4096 D=64 4 heads 78.3 -> 81.8,
+// T=2048 D=128 16 heads 64.1 -> 74.9, T=1024 9.3 -> 11.1.  Hence the bound, on |Q row| |K1 row| max|K2| in log2 units: Gaussian inputs with
 // a bound of 21 to 82 (their scores are 1/60 to 1/80 of it) show no excess with A (dQ 0.85 to 1.0), aligned inputs come
 // closer to their bound.
 constexpr float kScoreBound = 16.f;
@@ -685,7 +686,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
   } else if (warp < 16) {
     set_regs<kRegsLaunch, BwdRegs<D, LARGE>::kFold>();
     // ------------------------------------------------------------------ operand / fold warpgroups
-    // role 0: forms A two steps ahead, folds G into dK1 (registers) and dK2;  role 1: forms A' one step ahead, folds
+    // role 0: forms A two steps ahead, folds G into dK1 (registers) and dK2;  role 1: forms A' two steps ahead (large scores: one), folds
     // U into dSiLU(V1) and dV2.  The fold reads the accumulator as 16 x 256-bit fragments (thread t: rows t / 4 + 8 i,
     // columns 8 g + 2 (t % 4) and the next), which is also how ldmatrix hands out the K1 / SiLU(V1) tile: the sums
     // over the 32 rows of a warp are four rows within a thread and a 7-shuffle tree per 32 columns.
@@ -1408,9 +1409,9 @@ struct BwdPlan {
 // A tile's 128 rows of a shard lie q_mod apart, and each of its steps is executed for all of them: at 8 shards the rows of
 // a tile span 1024 queries, and one shard of T=1024 executes 0.31 of the whole call's cells instead of 0.125, of T=2048
 // 0.21, of T=4096 0.17, of windows 128/128/32/32 0.63.  The kernel that steps over queries executes just a shard's share, at
-// a higher price per cell: stepping over k costs 0.76 (D=64) to 0.78 of it per cell (0.82 to 0.9 for large scores).
-// ms per call of one of 8 shards, k / queries: T=1024 D=64 16 heads 3.22 / 1.12, T=2048 D=128 16 heads 19.9 / 11.4, T=4096
-// D=64 4 heads 14.7 / 13.4, those windows 0.77 / 0.51; of one of 2: 3.65 / 4.35, 38.7 / 44.8, 41.8 / 52.6, 0.95 / 1.96.
+// a higher price per cell: stepping over k costs 0.66 to 0.77 of it per cell (D=128 0.71; more for large scores).
+// ms per call of one of 8 shards, k / queries: T=1024 D=64 16 heads 1.85 / 1.12, T=2048 D=128 16 heads 13.1 / 11.0, T=4096
+// D=64 4 heads 13.7 / 13.3, those windows 0.79 / 0.55; of one of 2: 3.38 / 4.34, 35.2 / 45.4, 41.3 / 52.9, 0.97 / 2.09.
 constexpr double kCellPrice = 0.8;
 
 template <int D> BwdPlan make_plan(const TdpArgs& a) {

@@ -27,7 +27,7 @@
 //   warps 12-15  fold warpgroup: when a k-tile is finished, folds acc_x (times V2, soft-max over k) into
 //                the queries' running (max, sum, output) while the other warps start the next k-tile; with one reference for
 //                a head the sums just add up in registers, without exchanges between threads
-// What bounds it: the exponentials (65 % of the special-function unit's time at head dimension 64, 57 % at 128, where the products
+// What bounds it: the exponentials (66 % of the special-function unit's time at head dimension 64, 58 % at 128, where the products
 // take as long), the rest of the soft-max stage of a slab around them and the change of k-tiles.  A time trace of the form before had
 // 1300 cycles a stage against 1024 of exponentials, and 3300 to 4100 a change, 2000 of them the operands.  Operands with a thread on
 // one column of every 16th or 32nd row, norms only where a row's bound is asked for, and the fold without exchanges: T=512 D=64 bf16

@@ -38,7 +38,7 @@ def _fwd_case(B, N, T, D, dtype, causal, scale_in, alpha, seed, o_scale=1.0):
 @pytest.mark.parametrize("windows", [(None, None, None, None), (100, 70, 40, 30)])
 def test_forward_heads_with_small_and_large_logits_in_one_launch(D, dtype, windows):
     """The forward picks the soft-max warps' organisation per head from a head-wide score bound (column split with
-    the row's bound as reference / one warpgroup per tile with row maxima).  Heads of both kinds alternate here, so
+    the head's bound as reference / one warpgroup per tile with row maxima).  Heads of both kinds alternate here, so
     every CTA changes organisation between consecutive work items and the same barriers serve both."""
     B, N, T, alpha = 1, 6, 300, 1 / 8
     q, k1, k2, v1, v2, _ = orc.make_inputs(B, N, T, D, scale=1.0, seed=41 + D, dtype=torch.float32)
@@ -364,8 +364,8 @@ def test_forward_of_many_one_slab_items(D, scale):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_forward_with_and_without_the_score_bound(dtype):
-    """The forward takes the score bound |A_row| max|K1_j| as soft-max reference when the workspace has the tail for
-    the K1 row norms, and the two-pass row maximum when it has not: same result up to the rounding of P."""
+    """The forward takes the head's score bound (or a row's, |A_row| max|K1_j|) as soft-max reference when the workspace has
+    the tail for the statistics, and the two-pass row maximum when it has not: same result up to the rounding of P."""
     B, N, T, D, alpha = 1, 2, 384, 128, 1.0 / 128
     q, k1, k2, v1, v2, _ = orc.make_inputs(B, N, T, D, scale=0.5, seed=77, dtype=dtype)
     t = [x.to(DEV) for x in (q, k1, k2, v1, v2)]
