@@ -101,25 +101,43 @@ template <int D> struct BwdCfg {
 // The steps (q-tile, j-tile, k) of a call in the order they are cut: heads, q-tiles, j-tiles, k.  Causal mask
 // j <= q <= j + k1w,  k <= q <= k + k2w,  k - kkl <= j <= k + kkr:  a q-tile [qa, qb] meets the j-tiles of rows
 // [qa - k1w, qb], and a pair of tiles the k in [max(qa - k2w, ja - kkr), min(qb, jb + kkl)].
+// The j-tiles lie side by side (stride = JT, lead = 0), or, for a narrow band, overlap: tile jt belongs to the k in
+// [jt stride, jt stride + stride) and has all the rows j that these see, stride + kkl + kkr = JT of them (lead = kkl).  Then a k
+// meets one j-tile per q-tile, instead of (JT + kkl + kkr) / JT on average.
 struct BwdGeometry {
   int T, nq, q_mod, q_rem, causal;
   int k1w, k2w, kkl, kkr;  // windows of the causal mask (T or more = unbounded)
   int JT;                  // rows of a j-tile
+  int stride, lead;        // tile jt has the rows from jt * stride - lead on
   __host__ __device__ int q_tiles() const { return (nq + 127) / 128; }
   __host__ __device__ int first_q(int qt) const { return q_rem + qt * 128 * q_mod; }
   __host__ __device__ int last_q(int qt) const {
     const int i = qt * 128 + 127;
     return q_rem + (i < nq ? i : nq - 1) * q_mod;
   }
+  __host__ __device__ bool overlapping() const { return stride != JT; }
+  __host__ __device__ int j_row(int jt) const { return jt * stride - lead; }
+  __host__ __device__ int k_first(int qa) const {   // of the k that a query from qa on sees
+    const int reach = k2w < k1w + kkr ? k2w : k1w + kkr;
+    return qa > reach ? qa - reach : 0;
+  }
   __host__ __device__ int j_first(int qt) const {
+    if (overlapping()) return k_first(first_q(qt)) / stride;
     const int lo = first_q(qt) - k1w;
     return causal && lo > 0 ? lo / JT : 0;
   }
-  __host__ __device__ int j_last(int qt) const { return (causal ? last_q(qt) : T - 1) / JT; }
+  __host__ __device__ int j_last(int qt) const { return (causal ? last_q(qt) : T - 1) / stride; }
   __host__ __device__ int k_range(int qt, int jt, int& k0) const {   // number of steps of a pair of tiles
     k0 = 0;
     if (!causal) return T;
-    const int qa = first_q(qt), qb = last_q(qt), ja = jt * JT, jb = ja + JT - 1;
+    const int qa = first_q(qt), qb = last_q(qt);
+    if (overlapping()) {
+      const int a = k_first(qa), b = jt * stride;
+      k0 = a > b ? a : b;
+      const int k1 = qb < b + stride - 1 ? qb : b + stride - 1;
+      return k1 >= k0 ? k1 - k0 + 1 : 0;
+    }
+    const int ja = jt * JT, jb = ja + JT - 1;
     if (qa - k2w > k0) k0 = qa - k2w;
     if (ja - kkr > k0) k0 = ja - kkr;
     const int k1 = qb < jb + kkl ? qb : jb + kkl;
@@ -485,13 +503,13 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
         const float2 v = make_float2(__uint_as_float(v0), __uint_as_float(v1));
         return kScaled ? __ffma2_rn(v, make_float2(scale, scale), add) : __fadd2_rn(v, add);
       };
-      const int j0 = it.jt * JT + wg * CW;
+      const int j0 = g.j_row(it.jt) + wg * CW;
       for (int i = 0; i < it.len; ++i, ++n) {
         const int k = it.k0 + i;
         // columns this query sees at this k, relative to the thread's first: [lo, hi] (empty: hi < lo)
         int lo = -j0, hi = T - 1 - j0;
         if (g.causal) {
-          lo = max(q - g.k1w, k - g.kkl) - j0;
+          lo = max(max(q - g.k1w, k - g.kkl), 0) - j0;   // (an overlapping tile may begin ahead of row 0)
           hi = k <= q && q - k <= g.k2w ? min(q, k + g.kkr) - j0 : lo - 1;
         }
         if (!q_ok) hi = lo - 1;
@@ -931,12 +949,12 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
               const float2 a = acc[c16 * 8 + hl * 4 + g * 2 + r];
               const int lr = w * 32 + hl * 16 + r * 8 + (lane >> 2), lc = c16 * 16 + g * 8 + 2 * (lane & 3);
               if constexpr (D == 64) {
-                const int j = it.jt * JT + lr;
-                if (j < T) red_add2(base + (size_t)j * D + lc, a.x * jscale, a.y * jscale);
+                const int j = p.g.j_row(it.jt) + lr;
+                if (j >= 0 && j < T) red_add2(base + (size_t)j * D + lc, a.x * jscale, a.y * jscale);
               } else {
-                const int j = it.jt * JT + lc;
-                if (j < T) red_add(base + (size_t)j * D + lr, a.x * jscale);
-                if (j + 1 < T) red_add(base + (size_t)(j + 1) * D + lr, a.y * jscale);
+                const int j = p.g.j_row(it.jt) + lc;
+                if (j >= 0 && j < T) red_add(base + (size_t)j * D + lr, a.x * jscale);
+                if (j + 1 >= 0 && j + 1 < T) red_add(base + (size_t)(j + 1) * D + lr, a.y * jscale);
               }
             }
     }
@@ -1114,8 +1132,8 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
             tma_load_3d(smem + Cfg::kOffQ + b * 16384, &tmQ, &bars.tile_full, b * 64, it.qt * 128, it.bh);
             tma_load_3d(smem + Cfg::kOffDO + b * 16384, &tmDO, &bars.tile_full, b * 64, it.qt * 128, it.bh);
           }
-          tma_load_3d(smem + Cfg::kOffK1 + b * JT * 128, &tmK1, &bars.tile_full, b * 64, it.jt * JT, it.bh);
-          tma_load_3d(smem + Cfg::kOffK1 + Cfg::kTileJ + b * JT * 128, &tmSV1, &bars.tile_full, b * 64, it.jt * JT, it.bh);
+          tma_load_3d(smem + Cfg::kOffK1 + b * JT * 128, &tmK1, &bars.tile_full, b * 64, g.j_row(it.jt), it.bh);
+          tma_load_3d(smem + Cfg::kOffK1 + Cfg::kTileJ + b * JT * 128, &tmSV1, &bars.tile_full, b * 64, g.j_row(it.jt), it.bh);
         }
       }
       in_flight = true;
@@ -1418,10 +1436,32 @@ struct BwdPlan {
 // D=64 4 heads 13.7 / 13.3, those windows 0.79 / 0.55; of one of 2: 3.38 / 4.34, 35.2 / 45.4, 41.3 / 52.9, 0.97 / 2.09.
 constexpr double kCellPrice = 0.8;
 
+// What an item costs beside its steps (its tiles' way in, dK1's and dSiLU(V1)'s out), in steps; and the narrowest stride taken.
+// us per backward with tiles side by side / overlapping: 16 heads T=2048 D=64 fp16 windows 128/128/32/32 (stride 64) 1141 / 955,
+// 256/256/40/20 (68) 1719 / 1379, 8/8/4/4 (120) 560 / 534; 8 heads T=2000 200/100/48/48 (32) 631 / 482; D=128 16 heads T=2048
+// 128/128/16/16 (32 of 64) 1004 / 802.
+constexpr long kItemSteps = 3;
+constexpr int kMinStride = 8;
+
+// Steps and items of one head.
+long count_steps(const BwdGeometry& g, long& items) {
+  long steps = 0;
+  items = 0;
+  for (int qt = 0; qt < g.q_tiles(); ++qt)
+    for (int jt = g.j_first(qt); jt <= g.j_last(qt); ++jt) {
+      int k0;
+      const int n = g.k_range(qt, jt, k0);
+      steps += n;
+      items += n > 0;
+    }
+  return steps;
+}
+
 template <int D> BwdPlan make_plan(const TdpArgs& a) {
   BwdPlan p{};
   const int nq = a.q_rem < a.T ? (a.T - a.q_rem + a.q_mod - 1) / a.q_mod : 0;
-  p.g = BwdGeometry{a.T, nq, a.q_mod, a.q_rem, a.mask.causal, a.mask.k1w, a.mask.k2w, a.mask.kkl, a.mask.kkr, BwdCfg<D>::JT};
+  constexpr int JT = BwdCfg<D>::JT;
+  p.g = BwdGeometry{a.T, nq, a.q_mod, a.q_rem, a.mask.causal, a.mask.k1w, a.mask.k2w, a.mask.kkl, a.mask.kkr, JT, JT, 0};
   if (nq == 0) return p;
   const int first = tdp_bwd_first_count(a.T);
   const long long pairs = (min(a.mask.k1w, a.T - 1) + 1LL) * (min(a.mask.k2w, a.T - 1) + 1LL);   // (at most, of any query)
@@ -1432,11 +1472,20 @@ template <int D> BwdPlan make_plan(const TdpArgs& a) {
       return p;
     }
   }
-  for (int qt = 0; qt < p.g.q_tiles(); ++qt)
-    for (int jt = p.g.j_first(qt); jt <= p.g.j_last(qt); ++jt) {
-      int k0;
-      p.head_steps += p.g.k_range(qt, jt, k0);
+  long items;
+  p.head_steps = count_steps(p.g, items);
+  const int stride = JT - a.mask.kkl - a.mask.kkr;
+  if (a.mask.causal && stride >= kMinStride) {
+    BwdGeometry o = p.g;
+    o.stride = stride;
+    o.lead = a.mask.kkl;
+    long o_items;
+    const long o_steps = count_steps(o, o_items);
+    if (o_steps + kItemSteps * o_items < p.head_steps + kItemSteps * items) {
+      p.g = o;
+      p.head_steps = o_steps;
     }
+  }
   p.cells = (long long)p.head_steps * 128 * BwdCfg<D>::JT;
   if (a.q_mod > 1) {
     const long long cells = sm100_tdp_bwd_queries_cells(a.T, a.mask, a.q_mod, a.q_rem);

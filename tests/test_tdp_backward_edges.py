@@ -239,3 +239,40 @@ def test_rows_of_a_short_last_batch(T, D, dtype):
     ref = orc.tdp_backward(*[x.float() for x in t], 1.0 / D, True)
     for name, a, b in zip(NAMES, got, ref):
         assert_close(name, a, b, dtype)
+
+
+# j-tiles of 128 (head dimension 64) or 64 rows that overlap: the widest stride (no band at all), strides that leave a short last
+# tile, a band to one side, the narrowest stride taken and the first one that is not, windows narrower than the band and than a tile.
+BANDS = [(64, (70, 70, 0, 0)), (64, (200, 150, 32, 32)), (64, (40, 300, 1, 100)), (64, (300, 30, 90, 30)), (64, (120, 90, 60, 61)),
+         (64, (3, 9, 2, 5)), (128, (70, 70, 0, 0)), (128, (150, 130, 16, 16)), (128, (40, 300, 0, 40)), (128, (90, 300, 28, 28))]
+
+
+def _cells_side_by_side(T, D, windows):
+    """Cells of the tiles that do not overlap."""
+    k1w, k2w, kkl, kkr = windows
+    JT, n = 128 if D == 64 else 64, 0
+    for qa in range(0, T, 128):
+        qb = min(qa + 127, T - 1)
+        for ja in range(max(0, qa - k1w) // JT * JT, qb + 1, JT):
+            n += max(0, min(qb, ja + JT - 1 + kkl) - max(0, qa - k2w, ja - kkr) + 1)
+    return n * 128 * JT
+
+
+def test_overlapping_tiles_are_taken_where_they_execute_less():
+    for D, windows in BANDS:
+        cells, stride = _native.tdp_bwd_plan(2000, D, _native.BF16, True, *windows)[1], (128 if D == 64 else 64) - sum(windows[2:])
+        side_by_side = _cells_side_by_side(2000, D, windows)
+        assert (cells < side_by_side) if sum(windows[2:]) and stride >= 8 else (cells == side_by_side), (D, windows)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,scale", [(torch.float16, 0.5), (torch.bfloat16, 1.0)])
+@pytest.mark.parametrize("T", [127, 258, 391])
+@pytest.mark.parametrize("D,windows", BANDS)
+def test_overlapping_tiles(D, windows, T, dtype, scale):
+    t = orc.make_inputs(1, 2, T, D, scale=scale, seed=T + D, dtype=dtype)
+    alpha = 1.0 / D if scale < 1 else 1 / 8
+    got = _backward([x.to(DEV) for x in t[:5]], t[5].to(DEV), alpha, True, windows)
+    ref = orc.tdp_backward(*[x.float() for x in t], alpha, True, *windows, device=DEV)
+    for name, a, b in zip(NAMES, got, ref):
+        assert_close(name, a, b, dtype)
