@@ -965,21 +965,22 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
 // zero anything and no atomics are needed.  8 elements per thread and step; a row is held by D / 8 neighbouring lanes.
 // Bound by launch latency on short sequences (it replaces two kernels and a memset: 47.3 -> 43.9 us per call at B=1 N=8
 // T=64 D=64) and by memory on long ones, where it is < 0.1 % of the call.  Eight blocks per head (the portable cluster
-// size) as soon as each has a pass of work.
-constexpr int kPrepThreads = 256;
+// size) as soon as each has a pass of work, and blocks of 1024 threads for heads of more than two passes of those: 16 heads of T=2048
+// D=64 16 -> 11 us, windows 256/256/40/20 at T=2048 793 -> 785 us a call.
+constexpr int kPrepThreads = 256, kPrepMost = 1024;
 template <typename T16>
-__global__ void __launch_bounds__(kPrepThreads)
+__global__ void __launch_bounds__(kPrepMost)
 fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const T16* __restrict__ q,
                    const T16* __restrict__ k2, T16* __restrict__ sv1, float* __restrict__ stats, int head_elems, int D,
                    int BN, int blocks) {
   __shared__ float red[8][3];           // [block of the cluster]; used in the first block
-  __shared__ float wred[kPrepThreads / 32][3];
+  __shared__ float wred[kPrepMost / 32][3];
   const int bh = blockIdx.x / blocks, part = blockIdx.x % blocks;
   const size_t base = (size_t)bh * head_elems;
   const int lanes = D / 8;
   float m1 = 0.f, mq = 0.f, m2 = 0.f;
   // (the bound is the same for all lanes of a row: head_elems is a multiple of D)
-  for (int i = (part * kPrepThreads + threadIdx.x) * 8; i < head_elems; i += blocks * kPrepThreads * 8) {
+  for (int i = (part * blockDim.x + threadIdx.x) * 8; i < head_elems; i += blocks * blockDim.x * 8) {
     const uint4 v = *reinterpret_cast<const uint4*>(v1 + base + i);
     const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
     uint32_t o[4];
@@ -1026,8 +1027,7 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
   cluster_sync_all();   // every block of the cluster runs: its shared memory may be written (a block barrier as well)
   if (threadIdx.x < 3) {
     float m = 0.f;
-#pragma unroll
-    for (int w = 0; w < kPrepThreads / 32; ++w) m = fmaxf(m, wred[w][threadIdx.x]);
+    for (int w = 0; w < blockDim.x / 32; ++w) m = fmaxf(m, wred[w][threadIdx.x]);
     uint32_t dst;   // the first block's red[part][.]
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(&red[part][threadIdx.x])), "r"(0));
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(m) : "memory");
@@ -1052,6 +1052,7 @@ int prepare_fwd(const TdpArgs& a, T16** sv1_out, float** k1n_out) {
   const int head_elems = a.T * a.D;
   int blocks = 1;
   while (blocks < 8 && blocks * kPrepThreads * 8 < head_elems) blocks *= 2;
+  const int threads = blocks * kPrepThreads * 8 * 2 < head_elems ? kPrepMost : kPrepThreads;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1059,7 +1060,7 @@ int prepare_fwd(const TdpArgs& a, T16** sv1_out, float** k1n_out) {
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3((unsigned)(BN * blocks), 1, 1);
-  cfg.blockDim = dim3(kPrepThreads, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
   cfg.stream = a.stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
