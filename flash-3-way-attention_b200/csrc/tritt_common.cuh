@@ -151,7 +151,8 @@ size_t sm100_tdp_bwd_optional_workspace(int B, int N);   // behind it: statistic
 size_t sm100_tdp_fwd_optional_workspace(int B, int N, int T, int D, int dtype);
 // forward kernel for causal masks with a narrow (j, k) band (tiles of four queries x 32 K2 rows)
 bool sm100_tdp_fwd_band_applies(int T, const TdpMask& m);
-int sm100_tdp_fwd_band(const TdpArgs& a, const void* sv1, const float* k1n);
+// the scratch of the one that steps over the band's diagonals, behind the statistics in the forward's workspace
+size_t sm100_tdp_fwd_diag_workspace(int B, int N, int T, int D);
 
 // fp32 inputs, and bf16 inputs with TRITT_FLAG_WIDE_OPERANDS, on the tensor cores through fp16 operand copies
 bool tdp_wide_applies(int op, int T, int D, int dtype, const TdpMask& m, int flags);

@@ -43,6 +43,12 @@ __device__ __forceinline__ uint32_t column_mask(int lo, int hi) {
   return up & down;
 }
 
+// Bound on every score of a head, in log2 units: |s| max_q |Q_q| max |K2 element| max_j |K1_j|, s = alpha log2(e), from the forward's
+// statistics (fwd_prepare_kernel).
+__device__ __forceinline__ float head_bound(const float* stats, int BN, int bh, float s) {
+  return fabsf(s) * sqrtf(__ldg(stats + BN + bh)) * sqrtf(__ldg(stats + 2 * BN + bh)) * sqrtf(__ldg(stats + bh));
+}
+
 // Sum of v[0..31] over the 32 lanes of a warp, column-wise: on return lane i holds the
 // total of column i.  31 shuffles instead of 32 full reductions.
 __device__ __forceinline__ float warp_transpose_sum(float (&v)[32], int lane) {

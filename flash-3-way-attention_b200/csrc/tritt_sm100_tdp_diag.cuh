@@ -1,0 +1,111 @@
+// What the forward kernel that steps over the diagonals of a narrow band (tritt_sm100_tdp_fwd_diag.cu) shares with the one that serves
+// such calls otherwise (tritt_sm100_tdp_fwd_band.cu): which of the two does a call, and the pieces that the first one leaves.
+#pragma once
+
+#include "tritt_sm100_tdp.cuh"
+
+#include <type_traits>
+
+namespace tritt {
+
+constexpr int kDiagD = 64;                                // head dimension
+constexpr int kDiagAreaFloats = 128 * (kDiagD + 1);       // accumulator [D][128], sums [128]
+constexpr int kDiagAreas = 4;   // of a CTA: tiles begun before its part (by the parity of the tile), tiles begun in it
+constexpr float kDiagReferenceFraction = 0.142019f;       // (see kReferenceFraction of the general forward kernel)
+
+struct DiagGeometry {
+  int T, k1w, k2w, kkl, kkr;
+  long steps;      // of the call
+  int BN, grid;
+  __host__ __device__ int tiles() const { return (T + 127) / 128; }
+  __host__ __device__ int diagonals() const { return kkl + kkr + 1; }
+  __host__ __device__ long cut(long c) const { return steps * c / grid; }
+  __host__ __device__ int cta_of(long step) const { return (int)(((step + 1) * grid + steps - 1) / steps - 1); }   // the last c with cut(c) <= step
+  // the CTAs that have steps of query tile t
+  __host__ __device__ void ctas(int bh, int t, int& first, int& count) const {
+    const long row = (long)bh * tiles(), R = diagonals();
+    first = cta_of((row + (t > 0 ? t - 1 : 0)) * R);
+    count = cta_of((row + t + 1) * R - 1) - first + 1;
+  }
+};
+
+struct DiagParams {
+  void* out;
+  float* lse;
+  const void *k1, *v1;
+  const float* stats;    // [7][BN] (see fwd_prepare_kernel)
+  float* areas;          // [grid][kDiagAreas][kDiagAreaFloats]
+  DiagGeometry g;
+  float alpha, bound_limit;
+  int* status;
+};
+
+// Fills `p` and returns true if that kernel is asked; `workspace`: sm100_tdp_fwd_diag_workspace() bytes of scratch.
+bool sm100_tdp_fwd_diag_plan(const TdpArgs& a, const float* stats, void* workspace, size_t workspace_bytes, DiagParams& p);
+int sm100_tdp_fwd_diag(const TdpArgs& a, const DiagParams& p);
+// `sv1`: SiLU(V1) in the inputs' type; `k1n`: per-head largest squared K1 row norm, or null (both prepared by the caller);
+// `diag`: what sm100_tdp_fwd_diag() was launched with just before, or null.
+int sm100_tdp_fwd_band(const TdpArgs& a, const void* sv1, const float* k1n, const DiagParams* diag);
+
+namespace {
+
+// Statistics of fwd_prepare_kernel: arrays of BN values.
+enum { kK1 = 3, kK2 = 4, kV1 = 5, kV2 = 6 };   // largest |element|
+
+// fp16 only: the power of two that A carries, as in the backward (range_shift there), so that both form the same operand: the
+// largest that keeps the factor and the products below 2^15; W's likewise.
+template <typename T16> __device__ __forceinline__ int product_range(float x, float other) {
+  if constexpr (std::is_same<T16, __half>::value) {
+    if (!(x > 0.f) || !isfinite(x) || !(other > 0.f) || !isfinite(other)) return 0;
+    const int a = (__float_as_int(x) >> 23) - 127, b = (__float_as_int(other) >> 23) - 127;
+    return 14 - a - max(b + 1, 0);
+  }
+  return 0;
+}
+template <typename T16> __device__ __forceinline__ float pow2i(int e) {
+  return std::is_same<T16, __half>::value ? __int_as_float((127 + e) << 23) : 1.f;
+}
+
+// Whether the kernel that steps over diagonals does the call: the scores of all heads are small.  All threads of the block.
+__device__ __forceinline__ bool diag_takes(const DiagParams& p) {
+  bool large = false;   // (not >, so that a NaN counts as large)
+  for (int bh = threadIdx.x; bh < p.g.BN; bh += blockDim.x)
+    large |= !(head_bound(p.stats, p.g.BN, bh, p.alpha * kLog2e) <= p.bound_limit);
+  return !__syncthreads_or(large);
+}
+
+// The pieces of the query tiles that are cut -> their outputs.  A thread takes 16 columns of a row at a time.
+template <typename T16>
+__device__ __noinline__ void diag_merge(const DiagParams& p) {
+  const DiagGeometry& g = p.g;
+  const int tiles = g.tiles(), units = g.BN * tiles * (kDiagD / 16), per_block = blockDim.x / 128, row = threadIdx.x % 128;
+  for (int u = blockIdx.x * per_block + threadIdx.x / 128; u < units; u += gridDim.x * per_block) {
+    const int bh = u / (kDiagD / 16) / tiles, tile = u / (kDiagD / 16) % tiles, c0 = u % (kDiagD / 16) * 16, q = tile * 128 + row;
+    int first, pieces;
+    g.ctas(bh, tile, first, pieces);
+    if (pieces == 1 || q >= g.T) continue;   // (whole: written by its CTA)
+    float l = 0.f, v[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) v[c] = 0.f;
+#pragma unroll 2
+    for (int i = 0; i < pieces; ++i) {
+      const float* a = p.areas + ((size_t)(first + i) * kDiagAreas + (i == 0 ? 2 : 0) + (tile & 1)) * kDiagAreaFloats + row;
+      l += a[kDiagD * 128];
+#pragma unroll
+      for (int c = 0; c < 16; ++c) v[c] += a[(c0 + c) * 128];
+    }
+    const float* st = p.stats + bh;
+    const float scale = pow2i<T16>(-product_range<T16>(__ldg(st + kV1 * g.BN), __ldg(st + kV2 * g.BN))) / l;
+    T16* dst = (T16*)p.out + ((size_t)bh * g.T + q) * kDiagD + c0;
+#pragma unroll
+    for (int c = 0; c < 16; c += 8)
+      *reinterpret_cast<uint4*>(dst + c) =
+          make_uint4(pack2<T16>(v[c] * scale, v[c + 1] * scale), pack2<T16>(v[c + 2] * scale, v[c + 3] * scale),
+                     pack2<T16>(v[c + 4] * scale, v[c + 5] * scale), pack2<T16>(v[c + 6] * scale, v[c + 7] * scale));
+    if (c0 == 0)
+      p.lse[(size_t)bh * g.T + q] = (ceilf(head_bound(p.stats, g.BN, bh, p.alpha * kLog2e)) + kDiagReferenceFraction + log2f(l)) * kLn2;
+  }
+}
+
+}  // namespace
+}  // namespace tritt

@@ -39,7 +39,7 @@
 // is uniform over the rows), and rows with k > q get weight zero in the fold.
 #include "tritt_common.cuh"
 #include "tritt_sm100.cuh"
-#include "tritt_sm100_tdp.cuh"
+#include "tritt_sm100_tdp_diag.cuh"
 
 #include <type_traits>
 
@@ -960,25 +960,26 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
 
 // What both forward kernels need before they start, in one pass over the tensors: SiLU(V1) in the inputs' type and, when
 // `stats` is not null, the per-head statistics behind the score bounds,
-//   stats[bh] = max_j |K1[bh, j, :]|^2,  stats[BN + bh] = max_q |Q[bh, q, :]|^2,  stats[2 BN + bh] = max element^2 of K2[bh].
+//   stats[bh] = max_j |K1[bh, j, :]|^2,  stats[BN + bh] = max_q |Q[bh, q, :]|^2,  stats[2 BN + bh] = max element^2 of K2[bh],
+// and, where `count` is 7, the largest |element| of K1, K2, V1 and V2 in four more arrays.
 // A cluster of blocks takes one head: the maxima meet in the first block's shared memory, so that no launch has to
 // zero anything and no atomics are needed.  8 elements per thread and step; a row is held by D / 8 neighbouring lanes.
 // Bound by launch latency on short sequences (it replaces two kernels and a memset: 47.3 -> 43.9 us per call at B=1 N=8
 // T=64 D=64) and by memory on long ones, where it is < 0.1 % of the call.  Eight blocks per head (the portable cluster
 // size) as soon as each has a pass of work, and blocks of 1024 threads for heads of more than two passes of those: 16 heads of T=2048
 // D=64 16 -> 11 us, windows 256/256/40/20 at T=2048 793 -> 785 us a call.
-constexpr int kPrepThreads = 256, kPrepMost = 1024;
+constexpr int kPrepThreads = 256, kPrepMost = 1024, kStats = 7;
 template <typename T16>
 __global__ void __launch_bounds__(kPrepMost)
 fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const T16* __restrict__ q,
-                   const T16* __restrict__ k2, T16* __restrict__ sv1, float* __restrict__ stats, int head_elems, int D,
-                   int BN, int blocks) {
-  __shared__ float red[8][3];           // [block of the cluster]; used in the first block
-  __shared__ float wred[kPrepMost / 32][3];
+                   const T16* __restrict__ k2, const T16* __restrict__ v2, T16* __restrict__ sv1, float* __restrict__ stats, int count,
+                   int head_elems, int D, int BN, int blocks) {
+  __shared__ float red[8][kStats];      // [block of the cluster]; used in the first block
+  __shared__ float wred[kPrepMost / 32][kStats];
   const int bh = blockIdx.x / blocks, part = blockIdx.x % blocks;
   const size_t base = (size_t)bh * head_elems;
   const int lanes = D / 8;
-  float m1 = 0.f, mq = 0.f, m2 = 0.f;
+  float m[kStats] = {};
   // (the bound is the same for all lanes of a row: head_elems is a multiple of D)
   for (int i = (part * blockDim.x + threadIdx.x) * 8; i < head_elems; i += blocks * blockDim.x * 8) {
     const uint4 v = *reinterpret_cast<const uint4*>(v1 + base + i);
@@ -988,8 +989,18 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
     for (int e = 0; e < 4; ++e) {
       const float2 f = unpack2<T16>(wv[e]);
       o[e] = pack2<T16>(silu_f(f.x), silu_f(f.y));
+      m[5] = fmaxf(m[5], fmaxf(fabsf(f.x), fabsf(f.y)));
     }
     *reinterpret_cast<uint4*>(sv1 + base + i) = make_uint4(o[0], o[1], o[2], o[3]);
+    if (count == kStats) {
+      const uint4 x = *reinterpret_cast<const uint4*>(v2 + base + i);
+      const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = unpack2<T16>(w[e]);
+        m[6] = fmaxf(m[6], fmaxf(fabsf(f.x), fabsf(f.y)));
+      }
+    }
     if (stats) {
       const uint4 a = *reinterpret_cast<const uint4*>(k1 + base + i), b = *reinterpret_cast<const uint4*>(q + base + i),
                   c = *reinterpret_cast<const uint4*>(k2 + base + i);
@@ -1000,7 +1011,8 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
         const float2 x = unpack2<T16>(wa[e]), y = unpack2<T16>(wb[e]), z = unpack2<T16>(wc[e]);
         n1 = fmaf(x.x, x.x, fmaf(x.y, x.y, n1));
         nq = fmaf(y.x, y.x, fmaf(y.y, y.y, nq));
-        m2 = fmaxf(m2, fmaxf(z.x * z.x, z.y * z.y));
+        m[3] = fmaxf(m[3], fmaxf(fabsf(x.x), fabsf(x.y)));
+        m[4] = fmaxf(m[4], fmaxf(fabsf(z.x), fabsf(z.y)));
       }
       // (the lanes of a row are all here or all gone; which lanes of the warp are is not the same everywhere)
       const uint32_t row_lanes = ((lanes == 32 ? 0u : 1u << lanes) - 1u) << ((threadIdx.x & 31) / lanes * lanes);
@@ -1008,47 +1020,45 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
         n1 += __shfl_xor_sync(row_lanes, n1, o2);
         nq += __shfl_xor_sync(row_lanes, nq, o2);
       }
-      m1 = fmaxf(m1, n1);
-      mq = fmaxf(mq, nq);
+      m[0] = fmaxf(m[0], n1);
+      m[1] = fmaxf(m[1], nq);
     }
   }
   if (!stats) return;
 #pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) {
-    m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-    mq = fmaxf(mq, __shfl_xor_sync(0xffffffffu, mq, o));
-    m2 = fmaxf(m2, __shfl_xor_sync(0xffffffffu, m2, o));
-  }
+  for (int o = 16; o >= 1; o >>= 1)
+#pragma unroll
+    for (int e = 0; e < kStats; ++e) m[e] = fmaxf(m[e], __shfl_xor_sync(0xffffffffu, m[e], o));
+  m[2] = m[4] * m[4];
   if ((threadIdx.x & 31) == 0) {
-    wred[threadIdx.x >> 5][0] = m1;
-    wred[threadIdx.x >> 5][1] = mq;
-    wred[threadIdx.x >> 5][2] = m2;
+#pragma unroll
+    for (int e = 0; e < kStats; ++e) wred[threadIdx.x >> 5][e] = m[e];
   }
   cluster_sync_all();   // every block of the cluster runs: its shared memory may be written (a block barrier as well)
-  if (threadIdx.x < 3) {
-    float m = 0.f;
-    for (int w = 0; w < blockDim.x / 32; ++w) m = fmaxf(m, wred[w][threadIdx.x]);
+  if (threadIdx.x < kStats) {
+    float v = 0.f;
+    for (int w = 0; w < blockDim.x / 32; ++w) v = fmaxf(v, wred[w][threadIdx.x]);
     uint32_t dst;   // the first block's red[part][.]
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(&red[part][threadIdx.x])), "r"(0));
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(m) : "memory");
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(v) : "memory");
   }
   cluster_sync_all();
-  if (part == 0 && threadIdx.x < 3) {
-    float m = 0.f;
-    for (int c = 0; c < blocks; ++c) m = fmaxf(m, red[c][threadIdx.x]);
-    stats[(size_t)threadIdx.x * BN + bh] = m;
+  if (part == 0 && threadIdx.x < count) {
+    float v = 0.f;
+    for (int c = 0; c < blocks; ++c) v = fmaxf(v, red[c][threadIdx.x]);
+    stats[(size_t)threadIdx.x * BN + bh] = v;
   }
 }
 
-// SiLU(V1) at the head of the workspace and, when the workspace has the optional tail, the statistics (the returned
-// pointer is to the first of its three arrays of B*N values, the K1 row norms).
+// SiLU(V1) at the head of the workspace and, when the workspace has the optional tail, `count` arrays of statistics (the returned
+// pointer is to the first of its arrays of B*N values, the K1 row norms).
 template <typename T16>
-int prepare_fwd(const TdpArgs& a, T16** sv1_out, float** k1n_out) {
+int prepare_fwd(const TdpArgs& a, int count, T16** sv1_out, float** k1n_out) {
   const int BN = a.B * a.N;
   const size_t n = (size_t)BN * a.T * a.D, tail = align_up(n * 2, 256);
   T16* sv1 = (T16*)a.workspace;
   float* k1n = nullptr;
-  if (a.workspace_bytes >= tail + 3 * (size_t)BN * sizeof(float)) k1n = reinterpret_cast<float*>((char*)a.workspace + tail);
+  if (a.workspace_bytes >= tail + count * (size_t)BN * sizeof(float)) k1n = reinterpret_cast<float*>((char*)a.workspace + tail);
   const int head_elems = a.T * a.D;
   int blocks = 1;
   while (blocks < 8 && blocks * kPrepThreads * 8 < head_elems) blocks *= 2;
@@ -1065,7 +1075,7 @@ int prepare_fwd(const TdpArgs& a, T16** sv1_out, float** k1n_out) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   TRITT_CUDA_OK(cudaLaunchKernelEx(&cfg, fwd_prepare_kernel<T16>, (const T16*)a.v1, (const T16*)a.k1, (const T16*)a.q,
-                                   (const T16*)a.k2, sv1, k1n, head_elems, a.D, BN, blocks));
+                                   (const T16*)a.k2, (const T16*)a.v2, sv1, k1n, count, head_elems, a.D, BN, blocks));
   count_launch();
   *sv1_out = sv1;
   *k1n_out = k1n;
@@ -1078,9 +1088,17 @@ int launch_fwd(const TdpArgs& a) {
   const int BN = a.B * a.N;
   T16* sv1 = nullptr;
   float* k1n = nullptr;
-  int rc = prepare_fwd<T16>(a, &sv1, &k1n);
+  const bool band = sm100_tdp_fwd_band_applies(a.T, a.mask);
+  const size_t diag_offset = align_up(align_up((size_t)BN * a.T * D * 2, 256) + kStats * (size_t)BN * sizeof(float), 256);
+  DiagParams diag;
+  const bool by_diagonals =
+      band && a.workspace_bytes > diag_offset &&
+      sm100_tdp_fwd_diag_plan(a, nullptr, (char*)a.workspace + diag_offset, a.workspace_bytes - diag_offset, diag);
+  int rc = prepare_fwd<T16>(a, by_diagonals ? kStats : 3, &sv1, &k1n);
   if (rc) return rc;
-  if (sm100_tdp_fwd_band_applies(a.T, a.mask)) return sm100_tdp_fwd_band(a, sv1, k1n);
+  diag.stats = k1n;
+  if (by_diagonals && (rc = sm100_tdp_fwd_diag(a, diag))) return rc;
+  if (band) return sm100_tdp_fwd_band(a, sv1, k1n, by_diagonals ? &diag : nullptr);
   CUtensorMap tmK1, tmK2, tmSV1;
   if ((rc = make_tmap_3d(&tmK1, a.k1, 2, D, a.T, BN, 64, 128))) return rc;
   if ((rc = make_tmap_3d(&tmSV1, sv1, 2, D, a.T, BN, 64, 128))) return rc;
@@ -1134,7 +1152,8 @@ bool sm100_tdp_supported(int op, int T, int D, int dtype, const TdpMask& m) {
 size_t sm100_tdp_fwd_optional_workspace(int B, int N, int T, int D, int dtype) {
   if (dtype != TRITT_BF16 && dtype != TRITT_F16) return 0;
   const size_t n = (size_t)B * N * T * D;
-  return align_up(n * 2, 256) - n * 2 + align_up(3 * (size_t)B * N * sizeof(float), 256);
+  return align_up(n * 2, 256) - n * 2 + align_up(kStats * (size_t)B * N * sizeof(float), 256) +
+         align_up(sm100_tdp_fwd_diag_workspace(B, N, T, D), 256);
 }
 
 size_t sm100_tdp_workspace(int op, int B, int N, int T, int D, int dtype) {

@@ -18,11 +18,13 @@
 //   warp 1       tcgen05.mma issuer: S(t), then P V of tile t - 1, so that a tile's soft-max overlaps its neighbour's products
 //   warps 4-7    soft-max warpgroup of slot 0, warps 8-11 of slot 1 (one row per thread; they also form A)
 //   warps 12-15  fold warpgroup: warp g owns query q_g (the V2 factor comes from the block in shared memory)
+// Calls with small scores at head dimension 64 are left to the kernel that steps over diagonals (tritt_sm100_tdp_fwd_diag.cu), ahead of this
+// one, which then adds up the tiles that the other has cut.
 // The kernel is bound by the instruction issue of the soft-max and fold warps (a tile is 16 K exponentials with
 // per-element column masks for ~12 M flop), not by the tensor pipe or by memory.
 #include "tritt_common.cuh"
 #include "tritt_sm100.cuh"
-#include "tritt_sm100_tdp.cuh"
+#include "tritt_sm100_tdp_diag.cuh"
 
 #include <type_traits>
 
@@ -80,7 +82,8 @@ struct BandTile {
 template <int D, typename T16>
 __global__ void __launch_bounds__(kBandThreads, 1)
 tdp_fwd_band_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__ CUtensorMap tmK2b,
-                    const __grid_constant__ CUtensorMap tmV2b, const __grid_constant__ CUtensorMap tmSV1, BandParams p) {
+                    const __grid_constant__ CUtensorMap tmV2b, const __grid_constant__ CUtensorMap tmSV1, BandParams p,
+                    const __grid_constant__ DiagParams diag) {
   using Cfg = BandCfg<D>;
   constexpr int NS = Cfg::kStages;
   constexpr int KH = D / 64;
@@ -90,6 +93,11 @@ tdp_fwd_band_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_const
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (smem_u32(smem) & 1023u) {
     if (tid == 0 && p.status) atomicOr(p.status, 8);
+    return;
+  }
+  if (diag.g.grid > 0 && diag_takes(diag)) {
+    // the kernel that steps over diagonals has done the call: what is left are the tiles that it cut
+    diag_merge<T16>(diag);
     return;
   }
   if (tid == 0) {
@@ -494,7 +502,7 @@ tdp_fwd_band_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_const
 }
 
 template <int D, typename T16>
-int launch_band(const TdpArgs& a, const void* sv1, const float* k1n) {
+int launch_band(const TdpArgs& a, const void* sv1, const float* k1n, const DiagParams* diag) {
   using Cfg = BandCfg<D>;
   const int BN = a.B * a.N;
   CUtensorMap tmK1, tmK2b, tmV2b, tmSV1;
@@ -526,7 +534,7 @@ int launch_band(const TdpArgs& a, const void* sv1, const float* k1n) {
   TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
   const long items = (long)p.n_groups * BN;
   const int grid = (int)(items < num_sms() ? items : num_sms());
-  kern<<<grid, kBandThreads, Cfg::kSmem, a.stream>>>(tmK1, tmK2b, tmV2b, tmSV1, p);
+  kern<<<grid, kBandThreads, Cfg::kSmem, a.stream>>>(tmK1, tmK2b, tmV2b, tmSV1, p, diag ? *diag : DiagParams{});
   count_launch();
   TRITT_CUDA_OK(cudaGetLastError());
   return 0;
@@ -540,11 +548,10 @@ bool sm100_tdp_fwd_band_applies(int T, const TdpMask& m) {
   return m.causal && T > 128 && m.kkl + m.kkr <= 128 - kRK;
 }
 
-// `sv1`: SiLU(V1) in the inputs' type; `k1n`: per-head largest squared K1 row norm, or null (both prepared by the caller).
-int sm100_tdp_fwd_band(const TdpArgs& a, const void* sv1, const float* k1n) {
+int sm100_tdp_fwd_band(const TdpArgs& a, const void* sv1, const float* k1n, const DiagParams* diag) {
   if (a.dtype == TRITT_BF16)
-    return a.D == 128 ? launch_band<128, __nv_bfloat16>(a, sv1, k1n) : launch_band<64, __nv_bfloat16>(a, sv1, k1n);
-  return a.D == 128 ? launch_band<128, __half>(a, sv1, k1n) : launch_band<64, __half>(a, sv1, k1n);
+    return a.D == 128 ? launch_band<128, __nv_bfloat16>(a, sv1, k1n, diag) : launch_band<64, __nv_bfloat16>(a, sv1, k1n, diag);
+  return a.D == 128 ? launch_band<128, __half>(a, sv1, k1n, diag) : launch_band<64, __half>(a, sv1, k1n, diag);
 }
 
 }  // namespace tritt

@@ -1,0 +1,83 @@
+"""The forward of narrow bands by the kernel that steps over the band's diagonals: tile edges, cut query tiles, and whom it serves."""
+import pytest
+import torch
+
+from _parity import assert_close
+from oracle import trittention_oracle as orc
+from flash_trittention import _native
+
+DEV = "cuda:0"
+
+
+def _forward(t, alpha, windows, ws=None):
+    B, N, T, _ = t[0].shape
+    o, lse = torch.full_like(t[0], float("nan")), torch.full((B, N, T), float("nan"), device=DEV)
+    _native.tdp_fwd(*t, o, lse, alpha, True, *windows, ws=ws)
+    torch.cuda.synchronize()
+    assert _native.read_status(torch.device(DEV)) == 0, "a bounded barrier wait ran out"
+    return o, lse
+
+
+def _workspace_without_it(t):
+    """Room for SiLU(V1) and three statistics a head: the call runs on the kernel of four queries by 32 rows."""
+    B, N, T, D = t[0].shape
+    return torch.empty((B * N * T * D * 2 + 255) // 256 * 256 + 3 * B * N * 4, dtype=torch.uint8, device=DEV)
+
+
+def _inputs(heads, T, scale, dtype, seed):
+    return [x.to(DEV) for x in orc.make_inputs(1, heads, T, 64, scale=scale, seed=seed, dtype=dtype)[:5]]
+
+
+# The widest band and windows, the narrowest, bands to one side, and either window as the one that bounds the reach to 128; heads: enough
+# for the call to be asked of this kernel (a narrow window needs more), which also cuts query tiles between CTAs.
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T", [129, 255, 256, 257, 400])
+@pytest.mark.parametrize("windows,heads", [((128, 128, 48, 48), 20), ((128, 128, 96, 0), 20), ((128, 400, 0, 96), 12), ((300, 100, 28, 9), 20),
+                                           ((1, 1, 1, 1), 120), ((0, 9, 2, 5), 120)])
+def test_against_the_oracle(windows, heads, T, dtype):
+    t = _inputs(heads, T, 0.5, dtype, T + heads)
+    o, lse = _forward(t, 1 / 64, windows)
+    ref_o, ref_lse = orc.tdp_forward(*[x.float() for x in t], 1 / 64, True, *windows, device=DEV)
+    assert_close("o", o, ref_o, dtype)
+    # scores of order 0.1, operands of 8 or 11 bits: the log of a sum of exponentials moves by less than 2^-9 of the largest score
+    assert float((lse - ref_lse).abs().max()) <= 2e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_large_scores_of_one_head_are_left_to_the_other_kernel(dtype):
+    """Small scores: this kernel, whose roundings are others.  One head with large ones, or not finite: the whole call is the
+    other kernel's, bit for bit."""
+    windows, heads, T = (100, 128, 20, 30), 16, 300
+    t = _inputs(heads, T, 0.5, dtype, 1)
+    a, b = _forward(t, 1 / 64, windows), _forward(t, 1 / 64, windows, _workspace_without_it(t))
+    assert not torch.equal(a[0], b[0])
+    assert float((a[0].float() - b[0].float()).norm()) <= (2e-3 if dtype == torch.float16 else 1e-2) * float(b[0].float().norm())
+    for value in (60.0, float("inf")):
+        t[0][0, heads - 1, T - 1, 5] = value
+        t[1][0, heads - 1, 7, 5] = 50.0
+        a, b = _forward(t, 1 / 8, windows), _forward(t, 1 / 8, windows, _workspace_without_it(t))
+        assert torch.equal(a[0].nan_to_num(1e4), b[0].nan_to_num(1e4)) and torch.equal(a[1].nan_to_num(1e4), b[1].nan_to_num(1e4))
+
+
+@pytest.mark.gpu
+def test_captured_call_replays_for_new_inputs():
+    windows, heads, T = (128, 128, 32, 32), 16, 700
+    t = _inputs(heads, T, 0.5, torch.float16, 2)
+    o, lse = torch.empty_like(t[0]), torch.empty(1, heads, T, device=DEV)
+    ws = _native.workspace(_native.OP_TDP_FWD, 1, heads, T, 64, _native.F16, t[0].device)
+    call = lambda: _native.tdp_fwd(*t, o, lse, 1 / 64, True, *windows, ws=ws)
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call()
+    for scale, alpha_seed in ((0.5, 3), (0.4, 4)):
+        for x, y in zip(t, _inputs(heads, T, scale, torch.float16, alpha_seed)):
+            x.copy_(y)
+        for _ in range(3):
+            graph.replay()
+        torch.cuda.synchronize()
+        want = _forward(t, 1 / 64, windows)
+        assert torch.equal(o, want[0]) and torch.equal(lse, want[1])
