@@ -11,19 +11,23 @@
 // It serves calls whose scores are small: a bound on every score of a head is the soft-max reference of the head's rows.  Other calls
 // are left to tdp_fwd_band_kernel, behind this one, whose operand alpha Q K2 is also what the backward forms for large scores.
 //
-// A CTA has two slots, each with an accumulator, a soft-max warpgroup (a query per thread) and every other query tile: a step is
-// one d of one j-tile for both.  All steps of a call form one line (heads, j-tiles, d) that is cut in equal parts, one per
-// CTA; a query tile whose steps are cut leaves its accumulators in the workspace, and a kernel behind this one adds them up.
+// A CTA has two slots, each with an accumulator, two soft-max warpgroups (a query per thread, every other 32 of its columns) and every
+// other query tile: a step is one d of one j-tile for both.  All steps of a call form one line (heads, j-tiles, d) that is cut in
+// equal parts, one per CTA; a query tile whose steps are cut leaves its accumulators in the workspace, and a kernel behind this one
+// adds them up.
 //
-// What bounds it: the soft-max warps' share of a step (reads of the scores, exponentials, P back to tensor memory, waits), 3500 cycles
-// for both slots, of which the exponentials of the attended half take 1000 and the products 1200.  Forward, us per call, the kernel of 4 queries x
-// 32 rows -> this one: 16 heads T=2048 fp16 windows 128/128/32/32 471 -> 220, T=8192 1940 -> 810, T=2048 windows 8/8/4/4 124 -> 50,
-// 8 heads T=1000 124 -> 72, 16 heads T=500 128/128/48/48 123 -> 93; fp32 tensors, 8 heads T=2048 260 -> 133.
+// What bounds it: no single unit.  A step takes 2700 cycles for both slots; issue slots are 60 % busy, the exponentials' unit 48 %, tensor
+// cores 45 %, and a slot's chain (scores, exponentials, P, value product) is not hidden behind the other slot's alone.  One soft-max
+// warpgroup per slot walking all 128 columns took 3200 cycles (220 us for 189, 810 for 679 below).  Forward, us per call, the
+// kernel of 4 queries x 32 rows -> this one: 16 heads T=2048 fp16 windows 128/128/32/32 471 -> 189, T=8192 1940 -> 682, T=2048 windows
+// 8/8/4/4 124 -> 51, 8 heads T=1000 126 -> 65, 16 heads T=500 128/128/48/48 124 -> 82; fp32 tensors, 8 heads T=2048 262 -> 119.
+// Slower: masks of boundary columns by clamped FMAs (194 us for 189), a quarter of the exponentials as polynomials (194), value products
+// that start with the first warpgroup's half of P (190).
 //
-// 20 warps: 0-3 and 4-7: soft-max warpgroups of the slots; 8-15: form A and W, from K1 and SiLU(V1) rows in registers and K2 / V2 rows
-// in shared memory; 16 and 18 issue the score and the value products; 17: the line of work and all loads.  Three buffers of
-// scores are taken in turn, P lies over the first half of its scores: a slot's next scores wait for the other slot's last value
-// product, not for its own.
+// 28 warps: 0-7 and 8-15: soft-max warpgroups of the slots; 16-23: form A and W, from K1 and SiLU(V1) rows in registers and K2 / V2
+// rows in shared memory; 24 and 26 issue the score and the value products; 25: the line of work and all loads.  Three buffers of
+// scores are taken in turn, P of 32 columns lies over the first half of their scores: a slot's next scores wait for the other slot's
+// last value product, not for its own.
 #include "tritt_sm100_tdp_diag.cuh"
 
 #include <atomic>
@@ -32,10 +36,10 @@ namespace tritt {
 namespace {
 using namespace sm100;
 
-constexpr int kDiagThreads = 640;
-// Registers per thread: 640 threads are launched with 96 each, and split them anew (set_regs).
-constexpr int kDiagRegs = 96, kRegsSoftmax = 128, kRegsFormer = 80, kRegsService = 64;
-static_assert(2 * kRegsSoftmax + 2 * kRegsFormer + kRegsService <= 5 * kDiagRegs, "more registers than the launch has");
+constexpr int kDiagThreads = 896;
+// Registers per thread: 896 threads are launched with 72 each, and split them anew (set_regs).
+constexpr int kDiagRegs = 72, kRegsSoftmax = 72, kRegsFormer = 80, kRegsService = 56;
+static_assert(4 * kRegsSoftmax + 2 * kRegsFormer + kRegsService <= 7 * kDiagRegs, "more registers than the launch has");
 constexpr int kMaxBand = 96;        // kk_left + kk_right
 constexpr int kTile = 128 * kDiagD * 2; // a tile of 128 rows
 constexpr int kNB = 3;              // buffers of A and of W
@@ -43,7 +47,7 @@ constexpr int kNQ = 4;              // Q tiles
 constexpr int kNS = 3;              // buffers of scores
 constexpr int kWindow = (128 + kMaxBand) * kDiagD * 2;   // K2 / V2 rows of an item
 constexpr int kOffQ = 0, kOffA = kNQ * kTile, kOffW = kOffA + kNB * kTile, kOffK2 = kOffW + kNB * kTile,
-              kOffV2 = kOffK2 + kWindow, kOffBars = kOffV2 + kWindow, kSmem = kOffBars + 768;
+              kOffV2 = kOffK2 + kWindow, kOffL = kOffV2 + kWindow, kOffBars = kOffL + 4096, kSmem = kOffBars + 768;
 static_assert(kSmem <= 232448 && kOffK2 % 1024 == 0 && kWindow % 1024 == 0, "shared memory");
 constexpr int kTmemO = kNS * 128;   // accumulators
 constexpr int kItemSlots = 4;
@@ -66,7 +70,7 @@ struct DiagBarriers {
   uint64_t q_full[kNQ], q_free[kNQ];
   uint64_t a_ready[kNB], a_free[kNB], w_ready[kNB], w_free[kNB];
   // (s_ready doubled by the parity of the steps: a slot's next scores do not wait for it to have looked at these)
-  uint64_t s_ready[2][2], p_ready[2], pv_done[2], place_free[kNS];
+  uint64_t s_ready[2][2], p_ready[2], pv_done[2], place_free[kNS], l_ready[2];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -90,7 +94,7 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     bars.abort_flag = 0;
     for (int i = 0; i < kItemSlots; ++i) {
       mbar_init(&bars.item_full[i], 1);
-      mbar_init(&bars.item_free[i], 18);
+      mbar_init(&bars.item_free[i], 26);
     }
     mbar_init(&bars.win_full, 1);
     mbar_init(&bars.win_free, 8);
@@ -107,13 +111,14 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars.s_ready[i][0], 1);
       mbar_init(&bars.s_ready[i][1], 1);
-      mbar_init(&bars.p_ready[i], 4);
+      mbar_init(&bars.p_ready[i], 8);
+      mbar_init(&bars.l_ready[i], 8);
       mbar_init(&bars.pv_done[i], 1);
     }
     for (int i = 0; i < kNS; ++i) mbar_init(&bars.place_free[i], 1);
     fence_barrier_init();
   }
-  if (warp == 16) {
+  if (warp == 24) {
     tmem_alloc(&bars.tmem_base, 512);
     tmem_relinquish();
   }
@@ -136,14 +141,17 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   // (every lane has the same value; the reduction tells the compiler so)
   auto uniform = [](int v) -> int { return __reduce_max_sync(0xffffffffu, v); };
 
-  if (warp < 8) {
+  if (warp < 16) {
     set_regs<kDiagRegs, kRegsSoftmax>();
     // ------------------------------------------------------------------ soft-max warpgroups
-    const int x = warp >> 2, wq = warp & 3;
+    const int x = warp >> 3, half = warp >> 2 & 1, wq = warp & 3;
     const int row = wq * 32 + lane;
-    const uint32_t tB = tmem + ((uint32_t)(wq * 32) << 16), tO = tB + kTmemO + x * kDiagD;
+    const uint32_t tB = tmem + ((uint32_t)(wq * 32) << 16), tO = tB + kTmemO + x * kDiagD + half * (kDiagD / 2);
     uint32_t step = 0;        // steps so far
-    float l = 0.f;            // sum of the row's P
+    uint32_t ends = 0;        // query tiles so far
+    float l = 0.f;            // sum of this thread's P
+    // (sums of the row's two threads, of this query tile and, doubled, the next)
+    float* const row_l = reinterpret_cast<float*>(smem + kOffL) + x * 256 + row;
     for (uint32_t items = 0;; ++items) {
       if (!wait_all(&bars.item_full[items % kItemSlots], (items / kItemSlots) & 1)) break;
       const DiagItem& it = bars.items[items % kItemSlots];
@@ -171,17 +179,16 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const bool seen = mbar_test(&bars.pv_done[x], (step & 1) ^ 1);
         float2 sum = make_float2(0.f, 0.f);
 #pragma unroll 1
-        for (int c0 = 0; c0 < 128; c0 += 32) {
+        for (int c0 = 32 * half; c0 < 128; c0 += 64) {
           uint32_t w[16];
           const uint32_t mask = column_mask(lo - c0, hi - c0);
-          const bool all = __all_sync(0xffffffffu, mask == ~0u);
-          if (all || __any_sync(0xffffffffu, mask != 0u)) {
-            // (A read is waited for right where it is issued: its registers are written while it is under way, which the
-            // compiler does not know of.)
+          if (__any_sync(0xffffffffu, mask != 0u)) {
+            // (A read is waited for right where it is issued: its registers are written while it is under way, which the compiler
+            // does not know of.)
             uint32_t v[32];
             tmem_ld32(tS + c0, v);
             tmem_wait_ld(v);
-            if (all) {
+            if (__all_sync(0xffffffffu, mask == ~0u)) {
 #pragma unroll
               for (int c = 0; c < 32; c += 2) {
                 const float2 y = __ffma2_rn(make_float2(__uint_as_float(v[c]), __uint_as_float(v[c + 1])), sa2, nref);
@@ -202,7 +209,7 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
             for (int c = 0; c < 16; ++c) w[c] = 0u;
           }
-          tmem_st16(tS + c0 / 2, w);
+          tmem_st16(tS + c0, w);   // over these columns' scores
         }
         l += sum.x + sum.y;
         tmem_wait_st();
@@ -214,15 +221,21 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (!alive) break;
       if (!(flags & (own ? kEndOwn : kEndNext)) || tile >= g.tiles()) continue;
       // ---- the tile's output, or this CTA's piece of it
+      row_l[(ends & 1) * 512 + half * 128] = l;
+      arrive_warp(&bars.l_ready[x]);
       if (!wait_all(&bars.pv_done[x], (step - 1) & 1)) break;
       tc_fence_after();
+      if (!wait_all(&bars.l_ready[x], ends & 1)) break;
+      const float row_sum = row_l[(ends & 1) * 512] + row_l[(ends & 1) * 512 + 128];
+      ++ends;
       int first, pieces;
       g.ctas(bh, tile, first, pieces);
-      const float scale = pow2i<T16>(-eb) / l;
-      T16* const dst = (T16*)p.out + ((size_t)bh * T + q) * kDiagD;
-      float* const area = p.areas + ((size_t)blockIdx.x * kDiagAreas + ((int)blockIdx.x == first ? 2 : 0) + (tile & 1)) * kDiagAreaFloats + row;
+      const float scale = pow2i<T16>(-eb) / row_sum;
+      T16* const dst = (T16*)p.out + ((size_t)bh * T + q) * kDiagD + half * (kDiagD / 2);
+      float* const area = p.areas + ((size_t)blockIdx.x * kDiagAreas + ((int)blockIdx.x == first ? 2 : 0) + (tile & 1)) * kDiagAreaFloats +
+                          half * (kDiagD / 2) * 128 + row;
 #pragma unroll 1
-      for (int c0 = 0; c0 < kDiagD; c0 += 16) {
+      for (int c0 = 0; c0 < kDiagD / 2; c0 += 16) {
         uint32_t t[16];
         tmem_ld16(tO + c0, t);
         tmem_wait_ld(t);
@@ -242,17 +255,19 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         __syncwarp();   // (the lanes of rows beyond the sequence store nothing; the next read takes the whole warp)
       }
       tc_fence_before();
-      if (pieces > 1) area[kDiagD * 128] = l;
-      else if (q < T) p.lse[(size_t)bh * T + q] = (reference + log2f(l)) * kLn2;
+      if (half == 1) {
+        if (pieces > 1) area[kDiagD / 2 * 128] = row_sum;
+        else if (q < T) p.lse[(size_t)bh * T + q] = (reference + log2f(row_sum)) * kLn2;
+      }
       __syncwarp();
     }
-  } else if (warp < 16) {
+  } else if (warp < 24) {
     set_regs<kDiagRegs, kRegsFormer>();
     // ------------------------------------------------------------------ operands
     // A thread has one 16-byte column of every fourth row of its warp's share.  K1 stays in 16 bits (a product of two 16-bit
     // numbers is rounded once), SiLU(V1) in fp32, so that W is rounded once as well.
     constexpr int NR = 4;
-    const int col = lane & 7, row0 = (warp - 8) * 16 + (lane >> 3);
+    const int col = lane & 7, row0 = (warp - 16) * 16 + (lane >> 3);
     // (rows row0 + 4 i: the swizzle has two values)
     const uint32_t at[2] = {swz128(row0, col), swz128(row0 + 4, col) - 512};
     uint32_t step = 0;
@@ -338,7 +353,7 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     auto commit = [&](uint64_t* bar) {
       if (leader) mma_commit(bar);
     };
-    if (warp == 16) {
+    if (warp == 24) {
       // ---------------------------------------------------------------- scores
       const uint32_t qLo = desc_lo(smem_u32(smem + kOffQ), 16), aLo = desc_lo(smem_u32(smem + kOffA), 16);
       uint32_t step = 0, place = 0;
@@ -371,7 +386,7 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (flags & kEndOwn) commit(&bars.q_free[qn % kNQ]);
         if (flags & kEndNext) commit(&bars.q_free[(qn + 1) % kNQ]);
       }
-    } else if (warp == 18) {
+    } else if (warp == 26) {
       // ---------------------------------------------------------------- value products
       const uint32_t wLo = desc_lo(smem_u32(smem + kOffW), 16384);
       uint32_t step = 0, place = 0;
@@ -393,7 +408,7 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             tc_fence_after();
 #pragma unroll
             for (int k = 0; k < 8; ++k)
-              if (leader) mma_ts_lo(d, a + k * 8, w + k * (2048 >> 4), kHi, idesc_pv, k > 0 || !fresh ? 1u : 0u);
+              if (leader) mma_ts_lo(d, a + (k >> 1) * 32 + (k & 1) * 8, w + k * (2048 >> 4), kHi, idesc_pv, k > 0 || !fresh ? 1u : 0u);
             commit(&bars.place_free[place]);
             commit(&bars.pv_done[x]);
             place = place + 1 == kNS ? 0 : place + 1;
@@ -401,7 +416,7 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           commit(&bars.w_free[buf]);
         }
       }
-    } else if (warp == 17) {
+    } else if (warp == 25) {
       // ---------------------------------------------------------------- loader
       if (leader) {
         tma_prefetch_desc(&tmQ);
@@ -484,13 +499,13 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   // ------------------------------------------------------------------ teardown
   tc_fence_before();
   __syncthreads();
-  if (warp == 16) tmem_dealloc(tmem, 512);
+  if (warp == 24) tmem_dealloc(tmem, 512);
   if (tid == 0 && bars.abort_flag && p.status) atomicOr(p.status, 2);
 }
 
 constexpr int kMinSteps = 12;      // of a CTA
 // Tiles of a CTA of tdp_fwd_band_kernel (1.7 us each) from which on this kernel is asked.  Calls with small scores, tiles: us without it / with
-// it:  14: 39 / 44, 16: 39 / 44, 28: 85 / 56, 34: 72 / 39, 35: 72 / 51, 70: 124 / 72.  Calls with large scores pay for a kernel that
+// it:  14: 39 / 44, 16: 39 / 44, 28: 85 / 54, 34: 72 / 37, 35: 72 / 47, 70: 124 / 65.  Calls with large scores pay for a kernel that
 // does nothing: 28: 85 / 75 (the preparation became faster), 35: 84 / 84, 70: 124 / 124, 112: 189 / 192, 277: 469 / 469.
 constexpr long kMinBandTiles = 24;
 
