@@ -1,4 +1,4 @@
-"""Builds libtritt_sm100.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a.
+"""Builds libtritt_sm100.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a, and the host extension _host.so with g++.
 
     python flash-3-way-attention_b200/build.py [--force] [--verbose]
 
@@ -20,6 +20,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "build")
 LIB = os.path.join(HERE, "flash_trittention", "libtritt_sm100.so")
+HOST_SRC = os.path.join(CSRC, "host", "tritt_host.cpp")
+HOST = os.path.join(HERE, "flash_trittention", "_host.so")
 
 NVCC_FLAGS = [
     "-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
@@ -32,6 +34,25 @@ def _nvcc() -> str:
         if cand and os.path.exists(cand):
             return cand
     raise RuntimeError("nvcc not found")
+
+
+def build_host(force: bool = False) -> str:
+    """The extension module that makes a call's checks and allocations natively (a host program against PyTorch's headers)."""
+    if not force and os.path.exists(HOST) and os.path.getmtime(HOST) > os.path.getmtime(HOST_SRC):
+        return HOST
+    import sysconfig
+
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include", f"-I{cuda}", f"-I{sysconfig.get_paths()['include']}",
+           HOST_SRC, "-o", HOST, f"-L{root}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {HOST_SRC}:\n{r.stdout}\n{r.stderr}")
+    return HOST
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -64,6 +85,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    build_host(force)
     return LIB
 
 

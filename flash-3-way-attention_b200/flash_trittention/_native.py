@@ -7,8 +7,10 @@ from __future__ import annotations
 
 import ctypes as C
 import functools
+import importlib
 import os
 import threading
+import warnings
 
 import torch
 
@@ -33,6 +35,7 @@ SYMBOLS = (
 )
 
 _lib = None
+_host = None  # the extension module, once lib() has loaded it
 _lock = threading.Lock()
 _status = {}  # device index -> pinned int32 status word (created under _lock)
 _status_np = {}  # device index -> numpy view of the same word (a host read without any tensor machinery)
@@ -42,6 +45,30 @@ launches = 0  # kernels-enqueuing library calls made by this process (bench book
 
 class TrittError(RuntimeError):
     pass
+
+
+def host_forward(*args):
+    """A whole forward call by the native extension, ``csrc/host/tritt_host.cpp`` (whose function takes this one's place once
+    ``lib()`` has loaded it), or ``None``: the call is one for the Python code."""
+
+
+def host_backward(*args):
+    """The same for a backward call."""
+
+
+def _load_host(L):
+    global _host, host_forward, host_backward
+    try:
+        _host = importlib.import_module("._host", __package__)
+    except ImportError as e:
+        warnings.warn(f"the host extension of flash_trittention cannot be loaded ({e}): short calls take twice as long; build it "
+                      "with `python flash-3-way-attention_b200/build.py`", stacklevel=3)
+        return
+    _host.init(*(C.cast(f, C.c_void_p).value for f in (L.tritt_tdp_fwd, L.tritt_tdp_bwd, L.tritt_dps_fwd, L.tritt_dps_bwd,
+                                                       L.tritt_dps_bwd_saved, L.tritt_workspace_bytes_flags)))
+    for device, address in _status_ptr.items():
+        _host.set_status(device, address)
+    host_forward, host_backward = _host.forward, _host.backward
 
 
 def lib():
@@ -94,6 +121,7 @@ def lib():
                 L.tritt_selftest_umma.argtypes = [vp] * 5 + [i, vp, vp]
                 L.tritt_selftest_wait_expiry.restype = i
                 L.tritt_selftest_wait_expiry.argtypes = [i, C.c_longlong, vp, vp]
+                _load_host(L)
                 _lib = L
     return _lib
 
@@ -103,6 +131,15 @@ def dtype_code(dt: torch.dtype) -> int:
         return _DTYPES[dt]
     except KeyError:
         raise ValueError(f"unsupported dtype {dt}: expected float32, float16 or bfloat16") from None
+
+
+def host_result(out, what: str):
+    """The tensors of a host_forward / host_backward call; an error code is raised."""
+    global launches
+    if out.__class__ is int:
+        _check(out, what)
+    launches += 1
+    return out
 
 
 def _check(rc: int, what: str):
@@ -140,6 +177,8 @@ def status_word(device) -> torch.Tensor:
                 _status_np[key] = t.numpy()
                 _status_ptr[key] = t.data_ptr()
                 _status[key] = t
+                if _host is not None:
+                    _host.set_status(key, t.data_ptr())
     return t
 
 

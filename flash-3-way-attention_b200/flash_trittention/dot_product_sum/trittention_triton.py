@@ -14,32 +14,40 @@ import torch.nn as nn
 from .. import _native
 
 
+def _validate(q, k1, k2, v1, v2):
+    if not (q.shape == k1.shape == k2.shape == v1.shape == v2.shape):
+        raise ValueError(
+            f"Shape mismatch: q={q.shape}, k1={k1.shape}, k2={k2.shape}, v1={v1.shape}, v2={v2.shape}")
+    if not (q.dtype == k1.dtype == k2.dtype == v1.dtype == v2.dtype):
+        raise ValueError("q, k1, k2, v1, v2 must all have the same dtype")
+    if not (q.device == k1.device == k2.device == v1.device == v2.device):
+        raise ValueError("q, k1, k2, v1, v2 must all be on the same device")
+    if q.dim() != 4:
+        raise ValueError(f"expected [batch, heads, seq_len, head_dim] tensors, got shape {tuple(q.shape)}")
+    d = q.shape[-1]
+    if d <= 0 or d & (d - 1):
+        raise ValueError(f"head_dim must be a power of 2, got {d}")
+    if not q.is_cuda:
+        raise RuntimeError("TrittentionTriton runs on CUDA tensors only (there is no CPU path)")
+    _native.dtype_code(q.dtype)
+
+
 class TrittentionTritonFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k1, k2, v1, v2, causal, softmax_scale, k_diff, convert_to_float32=False,
                 input_precision=None):
-        if not (q.shape == k1.shape == k2.shape == v1.shape == v2.shape):
-            raise ValueError(
-                f"Shape mismatch: q={q.shape}, k1={k1.shape}, k2={k2.shape}, v1={v1.shape}, v2={v2.shape}")
-        if not (q.dtype == k1.dtype == k2.dtype == v1.dtype == v2.dtype):
-            raise ValueError("q, k1, k2, v1, v2 must all have the same dtype")
-        if not (q.device == k1.device == k2.device == v1.device == v2.device):
-            raise ValueError("q, k1, k2, v1, v2 must all be on the same device")
-        if q.dim() != 4:
-            raise ValueError(f"expected [batch, heads, seq_len, head_dim] tensors, got shape {tuple(q.shape)}")
-        d = q.shape[-1]
-        if d <= 0 or d & (d - 1):
-            raise ValueError(f"head_dim must be a power of 2, got {d}")
-        if not q.is_cuda:
-            raise RuntimeError("TrittentionTriton runs on CUDA tensors only (there is no CPU path)")
-        _native.dtype_code(q.dtype)
-        q, k1, k2, v1, v2 = (_native.aligned(t) for t in (q, k1, k2, v1, v2))
-        o = torch.empty_like(q)
-        m = q.new_empty(q.shape[:3], dtype=torch.float32)
         # convert_to_float32 asks for fp32 operands inside the kernels (reference trittention_triton.py:98-117
         # forwards it to its launches): the CUDA-core path computes in fp32 on every dtype
         flags = _native.FLAG_FORCE_SIMT if (convert_to_float32 or input_precision == "ieee") else 0
-        ws = _native.dps_fwd(q, k1, k2, v1, v2, o, m, softmax_scale, causal, k_diff, flags=flags)
+        out = _native.host_forward(_native.OP_DPS_FWD, q, k1, k2, v1, v2, softmax_scale, causal, flags, k_diff)
+        if out is not None:
+            o, m, ws = _native.host_result(out, "tritt_dps_fwd")
+        else:
+            _validate(q, k1, k2, v1, v2)
+            q, k1, k2, v1, v2 = (_native.aligned(t) for t in (q, k1, k2, v1, v2))
+            o = torch.empty_like(q)
+            m = q.new_empty(q.shape[:3], dtype=torch.float32)
+            ws = _native.dps_fwd(q, k1, k2, v1, v2, o, m, softmax_scale, causal, k_diff, flags=flags)
         # the forward's workspace holds the inner attention's results; kept for the backward (the reference saves
         # only the inputs, o and m and recomputes, trittention_triton.py:122-128)
         ctx.fwd_ws = ws if any(ctx.needs_input_grad[:5]) else None
@@ -57,12 +65,17 @@ class TrittentionTritonFunction(torch.autograd.Function):
         assert grad_output.shape == o.shape, f"Shape mismatch: O={o.shape}, dO={grad_output.shape}"
         assert o.device == grad_output.device, "O and dO must be on the same device"
         assert o.dtype == grad_output.dtype, "O and dO must have the same dtype"
-        grad_output = _native.aligned(grad_output)
-        dq, dk1, dk2, dv1, dv2 = (torch.empty_like(q) for _ in range(5))
-        _native.dps_bwd(q, k1, k2, v1, v2, o, grad_output, m, dq, dk1, dk2, dv1, dv2, ctx.softmax_scale,
-                        ctx.causal, ctx.k_diff, flags=ctx.flags, fwd_ws=ctx.fwd_ws)
+        grads = _native.host_backward(_native.OP_DPS_BWD, q, k1, k2, v1, v2, o, grad_output, m, ctx.softmax_scale,
+                                      ctx.causal, ctx.flags, ctx.k_diff, ctx.fwd_ws)
+        if grads is not None:
+            grads = _native.host_result(grads, "tritt_dps_bwd")
+        else:
+            grad_output = _native.aligned(grad_output)
+            grads = tuple(torch.empty_like(q) for _ in range(5))
+            _native.dps_bwd(q, k1, k2, v1, v2, o, grad_output, m, *grads, ctx.softmax_scale,
+                            ctx.causal, ctx.k_diff, flags=ctx.flags, fwd_ws=ctx.fwd_ws)
         ctx.fwd_ws = None
-        return dq, dk1, dk2, dv1, dv2, None, None, None, None, None
+        return grads + (None,) * 5
 
 
 class TrittentionTriton(nn.Module):

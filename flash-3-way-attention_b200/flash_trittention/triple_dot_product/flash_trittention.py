@@ -42,13 +42,6 @@ class FlashTrittention(torch.autograd.Function):
                 convert_to_float32, *extra):
         # `extra`: at most one more positional argument, True for the exact-fp32 CUDA-core kernels
         # (``input_precision="ieee"`` of the functional entry point); the reference's signature ends before it
-        _validate(Q, K1, K2, V1, V2)
-        seq_len = Q.shape[2]
-        Q, K1, K2, V1, V2 = (_native.aligned(t) for t in (Q, K1, K2, V1, V2))
-        k1_window, k2_window, kk_left, kk_right = process_masking_variables(
-            seq_len, k1_window, k2_window, kk_left, kk_right)
-        O = torch.empty_like(Q)
-        lse = Q.new_empty(Q.shape[:3], dtype=torch.float32)
         # convert_to_float32 asks for fp32 operands inside the kernel, which the reference then feeds to TF32 dot
         # products: here bf16 inputs get operands of TF32's 11 significant bits (fp16 copies) on the tensor cores;
         # fp16 inputs have them already, fp32 inputs always run that way
@@ -56,8 +49,19 @@ class FlashTrittention(torch.autograd.Function):
         if extra and extra[0]:
             flags = _native.FLAG_FORCE_SIMT
         ctx.n_extra = len(extra)
-        _native.tdp_fwd(Q, K1, K2, V1, V2, O, lse, softmax_scale, causal, k1_window, k2_window, kk_left, kk_right,
-                        flags=flags)
+        out = _native.host_forward(_native.OP_TDP_FWD, Q, K1, K2, V1, V2, softmax_scale, causal, flags, k1_window,
+                                   k2_window, kk_left, kk_right)
+        if out is not None:
+            O, lse = _native.host_result(out, "tritt_tdp_fwd")
+        else:
+            _validate(Q, K1, K2, V1, V2)
+            Q, K1, K2, V1, V2 = (_native.aligned(t) for t in (Q, K1, K2, V1, V2))
+            k1_window, k2_window, kk_left, kk_right = process_masking_variables(
+                Q.shape[2], k1_window, k2_window, kk_left, kk_right)
+            O = torch.empty_like(Q)
+            lse = Q.new_empty(Q.shape[:3], dtype=torch.float32)
+            _native.tdp_fwd(Q, K1, K2, V1, V2, O, lse, softmax_scale, causal, k1_window, k2_window, kk_left, kk_right,
+                            flags=flags)
         ctx.save_for_backward(Q, K1, K2, V1, V2, O, lse)
         ctx.softmax_scale = softmax_scale
         ctx.windows = (k1_window, k2_window, kk_left, kk_right)
@@ -68,14 +72,19 @@ class FlashTrittention(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dO):
         Q, K1, K2, V1, V2, O, lse = ctx.saved_tensors
-        dO = _native.aligned(dO)
-        if dO.dtype != Q.dtype:
-            dO = dO.to(Q.dtype)
-        dq, dk1, dk2, dv1, dv2 = (torch.empty_like(Q) for _ in range(5))
         k1_window, k2_window, kk_left, kk_right = ctx.windows
-        _native.tdp_bwd(Q, K1, K2, V1, V2, O, dO, lse, dq, dk1, dk2, dv1, dv2, ctx.softmax_scale, ctx.causal,
-                        k1_window, k2_window, kk_left, kk_right, flags=ctx.flags)
-        return (dq, dk1, dk2, dv1, dv2, None, None, None, None, None, None, None) + (None,) * ctx.n_extra
+        grads = _native.host_backward(_native.OP_TDP_BWD, Q, K1, K2, V1, V2, O, dO, lse, ctx.softmax_scale, ctx.causal,
+                                      ctx.flags, k1_window, k2_window, kk_left, kk_right, None)
+        if grads is not None:
+            grads = _native.host_result(grads, "tritt_tdp_bwd")
+        else:
+            dO = _native.aligned(dO)
+            if dO.dtype != Q.dtype:
+                dO = dO.to(Q.dtype)
+            grads = tuple(torch.empty_like(Q) for _ in range(5))
+            _native.tdp_bwd(Q, K1, K2, V1, V2, O, dO, lse, *grads, ctx.softmax_scale, ctx.causal,
+                            k1_window, k2_window, kk_left, kk_right, flags=ctx.flags)
+        return grads + (None,) * (7 + ctx.n_extra)
 
 
 def flash_trittention(
