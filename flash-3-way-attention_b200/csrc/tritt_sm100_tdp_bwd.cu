@@ -34,11 +34,20 @@
 // steps: T=2048 D=128 bf16 16 heads 114.5 -> 94.9 ms, T=4096 D=64 4 heads 140.5 -> 113.8 ms, T=512 D=64 fp16 16 heads 2.37
 // -> 1.59 ms, windows 128/128/32/32 at T=2048 4.54 -> 1.77 ms.
 //
+// Narrow bands (kk_left + kk_right <= 72, head dimension 64, small scores): tdp_bwd_diag_kernel, the same kernel with steps over the
+// diagonals d = k - j.  On a diagonal A [j,h] = K1[j,h] K2[j+d,h] and A' alike, all else as above, except that row j of G and U
+// belongs to one row k = j + d of dK2 and dV2: nothing is summed over rows, and a step adds two tiles of 128 x 64 to the fp32 sums
+// (vector reductions; the SMs together take 5.8 TB/s of them, twice what a step asks for) where stepping over k adds two rows.  All
+// 128 x 128 of an item's cells lie in the band, of which a step over k has a band's width.  What bounds it: the fold warps, 4800
+// cycles a step (operands 1500, fold 3100) whose spills and exchanges between lanes count most.  us per backward, steps over k ->
+// diagonals: 16 heads T=2048 fp16 windows 128/128/32/32 951 -> 617, 256/256/40/20 1378 -> 840, 8/8/4/4 529 -> 170, 400/400/36/36
+// 1818 -> 1400; without windows, band 32/32 T=1024 1094 -> 715, 16/16 T=512 322 -> 146.
+//
 // Tile shapes: the accumulators S | dP | G | U | dQ have to fit 512 columns of tensor memory.  Head dimension 64:
 // JT = 128, G and U as [j x h] (128 + 128 + 64 + 64 + 64).  Head dimension 128: JT = 64 and G, U transposed,
 // [h x j], so that their M extent is 128 (64 + 64 + 64 + 64 + 128); a JT of 128 would need 640 columns.
 //
-// CTA: 20 warps.  0-3 and 4-7: soft-max warpgroups (half of a step's columns each, one query per thread); 8-11: forms
+// CTA: 20 warps (both kernels).  0-3 and 4-7: soft-max warpgroups (half of a step's columns each, one query per thread); 8-11: forms
 // A and folds G; 12-15: forms A' and folds U; 16, 18, 19: issue the products S and dP, U, dQ and G (large scores: 16 all five,
 // 18 and 19 form R); 17: TMA and the K2 / V2 rows.  P and dS are written to shared memory, where both the transposed (U, G) and the plain (dQ) product can read them.
 #include "tritt_sm100_tdp.cuh"
@@ -56,10 +65,12 @@ constexpr int kBwdThreads = 640;
 // twice.  (80 / 128 / 64 or 96 / 120 / 48 for soft-max, fold and service warps in the small-score body: 5 to 8 % slower, as their
 // loops spill.)
 constexpr int kRegsLaunch = 96;
+// (Diagonals: the fold warps need more, what the service warps can spare.  Band 128/128/32/32 at T=2048, soft-max / fold / service:
+// 88 / 128 / 48 757 us, 88 / 136 / 32 671, 80 / 136 / 48 731, 80 / 144 / 32 748; twice as many fold warps of 72 registers 930.)
 // (Large scores at head dimension 128 have the service warps form 32 KB of R per step, and soft-max warps that hold half as many
 // columns as at 64: with 48 registers those service warps spill, 1.60 -> 1.90 ms at 16 heads of T=512.)
-template <int D, bool LARGE> struct BwdRegs {
-  static constexpr int kSoftmax = D == 128 && LARGE ? 80 : 88, kFold = 128, kService = D == 128 && LARGE ? 64 : 48;
+template <int D, bool LARGE, bool DIAG> struct BwdRegs {
+  static constexpr int kSoftmax = D == 128 && LARGE ? 80 : 88, kFold = DIAG ? 136 : 128, kService = DIAG ? 32 : D == 128 && LARGE ? 64 : 48;
   static_assert(2 * kSoftmax + 2 * kFold + kService <= 5 * kRegsLaunch, "more registers than the launch has");
 };
 constexpr int kVecBatch = 4;     // K2 / V2 rows per hand-over
@@ -75,8 +86,11 @@ constexpr int kVecSlots = 4;     // batches in flight
 // closer to their bound.
 constexpr float kScoreBound = 16.f;
 constexpr int kStatParts = 32, kStatFloats = 8;
+// Rows of a window of K2 or V2 (128 + kk_left + kk_right at most): what shared memory has left beside one A' instead of two and without the K1
+// and SiLU(V1) tiles.
+constexpr int kDiagRows = 200;
 
-template <int D> struct BwdCfg {
+template <int D, bool DIAG = false> struct BwdCfg {
   static constexpr int JT = D == 64 ? 128 : 64;       // rows j of an item
   static constexpr int CW = JT / 2;                   // columns of one soft-max thread
   static constexpr int kTileQ = 128 * D * 2;          // Q, dO
@@ -85,13 +99,15 @@ template <int D> struct BwdCfg {
   static constexpr int kOffQ = 0;
   static constexpr int kOffDO = kOffQ + kTileQ;
   static constexpr int kOffK1 = kOffDO + kTileQ;      // K1 | SiLU(V1)
-  static constexpr int kOffA = kOffK1 + 2 * kTileJ;   // A (two buffers) | A'
+  // DIAG: windows of K2 and V2 rows instead (K1 and SiLU(V1) go straight to the registers that keep them)
+  static constexpr int kWindow = kDiagRows * D * 2;
+  static constexpr int kOffA = kOffK1 + (DIAG ? 2 * kWindow : 2 * kTileJ);   // A (two buffers) | A'
   static constexpr int kOffP = kOffA + 3 * kTileJ;    // P | dS (two buffers)
   // R (see tdp_bwd_body), in blocks of 64 columns: over the SiLU(V1) tile, and behind P | dS
   static constexpr int kOffR0 = kOffK1 + kTileJ, kOffR1 = kOffP + 3 * kTileP;
   static constexpr int kOffVec = kOffR1 + (D / 64 - 1) * 16384;  // [slot][K2 rows | V2 rows][row of the batch][D], 16-bit
   static constexpr int kVecPart = kVecBatch * D * 2;  // bytes of a batch of rows of one tensor
-  static constexpr int kOffBars = kOffVec + kVecSlots * 2 * kVecPart;
+  static constexpr int kOffBars = kOffVec + (DIAG ? 0 : kVecSlots * 2 * kVecPart);
   static constexpr int kSmem = kOffBars + 512;
   static constexpr int kTmemS = 0, kTmemDP = JT, kTmemG = 2 * JT, kTmemU = kTmemG + 64, kTmemDQ = kTmemU + 64;
   static constexpr int kTmemQ = kTmemDQ + D, kTmemDO = kTmemQ + D / 2;   // 16-bit, two elements a column
@@ -109,6 +125,7 @@ struct BwdGeometry {
   int k1w, k2w, kkl, kkr;  // windows of the causal mask (T or more = unbounded)
   int JT;                  // rows of a j-tile
   int stride, lead;        // tile jt has the rows from jt * stride - lead on
+  bool diagonals;          // steps are the diagonals d = k - j, counted from -kkr
   __host__ __device__ int q_tiles() const { return (nq + 127) / 128; }
   __host__ __device__ int first_q(int qt) const { return q_rem + qt * 128 * q_mod; }
   __host__ __device__ int last_q(int qt) const {
@@ -123,6 +140,10 @@ struct BwdGeometry {
   }
   __host__ __device__ int j_first(int qt) const {
     if (overlapping()) return k_first(first_q(qt)) / stride;
+    if (diagonals) {
+      const int reach = k1w < k2w + kkl ? k1w : k2w + kkl, qa = first_q(qt);
+      return qa > reach ? (qa - reach) / JT : 0;
+    }
     const int lo = first_q(qt) - k1w;
     return causal && lo > 0 ? lo / JT : 0;
   }
@@ -138,6 +159,14 @@ struct BwdGeometry {
       return k1 >= k0 ? k1 - k0 + 1 : 0;
     }
     const int ja = jt * JT, jb = ja + JT - 1;
+    if (diagonals) {   // 0 <= j + d <= q,  q - k2w <= j + d
+      int d0 = qa - k2w - jb, d1 = qb - ja;
+      if (d0 < -jb) d0 = -jb;
+      if (d0 < -kkr) d0 = -kkr;
+      if (d1 > kkl) d1 = kkl;
+      k0 = d0 + kkr;
+      return d1 >= d0 ? d1 - d0 + 1 : 0;
+    }
     if (qa - k2w > k0) k0 = qa - k2w;
     if (ja - kkr > k0) k0 = ja - kkr;
     const int k1 = qb < jb + kkl ? qb : jb + kkl;
@@ -146,7 +175,7 @@ struct BwdGeometry {
 };
 
 struct BwdParams {
-  const void *q, *d_o, *k2, *v2;
+  const void *q, *d_o, *k2, *v2, *k1, *sv1;
   const float *lse, *drow;
   const float* stats;      // [BN][stat_parts][kStatFloats] (see tdp_bwd_prepare_kernel), or null
   int stat_parts;
@@ -156,6 +185,7 @@ struct BwdParams {
   int i_first;             // query rows (of the shard) before this one are not this kernel's
   long head_steps;         // steps of one head
   float alpha;
+  bool diag_asked;         // the kernel that steps over diagonals is ahead of this one, and does the call if all scores are small
   int* status;
 };
 
@@ -346,12 +376,24 @@ __device__ __forceinline__ bool large_scores(const BwdParams& p) {
   return __syncthreads_or(large);
 }
 
+// Whether all scores of the call are small (the same for every thread).
+__device__ __forceinline__ bool all_scores_small(const BwdParams& p) {
+  bool large = false;
+  for (int bh = threadIdx.x >> 5; bh < p.BN; bh += kBwdThreads / 32) {
+    const BwdStats st = head_stats(p, bh, threadIdx.x & 31);
+    large |= !(fabsf(p.alpha * kLog2e) * sqrtf(st.k1_row * st.q_row) * st.k2 <= kScoreBound);
+  }
+  return !__syncthreads_or(large);
+}
+
 // LARGE: S = R K1^T with R [q,h] = alpha*log2(e) * Q[q,h] * K2[k,h] instead of S = Q A^T (see kScoreBound).
-template <int D, typename T16, bool LARGE>
+template <int D, typename T16, bool LARGE, bool DIAG = false>
 __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUtensorMap& tmDO, const CUtensorMap& tmK1,
                                              const CUtensorMap& tmSV1, const BwdParams& p) {
-  using Cfg = BwdCfg<D>;
+  using Cfg = BwdCfg<D, DIAG>;
   constexpr int JT = Cfg::JT, CW = Cfg::CW;
+  constexpr bool kOneAp = LARGE || DIAG;   // a single buffer of A'
+  static_assert(!DIAG || (D == 64 && !LARGE), "steps over diagonals: head dimension 64, small scores");
   extern __shared__ __align__(1024) uint8_t smem[];
   static_assert(sizeof(BwdBarriers) <= 512, "barrier block too large");
   BwdBarriers& bars = *reinterpret_cast<BwdBarriers*>(smem + Cfg::kOffBars);
@@ -437,7 +479,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
   };
 
   if (warp < 8) {
-    set_regs<kRegsLaunch, BwdRegs<D, LARGE>::kSoftmax>();
+    set_regs<kRegsLaunch, BwdRegs<D, LARGE, DIAG>::kSoftmax>();
     // ------------------------------------------------------------------ soft-max warpgroups
     const int wg = warp >> 2, wq = warp & 3;
     const int row = wq * 32 + lane;
@@ -508,7 +550,11 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
         const int k = it.k0 + i;
         // columns this query sees at this k, relative to the thread's first: [lo, hi] (empty: hi < lo)
         int lo = -j0, hi = T - 1 - j0;
-        if (g.causal) {
+        if (DIAG) {   // (k counts diagonals from -kkr)
+          const int d = k - g.kkr;
+          lo = max(max(q - g.k1w, q - d - g.k2w), max(0, -d)) - j0;
+          hi = min(q, q - d) - j0;
+        } else if (g.causal) {
           lo = max(max(q - g.k1w, k - g.kkl), 0) - j0;   // (an overlapping tile may begin ahead of row 0)
           hi = k <= q && q - k <= g.k2w ? min(q, k + g.kkr) - j0 : lo - 1;
         }
@@ -706,7 +752,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       }
     }
   } else if (warp < 16) {
-    set_regs<kRegsLaunch, BwdRegs<D, LARGE>::kFold>();
+    set_regs<kRegsLaunch, BwdRegs<D, LARGE, DIAG>::kFold>();
     // ------------------------------------------------------------------ operand / fold warpgroups
     // role 0: forms A two steps ahead, folds G into dK1 (registers) and dK2;  role 1: forms A' two steps ahead (large scores: one), folds
     // U into dSiLU(V1) and dV2.  The fold reads the accumulator as 16 x 256-bit fragments (thread t: rows t / 4 + 8 i,
@@ -721,7 +767,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       return vec + ((vb0 + i / kVecBatch) % kVecSlots * 2 * kVecBatch + i % kVecBatch) * D;
     };
     const uint32_t tacc = tmem + ((uint32_t)(w * 32) << 16) + (role ? Cfg::kTmemU : Cfg::kTmemG);
-    const int ahead = LARGE ? 2 - role : 2;   // (A' has a second buffer, over the SiLU(V1) tile, where R does not need that)
+    const int ahead = kOneAp ? 2 - role : 2;   // (A' has a second buffer, over the SiLU(V1) tile, where R does not need that)
     // address of this lane's row of the four 8 x 8 blocks of (16-column group c16, 16-lane half hl) within a tile
     auto frag = [&](int c16, int hl) -> uint32_t {
       if constexpr (D == 64) {
@@ -732,6 +778,11 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
         const int ch = w * 4 + hl * 2 + ((lane >> 3) & 1), j = c16 * 16 + (lane >> 4) * 8 + (lane & 7);
         return (ch >> 3) * (JT * 128) + swz128(j, ch & 7);
       }
+    };
+    // (DIAG: row j of the tile meets row k = j + n - kkr on diagonal n, which is row j + n of the window)
+    const uint32_t window_u = smem_u32(smem + Cfg::kOffK1 + role * Cfg::kWindow);
+    auto window_frag = [&](int n, int c16, int hl) -> uint32_t {
+      return window_u + swz128(w * 32 + hl * 16 + (lane & 15) + n, c16 * 2 + (lane >> 4));
     };
     const uint32_t raw_u = smem_u32(smem + Cfg::kOffK1 + role * Cfg::kTileJ);
     const uint32_t formed_u = smem_u32(smem + Cfg::kOffA + role * 2 * Cfg::kTileJ);
@@ -747,10 +798,17 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       for (int c16 = 0; c16 < 4; ++c16)
 #pragma unroll
         for (int hl = 0; hl < 2; ++hl) {
-          if constexpr (D == 64) ldmatrix_x4(x[c16][hl], raw_u + frag(c16, hl));
+          if constexpr (DIAG) {
+            const T16* src = (const T16*)(role ? p.sv1 : p.k1) + (size_t)it.bh * T * D + c16 * 16 + 2 * (lane & 3);
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+              const int j = it.jt * JT + w * 32 + hl * 16 + (b & 1) * 8 + (lane >> 2);
+              x[c16][hl][b] = j < T ? __ldg(reinterpret_cast<const uint32_t*>(src + (size_t)j * D + (b >> 1) * 8)) : 0u;
+            }
+          } else if constexpr (D == 64) ldmatrix_x4(x[c16][hl], raw_u + frag(c16, hl));
           else ldmatrix_x4_trans(x[c16][hl], raw_u + frag(c16, hl));
         }
-      arrive_warp(&bars.tile_free);
+      if (!DIAG) arrive_warp(&bars.tile_free);
       const int ex = role ? it.eb : it.ea;   // (x carries 2^ex from here on)
       if (std::is_same<T16, __half>::value) {
         const float2 m = make_float2(pow2i<T16>(ex), pow2i<T16>(ex));
@@ -769,23 +827,48 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       const float jscale = role ? unshift : unshift_ds * p.alpha;
       const float zscale = jscale * pow2i<T16>(-ex);
       float* zrow = (role ? p.dv2 : p.dk2) + ((size_t)it.bh * T + it.k0) * D;
+      // (DIAG: only rows k that a query of the tile sees: the others' products are zero, or NaN beside an infinite row)
+      int k_row0 = 0;
+      unsigned k_rows = 0;
+      if (DIAG) {
+        const int k_lo = max(0, it.qt * 128 - g.k2w);
+        k_row0 = it.jt * JT - g.kkr + it.k0 + w * 32 + (lane >> 2) - k_lo;
+        k_rows = (unsigned)(min(it.qt * 128 + 128, T) - k_lo);
+      }
+      if (DIAG) zrow += (ptrdiff_t)(it.jt * JT - g.kkr + w * 32 + (lane >> 2)) * D + ((lane & 1) << 3) + ((lane & 2) << 1);
       auto form = [&](int i) -> bool {
         const uint32_t m = n + i;
         // The operand's buffer: the product of its last step has run (A: two steps before, through dQ; A': dP, two steps before,
         // or with a single buffer the step before).  At the first row of a batch half of the lanes look whether it is there.
-        const uint32_t mb = LARGE && role ? m - 1 : m, vb = vb0 + i / kVecBatch;
+        const uint32_t mb = kOneAp && role ? m - 1 : m, vb = vb0 + i / kVecBatch;
         uint64_t* const bar = role ? &bars.ap_free[mb & 1] : &bars.a_free[mb & 1];
-        const uint32_t parity = ((mb >> 1) & 1) ^ (LARGE && role ? 0 : 1);
-        const bool first = (i & (kVecBatch - 1)) == 0;
+        const uint32_t parity = ((mb >> 1) & 1) ^ (kOneAp && role ? 0 : 1);
+        const bool first = !DIAG && (i & (kVecBatch - 1)) == 0;
         if (!wait_two(bar, parity, first ? &bars.vec_full[vb % kVecSlots] : bar, first ? (vb / kVecSlots) & 1 : parity)) return false;
         const T16* v = vec_row(vb0, i);
-        const uint32_t dst = role == 0 ? formed_u + (m & 1) * Cfg::kTileJ : LARGE || !(m & 1) ? formed_u : raw_u;
+        const uint32_t dst = role == 0 ? formed_u + (m & 1) * Cfg::kTileJ : kOneAp || !(m & 1) ? formed_u : raw_u;
         uint32_t vr[4];   // head dimension 128: twice the element of row r
         if constexpr (D == 128) {
 #pragma unroll
           for (int r = 0; r < 4; ++r)
             vr[r] = __byte_perm(*reinterpret_cast<const uint16_t*>(v + w * 32 + r * 8 + (lane >> 2)), 0, 0x1010);
         }
+        if constexpr (DIAG) {
+          // (two fragments at a time, or each read waits for the store before; four spill)
+#pragma unroll
+          for (int c = 0; c < 8; c += 2) {
+            uint32_t a[2][4];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) ldmatrix_x4(a[e], window_frag(it.k0 + i, (c + e) >> 1, (c + e) & 1));
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int c16 = (c + e) >> 1, hl = (c + e) & 1;
+#pragma unroll
+              for (int b = 0; b < 4; ++b) a[e][b] = mul2<T16>(x[c16][hl][b], a[e][b]);
+              stmatrix_x4(dst + frag(c16, hl), a[e]);
+            }
+          }
+        } else
 #pragma unroll
         for (int c16 = 0; c16 < 4; ++c16) {
           uint32_t v0 = 0, v1 = 0;
@@ -803,7 +886,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
           }
         }
         fence_async_smem();
-        arrive_warp(role ? &bars.ap_ready[LARGE ? 0 : m & 1] : &bars.a_ready[m & 1]);
+        arrive_warp(role ? &bars.ap_ready[kOneAp ? 0 : m & 1] : &bars.a_ready[m & 1]);
         return true;
       };
       // (one loop, so that there is one copy of each of the two stages: step i0 forms operand i0, folds step i0 - ahead)
@@ -825,7 +908,47 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
         if (!alive) break;
         tc_fence_after();
         const T16* v = vec_row(vb0, i);
-        if constexpr (D == 64) {
+        if constexpr (DIAG) {
+          // Lanes are rows j, columns are h; row k = j + d of dK2 / dV2 gets K1 G / SiLU(V1) U.  Pairs of lanes swap halves, so that
+          // a reduction takes four columns of a thread (with two of them, without exchanges, 820 us where this took 757).  Eight
+          // rows by 16 columns at a time: with 16 by 16 the registers in flight spill (671 us for 642).
+          const int k = k_row0 + i;   // from the first row that a query of the tile sees
+          const bool odd = lane & 1;
+          const float2 zs = make_float2(zscale, zscale);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const int c16 = c >> 1, hl = c & 1;
+            uint32_t d[8], vw[4];
+            tmem_ld_16x256b_x2(tacc + ((uint32_t)(hl * 16) << 16) + c16 * 16, d);
+            ldmatrix_x4(vw, window_frag(it.k0 + i, c16, hl));
+            tmem_wait_ld();
+            if (c == 7) {
+              tc_fence_before();
+              arrive_warp(&bars.acc_free[role]);
+            }
+            // (all exchanges ahead of the reductions: one waits for the other's answer else)
+            float2 z0[2], z1[2], other[2];
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              const float2 g0 = make_float2(__uint_as_float(d[2 * r]), __uint_as_float(d[2 * r + 1]));
+              const float2 g1 = make_float2(__uint_as_float(d[4 + 2 * r]), __uint_as_float(d[5 + 2 * r]));
+              z0[r] = __fmul2_rn(__fmul2_rn(g0, unpack2<T16>(x[c16][hl][r])), zs);
+              z1[r] = __fmul2_rn(__fmul2_rn(g1, unpack2<T16>(x[c16][hl][2 + r])), zs);
+              other[r].x = __shfl_xor_sync(0xffffffffu, odd ? z0[r].x : z1[r].x, 1);
+              other[r].y = __shfl_xor_sync(0xffffffffu, odd ? z0[r].y : z1[r].y, 1);
+              float2& a0 = acc[c16 * 8 + hl * 4 + r];
+              float2& a1 = acc[c16 * 8 + hl * 4 + 2 + r];
+              a0 = __ffma2_rn(g0, unpack2<T16>(vw[r]), a0);
+              a1 = __ffma2_rn(g1, unpack2<T16>(vw[2 + r]), a1);
+            }
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              const float2 o = other[r], u = z0[r], v = z1[r];
+              if ((unsigned)(k + hl * 16 + r * 8) < k_rows)
+                red_add4(zrow + (hl * 16 + r * 8) * D + c16 * 16, odd ? o.x : u.x, odd ? o.y : u.y, odd ? v.x : o.x, odd ? v.y : o.y);
+            }
+          }
+        } else if constexpr (D == 64) {
           // lanes are rows j, columns are h
           float z2[8];
 #pragma unroll
@@ -928,11 +1051,12 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
           }
           red_add(zrow + w * 32 + (lane & 3) * 8 + (lane >> 2), zr[0] * zscale);
         }
-        if ((i & (kVecBatch - 1)) == kVecBatch - 1 || i == len - 1)
+        if (!DIAG && ((i & (kVecBatch - 1)) == kVecBatch - 1 || i == len - 1))
           arrive_warp(&bars.vec_empty[(vb0 + i / kVecBatch) % kVecSlots]);
         zrow += D;
       }
       if (!alive) break;
+      if (DIAG) arrive_warp(&bars.tile_free);   // (the window has been read)
       n += len;
       vb0 += (len + kVecBatch - 1) / kVecBatch;
       ++items;
@@ -959,7 +1083,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
             }
     }
   } else {
-   set_regs<kRegsLaunch, BwdRegs<D, LARGE>::kService>();
+   set_regs<kRegsLaunch, BwdRegs<D, LARGE, DIAG>::kService>();
    if (warp == 16 || (!LARGE && warp >= 18)) {
     const bool do_rows = warp == 16, do_u = LARGE || warp == 18, do_ds = LARGE || warp == 19;
     // ------------------------------------------------------------------ MMA issuer
@@ -1028,11 +1152,11 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
     };
     // (the first step of an item has no dP before it that anyone still reads)
     auto issue_dp = [&](uint32_t m, bool after) -> bool {
-      uint64_t* const ap = &bars.ap_ready[LARGE ? 0 : m & 1];
-      const uint32_t parity = (LARGE ? m : m >> 1) & 1;
+      uint64_t* const ap = &bars.ap_ready[kOneAp ? 0 : m & 1];
+      const uint32_t parity = (kOneAp ? m : m >> 1) & 1;
       if (!wait_two(ap, parity, after ? &bars.ds_ready[(m - 1) & 1] : ap, after ? ((m - 1) >> 1) & 1 : parity)) return false;
       tc_fence_after();
-      issue_rows(Cfg::kTmemDP, Cfg::kTmemDO, LARGE || !(m & 1) ? a2Lo : sv1Lo);
+      issue_rows(Cfg::kTmemDP, Cfg::kTmemDO, kOneAp || !(m & 1) ? a2Lo : sv1Lo);
       commit(&bars.dp_ready);
       commit(&bars.ap_free[m & 1]);
       return true;
@@ -1125,12 +1249,18 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
         break;
       }
       if (leader) {
-        mbar_arrive_expect_tx(&bars.tile_full, ((it.flags & kFirstOfQ) ? 2 * Cfg::kTileQ : 0) + 2 * Cfg::kTileJ);
+        mbar_arrive_expect_tx(&bars.tile_full, ((it.flags & kFirstOfQ) ? 2 * Cfg::kTileQ : 0) +
+                                                   (DIAG ? 2 * (128 + g.kkl + g.kkr) * D * 2 : 2 * Cfg::kTileJ));
 #pragma unroll
         for (int b = 0; b < D / 64; ++b) {
           if ((it.flags & kFirstOfQ)) {
             tma_load_3d(smem + Cfg::kOffQ + b * 16384, &tmQ, &bars.tile_full, b * 64, it.qt * 128, it.bh);
             tma_load_3d(smem + Cfg::kOffDO + b * 16384, &tmDO, &bars.tile_full, b * 64, it.qt * 128, it.bh);
+          }
+          if constexpr (DIAG) {   // (maps of K2 and V2)
+            tma_load_3d(smem + Cfg::kOffK1, &tmK1, &bars.tile_full, 0, it.jt * JT - g.kkr, it.bh);
+            tma_load_3d(smem + Cfg::kOffK1 + Cfg::kWindow, &tmSV1, &bars.tile_full, 0, it.jt * JT - g.kkr, it.bh);
+            continue;
           }
           tma_load_3d(smem + Cfg::kOffK1 + b * JT * 128, &tmK1, &bars.tile_full, b * 64, g.j_row(it.jt), it.bh);
           tma_load_3d(smem + Cfg::kOffK1 + Cfg::kTileJ + b * JT * 128, &tmSV1, &bars.tile_full, b * 64, g.j_row(it.jt), it.bh);
@@ -1138,6 +1268,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       }
       in_flight = true;
       ++items;
+      if (DIAG) continue;
       // K2 / V2 rows, a batch at a time (the last one of an item may be shorter)
       const size_t head = ((size_t)it.bh * T + it.k0) * D;
       for (int i = 0; i < it.len; i += kVecBatch, ++vb) {
@@ -1248,8 +1379,25 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                const __grid_constant__ CUtensorMap tmK1, const __grid_constant__ CUtensorMap tmSV1,
                const __grid_constant__ BwdParams p) {
+  if (p.diag_asked && all_scores_small(p)) {
+    if (threadIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");   // (as at the body's end)
+    return;
+  }
   if (large_scores(p)) tdp_bwd_body<D, T16, true>(tmQ, tmDO, tmK1, tmSV1, p);
   else tdp_bwd_body<D, T16, false>(tmQ, tmDO, tmK1, tmSV1, p);
+}
+
+template <typename T16>
+__global__ void __launch_bounds__(kBwdThreads, 1)
+tdp_bwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
+                    const __grid_constant__ CUtensorMap tmK2, const __grid_constant__ CUtensorMap tmV2,
+                    const __grid_constant__ BwdParams p) {
+  asm volatile("griddepcontrol.launch_dependents;");   // (tdp_bwd_kernel, which needs nothing of this one)
+  if (all_scores_small(p)) {
+    tdp_bwd_body<64, T16, false, true>(tmQ, tmDO, tmK2, tmV2, p);
+  } else if (threadIdx.x == 0) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // (as at the body's end)
+  }
 }
 
 // What the kernel needs before it starts, in one pass over the tensors (8 elements per thread and step): zeroed fp32
@@ -1393,13 +1541,13 @@ int check_registers(int launched) {
   return -30;
 }
 
-template <int D, typename T16, typename K>
-int check_kernel_registers(K kern) {
+template <auto kKernel>
+int check_kernel_registers() {
   static std::atomic<int> launched{0};   // (per kernel: a property of the compiled code, the same on every device)
   int n = launched.load(std::memory_order_relaxed);
   if (n == 0) {
     cudaFuncAttributes attr;
-    TRITT_CUDA_OK(cudaFuncGetAttributes(&attr, kern));
+    TRITT_CUDA_OK(cudaFuncGetAttributes(&attr, kKernel));
     n = attr.numRegs;
     launched.store(n, std::memory_order_relaxed);
   }
@@ -1424,6 +1572,8 @@ struct BwdPlan {
   BwdGeometry g;
   int i_first;        // query rows (of the shard) that the CUDA cores take, in exact fp32
   long head_steps;    // steps of the kernel per head
+  BwdGeometry diag;   // the steps of the kernel that steps over diagonals, if diag_steps > 0
+  long diag_steps;
   bool by_queries;    // the kernel that steps over queries instead: every row is its, as items of its own
   long long cells;    // cells (q, j, k) executed per head
 };
@@ -1443,6 +1593,12 @@ constexpr double kCellPrice = 0.8;
 constexpr long kItemSteps = 3;
 constexpr int kMinStride = 8;
 
+// Diagonals are taken where they are fewer by more than a step's higher price and a launch.  Steps and items of a CTA, k / diagonals: us
+// with k / diagonals, D=64:  140 / 123: 325 / 350, 74 / 62: 192 / 195, 30 / 25: 98 / 104, 1.4 / 0.3: 75 / 76, 15 / 9: 75 / 77,
+// 24 / 9: 87 / 79, 41 / 26: 124 / 110, 31 / 3: 104 / 76, 45 / 9: 135 / 80, 54 / 28: 146 / 114, 449 / 228: 951 / 617, 871 / 548: 1818 / 1400.
+// Calls with large scores pay for a kernel that does nothing: 449 / 228: 1051 / 1060, 82 / 12: 218 / 223.
+constexpr double kDiagPrice = 1.3, kDiagGain = 6;
+
 // Steps and items of one head.
 long count_steps(const BwdGeometry& g, long& items) {
   long steps = 0;
@@ -1461,7 +1617,7 @@ template <int D> BwdPlan make_plan(const TdpArgs& a) {
   BwdPlan p{};
   const int nq = a.q_rem < a.T ? (a.T - a.q_rem + a.q_mod - 1) / a.q_mod : 0;
   constexpr int JT = BwdCfg<D>::JT;
-  p.g = BwdGeometry{a.T, nq, a.q_mod, a.q_rem, a.mask.causal, a.mask.k1w, a.mask.k2w, a.mask.kkl, a.mask.kkr, JT, JT, 0};
+  p.g = BwdGeometry{a.T, nq, a.q_mod, a.q_rem, a.mask.causal, a.mask.k1w, a.mask.k2w, a.mask.kkl, a.mask.kkr, JT, JT, 0, false};
   if (nq == 0) return p;
   const int first = tdp_bwd_first_count(a.T);
   const long long pairs = (min(a.mask.k1w, a.T - 1) + 1LL) * (min(a.mask.k2w, a.T - 1) + 1LL);   // (at most, of any query)
@@ -1485,6 +1641,17 @@ template <int D> BwdPlan make_plan(const TdpArgs& a) {
       p.g = o;
       p.head_steps = o_steps;
     }
+  }
+  if (D == 64 && a.mask.causal && a.q_mod == 1 && 128 + a.mask.kkl + a.mask.kkr <= kDiagRows) {
+    p.diag = p.g;
+    p.diag.stride = JT;
+    p.diag.lead = 0;
+    p.diag.diagonals = true;
+    long d_items, k_items;
+    const long d_steps = count_steps(p.diag, d_items);
+    count_steps(p.g, k_items);
+    const double less = (double)(p.head_steps + kItemSteps * k_items) - kDiagPrice * (double)(d_steps + kItemSteps * d_items);
+    if (less * a.B * a.N >= kDiagGain * num_sms()) p.diag_steps = d_steps;
   }
   p.cells = (long long)p.head_steps * 128 * BwdCfg<D>::JT;
   if (a.q_mod > 1) {
@@ -1521,7 +1688,7 @@ int launch_bwd_sums(const TdpArgs& a, const BwdPlan& plan) {
   BwdParams p{};
   p.stats = stats;
   p.stat_parts = parts;
-  p.q = a.q; p.d_o = a.d_o; p.k2 = a.k2; p.v2 = a.v2; p.lse = a.lse_in; p.drow = drow;
+  p.q = a.q; p.d_o = a.d_o; p.k2 = a.k2; p.v2 = a.v2; p.k1 = a.k1; p.sv1 = sv1; p.lse = a.lse_in; p.drow = drow;
   p.dk1 = sums; p.dk2 = sums + n; p.dsv1 = sums + 2 * n; p.dv2 = sums + 3 * n; p.dq = sums + 4 * n;
   p.BN = BN;
   p.alpha = a.alpha;
@@ -1536,34 +1703,51 @@ int launch_bwd_sums(const TdpArgs& a, const BwdPlan& plan) {
     if (rc) return rc;
   }
   if (p.head_steps == 0) return 0;
-  const long total = p.head_steps * BN, sms = num_sms();   // (equal parts of the whole line of steps)
-  const int grid = (int)(total < sms ? total : sms);
-  CUtensorMap tmQ, tmDO, tmK1, tmSV1;
+  CUtensorMap tmQ, tmDO, tmK1, tmSV1, tmK2, tmV2;
   int rc;
   const size_t shard = (size_t)a.q_rem * D;   // first query row of the shard
   if ((rc = make_tmap_rows(&tmQ, (const T16*)a.q + shard, D, nq, BN, (uint64_t)a.q_mod * D, (uint64_t)a.T * D, 128))) return rc;
   if ((rc = make_tmap_rows(&tmDO, (const T16*)a.d_o + shard, D, nq, BN, (uint64_t)a.q_mod * D, (uint64_t)a.T * D, 128))) return rc;
   if ((rc = make_tmap_3d(&tmK1, a.k1, 2, D, a.T, BN, 64, Cfg::JT))) return rc;
   if ((rc = make_tmap_3d(&tmSV1, sv1, 2, D, a.T, BN, 64, Cfg::JT))) return rc;
-  auto kern = tdp_bwd_kernel<D, T16>;
-  if ((rc = check_kernel_registers<D, T16>(kern))) return rc;
-  TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
   // With exact first queries ahead of it the kernel starts as soon as all their blocks have: it needs the preparation pass,
   // which was done before they began, and nothing of theirs (both add to the sums).  us per backward
   // with this / one after the other: T=333 D=128 4 heads 192 / 198, T=128 D=64 64 heads 171 / 181, T=60 D=64 2 heads 29 / 35.
-  cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.gridDim = dim3((unsigned)grid, 1, 1);
-  cfg.blockDim = dim3(kBwdThreads, 1, 1);
-  cfg.dynamicSmemBytes = Cfg::kSmem;
-  cfg.stream = a.stream;
-  cfg.attrs = attr;
-  cfg.numAttrs = plan.i_first > 0 ? 1 : 0;
-  TRITT_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tmQ, tmDO, tmK1, tmSV1, p));
-  count_launch();
-  return 0;
+  auto launch = [&](auto kern, int smem_bytes, long steps, bool early, const CUtensorMap& m2, const CUtensorMap& m3) -> int {
+    TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
+    const long total = steps * BN, sms = num_sms();   // (equal parts of the whole line of steps)
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3((unsigned)(total < sms ? total : sms), 1, 1);
+    cfg.blockDim = dim3(kBwdThreads, 1, 1);
+    cfg.dynamicSmemBytes = smem_bytes;
+    cfg.stream = a.stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = early ? 1 : 0;
+    TRITT_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tmQ, tmDO, m2, m3, p));
+    count_launch();
+    return 0;
+  };
+  bool early = plan.i_first > 0;
+  if constexpr (D == 64) {
+    if (plan.diag_steps > 0 && stats) {
+      const uint32_t rows = 128 + a.mask.kkl + a.mask.kkr;
+      if ((rc = make_tmap_3d(&tmK2, a.k2, 2, D, a.T, BN, 64, rows))) return rc;
+      if ((rc = make_tmap_3d(&tmV2, a.v2, 2, D, a.T, BN, 64, rows))) return rc;
+      if ((rc = check_kernel_registers<tdp_bwd_diag_kernel<T16>>())) return rc;
+      p.g = plan.diag;
+      p.head_steps = plan.diag_steps;
+      if ((rc = launch(tdp_bwd_diag_kernel<T16>, BwdCfg<D, true>::kSmem, plan.diag_steps, early, tmK2, tmV2))) return rc;
+      p.g = plan.g;
+      p.head_steps = plan.head_steps;
+      p.diag_asked = true;
+      early = true;
+    }
+  }
+  if ((rc = check_kernel_registers<tdp_bwd_kernel<D, T16>>())) return rc;
+  return launch(tdp_bwd_kernel<D, T16>, Cfg::kSmem, plan.head_steps, early, tmK1, tmSV1);
 }
 
 template <typename T16>
