@@ -40,7 +40,7 @@
 // (vector reductions; the SMs together take 5.8 TB/s of them, twice what a step asks for) where stepping over k adds two rows.  All
 // 128 x 128 of an item's cells lie in the band, of which a step over k has a band's width.  What bounds it: the fold warps, 4800
 // cycles a step (operands 1500, fold 3100) whose spills and exchanges between lanes count most.  us per backward, steps over k ->
-// diagonals: 16 heads T=2048 fp16 windows 128/128/32/32 951 -> 617, 256/256/40/20 1378 -> 840, 8/8/4/4 529 -> 170, 400/400/36/36
+// diagonals: 16 heads T=2048 fp16 windows 128/128/32/32 951 -> 615, 256/256/40/20 1378 -> 830, 8/8/4/4 529 -> 164, 400/400/36/36
 // 1818 -> 1400; without windows, band 32/32 T=1024 1094 -> 715, 16/16 T=512 322 -> 146.
 //
 // Tile shapes: the accumulators S | dP | G | U | dQ have to fit 512 columns of tensor memory.  Head dimension 64:
@@ -647,6 +647,12 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
           const uint32_t tS = tmem + lane_base + Cfg::kTmemS + wg * CW, tDP = tmem + lane_base + Cfg::kTmemDP + wg * CW;
           constexpr int SN = D == 128 ? H : 8;   // (head dimension 64 has no registers for all of them)
           uint32_t s[H], sn[SN], dp[8];   // scores, then P; scores of the second half; dP
+          // (most steps over a diagonal are masked: a bit of a mask is one instruction, two comparisons are two)
+          uint32_t mask[2] = {0, 0};
+          if constexpr (DIAG) {
+            mask[0] = column_mask(lo, hi);
+            mask[1] = column_mask(lo - 32, hi - 32);
+          }
           // columns c.. of S -> P
           auto to_p = [&](int c, uint32_t* v, const uint32_t* x) {
             if (full) {
@@ -655,6 +661,14 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
                 const float2 y = scaled(x[e], x[e + 1], sa, nlse);
                 v[e] = __float_as_uint(exp2f(y.x));
                 v[e + 1] = __float_as_uint(exp2f(y.y));
+              }
+            } else if constexpr (DIAG) {
+#pragma unroll
+              for (int e = 0; e < 8; e += 2) {
+                const uint32_t m = mask[c >> 5] >> ((c + e) & 31);
+                const float2 y = scaled(x[e], x[e + 1], sa, nlse);
+                v[e] = m & 1u ? __float_as_uint(exp2f(y.x)) : 0u;
+                v[e + 1] = m & 2u ? __float_as_uint(exp2f(y.y)) : 0u;
               }
             } else {
 #pragma unroll
@@ -1598,7 +1612,7 @@ constexpr int kMinStride = 8;
 
 // Diagonals are taken where they are fewer by more than a step's higher price and a launch.  Steps and items of a CTA, k / diagonals: us
 // with k / diagonals, D=64:  140 / 123: 325 / 350, 74 / 62: 192 / 195, 30 / 25: 98 / 104, 1.4 / 0.3: 75 / 76, 15 / 9: 75 / 77,
-// 24 / 9: 87 / 79, 41 / 26: 124 / 110, 31 / 3: 104 / 76, 45 / 9: 135 / 80, 54 / 28: 146 / 114, 449 / 228: 951 / 617, 871 / 548: 1818 / 1400.
+// 24 / 9: 87 / 79, 41 / 26: 124 / 110, 31 / 3: 104 / 76, 45 / 9: 135 / 80, 54 / 28: 146 / 114, 449 / 228: 951 / 615, 871 / 548: 1818 / 1400.
 // Calls with large scores pay for a kernel that does nothing: 449 / 228: 1051 / 1060, 82 / 12: 218 / 223.
 constexpr double kDiagPrice = 1.3, kDiagGain = 6;
 
