@@ -66,6 +66,11 @@ template <typename T16> __device__ __forceinline__ float pow2i(int e) {
   return std::is_same<T16, __half>::value ? __int_as_float((127 + e) << 23) : 1.f;
 }
 
+// The soft-max reference of all rows of a head, from the bound on its scores: P = exp2(S - reference) is below 2^15 in fp16, 1 in bf16.
+template <typename T16> __device__ __forceinline__ float diag_reference(float bound) {
+  return ceilf(bound) + kDiagReferenceFraction - (std::is_same<T16, __half>::value ? 15.f : 0.f);
+}
+
 // Whether the kernel that steps over diagonals does the call: the scores of all heads are small.  All threads of the block.
 __device__ __forceinline__ bool diag_takes(const DiagParams& p) {
   bool large = false;   // (not >, so that a NaN counts as large)
@@ -103,7 +108,7 @@ __device__ __noinline__ void diag_merge(const DiagParams& p) {
           make_uint4(pack2<T16>(v[c] * scale, v[c + 1] * scale), pack2<T16>(v[c + 2] * scale, v[c + 3] * scale),
                      pack2<T16>(v[c + 4] * scale, v[c + 5] * scale), pack2<T16>(v[c + 6] * scale, v[c + 7] * scale));
     if (c0 == 0)
-      p.lse[(size_t)bh * g.T + q] = (ceilf(head_bound(p.stats, g.BN, bh, p.alpha * kLog2e)) + kDiagReferenceFraction + log2f(l)) * kLn2;
+      p.lse[(size_t)bh * g.T + q] = (diag_reference<T16>(head_bound(p.stats, g.BN, bh, p.alpha * kLog2e)) + log2f(l)) * kLn2;
   }
 }
 

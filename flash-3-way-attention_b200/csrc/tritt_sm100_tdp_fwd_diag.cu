@@ -444,7 +444,7 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             it.ea = product_range<T16>(__ldg(st + kK1 * g.BN), __ldg(st + kK2 * g.BN));
             it.eb = product_range<T16>(__ldg(st + kV1 * g.BN), __ldg(st + kV2 * g.BN));
             it.sa = pow2i<T16>(-it.ea) * fabsf(p.alpha * kLog2e);
-            it.reference = ceilf(bound) + kDiagReferenceFraction;
+            it.reference = diag_reference<T16>(bound);
           }
           it.bh = head;
           it.jt = (int)(tile - (long)head * tiles);
@@ -576,8 +576,8 @@ bool sm100_tdp_fwd_diag_plan(const TdpArgs& a, const float* stats, void* workspa
   p.areas = (float*)workspace;
   p.g = DiagGeometry{a.T, m.k1w, m.k2w, m.kkl, m.kkr, steps, a.B * a.N, grid};
   p.alpha = a.alpha;
-  // bf16: up to what the backward takes for small scores; fp16: P = exp2(S - reference) in [2^-13.2, 1], normal numbers
-  p.bound_limit = a.dtype == TRITT_BF16 ? 16.f : 6.f;
+  // bf16: up to what the backward takes for small scores; fp16: P = exp2(S - reference) in [2^-13.2, 2^15), normal numbers
+  p.bound_limit = a.dtype == TRITT_BF16 ? 16.f : 13.5f;
   p.status = a.status_word;
   return true;
 }

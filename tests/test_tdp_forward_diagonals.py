@@ -45,6 +45,25 @@ def test_against_the_oracle(windows, heads, T, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("sign", [1, -1])
+def test_fp16_scores_near_their_bound(sign):
+    """Queries, K1 and K2 rows that are all alike: every score is within a binade of the bound (8 to 13 in log2 units) or of its
+    negative, where P is 2^-12 at the reference that the bound gives."""
+    windows, heads, T = (128, 128, 32, 32), 16, 300
+    t = _inputs(heads, T, 0.1, torch.float16, 7)
+    for x in t[:3]:
+        x += 1
+    t[0] *= sign
+    alpha = 8.5 / 64 / 1.4427
+    a, b = _forward(t, alpha, windows), _forward(t, alpha, windows, _workspace_without_it(t))
+    assert not torch.equal(a[0], b[0])
+    ref_o, ref_lse = orc.tdp_forward(*[x.float() for x in t], alpha, True, *windows, device=DEV)
+    assert_close("o", a[0], ref_o, torch.float16)
+    # operands of 11 bits: a score of 13 (9 in natural units) moves by 9 * 2^-11 at most
+    assert float((a[1] - ref_lse).abs().max()) <= 5e-3
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_large_scores_of_one_head_are_left_to_the_other_kernel(dtype):
     """Small scores: this kernel, whose roundings are others.  One head with large ones, or not finite: the whole call is the
