@@ -961,7 +961,7 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
 // What both forward kernels need before they start, in one pass over the tensors: SiLU(V1) in the inputs' type and, when
 // `stats` is not null, the per-head statistics behind the score bounds,
 //   stats[bh] = max_j |K1[bh, j, :]|^2,  stats[BN + bh] = max_q |Q[bh, q, :]|^2,  stats[2 BN + bh] = max element^2 of K2[bh],
-// and, where `count` is 7, the largest |element| of K1, K2, V1 and V2 in four more arrays.
+// and, with COUNT 7, the largest |element| of K1, K2, V1 and V2 in four more arrays.
 // A cluster of blocks takes one head: the maxima meet in the first block's shared memory, so that no launch has to
 // zero anything and no atomics are needed.  8 elements per thread and step; a row is held by D / 8 neighbouring lanes.
 // Bound by launch latency on short sequences (it replaces two kernels and a memset: 47.3 -> 43.9 us per call at B=1 N=8
@@ -969,17 +969,17 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
 // size) as soon as each has a pass of work, and blocks of 1024 threads for heads of more than two passes of those: 16 heads of T=2048
 // D=64 16 -> 11 us, windows 256/256/40/20 at T=2048 793 -> 785 us a call.
 constexpr int kPrepThreads = 256, kPrepMost = 1024, kStats = 7;
-template <typename T16>
+template <typename T16, int COUNT>
 __global__ void __launch_bounds__(kPrepMost)
 fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const T16* __restrict__ q,
-                   const T16* __restrict__ k2, const T16* __restrict__ v2, T16* __restrict__ sv1, float* __restrict__ stats, int count,
-                   int head_elems, int D, int BN, int blocks) {
-  __shared__ float red[8][kStats];      // [block of the cluster]; used in the first block
-  __shared__ float wred[kPrepMost / 32][kStats];
+                   const T16* __restrict__ k2, const T16* __restrict__ v2, T16* __restrict__ sv1, float* __restrict__ stats, int head_elems,
+                   int D, int BN, int blocks) {
+  __shared__ float red[8][COUNT];      // [block of the cluster]; used in the first block
+  __shared__ float wred[kPrepMost / 32][COUNT];
   const int bh = blockIdx.x / blocks, part = blockIdx.x % blocks;
   const size_t base = (size_t)bh * head_elems;
   const int lanes = D / 8;
-  float m[kStats] = {};
+  float m[COUNT] = {};   // ([2]: the largest |element| of K2 until it is squared)
   // (the bound is the same for all lanes of a row: head_elems is a multiple of D)
   for (int i = (part * blockDim.x + threadIdx.x) * 8; i < head_elems; i += blocks * blockDim.x * 8) {
     const uint4 v = *reinterpret_cast<const uint4*>(v1 + base + i);
@@ -989,10 +989,10 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
     for (int e = 0; e < 4; ++e) {
       const float2 f = unpack2<T16>(wv[e]);
       o[e] = pack2<T16>(silu_f(f.x), silu_f(f.y));
-      m[5] = fmaxf(m[5], fmaxf(fabsf(f.x), fabsf(f.y)));
+      if constexpr (COUNT == kStats) m[5] = fmaxf(m[5], fmaxf(fabsf(f.x), fabsf(f.y)));
     }
     *reinterpret_cast<uint4*>(sv1 + base + i) = make_uint4(o[0], o[1], o[2], o[3]);
-    if (count == kStats) {
+    if constexpr (COUNT == kStats) {
       const uint4 x = *reinterpret_cast<const uint4*>(v2 + base + i);
       const uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
@@ -1011,8 +1011,8 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
         const float2 x = unpack2<T16>(wa[e]), y = unpack2<T16>(wb[e]), z = unpack2<T16>(wc[e]);
         n1 = fmaf(x.x, x.x, fmaf(x.y, x.y, n1));
         nq = fmaf(y.x, y.x, fmaf(y.y, y.y, nq));
-        m[3] = fmaxf(m[3], fmaxf(fabsf(x.x), fabsf(x.y)));
-        m[4] = fmaxf(m[4], fmaxf(fabsf(z.x), fabsf(z.y)));
+        if constexpr (COUNT == kStats) m[3] = fmaxf(m[3], fmaxf(fabsf(x.x), fabsf(x.y)));
+        m[2] = fmaxf(m[2], fmaxf(fabsf(z.x), fabsf(z.y)));
       }
       // (the lanes of a row are all here or all gone; which lanes of the warp are is not the same everywhere)
       const uint32_t row_lanes = ((lanes == 32 ? 0u : 1u << lanes) - 1u) << ((threadIdx.x & 31) / lanes * lanes);
@@ -1028,14 +1028,15 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1)
 #pragma unroll
-    for (int e = 0; e < kStats; ++e) m[e] = fmaxf(m[e], __shfl_xor_sync(0xffffffffu, m[e], o));
-  m[2] = m[4] * m[4];
+    for (int e = 0; e < COUNT; ++e) m[e] = fmaxf(m[e], __shfl_xor_sync(0xffffffffu, m[e], o));
+  if constexpr (COUNT == kStats) m[4] = m[2];
+  m[2] *= m[2];
   if ((threadIdx.x & 31) == 0) {
 #pragma unroll
-    for (int e = 0; e < kStats; ++e) wred[threadIdx.x >> 5][e] = m[e];
+    for (int e = 0; e < COUNT; ++e) wred[threadIdx.x >> 5][e] = m[e];
   }
   cluster_sync_all();   // every block of the cluster runs: its shared memory may be written (a block barrier as well)
-  if (threadIdx.x < kStats) {
+  if (threadIdx.x < COUNT) {
     float v = 0.f;
     for (int w = 0; w < blockDim.x / 32; ++w) v = fmaxf(v, wred[w][threadIdx.x]);
     uint32_t dst;   // the first block's red[part][.]
@@ -1043,7 +1044,7 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(v) : "memory");
   }
   cluster_sync_all();
-  if (part == 0 && threadIdx.x < count) {
+  if (part == 0 && threadIdx.x < COUNT) {
     float v = 0.f;
     for (int c = 0; c < blocks; ++c) v = fmaxf(v, red[c][threadIdx.x]);
     stats[(size_t)threadIdx.x * BN + bh] = v;
@@ -1074,8 +1075,9 @@ int prepare_fwd(const TdpArgs& a, int count, T16** sv1_out, float** k1n_out) {
   cfg.stream = a.stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  TRITT_CUDA_OK(cudaLaunchKernelEx(&cfg, fwd_prepare_kernel<T16>, (const T16*)a.v1, (const T16*)a.k1, (const T16*)a.q,
-                                   (const T16*)a.k2, (const T16*)a.v2, sv1, k1n, count, head_elems, a.D, BN, blocks));
+  TRITT_CUDA_OK(cudaLaunchKernelEx(&cfg, count == kStats ? fwd_prepare_kernel<T16, kStats> : fwd_prepare_kernel<T16, 3>, (const T16*)a.v1,
+                                   (const T16*)a.k1, (const T16*)a.q, (const T16*)a.k2, (const T16*)a.v2, sv1, k1n, head_elems, a.D, BN,
+                                   blocks));
   count_launch();
   *sv1_out = sv1;
   *k1n_out = k1n;
@@ -1094,7 +1096,8 @@ int launch_fwd(const TdpArgs& a) {
   const bool by_diagonals =
       band && a.workspace_bytes > diag_offset &&
       sm100_tdp_fwd_diag_plan(a, nullptr, (char*)a.workspace + diag_offset, a.workspace_bytes - diag_offset, diag);
-  int rc = prepare_fwd<T16>(a, by_diagonals ? kStats : 3, &sv1, &k1n);
+  // (the largest elements are for fp16's range shifts)
+  int rc = prepare_fwd<T16>(a, by_diagonals && std::is_same<T16, __half>::value ? kStats : 3, &sv1, &k1n);
   if (rc) return rc;
   diag.stats = k1n;
   if (by_diagonals && (rc = sm100_tdp_fwd_diag(a, diag))) return rc;
