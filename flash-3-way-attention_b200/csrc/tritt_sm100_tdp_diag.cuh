@@ -37,6 +37,7 @@ struct DiagParams {
   float* areas;          // [grid][kDiagAreas][kDiagAreaFloats]
   DiagGeometry g;
   float alpha, bound_limit;
+  bool early;      // tdp_fwd_band_kernel is launched ahead of the end of the kernel before it
   int* status;
 };
 

@@ -95,6 +95,7 @@ tdp_fwd_band_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_const
     if (tid == 0 && p.status) atomicOr(p.status, 8);
     return;
   }
+  if (diag.early) asm volatile("griddepcontrol.wait;" ::: "memory");
   if (diag.g.grid > 0 && diag_takes(diag)) {
     // the kernel that steps over diagonals has done the call: what is left are the tiles that it cut
     diag_merge<T16>(diag);
@@ -534,7 +535,17 @@ int launch_band(const TdpArgs& a, const void* sv1, const float* k1n, const DiagP
   TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
   const long items = (long)p.n_groups * BN;
   const int grid = (int)(items < num_sms() ? items : num_sms());
-  kern<<<grid, kBandThreads, Cfg::kSmem, a.stream>>>(tmK1, tmK2b, tmV2b, tmSV1, p, diag ? *diag : DiagParams{});
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3((unsigned)grid, 1, 1);
+  cfg.blockDim = dim3(kBandThreads, 1, 1);
+  cfg.dynamicSmemBytes = Cfg::kSmem;
+  cfg.stream = a.stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = diag && diag->early ? 1 : 0;
+  TRITT_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tmK1, tmK2b, tmV2b, tmSV1, p, diag ? *diag : DiagParams{}));
   count_launch();
   TRITT_CUDA_OK(cudaGetLastError());
   return 0;

@@ -89,7 +89,10 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     return;
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");   // (launched ahead of the preparation's end)
-  if (!diag_takes(p)) return;
+  if (!diag_takes(p)) {
+    asm volatile("griddepcontrol.launch_dependents;");   // (the band kernel, which waits for this one's end all the same)
+    return;
+  }
   if (tid == 0) {
     bars.abort_flag = 0;
     for (int i = 0; i < kItemSlots; ++i) {
@@ -508,6 +511,10 @@ constexpr int kMinSteps = 12;      // of a CTA
 // it:  14: 39 / 44, 16: 39 / 44, 28: 85 / 54, 34: 72 / 37, 35: 72 / 47, 70: 124 / 65.  Calls with large scores pay for a kernel that
 // does nothing: 28: 85 / 75 (the preparation became faster), 35: 84 / 84, 70: 124 / 124, 112: 189 / 192, 277: 469 / 469.
 constexpr long kMinBandTiles = 24;
+// Below this many the band kernel is launched ahead of this one's end: large scores, 16 heads, us without this kernel / with it / with it and
+// the early launch: T=400 fp16 118 / 119 / 118, T=600 bf16 118 / 121 / 119.5, T=1200 windows 16/16/8/8 80 / 85 / 82; but T=2048 128/128/32/32
+// 565 / 560 / 568 (small scores there 187 / 184).
+constexpr long kEarlyBandTiles = 128;
 
 long diag_steps(int B, int N, int T, int band) { return (long)B * N * ((T + 127) / 128) * (band + 1); }
 int diag_grid(long steps) { return (int)(steps / kMinSteps < num_sms() ? steps / kMinSteps : num_sms()); }
@@ -568,6 +575,7 @@ bool sm100_tdp_fwd_diag_plan(const TdpArgs& a, const float* stats, void* workspa
   const long band_tiles = ((long)a.B * a.N * ((a.T + 3) / 4) + num_sms() - 1) / num_sms() * ((min(m.k2w, m.k1w + m.kkr) + 35) / 32);
   if (band_tiles < kMinBandTiles) return false;
   p = DiagParams{};
+  p.early = band_tiles < kEarlyBandTiles;
   p.out = a.out_o;
   p.lse = a.out_lse;
   p.k1 = a.k1;
