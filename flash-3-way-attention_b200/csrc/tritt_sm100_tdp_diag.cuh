@@ -74,7 +74,7 @@ template <typename T16> __device__ __forceinline__ float diag_reference(float bo
 
 // Whether the kernel that steps over diagonals does the call: the scores of all heads are small.  All threads of the block.
 __device__ __forceinline__ bool diag_takes(const DiagParams& p) {
-  bool large = false;   // (not >, so that a NaN counts as large)
+  bool large = false;   // (not >: inf * 0 is large as well; a head with an element that is not finite has an infinite bound)
   for (int bh = threadIdx.x; bh < p.g.BN; bh += blockDim.x)
     large |= !(head_bound(p.stats, p.g.BN, bh, p.alpha * kLog2e) <= p.bound_limit);
   return !__syncthreads_or(large);

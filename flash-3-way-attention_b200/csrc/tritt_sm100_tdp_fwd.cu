@@ -961,7 +961,9 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
 // What both forward kernels need before they start, in one pass over the tensors: SiLU(V1) in the inputs' type and, when
 // `stats` is not null, the per-head statistics behind the score bounds,
 //   stats[bh] = max_j |K1[bh, j, :]|^2,  stats[BN + bh] = max_q |Q[bh, q, :]|^2,  stats[2 BN + bh] = max element^2 of K2[bh],
-// and, with COUNT 7, the largest |element| of K1, K2, V1 and V2 in four more arrays.
+// and, for a call that the kernel over diagonals is asked for (DIAG), fp16: the largest |element| of K1, K2, V1 and V2 in four more
+// arrays.  DIAG: a head with an element that is not finite has an infinite max_q |Q|^2, and so no bound on its scores: the maxima
+// pass over a NaN, and an infinite or NaN value reaches, as 0 * W, every query of two tiles of that kernel.
 // A cluster of blocks takes one head: the maxima meet in the first block's shared memory, so that no launch has to
 // zero anything and no atomics are needed.  8 elements per thread and step; a row is held by D / 8 neighbouring lanes.
 // Bound by launch latency on short sequences (it replaces two kernels and a memset: 47.3 -> 43.9 us per call at B=1 N=8
@@ -969,17 +971,26 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
 // size) as soon as each has a pass of work, and blocks of 1024 threads for heads of more than two passes of those: 16 heads of T=2048
 // D=64 16 -> 11 us, windows 256/256/40/20 at T=2048 793 -> 785 us a call.
 constexpr int kPrepThreads = 256, kPrepMost = 1024, kStats = 7;
-template <typename T16, int COUNT>
+template <typename T16, bool DIAG>
 __global__ void __launch_bounds__(kPrepMost)
 fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const T16* __restrict__ q,
                    const T16* __restrict__ k2, const T16* __restrict__ v2, T16* __restrict__ sv1, float* __restrict__ stats, int head_elems,
                    int D, int BN, int blocks) {
+  constexpr int COUNT = DIAG && std::is_same<T16, __half>::value ? kStats : 3;
   __shared__ float red[8][COUNT];      // [block of the cluster]; used in the first block
   __shared__ float wred[kPrepMost / 32][COUNT];
   const int bh = blockIdx.x / blocks, part = blockIdx.x % blocks;
   const size_t base = (size_t)bh * head_elems;
   const int lanes = D / 8;
   float m[COUNT] = {};   // ([2]: the largest |element| of K2 until it is squared)
+  // Bits 15 and 31 of `bad`: an exponent of all ones, the only one that the addition carries out of.
+  constexpr uint32_t kExponents = std::is_same<T16, __half>::value ? 0x7c007c00u : 0x7f807f80u, kLowest = kExponents & -kExponents;
+  uint32_t bad = 0;
+  auto look = [&](const uint4& v) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) bad |= (w[e] & kExponents) + (kLowest | kLowest << 16);
+  };
   // (the bound is the same for all lanes of a row: head_elems is a multiple of D)
   for (int i = (part * blockDim.x + threadIdx.x) * 8; i < head_elems; i += blocks * blockDim.x * 8) {
     const uint4 v = *reinterpret_cast<const uint4*>(v1 + base + i);
@@ -992,19 +1003,28 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
       if constexpr (COUNT == kStats) m[5] = fmaxf(m[5], fmaxf(fabsf(f.x), fabsf(f.y)));
     }
     *reinterpret_cast<uint4*>(sv1 + base + i) = make_uint4(o[0], o[1], o[2], o[3]);
-    if constexpr (COUNT == kStats) {
+    if constexpr (DIAG) {
       const uint4 x = *reinterpret_cast<const uint4*>(v2 + base + i);
-      const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+      look(v);
+      look(x);
+      if constexpr (COUNT == kStats) {
+        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 f = unpack2<T16>(w[e]);
-        m[6] = fmaxf(m[6], fmaxf(fabsf(f.x), fabsf(f.y)));
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = unpack2<T16>(w[e]);
+          m[6] = fmaxf(m[6], fmaxf(fabsf(f.x), fabsf(f.y)));
+        }
       }
     }
     if (stats) {
       const uint4 a = *reinterpret_cast<const uint4*>(k1 + base + i), b = *reinterpret_cast<const uint4*>(q + base + i),
                   c = *reinterpret_cast<const uint4*>(k2 + base + i);
       const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w}, wc[4] = {c.x, c.y, c.z, c.w};
+      if constexpr (DIAG) {
+        look(a);
+        look(b);
+        look(c);
+      }
       float n1 = 0.f, nq = 0.f;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -1025,6 +1045,7 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
     }
   }
   if (!stats) return;
+  if (DIAG && (bad & 0x80008000u)) m[1] = INFINITY;
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1)
 #pragma unroll
@@ -1051,15 +1072,15 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
   }
 }
 
-// SiLU(V1) at the head of the workspace and, when the workspace has the optional tail, `count` arrays of statistics (the returned
-// pointer is to the first of its arrays of B*N values, the K1 row norms).
+// SiLU(V1) at the head of the workspace and, when the workspace has the optional tail, the statistics (the returned pointer is to the
+// first of its arrays of B*N values, the K1 row norms); `diag`: those of the kernel over diagonals.
 template <typename T16>
-int prepare_fwd(const TdpArgs& a, int count, T16** sv1_out, float** k1n_out) {
+int prepare_fwd(const TdpArgs& a, bool diag, T16** sv1_out, float** k1n_out) {
   const int BN = a.B * a.N;
   const size_t n = (size_t)BN * a.T * a.D, tail = align_up(n * 2, 256);
   T16* sv1 = (T16*)a.workspace;
   float* k1n = nullptr;
-  if (a.workspace_bytes >= tail + count * (size_t)BN * sizeof(float)) k1n = reinterpret_cast<float*>((char*)a.workspace + tail);
+  if (a.workspace_bytes >= tail + (diag ? kStats : 3) * (size_t)BN * sizeof(float)) k1n = reinterpret_cast<float*>((char*)a.workspace + tail);
   const int head_elems = a.T * a.D;
   int blocks = 1;
   while (blocks < 8 && blocks * kPrepThreads * 8 < head_elems) blocks *= 2;
@@ -1075,7 +1096,7 @@ int prepare_fwd(const TdpArgs& a, int count, T16** sv1_out, float** k1n_out) {
   cfg.stream = a.stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  TRITT_CUDA_OK(cudaLaunchKernelEx(&cfg, count == kStats ? fwd_prepare_kernel<T16, kStats> : fwd_prepare_kernel<T16, 3>, (const T16*)a.v1,
+  TRITT_CUDA_OK(cudaLaunchKernelEx(&cfg, diag ? fwd_prepare_kernel<T16, true> : fwd_prepare_kernel<T16, false>, (const T16*)a.v1,
                                    (const T16*)a.k1, (const T16*)a.q, (const T16*)a.k2, (const T16*)a.v2, sv1, k1n, head_elems, a.D, BN,
                                    blocks));
   count_launch();
@@ -1096,8 +1117,7 @@ int launch_fwd(const TdpArgs& a) {
   const bool by_diagonals =
       band && a.workspace_bytes > diag_offset &&
       sm100_tdp_fwd_diag_plan(a, nullptr, (char*)a.workspace + diag_offset, a.workspace_bytes - diag_offset, diag);
-  // (the largest elements are for fp16's range shifts)
-  int rc = prepare_fwd<T16>(a, by_diagonals && std::is_same<T16, __half>::value ? kStats : 3, &sv1, &k1n);
+  int rc = prepare_fwd<T16>(a, by_diagonals, &sv1, &k1n);
   if (rc) return rc;
   diag.stats = k1n;
   if (by_diagonals && (rc = sm100_tdp_fwd_diag(a, diag))) return rc;

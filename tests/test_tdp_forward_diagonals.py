@@ -81,6 +81,22 @@ def test_large_scores_of_one_head_are_left_to_the_other_kernel(dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+def test_values_that_are_not_finite_reach_no_more_queries(value, dtype):
+    """Small scores but for one element, of any of the five tensors: the whole call is the other kernel's, bit for bit, and with it the
+    queries that 0 * inf reaches: tiles of four queries by 32 rows, where the products of this one would reach 256 queries."""
+    windows, heads, T = (100, 128, 20, 30), 16, 300
+    for which in range(5):
+        t = _inputs(heads, T, 0.5, dtype, 1)
+        t[which][0, heads - 1, 200, 63] = value
+        a, b = _forward(t, 1 / 64, windows), _forward(t, 1 / 64, windows, _workspace_without_it(t))
+        for x, y in zip(a, b):
+            assert torch.equal(x.isnan(), y.isnan()) and torch.equal(x.nan_to_num(1e4), y.nan_to_num(1e4)), which
+        assert a[0][0, :-1].isfinite().all() and a[0][0, -1, :64].isfinite().all(), which
+
+
+@pytest.mark.gpu
 def test_captured_call_replays_for_new_inputs():
     windows, heads, T = (128, 128, 32, 32), 16, 700
     t = _inputs(heads, T, 0.5, torch.float16, 2)
