@@ -137,6 +137,16 @@ struct BwdGeometry {
   }
   __host__ __device__ bool overlapping() const { return stride != JT; }
   __host__ __device__ int j_row(int jt) const { return jt * stride - lead; }
+  // rows [lo, hi) of j-tile jt, counted from its first, that the q-tile's sums may take: of an overlapping tile those that a query of
+  // the q-tile sees
+  __host__ __device__ void j_rows(int qt, int jt, int& lo, int& hi) const {
+    lo = 0;
+    hi = T - j_row(jt);
+    if (!overlapping()) return;
+    const int a = first_q(qt) - k1w;
+    lo = (a > 0 ? a : 0) - j_row(jt);
+    hi = last_q(qt) + 1 - j_row(jt);
+  }
   __host__ __device__ int k_first(int qa) const {   // of the k that a query from qa on sees
     const int reach = k2w < k1w + kkr ? k2w : k1w + kkr;
     return qa > reach ? qa - reach : 0;
@@ -826,6 +836,24 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
           else ldmatrix_x4_trans(x[c16][hl], raw_u + frag(c16, hl));
         }
       if (!DIAG) arrive_warp(&bars.tile_free);
+      int j_lo, j_hi;
+      if (!DIAG && g.overlapping()) {
+        g.j_rows(it.qt, it.jt, j_lo, j_hi);
+        // (rows beyond those that a query of the tile sees, which tiles side by side end with, would bring 0 * inf to its sums)
+#pragma unroll
+        for (int c16 = 0; c16 < 4; ++c16)
+#pragma unroll
+          for (int b = 0; b < 8; ++b) {
+            uint32_t& v = x[c16][b >> 2][b & 3];
+            if constexpr (D == 64) {
+              const int r = w * 32 + (b >> 2) * 16 + (b & 1) * 8 + (lane >> 2);
+              v = r >= j_lo && r < j_hi ? v : 0u;
+            } else {
+              const int r = c16 * 16 + (b >> 1 & 1) * 8 + 2 * (lane & 3);
+              v &= (r >= j_lo && r < j_hi ? 0xffffu : 0u) | (r + 1 >= j_lo && r + 1 < j_hi ? 0xffff0000u : 0u);
+            }
+          }
+      }
       const int ex = role ? it.eb : it.ea;   // (x carries 2^ex from here on)
       if (std::is_same<T16, __half>::value) {
         const float2 m = make_float2(pow2i<T16>(ex), pow2i<T16>(ex));
@@ -1078,7 +1106,8 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
       vb0 += (len + kVecBatch - 1) / kVecBatch;
       ++items;
       // ---- dK1 / dSiLU(V1) of this item
-      float* const base = (role ? p.dsv1 : p.dk1) + (size_t)it.bh * T * D;
+      p.g.j_rows(it.qt, it.jt, j_lo, j_hi);
+      float* const base = (role ? p.dsv1 : p.dk1) + ((ptrdiff_t)it.bh * T + p.g.j_row(it.jt)) * D;
 #pragma unroll
       for (int c16 = 0; c16 < 4; ++c16)
 #pragma unroll
@@ -1090,12 +1119,10 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
               const float2 a = acc[c16 * 8 + hl * 4 + g * 2 + r];
               const int lr = w * 32 + hl * 16 + r * 8 + (lane >> 2), lc = c16 * 16 + g * 8 + 2 * (lane & 3);
               if constexpr (D == 64) {
-                const int j = p.g.j_row(it.jt) + lr;
-                if (j >= 0 && j < T) red_add2(base + (size_t)j * D + lc, a.x * jscale, a.y * jscale);
+                if (lr >= j_lo && lr < j_hi) red_add2(base + lr * D + lc, a.x * jscale, a.y * jscale);
               } else {
-                const int j = p.g.j_row(it.jt) + lc;
-                if (j >= 0 && j < T) red_add(base + (size_t)j * D + lr, a.x * jscale);
-                if (j + 1 >= 0 && j + 1 < T) red_add(base + (size_t)(j + 1) * D + lr, a.y * jscale);
+                if (lc >= j_lo && lc < j_hi) red_add(base + lc * D + lr, a.x * jscale);
+                if (lc + 1 >= j_lo && lc + 1 < j_hi) red_add(base + (lc + 1) * D + lr, a.y * jscale);
               }
             }
     }

@@ -276,3 +276,33 @@ def test_overlapping_tiles(D, windows, T, dtype, scale):
     ref = orc.tdp_backward(*[x.float() for x in t], alpha, True, *windows, device=DEV)
     for name, a, b in zip(NAMES, got, ref):
         assert_close(name, a, b, dtype)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,windows", [(64, (128, 128, 30, 30)), (64, (60, 300, 0, 9)), (128, (128, 128, 16, 8)), (128, (30, 70, 0, 20))])
+@pytest.mark.parametrize("which", ["do", "q", "k1", "v1"])
+def test_a_row_that_is_not_finite_stays_in_its_tile_of_overlapping_ones(which, D, windows):
+    """The products of a tile of 128 queries see an infinite row (0 * inf) where tiles side by side would: query 100 keys below 128
+    alone, key 140 queries from 128 on alone, which the j-tiles overlap to both sides."""
+    T, dtype = 391, torch.bfloat16
+    t = [x.to(DEV) for x in orc.make_inputs(1, 2, T, D, scale=1.0, seed=D, dtype=dtype)]   # (scores too large for steps over diagonals)
+    bad = [x.clone() for x in t]
+    row = 100 if which in ("do", "q") else 140
+    bad[{"q": 0, "k1": 1, "v1": 3, "do": 5}[which]][:, :, row] = float("inf")
+    o, lse = torch.empty_like(t[0]), torch.empty(1, 2, T, device=DEV)
+    _native.tdp_fwd(*t[:5], o, lse, 1 / 8, True, *windows)
+    got, want = [torch.empty_like(o) for _ in range(5)], [torch.empty_like(o) for _ in range(5)]
+    for x, g in ((bad, got), (t, want)):
+        _native.tdp_bwd(*x[:5], o, x[5], lse, *g, 1 / 8, True, *windows)
+    torch.cuda.synchronize()
+    assert _native.read_status(torch.device(DEV)) == 0
+    for name, a, b in zip(NAMES, got, want):
+        if row == 100:
+            a, b = (x[:, :, 128:].float() for x in (a, b))
+        elif name == "dq":
+            a, b = (x[:, :, :128].float() for x in (a, b))
+        else:
+            continue   # (the keys' sums meet the row's own queries)
+        assert torch.isfinite(a).all(), f"{name}: {int((~torch.isfinite(a)).sum())} of {a.numel()} values are not finite"
+        # (two runs of the same sums: their order, and bf16's rounding)
+        assert float((a - b).norm()) <= 8e-3 * float(b.norm()), name
