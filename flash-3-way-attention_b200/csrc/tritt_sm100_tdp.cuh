@@ -4,6 +4,8 @@
 #include "tritt_common.cuh"
 #include "tritt_sm100.cuh"
 
+#include <type_traits>
+
 namespace tritt {
 namespace {
 
@@ -33,6 +35,12 @@ template <> __device__ __forceinline__ uint32_t mul2<__nv_bfloat16>(uint32_t a, 
 template <> __device__ __forceinline__ uint32_t mul2<__half>(uint32_t a, uint32_t b) {
   const __half2 v = __hmul2(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b));
   return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// Bit 15 and bit 31 of the result: the low and the high element's exponent is all ones, that is infinite or NaN (no other carries
+// out of it).  The other bits mean nothing.
+template <typename T16> __device__ __forceinline__ uint32_t not_finite(uint32_t v) {
+  return std::is_same<T16, __half>::value ? (v & 0x7c007c00u) + 0x04000400u : (v & 0x7f807f80u) + 0x00800080u;
 }
 
 // Bits c of [lo, hi] among 0..31: with a mask of a row's columns a per-element test is one logic instruction (a constant

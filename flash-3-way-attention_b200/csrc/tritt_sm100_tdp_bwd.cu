@@ -360,6 +360,7 @@ __device__ __forceinline__ void red_add4(float* p, float a, float b, float c, fl
 struct BwdStats {
   float k1, k2, sv1, v2;    // largest element of K1, K2, SiLU(V1), V2
   float k1_row, q_row, do_row, sv1_row;   // largest squared norm of a row
+  bool finite;              // all elements of Q, K1, K2, V1, V2 and dO are (the maxima pass over a NaN)
 };
 __device__ __forceinline__ BwdStats head_stats(const BwdParams& p, int bh, int lane) {
   float m[kStatFloats] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -368,11 +369,13 @@ __device__ __forceinline__ BwdStats head_stats(const BwdParams& p, int bh, int l
     const float4 x = __ldg(src), y = __ldg(src + 1);
     m[0] = x.x; m[1] = x.y; m[2] = x.z; m[3] = x.w; m[4] = y.x; m[5] = y.y; m[6] = y.z; m[7] = y.w;
   }
+  const bool finite = !__any_sync(0xffffffffu, __float_as_int(m[5]) < 0);   // (q_row's sign: see the preparation)
+  m[5] = fabsf(m[5]);
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1)
 #pragma unroll
     for (int i = 0; i < kStatFloats; ++i) m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], o));
-  return BwdStats{m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7]};
+  return BwdStats{m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], finite};
 }
 
 // Whether a head of this CTA's part may have large scores (the same for every thread; without statistics: yes).
@@ -389,12 +392,13 @@ __device__ __forceinline__ bool large_scores(const BwdParams& p) {
   return __syncthreads_or(large);
 }
 
-// Whether all scores of the call are small (the same for every thread).
+// Whether all scores of the call are small (the same for every thread).  A head with an element that is not finite counts as large: on a
+// diagonal such a row of K2 or V2 belongs to all queries of a tile that a row j = k - d meets, the tile before its own included.
 __device__ __forceinline__ bool all_scores_small(const BwdParams& p) {
   bool large = false;
   for (int bh = threadIdx.x >> 5; bh < p.BN; bh += kBwdThreads / 32) {
     const BwdStats st = head_stats(p, bh, threadIdx.x & 31);
-    large |= !(fabsf(p.alpha * kLog2e) * sqrtf(st.k1_row * st.q_row) * st.k2 <= kScoreBound);
+    large |= !st.finite || !(fabsf(p.alpha * kLog2e) * sqrtf(st.k1_row * st.q_row) * st.k2 <= kScoreBound);
   }
   return !__syncthreads_or(large);
 }
@@ -1464,6 +1468,11 @@ tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, co
     const uint4 x = *reinterpret_cast<const uint4*>(p);
     w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
   };
+  uint32_t bad = 0;   // (see not_finite)
+  auto look = [&](const uint32_t (&w)[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) bad |= not_finite<T16>(w[e]);
+  };
   auto grow = [](float& a, float2 x) { a = fmaxf(a, fmaxf(fabsf(x.x), fabsf(x.y))); };
   // (the lanes of a row are all here or all gone: head_elems is a multiple of D)
   for (int at = (part * kPrepThreads + threadIdx.x) * 8; at < head_elems; at += parts * kPrepThreads * 8) {
@@ -1493,9 +1502,14 @@ tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, co
     for (int s = lanes / 2; s >= 1; s >>= 1) dot += __shfl_xor_sync(row_lanes, dot, s);
     if ((threadIdx.x & (lanes - 1)) == 0) drow[i / D] = dot;
     if (stats) {
+      look(wv);
+      look(wb);
       words(k1 + i, wv);
       words(k2 + i, wa);
       words(v2 + i, wb);
+      look(wv);
+      look(wa);
+      look(wb);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         grow(k1_max, unpack2<T16>(wv[e]));
@@ -1503,6 +1517,7 @@ tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, co
         grow(v2_max, unpack2<T16>(wb[e]));
       }
       words(q + i, wa);
+      look(wa);
       float n1 = 0.f, nq = 0.f;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -1532,11 +1547,12 @@ tdp_bwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ o, co
 #pragma unroll
     for (int i = 0; i < kStatFloats; ++i) wmax[threadIdx.x >> 5][i] = w[i];
   }
-  __syncthreads();
+  const bool any_bad = __syncthreads_or(bad & 0x80008000u);
   if (threadIdx.x < kStatFloats) {
     float x = 0.f;
 #pragma unroll
-      for (int i = 0; i < kPrepThreads / 32; ++i) x = fmaxf(x, wmax[i][threadIdx.x]);
+    for (int i = 0; i < kPrepThreads / 32; ++i) x = fmaxf(x, wmax[i][threadIdx.x]);
+    if (threadIdx.x == 5 && any_bad) x = -x;   // q_row's sign: not all elements are finite
     stats[(size_t)blockIdx.x * kStatFloats + threadIdx.x] = x;
   }
 }

@@ -983,14 +983,8 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
   const size_t base = (size_t)bh * head_elems;
   const int lanes = D / 8;
   float m[COUNT] = {};   // ([2]: the largest |element| of K2 until it is squared)
-  // Bits 15 and 31 of `bad`: an exponent of all ones, the only one that the addition carries out of.
-  constexpr uint32_t kExponents = std::is_same<T16, __half>::value ? 0x7c007c00u : 0x7f807f80u, kLowest = kExponents & -kExponents;
   uint32_t bad = 0;
-  auto look = [&](const uint4& v) {
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) bad |= (w[e] & kExponents) + (kLowest | kLowest << 16);
-  };
+  auto look = [&](const uint4& v) { bad |= not_finite<T16>(v.x) | not_finite<T16>(v.y) | not_finite<T16>(v.z) | not_finite<T16>(v.w); };
   // (the bound is the same for all lanes of a row: head_elems is a multiple of D)
   for (int i = (part * blockDim.x + threadIdx.x) * 8; i < head_elems; i += blocks * blockDim.x * 8) {
     const uint4 v = *reinterpret_cast<const uint4*>(v1 + base + i);
