@@ -92,6 +92,7 @@ constexpr int kStatParts = 32, kStatFloats = 8;
 // Rows of a window of K2 or V2 (128 + kk_left + kk_right at most): what shared memory has left beside one A' instead of two and without the K1
 // and SiLU(V1) tiles.
 constexpr int kDiagRows = 200;
+constexpr int kPartHeads = 512;   // heads of a CTA's part, at most, where the kernel over diagonals is asked
 
 template <int D, bool DIAG = false> struct BwdCfg {
   static constexpr int JT = D == 64 ? 128 : 64;       // rows j of an item
@@ -111,7 +112,8 @@ template <int D, bool DIAG = false> struct BwdCfg {
   static constexpr int kOffVec = kOffR1 + (D / 64 - 1) * 16384;  // [slot][K2 rows | V2 rows][row of the batch][D], 16-bit
   static constexpr int kVecPart = kVecBatch * D * 2;  // bytes of a batch of rows of one tensor
   static constexpr int kOffBars = kOffVec + (DIAG ? 0 : kVecSlots * 2 * kVecPart);
-  static constexpr int kSmem = kOffBars + 512;
+  static constexpr int kOffHeads = kOffBars + 512;    // PartHeads' marks
+  static constexpr int kSmem = kOffHeads + (D == 64 ? kPartHeads : 0);
   static constexpr int kTmemS = 0, kTmemDP = JT, kTmemG = 2 * JT, kTmemU = kTmemG + 64, kTmemDQ = kTmemU + 64;
   static constexpr int kTmemQ = kTmemDQ + D, kTmemDO = kTmemQ + D / 2;   // 16-bit, two elements a column
   static_assert(kTmemDO + D / 2 <= 512 && kSmem <= 232448, "tensor / shared memory");
@@ -198,7 +200,7 @@ struct BwdParams {
   int i_first;             // query rows (of the shard) before this one are not this kernel's
   long head_steps;         // steps of one head
   float alpha;
-  bool diag_asked;         // the kernel that steps over diagonals is ahead of this one, and does the call if all scores are small
+  bool diag_asked;         // the heads that are diag_head() are the kernel's that steps over diagonals, the others the one's over k
   int* status;
 };
 
@@ -234,57 +236,6 @@ __device__ __forceinline__ void cta_part(const BwdParams& p, long& s0, long& s1)
   s0 = total / c * blockIdx.x + total % c * blockIdx.x / c;
   s1 = total / c * (blockIdx.x + 1) + total % c * (blockIdx.x + 1) / c;
 }
-
-// One CTA's part of the line of steps, item by item (walked by the loader warp, which hands the items to the others).
-struct BwdWalk {
-  const BwdGeometry& g;
-  long left;                    // steps of this CTA not handed out yet
-  int bh, qt, jt, k0, len;      // next item (len 0: none)
-
-  __device__ void step() {
-    if (++jt > g.j_last(qt)) {
-      if (++qt == g.q_tiles()) {
-        qt = 0;
-        ++bh;
-      }
-      jt = g.j_first(qt);
-    }
-  }
-  __device__ void find(long skip) {   // first item with steps, from (bh, qt, jt) on, less `skip` steps
-    len = 0;
-    while (left > 0) {
-      const int n = g.k_range(qt, jt, k0);
-      if (n > skip) {
-        k0 += (int)skip;
-        len = n - (int)skip < left ? n - (int)skip : (int)left;
-        left -= len;
-        return;
-      }
-      skip -= n;
-      step();
-    }
-  }
-  __device__ explicit BwdWalk(const BwdParams& p) : g(p.g) {
-    long s0, s1;
-    const long H = p.head_steps;
-    cta_part(p, s0, s1);
-    left = s1 - s0;
-    bh = (int)(s0 / H);
-    qt = 0;
-    jt = g.j_first(0);
-    find(s0 % H);
-  }
-  // hands out the item found last and looks for the one after it
-  __device__ BwdItem next(const BwdItem& prev) {
-    BwdItem it{bh, qt, jt, k0, len, 0, 0, 0, 0, {0, 0, 0}};
-    if (len == 0) return it;
-    if (bh != prev.bh || qt != prev.qt) it.flags |= kFirstOfQ;
-    step();
-    find(0);
-    if (len == 0 || bh != it.bh || qt != it.qt) it.flags |= kLastOfQ;
-    return it;
-  }
-};
 
 // fp16 only: the recomputed probabilities of a query that attends n pairs are ~1/n, which for late rows lies below
 // fp16's normal range (6e-5; 1/n = 2e-7 at q = 2048).  P and dS are therefore formed times 2^e, e = min(10, log2 of the
@@ -378,30 +329,100 @@ __device__ __forceinline__ BwdStats head_stats(const BwdParams& p, int bh, int l
   return BwdStats{m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], finite};
 }
 
-// Whether a head of this CTA's part may have large scores (the same for every thread; without statistics: yes).
-__device__ __forceinline__ bool large_scores(const BwdParams& p) {
+// Whether the head may have large scores: |S| <= |Q row| |K1 row| max|K2|, in log2 units, as S is.  (Not >: inf * 0 is large as well.
+// Rounded one by one, so that whoever asks gets the same answer.)
+__device__ __forceinline__ bool large_head(const BwdParams& p, const BwdStats& st) {
+  const float q = __fsqrt_rn(__fmul_rn(st.k1_row, st.q_row));
+  return !(__fmul_rn(__fmul_rn(fabsf(__fmul_rn(p.alpha, kLog2e)), q), st.k2) <= kScoreBound);
+}
+// Whether the head is the kernel's that steps over diagonals, if that is asked: small scores and finite elements.  (On a diagonal a row
+// of K2 or V2 meets all queries of a tile that a row j = k - d meets, the tile before its own included.)
+__device__ __forceinline__ bool diag_head(const BwdParams& p, const BwdStats& st) { return st.finite && !large_head(p, st); }
+
+// What the heads of this CTA's part are, the same for every thread.  (Only its own: a look at all heads of a call, by every CTA of
+// both kernels, took 5 % of a backward of 4096 heads of T=140.)
+struct PartHeads {
+  bool large;   // one may have large scores (without statistics: yes)
+  bool diag;    // one is diag_head()
+  bool others;  // one is not
+};
+template <int D, bool DIAG> __device__ __forceinline__ PartHeads part_heads(const BwdParams& p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* const marks = smem + BwdCfg<D, DIAG>::kOffHeads;   // of head bh: diag_head()
   long s0, s1;
   cta_part(p, s0, s1);
-  bool large = !p.stats;
+  PartHeads h{!p.stats, false, false};
   const int last = (int)((s1 - 1) / p.head_steps);
   for (int bh = (int)(s0 / p.head_steps) + (threadIdx.x >> 5); bh <= last && p.stats; bh += kBwdThreads / 32) {
     const BwdStats st = head_stats(p, bh, threadIdx.x & 31);
-    // |S| <= |Q row| |K1 row| max|K2|, in log2 units, as S is  (not >, so that a NaN counts as large)
-    large |= !(fabsf(p.alpha * kLog2e) * sqrtf(st.k1_row * st.q_row) * st.k2 <= kScoreBound);
+    const bool diag = diag_head(p, st);
+    h.large |= large_head(p, st);
+    h.diag |= diag;
+    h.others |= !diag;
+    if (p.diag_asked) marks[bh % kPartHeads] = diag;
   }
-  return __syncthreads_or(large);
+  h.large = __syncthreads_or(h.large);
+  if (p.diag_asked) {
+    h.diag = __syncthreads_or(h.diag);
+    h.others = __syncthreads_or(h.others);
+  }
+  return h;
 }
 
-// Whether all scores of the call are small (the same for every thread).  A head with an element that is not finite counts as large: on a
-// diagonal such a row of K2 or V2 belongs to all queries of a tile that a row j = k - d meets, the tile before its own included.
-__device__ __forceinline__ bool all_scores_small(const BwdParams& p) {
-  bool large = false;
-  for (int bh = threadIdx.x >> 5; bh < p.BN; bh += kBwdThreads / 32) {
-    const BwdStats st = head_stats(p, bh, threadIdx.x & 31);
-    large |= !st.finite || !(fabsf(p.alpha * kLog2e) * sqrtf(st.k1_row * st.q_row) * st.k2 <= kScoreBound);
+// One CTA's part of the line of steps, item by item (walked by the loader warp, which hands the items to the others).
+// `marks` (null: all are): only those heads of the part that are (DIAG) or are not marked (part_heads).
+template <bool DIAG> struct BwdWalk {
+  const BwdGeometry& g;
+  const uint8_t* marks;
+  long left;                    // steps of this CTA not handed out yet
+  int bh, qt, jt, k0, len;      // next item (len 0: none)
+
+  __device__ void step() {
+    if (++jt > g.j_last(qt)) {
+      if (++qt == g.q_tiles()) {
+        qt = 0;
+        ++bh;
+      }
+      jt = g.j_first(qt);
+    }
   }
-  return !__syncthreads_or(large);
-}
+  __device__ void find(long skip) {   // first item with steps, from (bh, qt, jt) on, less `skip` steps
+    while (left > 0) {
+      const int n = g.k_range(qt, jt, k0);
+      if (n > skip) {
+        k0 += (int)skip;
+        len = n - (int)skip < left ? n - (int)skip : (int)left;
+        left -= len;
+        if (!marks || (marks[bh % kPartHeads] != 0) == DIAG) return;
+        skip = 0;
+      } else {
+        skip -= n;
+      }
+      step();
+    }
+    len = 0;
+  }
+  __device__ BwdWalk(const BwdParams& p, const uint8_t* marks) : g(p.g), marks(marks) {
+    long s0, s1;
+    const long H = p.head_steps;
+    cta_part(p, s0, s1);
+    left = s1 - s0;
+    bh = (int)(s0 / H);
+    qt = 0;
+    jt = g.j_first(0);
+    find(s0 % H);
+  }
+  // hands out the item found last and looks for the one after it
+  __device__ BwdItem next(const BwdItem& prev) {
+    BwdItem it{bh, qt, jt, k0, len, 0, 0, 0, 0, {0, 0, 0}};
+    if (len == 0) return it;
+    if (bh != prev.bh || qt != prev.qt) it.flags |= kFirstOfQ;
+    step();
+    find(0);
+    if (len == 0 || bh != it.bh || qt != it.qt) it.flags |= kLastOfQ;
+    return it;
+  }
+};
 
 // LARGE: S = R K1^T with R [q,h] = alpha*log2(e) * Q[q,h] * K2[k,h] instead of S = Q A^T (see kScoreBound).
 template <int D, typename T16, bool LARGE, bool DIAG = false>
@@ -1273,7 +1294,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
     int bh = -1, ea = 0, eb = 0, er = 0, f = 0;
     uint32_t items = 0, vb = 0;
     bool alive = true, in_flight = false;
-    BwdWalk walk(p);
+    BwdWalk<DIAG> walk(p, D == 64 && p.diag_asked ? smem + Cfg::kOffHeads : nullptr);
     BwdItem it{-1, -1, 0, 0, 0, 0, 0, 0, 0, {0, 0, 0}};
     while (alive) {
       it = walk.next(it);
@@ -1422,16 +1443,24 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
   if (tid == 0 && bars.abort_flag && p.status) atomicOr(p.status, 4);
 }
 
+// A CTA that has nothing to do.  As at the body's end the kernel must not end before the one ahead of it, which may be running; one
+// block's wait is enough, and the others make room for what comes next (with a wait of all, a kernel over k began when the exact first
+// queries had ended: 997 us for 983 at 16 heads of T=2048, windows 128/128/0/0, large scores).
+__device__ __forceinline__ void end_without_work() {
+  if (blockIdx.x == 0 && threadIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 template <int D, typename T16>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 tdp_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                const __grid_constant__ CUtensorMap tmK1, const __grid_constant__ CUtensorMap tmSV1,
                const __grid_constant__ BwdParams p) {
-  if (p.diag_asked && all_scores_small(p)) {
-    if (threadIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");   // (as at the body's end)
+  const PartHeads heads = part_heads<D, false>(p);
+  if (p.diag_asked && !heads.others) {
+    end_without_work();
     return;
   }
-  if (large_scores(p)) tdp_bwd_body<D, T16, true>(tmQ, tmDO, tmK1, tmSV1, p);
+  if (heads.large) tdp_bwd_body<D, T16, true>(tmQ, tmDO, tmK1, tmSV1, p);
   else tdp_bwd_body<D, T16, false>(tmQ, tmDO, tmK1, tmSV1, p);
 }
 
@@ -1441,11 +1470,8 @@ tdp_bwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                     const __grid_constant__ CUtensorMap tmK2, const __grid_constant__ CUtensorMap tmV2,
                     const __grid_constant__ BwdParams p) {
   asm volatile("griddepcontrol.launch_dependents;");   // (tdp_bwd_kernel, which needs nothing of this one)
-  if (all_scores_small(p)) {
-    tdp_bwd_body<64, T16, false, true>(tmQ, tmDO, tmK2, tmV2, p);
-  } else if (threadIdx.x == 0) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");   // (as at the body's end)
-  }
+  if (part_heads<64, true>(p).diag) tdp_bwd_body<64, T16, false, true>(tmQ, tmDO, tmK2, tmV2, p);
+  else end_without_work();
 }
 
 // What the kernel needs before it starts, in one pass over the tensors (8 elements per thread and step): zeroed fp32
@@ -1792,17 +1818,18 @@ int launch_bwd_sums(const TdpArgs& a, const BwdPlan& plan) {
   };
   bool early = plan.i_first > 0;
   if constexpr (D == 64) {
-    if (plan.diag_steps > 0 && stats) {
+    const long least = plan.diag_steps < plan.head_steps ? plan.diag_steps : plan.head_steps, sms = num_sms();
+    if (plan.diag_steps > 0 && stats && BN / (least * BN < sms ? least * BN : sms) + 2 <= kPartHeads) {
       const uint32_t rows = 128 + a.mask.kkl + a.mask.kkr;
       if ((rc = make_tmap_3d(&tmK2, a.k2, 2, D, a.T, BN, 64, rows))) return rc;
       if ((rc = make_tmap_3d(&tmV2, a.v2, 2, D, a.T, BN, 64, rows))) return rc;
       if ((rc = check_kernel_registers<tdp_bwd_diag_kernel<T16>>())) return rc;
+      p.diag_asked = true;
       p.g = plan.diag;
       p.head_steps = plan.diag_steps;
       if ((rc = launch(tdp_bwd_diag_kernel<T16>, BwdCfg<D, true>::kSmem, plan.diag_steps, early, tmK2, tmV2))) return rc;
       p.g = plan.g;
       p.head_steps = plan.head_steps;
-      p.diag_asked = true;
       early = true;
     }
   }

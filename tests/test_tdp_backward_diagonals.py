@@ -68,6 +68,26 @@ def test_large_scores_of_one_head_are_left_to_the_other_kernel(dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("heads,T", [(40, 300), (200, 140), (5, 1500)])
+def test_heads_of_both_kinds(heads, T, dtype):
+    """Each head is the one kernel's or the other's: CTAs whose part has heads of one kind or of both, one or many of them."""
+    windows = (100, 128, 20, 30)
+    t, do = _inputs(heads, T, dtype, 6)
+    large, bad = [h for h in range(heads) if h % 7 in (1, 2) or h > heads - 3], heads // 2
+    for h in large:
+        t[0][0, h] *= 3
+        t[1][0, h] *= 3
+    t[4][0, bad, T - 1, 3] = float("inf")   # (which reaches the last queries; all other heads are the oracle's)
+    got, launched = _backward(t, do, 1 / 8, windows)
+    assert launched == 5
+    ref = orc.tdp_backward(*[x.float() for x in t], do.float(), 1 / 8, True, *windows, device=DEV)
+    for name, a, b in zip(NAMES, got, ref):
+        for h in [h for h in range(heads) if h != bad]:
+            assert_close(f"{name} of head {h}", a[:, h], b[:, h], dtype)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("value", [float("inf"), float("nan")])
 def test_a_query_that_is_not_finite_stays_in_its_tile(value):
     """An infinite or NaN upstream row of query 0: the products of its tile of 128 queries and keys see it (0 * inf), no other row."""
