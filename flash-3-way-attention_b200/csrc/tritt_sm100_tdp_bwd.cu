@@ -65,15 +65,15 @@ constexpr int kBwdThreads = 640;
 // twice.  (80 / 128 / 64 or 96 / 120 / 48 for soft-max, fold and service warps in the small-score body: 5 to 8 % slower, as their
 // loops spill.)
 constexpr int kRegsLaunch = 96;
-// (Large scores at head dimension 64: 88 / 136 / 32, although R's warps spill then: fp16 16 heads T=512 947 -> 931 us, not causal
-// 1880 -> 1850, bf16 T=2048 4 heads 10.7 -> 10.6 ms, 4 heads T=300 the same.  Small scores: 1687 us -> 1750 at 32 heads of T=512.)
+// (88 / 136 / 32 for large scores at head dimension 64, where R's warps spill then: fp16 16 heads T=512 916 -> 927 us, bf16 T=2048 4 heads
+// 10.45 -> 10.50 ms, windows 16/16/8/8 T=1200 380 -> 386, 128/128/0/0 T=2048 984 -> 989.  Small scores: 1687 us -> 1750 at 32 heads of T=512.)
 // (Diagonals: the fold warps need more, what the service warps can spare.  Band 128/128/32/32 at T=2048, soft-max / fold / service:
 // 88 / 128 / 48 757 us, 88 / 136 / 32 671, 80 / 136 / 48 731, 80 / 144 / 32 748; twice as many fold warps of 72 registers 930.)
 // (Large scores at head dimension 128 have the service warps form 32 KB of R per step, and soft-max warps that hold half as many
 // columns as at 64: with 48 registers those service warps spill, 1.60 -> 1.90 ms at 16 heads of T=512.)
 template <int D, bool LARGE, bool DIAG> struct BwdRegs {
-  static constexpr int kSoftmax = D == 128 && LARGE ? 80 : 88, kFold = DIAG || (D == 64 && LARGE) ? 136 : 128,
-                       kService = DIAG || (D == 64 && LARGE) ? 32 : D == 128 && LARGE ? 64 : 48;
+  static constexpr int kSoftmax = D == 128 && LARGE ? 80 : 88, kFold = DIAG ? 136 : 128,
+                       kService = DIAG ? 32 : D == 128 && LARGE ? 64 : 48;
   static_assert(2 * kSoftmax + 2 * kFold + kService <= 5 * kRegsLaunch, "more registers than the launch has");
 };
 constexpr int kVecBatch = 4;     // K2 / V2 rows per hand-over
