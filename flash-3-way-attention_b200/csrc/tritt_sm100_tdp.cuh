@@ -43,6 +43,27 @@ template <typename T16> __device__ __forceinline__ uint32_t not_finite(uint32_t 
   return std::is_same<T16, __half>::value ? (v & 0x7c007c00u) + 0x04000400u : (v & 0x7f807f80u) + 0x00800080u;
 }
 
+// The larger |element| of each half: of two, or, `NAN_TOO`, NaN if one is.
+template <bool NAN_TOO> __device__ __forceinline__ __half2 larger_abs(__half2 m, __half2 v) {
+  return NAN_TOO ? __hmax2_nan(m, __habs2(v)) : __hmax2(m, __habs2(v));
+}
+template <bool NAN_TOO> __device__ __forceinline__ __nv_bfloat162 larger_abs(__nv_bfloat162 m, __nv_bfloat162 v) {
+  return NAN_TOO ? __hmax2_nan(m, __habs2(v)) : __hmax2(m, __habs2(v));
+}
+template <typename T16> struct Pair;
+template <> struct Pair<__half> { using type = __half2; };
+template <> struct Pair<__nv_bfloat16> { using type = __nv_bfloat162; };
+// m's halves grown by the 8 elements of v
+template <typename T16, bool NAN_TOO> __device__ __forceinline__ void grow_abs(uint32_t& m, const uint4& v) {
+  using P = typename Pair<T16>::type;
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const P x = larger_abs<NAN_TOO>(*reinterpret_cast<const P*>(&m), *reinterpret_cast<const P*>(&w[e]));
+    m = *reinterpret_cast<const uint32_t*>(&x);
+  }
+}
+
 // Bits c of [lo, hi] among 0..31: with a mask of a row's columns a per-element test is one logic instruction (a constant
 // bit into a predicate) instead of two comparisons.
 __device__ __forceinline__ uint32_t column_mask(int lo, int hi) {
@@ -52,9 +73,10 @@ __device__ __forceinline__ uint32_t column_mask(int lo, int hi) {
 }
 
 // Bound on every score of a head, in log2 units: |s| max_q |Q_q| max |K2 element| max_j |K1_j|, s = alpha log2(e), from the forward's
-// statistics (fwd_prepare_kernel).
+// statistics (fwd_prepare_kernel).  (Rounded one by one, so that all kernels that ask get the same answer.)
 __device__ __forceinline__ float head_bound(const float* stats, int BN, int bh, float s) {
-  return fabsf(s) * sqrtf(__ldg(stats + BN + bh)) * sqrtf(__ldg(stats + 2 * BN + bh)) * sqrtf(__ldg(stats + bh));
+  const float q = __fsqrt_rn(__ldg(stats + BN + bh)), k2 = __fsqrt_rn(__ldg(stats + 2 * BN + bh)), k1 = __fsqrt_rn(__ldg(stats + bh));
+  return __fmul_rn(__fmul_rn(__fmul_rn(fabsf(s), q), k2), k1);
 }
 
 // Sum of v[0..31] over the 32 lanes of a warp, column-wise: on return lane i holds the

@@ -958,21 +958,22 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
   if (tid == 0 && bars.abort_flag && p.status) atomicOr(p.status, 2);
 }
 
-// What both forward kernels need before they start, in one pass over the tensors: SiLU(V1) in the inputs' type and, when
+// What the forward kernels need before they start, in one pass over the tensors: SiLU(V1) in the inputs' type and, when
 // `stats` is not null, the per-head statistics behind the score bounds,
 //   stats[bh] = max_j |K1[bh, j, :]|^2,  stats[BN + bh] = max_q |Q[bh, q, :]|^2,  stats[2 BN + bh] = max element^2 of K2[bh],
 // and, for a call that the kernel over diagonals is asked for (DIAG), fp16: the largest |element| of K1, K2, V1 and V2 in four more
-// arrays.  DIAG: a head with an element that is not finite has an infinite max_q |Q|^2, and so no bound on its scores: the maxima
-// pass over a NaN, and an infinite or NaN value reaches, as 0 * W, every query of two tiles of that kernel.
+// arrays.  DIAG: a head with an element that is not finite has an infinite max_q |Q|^2, and so no
+// bound on its scores: the maxima pass over a NaN, and an infinite or NaN value reaches, as 0 * W, every query of two tiles there.
 // A cluster of blocks takes one head: the maxima meet in the first block's shared memory, so that no launch has to
-// zero anything and no atomics are needed.  8 elements per thread and step; a row is held by D / 8 neighbouring lanes.
-// Bound by launch latency on short sequences (it replaces two kernels and a memset: 47.3 -> 43.9 us per call at B=1 N=8
-// T=64 D=64) and by memory on long ones, where it is < 0.1 % of the call.  Eight blocks per head (the portable cluster
-// size) as soon as each has a pass of work, and blocks of 1024 threads for heads of more than two passes of those: 16 heads of T=2048
-// D=64 16 -> 11 us, windows 256/256/40/20 at T=2048 793 -> 785 us a call.
-constexpr int kPrepThreads = 256, kPrepMost = 1024, kStats = 7;
+// zero anything and no atomics are needed.  8 elements per thread and pass; a row is held by D / 8 neighbouring lanes.
+// Bound by latency: a pass waits for its reads (1 us), a block for the cluster twice and for its launch.  So a head has as many blocks
+// (eight, the portable cluster size, at most) as the chip holds, each with a pass of work, and larger ones where that leaves many
+// passes (prepare_fwd).  us, blocks of 256 threads, eight a head -> the present ones: 16 heads T=1200 D=64 6.4 -> 5.8, T=2048
+// 8.7 -> 7.0, T=8192 30 -> 18, one head T=8192 25 -> 11, 1024 heads T=200 37 -> 24, 4096 heads T=140 131 -> 65.  DIAG with more reads
+// under way and half as many threads on an SM: T=1200 9.2 -> 5.6 in 32 and 64 registers.
+constexpr int kPrepThreads = 256, kPrepMost = 1024, kPrepMostDiag = 512, kStats = 7;
 template <typename T16, bool DIAG>
-__global__ void __launch_bounds__(kPrepMost)
+__global__ void __launch_bounds__(DIAG ? kPrepMostDiag : kPrepMost, 2)
 fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const T16* __restrict__ q,
                    const T16* __restrict__ k2, const T16* __restrict__ v2, T16* __restrict__ sv1, float* __restrict__ stats, int head_elems,
                    int D, int BN, int blocks) {
@@ -982,51 +983,44 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
   const int bh = blockIdx.x / blocks, part = blockIdx.x % blocks;
   const size_t base = (size_t)bh * head_elems;
   const int lanes = D / 8;
-  float m[COUNT] = {};   // ([2]: the largest |element| of K2 until it is squared)
-  uint32_t bad = 0;
-  auto look = [&](const uint4& v) { bad |= not_finite<T16>(v.x) | not_finite<T16>(v.y) | not_finite<T16>(v.z) | not_finite<T16>(v.w); };
+  float m[COUNT] = {};
+  uint32_t top_k1 = 0, top_k2 = 0, top_q = 0, top_v1 = 0, top_v2 = 0;   // largest |element|, of either half (DIAG: NaN if there is one)
   // (the bound is the same for all lanes of a row: head_elems is a multiple of D)
   for (int i = (part * blockDim.x + threadIdx.x) * 8; i < head_elems; i += blocks * blockDim.x * 8) {
+    // (all reads of a pass together: it waits for memory)
     const uint4 v = *reinterpret_cast<const uint4*>(v1 + base + i);
+    uint4 x, a, b, c;
+    if (DIAG) x = *reinterpret_cast<const uint4*>(v2 + base + i);
+    if (stats) {
+      a = *reinterpret_cast<const uint4*>(k1 + base + i);
+      b = *reinterpret_cast<const uint4*>(q + base + i);
+      c = *reinterpret_cast<const uint4*>(k2 + base + i);
+    }
     const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
     uint32_t o[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float2 f = unpack2<T16>(wv[e]);
       o[e] = pack2<T16>(silu_f(f.x), silu_f(f.y));
-      if constexpr (COUNT == kStats) m[5] = fmaxf(m[5], fmaxf(fabsf(f.x), fabsf(f.y)));
     }
     *reinterpret_cast<uint4*>(sv1 + base + i) = make_uint4(o[0], o[1], o[2], o[3]);
     if constexpr (DIAG) {
-      const uint4 x = *reinterpret_cast<const uint4*>(v2 + base + i);
-      look(v);
-      look(x);
-      if constexpr (COUNT == kStats) {
-        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = unpack2<T16>(w[e]);
-          m[6] = fmaxf(m[6], fmaxf(fabsf(f.x), fabsf(f.y)));
-        }
-      }
+      grow_abs<T16, true>(top_v1, v);
+      grow_abs<T16, true>(top_v2, x);
     }
     if (stats) {
-      const uint4 a = *reinterpret_cast<const uint4*>(k1 + base + i), b = *reinterpret_cast<const uint4*>(q + base + i),
-                  c = *reinterpret_cast<const uint4*>(k2 + base + i);
-      const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w}, wc[4] = {c.x, c.y, c.z, c.w};
+      const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
+      grow_abs<T16, DIAG>(top_k2, c);
       if constexpr (DIAG) {
-        look(a);
-        look(b);
-        look(c);
+        grow_abs<T16, true>(top_k1, a);
+        grow_abs<T16, true>(top_q, b);
       }
       float n1 = 0.f, nq = 0.f;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float2 x = unpack2<T16>(wa[e]), y = unpack2<T16>(wb[e]), z = unpack2<T16>(wc[e]);
-        n1 = fmaf(x.x, x.x, fmaf(x.y, x.y, n1));
-        nq = fmaf(y.x, y.x, fmaf(y.y, y.y, nq));
-        if constexpr (COUNT == kStats) m[3] = fmaxf(m[3], fmaxf(fabsf(x.x), fabsf(x.y)));
-        m[2] = fmaxf(m[2], fmaxf(fabsf(z.x), fabsf(z.y)));
+        const float2 y = unpack2<T16>(wa[e]), z = unpack2<T16>(wb[e]);
+        n1 = fmaf(y.x, y.x, fmaf(y.y, y.y, n1));
+        nq = fmaf(z.x, z.x, fmaf(z.y, z.y, nq));
       }
       // (the lanes of a row are all here or all gone; which lanes of the warp are is not the same everywhere)
       const uint32_t row_lanes = ((lanes == 32 ? 0u : 1u << lanes) - 1u) << ((threadIdx.x & 31) / lanes * lanes);
@@ -1039,7 +1033,20 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
     }
   }
   if (!stats) return;
-  if (DIAG && (bad & 0x80008000u)) m[1] = INFINITY;
+  auto larger_half = [](uint32_t v) {
+    const float2 f = unpack2<T16>(v);
+    return fmaxf(f.x, f.y);
+  };
+  m[2] = larger_half(top_k2);
+  if constexpr (COUNT == kStats) {
+    m[3] = larger_half(top_k1);
+    m[5] = larger_half(top_v1);
+    m[6] = larger_half(top_v2);
+  }
+  if constexpr (DIAG) {
+    const uint32_t bad = not_finite<T16>(top_k1) | not_finite<T16>(top_k2) | not_finite<T16>(top_q) | not_finite<T16>(top_v1) | not_finite<T16>(top_v2);
+    if (bad & 0x80008000u) m[1] = INFINITY;
+  }
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1)
 #pragma unroll
@@ -1067,7 +1074,7 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
 }
 
 // SiLU(V1) at the head of the workspace and, when the workspace has the optional tail, the statistics (the returned pointer is to the
-// first of its arrays of B*N values, the K1 row norms); `diag`: those of the kernel over diagonals.
+// first of its arrays of B*N values, the K1 row norms); `diag`: the kernel over diagonals is asked.
 template <typename T16>
 int prepare_fwd(const TdpArgs& a, bool diag, T16** sv1_out, float** k1n_out) {
   const int BN = a.B * a.N;
@@ -1076,9 +1083,21 @@ int prepare_fwd(const TdpArgs& a, bool diag, T16** sv1_out, float** k1n_out) {
   float* k1n = nullptr;
   if (a.workspace_bytes >= tail + (diag ? kStats : 3) * (size_t)BN * sizeof(float)) k1n = reinterpret_cast<float*>((char*)a.workspace + tail);
   const int head_elems = a.T * a.D;
+  // Blocks of 256 threads that an SM holds; a head's blocks; and the passes of one.  us with 1 / 2 / 4 / 8 blocks a head: 256 heads T=512
+  // 19.1 / 13.0 / 11.7 / 13.5 (diag 19.1 / 13.2 / 16.6 / 21.2), 1024 heads T=200 24.5 / 26.8 / 29.9 / 36.8.
+  const long resident = (long)num_sms() * (diag ? 4 : 8);
   int blocks = 1;
-  while (blocks < 8 && blocks * kPrepThreads * 8 < head_elems) blocks *= 2;
-  const int threads = blocks * kPrepThreads * 8 * 2 < head_elems ? kPrepMost : kPrepThreads;
+  while (blocks < 8 && blocks * kPrepThreads * 8 < head_elems && 2L * BN * blocks <= resident) blocks *= 2;
+  const int passes = (head_elems - 1) / (blocks * kPrepThreads * 8) + 1;
+  // Larger blocks where passes are many and SMs free.  us with 256 / 512 / 1024 threads (diag 256 / 512): 4 heads, 2 passes 3.8 / 3.3 / 4.2
+  // (3.6 / 3.3), 5 passes 6.0 / 4.9 / 5.4 (5.2 / 4.6), 8 passes 8.0 / 5.8 / 5.5; 16 heads, 3 passes 4.6 / 4.6 / 5.4 (4.3 / 4.8), 5 passes
+  // 6.2 / 5.8 / 7.8 (5.6 / 6.0), 8 passes 8.5 / 7.0 / 7.7 (7.6 / 7.2), 32 passes 29 / 19.8 / 18.1; 64 heads, 4 passes 7.2 / 7.6 / 10.8
+  // (7.5 / 10.0), 8 passes 12.4 / 11.6 / 15.4 (13.3 / 17.1).
+  const long grid = (long)BN * blocks, sms = num_sms();
+  const bool few = 2 * grid <= sms;
+  int threads = kPrepThreads;
+  if (passes > (few ? 1 : diag ? 6 : grid <= 2 * sms ? 2 : 4) && 2 * grid <= resident) threads = 512;
+  if (!diag && passes >= (few ? 8 : 16) && grid <= sms) threads = kPrepMost;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
