@@ -1,5 +1,5 @@
 // What the forward kernel that steps over the diagonals of a narrow band (tritt_sm100_tdp_fwd_diag.cu) shares with the one that serves
-// such calls otherwise (tritt_sm100_tdp_fwd_band.cu): which of the two does a call, and the pieces that the first one leaves.
+// such calls otherwise (tritt_sm100_tdp_fwd_band.cu): which of the two does a call, and the pieces of the query tiles that the first one cuts.
 #pragma once
 
 #include "tritt_sm100_tdp.cuh"
@@ -9,7 +9,8 @@
 namespace tritt {
 
 constexpr int kDiagD = 64;                                // head dimension
-constexpr int kDiagAreaFloats = 128 * (kDiagD + 1);       // accumulator [D][128], sums [128]
+constexpr int kDiagAreaFloats = 2 * 128 * (kDiagD / 2 + 1);   // of either half of the columns: accumulator [D / 2][128], sums [128]
+constexpr int kDiagArrivals = 16;
 constexpr int kDiagAreas = 4;   // of a CTA: tiles begun before its part (by the parity of the tile), tiles begun in it
 constexpr float kDiagReferenceFraction = 0.142019f;       // (see kReferenceFraction of the general forward kernel)
 
@@ -35,14 +36,16 @@ struct DiagParams {
   const void *k1, *v1;
   const float* stats;    // [7][BN] (see fwd_prepare_kernel)
   float* areas;          // [grid][kDiagAreas][kDiagAreaFloats]
+  unsigned* arrived;     // [grid][kDiagArrivals], zero: pieces there are of the tiles begun in a CTA's part, by the tile's parity and by warp
   DiagGeometry g;
   float alpha, bound_limit;
-  bool early;      // tdp_fwd_band_kernel is launched ahead of the end of the kernel before it
+  bool early;            // tdp_fwd_band_kernel is launched ahead of this kernel's end, and adds up the pieces
   int* status;
 };
 
-// Fills `p` and returns true if that kernel is asked; `workspace`: sm100_tdp_fwd_diag_workspace() bytes of scratch.
-bool sm100_tdp_fwd_diag_plan(const TdpArgs& a, const float* stats, void* workspace, size_t workspace_bytes, DiagParams& p);
+// Fills `p` but for the statistics and returns true if that kernel is asked; `workspace`: sm100_tdp_fwd_diag_workspace() bytes of scratch.
+// p.arrived[0 .. p.g.grid * kDiagArrivals) has to be zero when it starts.
+bool sm100_tdp_fwd_diag_plan(const TdpArgs& a, void* workspace, size_t workspace_bytes, DiagParams& p);
 int sm100_tdp_fwd_diag(const TdpArgs& a, const DiagParams& p);
 // `sv1`: SiLU(V1) in the inputs' type; `k1n`: per-head largest squared K1 row norm, or null (both prepared by the caller);
 // `diag`: what sm100_tdp_fwd_diag() was launched with just before, or null.
@@ -80,9 +83,14 @@ __device__ __forceinline__ bool diag_takes(const DiagParams& p) {
   return !__syncthreads_or(large);
 }
 
+// Piece i of query tile `tile`, whose first one is CTA `first`'s: one half of the columns.
+__device__ __forceinline__ float* diag_area(const DiagParams& p, int first, int i, int tile, int half) {
+  return p.areas + ((size_t)(first + i) * kDiagAreas + (i == 0 ? 2 : 0) + (tile & 1)) * kDiagAreaFloats + half * (kDiagAreaFloats / 2);
+}
+
 // The pieces of the query tiles that are cut -> their outputs.  A thread takes 16 columns of a row at a time.
 template <typename T16>
-__device__ __noinline__ void diag_merge(const DiagParams& p) {
+__device__ __forceinline__ void diag_merge(const DiagParams& p) {
   const DiagGeometry& g = p.g;
   const int tiles = g.tiles(), units = g.BN * tiles * (kDiagD / 16), per_block = blockDim.x / 128, row = threadIdx.x % 128;
   for (int u = blockIdx.x * per_block + threadIdx.x / 128; u < units; u += gridDim.x * per_block) {
@@ -95,10 +103,10 @@ __device__ __noinline__ void diag_merge(const DiagParams& p) {
     for (int c = 0; c < 16; ++c) v[c] = 0.f;
 #pragma unroll 2
     for (int i = 0; i < pieces; ++i) {
-      const float* a = p.areas + ((size_t)(first + i) * kDiagAreas + (i == 0 ? 2 : 0) + (tile & 1)) * kDiagAreaFloats + row;
-      l += a[kDiagD * 128];
+      const float* a = diag_area(p, first, i, tile, c0 / (kDiagD / 2)) + row;
+      l += a[kDiagD / 2 * 128];
 #pragma unroll
-      for (int c = 0; c < 16; ++c) v[c] += a[(c0 + c) * 128];
+      for (int c = 0; c < 16; ++c) v[c] += a[(c0 % (kDiagD / 2) + c) * 128];
     }
     const float* st = p.stats + bh;
     const float scale = pow2i<T16>(-product_range<T16>(__ldg(st + kV1 * g.BN), __ldg(st + kV2 * g.BN))) / l;

@@ -962,7 +962,7 @@ tdp_fwd_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__
 // `stats` is not null, the per-head statistics behind the score bounds,
 //   stats[bh] = max_j |K1[bh, j, :]|^2,  stats[BN + bh] = max_q |Q[bh, q, :]|^2,  stats[2 BN + bh] = max element^2 of K2[bh],
 // and, for a call that the kernel over diagonals is asked for (DIAG), fp16: the largest |element| of K1, K2, V1 and V2 in four more
-// arrays.  DIAG: a head with an element that is not finite has an infinite max_q |Q|^2, and so no
+// arrays.  DIAG: that kernel's counters are zeroed; a head with an element that is not finite has an infinite max_q |Q|^2, and so no
 // bound on its scores: the maxima pass over a NaN, and an infinite or NaN value reaches, as 0 * W, every query of two tiles there.
 // A cluster of blocks takes one head: the maxima meet in the first block's shared memory, so that no launch has to
 // zero anything and no atomics are needed.  8 elements per thread and pass; a row is held by D / 8 neighbouring lanes.
@@ -976,7 +976,7 @@ template <typename T16, bool DIAG>
 __global__ void __launch_bounds__(DIAG ? kPrepMostDiag : kPrepMost, 2)
 fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const T16* __restrict__ q,
                    const T16* __restrict__ k2, const T16* __restrict__ v2, T16* __restrict__ sv1, float* __restrict__ stats, int head_elems,
-                   int D, int BN, int blocks) {
+                   int D, int BN, int blocks, unsigned* __restrict__ counters, int n_counters) {
   constexpr int COUNT = DIAG && std::is_same<T16, __half>::value ? kStats : 3;
   __shared__ float red[8][COUNT];      // [block of the cluster]; used in the first block
   __shared__ float wred[kPrepMost / 32][COUNT];
@@ -984,6 +984,9 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
   const size_t base = (size_t)bh * head_elems;
   const int lanes = D / 8;
   float m[COUNT] = {};
+  if constexpr (DIAG) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_counters; i += gridDim.x * blockDim.x) counters[i] = 0;
+  }
   uint32_t top_k1 = 0, top_k2 = 0, top_q = 0, top_v1 = 0, top_v2 = 0;   // largest |element|, of either half (DIAG: NaN if there is one)
   // (the bound is the same for all lanes of a row: head_elems is a multiple of D)
   for (int i = (part * blockDim.x + threadIdx.x) * 8; i < head_elems; i += blocks * blockDim.x * 8) {
@@ -1076,7 +1079,7 @@ fwd_prepare_kernel(const T16* __restrict__ v1, const T16* __restrict__ k1, const
 // SiLU(V1) at the head of the workspace and, when the workspace has the optional tail, the statistics (the returned pointer is to the
 // first of its arrays of B*N values, the K1 row norms); `diag`: the kernel over diagonals is asked.
 template <typename T16>
-int prepare_fwd(const TdpArgs& a, bool diag, T16** sv1_out, float** k1n_out) {
+int prepare_fwd(const TdpArgs& a, const DiagParams* diag, T16** sv1_out, float** k1n_out) {
   const int BN = a.B * a.N;
   const size_t n = (size_t)BN * a.T * a.D, tail = align_up(n * 2, 256);
   T16* sv1 = (T16*)a.workspace;
@@ -1111,7 +1114,7 @@ int prepare_fwd(const TdpArgs& a, bool diag, T16** sv1_out, float** k1n_out) {
   cfg.numAttrs = 1;
   TRITT_CUDA_OK(cudaLaunchKernelEx(&cfg, diag ? fwd_prepare_kernel<T16, true> : fwd_prepare_kernel<T16, false>, (const T16*)a.v1,
                                    (const T16*)a.k1, (const T16*)a.q, (const T16*)a.k2, (const T16*)a.v2, sv1, k1n, head_elems, a.D, BN,
-                                   blocks));
+                                   blocks, diag ? diag->arrived : nullptr, diag ? diag->g.grid * kDiagArrivals : 0));
   count_launch();
   *sv1_out = sv1;
   *k1n_out = k1n;
@@ -1129,8 +1132,8 @@ int launch_fwd(const TdpArgs& a) {
   DiagParams diag;
   const bool by_diagonals =
       band && a.workspace_bytes > diag_offset &&
-      sm100_tdp_fwd_diag_plan(a, nullptr, (char*)a.workspace + diag_offset, a.workspace_bytes - diag_offset, diag);
-  int rc = prepare_fwd<T16>(a, by_diagonals, &sv1, &k1n);
+      sm100_tdp_fwd_diag_plan(a, (char*)a.workspace + diag_offset, a.workspace_bytes - diag_offset, diag);
+  int rc = prepare_fwd<T16>(a, by_diagonals ? &diag : nullptr, &sv1, &k1n);
   if (rc) return rc;
   diag.stats = k1n;
   if (by_diagonals && (rc = sm100_tdp_fwd_diag(a, diag))) return rc;

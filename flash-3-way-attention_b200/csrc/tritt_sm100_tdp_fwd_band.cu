@@ -79,7 +79,10 @@ struct BandTile {
   bool first, last;  // first / last k-block of its query group
 };
 
-template <int D, typename T16>
+// Alone, or behind the kernel over diagonals, which may have done the call.  (Kernels of their own: the sum of the pieces in this code
+// costs large scores 1.5 %, T=2048 bf16 windows 128/128/0/0 442 -> 449 us, 128/128/32/32 fp16 563 -> 567.)
+enum { kAlone, kBehindDiag, kBehindDiagMerge };
+template <int D, typename T16, int ROLE>
 __global__ void __launch_bounds__(kBandThreads, 1)
 tdp_fwd_band_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_constant__ CUtensorMap tmK2b,
                     const __grid_constant__ CUtensorMap tmV2b, const __grid_constant__ CUtensorMap tmSV1, BandParams p,
@@ -95,11 +98,16 @@ tdp_fwd_band_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_const
     if (tid == 0 && p.status) atomicOr(p.status, 8);
     return;
   }
-  if (diag.early) asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (diag.g.grid > 0 && diag_takes(diag)) {
-    // the kernel that steps over diagonals has done the call: what is left are the tiles that it cut
-    diag_merge<T16>(diag);
-    return;
+  if constexpr (ROLE == kBehindDiag) {
+    if (diag_takes(diag)) return;
+  }
+  if constexpr (ROLE == kBehindDiagMerge) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // (launched ahead of that kernel's end)
+    if (diag_takes(diag)) {
+      // the kernel that steps over diagonals has done the call: what is left are the tiles that it cut
+      diag_merge<T16>(diag);
+      return;
+    }
   }
   if (tid == 0) {
     bars.abort_flag = 0;
@@ -531,7 +539,10 @@ int launch_band(const TdpArgs& a, const void* sv1, const float* k1n, const DiagP
   p.bound_limit = std::is_same<T16, __nv_bfloat16>::value ? 40.f : 6.f;
   p.status = a.status_word;
   if (p.nq == 0) return 0;
-  auto kern = tdp_fwd_band_kernel<D, T16>;
+  constexpr int kBehind = D == kDiagD ? kBehindDiag : kAlone, kBehindMerge = D == kDiagD ? kBehindDiagMerge : kAlone;
+  auto kern = !diag         ? tdp_fwd_band_kernel<D, T16, kAlone>
+              : diag->early ? tdp_fwd_band_kernel<D, T16, kBehindMerge>
+                            : tdp_fwd_band_kernel<D, T16, kBehind>;
   TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
   const long items = (long)p.n_groups * BN;
   const int grid = (int)(items < num_sms() ? items : num_sms());

@@ -235,8 +235,8 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       g.ctas(bh, tile, first, pieces);
       const float scale = pow2i<T16>(-eb) / row_sum;
       T16* const dst = (T16*)p.out + ((size_t)bh * T + q) * kDiagD + half * (kDiagD / 2);
-      float* const area = p.areas + ((size_t)blockIdx.x * kDiagAreas + ((int)blockIdx.x == first ? 2 : 0) + (tile & 1)) * kDiagAreaFloats +
-                          half * (kDiagD / 2) * 128 + row;
+      auto area_of = [&](int i) -> float* { return diag_area(p, first, i, tile, half) + row; };
+      float* const area = area_of((int)blockIdx.x - first);
 #pragma unroll 1
       for (int c0 = 0; c0 < kDiagD / 2; c0 += 16) {
         uint32_t t[16];
@@ -258,10 +258,51 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         __syncwarp();   // (the lanes of rows beyond the sequence store nothing; the next read takes the whole warp)
       }
       tc_fence_before();
-      if (half == 1) {
-        if (pieces > 1) area[kDiagD / 2 * 128] = row_sum;
-        else if (q < T) p.lse[(size_t)bh * T + q] = (reference + log2f(row_sum)) * kLn2;
+      if (pieces == 1) {
+        if (half == 1 && q < T) p.lse[(size_t)bh * T + q] = (reference + log2f(row_sum)) * kLn2;
+        __syncwarp();
+        continue;
       }
+      area[kDiagD / 2 * 128] = row_sum;
+      if (p.early) {
+        __syncwarp();
+        continue;
+      }
+      // The warp that brings the last of the tile's pieces adds them up, for its rows and columns, in the order of the CTAs.
+      __threadfence();
+      __syncwarp();
+      unsigned arrived = 0;
+      if (lane == 0) arrived = atomicAdd(p.arrived + first * kDiagArrivals + (tile & 1) * 8 + half * 4 + wq, 1u);
+      if (__shfl_sync(0xffffffffu, arrived, 0) + 1 != (unsigned)pieces) continue;
+      __threadfence();
+      float sum = 0.f;
+      for (int i = 0; i < pieces; ++i) sum += __ldcg(area_of(i) + kDiagD / 2 * 128);
+      const float whole = pow2i<T16>(-eb) / sum;
+#pragma unroll 1
+      for (int c0 = 0; c0 < kDiagD / 2; c0 += 16) {
+        float v[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) v[c] = 0.f;
+        for (int i = 0; i < pieces; i += 2) {   // (two pieces' reads under way)
+          const float *const a = area_of(i) + c0 * 128, *const b = area_of(min(i + 1, pieces - 1)) + c0 * 128;
+          const float more = i + 1 < pieces ? 1.f : 0.f;
+          float x[16], y[16];
+#pragma unroll
+          for (int c = 0; c < 16; ++c) x[c] = __ldcg(a + c * 128);
+#pragma unroll
+          for (int c = 0; c < 16; ++c) y[c] = __ldcg(b + c * 128);
+#pragma unroll
+          for (int c = 0; c < 16; ++c) v[c] = fmaf(y[c], more, v[c] + x[c]);
+        }
+        if (q < T) {
+          uint32_t o[8];
+#pragma unroll
+          for (int c = 0; c < 16; c += 2) o[c / 2] = pack2<T16>(v[c] * whole, v[c + 1] * whole);
+          *reinterpret_cast<uint4*>(dst + c0) = make_uint4(o[0], o[1], o[2], o[3]);
+          *reinterpret_cast<uint4*>(dst + c0 + 8) = make_uint4(o[4], o[5], o[6], o[7]);
+        }
+      }
+      if (half == 1 && q < T) p.lse[(size_t)bh * T + q] = (reference + log2f(sum)) * kLn2;
       __syncwarp();
     }
   } else if (warp < 24) {
@@ -507,13 +548,14 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 }
 
 constexpr int kMinSteps = 12;      // of a CTA
-// Tiles of a CTA of tdp_fwd_band_kernel (1.7 us each) from which on this kernel is asked.  Calls with small scores, tiles: us without it / with
-// it:  14: 39 / 44, 16: 39 / 44, 28: 85 / 54, 34: 72 / 37, 35: 72 / 47, 70: 124 / 65.  Calls with large scores pay for a kernel that
-// does nothing: 28: 85 / 75 (the preparation became faster), 35: 84 / 84, 70: 124 / 124, 112: 189 / 192, 277: 469 / 469.
+size_t area_bytes(int grid) { return (size_t)grid * kDiagAreas * kDiagAreaFloats * sizeof(float); }
+size_t scratch_bytes(int grid) { return area_bytes(grid) + (size_t)grid * kDiagArrivals * sizeof(unsigned); }
+// Tiles of a CTA of tdp_fwd_band_kernel (1.7 us each) from which on this kernel is asked.
 constexpr long kMinBandTiles = 24;
-// Below this many the band kernel is launched ahead of this one's end: large scores, 16 heads, us without this kernel / with it / with it and
-// the early launch: T=400 fp16 118 / 119 / 118, T=600 bf16 118 / 121 / 119.5, T=1200 windows 16/16/8/8 80 / 85 / 82; but T=2048 128/128/32/32
-// 565 / 560 / 568 (small scores there 187 / 184).
+// ... and below which that kernel adds up the pieces, launched ahead of this one's end.  A CTA that brings the
+// last piece takes 7 us for them, most often at its end, the band kernel 3; in long calls the pieces of many tiles come in between.  us,
+// by the band kernel / here: 8 heads T=1000 fp16 61 / 65, 16 heads T=400 128/128/48/48 76.8 / 80.5, T=2048 8/8/4/4 42.6 / 44.8, T=2048
+// 128/128/32/32 181 / 179, T=8192 669 / 653, 4096 heads T=140 20/20/4/4 736 / 690.
 constexpr long kEarlyBandTiles = 128;
 
 long diag_steps(int B, int N, int T, int band) { return (long)B * N * ((T + 127) / 128) * (band + 1); }
@@ -562,16 +604,16 @@ int launch_diag(const TdpArgs& a, const DiagParams& p) {
 
 size_t sm100_tdp_fwd_diag_workspace(int B, int N, int T, int D) {
   if (D != kDiagD || T <= 128) return 0;
-  return (size_t)diag_grid(diag_steps(B, N, T, kMaxBand)) * kDiagAreas * kDiagAreaFloats * sizeof(float);
+  return scratch_bytes(diag_grid(diag_steps(B, N, T, kMaxBand)));
 }
 
-bool sm100_tdp_fwd_diag_plan(const TdpArgs& a, const float* stats, void* workspace, size_t workspace_bytes, DiagParams& p) {
+bool sm100_tdp_fwd_diag_plan(const TdpArgs& a, void* workspace, size_t workspace_bytes, DiagParams& p) {
   const TdpMask& m = a.mask;
   // (a query tile meets its own j-tile and the one before: q - j <= min(k1w, k2w + kkl) <= 128)
   if (a.D != kDiagD || a.q_mod != 1 || m.kkl + m.kkr > kMaxBand || (m.k1w > 128 && m.k2w + m.kkl > 128)) return false;
   const long steps = diag_steps(a.B, a.N, a.T, m.kkl + m.kkr);
   const int grid = diag_grid(steps);
-  if (grid < 1 || workspace_bytes < (size_t)grid * kDiagAreas * kDiagAreaFloats * sizeof(float)) return false;
+  if (grid < 1 || workspace_bytes < scratch_bytes(grid)) return false;
   const long band_tiles = ((long)a.B * a.N * ((a.T + 3) / 4) + num_sms() - 1) / num_sms() * ((min(m.k2w, m.k1w + m.kkr) + 35) / 32);
   if (band_tiles < kMinBandTiles) return false;
   p = DiagParams{};
@@ -580,11 +622,11 @@ bool sm100_tdp_fwd_diag_plan(const TdpArgs& a, const float* stats, void* workspa
   p.lse = a.out_lse;
   p.k1 = a.k1;
   p.v1 = a.v1;
-  p.stats = stats;
   p.areas = (float*)workspace;
+  p.arrived = (unsigned*)((char*)workspace + area_bytes(grid));
   p.g = DiagGeometry{a.T, m.k1w, m.k2w, m.kkl, m.kkr, steps, a.B * a.N, grid};
   p.alpha = a.alpha;
-  // bf16: up to what the backward takes for small scores; fp16: P = exp2(S - reference) in [2^-13.2, 2^15), normal numbers
+  // bf16: up to what the backward takes for small scores; fp16: P = exp2(S - reference) in [2^-12.7, 2^15), normal numbers
   p.bound_limit = a.dtype == TRITT_BF16 ? 16.f : 13.5f;
   p.status = a.status_word;
   return true;

@@ -45,6 +45,30 @@ def test_against_the_oracle(windows, heads, T, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("windows,heads,T", [((128, 128, 32, 32), 16, 1024), ((128, 128, 32, 32), 17, 1000), ((20, 20, 4, 4), 600, 140),
+                                             ((128, 128, 48, 48), 6, 2600)])
+def test_long_calls_add_up_their_pieces_in_the_kernel(windows, heads, T, dtype):
+    """From 128 tiles of the band kernel on (a CTA) the warp that brings the last piece of a tile adds them up, in the pieces' order:
+    the same bits each time, beside calls of other inputs in the same workspace."""
+    t, u = _inputs(heads, T, 0.5, dtype, T), _inputs(heads, T, 0.4, dtype, T + 1)
+    before = _native.lib().tritt_kernel_launches()
+    o, lse = _forward(t, 1 / 64, windows)
+    assert _native.lib().tritt_kernel_launches() - before == 3   # preparation, this kernel, the band kernel
+    ref_o, ref_lse = orc.tdp_forward(*[x.float() for x in t], 1 / 64, True, *windows, device=DEV)
+    assert_close("o", o, ref_o, dtype)
+    assert float((lse - ref_lse).abs().max()) <= 2e-3   # (as above)
+    ws = _native.workspace(_native.OP_TDP_FWD, 1, heads, T, 64, _native.dtype_code(dtype), o.device)
+    for _ in range(5):
+        _forward(u, 1 / 64, windows, ws)
+        again = _forward(t, 1 / 64, windows, ws)
+        assert torch.equal(again[0], o) and torch.equal(again[1], lse)
+    t[0][0, heads - 1] *= 400   # large scores: the band kernel, bit for bit
+    a, b = _forward(t, 1 / 64, windows, ws), _forward(t, 1 / 64, windows, _workspace_without_it(t))
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("sign", [1, -1])
 def test_fp16_scores_near_their_bound(sign):
     """Queries, K1 and K2 rows that are all alike: every score is within a binade of the bound (8 to 13 in log2 units) or of its
