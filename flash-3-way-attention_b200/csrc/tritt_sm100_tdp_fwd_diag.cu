@@ -550,15 +550,26 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 constexpr int kMinSteps = 12;      // of a CTA
 size_t area_bytes(int grid) { return (size_t)grid * kDiagAreas * kDiagAreaFloats * sizeof(float); }
 size_t scratch_bytes(int grid) { return area_bytes(grid) + (size_t)grid * kDiagArrivals * sizeof(unsigned); }
-// Tiles of a CTA of tdp_fwd_band_kernel (1.7 us each) from which on this kernel is asked.
-constexpr long kMinBandTiles = 24;
-// ... and below which that kernel adds up the pieces, launched ahead of this one's end.  A CTA that brings the
+// This kernel is asked where it costs less than the band kernel, in us: a step 1 (narrow windows, most columns masked) to 1.4, an item (a
+// j-tile) 1.3 beside its steps, launch and first item 14; a tile of the band kernel 1.6 to 2.  us of a call with small scores, by the
+// band kernel / here, of CTAs of steps / tiles: 12 / 17 (a diagonal an item) 38 / 42, 12 / 14 32 / 34, 13 / 14 33 / 36, 16 / 15 36 / 38, 36 / 18
+// (T=129 128/128/48/48) 36 / 57, 53 / 28 64 / 71, 65 / 42 86 / 88, 70 / 27 59 / 89;  114 / 81 163 / 150, 28 / 68 117 / 60, 42 / 47 96 / 76, 16 / 56 119 / 43,
+// 86 / 69 143 / 111, 112 / 280 466 / 179.
+constexpr double kStepPrice = 1, kFullStepPrice = 1.4, kItemPrice = 1.3, kLaunchPrice = 14, kTilePrice = 1.9;
+// Tiles of a CTA of tdp_fwd_band_kernel below which that kernel adds up the pieces, launched ahead of this one's end.  A CTA that brings the
 // last piece takes 7 us for them, most often at its end, the band kernel 3; in long calls the pieces of many tiles come in between.  us,
 // by the band kernel / here: 8 heads T=1000 fp16 61 / 65, 16 heads T=400 128/128/48/48 76.8 / 80.5, T=2048 8/8/4/4 42.6 / 44.8, T=2048
 // 128/128/32/32 181 / 179, T=8192 669 / 653, 4096 heads T=140 20/20/4/4 736 / 690.
 constexpr long kEarlyBandTiles = 128;
 
 long diag_steps(int B, int N, int T, int band) { return (long)B * N * ((T + 127) / 128) * (band + 1); }
+// Tiles of a CTA of tdp_fwd_band_kernel: the groups of four queries have a block of 32 K2 rows at first, and as many as reach back `reach`
+// rows from there on.
+double band_tiles_of_cta(long heads, int T, int reach) {
+  const int r = min(reach, T - 1), groups = (T + 3) / 4, growing = r / 4;
+  const double blocks = growing * (r / 64.0 + 1) + (groups - growing) * (double)((r + 35) / 32);   // of a head
+  return (double)((heads * groups + num_sms() - 1) / num_sms()) * blocks / groups;
+}
 int diag_grid(long steps) { return (int)(steps / kMinSteps < num_sms() ? steps / kMinSteps : num_sms()); }
 
 template <typename T16>
@@ -614,8 +625,10 @@ bool sm100_tdp_fwd_diag_plan(const TdpArgs& a, void* workspace, size_t workspace
   const long steps = diag_steps(a.B, a.N, a.T, m.kkl + m.kkr);
   const int grid = diag_grid(steps);
   if (grid < 1 || workspace_bytes < scratch_bytes(grid)) return false;
-  const long band_tiles = ((long)a.B * a.N * ((a.T + 3) / 4) + num_sms() - 1) / num_sms() * ((min(m.k2w, m.k1w + m.kkr) + 35) / 32);
-  if (band_tiles < kMinBandTiles) return false;
+  const double R = m.kkl + m.kkr + 1, part = (double)steps / grid;
+  const double band_tiles = band_tiles_of_cta((long)a.B * a.N, a.T, min(m.k2w, m.k1w + m.kkr));
+  const double filled = min(min(m.k1w, m.k2w) + 1, 128) / 128., step = kStepPrice + (kFullStepPrice - kStepPrice) * filled;
+  if (step * part + kItemPrice * (part / R + 1) + kLaunchPrice > kTilePrice * band_tiles) return false;
   p = DiagParams{};
   p.early = band_tiles < kEarlyBandTiles;
   p.out = a.out_o;

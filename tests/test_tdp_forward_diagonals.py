@@ -12,7 +12,9 @@ DEV = "cuda:0"
 def _forward(t, alpha, windows, ws=None):
     B, N, T, _ = t[0].shape
     o, lse = torch.full_like(t[0], float("nan")), torch.full((B, N, T), float("nan"), device=DEV)
+    before = _native.lib().tritt_kernel_launches()
     _native.tdp_fwd(*t, o, lse, alpha, True, *windows, ws=ws)
+    _forward.launched = _native.lib().tritt_kernel_launches() - before   # 3 (preparation, this kernel, the band kernel) where it is asked
     torch.cuda.synchronize()
     assert _native.read_status(torch.device(DEV)) == 0, "a bounded barrier wait ran out"
     return o, lse
@@ -33,11 +35,12 @@ def _inputs(heads, T, scale, dtype, seed):
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("T", [129, 255, 256, 257, 400])
-@pytest.mark.parametrize("windows,heads", [((128, 128, 48, 48), 20), ((128, 128, 96, 0), 20), ((128, 400, 0, 96), 12), ((300, 100, 28, 9), 20),
+@pytest.mark.parametrize("windows,heads", [((128, 128, 48, 48), 27), ((128, 128, 96, 0), 27), ((128, 400, 0, 96), 27), ((300, 100, 28, 9), 27),
                                            ((1, 1, 1, 1), 120), ((0, 9, 2, 5), 120)])
 def test_against_the_oracle(windows, heads, T, dtype):
     t = _inputs(heads, T, 0.5, dtype, T + heads)
     o, lse = _forward(t, 1 / 64, windows)
+    assert _forward.launched == (2 if T == 129 and sum(windows[2:]) == 96 else 3)   # (97 diagonals of a tile of one query cost more)
     ref_o, ref_lse = orc.tdp_forward(*[x.float() for x in t], 1 / 64, True, *windows, device=DEV)
     assert_close("o", o, ref_o, dtype)
     # scores of order 0.1, operands of 8 or 11 bits: the log of a sum of exponentials moves by less than 2^-9 of the largest score
@@ -52,9 +55,8 @@ def test_long_calls_add_up_their_pieces_in_the_kernel(windows, heads, T, dtype):
     """From 128 tiles of the band kernel on (a CTA) the warp that brings the last piece of a tile adds them up, in the pieces' order:
     the same bits each time, beside calls of other inputs in the same workspace."""
     t, u = _inputs(heads, T, 0.5, dtype, T), _inputs(heads, T, 0.4, dtype, T + 1)
-    before = _native.lib().tritt_kernel_launches()
     o, lse = _forward(t, 1 / 64, windows)
-    assert _native.lib().tritt_kernel_launches() - before == 3   # preparation, this kernel, the band kernel
+    assert _forward.launched == 3
     ref_o, ref_lse = orc.tdp_forward(*[x.float() for x in t], 1 / 64, True, *windows, device=DEV)
     assert_close("o", o, ref_o, dtype)
     assert float((lse - ref_lse).abs().max()) <= 2e-3   # (as above)
@@ -66,6 +68,17 @@ def test_long_calls_add_up_their_pieces_in_the_kernel(windows, heads, T, dtype):
     t[0][0, heads - 1] *= 400   # large scores: the band kernel, bit for bit
     a, b = _forward(t, 1 / 64, windows, ws), _forward(t, 1 / 64, windows, _workspace_without_it(t))
     assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("windows,heads,T,asked", [((128, 128, 32, 32), 8, 1000, True), ((27, 22, 11, 38), 32, 768, False), ((1, 2, 47, 10), 8, 2052, False),
+                                                   ((4, 27, 35, 4), 32, 1265, True), ((60, 60, 30, 30), 4, 1000, False),
+                                                   ((20, 20, 40, 40), 16, 1000, False), ((128, 128, 48, 48), 22, 129, False), ((1, 1, 0, 0), 32, 300, False), ((99, 18, 24, 19), 64, 747, True)])
+def test_asked_where_its_steps_cost_less_than_the_other_kernels_tiles(windows, heads, T, asked):
+    """Narrow windows leave the band kernel one tile for four queries, and a wide band this one many diagonals (89 us for 59), a second tile of
+    one query doubles them (57 for 36), and a single diagonal is an item of one step (42 for 38)."""
+    _forward(_inputs(heads, T, 0.5, torch.float16, 1), 1 / 64, windows)
+    assert _forward.launched == (3 if asked else 2)
 
 
 @pytest.mark.gpu
