@@ -16,9 +16,9 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <array>
 #include <climits>
 #include <map>
-#include <tuple>
 
 namespace {
 
@@ -35,6 +35,7 @@ using Bwd1Saved = int (*)(const void*, const void*, const void*, const void*, co
                           void*, void*, void*, void*, int, int, int, int, int, float, int, int, void*, size_t, const void*, size_t, int*,
                           int, void*);
 using WorkspaceBytes = size_t (*)(int, int, int, int, int, int, int);
+using FwdWorkspace = size_t (*)(int, int, int, int, int, int, int, int, int, int, int, int);
 
 enum { kTdpFwd, kTdpBwd, kDpsFwd, kDpsBwd };   // as in tritt.h
 constexpr int kDevices = 64;
@@ -48,9 +49,10 @@ struct Entries {
   Bwd1 dps_bwd;
   Bwd1Saved dps_bwd_saved;
   WorkspaceBytes workspace_bytes;
+  FwdWorkspace tdp_fwd_workspace;
 } lib{};
 volatile int* status_words[kDevices] = {};
-std::map<std::tuple<int, int, int, int, int, int, int>, size_t> workspace_sizes;
+std::map<std::array<int, 12>, size_t> workspace_sizes;
 
 // The call's tensors have one shape [B, N, T, D], type and device.
 struct Shape {
@@ -110,16 +112,6 @@ bool read_float(PyObject* o, float& v) {
   return true;
 }
 
-size_t workspace_size(int op, const Shape& s, int flags) {
-  if (op >= kDpsFwd) flags = 0;
-  const auto key = std::make_tuple(op, s.B, s.N, s.T, s.D, s.dtype, flags);
-  const auto it = workspace_sizes.find(key);
-  if (it != workspace_sizes.end()) return it->second;
-  if (workspace_sizes.size() >= 1024) workspace_sizes.clear();
-  const size_t n = lib.workspace_bytes(op, s.B, s.N, s.T, s.D, s.dtype, flags);
-  return workspace_sizes[key] = n < 256 ? 256 : n;
-}
-
 // The scalars of a call, from argument i on: scale, causal, flags, windows (four, or the one of the dot-product-sum).
 struct Scalars {
   float scale;
@@ -135,6 +127,20 @@ bool read_scalars(PyObject* const* a, int op, const Shape& s, Scalars& c) {
   // (a kernel of an earlier call gave up, or the word is not there yet: Python reports, or makes it)
   c.status = const_cast<int*>(status_words[s.device]);
   return lib.tdp_fwd != nullptr && c.status != nullptr && *status_words[s.device] == 0;
+}
+
+size_t workspace_size(int op, const Shape& s, const Scalars& c) {
+  std::array<int, 12> key = {op, s.B, s.N, s.T, s.D, s.dtype, op < kDpsFwd ? c.flags : 0, 0, 0, 0, 0, 0};
+  if (op == kTdpFwd) {   // (what the forward makes use of depends on the mask)
+    key[7] = c.causal;
+    for (int i = 0; i < 4; ++i) key[8 + i] = c.w[i];
+  }
+  const auto it = workspace_sizes.find(key);
+  if (it != workspace_sizes.end()) return it->second;
+  if (workspace_sizes.size() >= 1024) workspace_sizes.clear();
+  const size_t n = op == kTdpFwd ? lib.tdp_fwd_workspace(s.B, s.N, s.T, s.D, s.dtype, c.causal, c.w[0], c.w[1], c.w[2], c.w[3], 1, c.flags)
+                                 : lib.workspace_bytes(op, s.B, s.N, s.T, s.D, s.dtype, key[6]);
+  return workspace_sizes[key] = n < 256 ? 256 : n;
 }
 
 // The interpreter's lock is not held while device memory is allocated (which may wait for the device) and kernels are launched.
@@ -176,7 +182,7 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   void* in[5];
   for (int i = 0; i < 5; ++i)
     if (!(in[i] = operand(a[1 + i], s))) Py_RETURN_NONE;
-  const size_t bytes = workspace_size(op, s, c.flags);
+  const size_t bytes = workspace_size(op, s, c);
   at::Tensor out[3];
   int rc;
   {
@@ -229,7 +235,7 @@ PyObject* backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     saved_bytes = (size_t)w.numel();
   }
   const float* const l = (const float*)lse.data_ptr();
-  const size_t bytes = workspace_size(op, s, c.flags);
+  const size_t bytes = workspace_size(op, s, c);
   at::Tensor out[6];
   int rc = 0;
   {
@@ -258,11 +264,12 @@ PyObject* backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// init(addresses of tritt_tdp_fwd, tritt_tdp_bwd, tritt_dps_fwd, tritt_dps_bwd, tritt_dps_bwd_saved, tritt_workspace_bytes_flags)
+// init(addresses of tritt_tdp_fwd, tritt_tdp_bwd, tritt_dps_fwd, tritt_dps_bwd, tritt_dps_bwd_saved, tritt_workspace_bytes_flags,
+// tritt_tdp_fwd_workspace)
 PyObject* init(PyObject*, PyObject* args) {
-  unsigned long long f[6];
-  if (!PyArg_ParseTuple(args, "KKKKKK", f, f + 1, f + 2, f + 3, f + 4, f + 5)) return nullptr;
-  lib = {(Fwd4)f[0], (Bwd4)f[1], (Fwd1)f[2], (Bwd1)f[3], (Bwd1Saved)f[4], (WorkspaceBytes)f[5]};
+  unsigned long long f[7];
+  if (!PyArg_ParseTuple(args, "KKKKKKK", f, f + 1, f + 2, f + 3, f + 4, f + 5, f + 6)) return nullptr;
+  lib = {(Fwd4)f[0], (Bwd4)f[1], (Fwd1)f[2], (Bwd1)f[3], (Bwd1Saved)f[4], (WorkspaceBytes)f[5], (FwdWorkspace)f[6]};
   Py_RETURN_NONE;
 }
 

@@ -154,6 +154,20 @@ size_t tritt_workspace_bytes_flags(int op, int B, int N, int T, int D, int dtype
   return align_up(a > b ? a : b, 256);
 }
 
+size_t tritt_tdp_fwd_workspace(int B, int N, int T, int D, int dtype, int causal, int k1_window, int k2_window, int kk_left,
+                               int kk_right, int q_mod, int flags) {
+  if (B <= 0 || N <= 0 || T <= 0 || D <= 0) return 0;
+  const TdpMask m = make_tdp_mask(causal, T, k1_window, k2_window, kk_left, kk_right);
+  size_t n;
+  if (tdp_wide_applies(TRITT_OP_TDP_FWD, T, D, dtype, m, flags))
+    n = tdp_wide_workspace(TRITT_OP_TDP_FWD, B, N, T, D, &m, q_mod);
+  else if (use_sm100(TRITT_OP_TDP_FWD, T, D, dtype, m, flags))
+    n = sm100_tdp_workspace(TRITT_OP_TDP_FWD, B, N, T, D, dtype) + sm100_tdp_fwd_optional_workspace(B, N, T, D, dtype, &m, q_mod);
+  else
+    n = simt_tdp_workspace(TRITT_OP_TDP_FWD, B, N, T, D, dtype);
+  return align_up(n, 256);
+}
+
 size_t tritt_tdp_bwd_partials_offset(int, int, int, int, int) { return 0; }
 
 // Bytes of scratch the forward cannot run without on the kernel family it will take (the optional tail of the

@@ -148,15 +148,17 @@ int sm100_tdp_bwd_check_registers(int launched);   // 0, or -30 if the backward 
 size_t sm100_tdp_workspace(int op, int B, int N, int T, int D, int dtype);
 size_t sm100_tdp_bwd_workspace(int B, int N, int T, int D);
 size_t sm100_tdp_bwd_optional_workspace(int B, int N);   // behind it: statistics for the range shifts
-size_t sm100_tdp_fwd_optional_workspace(int B, int N, int T, int D, int dtype);
+// ... of a call with this mask and query sharding, or (null) of any
+size_t sm100_tdp_fwd_optional_workspace(int B, int N, int T, int D, int dtype, const TdpMask* m = nullptr, int q_mod = 1);
 // forward kernel for causal masks with a narrow (j, k) band (tiles of four queries x 32 K2 rows)
 bool sm100_tdp_fwd_band_applies(int T, const TdpMask& m);
-// the scratch of the one that steps over the band's diagonals, behind the statistics in the forward's workspace
-size_t sm100_tdp_fwd_diag_workspace(int B, int N, int T, int D);
+// the scratch of the one that steps over the band's diagonals, behind the statistics in the forward's workspace: of a call with this mask
+// and query sharding (0: it is not asked), or (null) the most of any
+size_t sm100_tdp_fwd_diag_workspace(int B, int N, int T, int D, const TdpMask* m, int q_mod);
 
 // fp32 inputs, and bf16 inputs with TRITT_FLAG_WIDE_OPERANDS, on the tensor cores through fp16 operand copies
 bool tdp_wide_applies(int op, int T, int D, int dtype, const TdpMask& m, int flags);
-size_t tdp_wide_workspace(int op, int B, int N, int T, int D);
+size_t tdp_wide_workspace(int op, int B, int N, int T, int D, const TdpMask* m = nullptr, int q_mod = 1);
 int tdp_wide_fwd(const TdpArgs& a);
 int tdp_wide_bwd(const TdpArgs& a);
 

@@ -1188,11 +1188,11 @@ bool sm100_tdp_supported(int op, int T, int D, int dtype, const TdpMask& m) {
 }
 
 // Extra bytes behind the forward's SiLU(V1) copy that enable the score bound (the forward runs without them too).
-size_t sm100_tdp_fwd_optional_workspace(int B, int N, int T, int D, int dtype) {
+size_t sm100_tdp_fwd_optional_workspace(int B, int N, int T, int D, int dtype, const TdpMask* m, int q_mod) {
   if (dtype != TRITT_BF16 && dtype != TRITT_F16) return 0;
   const size_t n = (size_t)B * N * T * D;
-  return align_up(n * 2, 256) - n * 2 + align_up(kStats * (size_t)B * N * sizeof(float), 256) +
-         align_up(sm100_tdp_fwd_diag_workspace(B, N, T, D), 256);
+  const size_t diag = sm100_tdp_fwd_diag_workspace(B, N, T, D, m, q_mod);
+  return align_up(n * 2, 256) - n * 2 + align_up((diag ? kStats : 3) * (size_t)B * N * sizeof(float), 256) + align_up(diag, 256);
 }
 
 size_t sm100_tdp_workspace(int op, int B, int N, int T, int D, int dtype) {

@@ -613,24 +613,29 @@ int launch_diag(const TdpArgs& a, const DiagParams& p) {
 
 }  // namespace
 
-size_t sm100_tdp_fwd_diag_workspace(int B, int N, int T, int D) {
+size_t sm100_tdp_fwd_diag_workspace(int B, int N, int T, int D, const TdpMask* mask, int q_mod) {
   if (D != kDiagD || T <= 128) return 0;
-  return scratch_bytes(diag_grid(diag_steps(B, N, T, kMaxBand)));
+  if (!mask) return scratch_bytes(diag_grid(diag_steps(B, N, T, kMaxBand)));
+  const TdpMask& m = *mask;
+  // (a query tile meets its own j-tile and the one before: q - j <= min(k1w, k2w + kkl) <= 128)
+  if (!m.causal || q_mod != 1 || m.kkl + m.kkr > kMaxBand || (m.k1w > 128 && m.k2w + m.kkl > 128)) return 0;
+  const long steps = diag_steps(B, N, T, m.kkl + m.kkr);
+  const int grid = diag_grid(steps);
+  if (grid < 1) return 0;
+  const double R = m.kkl + m.kkr + 1, part = (double)steps / grid;
+  const double filled = min(min(m.k1w, m.k2w) + 1, 128) / 128., step = kStepPrice + (kFullStepPrice - kStepPrice) * filled;
+  if (step * part + kItemPrice * (part / R + 1) + kLaunchPrice > kTilePrice * band_tiles_of_cta((long)B * N, T, min(m.k2w, m.k1w + m.kkr))) return 0;
+  return scratch_bytes(grid);
 }
 
 bool sm100_tdp_fwd_diag_plan(const TdpArgs& a, void* workspace, size_t workspace_bytes, DiagParams& p) {
   const TdpMask& m = a.mask;
-  // (a query tile meets its own j-tile and the one before: q - j <= min(k1w, k2w + kkl) <= 128)
-  if (a.D != kDiagD || a.q_mod != 1 || m.kkl + m.kkr > kMaxBand || (m.k1w > 128 && m.k2w + m.kkl > 128)) return false;
+  const size_t need = sm100_tdp_fwd_diag_workspace(a.B, a.N, a.T, a.D, &m, a.q_mod);
+  if (need == 0 || workspace_bytes < need) return false;
   const long steps = diag_steps(a.B, a.N, a.T, m.kkl + m.kkr);
   const int grid = diag_grid(steps);
-  if (grid < 1 || workspace_bytes < scratch_bytes(grid)) return false;
-  const double R = m.kkl + m.kkr + 1, part = (double)steps / grid;
-  const double band_tiles = band_tiles_of_cta((long)a.B * a.N, a.T, min(m.k2w, m.k1w + m.kkr));
-  const double filled = min(min(m.k1w, m.k2w) + 1, 128) / 128., step = kStepPrice + (kFullStepPrice - kStepPrice) * filled;
-  if (step * part + kItemPrice * (part / R + 1) + kLaunchPrice > kTilePrice * band_tiles) return false;
   p = DiagParams{};
-  p.early = band_tiles < kEarlyBandTiles;
+  p.early = band_tiles_of_cta((long)a.B * a.N, a.T, min(m.k2w, m.k1w + m.kkr)) < kEarlyBandTiles;
   p.out = a.out_o;
   p.lse = a.out_lse;
   p.k1 = a.k1;

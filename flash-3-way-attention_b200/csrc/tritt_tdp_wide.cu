@@ -100,11 +100,11 @@ bool tdp_wide_applies(int op, int T, int D, int dtype, const TdpMask& m, int fla
   return asked && sm100_tdp_supported(op, T, D, TRITT_F16, m);
 }
 
-size_t tdp_wide_workspace(int op, int B, int N, int T, int D) {
+size_t tdp_wide_workspace(int op, int B, int N, int T, int D, const TdpMask* m, int q_mod) {
   const size_t n = (size_t)B * N * T * D;
   if (op == TRITT_OP_TDP_FWD)
     return 6 * half_seg(n) + align_up(sm100_tdp_workspace(op, B, N, T, D, TRITT_F16) +
-                                      sm100_tdp_fwd_optional_workspace(B, N, T, D, TRITT_F16), 256);
+                                      sm100_tdp_fwd_optional_workspace(B, N, T, D, TRITT_F16, m, q_mod), 256);
   return 7 * half_seg(n) + 256 + align_up(sm100_tdp_workspace(op, B, N, T, D, TRITT_F16), 256) +
          sm100_tdp_bwd_optional_workspace(B, N);
 }

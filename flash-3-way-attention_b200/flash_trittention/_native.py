@@ -27,7 +27,7 @@ _DTYPES = {torch.float32: F32, torch.float16: F16, torch.bfloat16: BF16}
 # every symbol include/tritt.h declares
 SYMBOLS = (
     "tritt_version", "tritt_kernel_launches", "tritt_last_error", "tritt_workspace_bytes", "tritt_workspace_bytes_flags",
-    "tritt_tdp_fwd_min_workspace", "tritt_tdp_path", "tritt_dps_path", "tritt_tdp_fwd",
+    "tritt_tdp_fwd_workspace", "tritt_tdp_fwd_min_workspace", "tritt_tdp_path", "tritt_dps_path", "tritt_tdp_fwd",
     "tritt_tdp_bwd", "tritt_tdp_bwd_finalize", "tritt_tdp_bwd_partials_offset", "tritt_dps_fwd",
     "tritt_dps_bwd", "tritt_dps_bwd_saved", "tritt_selftest_umma", "tritt_selftest_wait_expiry", "tritt_tdp_fwd_noalloc",
     "tritt_noalloc_scratch_bytes", "tritt_selftest_bwd_registers",
@@ -65,7 +65,8 @@ def _load_host(L):
                       "with `python flash-3-way-attention_b200/build.py`", stacklevel=3)
         return
     _host.init(*(C.cast(f, C.c_void_p).value for f in (L.tritt_tdp_fwd, L.tritt_tdp_bwd, L.tritt_dps_fwd, L.tritt_dps_bwd,
-                                                       L.tritt_dps_bwd_saved, L.tritt_workspace_bytes_flags)))
+                                                       L.tritt_dps_bwd_saved, L.tritt_workspace_bytes_flags,
+                                                       L.tritt_tdp_fwd_workspace)))
     for device, address in _status_ptr.items():
         _host.set_status(device, address)
     host_forward, host_backward = _host.forward, _host.backward
@@ -90,6 +91,8 @@ def lib():
                 L.tritt_workspace_bytes.argtypes = [i] * 6
                 L.tritt_workspace_bytes_flags.restype = sz
                 L.tritt_workspace_bytes_flags.argtypes = [i] * 7
+                L.tritt_tdp_fwd_workspace.restype = sz
+                L.tritt_tdp_fwd_workspace.argtypes = [i] * 12
                 L.tritt_tdp_fwd_min_workspace.restype = sz
                 L.tritt_tdp_fwd_min_workspace.argtypes = [i] * 11
                 L.tritt_tdp_path.restype = i
@@ -232,6 +235,19 @@ def _workspace_bytes(op: int, B: int, N: int, T: int, D: int, dtype: int, flags:
     return max(int(lib().tritt_workspace_bytes_flags(op, B, N, T, D, dtype, flags)), 256)
 
 
+@functools.lru_cache(maxsize=1024)
+def _tdp_fwd_workspace_bytes(*args) -> int:
+    return max(int(lib().tritt_tdp_fwd_workspace(*args)), 256)
+
+
+def tdp_fwd_workspace(B: int, N: int, T: int, D: int, dtype: int, causal, k1w, k2w, kkl, kkr, device, q_mod: int = 1,
+                      flags: int = 0) -> torch.Tensor:
+    """What a forward with these windows makes use of (``workspace`` holds the most that any mask does)."""
+    n = _tdp_fwd_workspace_bytes(B, N, T, D, dtype, int(bool(causal)), _win(k1w, T), _win(k2w, T), _win(kkl, T), _win(kkr, T), q_mod,
+                                 flags)
+    return torch.empty(n, dtype=torch.uint8, device=device)
+
+
 def workspace(op: int, B: int, N: int, T: int, D: int, dtype: int, device, flags: int = 0) -> torch.Tensor:
     return torch.empty(_workspace_bytes(op, B, N, T, D, dtype, flags), dtype=torch.uint8, device=device)
 
@@ -287,14 +303,14 @@ def dps_path(T, D, dtype, k_diff, flags=0) -> int:
 
 
 def tdp_fwd(q, k1, k2, v1, v2, o, lse, alpha, causal, k1w, k2w, kkl, kkr, q_mod=1, q_rem=0, flags=0, ws=None):
-    """``ws``: a caller-provided workspace (uint8 tensor) instead of one of ``tritt_workspace_bytes`` bytes."""
+    """``ws``: a caller-provided workspace (uint8 tensor) instead of one of ``tritt_tdp_fwd_workspace`` bytes."""
     global launches
     B, N, T, D = q.shape
     dt = dtype_code(q.dtype)
     check_status(q.device, synchronize=False)
     with _on_device(q.device):
         if ws is None:
-            ws = workspace(OP_TDP_FWD, B, N, T, D, dt, q.device, flags)
+            ws = tdp_fwd_workspace(B, N, T, D, dt, causal, k1w, k2w, kkl, kkr, q.device, q_mod, flags)
         rc = lib().tritt_tdp_fwd(q.data_ptr(), k1.data_ptr(), k2.data_ptr(), v1.data_ptr(), v2.data_ptr(),
                                  o.data_ptr(), lse.data_ptr(), B, N, T, D, dt, float(alpha), int(bool(causal)),
                                  _win(k1w, T), _win(k2w, T), _win(kkl, T), _win(kkr, T), q_mod, q_rem,

@@ -69,9 +69,11 @@ unsigned long long tritt_kernel_launches(void);
 const char* tritt_last_error(void);
 
 /* Bytes of caller-provided scratch to pass to the given operation (0 if none).  For TRITT_OP_TDP_FWD on 16-bit inputs
-   the figure includes a small tail (three floats per (batch, head), behind the SiLU(V1) copy of B*N*T*D elements) that
-   lets the forward bound its scores and skip the row-maximum pass; a workspace without the tail is accepted and runs
-   the two-pass soft-max.  For TRITT_OP_TDP_BWD on the tensor cores it includes a tail of about 1 KiB per (batch, head)
+   the figure includes a tail behind the SiLU(V1) copy of B*N*T*D elements: up to seven floats per (batch, head), which
+   let the forward bound its scores and skip the row-maximum pass, and for head dimension 64 and T > 128 up to 20 MB
+   (4 * 33 KB per SM) for the kernel that serves narrow bands with small scores.  A workspace without the last part is
+   accepted and runs the slower kernel there, one without the tail the two-pass soft-max.  tritt_tdp_fwd_workspace()
+   gives what a call with known windows uses: calls without a narrow band have no need of the 20 MB.  For TRITT_OP_TDP_BWD on the tensor cores it includes a tail of about 1 KiB per (batch, head)
    for the largest elements behind the range shifts of fp16 products; a workspace without it is accepted and forms them
    without regard to their size, times alpha (at most 1, to a power of two) for the keys: small keys or values then lose
    bits to fp16's subnormals, and keys whose products times alpha reach 65504 overflow. */
@@ -80,7 +82,10 @@ size_t tritt_workspace_bytes(int op, int B, int N, int T, int D, int dtype);
    inputs by the fp16 operand copies; tritt_workspace_bytes() equals flags = 0). */
 size_t tritt_workspace_bytes_flags(int op, int B, int N, int T, int D, int dtype, int flags);
 
-/* Bytes of scratch tritt_tdp_fwd cannot run without for these arguments (the optional score-bound tail excluded). */
+/* Bytes of scratch that tritt_tdp_fwd makes use of for these arguments: never more than tritt_workspace_bytes_flags(). */
+size_t tritt_tdp_fwd_workspace(int B, int N, int T, int D, int dtype, int causal, int k1_window, int k2_window, int kk_left,
+                               int kk_right, int q_mod, int flags);
+/* Bytes of scratch tritt_tdp_fwd cannot run without for these arguments (the optional tail excluded). */
 size_t tritt_tdp_fwd_min_workspace(int B, int N, int T, int D, int dtype, int causal, int k1_window, int k2_window,
                                    int kk_left, int kk_right, int flags);
 

@@ -40,6 +40,22 @@ def test_workspace_sizes():
     assert lib.tritt_workspace_bytes(_native.OP_TDP_FWD, 0, N, T, D, 0) == 0
 
 
+@pytest.mark.parametrize("dtype", [_native.F16, _native.BF16, _native.F32])
+def test_the_forwards_workspace_goes_by_its_windows(dtype):
+    """SiLU(V1), or the fp16 copies of fp32 tensors, and a little more, but where the kernel over a narrow band's diagonals is asked; never
+    more than the size for any mask, never less than the least."""
+    lib = _native.lib()
+    B, N, T, D = 4, 8, 2048, 64
+    n, most = B * N * T * D * (2 if dtype != _native.F32 else 14), lib.tritt_workspace_bytes(_native.OP_TDP_FWD, B, N, T, D, dtype)
+    for causal, windows, q_mod, large in [(0, (T, T, T, T), 1, False), (1, (T, T, T, T), 1, False), (1, (128, 128, 32, 32), 1, True),
+                                          (1, (128, 128, 32, 32), 2, False), (0, (128, 128, 32, 32), 1, False), (1, (300, 300, 32, 32), 1, False),
+                                          (1, (128, 128, 90, 32), 1, False), (1, (128, 128, 96, 0), 1, True)]:
+        got = lib.tritt_tdp_fwd_workspace(B, N, T, D, dtype, causal, *windows, q_mod, 0)
+        assert lib.tritt_tdp_fwd_min_workspace(B, N, T, D, dtype, causal, *windows, 0) <= got <= most
+        assert (n + 15e6 < got) if large else (n < got <= n + 8192), (causal, windows, q_mod)
+    assert lib.tritt_tdp_fwd_workspace(B, N, T, 48, dtype, 1, T, T, T, T, 1, 0) == 0   # (the CUDA cores' kernel needs none)
+
+
 def test_c_abi_rejects_bad_arguments_without_a_device():
     lib = _native.lib()
     buf = ctypes.create_string_buffer(4096 + 256)

@@ -80,6 +80,24 @@ def test_against_the_python_code(op, kw, dtype, monkeypatch):
     assert _native.read_status(DEV) == 0
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("take", [False, True])
+@pytest.mark.parametrize("windows,most", [((None,) * 4, 12e6), ((128, 128, 32, 32), 40e6)])
+def test_a_forward_allocates_what_its_windows_need(windows, most, take, monkeypatch):
+    ins = _tensors((4, 8, 600, 64), torch.float16, grad=False)
+    kw = dict(softmax_scale=1 / 64, k1_window=windows[0], k2_window=windows[1], kk_left=windows[2], kk_right=windows[3])
+    _loaded()
+    _native.status_word(DEV)
+    Counted(monkeypatch, take)
+    flash_trittention(*ins, **kw)
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    flash_trittention(*ins, **kw)
+    used = torch.cuda.max_memory_allocated() - before
+    assert used <= most and (windows[0] is None or used > 16e6)   # (tensors of 2.5 MB; the areas of a narrow band 20 MB)
+
+
 class Labelled(torch.Tensor):
     pass
 
