@@ -20,36 +20,23 @@
 #include <climits>
 #include <map>
 
+#include "tritt.h"
+
 namespace {
 
-using Fwd4 = int (*)(const void*, const void*, const void*, const void*, const void*, void*, float*, int, int, int, int, int, float, int,
-                     int, int, int, int, int, int, void*, size_t, int*, int, void*);
-using Bwd4 = int (*)(const void*, const void*, const void*, const void*, const void*, const void*, const void*, const float*, void*, void*,
-                     void*, void*, void*, int, int, int, int, int, float, int, int, int, int, int, int, int, void*, size_t, int*, int,
-                     void*);
-using Fwd1 = int (*)(const void*, const void*, const void*, const void*, const void*, void*, float*, int, int, int, int, int, float, int,
-                     int, void*, size_t, int*, int, void*);
-using Bwd1 = int (*)(const void*, const void*, const void*, const void*, const void*, const void*, const void*, const float*, void*, void*,
-                     void*, void*, void*, int, int, int, int, int, float, int, int, void*, size_t, int*, int, void*);
-using Bwd1Saved = int (*)(const void*, const void*, const void*, const void*, const void*, const void*, const void*, const float*, void*,
-                          void*, void*, void*, void*, int, int, int, int, int, float, int, int, void*, size_t, const void*, size_t, int*,
-                          int, void*);
-using WorkspaceBytes = size_t (*)(int, int, int, int, int, int, int);
-using FwdWorkspace = size_t (*)(int, int, int, int, int, int, int, int, int, int, int, int);
-
-enum { kTdpFwd, kTdpBwd, kDpsFwd, kDpsBwd };   // as in tritt.h
+enum { kTdpFwd = TRITT_OP_TDP_FWD, kTdpBwd = TRITT_OP_TDP_BWD, kDpsFwd = TRITT_OP_DPS_FWD, kDpsBwd = TRITT_OP_DPS_BWD };
 constexpr int kDevices = 64;
 constexpr int kNotPlain = INT_MIN;   // no code of the library's
 
 // Everything below is read and written with the interpreter's lock held.
-struct Entries {
-  Fwd4 tdp_fwd;
-  Bwd4 tdp_bwd;
-  Fwd1 dps_fwd;
-  Bwd1 dps_bwd;
-  Bwd1Saved dps_bwd_saved;
-  WorkspaceBytes workspace_bytes;
-  FwdWorkspace tdp_fwd_workspace;
+struct Entries {   // (the addresses come from Python, which has loaded the library)
+  decltype(&tritt_tdp_fwd) tdp_fwd;
+  decltype(&tritt_tdp_bwd) tdp_bwd;
+  decltype(&tritt_dps_fwd) dps_fwd;
+  decltype(&tritt_dps_bwd) dps_bwd;
+  decltype(&tritt_dps_bwd_saved) dps_bwd_saved;
+  decltype(&tritt_workspace_bytes_flags) workspace_bytes;
+  decltype(&tritt_tdp_fwd_workspace) tdp_fwd_workspace;
 } lib{};
 volatile int* status_words[kDevices] = {};
 std::map<std::array<int, 12>, size_t> workspace_sizes;
@@ -69,7 +56,7 @@ bool aligned(const void* p) { return p != nullptr && (reinterpret_cast<uintptr_t
 bool read_shape(const at::Tensor& q, Shape& s) {
   if (!usable(q) || q.dim() != 4) return false;
   s.type = q.scalar_type();
-  s.dtype = s.type == at::kFloat ? 0 : s.type == at::kHalf ? 1 : s.type == at::kBFloat16 ? 2 : -1;
+  s.dtype = s.type == at::kFloat ? TRITT_F32 : s.type == at::kHalf ? TRITT_F16 : s.type == at::kBFloat16 ? TRITT_BF16 : -1;
   for (int i = 0; i < 4; ++i)
     if (q.size(i) > INT_MAX) return false;
   s.B = (int)q.size(0);
@@ -269,7 +256,8 @@ PyObject* backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* init(PyObject*, PyObject* args) {
   unsigned long long f[7];
   if (!PyArg_ParseTuple(args, "KKKKKKK", f, f + 1, f + 2, f + 3, f + 4, f + 5, f + 6)) return nullptr;
-  lib = {(Fwd4)f[0], (Bwd4)f[1], (Fwd1)f[2], (Bwd1)f[3], (Bwd1Saved)f[4], (WorkspaceBytes)f[5], (FwdWorkspace)f[6]};
+  lib = {(decltype(lib.tdp_fwd))f[0],       (decltype(lib.tdp_bwd))f[1],         (decltype(lib.dps_fwd))f[2],          (decltype(lib.dps_bwd))f[3],
+         (decltype(lib.dps_bwd_saved))f[4], (decltype(lib.workspace_bytes))f[5], (decltype(lib.tdp_fwd_workspace))f[6]};
   Py_RETURN_NONE;
 }
 
@@ -291,4 +279,12 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__host() {
+  PyObject* m = PyModule_Create(&module);
+  // (the version whose headers this was compiled with: objects' layouts are its own)
+  if (m && PyModule_AddStringConstant(m, "torch_version", TRITT_TORCH_VERSION) < 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

@@ -59,11 +59,15 @@ def host_backward(*args):
 def _load_host(L):
     global _host, host_forward, host_backward
     try:
-        _host = importlib.import_module("._host", __package__)
+        host = importlib.import_module("._host", __package__)
+        built_for = getattr(host, "torch_version", "another version")
+        if built_for != torch.__version__:
+            raise ImportError(f"built for PyTorch {built_for}, not {torch.__version__}")
     except ImportError as e:
         warnings.warn(f"the host extension of flash_trittention cannot be loaded ({e}): short calls take twice as long; build it "
                       "with `python flash-3-way-attention_b200/build.py`", stacklevel=3)
         return
+    _host = host
     _host.init(*(C.cast(f, C.c_void_p).value for f in (L.tritt_tdp_fwd, L.tritt_tdp_bwd, L.tritt_dps_fwd, L.tritt_dps_bwd,
                                                        L.tritt_dps_bwd_saved, L.tritt_workspace_bytes_flags,
                                                        L.tritt_tdp_fwd_workspace)))

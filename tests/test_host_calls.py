@@ -1,4 +1,7 @@
 """Calls made by the native host extension against the same calls made by the Python code, and whom it leaves to that code."""
+import importlib.util
+import os
+
 import pytest
 import torch
 
@@ -21,6 +24,44 @@ def test_what_the_extension_does_not_take():
     assert host.forward(_native.OP_TDP_FWD, *[x] * 5, *SCALARS, 1, 1, 1, 1) is None          # not on a GPU
     assert host.forward(_native.OP_TDP_FWD, *["q"] * 5, *SCALARS, 1, 1, 1, 1) is None
     assert host.backward(_native.OP_DPS_BWD, *[x] * 8, *SCALARS, 4, None) is None
+
+
+def test_an_extension_for_another_pytorch_is_not_used(monkeypatch):
+    L = _native.lib()
+    for name in ("_host", "host_forward", "host_backward"):
+        monkeypatch.setattr(_native, name, None)
+    monkeypatch.setattr(torch, "__version__", "0.1")
+    with pytest.warns(UserWarning, match="built for PyTorch .* not 0.1"):
+        _native._load_host(L)
+    assert _native._host is None and _native.host_forward is None
+
+
+def test_the_extension_is_rebuilt_for_what_it_depends_on(monkeypatch, tmp_path):
+    path = os.path.join(os.path.dirname(os.path.dirname(_native.LIB_PATH)), "build.py")
+    spec = importlib.util.spec_from_file_location("tritt_build", path)
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    files = {name: str(tmp_path / name) for name in ("HOST", "HOST_STAMP", "HOST_SRC", "ABI_HEADER")}
+    for i, (name, f) in enumerate(files.items()):
+        monkeypatch.setattr(build, name, f)
+        open(f, "w").close()
+        os.utime(f, (1000, 1000))
+    recipe = build._host_recipe()
+    os.utime(files["HOST"], (2000, 2000))
+    assert not build.host_is_current(recipe)   # an extension of which nothing is known
+    with open(files["HOST_STAMP"], "w") as f:
+        f.write("\n".join(recipe))
+    assert build.host_is_current(recipe)
+    for name in ("HOST_SRC", "ABI_HEADER"):
+        os.utime(files[name], (3000, 3000))
+        assert not build.host_is_current(recipe), name
+        os.utime(files[name], (1000, 1000))
+    monkeypatch.setattr(torch, "__version__", "0.1")
+    assert not build.host_is_current(build._host_recipe())
+    # without a compiler the library is built alone
+    monkeypatch.setattr(build.shutil, "which", lambda name: None)
+    with pytest.warns(UserWarning, match="host extension was not built.*g.. not found"):
+        build.build_host_if_possible()
 
 
 class Counted:
