@@ -64,6 +64,25 @@ template <typename T16, bool NAN_TOO> __device__ __forceinline__ void grow_abs(u
   }
 }
 
+// fp16 only: A = K1 K2 and A' = SiLU(V1) V2 (the forward's W) are products of two small factors (keys of 0.01: 1e-4, against a smallest normal
+// value of 6e-5) or of two large ones (beyond 65504 from 256 on), so one factor, x, is taken times a power of two per head:
+// the largest that keeps both itself and the largest product the head's elements allow below 2^15.  With the other factor's
+// largest element at 1 or above the largest product has 28 binades of normal numbers below it, at 2^-b 28 - b.
+// The power is divided out in fp32, of S and dP in the soft-max warps and of the sums.  bf16 has fp32's range: 0.
+// Without statistics (or with infinite ones) the power is `otherwise`.
+template <typename T16> __device__ __forceinline__ int range_shift(float x, float other, int otherwise) {
+  if constexpr (std::is_same<T16, __half>::value) {
+    if (!(x > 0.f) || !isfinite(x) || !(other > 0.f) || !isfinite(other)) return otherwise;
+    const int a = (__float_as_int(x) >> 23) - 127, b = (__float_as_int(other) >> 23) - 127;
+    return 14 - a - max(b + 1, 0);
+  }
+  return 0;
+}
+// 2^e for the shifts of fp16 operands, exact, |e| <= 126 (1, without looking at e, for bf16, whose shifts are all 0)
+template <typename T16> __device__ __forceinline__ float pow2i(int e) {
+  return std::is_same<T16, __half>::value ? __int_as_float((127 + e) << 23) : 1.f;
+}
+
 // Bits c of [lo, hi] among 0..31: with a mask of a row's columns a per-element test is one logic instruction (a constant
 // bit into a predicate) instead of two comparisons.
 __device__ __forceinline__ uint32_t column_mask(int lo, int hi) {

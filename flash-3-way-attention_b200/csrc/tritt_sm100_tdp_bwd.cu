@@ -253,20 +253,6 @@ __device__ __forceinline__ int prob_shift(int q, int causal, int T, int k1w, int
   return 0;
 }
 
-// fp16 only: A = K1 K2 and A' = SiLU(V1) V2 are products of two small factors (keys of 0.01: 1e-4, against a smallest normal
-// value of 6e-5) or of two large ones (beyond 65504 from 256 on), so one factor, x, is taken times a power of two per head:
-// the largest that keeps both itself and the largest product the head's elements allow below 2^15.  With the other factor's
-// largest element at 1 or above the largest product has 28 binades of normal numbers below it, at 2^-b 28 - b.
-// The power is divided out in fp32, of S and dP in the soft-max warps and of the sums.  bf16 has fp32's range: 0.
-// Without statistics (or with infinite ones) the power is `otherwise`.
-template <typename T16> __device__ __forceinline__ int range_shift(float x, float other, int otherwise) {
-  if constexpr (std::is_same<T16, __half>::value) {
-    if (!(x > 0.f) || !isfinite(x) || !(other > 0.f) || !isfinite(other)) return otherwise;
-    const int a = (__float_as_int(x) >> 23) - 127, b = (__float_as_int(other) >> 23) - 127;
-    return 14 - a - max(b + 1, 0);
-  }
-  return 0;
-}
 // A's power without statistics: as large as alpha log2(e), so that keys of 300 under an alpha of 1/64 do not overflow, and at most
 // 1; 2^-17 keeps every product of two fp16 numbers finite.
 __device__ __forceinline__ int alpha_shift(float alpha) {
@@ -290,11 +276,6 @@ template <typename T16> __device__ __forceinline__ int ds_shift(float bound) {
     return min(24, max(0, 3 - ((__float_as_int(bound) >> 23) - 127)));
   }
   return 0;
-}
-
-// 2^e for the shifts above, exact, |e| <= 126 (1, without looking at e, for bf16, whose shifts are all 0)
-template <typename T16> __device__ __forceinline__ float pow2i(int e) {
-  return std::is_same<T16, __half>::value ? __int_as_float((127 + e) << 23) : 1.f;
 }
 
 __device__ __forceinline__ void red_add(float* p, float v) {

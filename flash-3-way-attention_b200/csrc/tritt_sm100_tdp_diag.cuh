@@ -56,20 +56,6 @@ namespace {
 // Statistics of fwd_prepare_kernel: arrays of BN values.
 enum { kK1 = 3, kK2 = 4, kV1 = 5, kV2 = 6 };   // largest |element|
 
-// fp16 only: the power of two that A carries, as in the backward (range_shift there), so that both form the same operand: the
-// largest that keeps the factor and the products below 2^15; W's likewise.
-template <typename T16> __device__ __forceinline__ int product_range(float x, float other) {
-  if constexpr (std::is_same<T16, __half>::value) {
-    if (!(x > 0.f) || !isfinite(x) || !(other > 0.f) || !isfinite(other)) return 0;
-    const int a = (__float_as_int(x) >> 23) - 127, b = (__float_as_int(other) >> 23) - 127;
-    return 14 - a - max(b + 1, 0);
-  }
-  return 0;
-}
-template <typename T16> __device__ __forceinline__ float pow2i(int e) {
-  return std::is_same<T16, __half>::value ? __int_as_float((127 + e) << 23) : 1.f;
-}
-
 // The soft-max reference of all rows of a head, from the bound on its scores: P = exp2(S - reference) is below 2^15 in fp16, 1 in bf16.
 template <typename T16> __device__ __forceinline__ float diag_reference(float bound) {
   return ceilf(bound) + kDiagReferenceFraction - (std::is_same<T16, __half>::value ? 15.f : 0.f);
@@ -109,7 +95,7 @@ __device__ __forceinline__ void diag_merge(const DiagParams& p) {
       for (int c = 0; c < 16; ++c) v[c] += a[(c0 % (kDiagD / 2) + c) * 128];
     }
     const float* st = p.stats + bh;
-    const float scale = pow2i<T16>(-product_range<T16>(__ldg(st + kV1 * g.BN), __ldg(st + kV2 * g.BN))) / l;
+    const float scale = pow2i<T16>(-range_shift<T16>(__ldg(st + kV1 * g.BN), __ldg(st + kV2 * g.BN), 0)) / l;
     T16* dst = (T16*)p.out + ((size_t)bh * g.T + q) * kDiagD + c0;
 #pragma unroll
     for (int c = 0; c < 16; c += 8)

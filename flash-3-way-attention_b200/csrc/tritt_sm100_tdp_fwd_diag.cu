@@ -485,8 +485,8 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             joined = false;
             const float* st = p.stats + head;
             const float bound = head_bound(p.stats, g.BN, head, p.alpha * kLog2e);
-            it.ea = product_range<T16>(__ldg(st + kK1 * g.BN), __ldg(st + kK2 * g.BN));
-            it.eb = product_range<T16>(__ldg(st + kV1 * g.BN), __ldg(st + kV2 * g.BN));
+            it.ea = range_shift<T16>(__ldg(st + kK1 * g.BN), __ldg(st + kK2 * g.BN), 0);
+            it.eb = range_shift<T16>(__ldg(st + kV1 * g.BN), __ldg(st + kV2 * g.BN), 0);
             it.sa = pow2i<T16>(-it.ea) * fabsf(p.alpha * kLog2e);
             it.reference = diag_reference<T16>(bound);
           }
