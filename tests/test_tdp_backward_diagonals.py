@@ -129,6 +129,18 @@ def test_a_key_that_is_not_finite_reaches_no_query_of_the_tile_before(which, val
 
 
 @pytest.mark.gpu
+def test_fp32_tensors():
+    """Through their fp16 copies: dO's largest element, the copies, and what a 16-bit call launches."""
+    windows = (128, 128, 36, 36)
+    t, do = _inputs(60, 391, torch.float32, 7)
+    got, launched = _backward(t, do, 1 / 64, windows)
+    assert launched == 7
+    ref = orc.tdp_backward(*t, do, 1 / 64, True, *windows, device=DEV)
+    for name, a, b in zip(NAMES, got, ref):
+        assert_close(name, a, b, torch.float16)
+
+
+@pytest.mark.gpu
 def test_capture():
     windows = (128, 128, 36, 36)
     t, do = _inputs(60, 391, torch.bfloat16, 5)

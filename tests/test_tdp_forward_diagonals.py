@@ -100,6 +100,45 @@ def test_fp16_scores_near_their_bound(sign):
     assert float((a[1] - ref_lse).abs().max()) <= 5e-3
 
 
+def _bound(t):
+    """|Q row| |K1 row| max|K2|, the factor of alpha in the bound on a head's scores, of the head that has the largest."""
+    q, k1, k2 = (x[0].float() for x in t[:3])
+    return float((q.norm(dim=-1).amax(-1) * k1.norm(dim=-1).amax(-1) * k2.abs().amax((1, 2))).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sign", [1, -1])
+@pytest.mark.parametrize("dtype,limit", [(torch.bfloat16, 16), (torch.float16, 13.5)])
+def test_scores_just_within_the_bound_and_just_beyond(dtype, limit, sign):
+    """Rows that are all alike, and an alpha that puts the bound one part in a thousand below the limit, or above it."""
+    windows, heads, T = (128, 128, 32, 32), 16, 300
+    t = _inputs(heads, T, 0.1, dtype, 8)
+    for x in t[:3]:
+        x += 1
+    t[0] *= sign
+    for factor in (0.999, 1.001):
+        alpha = factor * limit / _bound(t) / 1.4426950408889634
+        a, b = _forward(t, alpha, windows), _forward(t, alpha, windows, _workspace_without_it(t))
+        assert torch.equal(a[0], b[0]) == (factor > 1)
+        ref_o, ref_lse = orc.tdp_forward(*[x.float() for x in t], alpha, True, *windows, device=DEV)
+        assert_close("o", a[0], ref_o, dtype)
+        # a score of 11 (9 in fp16) in natural units moves by its operands' rounding, 2^-9 (2^-12) of it, twice
+        assert float((a[1] - ref_lse).abs().max()) <= (0.045 if dtype == torch.bfloat16 else 5e-3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T", [300, 1024])
+def test_fp32_tensors(T):
+    """Through their fp16 copies: the conversions to and from, the preparation and the two kernels."""
+    windows, heads = (128, 128, 32, 32), 16
+    t = _inputs(heads, T, 0.5, torch.float32, T)
+    o, lse = _forward(t, 1 / 64, windows)
+    assert _forward.launched == 5
+    ref_o, ref_lse = orc.tdp_forward(*t, 1 / 64, True, *windows, device=DEV)
+    assert_close("o", o, ref_o, torch.float16)   # (the operands' and the output's type)
+    assert float((lse - ref_lse).abs().max()) <= 2e-3
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_large_scores_of_one_head_are_left_to_the_other_kernel(dtype):
