@@ -40,8 +40,9 @@
 // (vector reductions; the SMs together take 5.8 TB/s of them, twice what a step asks for) where stepping over k adds two rows.  All
 // 128 x 128 of an item's cells lie in the band, of which a step over k has a band's width.  What bounds it: the fold warps, 4800
 // cycles a step (operands 1500, fold 3100) whose spills and exchanges between lanes count most.  us per backward, steps over k ->
-// diagonals: 16 heads T=2048 fp16 windows 128/128/32/32 951 -> 615, 256/256/40/20 1378 -> 830, 8/8/4/4 529 -> 164, 400/400/36/36
-// 1818 -> 1400; without windows, band 32/32 T=1024 1094 -> 715, 16/16 T=512 322 -> 146.
+// diagonals: 16 heads T=2048 fp16 windows 128/128/32/32 951 -> 606, 256/256/40/20 1378 -> 808, 8/8/4/4 529 -> 150, 400/400/36/36
+// 1818 -> 1366; without windows, band 32/32 T=1024 1094 -> 690, 16/16 T=512 322 -> 133.  A head is this kernel's or the one's over k
+// (diag_head), as its scores and elements are.
 //
 // Tile shapes: the accumulators S | dP | G | U | dQ have to fit 512 columns of tensor memory.  Head dimension 64:
 // JT = 128, G and U as [j x h] (128 + 128 + 64 + 64 + 64).  Head dimension 128: JT = 64 and G, U transposed,
@@ -61,8 +62,8 @@ using namespace sm100;
 
 constexpr int kBwdThreads = 640;
 // Registers per thread: 640 threads are launched with 96 each (480 per lane of the five warpgroups) and split them anew.  The
-// shares are tight: the two bodies spill 380 to 530 bytes a thread together, most of it what an item or a step reads once or
-// twice.  (80 / 128 / 64 or 96 / 120 / 48 for soft-max, fold and service warps in the small-score body: 5 to 8 % slower, as their
+// shares are tight: the two bodies spill 420 to 520 bytes a thread together, the one over diagonals 280 to 350, most of it what an item
+// or a step reads once or twice.  (80 / 128 / 64 or 96 / 120 / 48 for soft-max, fold and service warps in the small-score body: 5 to 8 % slower, as their
 // loops spill.)
 constexpr int kRegsLaunch = 96;
 // (88 / 136 / 32 for large scores at head dimension 64, where R's warps spill then: fp16 16 heads T=512 916 -> 927 us, bf16 T=2048 4 heads
@@ -489,7 +490,7 @@ __device__ __forceinline__ void tdp_bwd_body(const CUtensorMap& tmQ, const CUten
     const int4 a = *reinterpret_cast<const int4*>(&bars.items[items % kItemSlots]);
     const int4 b = *reinterpret_cast<const int4*>(&bars.items[items % kItemSlots].len);
     // (every lane has the same; the reductions tell the compiler so, which keeps what follows from them on the uniform datapath:
-    // backward of T=2048 D=128 bf16 16 heads 64.7 -> 63.2 ms, T=512 D=64 fp16 not causal 1.67 -> 1.62, T=333 D=128 169 -> 165 us)
+    // with large scores 16 heads T=512 D=64 fp16 936 -> 927 us, 4 heads T=300 123 -> 122; with small ones less than runs differ)
     auto uniform = [](int v) -> int { return __reduce_max_sync(0xffffffffu, v); };
     it.bh = uniform(a.x); it.qt = uniform(a.y); it.jt = uniform(a.z); it.k0 = uniform(a.w);
     it.len = uniform(b.x); it.flags = uniform(b.y); it.ea = uniform(b.z); it.eb = uniform(b.w);
@@ -1663,7 +1664,8 @@ constexpr int kMinStride = 8;
 // Diagonals are taken where they are fewer by more than a step's higher price and a launch.  Steps and items of a CTA, k / diagonals: us
 // with k / diagonals, D=64:  140 / 123: 325 / 350, 74 / 62: 192 / 195, 30 / 25: 98 / 104, 1.4 / 0.3: 75 / 76, 15 / 9: 75 / 77,
 // 24 / 9: 87 / 79, 41 / 26: 124 / 110, 31 / 3: 104 / 76, 45 / 9: 135 / 80, 54 / 28: 146 / 114, 449 / 228: 951 / 615, 871 / 548: 1818 / 1400.
-// Calls with large scores pay for a kernel that does nothing: 449 / 228: 1051 / 1060, 82 / 12: 218 / 223.
+// Calls with large scores pay for a kernel that does nothing, without / with it: 16 heads T=2048 windows 128/128/0/0 978 / 983, T=512 band 0/0
+// 332 / 334, 8 heads T=633 windows 19/9/2/3 118 / 120.
 constexpr double kDiagPrice = 1.3, kDiagGain = 6;
 
 // Steps and items of one head.

@@ -18,8 +18,8 @@
 //   warp 1       tcgen05.mma issuer: S(t), then P V of tile t - 1, so that a tile's soft-max overlaps its neighbour's products
 //   warps 4-7    soft-max warpgroup of slot 0, warps 8-11 of slot 1 (one row per thread; they also form A)
 //   warps 12-15  fold warpgroup: warp g owns query q_g (the V2 factor comes from the block in shared memory)
-// Calls with small scores at head dimension 64 are left to the kernel that steps over diagonals (tritt_sm100_tdp_fwd_diag.cu), ahead of this
-// one, which then adds up the tiles that the other has cut.
+// Calls with small scores at head dimension 64 are left to the kernel that steps over diagonals (tritt_sm100_tdp_fwd_diag.cu), which is
+// launched ahead of this one where such a call pays; in short calls this one then adds up the tiles that the other has cut.
 // The kernel is bound by the instruction issue of the soft-max and fold warps (a tile is 16 K exponentials with
 // per-element column masks for ~12 M flop), not by the tensor pipe or by memory.
 #include "tritt_common.cuh"

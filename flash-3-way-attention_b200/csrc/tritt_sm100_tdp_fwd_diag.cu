@@ -8,19 +8,21 @@
 // is attended.  (Tiles of 4 queries x 32 K2 rows against a slab of 128 columns, tdp_fwd_band_kernel, fill a third of the slab and
 // pay for an operand, a fold and two reads of the accumulator per slab.)
 //
-// It serves calls whose scores are small: a bound on every score of a head is the soft-max reference of the head's rows.  Other calls
-// are left to tdp_fwd_band_kernel, behind this one, whose operand alpha Q K2 is also what the backward forms for large scores.
+// It serves calls whose scores are small and whose elements are finite: a bound on every score of a head is the soft-max reference of the
+// head's rows.  Other calls are left to tdp_fwd_band_kernel, behind this one, whose operand alpha Q K2 is also what the backward forms for
+// large scores; they pay 1 to 3 us for a kernel that ends at once.
 //
 // A CTA has two slots, each with an accumulator, two soft-max warpgroups (a query per thread, every other 32 of its columns) and every
 // other query tile: a step is one d of one j-tile for both.  All steps of a call form one line (heads, j-tiles, d) that is cut in
-// equal parts, one per CTA; a query tile whose steps are cut leaves its accumulators in the workspace, and a kernel behind this one
-// adds them up.
+// equal parts, one per CTA; a query tile whose steps are cut leaves its accumulators in the workspace, which the warp that brings the last
+// piece adds up, or in short calls (kEarlyBandTiles) the band kernel behind this one.
 //
-// What bounds it: no single unit.  A step takes 2700 cycles for both slots; issue slots are 60 % busy, the exponentials' unit 48 %, tensor
-// cores 45 %, and a slot's chain (scores, exponentials, P, value product) is not hidden behind the other slot's alone.  One soft-max
-// warpgroup per slot walking all 128 columns took 3200 cycles (220 us for 189, 810 for 679 below).  Forward, us per call, the
-// kernel of 4 queries x 32 rows -> this one: 16 heads T=2048 fp16 windows 128/128/32/32 471 -> 189, T=8192 1940 -> 682, T=2048 windows
-// 8/8/4/4 124 -> 51, 8 heads T=1000 126 -> 65, 16 heads T=500 128/128/48/48 124 -> 82; fp32 tensors, 8 heads T=2048 262 -> 119.
+// What bounds it: no single unit.  A step takes 2700 cycles for both slots (160 of 180 us at T=2048; the rest are the preparation, 8, the
+// launch, the first loads of items and the pieces); issue slots are 60 % busy, the exponentials' unit 48 %, tensor cores 39 %, and a slot's
+// chain (scores, exponentials, P, value product) is not hidden behind the other slot's alone.  One soft-max warpgroup per slot walking all
+// 128 columns took 3200 cycles.  Device time of a forward, us, the kernel of 4 queries x 32 rows -> this one: 16 heads T=2048 fp16 windows
+// 128/128/32/32 466 -> 180, T=8192 1933 -> 654, T=2048 windows 8/8/4/4 120 -> 43, 8 heads T=1000 117 -> 60, 16 heads T=500 128/128/48/48
+// 119 -> 75; fp32 tensors, 8 heads T=2048 254 -> 111.
 // Slower: masks of boundary columns by clamped FMAs (194 us for 189), a quarter of the exponentials as polynomials (194), value products
 // that start with the first warpgroup's half of P (190).
 //

@@ -211,7 +211,8 @@ int tritt_selftest_wait_expiry(int skip_arrival, long long limit_ticks, int* sta
 /*
  * What tritt_tdp_bwd does with these arguments on the tensor cores, per head (host only, for tests and planning):
  *   out[0]  query rows that run in exact fp32 on the CUDA cores (of the shard, from its first)
- *   out[1]  cells (q, j, k) that the tensor-core kernel executes, masked ones among them
+ *   out[1]  cells (q, j, k) that the tensor-core kernel executes, masked ones among them (for a narrow band whose heads may
+ *           go to the kernel that steps over diagonals: what the one over k would execute)
  *   out[2]  1 if that is the kernel that steps over queries (query shards), 0 if it steps over k
  * -12 if the call does not run on the tensor cores.  No counterpart in the reference.
  */
