@@ -18,7 +18,7 @@
 // piece adds up, or in short calls (kEarlyBandTiles) the band kernel behind this one.
 //
 // What bounds it: no single unit.  A step takes 2700 cycles for both slots (160 of 180 us at T=2048; the rest are the preparation, 8, the
-// launch, the first loads of items and the pieces); issue slots are 60 % busy, the exponentials' unit 48 %, tensor cores 39 %, and a slot's
+// launch, the first loads of items and the pieces); issue slots are 59 % busy, the exponentials' unit 47 %, tensor cores 38 %, and a slot's
 // chain (scores, exponentials, P, value product) is not hidden behind the other slot's alone.  One soft-max warpgroup per slot walking all
 // 128 columns took 3200 cycles.  Device time of a forward, us, the kernel of 4 queries x 32 rows -> this one: 16 heads T=2048 fp16 windows
 // 128/128/32/32 466 -> 180, T=8192 1933 -> 654, T=2048 windows 8/8/4/4 120 -> 43, 8 heads T=1000 117 -> 60, 16 heads T=500 128/128/48/48
