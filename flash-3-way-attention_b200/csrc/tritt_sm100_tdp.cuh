@@ -92,9 +92,11 @@ __device__ __forceinline__ uint32_t column_mask(int lo, int hi) {
 }
 
 // Bound on every score of a head, in log2 units: |s| max_q |Q_q| max |K2 element| max_j |K1_j|, s = alpha log2(e), from the forward's
-// statistics (fwd_prepare_kernel).  (Rounded one by one, so that all kernels that ask get the same answer.)
-__device__ __forceinline__ float head_bound(const float* stats, int BN, int bh, float s) {
-  const float q = __fsqrt_rn(__ldg(stats + BN + bh)), k2 = __fsqrt_rn(__ldg(stats + 2 * BN + bh)), k1 = __fsqrt_rn(__ldg(stats + bh));
+// statistics (fwd_prepare_kernel).  (Rounded one by one, so that all kernels that ask get the same answer.
+// FIRST: reads that the compiler keeps behind a wait for the preparation, as __ldg's need not be.)
+template <bool FIRST = false> __device__ __forceinline__ float head_bound(const float* stats, int BN, int bh, float s) {
+  auto read = [](const float* p) { return FIRST ? __ldcg(p) : __ldg(p); };
+  const float q = __fsqrt_rn(read(stats + BN + bh)), k2 = __fsqrt_rn(read(stats + 2 * BN + bh)), k1 = __fsqrt_rn(read(stats + bh));
   return __fmul_rn(__fmul_rn(__fmul_rn(fabsf(s), q), k2), k1);
 }
 

@@ -65,7 +65,7 @@ template <typename T16> __device__ __forceinline__ float diag_reference(float bo
 __device__ __forceinline__ bool diag_takes(const DiagParams& p) {
   bool large = false;   // (not >: inf * 0 is large as well; a head with an element that is not finite has an infinite bound)
   for (int bh = threadIdx.x; bh < p.g.BN; bh += blockDim.x)
-    large |= !(head_bound(p.stats, p.g.BN, bh, p.alpha * kLog2e) <= p.bound_limit);
+    large |= !(head_bound<true>(p.stats, p.g.BN, bh, p.alpha * kLog2e) <= p.bound_limit);
   return !__syncthreads_or(large);
 }
 
