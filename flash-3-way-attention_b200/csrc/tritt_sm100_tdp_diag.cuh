@@ -39,7 +39,8 @@ struct DiagParams {
   unsigned* arrived;     // [grid][kDiagArrivals], zero: pieces there are of the tiles begun in a CTA's part, by the tile's parity and by warp
   DiagGeometry g;
   float alpha, bound_limit;
-  bool early;            // tdp_fwd_band_kernel is launched ahead of this kernel's end, and adds up the pieces
+  bool band_merges;      // tdp_fwd_band_kernel adds up the pieces
+  bool early;            // ... and is launched ahead of this kernel's end
   int* status;
 };
 

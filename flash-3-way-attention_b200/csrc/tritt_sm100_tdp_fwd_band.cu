@@ -102,7 +102,7 @@ tdp_fwd_band_kernel(const __grid_constant__ CUtensorMap tmK1, const __grid_const
     if (diag_takes(diag)) return;
   }
   if constexpr (ROLE == kBehindDiagMerge) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");   // (launched ahead of that kernel's end)
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // (it may be launched ahead of that kernel's end)
     if (diag_takes(diag)) {
       // the kernel that steps over diagonals has done the call: what is left are the tiles that it cut
       diag_merge<T16>(diag);
@@ -540,9 +540,9 @@ int launch_band(const TdpArgs& a, const void* sv1, const float* k1n, const DiagP
   p.status = a.status_word;
   if (p.nq == 0) return 0;
   constexpr int kBehind = D == kDiagD ? kBehindDiag : kAlone, kBehindMerge = D == kDiagD ? kBehindDiagMerge : kAlone;
-  auto kern = !diag         ? tdp_fwd_band_kernel<D, T16, kAlone>
-              : diag->early ? tdp_fwd_band_kernel<D, T16, kBehindMerge>
-                            : tdp_fwd_band_kernel<D, T16, kBehind>;
+  auto kern = !diag               ? tdp_fwd_band_kernel<D, T16, kAlone>
+              : diag->band_merges ? tdp_fwd_band_kernel<D, T16, kBehindMerge>
+                                  : tdp_fwd_band_kernel<D, T16, kBehind>;
   TRITT_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
   const long items = (long)p.n_groups * BN;
   const int grid = (int)(items < num_sms() ? items : num_sms());

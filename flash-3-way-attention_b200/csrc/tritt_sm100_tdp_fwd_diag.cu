@@ -15,7 +15,7 @@
 // A CTA has two slots, each with an accumulator, two soft-max warpgroups (a query per thread, every other 32 of its columns) and every
 // other query tile: a step is one d of one j-tile for both.  All steps of a call form one line (heads, j-tiles, d) that is cut in
 // equal parts, one per CTA; a query tile whose steps are cut leaves its accumulators in the workspace, which the warp that brings the last
-// piece adds up, or in short calls (kEarlyBandTiles) the band kernel behind this one.
+// piece adds up, or in short calls (kMergingBandTiles) the band kernel behind this one.
 //
 // What bounds it: no single unit.  A step takes 2700 cycles for both slots (160 of 180 us at T=2048; the rest are the preparation, 8, the
 // launch, the first loads of items and the pieces); issue slots are 59 % busy, the exponentials' unit 47 %, tensor cores 38 %, and a slot's
@@ -266,7 +266,7 @@ tdp_fwd_diag_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         continue;
       }
       area[kDiagD / 2 * 128] = row_sum;
-      if (p.early) {
+      if (p.band_merges) {
         __syncwarp();
         continue;
       }
@@ -562,7 +562,10 @@ constexpr double kStepPrice = 1, kFullStepPrice = 1.4, kItemPrice = 1.3, kLaunch
 // last piece takes 7 us for them, most often at its end, the band kernel 3; in long calls the pieces of many tiles come in between.  us,
 // by the band kernel / here: 8 heads T=1000 fp16 61 / 65, 16 heads T=400 128/128/48/48 76.8 / 80.5, T=2048 8/8/4/4 42.6 / 44.8, T=2048
 // 128/128/32/32 181 / 179, T=8192 669 / 653, 4096 heads T=140 20/20/4/4 736 / 690.
-constexpr long kEarlyBandTiles = 128;
+constexpr long kMergingBandTiles = 128;
+// ... and below which it is launched ahead of this one's end.  Large scores, us early / not: 16 heads T=1200 16/16/8/8 81 / 83, T=2048 13/2/12/2
+// (56 tiles) 123 / 127; but with inputs that are not in L2 yet, where its CTAs then run slower, 32 heads T=1480 (80) 186 / 181, T=1726 (94) 232 / 208.
+constexpr long kEarlyBandTiles = 80;
 
 long diag_steps(int B, int N, int T, int band) { return (long)B * N * ((T + 127) / 128) * (band + 1); }
 // Tiles of a CTA of tdp_fwd_band_kernel: the groups of four queries have a block of 32 K2 rows at first, and as many as reach back `reach`
@@ -637,7 +640,9 @@ bool sm100_tdp_fwd_diag_plan(const TdpArgs& a, void* workspace, size_t workspace
   const long steps = diag_steps(a.B, a.N, a.T, m.kkl + m.kkr);
   const int grid = diag_grid(steps);
   p = DiagParams{};
-  p.early = band_tiles_of_cta((long)a.B * a.N, a.T, min(m.k2w, m.k1w + m.kkr)) < kEarlyBandTiles;
+  const double band_tiles = band_tiles_of_cta((long)a.B * a.N, a.T, min(m.k2w, m.k1w + m.kkr));
+  p.band_merges = band_tiles < kMergingBandTiles;
+  p.early = band_tiles < kEarlyBandTiles;
   p.out = a.out_o;
   p.lse = a.out_lse;
   p.k1 = a.k1;
