@@ -1092,15 +1092,16 @@ int prepare_fwd(const TdpArgs& a, const DiagParams* diag, T16** sv1_out, float**
   int blocks = 1;
   while (blocks < 8 && blocks * kPrepThreads * 8 < head_elems && 2L * BN * blocks <= resident) blocks *= 2;
   const int passes = (head_elems - 1) / (blocks * kPrepThreads * 8) + 1;
-  // Larger blocks where passes are many and SMs free.  us with 256 / 512 / 1024 threads (diag 256 / 512): 4 heads, 2 passes 3.8 / 3.3 / 4.2
-  // (3.6 / 3.3), 5 passes 6.0 / 4.9 / 5.4 (5.2 / 4.6), 8 passes 8.0 / 5.8 / 5.5; 16 heads, 3 passes 4.6 / 4.6 / 5.4 (4.3 / 4.8), 5 passes
-  // 6.2 / 5.8 / 7.8 (5.6 / 6.0), 8 passes 8.5 / 7.0 / 7.7 (7.6 / 7.2), 32 passes 29 / 19.8 / 18.1; 64 heads, 4 passes 7.2 / 7.6 / 10.8
-  // (7.5 / 10.0), 8 passes 12.4 / 11.6 / 15.4 (13.3 / 17.1).
+  // Larger blocks where passes are many and SMs free.  us with 256 / 512 / 1024 threads (diag 256 / 512), inputs in L2, and in HBM in
+  // brackets: 8 heads, 4 passes 5.3 / 4.1 / 4.3 [8.4 / 5.8 / 4.8] (4.7 / 4.0 [6.6 / 5.0]); 16 heads, 2 passes 4.0 / 3.8 / 5.7 [5.6 / 4.4 / 6.0]
+  // (3.8 / 4.1 [4.8 / 4.6]), 5 passes 6.3 / 6.0 / 7.3 [10.2 / 8.0 / 8.1] (5.7 / 6.1 [8.2 / 7.5]), 8 passes 8.7 / 7.1 / 7.7 [14.8 / 9.8 / 8.5]
+  // (7.7 / 7.3 [11.4 / 8.9]), 32 passes 31 / 20 / 18 [50 / 30 / 21]; 32 heads, 3 passes 4.9 / 5.0 / 6.0 [8.0 / 7.0 / 6.5] (4.6 / 5.3 [7.0 / 6.8]),
+  // 7 passes 8.1 / 7.3 / 7.8 [14.7 / 11.2 / 9.6] (7.4 / 7.4 [12.1 / 10.6]); 64 heads, 4 passes 7.1 / 7.6 / 10.8 [11.5 / 10.0 / 12.6] (7.5 / 10.0 [11.0 / 13.1]).
   const long grid = (long)BN * blocks, sms = num_sms();
   const bool few = 2 * grid <= sms;
   int threads = kPrepThreads;
-  if (passes > (few ? 1 : diag ? 6 : grid <= 2 * sms ? 2 : 4) && 2 * grid <= resident) threads = 512;
-  if (!diag && passes >= (few ? 8 : 16) && grid <= sms) threads = kPrepMost;
+  if (passes >= (few || !diag ? 2 : 4) && 2 * grid <= resident) threads = 512;
+  if (!diag && passes >= (few ? 4 : 6) && grid <= 2 * sms) threads = kPrepMost;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
