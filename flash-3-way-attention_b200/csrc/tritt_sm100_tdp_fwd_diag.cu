@@ -553,11 +553,11 @@ constexpr int kMinSteps = 12;      // of a CTA
 size_t area_bytes(int grid) { return (size_t)grid * kDiagAreas * kDiagAreaFloats * sizeof(float); }
 size_t scratch_bytes(int grid) { return area_bytes(grid) + (size_t)grid * kDiagArrivals * sizeof(unsigned); }
 // This kernel is asked where it costs less than the band kernel, in us: a step 1 (narrow windows, most columns masked) to 1.4, an item (a
-// j-tile) 1.3 beside its steps, launch and first item 14; a tile of the band kernel 1.6 to 2.  us of a call with small scores, by the
-// band kernel / here, of CTAs of steps / tiles: 12 / 17 (a diagonal an item) 38 / 42, 12 / 14 32 / 34, 13 / 14 33 / 36, 16 / 15 36 / 38, 36 / 18
+// j-tile) 1.3 beside its steps, launch and first item 14, and 3 more, as large scores pay 2 to 3 for the question; a tile of the band kernel
+// 1.6 to 2.1.  us of a call with small scores, by the band kernel / here, of CTAs of steps / tiles: 12 / 17 (a diagonal an item) 38 / 42, 12 / 14 32 / 34, 13 / 14 33 / 36, 16 / 15 36 / 38, 36 / 18
 // (T=129 128/128/48/48) 36 / 57, 53 / 28 64 / 71, 65 / 42 86 / 88, 70 / 27 59 / 89;  114 / 81 163 / 150, 28 / 68 117 / 60, 42 / 47 96 / 76, 16 / 56 119 / 43,
 // 86 / 69 143 / 111, 112 / 280 466 / 179.
-constexpr double kStepPrice = 1, kFullStepPrice = 1.4, kItemPrice = 1.3, kLaunchPrice = 14, kTilePrice = 1.9;
+constexpr double kStepPrice = 1, kFullStepPrice = 1.4, kItemPrice = 1.3, kLaunchPrice = 17, kTilePrice = 2;
 // Tiles of a CTA of tdp_fwd_band_kernel below which that kernel adds up the pieces, launched ahead of this one's end.  A CTA that brings the
 // last piece takes 7 us for them, most often at its end, the band kernel 3; in long calls the pieces of many tiles come in between.  us,
 // by the band kernel / here: 8 heads T=1000 fp16 61 / 65, 16 heads T=400 128/128/48/48 76.8 / 80.5, T=2048 8/8/4/4 42.6 / 44.8, T=2048
